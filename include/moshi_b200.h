@@ -570,6 +570,15 @@ int b200_op_linear_sk(const void* x_dev, const void* w_tiles_dev, void* y_dev, c
  * (b200_op_linear_sk with smem_budget = -1 keeps the swap-AB kernels at every M: the comparison row of tools/kbench.py.) */
 int b200_op_linear_ns(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K,
                       int epi, int gate_rows, int cluster, void* stream);
+/* The decoder LM's linear for more than 256 activation rows (csrc/gemm_wide.cu): y[M,N] = x[M,K] . w^T over packed tiles
+ * (b200_op_pack_tiles, epi 0) or, with packed = 0, a row-major w [N,K].  ldy: elements per result row; splits: ranges
+ * that k is cut into (0 = the handle's choice).  K % 8 == 0.  Synchronises unless splits = 1 (test helper). */
+int b200_op_linear_wide(const void* x_dev, const void* w_dev, void* y_dev, int M, int N, int K, int ldy, int packed, int splits, void* stream);
+/* The routed experts' grouped product: counts_host[E] rows of x (neighbouring rows, expert after expert; sum = M) times the expert's
+ * row-major w [E,N,K]; act as the handle's epilogues: 0 none, 1 relu^2, 2 clamped gated unit (limit) and 3 silu gated unit on rows
+ * that interleave gate and value (y has N / 2 columns), 4 erf GELU.  ldy: elements per result row.  Synchronises (test helper). */
+int b200_op_grouped_wide(const void* x_dev, const void* w_dev, void* y_dev, const int32_t* counts_host, int E, int M, int N, int K, int ldy,
+                         int act, float limit, void* stream);
 /* Up to how many activation rows the linears take the GEMV path (plain 16-byte loads on the CUDA cores instead of the
  * tensor-core GEMM; csrc/gemm_sk.cu): 0..4, default 2 (or B200_GEMV_MAX_M).  Returns the previous value. */
 int b200_op_set_gemv_max_rows(int max_rows);

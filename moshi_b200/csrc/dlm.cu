@@ -17,6 +17,7 @@
 #include "dlm_mixers4.cuh"
 #include "dlm_mixers5.cuh"
 #include "gemm_sk.cuh"
+#include "gemm_wide.cuh"
 #include "lm_kernels.cuh"
 
 using namespace b200;
@@ -258,6 +259,12 @@ int linear<float>(b200_dlm* h, const float* x, long long ldx, const Weight& w, f
 
 template <>
 int linear<bf16>(b200_dlm* h, const bf16* x, long long ldx, const Weight& w, bf16* y, long long ldy, int M) {
+  if (w.tiles && M > 256 && ldx % 8 == 0) {
+    tc::WideGemm g;
+    g.x = x; g.ldx = ldx; g.x_rows = M; g.w = w.tiles; g.packed = true; g.y = y; g.ldy = ldy; g.M = M; g.N = w.N; g.K = w.K; g.err = h->err;
+    g.ws = h->sk_ws; g.ws_bytes = tc::sk_workspace_bytes(256); g.counters = h->sk_counters; g.n_counters = tc::SK_MAX_TILES;
+    if (tc::wide_supported(g)) return tc::wide_gemm(g, h->stream);
+  }
   if (w.tiles && ldx % 8 == 0 && ldy % 8 == 0) {
     tc::SkTuning t;
     for (int m0 = 0; m0 < M; m0 += 256) {          // the LM's GEMM takes up to 256 rows per launch
