@@ -147,7 +147,8 @@ struct b200_dlm {
   float *embw = nullptr, *h32 = nullptr, *qkv32 = nullptr, *scan32 = nullptr, *gate32 = nullptr, *attn32 = nullptr, *route32 = nullptr, *moe_w = nullptr, *scan_prep = nullptr, *scan_v = nullptr;
   void *mixo2 = nullptr, *obuf2 = nullptr, *yexp = nullptr;
   int *moe_idx = nullptr, *moe_rank = nullptr, *moe_perm = nullptr, *moe_row_tok = nullptr, *moe_tile_e = nullptr, *moe_tile_r0 = nullptr,
-      *moe_tile_n = nullptr, *moe_ntiles = nullptr;
+      *moe_tile_n = nullptr, *moe_ntiles = nullptr;      // moe_ntiles: tiles, rows
+  bf16* moe_x = nullptr;               // [pairs][width] the tokens' rows in the grouped order
   float* sk_ws = nullptr; int* sk_counters = nullptr;
   tc::GemmPlanCache plans;
   // parallel-residual block: recurrences that cannot run as segments (the delta rule) take the step's entries whole
@@ -835,6 +836,25 @@ int window_attention(b200_dlm* h, const Layer& L, int n_tok, int max_ctx, long l
 }
 
 // routed experts on the rows of hb -> yexp [tokens * top][W] (row t * top + k = the k-th chosen expert's output for token t)
+// the routed experts' two products on the tensor cores: the tokens' rows are copied into the grouped order once, so that a tile's rows are
+// neighbours; act: the first product's epilogue (WIDE_*), its result has F columns
+int grouped_products(b200_dlm* h, const Layer& L, const bf16* hb, int n_tok, int N1, int act, float limit) {
+  const int W = h->cfg.width, F = L.c.ff, pairs = n_tok * L.c.top, E = L.c.experts;
+  B200_LAUNCH(moe_gather_kernel, pairs, 128, 0, h->stream, reinterpret_cast<const uint4*>(hb), h->moe_row_tok, h->moe_ntiles + 1, reinterpret_cast<uint4*>(h->moe_x), W / 8);
+  tc::WideGemm g;
+  g.tile_e = h->moe_tile_e; g.tile_r0 = h->moe_tile_r0; g.tile_n = h->moe_tile_n; g.n_tiles = h->moe_ntiles;
+  g.max_tiles = ceil_div(pairs, tc::WIDE_EXPERT_ROWS) + std::min(E, pairs);
+  g.max_rows = n_tok;                  // a token chooses an expert once
+  g.M = pairs; g.x_rows = pairs; g.err = h->err;
+  tc::WideGemm down = g;
+  g.x = h->moe_x; g.ldx = W; g.w = L.ups; g.w_rows = (long long)E * N1; g.e_rows = N1; g.N = N1; g.K = W;
+  g.y = static_cast<bf16*>(h->act); g.ldy = F; g.act = act; g.limit = limit;
+  B200_TRY(tc::wide_gemm(g, h->stream));
+  down.x = static_cast<const bf16*>(h->act); down.ldx = F; down.w = L.downs; down.w_rows = (long long)E * W; down.e_rows = W; down.N = W; down.K = F;
+  down.y = static_cast<bf16*>(h->yexp); down.ldy = W; down.y_rows = h->moe_perm;
+  return tc::wide_gemm(down, h->stream);
+}
+
 template <typename T>
 int routed_experts(b200_dlm* h, const Layer& L, const T* hb, int n_tok) {
   const int W = h->cfg.width, E = L.c.experts, top = L.c.top, F = L.c.ff, pairs = n_tok * top;
@@ -843,7 +863,7 @@ int routed_experts(b200_dlm* h, const Layer& L, const T* hb, int n_tok) {
   B200_LAUNCH(moe_route_kernel, ceil_div(n_tok, 4), 128, 0, st, h->route32, E, top, h->moe_idx, h->moe_w, n_tok);
   bool mma = false;
   if constexpr (sizeof(T) == 2) mma = h->attn_tc && W % 16 == 0 && F % 16 == 0;
-  const int tile_m = mma ? 128 : 64;
+  const int tile_m = mma ? tc::WIDE_EXPERT_ROWS : 64;
   B200_LAUNCH(moe_group_kernel, 1, 1024, (size_t)2 * E * sizeof(int), st, h->moe_idx, pairs, top, E, h->moe_rank, h->moe_perm, h->moe_row_tok,
               h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, tile_m);
   B200_TRY(check_launch("moe route / group"));
@@ -853,17 +873,7 @@ int routed_experts(b200_dlm* h, const Layer& L, const T* hb, int n_tok) {
   const T* ups = static_cast<const T*>(L.ups);
   const T* downs = static_cast<const T*>(L.downs);
   if (mma) {
-    if constexpr (sizeof(T) == 2) {
-      static bool attr_set = false;
-      if (!attr_set) {
-        B200_CUDA(cudaFuncSetAttribute(grouped_gemm_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GG_SMEM));
-        attr_set = true;
-      }
-      B200_LAUNCH(grouped_gemm_mma_kernel, dim3(ceil_div(F, 128), max_tiles), 256, GG_SMEM, st, hb, (long long)W, h->moe_row_tok, ups, (long long)W, (long long)F * W,
-                  act, (long long)F, (const int*)nullptr, h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, F, W, 1);
-      B200_LAUNCH(grouped_gemm_mma_kernel, dim3(ceil_div(W, 128), max_tiles), 256, GG_SMEM, st, act, (long long)F, (const int*)nullptr, downs, (long long)F, (long long)W * F,
-                  yexp, (long long)W, h->moe_perm, h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, W, F, 0);
-    }
+    if constexpr (sizeof(T) == 2) B200_TRY(grouped_products(h, L, hb, n_tok, F, tc::WIDE_RELU2, 0.f));
   } else {
     B200_LAUNCH((grouped_gemm_kernel<T, T, T>), dim3(ceil_div(F, 64), max_tiles), 256, 0, st, hb, (long long)W, h->moe_row_tok, ups, (long long)W, (long long)F * W,
                 act, (long long)F, (const int*)nullptr, h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, F, W, 1);
@@ -1809,7 +1819,7 @@ int routed_experts_glu(b200_dlm* h, const Layer& L, const T* hb, int n_tok) {
   }
   bool mma = false;
   if constexpr (sizeof(T) == 2) mma = h->attn_tc && W % 16 == 0 && F % 16 == 0;
-  const int tile_m = mma ? 128 : 64;
+  const int tile_m = mma ? tc::WIDE_EXPERT_ROWS : 64;
   B200_LAUNCH(moe_group_kernel, 1, 1024, (size_t)2 * E * sizeof(int), st, h->moe_idx, pairs, top, E, h->moe_rank, h->moe_perm, h->moe_row_tok,
               h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, tile_m);
   B200_TRY(check_launch("moe route / group"));
@@ -1821,18 +1831,9 @@ int routed_experts_glu(b200_dlm* h, const Layer& L, const T* hb, int n_tok) {
   const T* downs = static_cast<const T*>(L.downs);
   const long long n = (long long)pairs * F;
   if (mma) {
-    if constexpr (sizeof(T) == 2) {
-      static bool attr_set = false;
-      if (!attr_set) {
-        B200_CUDA(cudaFuncSetAttribute(grouped_gemm_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GG_SMEM));
-        attr_set = true;
-      }
-      // gate and value rows of an expert are interleaved, so the first product's epilogue holds both of an output in one thread
-      B200_LAUNCH(grouped_gemm_mma_kernel, dim3(ceil_div(N1, 128), max_tiles), 256, GG_SMEM, st, hb, (long long)W, h->moe_row_tok, ups, (long long)W, (long long)N1 * W,
-                  act, (long long)F, (const int*)nullptr, h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, N1, W, gelu ? 4 : silu ? 3 : 2, L.c.expert_limit);
-      B200_LAUNCH(grouped_gemm_mma_kernel, dim3(ceil_div(W, 128), max_tiles), 256, GG_SMEM, st, act, (long long)F, (const int*)nullptr, downs, (long long)F, (long long)W * F,
-                  yexp, (long long)W, h->moe_perm, h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, W, F, 0, 0.f);
-    }
+    // gate and value rows of an expert are interleaved, so the first product's epilogue holds both of an output in one thread
+    if constexpr (sizeof(T) == 2)
+      B200_TRY(grouped_products(h, L, hb, n_tok, N1, gelu ? tc::WIDE_GELU : silu ? tc::WIDE_SILU_GLU : tc::WIDE_CLAMPED_GLU, L.c.expert_limit));
   } else {
     B200_LAUNCH((grouped_gemm_kernel<T, T, T>), dim3(ceil_div(N1, 64), max_tiles), 256, 0, st, hb, (long long)W, h->moe_row_tok, ups, (long long)W, (long long)N1 * W,
                 gelu ? act : act2, (long long)N1, (const int*)nullptr, h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, N1, W, gelu ? 4 : 0);
@@ -2851,7 +2852,8 @@ int b200_dlm_cache_begin(b200_dlm* h, int slots, int capacity, int max_step_toke
       B200_TRY(A.alloc_t(&h->moe_tile_e, tiles));
       B200_TRY(A.alloc_t(&h->moe_tile_r0, tiles));
       B200_TRY(A.alloc_t(&h->moe_tile_n, tiles));
-      B200_TRY(A.alloc_t(&h->moe_ntiles, 1));
+      B200_TRY(A.alloc_t(&h->moe_ntiles, 2));
+      if (!h->f32) B200_TRY(A.alloc_t(&h->moe_x, (size_t)pairs * W, false));
       B200_TRY(A.alloc(&h->yexp, pairs * W * es));
       B200_TRY(A.alloc(&h->act2, T * 2 * max_eff * es));
       max_ff = std::max(max_ff, max_eff);       // the experts' hidden rows: one per (token, chosen expert)
@@ -2890,7 +2892,8 @@ int b200_dlm_cache_begin(b200_dlm* h, int slots, int capacity, int max_step_toke
       B200_TRY(A.alloc_t(&h->moe_tile_e, tiles));
       B200_TRY(A.alloc_t(&h->moe_tile_r0, tiles));
       B200_TRY(A.alloc_t(&h->moe_tile_n, tiles));
-      B200_TRY(A.alloc_t(&h->moe_ntiles, 1));
+      B200_TRY(A.alloc_t(&h->moe_ntiles, 2));
+      if (!h->f32) B200_TRY(A.alloc_t(&h->moe_x, (size_t)pairs * W, false));
       B200_TRY(A.alloc(&h->yexp, pairs * W * es));
       max_ff *= max_top;        // the experts' hidden rows: one per (token, chosen expert)
     }

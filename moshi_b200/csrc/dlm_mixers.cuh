@@ -1068,7 +1068,7 @@ __global__ void __launch_bounds__(256) sublayer_end_kernel(float* __restrict__ x
 // Routed experts.  moe_route_kernel: per token (one warp) the `top` largest router logits (ties: the lower index) and the
 // softmax over those alone.  moe_group_kernel (ONE CTA): sorts the (token, choice) pairs by expert: pos-th row of the grouped
 // order is pair perm[pos] of token row_tok[pos], and cuts every expert's rows into tiles of tile_m for the grouped products
-// (tile -> expert, first row, rows); n_tiles[0] = number of tiles.  The order inside an expert follows the atomics and may
+// (tile -> expert, first row, rows); n_tiles = {number of tiles, number of rows}.  The order inside an expert follows the atomics and may
 // differ from run to run; a row's result does not depend on it (every row of a product is summed on its own).  Choices from E
 // on stand for no feed-forward and get no row.
 // ---------------------------------------------------------------------------------------------------------------------------
@@ -1118,6 +1118,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int* __restrict__
       o += cnt[e];
     }
     n_tiles[0] = nt;
+    n_tiles[1] = o;
   }
   __syncthreads();
   for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
@@ -1126,6 +1127,15 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int* __restrict__
     perm[pos] = i;
     row_tok[pos] = i / top;
   }
+}
+
+// the grouped order's rows side by side: out[pos] = x[row_tok[pos]], row16 16-byte pieces per row
+__global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ row_tok, const int* __restrict__ n_rows,
+                                                         uint4* __restrict__ out, int row16) {
+  if ((int)blockIdx.x >= n_rows[0]) return;
+  const uint4* src = x + (long long)row_tok[blockIdx.x] * row16;
+  uint4* dst = out + (long long)blockIdx.x * row16;
+  for (int i = threadIdx.x; i < row16; i += blockDim.x) dst[i] = src[i];
 }
 
 // Grouped product of the routed experts: for tile (expert e, rows pos0 .. pos0 + n - 1 of the grouped order)
@@ -1184,109 +1194,11 @@ __global__ void __launch_bounds__(256) grouped_gemm_kernel(const TA* __restrict_
     }
 }
 
-// The same grouped product on the tensor cores (mma.sync m16n8k16, bf16 in, fp32 accumulate): K a multiple of 16, rows of A
-// and B on 16-byte boundaries; act 2: gate and value rows of B alternate and the epilogue writes
-// min(g, limit) * sigmoid(1.702 min(g, limit)) * (clamp(u, -limit, limit) + 1) into column n / 2, act 3 silu(g) * u;
-// act 4: erf GELU of every column.  CTA tile 128 x 128 (tiles of 128 rows in the tile table), 8 warps of 32 x 64, 64-element
-// k-steps through two shared-memory buffers filled by cp.async (chunks outside M, N or K are zero-filled by a copy of size 0).
+// 16 bytes into shared memory; zeros where the source does not exist (a copy of size 0)
 __device__ __forceinline__ void cp_async_16_or_zero(void* smem_dst, const void* src, bool valid) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   const int n = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-
-constexpr int GG_BM = 128, GG_BN = 128, GG_BK = 64, GG_ST = GG_BK + 8;
-constexpr size_t GG_SMEM = (size_t)2 * (GG_BM + GG_BN) * GG_ST * 2 + GG_BM * 4;
-
-__global__ void __launch_bounds__(256, 2) grouped_gemm_mma_kernel(const bf16* __restrict__ A, long long lda, const int* __restrict__ a_rows,
-                                                                  const bf16* __restrict__ B, long long ldb, long long sb, bf16* __restrict__ C,
-                                                                  long long ldc, const int* __restrict__ c_rows, const int* __restrict__ tile_expert,
-                                                                  const int* __restrict__ tile_row0, const int* __restrict__ tile_rows,
-                                                                  const int* __restrict__ n_tiles, int N, int K, int act, float limit = 0.f) {
-  constexpr int BM = GG_BM, BN = GG_BN, BK = GG_BK, ST = GG_ST;
-  if ((int)blockIdx.y >= n_tiles[0]) return;
-  extern __shared__ __align__(16) unsigned char gg_smem[];
-  bf16 (*As)[BM][ST] = reinterpret_cast<bf16 (*)[BM][ST]>(gg_smem);                                  // [2][BM][ST]
-  bf16 (*Bs)[BN][ST] = reinterpret_cast<bf16 (*)[BN][ST]>(gg_smem + (size_t)2 * BM * ST * 2);        // [2][BN][ST]
-  int* arow = reinterpret_cast<int*>(gg_smem + (size_t)2 * (BM + BN) * ST * 2);
-  const int pos0 = tile_row0[blockIdx.y], M = tile_rows[blockIdx.y];
-  B += (long long)tile_expert[blockIdx.y] * sb;
-  const int n0 = blockIdx.x * BN;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3, mi = lane >> 3;
-  const int wm = (warp & 3) * 32, wn = (warp >> 2) * 64;
-  if (threadIdx.x < BM) arow[threadIdx.x] = threadIdx.x < M ? (a_rows ? a_rows[pos0 + threadIdx.x] : pos0 + threadIdx.x) : 0;
-  __syncthreads();
-  float acc[2][8][4];
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b) { acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.f; }
-  auto load = [&](int k0, int buf) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = threadIdx.x + 256 * j;
-      const int rr = c >> 3, kk = (c & 7) * 8;
-      const bool va = rr < M && k0 + kk < K, vb = n0 + rr < N && k0 + kk < K;
-      cp_async_16_or_zero(&As[buf][rr][kk], va ? A + (long long)arow[rr] * lda + k0 + kk : A, va);
-      cp_async_16_or_zero(&Bs[buf][rr][kk], vb ? B + (long long)(n0 + rr) * ldb + k0 + kk : B, vb);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  load(0, 0);
-  for (int k0 = 0, it = 0; k0 < K; k0 += BK, ++it) {
-    const int buf = it & 1;
-    if (k0 + BK < K) { load(k0 + BK, buf ^ 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-    else asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-#pragma unroll
-    for (int ks = 0; ks < BK / 16; ++ks) {
-      unsigned a[2][4];
-#pragma unroll
-      for (int mf = 0; mf < 2; ++mf) ldmatrix_x4(a[mf], &As[buf][wm + mf * 16 + (mi & 1) * 8 + (lane & 7)][ks * 16 + (mi >> 1) * 8]);
-#pragma unroll
-      for (int np = 0; np < 4; ++np) {
-        unsigned b[4];
-        ldmatrix_x4(b, &Bs[buf][wn + np * 16 + (mi >> 1) * 8 + (lane & 7)][ks * 16 + (mi & 1) * 8]);
-#pragma unroll
-        for (int mf = 0; mf < 2; ++mf) {
-          mma_bf16_16816(acc[mf][2 * np], a[mf], b[0], b[1]);
-          mma_bf16_16816(acc[mf][2 * np + 1], a[mf], b[2], b[3]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  const bool pair_ok = (ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(C) & 3) == 0;      // two columns in one 4-byte store
-#pragma unroll
-  for (int mf = 0; mf < 2; ++mf)
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      const int m = wm + mf * 16 + g + 8 * hf;
-      if (m >= M) continue;
-      const long long crow = c_rows ? c_rows[pos0 + m] : pos0 + m;
-#pragma unroll
-      for (int nb = 0; nb < 8; ++nb) {
-        const int n = n0 + wn + nb * 8 + 2 * t4;
-        float v0 = acc[mf][nb][2 * hf], v1 = acc[mf][nb][2 * hf + 1];
-        if (act == 2 || act == 3) {      // rows of B interleave gate and value: columns (n, n + 1) are one output, column n / 2 of C
-          if (n + 1 < N && act == 3) {
-            C[crow * ldc + (n >> 1)] = __float2bfloat16_rn(v0 / (1.f + expf(-v0)) * v1);
-          } else if (n + 1 < N) {
-            const float g = fminf(v0, limit), u = fminf(fmaxf(v1, -limit), limit);
-            C[crow * ldc + (n >> 1)] = __float2bfloat16_rn(g / (1.f + expf(-1.702f * g)) * (u + 1.f));
-          }
-          continue;
-        }
-        if (act == 4) { v0 = 0.5f * v0 * (1.f + erff(v0 * 0.7071067811865476f)); v1 = 0.5f * v1 * (1.f + erff(v1 * 0.7071067811865476f)); }
-        else if (act) { v0 = fmaxf(v0, 0.f); v0 *= v0; v1 = fmaxf(v1, 0.f); v1 *= v1; }
-        if (n + 1 < N && pair_ok) {
-          *reinterpret_cast<unsigned*>(C + crow * ldc + n) = pack_bf16(v0, v1);
-        } else {
-          if (n < N) C[crow * ldc + n] = __float2bfloat16_rn(v0);
-          if (n + 1 < N) C[crow * ldc + n + 1] = __float2bfloat16_rn(v1);
-        }
-      }
-    }
 }
 
 // logits <- cap * tanh(logits / cap) on fp32 rows; `in` may be the padded bf16 rows of the tensor-core head (ld elements per row)

@@ -9,7 +9,9 @@
 //     once and the rows stay in L2; two accumulators in TMEM, the epilogue of a tile runs under the products of the next.
 //   * weights either as the packed SWIZZLE_128B tiles of gemm_sk.cu (fetched as they are by an unswizzled box) or row-major (swizzled
 //     by the TMA unit): the packed form serves the decoding kernels too, and nothing is held twice.
-//   * grouped products: the row tiles come from a table on the device (expert, first row, rows), rows of one expert being neighbours.
+//   * grouped products: the row tiles come from a table on the device (expert, first row, rows), rows of one expert being neighbours; few
+//     rows per expert make it a stream of the experts' weights, up to 192 KB of them in flight per SM.  16 experts of width 2048 and
+//     hidden size 4096, both products: 2000 rows 450 -> 170 us, 16 rows 191 -> 114 us (the mma.sync kernel before had two stages of 64 k).
 //
 // Bound by the tensor pipe: 2048 x 2048 -> 14848 columns 94 us (1321 TFLOP/s, 0.79 of the measured cuBLAS rate; cuBLAS itself 90 us), 2048 x
 // 8192 -> 2048 52 us (1325); with one launch of gemm_ns.cu per 256 rows, 58 of 148 SMs busy at a time, the four linears of such a layer took
