@@ -258,12 +258,17 @@ int linear<float>(b200_dlm* h, const float* x, long long ldx, const Weight& w, f
   return gemm_nt(h->stream, x, ldx, 0, static_cast<const float*>(w.rm), (long long)w.K, 0, y, ldy, 0, M, w.N, w.K, 1, 1.f);
 }
 
+tc::WideGemm wide_linear(b200_dlm* h, const bf16* x, long long ldx, const Weight& w, bf16* y, long long ldy, int M) {
+  tc::WideGemm g;
+  g.x = x; g.ldx = ldx; g.x_rows = M; g.w = w.tiles; g.packed = true; g.y = y; g.ldy = ldy; g.M = M; g.N = w.N; g.K = w.K; g.err = h->err;
+  g.ws = h->sk_ws; g.ws_bytes = tc::sk_workspace_bytes(256); g.counters = h->sk_counters; g.n_counters = tc::SK_MAX_TILES;
+  return g;
+}
+
 template <>
 int linear<bf16>(b200_dlm* h, const bf16* x, long long ldx, const Weight& w, bf16* y, long long ldy, int M) {
   if (w.tiles && M > 256 && ldx % 8 == 0) {
-    tc::WideGemm g;
-    g.x = x; g.ldx = ldx; g.x_rows = M; g.w = w.tiles; g.packed = true; g.y = y; g.ldy = ldy; g.M = M; g.N = w.N; g.K = w.K; g.err = h->err;
-    g.ws = h->sk_ws; g.ws_bytes = tc::sk_workspace_bytes(256); g.counters = h->sk_counters; g.n_counters = tc::SK_MAX_TILES;
+    const tc::WideGemm g = wide_linear(h, x, ldx, w, y, ldy, M);
     if (tc::wide_supported(g)) return tc::wide_gemm(g, h->stream);
   }
   if (w.tiles && ldx % 8 == 0 && ldy % 8 == 0) {
@@ -277,6 +282,19 @@ int linear<bf16>(b200_dlm* h, const bf16* x, long long ldx, const Weight& w, bf1
   }
   if (!w.rm) B200_FAIL(B200_ERR_STATE, "decoder LM: a packed linear met an unaligned activation stride");
   return gemm_nt(h->stream, x, ldx, 0, static_cast<const bf16*>(w.rm), (long long)w.K, 0, y, ldy, 0, M, w.N, w.K, 1, 1.f);
+}
+
+// the concatenated projection of a gated parallel block; for many tokens the columns of W_up go through relu(.)^2 straight to act
+template <typename T>
+int projection_with_unit(b200_dlm* h, const Layer& L, const T* hb, T* proj, T* act, int M, bool* done) {
+  if constexpr (sizeof(T) == 2) {
+    if (L.cat.tiles && M > 256 && L.c.mlp == B200_MLP_DENSE_RELU2 && L.off_up % 32 == 0 && L.c.ff % 32 == 0) {
+      tc::WideGemm g = wide_linear(h, hb, h->cfg.width, L.cat, proj, L.ldp, M);
+      g.act_from = L.off_up; g.act_to = L.off_up + L.c.ff; g.y2 = act; g.ldy2 = L.c.ff;
+      if (tc::wide_supported(g)) { *done = true; return tc::wide_gemm(g, h->stream); }
+    }
+  }
+  return linear<T>(h, hb, h->cfg.width, L.cat, proj, L.ldp, M);
 }
 
 template <typename T, int NCH, int RPW>
@@ -377,6 +395,14 @@ int mark(b200_dlm* h, int cls) {       // cls >= 0 opens an interval of that cla
 }
 #define TIMED(cls, ...) do { B200_TRY(mark(h, cls)); __VA_ARGS__; B200_TRY(mark(h, -1)); } while (0)
 
+// the head's rows (bf16 of ld elements each, or null: fp32 in place) -> h->logits and the caller's buffer
+int finish_logits(b200_dlm* h, const bf16* in_bf, long long ld, int n_want, int mode, float c, float* logits_out) {
+  const long long n = (long long)n_want * h->cfg.vocab;
+  const int vec = h->cfg.vocab % 8 == 0 && ((uintptr_t)logits_out & 15) == 0;
+  B200_LAUNCH(logit_rows_kernel, (unsigned)ceil_div64(n, vec ? 2048 : 256), 256, 0, h->stream, in_bf, ld, h->logits, logits_out, h->cfg.vocab, n, mode, c, vec);
+  return check_launch("logits");
+}
+
 template <typename T>
 int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out) {
   const b200_dlm_config& c = h->cfg;
@@ -392,7 +418,9 @@ int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out
     const Layer& L = h->layers[li];
     const int H = L.c.a.heads, dk = L.c.a.dim, dv = L.c.a.vdim, r = L.c.a.kv_rank;
     T* proj = static_cast<T*>(h->proj);
-    TIMED(CLS_LINEAR, B200_TRY(linear<T>(h, hb, W, L.cat, proj, L.ldp, n_tok)));
+    T* act = static_cast<T*>(h->act);
+    bool squared = false;                // the feed-forward's unit is done by the projection's epilogue
+    TIMED(CLS_LINEAR, B200_TRY(projection_with_unit<T>(h, L, hb, proj, act, n_tok, &squared)));
     // mixer: latent attention
     TIMED(CLS_ELEMENTWISE, B200_LAUNCH(latent_append_kernel<T>, ceil_div(n_tok, 4), 128, 0, st, proj, (long long)L.ldp, L.off_dkv, L.cnorm, static_cast<T*>(L.cache),
                 h->cap, r, meta + h->off_slot, meta + h->off_pos, n_tok, c.norm_eps));
@@ -409,9 +437,8 @@ int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out
     // feed-forward
     T* ffo = nullptr;
     if (L.c.mlp == B200_MLP_DENSE_RELU2) {
-      T* act = static_cast<T*>(h->act);
       const long long n = (long long)n_tok * L.c.ff;
-      TIMED(CLS_ELEMENTWISE, B200_LAUNCH(relu2_kernel<T>, (unsigned)ceil_div64(n, 256), 256, 0, st, proj, (long long)L.ldp, L.off_up, act, L.c.ff, n));
+      if (!squared) TIMED(CLS_ELEMENTWISE, B200_LAUNCH(relu2_kernel<T>, (unsigned)ceil_div64(n, 256), 256, 0, st, proj, (long long)L.ldp, L.off_up, act, L.c.ff, n));
       ffo = static_cast<T*>(h->ffo);
       TIMED(CLS_LINEAR, B200_TRY(linear<T>(h, act, L.c.ff, L.down, ffo, W, n_tok)));
     }
@@ -427,8 +454,7 @@ int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out
     if (h->head.tiles) {
       const int ldl = (c.vocab + 7) / 8 * 8;
       TIMED(CLS_LINEAR, B200_TRY(linear<bf16>(h, reinterpret_cast<const bf16*>(hf), W, h->head, h->head_bf, ldl, n_want)));
-      const long long n = (long long)n_want * c.vocab;
-      B200_LAUNCH(rows_to_f32_kernel, (unsigned)ceil_div64(n, 256), 256, 0, st, h->head_bf, (long long)ldl, h->logits, c.vocab, n);
+      return finish_logits(h, h->head_bf, ldl, n_want, LOGITS_PLAIN, 0.f, logits_out);
     } else {
       TIMED(CLS_LINEAR, B200_TRY(gemm_nt(st, hf, (long long)W, 0, static_cast<const T*>(h->head.rm), (long long)W, 0, h->logits, (long long)c.vocab, 0, n_want, c.vocab, W, 1, 1.f)));
     }
@@ -971,15 +997,13 @@ int step_sandwich(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits
   if (n_want > 0) {
     T* hf = static_cast<T*>(h->hf);
     TIMED(CLS_ELEMENTWISE, B200_LAUNCH(rmsnorm_rows_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, hf, W, c.norm_eps));
-    const long long n = (long long)n_want * c.vocab;
     if (h->head.tiles) {
       const int ldl = (c.vocab + 7) / 8 * 8;
       TIMED(CLS_LINEAR, B200_TRY(linear<bf16>(h, reinterpret_cast<const bf16*>(hf), W, h->head, h->head_bf, ldl, n_want)));
-      B200_LAUNCH(softcap_rows_kernel, (unsigned)ceil_div64(n, 256), 256, 0, st, h->head_bf, (long long)ldl, h->logits, c.vocab, n, c.logit_softcap);
+      return finish_logits(h, h->head_bf, ldl, n_want, c.logit_softcap > 0.f ? LOGITS_SOFTCAP : LOGITS_PLAIN, c.logit_softcap, logits_out);
     } else {
       TIMED(CLS_LINEAR, B200_TRY(gemm_nt(st, hf, (long long)W, 0, static_cast<const T*>(h->head.rm), (long long)W, 0, h->logits, (long long)c.vocab, 0, n_want, c.vocab, W, 1, 1.f)));
-      if (c.logit_softcap > 0.f)
-        B200_LAUNCH(softcap_rows_kernel, (unsigned)ceil_div64(n, 256), 256, 0, st, (const bf16*)nullptr, 0LL, h->logits, c.vocab, n, c.logit_softcap);
+      if (c.logit_softcap > 0.f) return finish_logits(h, nullptr, 0, n_want, LOGITS_SOFTCAP, c.logit_softcap, logits_out);
     }
     if (logits_out)
       B200_CUDA(cudaMemcpyAsync(logits_out, h->logits, (size_t)n_want * c.vocab * 4, cudaMemcpyDeviceToDevice, st));
@@ -1985,7 +2009,7 @@ int step_parallel(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits
       yexp = static_cast<const T*>(h->yexp);
     }
     const bool side = c.side_dim > 0;      // the token input comes behind the sum
-    auto block_end = n_tok <= 592 && W <= 4096 ? parallel_block_end_kernel<T, true> : parallel_block_end_kernel<T, false>;
+    auto block_end = parallel_block_end_kernel<T>;
     float* trace = h->trace_layers ? h->trace + (long long)li * stride : nullptr;
     const float *step = last ? nullptr : h->layers[li + 1].step, *w_next = last ? nullptr : h->layers[li + 1].n1w;
     TIMED(CLS_ELEMENTWISE, B200_LAUNCH(block_end, n_tok, 256, 0, st, h->xin, mixo, ffo, yexp, h->moe_w, L.c.top, side ? nullptr : trace, side ? nullptr : w_next, hb, W, c.norm_eps,
@@ -2001,8 +2025,7 @@ int step_parallel(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits
     if (h->head.tiles) {
       const int ldl = (c.vocab + 7) / 8 * 8;
       TIMED(CLS_LINEAR, B200_TRY(linear<bf16>(h, reinterpret_cast<const bf16*>(hf), W, h->head, h->head_bf, ldl, n_want)));
-      const long long n = (long long)n_want * c.vocab;
-      B200_LAUNCH(rows_to_f32_kernel, (unsigned)ceil_div64(n, 256), 256, 0, st, h->head_bf, (long long)ldl, h->logits, c.vocab, n);
+      return finish_logits(h, h->head_bf, ldl, n_want, LOGITS_PLAIN, 0.f, logits_out);
     } else {
       TIMED(CLS_LINEAR, B200_TRY(gemm_nt(st, hf, (long long)W, 0, static_cast<const T*>(h->head.rm), (long long)W, 0, h->logits, (long long)c.vocab, 0, n_want, c.vocab, W, 1, 1.f)));
     }
@@ -2322,11 +2345,10 @@ int step_streams(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_
   if (n_want > 0) {
     T* hf = static_cast<T*>(h->hf);
     TIMED(CLS_ELEMENTWISE, B200_LAUNCH(rmsnorm_rows_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, hf, W, c.norm_eps));
-    const long long n = (long long)n_want * c.vocab;
     if (h->head.tiles) {
       const int ldl = (c.vocab + 7) / 8 * 8;
       TIMED(CLS_LINEAR, B200_TRY(linear<bf16>(h, reinterpret_cast<const bf16*>(hf), W, h->head, h->head_bf, ldl, n_want)));
-      B200_LAUNCH(scale_rows_kernel, (unsigned)ceil_div64(n, 256), 256, 0, st, h->head_bf, (long long)ldl, h->logits, c.vocab, n, c.logit_scale);
+      return finish_logits(h, h->head_bf, ldl, n_want, LOGITS_SCALE, c.logit_scale, logits_out);
     } else {
       TIMED(CLS_LINEAR, B200_TRY(gemm_nt(st, hf, (long long)W, 0, static_cast<const T*>(h->head.rm), (long long)W, 0, h->logits, (long long)c.vocab, 0, n_want, c.vocab, W, 1, c.logit_scale)));
     }

@@ -50,6 +50,14 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* __restri
   __shared__ float red[32];
   const long long src = rows ? rows[blockIdx.x] : blockIdx.x;
   const float* xr = x + src * W;
+  if (W % 8 == 0 && W <= ROW_VEC) {
+    float v[ROW_RUNS][8];
+#pragma unroll
+    for (int k = 0; k < ROW_RUNS; ++k)
+      if (row_run(k) < W) load8(xr + row_run(k), v[k]);
+    row_norm<T>(v, w, nullptr, out + (long long)blockIdx.x * W, W, eps, false, red);
+    return;
+  }
   const float r = block_rrms(xr, W, eps, red);
   for (int i = threadIdx.x; i < W; i += blockDim.x) out[(long long)blockIdx.x * W + i] = from_f<T>(xr[i] * r * w[i]);
 }
@@ -526,17 +534,6 @@ __global__ void rows_from_f32_kernel(const float* __restrict__ in, T* __restrict
 // tokens share a read of the weights, few tokens spread over the GPU.  The sum over k has the same order in every layout: a lane
 // adds runs of eight elements (single elements where rows do not start on 16 bytes), then the lanes meet.
 // ---------------------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
-  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-__device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
-  const uint4 a = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&a);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
-}
-
 template <typename T, int TOK>
 __global__ void __launch_bounds__(256) small_proj_f32_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ w, const float* __restrict__ b,
                                                              float* __restrict__ out, int M, int N, int K, int vec) {
@@ -1199,15 +1196,6 @@ __device__ __forceinline__ void cp_async_16_or_zero(void* smem_dst, const void* 
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   const int n = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-
-// logits <- cap * tanh(logits / cap) on fp32 rows; `in` may be the padded bf16 rows of the tensor-core head (ld elements per row)
-__global__ void softcap_rows_kernel(const bf16* __restrict__ in_bf, long long ld, float* __restrict__ out, int V, long long n, float cap) {
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n) return;
-  const long long row = i / V;
-  const float v = in_bf ? __bfloat162float(in_bf[row * ld + (i - row * V)]) : out[i];
-  out[i] = cap > 0.f ? cap * tanhf(v / cap) : v;
 }
 
 }  // namespace dlm

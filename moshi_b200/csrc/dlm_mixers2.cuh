@@ -41,6 +41,22 @@ __global__ void __launch_bounds__(256) embed_scale_norm_kernel(const int* __rest
   if (bad) { if (threadIdx.x == 0) atomicOr(err, ERR_TOKEN); id = 0; }
   const T* row = table + (long long)id * W;
   float* x = xin + t * W;
+  if (W % 8 == 0 && W <= ROW_VEC) {
+    float v[ROW_RUNS][8];
+#pragma unroll
+    for (int k = 0; k < ROW_RUNS; ++k) {
+      const int i = row_run(k);
+      if (i >= W) break;
+      float s[8];
+      load8(row + i, v[k]);
+      if (step) load8(step + i, s);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[k][e] = (bad ? 0.f : v[k][e] * scale) + (step ? s[e] : 0.f);
+      store8(x + i, v[k]);
+    }
+    row_norm<T>(v, w1, nullptr, h + t * W, W, eps, layer != 0, red);
+    return;
+  }
   for (int i = threadIdx.x; i < W; i += blockDim.x) x[i] = (bad ? 0.f : to_f(row[i]) * scale) + (step ? step[i] : 0.f);
   __syncthreads();
   block_norm<T>(x, w1, h + t * W, W, eps, layer, red);
@@ -49,9 +65,8 @@ __global__ void __launch_bounds__(256) embed_scale_norm_kernel(const int* __rest
 // End of a parallel block, one CTA per token:  x <- x + mix + ff,  ff = a dense feed-forward's row | sum_k ew[t][k] * rows of
 // the chosen experts (the row of h itself for a choice from n_exp on: an identity expert) | both | nothing;  optional copy of x
 // (per-layer trace);  x <- x + step (the vector in front of a pass, when given);  optional h = norm(x) * w_next for the next layer.
-// REG (few tokens, W <= 4096): the row stays in registers between the sum and the norm, which shortens the chain of a CTA; many tokens
-// fill the SMs better with the smaller kernel.
-template <typename T, bool REG>
+// Rows of up to ROW_VEC elements are held in registers in runs of eight.
+template <typename T>
 __global__ void __launch_bounds__(256) parallel_block_end_kernel(float* __restrict__ xin, const T* __restrict__ mix, const T* __restrict__ ff,
                                                                  const T* __restrict__ yexp, const float* __restrict__ ew, int top,
                                                                  float* __restrict__ trace, const float* __restrict__ w_next, T* h,
@@ -73,35 +88,43 @@ __global__ void __launch_bounds__(256) parallel_block_end_kernel(float* __restri
     }
     return x[i] + y;
   };
-  if constexpr (REG) {
-    constexpr int NR = 16;
-    float v[NR], s = 0.f;
+  if (W % 8 == 0 && W <= ROW_VEC) {
+    float v[ROW_RUNS][8];
 #pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const int i = threadIdx.x + 256 * k;
-      v[k] = i < W ? updated(i) : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const int i = threadIdx.x + 256 * k;
+    for (int k = 0; k < ROW_RUNS; ++k) {
+      const int i = row_run(k);
       if (i >= W) break;
-      if (trace) trace[t * W + i] = v[k];
-      if (step) v[k] += step[i];
-      x[i] = v[k];
-      s += v[k];
-    }
-    if (!w_next) return;
-    const float mean = layer ? block_sum(s, red) / (float)W : 0.f;
-    float q = 0.f;
+      float y[8], f[8];
+      load8(x + i, v[k]);
+      load8(mix + t * W + i, y);
+      if (ff) {
+        load8(ff + t * W + i, f);
 #pragma unroll
-    for (int k = 0; k < NR; ++k)
-      if (threadIdx.x + 256 * k < W) { const float d = v[k] - mean; q = fmaf(d, d, q); }
-    const float r = 1.f / sqrtf(block_sum(q, red) / (float)W + eps);
+        for (int e = 0; e < 8; ++e) y[e] += f[e];
+      }
+      if (yexp) {
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int j = 0; j < top; ++j) {
+          const float wj = ew[t * top + j];
+          load8(choice && choice[t * top + j] >= n_exp ? h + t * W + i : yexp + (t * top + j) * W + i, f);
 #pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const int i = threadIdx.x + 256 * k;
-      if (i < W) h[t * W + i] = from_f<T>((v[k] - mean) * r * w_next[i]);
+          for (int e = 0; e < 8; ++e) acc[e] = fmaf(wj, f[e], acc[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) y[e] += acc[e];
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[k][e] += y[e];
+      if (trace) store8(trace + t * W + i, v[k]);
+      if (step) {
+        load8(step + i, f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[k][e] += f[e];
+      }
+      store8(x + i, v[k]);
     }
+    if (w_next) row_norm<T>(v, w_next, nullptr, h + t * W, W, eps, layer != 0, red);
     return;
   }
   for (int i = threadIdx.x; i < W; i += blockDim.x) {

@@ -280,14 +280,6 @@ __global__ void __launch_bounds__(256) chdelta_gram_kernel(DeltaChunkParams p) {
   }
 }
 
-// rows of logits times a constant: bf16 rows with a padded stride (in_bf given) or fp32 in place -> fp32 [rows][V]
-__global__ void scale_rows_kernel(const bf16* __restrict__ in_bf, long long ld, float* __restrict__ out, int V, long long n, float scale) {
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n) return;
-  const long long row = i / V;
-  const float v = in_bf ? __bfloat162float(in_bf[row * ld + (i - row * V)]) : out[i];
-  out[i] = v * scale;
-}
 
 __global__ void identity_kernel(float* __restrict__ m, int n) {
   const int i = blockIdx.x * 256 + threadIdx.x;

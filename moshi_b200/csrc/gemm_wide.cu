@@ -46,6 +46,7 @@ struct WideP {
   const int* y_rows;                                  // grouped: result row of every row (null: the row itself)
   int e_rows;                                         // grouped: weight rows per expert
   int vec;                                            // results in 16-byte stores
+  int act_from, act_to; __nv_bfloat16* y2; long long ldy2;
   uint32_t stage_bytes;
   uint32_t a_bytes;                                   // bytes of a box of x rows (128 rows; fewer where no tile has more)
   int* err;
@@ -161,7 +162,7 @@ __device__ __forceinline__ void store_run(__nv_bfloat16* row, int col, int cols,
 }
 
 // 32 neighbouring sums of one row through the epilogue
-__device__ __forceinline__ void finish_run(const WideP& p, __nv_bfloat16* y, int n, float* v) {
+__device__ __forceinline__ void finish_run(const WideP& p, __nv_bfloat16* y, long long yr, int n, float* v) {
   if (p.act == WIDE_CLAMPED_GLU || p.act == WIDE_SILU_GLU) {      // weight rows interleave gate and value
     float o[16];
 #pragma unroll
@@ -177,14 +178,16 @@ __device__ __forceinline__ void finish_run(const WideP& p, __nv_bfloat16* y, int
     store_run<16>(y, n >> 1, p.N >> 1, o, p.vec);
     return;
   }
-  if (p.act == WIDE_RELU2) {
+  const bool aside = n >= p.act_from && n < p.act_to;
+  if (p.act == WIDE_RELU2 || aside) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) { v[j] = fmaxf(v[j], 0.f); v[j] *= v[j]; }
   } else if (p.act == WIDE_GELU) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = 0.5f * v[j] * (1.f + erff(v[j] * 0.7071067811865476f));
   }
-  store_run<32>(y, n, p.N, v, p.vec);
+  if (aside) store_run<32>(p.y2 + yr * p.ldy2, n - p.act_from, p.act_to - p.act_from, v, p.vec);
+  else store_run<32>(y, n, p.N, v, p.vec);
 }
 
 // whether all 128 epilogue threads say so (a barrier of theirs)
@@ -364,7 +367,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
               }
             }
           }
-          if (row_ok && n < p.N) finish_run(p, y, n, v);
+          if (row_ok && n < p.N) finish_run(p, y, yr, n, v);
         }
       }
       if (whole) {
@@ -461,6 +464,11 @@ int wide_gemm(const WideGemm& g, cudaStream_t st) {
   p.M = g.M; p.N = g.N; p.num_kb = ceil_div(g.K, BK); p.packed = g.packed ? 1 : 0; p.act = g.act; p.limit = g.limit;
   p.y = g.y; p.ldy = g.ldy; p.err = g.err;
   p.vec = g.ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(g.y) & 15) == 0;
+  if (g.act_to > 0) {
+    if (g.tile_e || g.act != WIDE_STORE || !g.y2 || (g.act_from | g.act_to) % 32 || g.act_to > g.N) B200_FAIL(B200_ERR_SHAPE, "wide GEMM: bad range of activated columns");
+    p.act_from = g.act_from; p.act_to = g.act_to; p.y2 = g.y2; p.ldy2 = g.ldy2;
+    p.vec = p.vec && g.ldy2 % 8 == 0 && (reinterpret_cast<uintptr_t>(g.y2) & 15) == 0;
+  }
   if (g.tile_e) {
     p.tile_e = g.tile_e; p.tile_r0 = g.tile_r0; p.tile_n = g.tile_n; p.n_tiles = g.n_tiles; p.y_rows = g.y_rows; p.e_rows = g.e_rows;
     p.mt = g.max_tiles; p.nt = ceil_div(g.N, 256); p.splits = 1; p.kb_per = p.num_kb;

@@ -16,6 +16,8 @@ struct WideGemm {
   __nv_bfloat16* y = nullptr; long long ldy = 0;
   int M = 0, N = 0, K = 0;                   // N: weight rows (of one expert)
   int act = WIDE_STORE; float limit = 0.f;
+  // columns [act_from, act_to), both multiples of 32, go through relu(.)^2 to y2 instead (act_to = 0: none; WIDE_STORE only)
+  int act_from = 0, act_to = 0; __nv_bfloat16* y2 = nullptr; long long ldy2 = 0;
   // grouped product: tiles of up to WIDE_EXPERT_ROWS neighbouring rows of one expert, listed on the device; at most max_tiles of them
   const int *tile_e = nullptr, *tile_r0 = nullptr, *tile_n = nullptr, *n_tiles = nullptr, *y_rows = nullptr;
   int max_tiles = 0, e_rows = 0, max_rows = 0;      // max_rows: no expert has more (0: unknown)
