@@ -10,6 +10,8 @@
 // depth-wise up-sampling, LayerNorm / RoPE / ring attention and the residual VQ are small SIMT kernels.
 #include "mimi_kernels.cuh"
 #include "mimi_tc.cuh"
+#include "mimi_lin.cuh"
+#include "mimi_rvq.cuh"
 #include "mimi_tm_kernels.cuh"
 
 using namespace b200;
@@ -41,6 +43,7 @@ struct SeaLayer {
 struct TrLayer {
   const float *n1w, *n1b, *n2w, *n2b, *ls1, *ls2;
   mtc::TcLayer in_proj, out_proj, l1, l2;
+  const float *w_in = nullptr, *w_out = nullptr, *w_1 = nullptr, *w_2 = nullptr;      // row-major fp32 for few tokens (null: not a shape of mimi_lin_kernel)
   float *kc = nullptr, *vc = nullptr;
 };
 
@@ -81,6 +84,9 @@ struct b200_mimi {
   Transformer enc_tr, dec_tr;
   // quantizer
   float *wT[2] = {nullptr, nullptr}, *woT[2] = {nullptr, nullptr};
+  float *w_rvq_in = nullptr, *w_rvq_out = nullptr;      // both quantizers' projections as one product: [2 Dq][C], [C][2 Dq] (null: not a shape of mimi_rvq.cuh)
+  float *rvq_proj = nullptr, *rvq_step_res[2][2] = {}, *rvq_step_best[2][2] = {}, *rvq_sum = nullptr;      // per streaming batch
+  int* rvq_step_idx[2][2] = {};
   float *cb[2] = {nullptr, nullptr}, *cbT[2] = {nullptr, nullptr}, *cnorm[2] = {nullptr, nullptr};
   int stored_levels[2] = {0, 0};
   // per-batch buffers
@@ -115,6 +121,7 @@ struct b200_mimi {
   float* tap_scratch = nullptr; size_t tap_scratch_n = 0;
   std::map<std::string, Tap> taps;
   int64_t weight_bytes = 0;
+  bool tr_cuda_cores = false;                  // the bottleneck transformers run on mimi_lin_kernel / mimi_attn_kernel at this batch
 };
 
 namespace {
@@ -319,9 +326,15 @@ int keep(b200_mimi* h, const std::string& name, std::vector<int64_t> shape, cons
   return B200_OK;
 }
 
-int keep_linear(b200_mimi* h, const std::string& name, int M, int K, mtc::TcLayer& L) {
+int keep_linear(b200_mimi* h, const std::string& name, int M, int K, mtc::TcLayer& L, const float** rows) {
   const float* src = nullptr;
   B200_TRY(get_f32(h, name, {M, K}, &src));
+  if (lin_takes(M, K)) {
+    float* copy = nullptr;
+    B200_TRY(h->weights.alloc_t(&copy, (size_t)M * K, false));
+    B200_CUDA(cudaMemcpyAsync(copy, src, (size_t)M * K * 4, cudaMemcpyDeviceToDevice, nullptr));
+    *rows = copy;
+  }
   B200_TRY(pack_tc(h, L, src, M, K, 1));       // nn.Linear weight [out][in] is already [N][K]
   L.kind = 2; L.dil = 1; L.stride = 1; L.bias = nullptr; L.bias_mod = M;
   B200_CUDA(cudaDeviceSynchronize());
@@ -336,14 +349,14 @@ int pack_transformer(b200_mimi* h, const std::string& prefix, Transformer& tr) {
   for (int li = 0; li < c.tr_num_layers; ++li) {
     const std::string p = prefix + ".transformer.layers." + std::to_string(li);
     TrLayer& L = tr.layers[li];
-    B200_TRY(keep_linear(h, p + ".self_attn.in_projs.0.weight", 3 * d, d, L.in_proj));
-    B200_TRY(keep_linear(h, p + ".self_attn.out_projs.0.weight", d, d, L.out_proj));
+    B200_TRY(keep_linear(h, p + ".self_attn.in_projs.0.weight", 3 * d, d, L.in_proj, &L.w_in));
+    B200_TRY(keep_linear(h, p + ".self_attn.out_projs.0.weight", d, d, L.out_proj, &L.w_out));
     B200_TRY(keep(h, p + ".norm1.weight", {d}, &L.n1w));
     B200_TRY(keep(h, p + ".norm1.bias", {d}, &L.n1b));
     B200_TRY(keep(h, p + ".norm2.weight", {d}, &L.n2w));
     B200_TRY(keep(h, p + ".norm2.bias", {d}, &L.n2b));
-    B200_TRY(keep_linear(h, p + ".linear1.weight", ff, d, L.l1));
-    B200_TRY(keep_linear(h, p + ".linear2.weight", d, ff, L.l2));
+    B200_TRY(keep_linear(h, p + ".linear1.weight", ff, d, L.l1, &L.w_1));
+    B200_TRY(keep_linear(h, p + ".linear2.weight", d, ff, L.l2, &L.w_2));
     B200_TRY(keep(h, p + ".layer_scale_1.scale", {d}, &L.ls1));
     B200_TRY(keep(h, p + ".layer_scale_2.scale", {d}, &L.ls2));
   }
@@ -353,6 +366,11 @@ int pack_transformer(b200_mimi* h, const std::string& prefix, Transformer& tr) {
 int pack_quantizer(b200_mimi* h) {
   const auto& c = h->cfg;
   const char* names[2] = {"rvq_first", "rvq_rest"};
+  const bool together = c.q_dimension == RVL_D && c.dimension == 2 * RVL_D && c.q_bins % RVL_CODES == 0;
+  if (together) {
+    B200_TRY(h->weights.alloc_t(&h->w_rvq_in, (size_t)2 * c.q_dimension * c.dimension, false));
+    B200_TRY(h->weights.alloc_t(&h->w_rvq_out, (size_t)2 * c.q_dimension * c.dimension, false));
+  }
   h->stored_levels[0] = c.q_n_semantic;
   h->stored_levels[1] = c.q_n_q - c.q_n_semantic;
   for (int w = 0; w < 2; ++w) {
@@ -362,10 +380,14 @@ int pack_quantizer(b200_mimi* h) {
     B200_TRY(h->weights.alloc_t(&h->wT[w], (size_t)c.q_dimension * c.dimension, false));
     B200_LAUNCH(transpose_kernel, (unsigned)ceil_div64((long long)c.q_dimension * c.dimension, 256), 256, 0, 0, src,
                 h->wT[w], c.q_dimension, c.dimension);
+    if (together) B200_CUDA(cudaMemcpyAsync(h->w_rvq_in + (size_t)w * c.q_dimension * c.dimension, src, (size_t)c.q_dimension * c.dimension * 4, cudaMemcpyDeviceToDevice, nullptr));
     B200_TRY(get_f32(h, p + ".output_proj.weight", {c.dimension, c.q_dimension, 1}, &src));
     B200_TRY(h->weights.alloc_t(&h->woT[w], (size_t)c.q_dimension * c.dimension, false));
     B200_LAUNCH(transpose_kernel, (unsigned)ceil_div64((long long)c.q_dimension * c.dimension, 256), 256, 0, 0, src,
                 h->woT[w], c.dimension, c.q_dimension);
+    if (together)
+      B200_CUDA(cudaMemcpy2DAsync(h->w_rvq_out + (size_t)w * c.q_dimension, (size_t)2 * c.q_dimension * 4, src, (size_t)c.q_dimension * 4, (size_t)c.q_dimension * 4,
+                                  c.dimension, cudaMemcpyDeviceToDevice, nullptr));
     const int L = h->stored_levels[w];
     const size_t per = (size_t)c.q_bins * c.q_dimension;
     B200_TRY(h->weights.alloc_t(&h->cb[w], per * L, false));
@@ -402,6 +424,37 @@ int run_transformer(b200_mimi* h, Transformer& tr, const float* x_in, float* x, 
   const auto& c = h->cfg;
   const int B = h->batch, ntok = B * T, d = c.tr_d_model, H = c.tr_num_heads, D = d / H;
   const float nl = -logf(c.tr_max_period) * 2.f / (float)D;
+  if (h->tr_cuda_cores) {
+    for (size_t li = 0; li < tr.layers.size(); ++li) {
+      TrLayer& L = tr.layers[li];
+      const float* cur = li == 0 ? x_in : x;
+      auto lin = [&](const float* in, const float* w, int N, int K, int epi, float* y) {
+        LinP q;
+        memset(&q, 0, sizeof(q));
+        q.x = in; q.w = w; q.n_tok = ntok; q.N = N; q.K = K; q.T = T; q.epi = epi; q.y = y; q.eps = 1e-5f;
+        return q;
+      };
+      LinP q = lin(cur, L.w_in, 3 * d, d, LIN_STORE, h->tr_qkv);
+      q.gamma = L.n1w; q.beta = L.n1b;
+      B200_TRY(lin_launch(q, h->body));
+      MimiAttn a;
+      a.qkv = h->tr_qkv; a.kc = L.kc; a.vc = L.vc; a.out = h->tr_ao_hi; a.offset = tr.offset; a.exec_mask = h->exec_mask; a.H = H; a.cap = c.tr_context;
+      a.context = c.tr_context; a.neg_log_period_2_over_d = nl;
+      B200_TRY(attn_launch(a, B, T, h->body));
+      q = lin(h->tr_ao_hi, L.w_out, d, d, LIN_RESIDUAL, x);
+      q.res = cur; q.scale = L.ls1;
+      B200_TRY(lin_launch(q, h->body));
+      q = lin(x, L.w_1, c.tr_dim_feedforward, d, LIN_GELU, h->tr_h_hi);
+      q.gamma = L.n2w; q.beta = L.n2b;
+      B200_TRY(lin_launch(q, h->body));
+      q = lin(h->tr_h_hi, L.w_2, d, c.tr_dim_feedforward, LIN_RESIDUAL, x);
+      const mtc::TcParams& e = L.l2.p;           // the decoder's last layer also feeds dec[0]
+      q.res = x; q.scale = L.ls2; q.a_hi = e.a_hi; q.a_lo = e.a_lo; q.a_sb = e.a_sb; q.a_row = e.a_row; q.a_elu = e.act_elu;
+      B200_TRY(lin_launch(q, h->body));
+    }
+    B200_LAUNCH(advance_offsets_kernel, ceil_div(B, 128), 128, 0, h->body, tr.offset, h->exec_mask, B, T);
+    return check_launch("mimi transformer");
+  }
   const size_t attn_smem = (size_t)(T * D + T * c.tr_context) * sizeof(float);
   for (size_t li = 0; li < tr.layers.size(); ++li) {
     TrLayer& L = tr.layers[li];
@@ -530,6 +583,79 @@ int ensure_rvq_workspace(b200_mimi* h, int Q) {
   }
   h->rvq_cap = Q;
   return B200_OK;
+}
+
+// the frame's latents [B][C] -> codes, one launch per level (mimi_rvq.cuh)
+int quantize_frame(b200_mimi* h, const float* lat, long long* codes, long long cs_b, long long cs_k) {
+  const auto& c = h->cfg;
+  const int Q = h->batch, n_chunks = c.q_bins / RVL_CODES;
+  LinP p;
+  memset(&p, 0, sizeof(p));
+  p.x = lat; p.w = h->w_rvq_in; p.n_tok = Q; p.N = 2 * RVL_D; p.K = c.dimension; p.T = 1; p.epi = LIN_STORE; p.y = h->rvq_proj;
+  B200_TRY(lin_launch(p, h->body));
+  int levels[2];
+  levels[0] = std::min(c.q_n_semantic, h->num_codebooks);
+  levels[1] = h->num_codebooks - levels[0];
+  const int max_levels = std::max(levels[0], levels[1]);
+  const size_t per = (size_t)c.q_bins * RVL_D;
+  for (int level = 0; level < max_levels; ++level) {
+    RvqStep a;
+    memset(&a, 0, sizeof(a));
+    const int cur = level & 1, old = cur ^ 1;
+    for (int w = 0; w < 2; ++w) {
+      a.res_in[w] = level < 2 ? h->rvq_proj + w * RVL_D : h->rvq_step_res[w][cur];      // what the launch before the last one left
+      a.res_out[w] = h->rvq_step_res[w][old];
+      a.cb[w] = h->cb[w] + per * level; a.cnorm[w] = h->cnorm[w] + (size_t)c.q_bins * level;
+      a.cb_prev[w] = level ? a.cb[w] - per : a.cb[w];
+      a.best[w] = h->rvq_step_best[w][cur]; a.idx[w] = h->rvq_step_idx[w][cur];
+      a.prev_best[w] = h->rvq_step_best[w][old]; a.prev_idx[w] = h->rvq_step_idx[w][old];
+      a.active[w] = level < levels[w];
+      a.prev_active[w] = level > 0 && level - 1 < levels[w];
+      a.prev_code[w] = (w == 0 ? 0 : levels[0]) + level - 1;
+    }
+    a.res_in_ld = level < 2 ? 2 * RVL_D : RVL_D;
+    a.codes = codes; a.cs_b = cs_b; a.cs_k = cs_k; a.n_query = Q; a.bins = c.q_bins; a.n_chunks = n_chunks;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)n_chunks, (unsigned)ceil_div(Q, RVL_Q), 2); cfg.blockDim = dim3(128); cfg.stream = h->body;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, rvq_level_kernel, a);
+    if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "rvq_level launch failed: %s", cudaGetErrorString(e));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+  }
+  RvqLevelArgs f;                                // the last level's choice
+  memset(&f, 0, sizeof(f));
+  const int last = (max_levels - 1) & 1;
+  for (int w = 0; w < 2; ++w) {
+    f.res[w] = h->rvq_step_res[w][last]; f.cb[w] = h->cb[w] + per * (max_levels - 1);
+    f.part_best[w] = h->rvq_step_best[w][last]; f.part_idx[w] = h->rvq_step_idx[w][last];
+    f.active[w] = levels[w] == max_levels;
+    f.code_index[w] = (w == 0 ? 0 : levels[0]) + max_levels - 1;
+  }
+  f.codes = codes; f.cs_b = cs_b; f.cs_k = cs_k; f.cs_f = 1; f.n_query = Q; f.n_frames = 1; f.Dq = RVL_D; f.bins = c.q_bins; f.n_chunks = n_chunks;
+  B200_LAUNCH(rvq_pick_kernel, dim3(Q, 2), 128, 0, h->body, f);
+  return check_launch("rvq_encode");
+}
+
+// codes [B][K] of one frame -> quantized latents [B][C]
+int dequantize_frame(b200_mimi* h, const long long* codes, long long cs_b, long long cs_k, int n_codebooks, float* out) {
+  const auto& c = h->cfg;
+  if (n_codebooks < 1 || n_codebooks > c.q_n_q) B200_FAIL(B200_ERR_SHAPE, "decode: %d codebooks", n_codebooks);
+  RvqGather a;
+  a.codes = codes; a.cs_b = cs_b; a.cs_k = cs_k; a.out = h->rvq_sum; a.bins = c.q_bins; a.err = h->err;
+  for (int w = 0; w < 2; ++w) a.cb[w] = h->cb[w];
+  a.levels[0] = std::min(c.q_n_semantic, n_codebooks);
+  a.levels[1] = n_codebooks - a.levels[0];
+  a.level_offset[0] = 0; a.level_offset[1] = a.levels[0];
+  B200_LAUNCH(rvq_gather_kernel, h->batch, 128, 0, h->body, a);
+  LinP p;
+  memset(&p, 0, sizeof(p));
+  p.x = h->rvq_sum; p.w = h->w_rvq_out; p.n_tok = h->batch; p.N = c.dimension; p.K = 2 * RVL_D; p.T = 1; p.epi = LIN_STORE; p.y = out;
+  B200_TRY(lin_launch(p, h->body));
+  return check_launch("rvq_decode");
 }
 
 int quantize_cols(b200_mimi* h, const float* lat, long long lb, long long lc, long long lt, int n_cols,
@@ -915,6 +1041,9 @@ int b200_mimi_streaming_begin(b200_mimi* h, int batch, void* stream) {
   // transformers
   const int H = c.tr_num_heads, D = d / H, ff = c.tr_dim_feedforward;
   const size_t ntok = (size_t)B * T;
+  // encode + decode of a frame on these kernels against mimi_tc_kernel: 1 session 0.77 / 1.49 ms, 8 sessions 1.19 / 1.55, 24 sessions 1.51 / 1.71,
+  // 40 sessions (80 tokens) 1.99 both, 64 sessions 2.39 / 2.19: a product over 80 tokens is worth the tensor cores' two launches
+  h->tr_cuda_cores = (int)ntok <= 64 && D == 64 && d == 512 && T <= 4 && lin_takes(3 * d, d) && lin_takes(d, ff) && lin_takes(ff, d);
   B200_TRY(A.alloc_t(&h->tr_xn_hi, ntok * d));
   B200_TRY(A.alloc_t(&h->tr_xn_lo, ntok * d));
   B200_TRY(A.alloc_t(&h->tr_qkv, ntok * 3 * d));
@@ -963,6 +1092,16 @@ int b200_mimi_streaming_begin(b200_mimi* h, int batch, void* stream) {
       }
       B200_TRY(plan_layer(h, L.l2, h->tr_h_hi, h->tr_h_lo, T, 0, T));
     }
+  }
+  if (h->w_rvq_in) {
+    B200_TRY(A.alloc_t(&h->rvq_proj, (size_t)B * 2 * RVL_D));
+    B200_TRY(A.alloc_t(&h->rvq_sum, (size_t)B * 2 * RVL_D));
+    for (int w = 0; w < 2; ++w)
+      for (int i = 0; i < 2; ++i) {
+        B200_TRY(A.alloc_t(&h->rvq_step_res[w][i], (size_t)B * RVL_D));
+        B200_TRY(A.alloc_t(&h->rvq_step_best[w][i], (size_t)B * (c.q_bins / RVL_CODES)));
+        B200_TRY(A.alloc_t(&h->rvq_step_idx[w][i], (size_t)B * (c.q_bins / RVL_CODES)));
+      }
   }
   B200_TRY(A.alloc_t(&h->scratch_codes, (size_t)B * c.q_n_q));
   B200_TRY(A.alloc_t(&h->enc_codes, (size_t)B * c.q_n_q));
@@ -1082,6 +1221,7 @@ int b200_mimi_encode(b200_mimi* h, const float* pcm_dev, int n_frames, int64_t* 
     B200_TRY(load_frame(h, pcm_dev, n_frames, f));
     B200_TRY(run_captured(h, &h->enc_graph, &h->enc_graph_kernels, [&]() -> int {
       B200_TRY(encode_body(h));
+      if (h->w_rvq_in) return quantize_frame(h, h->latent, h->enc_codes, K, 1);
       return quantize_cols(h, h->latent, d, 1, 1, 1, h->enc_codes, K, 1, 1);
     }));
     // enc_codes [B][K] -> codes[b][k][f]
@@ -1115,7 +1255,8 @@ int b200_mimi_decode(b200_mimi* h, const int64_t* codes_dev, int n_codebooks, in
     B200_CUDA(cudaMemcpy2DAsync(h->dec_codes, 8, reinterpret_cast<const long long*>(codes_dev) + f, (size_t)n_frames * 8, 8,
                                 (size_t)h->batch * n_codebooks, cudaMemcpyDeviceToDevice, h->stream));
     B200_TRY(run_captured(h, &h->dec_graph, &h->dec_graph_kernels, [&]() -> int {
-      B200_TRY(dequantize_cols(h, h->dec_codes, n_codebooks, 1, 1, n_codebooks, 1, h->latent_q, d, 1, 1));
+      if (h->w_rvq_out) B200_TRY(dequantize_frame(h, h->dec_codes, n_codebooks, 1, n_codebooks, h->latent_q));
+      else B200_TRY(dequantize_cols(h, h->dec_codes, n_codebooks, 1, 1, n_codebooks, 1, h->latent_q, d, 1, 1));
       return decode_latent_body(h);
     }));
     B200_CUDA(cudaMemcpy2DAsync(pcm_dev + (size_t)f * fs, (size_t)fs * n_frames * 4, h->out_frame, (size_t)fs * 4,

@@ -461,6 +461,7 @@ static __global__ void __launch_bounds__(128) rvq_pick_kernel(const RvqLevelArgs
       const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
       if (ob < best || (ob == best && oi < bidx)) { best = ob; bidx = oi; }
     }
+    if (bidx >= a.bins) bidx = 0;                // no minimum among the scores of a latent that is not a number
     if (threadIdx.x == 0) {
       s_choice = bidx;
       const int b = q / a.n_frames, f = q % a.n_frames;
