@@ -19,6 +19,24 @@ typedef __nv_bfloat16 bf16;
 // (gemm_sk.cu): triggering at entry lets its CTAs take free SM resources and start streaming weights
 // while this kernel runs; the GEMM itself waits (griddepcontrol.wait) before it touches activations.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launch that may begin while the preceding kernel drains: the kernel calls pdl_wait() before it touches what that one writes or reads.
+// Between the kernels of a step a plain launch costs 1.5-2 us of idle GPU.
+template <typename... P, typename... A>
+inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return B200_OK;
+}
 
 __device__ __forceinline__ void unpack8(const uint4& v, float* f) {
   const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
@@ -161,6 +179,7 @@ static __global__ void dep_input_kernel(const bf16* __restrict__ din /*[B][ld]*/
                                  const bf16* __restrict__ table /*[V][dd]*/, const long long* __restrict__ prev /*[Bt]*/,
                                  bf16* __restrict__ x /*[B][dd]*/, int B, int dd, int Bt, int vocab, int* err) {
   pdl_trigger();
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B * dd) return;
   const int b = i / dd, c = i % dd;
@@ -238,12 +257,48 @@ static __global__ void __launch_bounds__(256) rmsnorm_kernel(const bf16* __restr
   pdl_trigger();
   const int row = blockIdx.x;
   const bf16* xr = x + (long long)row * dim;
+  __shared__ float red[32];
+  if (dim % 8 == 0 && dim <= 8 * 256 * 2) {      // the row in registers, every load in flight at once
+    uint4 v[2], al[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if ((threadIdx.x + 256 * k) * 8 < dim) al[k] = *reinterpret_cast<const uint4*>(alpha + (threadIdx.x + 256 * k) * 8);
+    pdl_wait();
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = (threadIdx.x + 256 * k) * 8;
+      if (c >= dim) break;
+      v[k] = *reinterpret_cast<const uint4*>(xr + c);
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[k]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { const float2 f = __bfloat1622float2(h[e]); ss += f.x * f.x + f.y * f.y; }
+    }
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    const float r = rsqrtf(eps + warp_sum((threadIdx.x & 31) < 8 ? red[threadIdx.x & 31] : 0.f) / (float)dim);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = (threadIdx.x + 256 * k) * 8;
+      if (c >= dim) break;
+      const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162*>(&v[k]), *a = reinterpret_cast<const __nv_bfloat162*>(&al[k]);
+      __nv_bfloat162 o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(h[e]), g = __bfloat1622float2(a[e]);
+        o[e] = __floats2bfloat162_rn(f.x * (g.x * r), f.y * (g.y * r));
+      }
+      *reinterpret_cast<uint4*>(y + (long long)row * dim + c) = *reinterpret_cast<const uint4*>(o);
+    }
+    return;
+  }
+  pdl_wait();
   float ss = 0.f;
   for (int c = threadIdx.x * 2; c < dim; c += blockDim.x * 2) {
     const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(xr + c));
     ss += v.x * v.x + v.y * v.y;
   }
-  __shared__ float red[32];
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
@@ -284,6 +339,20 @@ inline int attn_pick_splits(int B, int H, int cap) {
   return ns;
 }
 
+// The same for the 16-bit ring, whose kernel gives a session only the ranges that its own history fills (at least min_per keys each).  Few
+// (session, head) pairs: ranges of 64 keys and more.  592 to 1183 pairs are one uneven wave: ranges of 512 keys even it out (24 full rings
+// 218 -> 196 us, 24 sessions of 0 to 3000 frames 91 -> 86).  From 1184 on whole rings stream best (104 full rings 718 us, in ranges of 512 773).
+inline int attn_ragged_splits(int B, int H, int cap, int* min_per) {
+  const int pairs = B * H;
+  int ns = 1;
+  *min_per = cap;
+  if (pairs < 148 * 4) { ns = (148 * 4 + pairs - 1) / pairs; *min_per = 64; }
+  else if (pairs < 148 * 8) { ns = (cap + 511) / 512; *min_per = 512; }
+  if (ns > 16) ns = 16;
+  const int max_by_len = (cap + 63) / 64;
+  return ns > max_by_len ? max_by_len : ns;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Fused temporal attention step (T = 1, D = 128): RoPE(q, k) + ring append + split-KV attention +
 // split combine in ONE launch (transformer.py:557-597).
@@ -298,7 +367,7 @@ struct AttnStep {
   const bf16* qkv; bf16* kc; bf16* vc; bf16* out;
   float* part; int* counters;                  // [B*H][nsplit][ATT_D + 2], [B*H] (zero between launches)
   const long long* pos; const uint8_t* exec_mask;
-  int H, cap, nsplit; float neg_log_period_2_over_d;
+  int H, cap, nsplit, min_per; float neg_log_period_2_over_d;      // nsplit <= 32: ranges at most; min_per: keys of a range at least
 };
 
 template <int ATT_U>       // keys per half-warp per register buffer
@@ -313,50 +382,16 @@ static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const Att
   const long long p = a.pos[b];
   long long n_valid = p + (exec ? 1 : 0);
   if (n_valid > a.cap) n_valid = a.cap;
-  const int per = (int)((n_valid + a.nsplit - 1) / a.nsplit);
+  const int per = max(a.min_per, (int)((n_valid + a.nsplit - 1) / a.nsplit));
+  const int splits = max(1, (int)((n_valid + per - 1) / per));      // ranges in use
+  if (split >= splits) return;
   const int s0 = split * per;
   const int s1 = (int)min((long long)(s0 + per), n_valid);
   const int slot_new = (int)(p % a.cap);
   const bf16* base = a.qkv + (long long)b * 3 * C + h * ATT_D;
   const float fpos = (float)p;
-
-  if (exec && slot_new >= s0 && slot_new < s1) {    // CTA-uniform: this CTA owns the new key's slot
-    if (tid < ATT_D / 2) {
-      const int pr = tid;
-      float kr = bf2f(base[C + 2 * pr]), ki = bf2f(base[C + 2 * pr + 1]);
-      const float freq = expf((float)pr * a.neg_log_period_2_over_d);
-      float sn, cs;
-      sincosf(freq * fpos, &sn, &cs);
-      const float c2 = kr * cs - ki * sn, d2 = kr * sn + ki * cs;
-      const long long o = ((long long)bh * a.cap + slot_new) * ATT_D + 2 * pr;
-      *reinterpret_cast<__nv_bfloat162*>(a.kc + o) = __floats2bfloat162_rn(c2, d2);
-      *reinterpret_cast<__nv_bfloat162*>(a.vc + o) = *reinterpret_cast<const __nv_bfloat162*>(base + 2 * C + 2 * pr);
-    }
-    __syncthreads();
-  }
-
-  float qf[8];
-  {
-    float raw[8];
-    unpack8(*reinterpret_cast<const uint4*>(base + l16 * 8), raw);
-    const float scale = 0.08838834764831845f;       // 1/sqrt(128)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int pr = l16 * 4 + j;
-      const float freq = expf((float)pr * a.neg_log_period_2_over_d);
-      float sn, cs;
-      sincosf(freq * fpos, &sn, &cs);
-      const float qr = raw[2 * j], qi = raw[2 * j + 1];
-      qf[2 * j] = rbf(qr * cs - qi * sn) * scale;
-      qf[2 * j + 1] = rbf(qr * sn + qi * cs) * scale;
-    }
-  }
-
   const bf16* kb = a.kc + (long long)bh * a.cap * ATT_D + l16 * 8;
   const bf16* vb = a.vc + (long long)bh * a.cap * ATT_D + l16 * 8;
-  float m = -INFINITY, l = 0.f, acc[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
 
   // Groups of U keys per half-warp, double-buffered in registers: the loads of group i + 1 are in flight while group i
   // is reduced (same structure as attn_step_q8_kernel below).
@@ -371,6 +406,45 @@ static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const Att
       gp.v[u] = *reinterpret_cast<const uint4*>(vb + (long long)ss * ATT_D);
     }
   };
+  Group ga, gb;
+  if (s0 < s1) load_group(s0, ga);                  // older keys depend on nothing in this step
+  float sn4[4], cs4[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) sincosf(expf((float)(l16 * 4 + j) * a.neg_log_period_2_over_d) * fpos, &sn4[j], &cs4[j]);
+  pdl_wait();
+
+  if (exec && slot_new >= s0 && slot_new < s1) {    // CTA-uniform: this CTA owns the new key's slot
+    if (tid < ATT_D / 2) {
+      const int pr = tid;
+      float kr = bf2f(base[C + 2 * pr]), ki = bf2f(base[C + 2 * pr + 1]);
+      const float freq = expf((float)pr * a.neg_log_period_2_over_d);
+      float sn, cs;
+      sincosf(freq * fpos, &sn, &cs);
+      const float c2 = kr * cs - ki * sn, d2 = kr * sn + ki * cs;
+      const long long o = ((long long)bh * a.cap + slot_new) * ATT_D + 2 * pr;
+      *reinterpret_cast<__nv_bfloat162*>(a.kc + o) = __floats2bfloat162_rn(c2, d2);
+      *reinterpret_cast<__nv_bfloat162*>(a.vc + o) = *reinterpret_cast<const __nv_bfloat162*>(base + 2 * C + 2 * pr);
+    }
+    __syncthreads();
+    load_group(s0, ga);                             // the slot may be among the first keys
+  }
+
+  float qf[8];
+  {
+    float raw[8];
+    unpack8(*reinterpret_cast<const uint4*>(base + l16 * 8), raw);
+    const float scale = 0.08838834764831845f;       // 1/sqrt(128)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float qr = raw[2 * j], qi = raw[2 * j + 1];
+      qf[2 * j] = rbf(qr * cs4[j] - qi * sn4[j]) * scale;
+      qf[2 * j + 1] = rbf(qr * sn4[j] + qi * cs4[j]) * scale;
+    }
+  }
+  float m = -INFINITY, l = 0.f, acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+
   auto reduce_group = [&](int kb0, const Group& gp) {
     const int s = kb0 + hw * U;
 #pragma unroll
@@ -396,8 +470,6 @@ static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const Att
       }
     }
   };
-  Group ga, gb;
-  if (s0 < s1) load_group(s0, ga);
   for (int kb0 = s0; kb0 < s1; kb0 += 16 * U) {     // CTA-uniform trip count and branches (shuffles inside reduce_group)
     const int k1 = kb0 + 8 * U, k2 = kb0 + 16 * U;
     if (k1 < s1) load_group(k1, gb);
@@ -424,7 +496,7 @@ static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const Att
     L += sm_l[w] * c;
     A += sm_acc[w][tid] * c;
   }
-  if (a.nsplit == 1) {
+  if (splits == 1) {
     a.out[(long long)bh * ATT_D + tid] = f2bf(L > 0.f ? A / L : 0.f);
     return;
   }
@@ -435,22 +507,22 @@ static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const Att
   __syncthreads();
   if (tid == 0) {
     const int old = atomicAdd(a.counters + bh, 1);
-    s_last = old == a.nsplit - 1;
+    s_last = old == splits - 1;
     if (s_last) a.counters[bh] = 0;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
   const float* pp = a.part + (long long)bh * a.nsplit * (ATT_D + 2);
-  float MM = -INFINITY;
-  for (int s = 0; s < a.nsplit; ++s) MM = fmaxf(MM, __ldcg(pp + s * (ATT_D + 2) + ATT_D));
-  float LL = 0.f, AA = 0.f;
-  for (int s = 0; s < a.nsplit; ++s) {
-    const float ms = __ldcg(pp + s * (ATT_D + 2) + ATT_D);
-    const float c = ms == -INFINITY ? 0.f : __expf(ms - MM);
-    LL += __ldcg(pp + s * (ATT_D + 2) + ATT_D + 1) * c;
-    AA += __ldcg(pp + s * (ATT_D + 2) + tid) * c;
-  }
+  // lane s holds range s's maximum and sum: two round trips to L2 whatever the number of ranges
+  const float ms = lane < splits ? __ldcg(pp + lane * (ATT_D + 2) + ATT_D) : -INFINITY;
+  const float ls = lane < splits ? __ldcg(pp + lane * (ATT_D + 2) + ATT_D + 1) : 0.f;
+  const float MM = warp_max(ms);
+  const float cf = ms == -INFINITY ? 0.f : __expf(ms - MM);
+  const float LL = warp_sum(ls * cf);
+  float AA = 0.f;
+#pragma unroll 8
+  for (int s = 0; s < splits; ++s) AA += __ldcg(pp + s * (ATT_D + 2) + tid) * __shfl_sync(0xffffffffu, cf, s);
   a.out[(long long)bh * ATT_D + tid] = f2bf(LL > 0.f ? AA / LL : 0.f);
 }
 
@@ -714,6 +786,7 @@ constexpr int DEP_MAX_Q = 16;              // dep_q of the largest family member
 static __global__ void dep_attn_step_kernel(const bf16* __restrict__ qkv /*[B][3*H*D]*/, bf16* __restrict__ kc,
                                      bf16* __restrict__ vc, bf16* __restrict__ out, int B, int H, int cap, int step) {
   pdl_trigger();
+  pdl_wait();
   constexpr int D = 64;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= B * H) return;
@@ -939,6 +1012,7 @@ static __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const bf1
                                                                 long long* __restrict__ out, int card, int use_sampling,
                                                                 float temp, int top_k) {
   pdl_trigger();
+  pdl_wait();
   const int row = blockIdx.x;
   sample_row(logits_all + (long long)row * ld, noise + (long long)row * noise_ld, out + row, card, use_sampling, temp, top_k);
 }

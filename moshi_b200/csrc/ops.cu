@@ -156,7 +156,9 @@ int b200_op_attn_step(const void* qkv_dev, void* k_dev, void* v_dev, void* out_d
   using namespace b200::lm;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (B < 1 || H < 1 || cap < 1) B200_FAIL(B200_ERR_SHAPE, "op_attn_step: bad shape");
-  if (nsplit <= 0) nsplit = attn_pick_splits(B, H, cap);
+  int min_per = 1;
+  if (nsplit <= 0) nsplit = attn_ragged_splits(B, H, cap, &min_per);
+  if (nsplit > 32) B200_FAIL(B200_ERR_SHAPE, "op_attn_step: more than 32 splits");
   static float* part = nullptr;
   static int* counters = nullptr;
   static size_t part_n = 0, cnt_n = 0;
@@ -175,7 +177,7 @@ int b200_op_attn_step(const void* qkv_dev, void* k_dev, void* v_dev, void* out_d
   AttnStep a;
   a.qkv = static_cast<const bf16*>(qkv_dev); a.kc = static_cast<bf16*>(k_dev); a.vc = static_cast<bf16*>(v_dev);
   a.out = static_cast<bf16*>(out_dev); a.part = part; a.counters = counters;
-  a.pos = reinterpret_cast<const long long*>(pos_dev); a.exec_mask = exec_mask_dev; a.H = H; a.cap = cap; a.nsplit = nsplit;
+  a.pos = reinterpret_cast<const long long*>(pos_dev); a.exec_mask = exec_mask_dev; a.H = H; a.cap = cap; a.nsplit = nsplit; a.min_per = min_per;
   a.neg_log_period_2_over_d = -logf(max_period) * 2.f / (float)ATT_D;
   dim3 grid(B * H, nsplit);
   if (attn_group_keys() == 2) B200_LAUNCH(attn_step_kernel<2>, grid, ATT_THREADS, 0, st, a);
