@@ -675,7 +675,10 @@ int b200_lm_streaming_begin(b200_lm* h, int batch, void* stream) {
   // One or two sessions: the depformer's linears take the GEMV path and the PDL-chained launches beat the persistent kernel
   // (B=1: 5.5 vs 6.4 ms per LM step, B=2: 6.2 vs 7.1; profiles/r01_r_*).  B200_DEP_FUSED=2 forces the kernel at any batch.
   // Under classifier-free guidance the two halves of the batch meet before every sampler (lm.py:828-833): launch chain.
-  const bool dep_small = B <= tc::sk_gemv_max_m() && h->dep_fused != 2;
+  tc::DepFusedConfig few;
+  memset(&few, 0, sizeof(few));
+  few.B = B; few.dd = dd; few.F = c.depformer_ffn_hidden; few.card = c.card;
+  const bool dep_small = B <= tc::sk_gemv_max_m() && h->dep_fused != 2 && !tc::dep_fused_in_registers(few);
   h->depf = nullptr;
   if (c.dep_q > 0 && !cfg && !c.quantize && h->dep_fused && !dep_small && B <= 256 && dd <= 1024 && dd % 64 == 0) {
     tc::DepFusedConfig fc;
