@@ -628,6 +628,11 @@ int b200_op_attn_step_q8(const void* qkv_dev, void* k8_dev, void* v8_dev, float*
  * 64, 128, .., 512 elements take the mma kernel (as in the handle); 0: always the CUDA-core kernel.  Synchronises (test helper). */
 int b200_op_latent_attention(const float* qa_dev, const void* latents_dev, int dtype, const float* sink_dev, float* out_dev,
                              int T, int H, int r, int pos0, int nsplit, int tensor_cores, void* stream);
+/* The decoder LM's attention of a long portion (csrc/dlm_flash.cu) for one request: q bf16 [T][H * 128], k [pos0 + T][H * 128], vt the values
+ * transposed, [H * 128][ldv] with a column per key (ldv a multiple of 8), sink f32 [H] or NULL; query t sits at position pos0 + t and sees keys
+ * 0 .. pos0 + t; out bf16 [T][H * 128].  Enqueues on the stream. */
+int b200_op_prefill_attention(const void* q_dev, const void* k_dev, const void* vt_dev, const float* sink_dev, void* out_dev, int T, int H, int pos0,
+                              int ldv, float scale, void* stream);
 int b200_op_sample(const void* logits_bf16_dev, const float* noise_dev, int64_t* out_dev, int B,
                    int card, int use_sampling, float temp, int top_k, void* stream);
 

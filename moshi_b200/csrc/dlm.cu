@@ -10,6 +10,7 @@
 
 #include <cmath>
 
+#include "dlm_flash.cuh"
 #include "dlm_kernels.cuh"
 #include "dlm_mixers.cuh"
 #include "dlm_mixers2.cuh"
@@ -37,6 +38,7 @@ struct Layer {
   int ncat = 0, ldp = 0, off_q = 0, off_dkv = 0, off_up = 0, off_g1 = 0, off_g2 = 0;
   Weight cat, o, down;                 // [q | dkv | up | gate1 | gate2] x width;  width x (heads * vdim);  width x ff
   void *ukT = nullptr, *uv = nullptr;  // [H][r][dim] (transposed per head), [H * vdim][r]
+  void* uk = nullptr;                  // [H * dim][r]: long portions expand the latents to keys (null: not a shape of dlm_flash.cu)
   float *n1w = nullptr, *n1b = nullptr, *cnorm = nullptr, *sink = nullptr, *b1 = nullptr, *b2 = nullptr, *avg = nullptr;
   void* cache = nullptr;               // [slots][cap][r]
   int sig = 0;                         // index of the layer's attention tile list
@@ -143,6 +145,11 @@ struct b200_dlm {
   int scan_seg = 256, n_units = 0, max_seg_units = 0, off_ent_seg = 0, off_ent_nseg = 0, off_ent_buf = 0;
   struct ScanUnit { int tok0, ntok, seg, buf; };
   std::vector<ScanUnit> units;
+  // the step's entries; long portions of the gated block attend on keys and values expanded from the latents, [flash_rows][H * dim] and
+  // transposed [H * vdim][flash_rows], one request after another
+  struct Portion { int tok0, n, slot, pos0; };
+  std::vector<Portion> portions;
+  bf16 *flash_k = nullptr, *flash_v = nullptr; int flash_rows = 0;
   float *segS = nullptr, *segB = nullptr, *segM = nullptr, *tokM = nullptr, *corr = nullptr;
   float *embw = nullptr, *h32 = nullptr, *qkv32 = nullptr, *scan32 = nullptr, *gate32 = nullptr, *attn32 = nullptr, *route32 = nullptr, *moe_w = nullptr, *scan_prep = nullptr, *scan_v = nullptr;
   void *mixo2 = nullptr, *obuf2 = nullptr, *yexp = nullptr;
@@ -403,6 +410,35 @@ int finish_logits(b200_dlm* h, const bf16* in_bf, long long ld, int n_want, int 
   return check_launch("logits");
 }
 
+// Attention of long portions: scoring in the latent space costs r + r products per query, head and key where keys and values of the heads'
+// own size cost 128 + 128, and expanding a latent to all heads is paid once for all queries.  Worth it from 128 queries on (2048 tokens, 16
+// heads, r = 512: 497 us per layer with the folds around the latent kernel, 90 us expanded); shorter portions stay in the latent space.
+constexpr int EXPAND_FROM = 128;
+bool expands_latents(const b200_dlm* h, const Layer& L, int max_ctx) {
+  if (!L.uk || !h->attn_tc || max_ctx > h->flash_rows || !(L.c.a.scale > 0.f) || (L.ldp | L.off_q) % 8) return false;
+  for (const auto& q : h->portions)
+    if (q.n < EXPAND_FROM) return false;
+  return true;
+}
+int expanded_attention(b200_dlm* h, const Layer& L, const bf16* proj, bf16* ob) {
+  const int H = L.c.a.heads, r = L.c.a.kv_rank;
+  const bf16 *uk = static_cast<const bf16*>(L.uk), *uv = static_cast<const bf16*>(L.uv);
+  for (const auto& q : h->portions) {
+    const int ctx = q.pos0 + q.n;
+    const bf16* lat = static_cast<const bf16*>(L.cache) + (size_t)q.slot * h->cap * r;
+    tc::WideGemm k;
+    k.x = lat; k.ldx = r; k.x_rows = ctx; k.w = uk; k.w_rows = H * FLASH_D; k.y = h->flash_k; k.ldy = H * FLASH_D; k.M = ctx; k.N = H * FLASH_D; k.K = r; k.err = h->err;
+    tc::WideGemm v;
+    v.x = uv; v.ldx = r; v.x_rows = H * FLASH_D; v.w = lat; v.w_rows = ctx; v.y = h->flash_v; v.ldy = h->flash_rows; v.M = H * FLASH_D; v.N = ctx; v.K = r; v.err = h->err;
+    TIMED(CLS_FOLD, B200_TRY(tc::wide_gemm(k, h->stream)); B200_TRY(tc::wide_gemm(v, h->stream)));
+    FlashAttn a;
+    a.q = proj + (size_t)q.tok0 * L.ldp + L.off_q; a.ldq = L.ldp; a.k = h->flash_k; a.ldk = H * FLASH_D; a.vt = h->flash_v; a.ldv = h->flash_rows;
+    a.sink = L.sink; a.out = ob + (size_t)q.tok0 * H * FLASH_D; a.ldo = H * FLASH_D; a.T = q.n; a.pos0 = q.pos0; a.H = H; a.scale = L.c.a.scale; a.err = h->err;
+    TIMED(CLS_ATTN, B200_TRY(flash_attention(a, h->stream)));
+  }
+  return B200_OK;
+}
+
 template <typename T>
 int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out) {
   const b200_dlm_config& c = h->cfg;
@@ -424,14 +460,18 @@ int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out
     // mixer: latent attention
     TIMED(CLS_ELEMENTWISE, B200_LAUNCH(latent_append_kernel<T>, ceil_div(n_tok, 4), 128, 0, st, proj, (long long)L.ldp, L.off_dkv, L.cnorm, static_cast<T*>(L.cache),
                 h->cap, r, meta + h->off_slot, meta + h->off_pos, n_tok, c.norm_eps));
-    // query folded through W_uk (and the score scale): qa[t][h][:] = scale * q[t][h][:] . W_uk[h]
-    TIMED(CLS_FOLD, B200_TRY(head_gemm(st, proj + L.off_q, (long long)L.ldp, (long long)dk, static_cast<const T*>(L.ukT), (long long)dk, (long long)r * dk, h->qa,
-                     (long long)H * r, (long long)r, n_tok, r, dk, H, L.c.a.scale, h->attn_tc != 0)));
-    TIMED(CLS_ATTN, B200_TRY(attention<T>(h, L, max_ctx)));
-    // values: o[t][h][:] = W_uv[h] . (sum_j p_j c_j)
     T* ob = static_cast<T*>(h->obuf);
-    TIMED(CLS_FOLD, B200_TRY(head_gemm(st, h->ol, (long long)H * r, (long long)r, static_cast<const T*>(L.uv), (long long)r, (long long)dv * r, ob, (long long)H * dv,
-                     (long long)dv, n_tok, dv, r, H, 1.f, h->attn_tc != 0)));
+    if (expands_latents(h, L, max_ctx)) {
+      if constexpr (sizeof(T) == 2) B200_TRY(expanded_attention(h, L, proj, ob));
+    } else {
+      // query folded through W_uk (and the score scale): qa[t][h][:] = scale * q[t][h][:] . W_uk[h]
+      TIMED(CLS_FOLD, B200_TRY(head_gemm(st, proj + L.off_q, (long long)L.ldp, (long long)dk, static_cast<const T*>(L.ukT), (long long)dk, (long long)r * dk, h->qa,
+                       (long long)H * r, (long long)r, n_tok, r, dk, H, L.c.a.scale, h->attn_tc != 0)));
+      TIMED(CLS_ATTN, B200_TRY(attention<T>(h, L, max_ctx)));
+      // values: o[t][h][:] = W_uv[h] . (sum_j p_j c_j)
+      TIMED(CLS_FOLD, B200_TRY(head_gemm(st, h->ol, (long long)H * r, (long long)r, static_cast<const T*>(L.uv), (long long)r, (long long)dv * r, ob, (long long)H * dv,
+                       (long long)dv, n_tok, dv, r, H, 1.f, h->attn_tc != 0)));
+    }
     T* mixo = static_cast<T*>(h->mixo);
     TIMED(CLS_LINEAR, B200_TRY(linear<T>(h, ob, (long long)H * dv, L.o, mixo, W, n_tok)));
     // feed-forward
@@ -2602,7 +2642,8 @@ int b200_dlm_finalize(b200_dlm* h) {
       if (h->f32) B200_LAUNCH(head_transpose_kernel<float>, (unsigned)ceil_div64(n, 256), 256, 0, nullptr, static_cast<const float*>(uk), static_cast<float*>(L.ukT), (int)H, (int)dk, (int)r);
       else B200_LAUNCH(head_transpose_kernel<bf16>, (unsigned)ceil_div64(n, 256), 256, 0, nullptr, static_cast<const bf16*>(uk), static_cast<bf16*>(L.ukT), (int)H, (int)dk, (int)r);
       B200_TRY(check_launch("head_transpose"));
-      drop.push_back(uk);
+      if (!h->f32 && dk == FLASH_D && dv == FLASH_D && r % 8 == 0) L.uk = uk;
+      else drop.push_back(uk);
       h->weight_bytes += n * es;
     }
     B200_TRY(matrix(p + "mix.uv", H * dv, r, &L.uv));
@@ -2886,6 +2927,15 @@ int b200_dlm_cache_begin(b200_dlm* h, int slots, int capacity, int max_step_toke
     B200_TRY(A.alloc_t(&h->ol, T * max_hr));
     h->part_floats = (size_t)600 * 16 * (max_r + 2);
     B200_TRY(A.alloc(&h->ffo, T * W * es));
+    // expanded keys and values of one request; beyond 16384 tokens of context portions stay in the latent space
+    size_t hd = 0;
+    for (auto& L : h->layers) if (L.uk) hd = std::max(hd, (size_t)L.c.a.heads * FLASH_D);
+    h->flash_rows = 0;
+    if (hd) {
+      h->flash_rows = (std::min(capacity, 16384) + 7) / 8 * 8;
+      B200_TRY(A.alloc_t(&h->flash_k, hd * h->flash_rows, false));
+      B200_TRY(A.alloc_t(&h->flash_v, hd * h->flash_rows, false));
+    }
   } else {
     B200_TRY(A.alloc_t(&h->h32, T * W));
     B200_TRY(A.alloc_t(&h->qkv32, T * max_qkv));
@@ -3015,9 +3065,11 @@ int b200_dlm_step(b200_dlm* h, int n_entries, const int32_t* slots_host, const i
   int* m = h->meta_pin;
   int t = 0, max_ctx = 0, n_seg_units = 0, n_chunks = 0;
   h->units.clear();
+  h->portions.clear();
   for (auto& s : h->sigs) s.count = 0;
   for (int e = 0; e < n_entries; ++e) {
     const int s = slots_host[e], n = counts_host[e], base = h->len[s];
+    h->portions.push_back({t, n, s, base});
     for (auto& sg : h->sigs) {
       const int rows = n * sg.H;
       for (int r0 = 0; r0 < rows; r0 += sg.rpt) {

@@ -1,0 +1,73 @@
+"""GPU: attention of long prompt portions (csrc/dlm_flash.cu) against the softmax in fp32, alone and inside a model."""
+import ctypes as C
+
+import pytest
+import torch
+
+from .util import cptr
+
+pytestmark = pytest.mark.gpu
+
+
+def _want(q, k, v, sink, pos0, scale):
+    T, H, _ = q.shape
+    s = torch.einsum("thd,nhd->htn", q.float(), k.float()) * scale
+    n = torch.arange(k.shape[0], device=q.device)
+    s = s.masked_fill(n[None, None, :] > (pos0 + torch.arange(T, device=q.device))[None, :, None], -torch.inf)
+    if sink is not None:
+        s = torch.cat([s, sink.view(-1, 1, 1).expand(-1, T, 1)], -1)
+    return torch.einsum("htn,nhd->thd", torch.softmax(s, -1)[..., :k.shape[0]], v.float())
+
+
+@pytest.mark.parametrize("T,pos0,H,spread", [(1, 0, 1, 1.0), (127, 0, 2, 1.0), (128, 0, 3, 4.0), (129, 1, 2, 1.0), (300, 77, 2, 8.0), (640, 129, 1, 1.0), (1000, 0, 16, 2.0)])
+@pytest.mark.parametrize("with_sink", [True, False])
+def test_attention_of_a_portion(T, pos0, H, spread, with_sink):
+    """Tiles that end before, on and behind their edge, one key to many tiles, scores whose maximum keeps moving (spread)."""
+    from moshi_b200 import _lib
+    lib = _lib.lib()
+    g = torch.Generator().manual_seed(T + pos0)
+    ctx, ld = pos0 + T, (pos0 + T + 15) // 8 * 8
+    q, k, v = (torch.randn(n, H, 128, generator=g).bfloat16().cuda() for n in (T, ctx, ctx))
+    k *= (1 + spread * torch.arange(ctx, device="cuda") / ctx).bfloat16()[:, None, None]
+    vt = torch.full((H * 128, ld), float("nan"), dtype=torch.bfloat16, device="cuda")
+    vt[:, :ctx] = v.reshape(ctx, -1).t()
+    sink = torch.randn(H, generator=g).cuda() if with_sink else None
+    out = torch.full((T, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    _lib.check(lib.b200_op_prefill_attention(cptr(q), cptr(k), cptr(vt), cptr(sink), cptr(out), T, H, pos0, ld, 128 ** -0.5,
+                                             C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    want = _want(q, k, v, sink, pos0, 128 ** -0.5)
+    assert not torch.isnan(out.float()).any()
+    # the weights and the result are each rounded to bf16, eight significant bits: half a unit is up to 2^-8 of the value, so 2^-7 of the
+    # weighted sum of |v| (which bounds the result) in all, plus fp32 order
+    bound = 2.0 ** -7 * _want(q, k, v.abs(), sink, pos0, 128 ** -0.5) + 1e-4
+    assert ((out.float() - want).abs() <= bound).all(), float(((out.float() - want).abs() - bound).max())
+
+
+def test_long_portions_agree_with_short_ones():
+    """A request taken as one portion, as portions on both sides of the line between the two kernels, and beside another long one."""
+    from moshi_b200.config import DecoderLMConfig
+    from moshi_b200.models import DecoderLMGen, loaders
+    lay = {"type": "latent_attention", "mixer": {"heads": 2, "dim": 128, "vdim": 128, "kv_rank": 64, "scale": 128 ** -0.5}, "mlp": {"kind": "dense", "ff": 512}}
+    cfg = DecoderLMConfig.from_dict({"architecture": "Likosun", "vocab": 320, "width": 256, "embedding": {"scale": 1.0}, "residual_mult": 0.5,
+                                     "norm": {"eps": 1e-6}, "layers": [lay] * 2})
+    model = loaders.get_decoder_lm(None, cfg, device="cuda:0", synth_seed=5)
+    g = torch.Generator().manual_seed(3)
+    toks = torch.randint(0, 320, (300,), generator=g).tolist()
+    other = torch.randint(0, 320, (150,), generator=g).tolist()
+
+    def run(cuts, beside=False):
+        with DecoderLMGen(model, slots=2, capacity=320, max_step_tokens=512) as gen:
+            out, at = [], 0
+            for n in cuts:
+                entries = [(1, toks[at:at + n])] + ([(0, other)] if beside else [])
+                out.append(gen.step(entries, range(n)))
+                at += n
+            assert gen.error_flags() == 0
+            return torch.cat(out)
+
+    whole = run([300])
+    for cuts, beside in (([128, 172], False), ([100, 100, 100], False), ([127, 173], False), ([300], True)):
+        got = run(cuts, beside)
+        # two bf16 layers: what the model tests allow between ways of cutting a prompt
+        assert ((got - whole).norm() / whole.norm()) < 1e-2, cuts
