@@ -93,30 +93,34 @@ __device__ __forceinline__ void reg_product(const RegW& w, int groups, int num_k
     for (int a = 0; a < A; ++a)
 #pragma unroll
       for (int n = 0; n < NT; ++n) acc[gi][a][n][0] = acc[gi][a][n][1] = acc[gi][a][n][2] = acc[gi][a][n][3] = 0.f;
-  uint4 xb[KBW][2][NT];
+  constexpr int AHEAD = NT == 1 || KBW <= 2 ? KBW : 2;      // activations in flight: what the registers beside the weights hold
 #pragma unroll
-  for (int j = 0; j < KBW; ++j)
+  for (int j0 = 0; j0 < KBW; j0 += AHEAD) {
+    uint4 xb[AHEAD][2][NT];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int j = 0; j < AHEAD; ++j)
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
-        if (warp * KBW + j < num_kb) xb[j][h][n] = x(8 * n + g, (warp * KBW + j) * 128 + h * 64 + t * 16);
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-  for (int j = 0; j < KBW; ++j) {
-    if (warp * KBW + j >= num_kb) break;
+        for (int n = 0; n < NT; ++n)
+          if (warp * KBW + j0 + j < num_kb) xb[j][h][n] = x(8 * n + g, (warp * KBW + j0 + j) * 128 + h * 64 + t * 16);
 #pragma unroll
-    for (int gi = 0; gi < G; ++gi) {
-      if ((int)(blockIdx.x + gi * gridDim.x) >= groups) break;
+    for (int j = 0; j < AHEAD; ++j) {
+      if (warp * KBW + j0 + j >= num_kb) break;
 #pragma unroll
-      for (int a = 0; a < A; ++a) {
-        const uint4 (&f)[4] = w.f[(gi * KBW + j) * A + a];
+      for (int gi = 0; gi < G; ++gi) {
+        if ((int)(blockIdx.x + gi * gridDim.x) >= groups) break;
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int a = 0; a < A; ++a) {
+          const uint4 (&f)[4] = w.f[(gi * KBW + j0 + j) * A + a];
 #pragma unroll
-          for (int n = 0; n < NT; ++n) {
-            reg_mma(acc[gi][a][n], f[2 * h].x, f[2 * h + 1].x, f[2 * h].y, f[2 * h + 1].y, xb[j][h][n].x, xb[j][h][n].y);
-            reg_mma(acc[gi][a][n], f[2 * h].z, f[2 * h + 1].z, f[2 * h].w, f[2 * h + 1].w, xb[j][h][n].z, xb[j][h][n].w);
-          }
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+              reg_mma(acc[gi][a][n], f[2 * h].x, f[2 * h + 1].x, f[2 * h].y, f[2 * h + 1].y, xb[j][h][n].x, xb[j][h][n].y);
+              reg_mma(acc[gi][a][n], f[2 * h].z, f[2 * h + 1].z, f[2 * h].w, f[2 * h + 1].w, xb[j][h][n].z, xb[j][h][n].w);
+            }
+        }
       }
     }
   }
