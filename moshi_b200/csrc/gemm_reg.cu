@@ -166,22 +166,36 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(EPI, NT)) gemm_reg_kernel
   }
   __syncthreads();
   if (arrived != p.S - 1) return;
-  const float* part = p.ws + (size_t)tile * p.S * SLOT;
-  for (int i = threadIdx.x; i < p.M * ROWS; i += THREADS) {
-    const int m = i / ROWS, r = i - m * ROWS, n = tile * ROWS + r;
-    if (n >= p.out_rows) continue;
-    float v[2];
+  // four neighbouring rows of one token per thread, eight ranges' loads in flight
+  const float4* part = reinterpret_cast<const float4*>(p.ws + (size_t)tile * p.S * SLOT);
+  for (int i = threadIdx.x; i < p.M * (ROWS / 4); i += THREADS) {
+    const int m = i / (ROWS / 4), r4 = i - m * (ROWS / 4);
+    Acc v[2][4];
 #pragma unroll
     for (int a = 0; a < A; ++a) {
-      Acc s = 0;
-#pragma unroll 8
-      for (int q = 0; q < p.S; ++q) {
-        const float f = __ldcg(part + (size_t)q * SLOT + (a * 8 * NT + m) * ROWS + r);
-        if constexpr (I8) s += __float_as_int(f); else s += f;
+      v[a][0] = v[a][1] = v[a][2] = v[a][3] = 0;
+      const float4* q = part + (a * 8 * NT + m) * (ROWS / 4) + r4;
+      for (int s0 = 0; s0 < p.S; s0 += 8) {
+        float4 f[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (s0 + u < p.S) f[u] = __ldcg(q + (size_t)(s0 + u) * (SLOT / 4));
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (s0 + u >= p.S) break;
+          if constexpr (I8) {
+            v[a][0] += __float_as_int(f[u].x); v[a][1] += __float_as_int(f[u].y); v[a][2] += __float_as_int(f[u].z); v[a][3] += __float_as_int(f[u].w);
+          } else {
+            v[a][0] += f[u].x; v[a][1] += f[u].y; v[a][2] += f[u].z; v[a][3] += f[u].w;
+          }
+        }
       }
-      v[a] = bits(s);
     }
-    finish<EPI, I8>(p, m, n, v[0], v[A - 1]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int n = tile * ROWS + r4 * 4 + e;
+      if (n < p.out_rows) finish<EPI, I8>(p, m, n, bits(v[0][e]), bits(v[A - 1][e]));
+    }
   }
 }
 
@@ -193,6 +207,16 @@ cudaError_t launch_nt(const cudaLaunchConfig_t& cfg, const RegP& p) {
 }
 
 }  // namespace
+
+// Where the kernel is ahead of gemm_sk.cu (7B shapes, bf16, us): everything up to 8 rows (4096 -> 4096 22.9 -> 10.8, -> 12288 30.9 -> 22.1); up to 32
+// rows too (32 rows 41.0 -> 17.0 and 35.7 -> 29.8) but for gated pairs beyond 16 rows, whose fragments leave one CTA per SM (52 -> 64), and
+// for 16-bit weights of more tiles than SMs beyond 8 rows, where whole tiles per CTA leave the second CTA of an SM idle (250 tiles, 32 rows
+// 55.6 -> 67.9; 8 rows 53.8 -> 51.9; int8 39.4 -> 38.1).
+bool reg_wins(int M, int N, int epi, int gate_rows, bool i8, int sms) {
+  const int tiles = ((epi == EPI_GATE ? gate_rows : N) + ROWS - 1) / ROWS;
+  if (epi == EPI_GATE && M > 16) return false;
+  return i8 || M <= 8 || tiles <= sms;
+}
 
 bool reg_supported(int M, const void* x, long long ldx_bytes) {
   return M >= 1 && M <= REG_MAX_M && ldx_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
