@@ -51,6 +51,26 @@ extern std::atomic<int64_t> g_launches;
     b200::g_launches.fetch_add(1, std::memory_order_relaxed);                  \
   } while (0)
 
+// Launch that may begin while the preceding kernel of the stream drains (programmatic dependent launch): the kernel calls griddepcontrol.wait
+// before it touches anything that an earlier kernel writes or reads.  Between the plain launches of a chain of small kernels the GPU
+// stands still for 1.5-2 us each.  Such a kernel takes __restrict__ only on weights and tables: a load that the compiler knows to be
+// invariant may move above the wait, and then reads what the preceding kernel has not written yet.
+template <typename... P, typename... A>
+inline int launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return B200_OK;
+}
+#define EARLY_LAUNCH(kernel, grid, block, smem, stream, ...) B200_TRY(b200::launch_early(kernel, dim3(grid), dim3(block), smem, stream, __VA_ARGS__))
+
 inline int check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

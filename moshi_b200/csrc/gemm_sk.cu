@@ -892,8 +892,8 @@ __global__ void pack_tiles_i8_pre_kernel(const int8_t* __restrict__ q, uint4* __
   out[idx] = make_uint4(words[0], words[1], words[2], words[3]);
 }
 // activations: x [M][K] bf16 (row stride ldx) -> xq int8 [M][K], sa[m] = absmax of the row
-__global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int8_t* __restrict__ xq,
-                                                           float* __restrict__ sa, int K) {
+__global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16* x, long long ldx, int8_t* xq,
+                                                           float* sa, int K) {
   const int row = blockIdx.x;
   const __nv_bfloat16* xr = x + (long long)row * ldx;
   float mx = 0.f;

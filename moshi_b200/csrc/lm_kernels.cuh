@@ -21,23 +21,6 @@ typedef __nv_bfloat16 bf16;
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launch that may begin while the preceding kernel drains: the kernel calls pdl_wait() before it touches what that one writes or reads.
-// Between the kernels of a step a plain launch costs 1.5-2 us of idle GPU.
-template <typename... P, typename... A>
-inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = grid; cfg.blockDim = block; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-  if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return B200_OK;
-}
-
 __device__ __forceinline__ void unpack8(const uint4& v, float* f) {
   const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
@@ -175,9 +158,9 @@ static __global__ void lm_embed_sum_kernel(const EmbedTables t, const long long*
 
 // depformer input: x = depformer_in[k](transformer_out) + emb(prev)   (lm.py:475-486); with CFG the rows [Bt, 2*Bt) reuse the
 // tokens of rows [0, Bt) (lm.py:824-826)
-static __global__ void dep_input_kernel(const bf16* __restrict__ din /*[B][ld]*/, long long ld, int col0,
-                                 const bf16* __restrict__ table /*[V][dd]*/, const long long* __restrict__ prev /*[Bt]*/,
-                                 bf16* __restrict__ x /*[B][dd]*/, int B, int dd, int Bt, int vocab, int* err) {
+static __global__ void dep_input_kernel(const bf16* din /*[B][ld]*/, long long ld, int col0,
+                                 const bf16* table /*[V][dd]*/, const long long* prev /*[Bt]*/,
+                                 bf16* x /*[B][dd]*/, int B, int dd, int Bt, int vocab, int* err) {
   pdl_trigger();
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -252,8 +235,8 @@ static __global__ void lm_noise_kernel(float* __restrict__ noise, long long n, u
 // RMSNorm with fp32 math, eps 1e-8 (transformer.py:45-58): y = bf16(x * (alpha * rsqrt(eps + mean(x^2))))
 // Optionally fuses the preceding residual add: x <- bf16(x + upd) first (transformer.py:769,777).
 // ---------------------------------------------------------------------------------------------
-static __global__ void __launch_bounds__(256) rmsnorm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ alpha,
-                                                      bf16* __restrict__ y, int dim, float eps) {
+static __global__ void __launch_bounds__(256) rmsnorm_kernel(const bf16* x, const bf16* alpha,
+                                                      bf16* y, int dim, float eps) {
   pdl_trigger();
   const int row = blockIdx.x;
   const bf16* xr = x + (long long)row * dim;
@@ -783,8 +766,8 @@ constexpr int DEP_MAX_Q = 16;              // dep_q of the largest family member
 
 // Depformer attention step: the new key/value of sub-step `step` is appended to the per-frame cache and the query
 // attends over step + 1 keys; no positional embedding (depformer_pos_emb = "none").  One warp per (b, h), D = 64.
-static __global__ void dep_attn_step_kernel(const bf16* __restrict__ qkv /*[B][3*H*D]*/, bf16* __restrict__ kc,
-                                     bf16* __restrict__ vc, bf16* __restrict__ out, int B, int H, int cap, int step) {
+static __global__ void dep_attn_step_kernel(const bf16* qkv /*[B][3*H*D]*/, bf16* kc,
+                                     bf16* vc, bf16* out, int B, int H, int cap, int step) {
   pdl_trigger();
   pdl_wait();
   constexpr int D = 64;
@@ -1007,9 +990,9 @@ static __device__ void sample_row(const bf16* __restrict__ logits, const float* 
   }
 }
 
-static __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const bf16* __restrict__ logits_all, long long ld,
-                                                                const float* __restrict__ noise, long long noise_ld,
-                                                                long long* __restrict__ out, int card, int use_sampling,
+static __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const bf16* logits_all, long long ld,
+                                                                const float* noise, long long noise_ld,
+                                                                long long* out, int card, int use_sampling,
                                                                 float temp, int top_k) {
   pdl_trigger();
   pdl_wait();
