@@ -32,7 +32,11 @@ using namespace tcp;
 
 constexpr int EPI_STORE = 0, EPI_RESADD = 1, EPI_GATE = 2;
 constexpr int BLOCK_ROWS = 128, BLOCK_K = 64, UMMA_K = 16;
-constexpr int NUM_THREADS = 192;             // warp 0 producer, warp 1 MMA, warps 2-5 epilogue
+// warp 0 producer, warp 1 MMA, warps 2-17 epilogue: four per TMEM quadrant, every fourth run of 16 columns each.  The epilogue is a chain
+// of latencies per run (TMEM load, silu, store) that nothing hides.  One warp per quadrant: the gated product 22528 x 4096 took 57.5 us at
+// 104 sessions and 92.4 at 200, of which 29 did not depend on K (half the K: 43.3); four: 41.8 and 60.2.  Plain products gain 0-1 us.
+constexpr int NUM_THREADS = 576;
+constexpr int EPI_STEP = 64;                 // columns between the runs of one epilogue warp
 constexpr int TILE_BYTES = BLOCK_ROWS * BLOCK_K * 2;
 constexpr int A_BYTES = 128 * BLOCK_K * 2;   // one activation box: 128 session rows x 64 k
 constexpr int MAX_STAGES = 8;
@@ -187,7 +191,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
     __syncwarp();
   }
 
-  const int q4 = warp & 3;
+  const int q4 = warp & 3, run0 = ((warp - 2) >> 2) * 16;             // TMEM quadrant; first run of columns of an epilogue warp
   const int my_c0 = col_begin(width, p.CS, me), my_c1 = col_begin(width, p.CS, me + 1);
   if (warp >= 2) {
     mbar_wait(tfull, 0);
@@ -206,7 +210,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
           const int c0q = col_begin(width, p.CS, q), c1q = col_begin(width, p.CS, q + 1);
           const int slot = me < q ? me : me - 1;
           const uint32_t dst = ns_map_to_rank(base + (uint32_t)((slot * 128 + q4 * 32 + lane) * p.ldw) * 4u, (uint32_t)q);
-          for (int c = c0q; c < c1q; c += 16) {
+          for (int c = c0q + run0; c < c1q; c += EPI_STEP) {
             uint32_t r[16];
             if (n_items > 0) {
               tmem_ld16(lane_addr + (uint32_t)c, r);
@@ -230,7 +234,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
       if (EPI == EPI_GATE) {
         // columns j (gate) and 128 + j (value) of the same output; CS == 1 (the pair never needs a split: 88 units at 7B)
         const int nb = unit * BLOCK_ROWS;
-        for (int c = 0; c < 128; c += 16) {
+        for (int c = run0; c < 128; c += EPI_STEP) {
           uint32_t g[16], u[16];
           tmem_ld16(lane_addr + (uint32_t)c, g);
           tmem_ld16(lane_addr + (uint32_t)(128 + c), u);
@@ -248,7 +252,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
         }
       } else {
         const int nb = tile0 * BLOCK_ROWS;
-        for (int c = my_c0; c < my_c1; c += 16) {
+        for (int c = my_c0 + run0; c < my_c1; c += EPI_STEP) {
           float acc[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) acc[j] = 0.f;
