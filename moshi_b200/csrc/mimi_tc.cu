@@ -109,7 +109,7 @@ mimi_tc_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull0 + 8 * a, 1);
-      mbar_init(tempty0 + 8 * a, 4);           // one arrival per epilogue warp
+      mbar_init(tempty0 + 8 * a, TC_EPI_WARPS);           // one arrival per epilogue warp
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -191,7 +191,7 @@ mimi_tc_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant
     __syncwarp();
   } else {
     // ===== epilogue: TMEM lane = GEMM row = one (session, step) =====
-    const int q = warp & 3;
+    const int q = warp & 3, run0 = ((warp - 2) >> 2) * 16;        // TMEM quadrant; first of this warp's runs of 16 columns
     const int row = q * 32 + lane;
     const int bi = row / p.tt, ti = row - bi * p.tt;
     int acc = 0; uint32_t acc_bits = 0u;
@@ -204,7 +204,7 @@ mimi_tc_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant
       tc_fence_after();
       const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * p.NT);
       const int n_base = tl.n * p.NT;
-      for (int c0 = 0; c0 < p.NT; c0 += 16) {
+      for (int c0 = run0; c0 < p.NT; c0 += 4 * TC_EPI_WARPS) {
         uint32_t r[16];
         tmem_ld16(lane_addr + (uint32_t)c0, r);
         tmem_ld_wait();

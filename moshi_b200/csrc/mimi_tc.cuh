@@ -34,7 +34,9 @@ namespace mtc {
 constexpr int TC_ROWS = 128;            // GEMM rows (tokens) per tile = UMMA M
 constexpr int TC_KB = 32;               // fp32 elements per k-block row: 128 bytes = one SWIZZLE_128B row
 constexpr int TC_MAX_NT = 128;          // output features per tile = UMMA N (<= 128: 64 KB per stage, 3 stages)
-constexpr int TC_THREADS = 192;
+constexpr int TC_EPI_WARPS = 16;         // four per TMEM quadrant: the epilogue is a chain of latencies per run of 16 features
+                                        // (one per quadrant: a frame of 40 sessions took 1982 us, of one session 739; four: 1850 and 690)
+constexpr int TC_THREADS = 64 + 32 * TC_EPI_WARPS;
 constexpr int TC_MAX_STAGES = 6;
 
 enum { TC_EPI_CONV = 0, TC_EPI_GELU = 1, TC_EPI_RES_SCALE = 2 };
