@@ -56,19 +56,25 @@ extern std::atomic<int64_t> g_launches;
 // stands still for 1.5-2 us each.  Such a kernel takes __restrict__ only on weights and tables: a load that the compiler knows to be
 // invariant may move above the wait, and then reads what the preceding kernel has not written yet.
 template <typename... P, typename... A>
-inline int launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+inline int launch_early_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  cfg.attrs = attr; cfg.numAttrs = early ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
   if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return B200_OK;
 }
+template <typename... P, typename... A>
+inline int launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  return launch_early_if(true, kernel, grid, block, smem, st, args...);
+}
+#define EARLY_LAUNCH_IF(early, kernel, grid, block, smem, stream, ...) \
+  B200_TRY(b200::launch_early_if(early, kernel, dim3(grid), dim3(block), smem, stream, __VA_ARGS__))
 #define EARLY_LAUNCH(kernel, grid, block, smem, stream, ...) B200_TRY(b200::launch_early(kernel, dim3(grid), dim3(block), smem, stream, __VA_ARGS__))
 
 inline int check_launch(const char* what) {

@@ -231,6 +231,11 @@ int seal_weight(b200_dlm* h, Weight& w, void* rm, int N, int K, std::vector<void
   return B200_OK;
 }
 
+// Routed blocks of so many tokens launch their elementwise kernels the ordinary way: they fill the chip several times over, and a grid that
+// already waits on the SMs is in the way of the one at work (5 x 230 tokens: 1299 us with early launches, 1264 without; 8 tokens: 6894 us
+// for twelve generation steps without, 6778 with).
+constexpr int EARLY_TOKENS = 512;
+
 template <typename TA, typename TB, typename TC>
 int gemm_nt(cudaStream_t st, const TA* A, long long lda, long long sa, const TB* B, long long ldb, long long sb, TC* C, long long ldc,
             long long sc, int M, int N, int K, int batch, float alpha, int accumulate = 0, int outer = 1, long long sa2 = 0, long long sb2 = 0,
@@ -249,7 +254,7 @@ int head_gemm(cudaStream_t st, const TA* A, long long lda, long long sa, const T
     const bool aligned = lda % AE == 0 && sa % AE == 0 && ldb % 8 == 0 && sb % 8 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)B % 16 == 0;
     if (tensor_cores && K % 16 == 0 && aligned) {
       dim3 grid(ceil_div(N, 64), ceil_div(M, 64), batch);
-      B200_LAUNCH((gemm_nt_mma_kernel<TA, TC>), grid, 128, 0, st, A, lda, sa, B, ldb, sb, C, ldc, sc, M, N, K, alpha, gate, ldg, sg);
+      EARLY_LAUNCH((gemm_nt_mma_kernel<TA, TC>), grid, 128, 0, st, A, lda, sa, B, ldb, sb, C, ldc, sc, M, N, K, alpha, gate, ldg, sg);
       return check_launch("gemm_nt_mma");
     }
   }
@@ -280,6 +285,7 @@ int linear<bf16>(b200_dlm* h, const bf16* x, long long ldx, const Weight& w, bf1
   }
   if (w.tiles && ldx % 8 == 0 && ldy % 8 == 0) {
     tc::SkTuning t;
+    t.pdl = 1;
     for (int m0 = 0; m0 < M; m0 += 256) {          // the LM's GEMM takes up to 256 rows per launch
       const int m = std::min(256, M - m0);
       B200_TRY(tc::sk_linear(h->plans, x + (long long)m0 * ldx, ldx, w.tiles, y + (long long)m0 * ldy, ldy, nullptr, 0, m, w.N, w.K, 0, 0,
@@ -339,7 +345,7 @@ int launch_attn_mma(cudaStream_t st, const AttnParams& p, int tiles) {
     B200_CUDA(cudaFuncSetAttribute(latent_attn_mma_kernel<NKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     attr_set = true;
   }
-  B200_LAUNCH(latent_attn_mma_kernel<NKS>, dim3(tiles, p.nsplit), 128, smem, st, p);
+  EARLY_LAUNCH(latent_attn_mma_kernel<NKS>, dim3(tiles, p.nsplit), 128, smem, st, p);
   return check_launch("latent_attn_mma");
 }
 
@@ -369,7 +375,7 @@ int run_attention(cudaStream_t st, AttnParams p, int tiles, int rpt, bool tensor
   else if (r <= 576) B200_TRY((launch_attn<T, 18, 4>(st, p, tiles, p.nsplit)));
   else B200_TRY((launch_attn<T, 32, 2>(st, p, tiles, p.nsplit)));
   if (p.nsplit > 1) {
-    B200_LAUNCH(latent_attn_merge_kernel, dim3(tiles, rpt), 128, 0, st, p.part, p.tile_row0, p.tile_rows, p.out, r, p.nsplit, rpt, p.gate, p.ldg, p.H);
+    EARLY_LAUNCH(latent_attn_merge_kernel, dim3(tiles, rpt), 128, 0, st, p.part, p.tile_row0, p.tile_rows, p.out, r, p.nsplit, rpt, p.gate, p.ldg, p.H);
     B200_TRY(check_launch("latent_attn_merge"));
   }
   return B200_OK;
@@ -406,7 +412,7 @@ int mark(b200_dlm* h, int cls) {       // cls >= 0 opens an interval of that cla
 int finish_logits(b200_dlm* h, const bf16* in_bf, long long ld, int n_want, int mode, float c, float* logits_out) {
   const long long n = (long long)n_want * h->cfg.vocab;
   const int vec = h->cfg.vocab % 8 == 0 && ((uintptr_t)logits_out & 15) == 0;
-  B200_LAUNCH(logit_rows_kernel, (unsigned)ceil_div64(n, vec ? 2048 : 256), 256, 0, h->stream, in_bf, ld, h->logits, logits_out, h->cfg.vocab, n, mode, c, vec);
+  EARLY_LAUNCH(logit_rows_kernel, (unsigned)ceil_div64(n, vec ? 2048 : 256), 256, 0, h->stream, in_bf, ld, h->logits, logits_out, h->cfg.vocab, n, mode, c, vec);
   return check_launch("logits");
 }
 
@@ -446,10 +452,10 @@ int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out
   cudaStream_t st = h->stream;
   const int* meta = h->meta_dev;
   const long long stride = (long long)h->tmax * W;
-  TIMED(CLS_ELEMENTWISE, B200_LAUNCH(embed_kernel<T>, n_tok, 256, 0, st, meta + h->off_tok, static_cast<const T*>(h->embed), c.vocab, W, c.embedding_scale,
+  TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(embed_kernel<T>, n_tok, 256, 0, st, meta + h->off_tok, static_cast<const T*>(h->embed), c.vocab, W, c.embedding_scale,
               h->xin, h->stack, h->err));
   T* hb = static_cast<T*>(h->hbuf);
-  TIMED(CLS_ELEMENTWISE, B200_LAUNCH(layernorm_kernel<T>, n_tok, 256, 0, st, h->xin, (const int*)nullptr, h->layers[0].n1w, h->layers[0].n1b, hb, W, c.norm_eps));
+  TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(layernorm_kernel<T>, n_tok, 256, 0, st, h->xin, (const int*)nullptr, h->layers[0].n1w, h->layers[0].n1b, hb, W, c.norm_eps));
   for (int li = 0; li < c.n_layers; ++li) {
     const Layer& L = h->layers[li];
     const int H = L.c.a.heads, dk = L.c.a.dim, dv = L.c.a.vdim, r = L.c.a.kv_rank;
@@ -458,7 +464,7 @@ int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out
     bool squared = false;                // the feed-forward's unit is done by the projection's epilogue
     TIMED(CLS_LINEAR, B200_TRY(projection_with_unit<T>(h, L, hb, proj, act, n_tok, &squared)));
     // mixer: latent attention
-    TIMED(CLS_ELEMENTWISE, B200_LAUNCH(latent_append_kernel<T>, ceil_div(n_tok, 4), 128, 0, st, proj, (long long)L.ldp, L.off_dkv, L.cnorm, static_cast<T*>(L.cache),
+    TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(latent_append_kernel<T>, ceil_div(n_tok, 4), 128, 0, st, proj, (long long)L.ldp, L.off_dkv, L.cnorm, static_cast<T*>(L.cache),
                 h->cap, r, meta + h->off_slot, meta + h->off_pos, n_tok, c.norm_eps));
     T* ob = static_cast<T*>(h->obuf);
     if (expands_latents(h, L, max_ctx)) {
@@ -478,19 +484,19 @@ int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out
     T* ffo = nullptr;
     if (L.c.mlp == B200_MLP_DENSE_RELU2) {
       const long long n = (long long)n_tok * L.c.ff;
-      if (!squared) TIMED(CLS_ELEMENTWISE, B200_LAUNCH(relu2_kernel<T>, (unsigned)ceil_div64(n, 256), 256, 0, st, proj, (long long)L.ldp, L.off_up, act, L.c.ff, n));
+      if (!squared) TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(relu2_kernel<T>, (unsigned)ceil_div64(n, 256), 256, 0, st, proj, (long long)L.ldp, L.off_up, act, L.c.ff, n));
       ffo = static_cast<T*>(h->ffo);
       TIMED(CLS_LINEAR, B200_TRY(linear<T>(h, act, L.c.ff, L.down, ffo, W, n_tok)));
     }
     const bool last = li + 1 == c.n_layers;
-    TIMED(CLS_ELEMENTWISE, B200_LAUNCH(block_end_kernel<T>, n_tok, 256, 0, st, h->xin, mixo, ffo, proj, (long long)L.ldp, L.off_g1, L.off_g2, L.b1, L.b2, c.residual_mult,
+    TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(block_end_kernel<T>, n_tok, 256, 0, st, h->xin, mixo, ffo, proj, (long long)L.ldp, L.off_g1, L.off_g2, L.b1, L.b2, c.residual_mult,
                 h->stack, stride, li, L.avg, h->trace_layers ? h->trace + (long long)li * stride : nullptr,
                 last ? nullptr : h->layers[li + 1].n1w, last ? nullptr : h->layers[li + 1].n1b, hb, W, c.norm_eps));
   }
   B200_TRY(check_launch("decoder LM layers"));
   if (n_want > 0) {
     T* hf = static_cast<T*>(h->hf);
-    TIMED(CLS_ELEMENTWISE, B200_LAUNCH(layernorm_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, h->fnb, hf, W, c.norm_eps));
+    TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(layernorm_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, h->fnb, hf, W, c.norm_eps));
     if (h->head.tiles) {
       const int ldl = (c.vocab + 7) / 8 * 8;
       TIMED(CLS_LINEAR, B200_TRY(linear<bf16>(h, reinterpret_cast<const bf16*>(hf), W, h->head, h->head_bf, ldl, n_want)));
@@ -725,7 +731,7 @@ int small_proj(b200_dlm* h, const T* x, long long ldx, const void* w, const floa
   const int vec = K % 8 == 0 && (ldx * sizeof(T)) % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
   const size_t row = (size_t)K * sizeof(T);
   if (M >= 512 && 8 * row <= 100 * 1024) B200_LAUNCH((small_proj_f32_kernel<T, 8>), dim3(ceil_div(M, 8), ceil_div(N, 32)), 256, 8 * row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
-  else B200_LAUNCH((small_proj_f32_kernel<T, 1>), dim3(M, M >= 512 ? 1 : ceil_div(N, 8)), 256, row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
+  else EARLY_LAUNCH_IF(M < EARLY_TOKENS, (small_proj_f32_kernel<T, 1>), dim3(M, M >= 512 ? 1 : ceil_div(N, 8)), 256, row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
   return check_launch("small_proj_f32");
 }
 
@@ -890,7 +896,7 @@ int window_attention(b200_dlm* h, const Layer& L, int n_tok, int max_ctx, long l
   B200_TRY(check_launch("window_attn"));
   if (nsplit > 1) {
     float* merged = h->f32 ? static_cast<float*>(h->obuf) : h->attn32;
-    B200_LAUNCH(latent_attn_merge_kernel, dim3(s.count, rpt), 128, 0, h->stream, h->part, p.tile_row0, p.tile_rows, merged, a.vdim, nsplit, rpt);
+    EARLY_LAUNCH(latent_attn_merge_kernel, dim3(s.count, rpt), 128, 0, h->stream, h->part, p.tile_row0, p.tile_rows, merged, a.vdim, nsplit, rpt, (const float*)nullptr, 0, 1);
     B200_TRY(check_launch("window_attn merge"));
     if (!h->f32) {
       const long long n = (long long)n_tok * a.heads * a.vdim;
@@ -906,7 +912,7 @@ int window_attention(b200_dlm* h, const Layer& L, int n_tok, int max_ctx, long l
 // neighbours; act: the first product's epilogue (WIDE_*), its result has F columns
 int grouped_products(b200_dlm* h, const Layer& L, const bf16* hb, int n_tok, int N1, int act, float limit) {
   const int W = h->cfg.width, F = L.c.ff, pairs = n_tok * L.c.top, E = L.c.experts;
-  B200_LAUNCH(moe_gather_kernel, pairs, 128, 0, h->stream, reinterpret_cast<const uint4*>(hb), h->moe_row_tok, h->moe_ntiles + 1, reinterpret_cast<uint4*>(h->moe_x), W / 8);
+  EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, moe_gather_kernel, pairs, 128, 0, h->stream, reinterpret_cast<const uint4*>(hb), h->moe_row_tok, h->moe_ntiles + 1, reinterpret_cast<uint4*>(h->moe_x), W / 8);
   tc::WideGemm g;
   g.tile_e = h->moe_tile_e; g.tile_r0 = h->moe_tile_r0; g.tile_n = h->moe_tile_n; g.n_tiles = h->moe_ntiles;
   g.max_tiles = ceil_div(pairs, tc::WIDE_EXPERT_ROWS) + std::min(E, pairs);
@@ -926,11 +932,11 @@ int routed_experts(b200_dlm* h, const Layer& L, const T* hb, int n_tok) {
   const int W = h->cfg.width, E = L.c.experts, top = L.c.top, F = L.c.ff, pairs = n_tok * top;
   cudaStream_t st = h->stream;
   B200_TRY(small_proj<T>(h, hb, W, L.router, nullptr, h->route32, n_tok, E, W));
-  B200_LAUNCH(moe_route_kernel, ceil_div(n_tok, 4), 128, 0, st, h->route32, E, top, h->moe_idx, h->moe_w, n_tok);
+  EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, moe_route_kernel, ceil_div(n_tok, 4), 128, 0, st, h->route32, E, top, h->moe_idx, h->moe_w, n_tok);
   bool mma = false;
   if constexpr (sizeof(T) == 2) mma = h->attn_tc && W % 16 == 0 && F % 16 == 0;
   const int tile_m = mma ? tc::WIDE_EXPERT_ROWS : 64;
-  B200_LAUNCH(moe_group_kernel, 1, 1024, (size_t)2 * E * sizeof(int), st, h->moe_idx, pairs, top, E, h->moe_rank, h->moe_perm, h->moe_row_tok,
+  EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, moe_group_kernel, 1, 1024, (size_t)2 * E * sizeof(int), st, h->moe_idx, pairs, top, E, h->moe_rank, h->moe_perm, h->moe_row_tok,
               h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, tile_m);
   B200_TRY(check_launch("moe route / group"));
   const int max_tiles = ceil_div(pairs, tile_m) + std::min(E, pairs);
@@ -1036,7 +1042,7 @@ int step_sandwich(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits
   B200_TRY(check_launch("decoder LM layers"));
   if (n_want > 0) {
     T* hf = static_cast<T*>(h->hf);
-    TIMED(CLS_ELEMENTWISE, B200_LAUNCH(rmsnorm_rows_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, hf, W, c.norm_eps));
+    TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(rmsnorm_rows_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, hf, W, c.norm_eps));
     if (h->head.tiles) {
       const int ldl = (c.vocab + 7) / 8 * 8;
       TIMED(CLS_LINEAR, B200_TRY(linear<bf16>(h, reinterpret_cast<const bf16*>(hf), W, h->head, h->head_bf, ldl, n_want)));
@@ -1677,7 +1683,7 @@ int launch_map_mma(cudaStream_t st, const MapAttnParams& p, size_t smem) {
     B200_CUDA(cudaFuncSetAttribute((map_attn_mma_kernel<NM, VT, SK>), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     attr_set = true;
   }
-  B200_LAUNCH((map_attn_mma_kernel<NM, VT, SK>), dim3(p.n_tiles * p.G, p.nsplit), 128, smem, st, p);
+  EARLY_LAUNCH_IF(SK, (map_attn_mma_kernel<NM, VT, SK>), dim3(p.n_tiles * p.G, p.nsplit), 128, smem, st, p);
   return check_launch("map_attn_mma");
 }
 
@@ -1715,7 +1721,7 @@ int map_attention(b200_dlm* h, const Layer& L, int n_tok, int max_ctx) {
     p.head_rows = n_tok >= 512 ? 1 : ceil_div(p.Hm + (own ? p.Gm : 0), 8);      // few tokens: one (head, map) per warp
     const dim3 grid(n_tok, p.head_rows + ceil_div(L.glu_ff, GLU_SLICE));
     const size_t smem = (size_t)8 * a.dim * sizeof(float);
-    TIMED(CLS_ELEMENTWISE, if (mma) B200_LAUNCH((head_prep_kernel<T, bf16>), grid, 256, smem, st, p); else B200_LAUNCH((head_prep_kernel<T, float>), grid, 256, smem, st, p));
+    TIMED(CLS_ELEMENTWISE, if (mma) EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, (head_prep_kernel<T, bf16>), grid, 256, smem, st, p); else EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, (head_prep_kernel<T, float>), grid, 256, smem, st, p));
     B200_TRY(check_launch("head_prep"));
   }
   const bool one = mma && h->max_entry_tokens * rep <= 16;
@@ -1750,7 +1756,7 @@ int map_attention(b200_dlm* h, const Layer& L, int n_tok, int max_ctx) {
     B200_TRY(check_launch("map_attn"));
   }
   if (nsplit > 1) {
-    B200_LAUNCH((map_attn_merge_kernel<T, NM>), dim3(ctas, ceil_div(s.rpt, 4)), 128, 0, st, p);
+    EARLY_LAUNCH((map_attn_merge_kernel<T, NM>), dim3(ctas, ceil_div(s.rpt, 4)), 128, 0, st, p);
     B200_TRY(check_launch("map_attn_merge"));
   }
   return mark(h, -1);
@@ -1875,16 +1881,16 @@ int routed_experts_glu(b200_dlm* h, const Layer& L, const T* hb, int n_tok) {
       B200_CUDA(cudaFuncSetAttribute(moe_route_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       attr_set = true;
     }
-    B200_LAUNCH(moe_route_grouped_kernel, ceil_div(n_tok, 4), 128, smem, st, h->small32 + L.s_router, (long long)L.nsmall, L.correction, n, top, groups, L.c.groups_keep,
+    EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, moe_route_grouped_kernel, ceil_div(n_tok, 4), 128, smem, st, h->small32 + L.s_router, (long long)L.nsmall, L.correction, n, top, groups, L.c.groups_keep,
                 gelu ? 1 : 0, gelu ? 2 : 1, gelu ? 1 : 0, L.c.router_scale, h->moe_idx, h->moe_w, n_tok);
   } else {
-    B200_LAUNCH(moe_route_sigmoid_kernel, ceil_div(n_tok, 4), 128, 0, st, h->small32 + L.s_router, (long long)L.nsmall, L.correction, E, top, L.c.router_scale,
+    EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, moe_route_sigmoid_kernel, ceil_div(n_tok, 4), 128, 0, st, h->small32 + L.s_router, (long long)L.nsmall, L.correction, E, top, L.c.router_scale,
                 h->moe_idx, h->moe_w, n_tok);
   }
   bool mma = false;
   if constexpr (sizeof(T) == 2) mma = h->attn_tc && W % 16 == 0 && F % 16 == 0;
   const int tile_m = mma ? tc::WIDE_EXPERT_ROWS : 64;
-  B200_LAUNCH(moe_group_kernel, 1, 1024, (size_t)2 * E * sizeof(int), st, h->moe_idx, pairs, top, E, h->moe_rank, h->moe_perm, h->moe_row_tok,
+  EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, moe_group_kernel, 1, 1024, (size_t)2 * E * sizeof(int), st, h->moe_idx, pairs, top, E, h->moe_rank, h->moe_perm, h->moe_row_tok,
               h->moe_tile_e, h->moe_tile_r0, h->moe_tile_n, h->moe_ntiles, tile_m);
   B200_TRY(check_launch("moe route / group"));
   const int max_tiles = ceil_div(pairs, tile_m) + std::min(E, pairs);
@@ -1980,10 +1986,10 @@ int step_parallel(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits
   T* proj = static_cast<T*>(h->proj);
   T* ob = static_cast<T*>(h->obuf);
   T* mixo = static_cast<T*>(h->mixo);
-  TIMED(CLS_ELEMENTWISE, B200_LAUNCH(embed_scale_norm_kernel<T>, n_tok, 256, 0, st, meta + h->off_tok, static_cast<const T*>(h->embed), c.vocab, W, c.embedding_scale,
+  TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(embed_scale_norm_kernel<T>, n_tok, 256, 0, st, meta + h->off_tok, static_cast<const T*>(h->embed), c.vocab, W, c.embedding_scale,
                                      h->layers[0].n1w, h->xin, hb, c.norm_eps, h->err, c.norm == B200_NORM_LAYER, h->layers[0].step));
   for (const auto& r : h->rots)
-    TIMED(CLS_ELEMENTWISE, B200_LAUNCH(rotary_table_kernel, n_tok, 64, 0, st, tok_pos, r.freq, r.m.rot_dims / 2, r.amp, r.table));
+    TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(rotary_table_kernel, n_tok, 64, 0, st, tok_pos, r.freq, r.m.rot_dims / 2, r.amp, r.table));
   const int n_runs = (int)h->layers.size();
   for (int li = 0; li < n_runs; ++li) {
     const Layer& L = h->layers[li];
@@ -2052,7 +2058,7 @@ int step_parallel(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits
     auto block_end = parallel_block_end_kernel<T>;
     float* trace = h->trace_layers ? h->trace + (long long)li * stride : nullptr;
     const float *step = last ? nullptr : h->layers[li + 1].step, *w_next = last ? nullptr : h->layers[li + 1].n1w;
-    TIMED(CLS_ELEMENTWISE, B200_LAUNCH(block_end, n_tok, 256, 0, st, h->xin, mixo, ffo, yexp, h->moe_w, L.c.top, side ? nullptr : trace, side ? nullptr : w_next, hb, W, c.norm_eps,
+    TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, block_end, n_tok, 256, 0, st, h->xin, mixo, ffo, yexp, h->moe_w, L.c.top, side ? nullptr : trace, side ? nullptr : w_next, hb, W, c.norm_eps,
                                        c.norm == B200_NORM_LAYER,
                                        L.c.identity > 0 ? h->moe_idx : (const int*)nullptr, L.c.experts, side ? nullptr : step));
     if (side) B200_TRY(token_input<T>(h, L, n_tok, trace, step, w_next));
@@ -2060,8 +2066,8 @@ int step_parallel(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits
   B200_TRY(check_launch("decoder LM layers"));
   if (n_want > 0) {
     T* hf = static_cast<T*>(h->hf);
-    TIMED(CLS_ELEMENTWISE, if (c.norm == B200_NORM_LAYER) B200_LAUNCH(layernorm_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, (const float*)nullptr, hf, W, c.norm_eps);
-          else B200_LAUNCH(rmsnorm_rows_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, hf, W, c.norm_eps));
+    TIMED(CLS_ELEMENTWISE, if (c.norm == B200_NORM_LAYER) EARLY_LAUNCH(layernorm_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, (const float*)nullptr, hf, W, c.norm_eps);
+          else EARLY_LAUNCH(rmsnorm_rows_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, hf, W, c.norm_eps));
     if (h->head.tiles) {
       const int ldl = (c.vocab + 7) / 8 * 8;
       TIMED(CLS_LINEAR, B200_TRY(linear<bf16>(h, reinterpret_cast<const bf16*>(hf), W, h->head, h->head_bf, ldl, n_want)));
@@ -2371,7 +2377,7 @@ int step_streams(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_
       T* upb = static_cast<T*>(h->act2);
       TIMED(CLS_LINEAR, B200_TRY(linear<T>(h, hb, W, L.up, upb, L.c.ff, n_tok)));
       const long long n = (long long)n_tok * L.c.ff;
-      TIMED(CLS_ELEMENTWISE, B200_LAUNCH(relu2_kernel<T>, (unsigned)ceil_div64(n, 256), 256, 0, st, upb, (long long)L.c.ff, 0, act, L.c.ff, n));
+      TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(relu2_kernel<T>, (unsigned)ceil_div64(n, 256), 256, 0, st, upb, (long long)L.c.ff, 0, act, L.c.ff, n));
       T* ffo = static_cast<T*>(h->ffo);
       TIMED(CLS_LINEAR, B200_TRY(linear<T>(h, act, L.c.ff, L.down, ffo, W, n_tok)));
       TIMED(CLS_ELEMENTWISE, B200_TRY(streams_end<T>(h, ffo, 1.f, (const T*)nullptr, 0.f, L.hc_mix[1], L.hc_out[1], trace, last ? h->xin : nullptr, nx ? nx->hc_in[0] : nullptr,
@@ -2384,7 +2390,7 @@ int step_streams(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_
   B200_TRY(check_launch("decoder LM layers"));
   if (n_want > 0) {
     T* hf = static_cast<T*>(h->hf);
-    TIMED(CLS_ELEMENTWISE, B200_LAUNCH(rmsnorm_rows_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, hf, W, c.norm_eps));
+    TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(rmsnorm_rows_kernel<T>, n_want, 256, 0, st, h->xin, meta + h->off_want, h->fnw, hf, W, c.norm_eps));
     if (h->head.tiles) {
       const int ldl = (c.vocab + 7) / 8 * 8;
       TIMED(CLS_LINEAR, B200_TRY(linear<bf16>(h, reinterpret_cast<const bf16*>(hf), W, h->head, h->head_bf, ldl, n_want)));

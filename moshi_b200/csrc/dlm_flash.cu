@@ -102,6 +102,8 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<const uint32_t*>(smem_raw + (tptr - raw));
   const uint32_t tmem_o = tmem + 256;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -307,7 +309,15 @@ int flash_attention(const FlashAttn& a, cudaStream_t st) {
   }
   FlashP p;
   p.sink = a.sink; p.out = a.out; p.ldo = a.ldo; p.T = a.T; p.pos0 = a.pos0; p.H = a.H; p.q_tiles = ceil_div(a.T, ROWS); p.scale2 = a.scale * LOG2E; p.err = a.err;
-  flash_attention_kernel<<<p.q_tiles * a.H, THREADS, SMEM, st>>>(mq, mk, mv, p);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(p.q_tiles * a.H)); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = SMEM; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, flash_attention_kernel, mq, mk, mv, p);
+  if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "flash_attention launch failed: %s", cudaGetErrorString(e));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return check_launch("flash_attention");
 }

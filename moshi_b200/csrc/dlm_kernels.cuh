@@ -107,8 +107,10 @@ __device__ __forceinline__ void block_layernorm(const float* __restrict__ x, con
 
 // x = table[token] * scale -> the layer-input stream and slot 0 of the per-layer result stack
 template <typename T>
-__global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ tokens, const T* __restrict__ table, int vocab, int W, float scale,
-                                                    float* __restrict__ xin, float* __restrict__ x0, int* __restrict__ err) {
+__global__ void __launch_bounds__(256) embed_kernel(const int* tokens, const T* __restrict__ table, int vocab, int W, float scale,
+                                                    float* xin, float* x0, int* err) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   const int t = blockIdx.x;
   int id = tokens[t];
   if (id < 0 || id >= vocab) {
@@ -125,8 +127,10 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
 
 // h[row] = layernorm(x[rows ? rows[row] : row])
 template <typename T>
-__global__ void __launch_bounds__(256) layernorm_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w,
-                                                        const float* __restrict__ b, T* __restrict__ out, int W, float eps) {
+__global__ void __launch_bounds__(256) layernorm_kernel(const float* x, const int* rows, const float* __restrict__ w,
+                                                        const float* __restrict__ b, T* out, int W, float eps) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   __shared__ float red[32];
   const int src = rows ? rows[blockIdx.x] : blockIdx.x;
   if (W % 8 == 0 && W <= ROW_VEC) {
@@ -145,13 +149,15 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const float* __restrict_
 //   x    <- sum_{j <= li + 1} avg[j] * stack[j]            (what the next layer, or the output norm, reads)
 //   h    <- layernorm(x) with the NEXT layer's norm (when given)
 template <typename T>
-__global__ void __launch_bounds__(256) block_end_kernel(float* __restrict__ xin, const T* __restrict__ mix, const T* __restrict__ ff,
-                                                        const T* __restrict__ proj, long long ldp, int off_g1, int off_g2,
+__global__ void __launch_bounds__(256) block_end_kernel(float* xin, const T* mix, const T* ff,
+                                                        const T* proj, long long ldp, int off_g1, int off_g2,
                                                         const float* __restrict__ b1, const float* __restrict__ b2, float mult,
-                                                        float* __restrict__ stack, long long stack_stride, int li,
-                                                        const float* __restrict__ avg, float* __restrict__ trace,
-                                                        const float* __restrict__ nw, const float* __restrict__ nb, T* __restrict__ h,
+                                                        float* stack, long long stack_stride, int li,
+                                                        const float* __restrict__ avg, float* trace,
+                                                        const float* __restrict__ nw, const float* __restrict__ nb, T* h,
                                                         int W, float eps) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   __shared__ float red[32];
   const long long t = blockIdx.x;
   float* x = xin + t * W;
@@ -214,9 +220,11 @@ __global__ void __launch_bounds__(256) block_end_kernel(float* __restrict__ xin,
 
 // latent of the new tokens: c = raw / sqrt(mean(raw^2) + eps) * w, appended to the slot's cache rows; one warp per token
 template <typename T>
-__global__ void __launch_bounds__(128) latent_append_kernel(const T* __restrict__ proj, long long ldp, int off, const float* __restrict__ w,
-                                                            T* __restrict__ cache, int cap, int r, const int* __restrict__ tok_slot,
-                                                            const int* __restrict__ tok_pos, int n_tok, float eps) {
+__global__ void __launch_bounds__(128) latent_append_kernel(const T* proj, long long ldp, int off, const float* __restrict__ w,
+                                                            T* cache, int cap, int r, const int* tok_slot,
+                                                            const int* tok_pos, int n_tok, float eps) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5), l = threadIdx.x & 31;
   if (t >= n_tok) return;
   const T* raw = proj + (long long)t * ldp + off;
@@ -229,7 +237,9 @@ __global__ void __launch_bounds__(128) latent_append_kernel(const T* __restrict_
 
 // out = relu(x)^2
 template <typename T>
-__global__ void __launch_bounds__(256) relu2_kernel(const T* __restrict__ proj, long long ldp, int off, T* __restrict__ out, int F, long long n) {
+__global__ void __launch_bounds__(256) relu2_kernel(const T* proj, long long ldp, int off, T* out, int F, long long n) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   const long long t = i / F; const int f = (int)(i - t * F);
@@ -533,6 +543,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
 
 template <int NKS>      // 16-element steps of a warp's share of the latent: r = 64 * NKS
 __global__ void __launch_bounds__(128, 3) latent_attn_mma_kernel(AttnParams p) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   // r = 512: 75 KB per CTA, three CTAs per SM.  Keys arrive by bulk copies (one per key, issued by the lanes of warp 0) that
   // complete on an mbarrier per buffer, so no thread spends instructions on staging.  A row of partial scores is 32 floats; its 8-float blocks are permuted by the
   // row (block ^ (row & 3)) so that neither the stores nor the loads meet in a bank.
@@ -714,10 +726,12 @@ __global__ void __launch_bounds__(128, 3) latent_attn_mma_kernel(AttnParams p) {
 // merges the splits of one row: out = sum_s o_s exp(m_s - M) / sum_s l_s exp(m_s - M); one CTA per row, grid (tiles, rows).
 // Every warp computes the split weights (lane s owns splits s and s + 32); then a thread owns element pairs of the row and
 // sums them over the splits with independent 8-byte loads (scalar loads when the latent size is odd).
-__global__ void __launch_bounds__(128) latent_attn_merge_kernel(const float* __restrict__ part, const int* __restrict__ tile_row0,
-                                                                const int* __restrict__ tile_rows, float* __restrict__ out, int r,
-                                                                int nsplit, int rows_per_tile, const float* __restrict__ gate = nullptr,
+__global__ void __launch_bounds__(128) latent_attn_merge_kernel(const float* part, const int* tile_row0,
+                                                                const int* tile_rows, float* out, int r,
+                                                                int nsplit, int rows_per_tile, const float* gate = nullptr,
                                                                 int ldg = 0, int H = 1) {      // gate: row (token, head) times sigmoid(gate[token * ldg + head])
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   __shared__ float wsm[64];
   const int tile = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lr = blockIdx.y;
@@ -768,10 +782,12 @@ __global__ void __launch_bounds__(128) latent_attn_merge_kernel(const float* __r
 // memory), B bf16, C fp32 or bf16.  K a multiple of 16; M and N are free (zero-filled edges).  CTA tile 64 x 64, 4 warps of
 // 16 rows x 64 columns, 32-element k-steps through shared memory.  gate: as in gemm_nt_kernel.
 template <typename TA, typename TC>
-__global__ void __launch_bounds__(128) gemm_nt_mma_kernel(const TA* __restrict__ A, long long lda, long long sa, const bf16* __restrict__ B,
-                                                          long long ldb, long long sb, TC* __restrict__ C, long long ldc, long long sc,
-                                                          int M, int N, int K, float alpha, const TC* __restrict__ gate = nullptr,
+__global__ void __launch_bounds__(128) gemm_nt_mma_kernel(const TA* A, long long lda, long long sa, const bf16* __restrict__ B,
+                                                          long long ldb, long long sb, TC* C, long long ldc, long long sc,
+                                                          int M, int N, int K, float alpha, const TC* gate = nullptr,
                                                           long long ldg = 0, long long sg = 0) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   constexpr int BM = 64, BN = 64, BK = 32, ST = BK + 8;
   __shared__ __align__(16) bf16 As[BM][ST];
   __shared__ __align__(16) bf16 Bs[BN][ST];
@@ -852,8 +868,10 @@ __global__ void __launch_bounds__(128) gemm_nt_mma_kernel(const TA* __restrict__
 // cap * tanh(. / cap) or times a factor.  Runs of eight (vec) move at HBM's rate: 1000 rows of 32000 took 94 us element by element and 43 us
 // more for the copy to the caller's buffer, both together now 56.
 enum { LOGITS_PLAIN = 0, LOGITS_SOFTCAP = 1, LOGITS_SCALE = 2 };
-__global__ void __launch_bounds__(256) logit_rows_kernel(const bf16* __restrict__ in_bf, long long ld, float* out, float* out2, int V, long long n, int mode,
+__global__ void __launch_bounds__(256) logit_rows_kernel(const bf16* in_bf, long long ld, float* out, float* out2, int V, long long n, int mode,
                                                          float c, int vec) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * (vec ? 8 : 1);
   if (i >= n) return;
   const long long row = i / V;

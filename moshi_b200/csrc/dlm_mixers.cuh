@@ -45,8 +45,10 @@ __global__ void __launch_bounds__(256) embed_norm_kernel(const int* __restrict__
 
 // out[row] = rms_norm(x[rows ? rows[row] : row]) * w
 template <typename T>
-__global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w,
-                                                           T* __restrict__ out, int W, float eps) {
+__global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* x, const int* rows, const float* __restrict__ w,
+                                                           T* out, int W, float eps) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   __shared__ float red[32];
   const long long src = rows ? rows[blockIdx.x] : blockIdx.x;
   const float* xr = x + src * W;
@@ -535,8 +537,10 @@ __global__ void rows_from_f32_kernel(const float* __restrict__ in, T* __restrict
 // adds runs of eight elements (single elements where rows do not start on 16 bytes), then the lanes meet.
 // ---------------------------------------------------------------------------------------------------------------------------
 template <typename T, int TOK>
-__global__ void __launch_bounds__(256) small_proj_f32_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ w, const float* __restrict__ b,
-                                                             float* __restrict__ out, int M, int N, int K, int vec) {
+__global__ void __launch_bounds__(256) small_proj_f32_kernel(const T* x, long long ldx, const T* __restrict__ w, const float* __restrict__ b,
+                                                             float* out, int M, int N, int K, int vec) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   extern __shared__ __align__(16) unsigned char sp_smem[];
   T* xs = reinterpret_cast<T*>(sp_smem);                 // [TOK][K]
   const long long t0 = (long long)blockIdx.x * TOK;
@@ -1069,8 +1073,10 @@ __global__ void __launch_bounds__(256) sublayer_end_kernel(float* __restrict__ x
 // differ from run to run; a row's result does not depend on it (every row of a product is summed on its own).  Choices from E
 // on stand for no feed-forward and get no row.
 // ---------------------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict__ logits, int E, int top, int* __restrict__ idx,
-                                                        float* __restrict__ wts, int n_tok) {
+__global__ void __launch_bounds__(128) moe_route_kernel(const float* logits, int E, int top, int* idx,
+                                                        float* wts, int n_tok) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= n_tok) return;
   const float* z = logits + (long long)t * E;
@@ -1098,9 +1104,11 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
   if (lane < top) wts[(long long)t * top + lane] /= den;
 }
 
-__global__ void __launch_bounds__(1024) moe_group_kernel(const int* __restrict__ idx, int n_pairs, int top, int E, int* __restrict__ rank,
-                                                         int* __restrict__ perm, int* __restrict__ row_tok, int* __restrict__ tile_expert,
-                                                         int* __restrict__ tile_row0, int* __restrict__ tile_rows, int* __restrict__ n_tiles, int tile_m) {
+__global__ void __launch_bounds__(1024) moe_group_kernel(const int* idx, int n_pairs, int top, int E, int* rank,
+                                                         int* perm, int* row_tok, int* tile_expert,
+                                                         int* tile_row0, int* tile_rows, int* n_tiles, int tile_m) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   extern __shared__ int cnt[];          // [E] counts, then [E] offsets
   int* off = cnt + E;
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
@@ -1127,8 +1135,10 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int* __restrict__
 }
 
 // the grouped order's rows side by side: out[pos] = x[row_tok[pos]], row16 16-byte pieces per row
-__global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ row_tok, const int* __restrict__ n_rows,
-                                                         uint4* __restrict__ out, int row16) {
+__global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* x, const int* row_tok, const int* n_rows,
+                                                         uint4* out, int row16) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   if ((int)blockIdx.x >= n_rows[0]) return;
   const uint4* src = x + (long long)row_tok[blockIdx.x] * row16;
   uint4* dst = out + (long long)blockIdx.x * row16;

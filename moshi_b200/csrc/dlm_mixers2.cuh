@@ -31,9 +31,11 @@ __device__ __forceinline__ void block_norm(const float* __restrict__ x, const fl
 
 // x = table[token] * scale (+ step: the vector in front of a pass) -> residual stream (fp32);  h = norm(x) * w1 -> T
 template <typename T>
-__global__ void __launch_bounds__(256) embed_scale_norm_kernel(const int* __restrict__ tokens, const T* __restrict__ table, int vocab, int W, float scale,
-                                                               const float* __restrict__ w1, float* __restrict__ xin, T* __restrict__ h, float eps,
-                                                               int* __restrict__ err, int layer, const float* __restrict__ step = nullptr) {
+__global__ void __launch_bounds__(256) embed_scale_norm_kernel(const int* tokens, const T* __restrict__ table, int vocab, int W, float scale,
+                                                               const float* __restrict__ w1, float* xin, T* h, float eps,
+                                                               int* err, int layer, const float* step = nullptr) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   __shared__ float red[32];
   const long long t = blockIdx.x;
   int id = tokens[t];
@@ -67,11 +69,13 @@ __global__ void __launch_bounds__(256) embed_scale_norm_kernel(const int* __rest
 // (per-layer trace);  x <- x + step (the vector in front of a pass, when given);  optional h = norm(x) * w_next for the next layer.
 // Rows of up to ROW_VEC elements are held in registers in runs of eight.
 template <typename T>
-__global__ void __launch_bounds__(256) parallel_block_end_kernel(float* __restrict__ xin, const T* __restrict__ mix, const T* __restrict__ ff,
-                                                                 const T* __restrict__ yexp, const float* __restrict__ ew, int top,
-                                                                 float* __restrict__ trace, const float* __restrict__ w_next, T* h,
-                                                                 int W, float eps, int layer = 0, const int* __restrict__ choice = nullptr, int n_exp = 0,
-                                                                 const float* __restrict__ step = nullptr) {
+__global__ void __launch_bounds__(256) parallel_block_end_kernel(float* xin, const T* mix, const T* ff,
+                                                                 const T* yexp, const float* ew, int top,
+                                                                 float* trace, const float* __restrict__ w_next, T* h,
+                                                                 int W, float eps, int layer = 0, const int* choice = nullptr, int n_exp = 0,
+                                                                 const float* step = nullptr) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   __shared__ float red[32];
   const long long t = blockIdx.x;
   float* x = xin + t * W;
@@ -890,8 +894,10 @@ __global__ void __launch_bounds__(256) interleaved_glu_kernel(const T* __restric
 
 // Router with sigmoid scores, per token (one warp): s = sigmoid(logit); the `top` experts with the largest s + correction are
 // chosen (ties: the lower index); their weights are s / (sum of the chosen s + 1e-20) * out_scale.
-__global__ void __launch_bounds__(128) moe_route_sigmoid_kernel(const float* __restrict__ logits, long long ldl, const float* __restrict__ correction,
-                                                                int E, int top, float out_scale, int* __restrict__ idx, float* __restrict__ wts, int n_tok) {
+__global__ void __launch_bounds__(128) moe_route_sigmoid_kernel(const float* logits, long long ldl, const float* __restrict__ correction,
+                                                                int E, int top, float out_scale, int* idx, float* wts, int n_tok) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= n_tok) return;
   const float* z = logits + (long long)t * ldl;

@@ -16,8 +16,10 @@ namespace dlm {
 
 // cos and sin of pos * freq[i] (evaluated in double), times amp: rot[token] = [half] cosines, [half] sines.  One launch per step
 // serves every layer with this rotation.
-__global__ void __launch_bounds__(64) rotary_table_kernel(const int* __restrict__ tok_pos, const double* __restrict__ freq, int half, float amp,
-                                                          float* __restrict__ rot) {
+__global__ void __launch_bounds__(64) rotary_table_kernel(const int* tok_pos, const double* __restrict__ freq, int half, float amp,
+                                                          float* rot) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   rotary_fill(rot + (long long)blockIdx.x * 2 * half, half, tok_pos[blockIdx.x], freq, amp);
 }
 
@@ -81,6 +83,8 @@ struct HeadPrepParams {
 
 template <typename T, typename TQ>
 __global__ void __launch_bounds__(256) head_prep_kernel(HeadPrepParams p) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   extern __shared__ float prep_buf[];   // [8 warps][dim]
   const long long t = blockIdx.x;
   const T* row = static_cast<const T*>(p.proj) + t * p.ld;
@@ -282,6 +286,8 @@ __global__ void __launch_bounds__(256) map_attn_kernel(MapAttnParams p) {
 // merges the key splits, one warp per row; grid (tiles * G, rows / 4)
 template <typename T, int NM>
 __global__ void __launch_bounds__(128) map_attn_merge_kernel(MapAttnParams p) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   const int tile = blockIdx.x / p.G, g = blockIdx.x % p.G, r = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= p.tile_rows[tile]) return;
   const int vdim = p.vdim, PS = NM * (vdim + 2);
@@ -351,6 +357,8 @@ inline size_t map_attn_mma_smem(int nm, int dim, int VT, bool sk) {
 
 template <int NM, int VT, bool SK>
 __global__ void __launch_bounds__(128, 2) map_attn_mma_kernel(MapAttnParams p) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   constexpr int MR = SK ? 16 : 64, KT = DA_KT, NP = SK ? 1 : 4, VS = VT * 16 + 8;
   constexpr float L2E = 1.4426950408889634f;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -663,9 +671,11 @@ __global__ void __launch_bounds__(128, 2) map_attn_mma_kernel(MapAttnParams p) {
 // largest choice scores may be chosen.  The `top` largest choice scores are chosen (ties: the lower index); their weights are s as
 // it is, or (renorm) s / (sum of the chosen s + 1e-20) * out_scale.
 // ---------------------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) moe_route_grouped_kernel(const float* __restrict__ logits, long long ldl, const float* __restrict__ correction, int n,
+__global__ void __launch_bounds__(128) moe_route_grouped_kernel(const float* logits, long long ldl, const float* __restrict__ correction, int n,
                                                                 int top, int n_groups, int keep, int sigmoid, int group_sum, int renorm, float out_scale,
-                                                                int* __restrict__ idx, float* __restrict__ wts, int n_tok) {
+                                                                int* idx, float* wts, int n_tok) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   extern __shared__ float route_buf[];      // per warp: [n] scores, [n] choice scores, [n_groups] group scores
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x * 4 + warp;
   if (t >= n_tok) return;

@@ -220,8 +220,6 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   const int rank = CG == 2 ? (int)(blockIdx.x & 1) : 0;
   const int first = blockIdx.x / CG, step = gridDim.x / CG;
   const bool grouped = p.tile_e != nullptr;
-  const int mt = grouped ? p.n_tiles[0] : p.mt;
-  const int tiles = mt * p.nt, units = tiles * p.splits;      // unit: a tile's sums over one range of k
 
   if (threadIdx.x == 0) {
     quit = 0;
@@ -243,6 +241,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   pair_sync<CG>();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<const uint32_t*>(smem_raw + (tptr - raw));
+  pdl_trigger();
+  pdl_wait();                                           // set-up ran under the preceding kernel; rows, tile table and results are its business too
+  const int mt = grouped ? p.n_tiles[0] : p.mt;
+  const int tiles = mt * p.nt, units = tiles * p.splits;      // unit: a tile's sums over one range of k
 
   if (warp == 0) {
     if (lane == 0) {
@@ -437,10 +439,12 @@ int launch(const WideGemm& g, WideP p, int clusters, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(std::min(clusters, p.mt * p.nt * p.splits) * CG)); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CG; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = CG > 1 ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CG; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = CG > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_wide_kernel<CG, BN>, mx, mw, p);
   if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "gemm_wide launch failed: %s", cudaGetErrorString(e));
   g_launches.fetch_add(1, std::memory_order_relaxed);
