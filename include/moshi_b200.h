@@ -607,6 +607,9 @@ int b200_op_conv1d(const float* x_dev, const float* w_dev, const float* bias_dev
  *                          LAST INPUT STEP previous [B,Cin,1] instead of the overlap-add partial (the same information,
  *                          conv.py:349-361); Cin % 32 == 0. */
 int b200_op_tc_linear_f32(const float* x_dev, const float* w_dev, float* y_dev, int M, int N, int K, void* stream);
+/* Row-major fp32 weights out of what a Mimi handle keeps of them (packed hi / lo tiles and one bit per weight; csrc/mimi_lin.cuh), as
+ * b200_mimi_streaming_begin makes them for small batches: rows[N,K] = w[N,K] bit for bit.  K % 512 == 0, N % 16 == 0.  Synchronises (test helper). */
+int b200_op_tc_rows(const float* w_dev, float* rows_dev, int N, int K, void* stream);
 int b200_op_tc_conv1d(const float* x_dev, const float* w_dev, const float* bias_dev, float* prev_dev, const uint8_t* exec_mask_dev,
                       float* y_dev, int B, int Cin, int Cout, int T, int K, int stride, int dilation, int elu_in, int transposed,
                       void* stream);

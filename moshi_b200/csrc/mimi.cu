@@ -43,7 +43,8 @@ struct SeaLayer {
 struct TrLayer {
   const float *n1w, *n1b, *n2w, *n2b, *ls1, *ls2;
   mtc::TcLayer in_proj, out_proj, l1, l2;
-  const float *w_in = nullptr, *w_out = nullptr, *w_1 = nullptr, *w_2 = nullptr;      // row-major fp32 for few tokens (null: not a shape of mimi_lin_kernel)
+  uint32_t *b_in = nullptr, *b_out = nullptr, *b_1 = nullptr, *b_2 = nullptr;         // what the packed tiles lost of the weights (null: not a shape of mimi_lin_kernel)
+  float *w_in = nullptr, *w_out = nullptr, *w_1 = nullptr, *w_2 = nullptr;            // row-major fp32 while a batch of few tokens streams
   float *kc = nullptr, *vc = nullptr;
 };
 
@@ -326,14 +327,13 @@ int keep(b200_mimi* h, const std::string& name, std::vector<int64_t> shape, cons
   return B200_OK;
 }
 
-int keep_linear(b200_mimi* h, const std::string& name, int M, int K, mtc::TcLayer& L, const float** rows) {
+int keep_linear(b200_mimi* h, const std::string& name, int M, int K, mtc::TcLayer& L, uint32_t** lost) {
   const float* src = nullptr;
   B200_TRY(get_f32(h, name, {M, K}, &src));
   if (lin_takes(M, K)) {
-    float* copy = nullptr;
-    B200_TRY(h->weights.alloc_t(&copy, (size_t)M * K, false));
-    B200_CUDA(cudaMemcpyAsync(copy, src, (size_t)M * K * 4, cudaMemcpyDeviceToDevice, nullptr));
-    *rows = copy;
+    B200_TRY(h->weights.alloc_t(lost, lin_lost_words(M, K), false));
+    B200_TRY(lin_lost_bits(src, *lost, M, K, nullptr));
+    h->weight_bytes += (int64_t)lin_lost_words(M, K) * 4;
   }
   B200_TRY(pack_tc(h, L, src, M, K, 1));       // nn.Linear weight [out][in] is already [N][K]
   L.kind = 2; L.dil = 1; L.stride = 1; L.bias = nullptr; L.bias_mod = M;
@@ -349,14 +349,14 @@ int pack_transformer(b200_mimi* h, const std::string& prefix, Transformer& tr) {
   for (int li = 0; li < c.tr_num_layers; ++li) {
     const std::string p = prefix + ".transformer.layers." + std::to_string(li);
     TrLayer& L = tr.layers[li];
-    B200_TRY(keep_linear(h, p + ".self_attn.in_projs.0.weight", 3 * d, d, L.in_proj, &L.w_in));
-    B200_TRY(keep_linear(h, p + ".self_attn.out_projs.0.weight", d, d, L.out_proj, &L.w_out));
+    B200_TRY(keep_linear(h, p + ".self_attn.in_projs.0.weight", 3 * d, d, L.in_proj, &L.b_in));
+    B200_TRY(keep_linear(h, p + ".self_attn.out_projs.0.weight", d, d, L.out_proj, &L.b_out));
     B200_TRY(keep(h, p + ".norm1.weight", {d}, &L.n1w));
     B200_TRY(keep(h, p + ".norm1.bias", {d}, &L.n1b));
     B200_TRY(keep(h, p + ".norm2.weight", {d}, &L.n2w));
     B200_TRY(keep(h, p + ".norm2.bias", {d}, &L.n2b));
-    B200_TRY(keep_linear(h, p + ".linear1.weight", ff, d, L.l1, &L.w_1));
-    B200_TRY(keep_linear(h, p + ".linear2.weight", d, ff, L.l2, &L.w_2));
+    B200_TRY(keep_linear(h, p + ".linear1.weight", ff, d, L.l1, &L.b_1));
+    B200_TRY(keep_linear(h, p + ".linear2.weight", d, ff, L.l2, &L.b_2));
     B200_TRY(keep(h, p + ".layer_scale_1.scale", {d}, &L.ls1));
     B200_TRY(keep(h, p + ".layer_scale_2.scale", {d}, &L.ls2));
   }
@@ -370,6 +370,7 @@ int pack_quantizer(b200_mimi* h) {
   if (together) {
     B200_TRY(h->weights.alloc_t(&h->w_rvq_in, (size_t)2 * c.q_dimension * c.dimension, false));
     B200_TRY(h->weights.alloc_t(&h->w_rvq_out, (size_t)2 * c.q_dimension * c.dimension, false));
+    h->weight_bytes += (int64_t)4 * c.q_dimension * c.dimension * 4;
   }
   h->stored_levels[0] = c.q_n_semantic;
   h->stored_levels[1] = c.q_n_q - c.q_n_semantic;
@@ -1051,6 +1052,23 @@ int b200_mimi_streaming_begin(b200_mimi* h, int batch, void* stream) {
   B200_TRY(A.alloc_t(&h->tr_ao_lo, ntok * d));
   B200_TRY(A.alloc_t(&h->tr_h_hi, ntok * ff));
   B200_TRY(A.alloc_t(&h->tr_h_lo, ntok * ff));
+  if (h->tr_cuda_cores) {                        // freed with the rest of the batch's buffers
+    const size_t per_layer = (size_t)4 * d * d + (size_t)2 * ff * d;
+    float* next = nullptr;
+    B200_TRY(A.alloc_t(&next, per_layer * (h->enc_tr.layers.size() + h->dec_tr.layers.size()), false));
+    for (Transformer* tr : {&h->enc_tr, &h->dec_tr})
+      for (auto& L : tr->layers) {
+        auto rows = [&](const mtc::TcLayer& G, const uint32_t* lost, float** out) -> int {
+          *out = next;
+          next += (size_t)G.N * G.Cin;
+          return lin_rows(G.wt, lost, *out, G.N, G.Cin, G.NT, nullptr);
+        };
+        B200_TRY(rows(L.in_proj, L.b_in, &L.w_in));
+        B200_TRY(rows(L.out_proj, L.b_out, &L.w_out));
+        B200_TRY(rows(L.l1, L.b_1, &L.w_1));
+        B200_TRY(rows(L.l2, L.b_2, &L.w_2));
+      }
+  }
   for (int which = 0; which < 2; ++which) {
     Transformer* tr = which == 0 ? &h->enc_tr : &h->dec_tr;
     const float* x_in = which == 0 ? h->tok_in_enc : h->tok_in_dec;

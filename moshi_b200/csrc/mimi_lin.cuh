@@ -149,6 +149,37 @@ __global__ void __launch_bounds__(128) mimi_lin_kernel(const LinP p) {
 
 inline bool lin_takes(int N, int K) { return K % 512 == 0 && N % 16 == 0; }
 
+// The row-major weights are held only while a batch small enough for mimi_lin_kernel streams: 201 MB that a full server has no use for, an
+// eighth of a session's rings.  They come back from the packed hi / lo tiles (mimi_tc.cu) bit for bit: hi is the weight rounded to 11
+// significant bits, so the remainder r = w - hi is exact and has at most 12, and lo is r rounded away from zero at the 11th; all that is
+// lost is whether the 12th was set.  In the encoding of a float that rounding adds bit 12 to r where r has it; that bit is kept, one
+// per weight (6.3 MB), and taken off again.  Only the sign of a zero, and weights below 2^-100, where r is no normal number, may differ.
+static __global__ void __launch_bounds__(256) lin_lost_bits_kernel(const float* w, uint32_t* bits) {      // grid N * K / 256
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  const float v = w[i];
+  float hi, lo;
+  mtc::split_tf32(v, hi, lo);
+  const uint32_t word = __ballot_sync(0xffffffffu, (__float_as_uint(v - hi) >> 12) & 1u);
+  if ((threadIdx.x & 31) == 0) bits[i >> 5] = word;
+}
+static __global__ void __launch_bounds__(256) lin_rows_kernel(const float* tiles, const uint32_t* bits, float* rows, int K, int NT) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  const int n = (int)(i / K), k = (int)(i - (long long)n * K), r = n % NT;
+  // 16-byte piece c of a tile row lies at position c ^ (row & 7); the lo tile follows the hi tile of its k-block
+  const long long o = (((long long)(n / NT) * (K / mtc::TC_KB) + k / mtc::TC_KB) * 2 * NT + r) * mtc::TC_KB + ((((k & 31) >> 2) ^ (r & 7)) << 2) + (k & 3);
+  const uint32_t lost = (bits[i >> 5] >> (i & 31)) & 1u;
+  rows[i] = tiles[o] + __uint_as_float(__float_as_uint(tiles[o + (long long)NT * mtc::TC_KB]) - (lost << 12));
+}
+inline size_t lin_lost_words(int N, int K) { return (size_t)N * K / 32; }
+inline int lin_lost_bits(const float* w, uint32_t* bits, int N, int K, cudaStream_t st) {
+  B200_LAUNCH(lin_lost_bits_kernel, (unsigned)((long long)N * K / 256), 256, 0, st, w, bits);
+  return check_launch("lin_lost_bits");
+}
+inline int lin_rows(const uint8_t* tiles, const uint32_t* bits, float* rows, int N, int K, int NT, cudaStream_t st) {
+  B200_LAUNCH(lin_rows_kernel, (unsigned)((long long)N * K / 256), 256, 0, st, reinterpret_cast<const float*>(tiles), bits, rows, K, NT);
+  return check_launch("lin_rows");
+}
+
 template <int NO, int TOK, int KC>
 int lin_launch_one(const LinP& p, cudaStream_t st) {
   cudaLaunchConfig_t cfg;

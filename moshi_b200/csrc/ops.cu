@@ -2,6 +2,7 @@
 #include "gemm_sk.cuh"
 #include "lm_kernels.cuh"
 #include "mimi_kernels.cuh"
+#include "mimi_lin.cuh"
 #include "mimi_tc.cuh"
 
 using namespace b200;
@@ -303,6 +304,20 @@ int tc_tile_shape(int T, int* tt, int* bb) {
 
 extern "C" {
 
+int b200_op_tc_rows(const float* w_dev, float* rows_dev, int N, int K, void* stream) {
+  using namespace b200::mtc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (!w_dev || !rows_dev || N < 1 || K < 1 || !mimi::lin_takes(N, K)) B200_FAIL(B200_ERR_SHAPE, "op_tc_rows: bad shape");
+  DevBufs d;
+  uint8_t* wt; uint32_t* lost;
+  B200_TRY(d.get(&wt, tc_packed_bytes(N, K, 1)));
+  B200_TRY(d.get(&lost, mimi::lin_lost_words(N, K) * 4));
+  B200_TRY(tc_pack_weights(w_dev, wt, N, K, 1, st));
+  B200_TRY(mimi::lin_lost_bits(w_dev, lost, N, K, st));
+  B200_TRY(mimi::lin_rows(wt, lost, rows_dev, N, K, N >= TC_MAX_NT ? TC_MAX_NT : N, st));
+  B200_CUDA(cudaStreamSynchronize(st));
+  return B200_OK;
+}
 int b200_op_tc_linear_f32(const float* x_dev, const float* w_dev, float* y_dev, int M, int N, int K, void* stream) {
   using namespace b200::mtc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
