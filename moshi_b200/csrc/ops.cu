@@ -159,7 +159,6 @@ int b200_op_attn_step(const void* qkv_dev, void* k_dev, void* v_dev, void* out_d
   if (B < 1 || H < 1 || cap < 1) B200_FAIL(B200_ERR_SHAPE, "op_attn_step: bad shape");
   int min_per = 1;
   if (nsplit <= 0) nsplit = attn_ragged_splits(B, H, cap, &min_per);
-  if (nsplit > 32) B200_FAIL(B200_ERR_SHAPE, "op_attn_step: more than 32 splits");
   static float* part = nullptr;
   static int* counters = nullptr;
   static size_t part_n = 0, cnt_n = 0;

@@ -1,0 +1,39 @@
+"""GPU: the temporal attention step with any number of key ranges asked for."""
+import ctypes as C
+
+import pytest
+import torch
+
+from .util import cptr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nsplit", [1, 2, 31, 32, 33, 64, 65, 100])
+@pytest.mark.parametrize("fills", [(0, 40), (99, 250), (1000, 63)])
+def test_ranges_of_keys(nsplit, fills):
+    """Fewer keys than ranges, ranges that fill one, two and more rounds of 32, a full ring; against 64 bits and, among themselves, one merge for all."""
+    from moshi_b200 import _lib
+    B, H, cap, D = len(fills), 2, 250, 128
+    g = torch.Generator().manual_seed(sum(fills))
+    qkv = torch.randn(B, 3, H, D, generator=g).bfloat16().cuda()
+    k, v = (torch.randn(B, H, cap, D, generator=g).bfloat16().cuda() for _ in range(2))
+    pos, mask = torch.tensor(fills, device="cuda"), torch.ones(B, dtype=torch.uint8, device="cuda")
+    out = torch.full((B, H * D), float("nan"), dtype=torch.bfloat16, device="cuda")
+    for _ in range(2):                                        # the arrival counters are left as they were found
+        kk, vv = k.clone(), v.clone()
+        _lib.check(_lib.lib().b200_op_attn_step(cptr(qkv), cptr(kk), cptr(vv), cptr(out), cptr(pos), cptr(mask), B, H, cap, nsplit, 10000.0,
+                                                C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    freq = torch.exp(torch.arange(D // 2, device="cuda").double() * (-torch.log(torch.tensor(10000.0).double()) * 2 / D))
+    for b, p in enumerate(fills):
+        c, s = torch.cos(p * freq), torch.sin(p * freq)
+        e, o = qkv[b, 0, :, 0::2].double(), qkv[b, 0, :, 1::2].double()
+        q = torch.stack([e * c - o * s, e * s + o * c], -1).reshape(H, D)
+        n = min(p + 1, cap)
+        w = torch.softmax(torch.einsum("hd,hnd->hn", q, kk[b, :, :n].double()) / D ** 0.5, -1)
+        want = torch.einsum("hn,hnd->hd", w, vv[b, :, :n].double()).reshape(-1)
+        # the turned query and the result are rounded to bf16 once each: scores move by up to 2^-9 * sum |q k| / sqrt(D) (about 0.02 for
+        # normal vectors), weights by that factor, the result by its half ulp
+        tol = 0.03 * torch.einsum("hn,hnd->hd", w, vv[b, :, :n].double().abs()).reshape(-1) + 1e-3
+        assert ((out[b].double() - want).abs() <= tol).all()
