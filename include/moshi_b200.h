@@ -258,11 +258,18 @@ int b200_lm_set_offset_cpu(b200_lm* h, int64_t value);
 /* Synchronises the handle's stream, returns and clears the device error flags.  The kernels never read out of bounds:
  * a token id outside its embedding table (anything but [0, card] and -1; the reference hits a device assert in F.embedding,
  * lm_utils.py:103-121) embeds as the zero row and raises B200_FLAG_TOKEN_RANGE; the *_host entry points check the flags at
- * their own synchronisation and return B200_ERR_INVALID. */
+ * their own synchronisation and return B200_ERR_INVALID.  B200_FLAG_WAIT: a wait inside the depformer kernel ran out (ten seconds), the
+ * frame's audio tokens are not valid; B200_ERR_CUDA from the *_host entry points and from the next step of the others. */
 #define B200_FLAG_TOKEN_RANGE 1
 #define B200_FLAG_CODE_RANGE 2
 #define B200_FLAG_KV_CAPACITY 4
+#define B200_FLAG_WAIT 8
 int b200_lm_error_flags(b200_lm* h, int* flags_out);
+/* What the gravest of the raised flags means, in words ("" for 0).  Needs no device. */
+const char* b200_lm_flag_text(int flags);
+/* B200_ERR_CUDA, once, if a finished step raised B200_FLAG_WAIT since it was last reported; reads a word of host memory, no synchronisation.
+ * Every step asks this first. */
+int b200_lm_check_waits(b200_lm* h);
 /* Algorithmic HBM bytes of one step at the current batch and ring fill: weights once
  * + per-row KV read/append + embeddings + logits. */
 int64_t b200_lm_algorithmic_bytes(b200_lm* h, int kv_fill);

@@ -134,6 +134,8 @@ _PROTOTYPES: dict[str, tuple[tp.Any, list]] = {
     "b200_lm_get_offset_cpu": (C.c_int64, [_P]),
     "b200_lm_set_offset_cpu": (_I, [_P, C.c_int64]),
     "b200_lm_error_flags": (_I, [_P, C.POINTER(_I)]),
+    "b200_lm_flag_text": (C.c_char_p, [_I]),
+    "b200_lm_check_waits": (_I, [_P]),
     # decoder LM (text-only layer-list models)
     "b200_dlm_create": (_I, [C.POINTER(DLMConfigC), C.POINTER(_P)]),
     "b200_dlm_load_tensor": (_I, [_P, C.c_char_p, _P, _I, _I, C.POINTER(C.c_int64)]),

@@ -75,6 +75,8 @@ struct DepParams {
   const float* noise; long long noise_ld; int noise_off, ka; // Exp(1) noise, row stride, offset of sub-step 0, per-step width
   int use_sampling, top_k; float temp;
   unsigned* bar;                                             // grid barrier counter (zero at launch)
+  unsigned long long wait_ns; unsigned wait_mask;            // dep_reg.cuh: a barrier's limit, looked at every wait_mask + 1 polls
+  volatile int* gave_up;                                     // host word raised when it ran out, may be null
   unsigned long long* trace;                                 // optional [DEP_TRACE_SLOTS]: %globaltimer of CTA 0 after every grid barrier
 };
 
@@ -565,7 +567,9 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   p.logits = static_cast<bf16*>(c.logits); p.audio_tokens = c.audio_tokens;
   p.noise = c.noise; p.noise_ld = c.noise_ld; p.noise_off = c.noise_off; p.ka = c.ka;
   p.use_sampling = c.use_sampling; p.top_k = c.top_k; p.temp = c.temp;
-  p.bar = c.bar; p.trace = c.trace;
+  p.bar = c.bar; p.trace = c.trace; p.gave_up = c.gave_up;
+  p.wait_ns = c.wait_ns > 0 ? (unsigned long long)c.wait_ns : (unsigned long long)WAIT_LIMIT_NS;
+  p.wait_mask = p.wait_ns < 1000000000ull ? 0u : 4095u;
   B200_TRY(make_map(enc, &d->map_xn, c.xn, c.B, c.dd, p.Mpad));
   B200_TRY(make_map(enc, &d->map_ao, c.ao, c.B, c.dd, p.Mpad));
   B200_TRY(make_map(enc, &d->map_h, c.hbuf, c.B, c.F, p.Mpad));

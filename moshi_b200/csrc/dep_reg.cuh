@@ -11,14 +11,14 @@
 // Frame of 1 session 2.0 (as a chain of launches) -> 1.35 ms, 8 sessions 2.6 (dep_fused_kernel) -> 1.39, 16 sessions 2.7 -> 2.0: 264 barriers of
 // about 5 us, of which the release of the epilogue's stores, the counter and the poll take half.
 //
-// A barrier that is not met within ten seconds raises the error flag and ends the kernel.
+// A barrier that is not met within ten seconds ends the kernel; the frame's remaining tokens are then the frame's before.  It raises ERR_WAIT, and a
+// word on the host that the handle's next call looks at without a synchronisation.
 #pragma once
 
 constexpr int REG_B = 16;                    // sessions at most
 constexpr int REG_FRAGS = 8;                 // (group, k-block, gate / value) fragments a warp holds: 4 pieces each
 constexpr int REG_GROUPS = 2;                // 16-row groups per CTA at most
 constexpr int REG_KB_SHORT = 2, REG_KB_LONG = 6;      // k-blocks per warp: dd <= 1024, F <= 3072
-constexpr int REG_ERR_WAIT = 8;
 
 struct RegW { uint4 f[REG_FRAGS][4]; };
 
@@ -33,20 +33,20 @@ __device__ __forceinline__ void reg_mma(float (&d)[4], uint32_t a0, uint32_t a1,
 }
 
 // all CTAs meet; false: not within the limit
-__device__ __forceinline__ bool reg_grid_sync(unsigned* bar, unsigned& epoch, int* ok) {
+__device__ __forceinline__ bool reg_grid_sync(const DepParams& p, unsigned& epoch, int* ok) {
   __syncthreads();
   if (threadIdx.x == 0) {
     epoch += 1;
     const unsigned target = epoch * gridDim.x;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.bar) : "memory");
     unsigned spins = 0;
     uint64_t t0 = 0;
     int met = 1;
-    while (ld_acquire(bar) < target) {
-      if ((++spins & 4095u) == 0u) {
+    while (ld_acquire(p.bar) < target) {
+      if ((++spins & p.wait_mask) == 0u) {
         const uint64_t now = global_timer_ns();
         if (t0 == 0) t0 = now;
-        else if (now - t0 > WAIT_LIMIT_NS) { met = 0; break; }
+        else if (now - t0 > p.wait_ns) { met = 0; break; }
       }
     }
     *ok = met;
@@ -264,20 +264,20 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
   reg_load<1, REG_KB_SHORT, 2>(w, p.w[0].in_w, gin, kd);
   for (int k = 0; k < p.dep_q; ++k) {
     input_rows(p, k);
-    if (!reg_grid_sync(p.bar, epoch, &ok)) break;
+    if (!reg_grid_sync(p, epoch, &ok)) break;
     for (int l = 0; l < p.L; ++l) {
       const DepLayerW lw = p.w[k * p.L + l];
       reg_stage<NT>(p, p.n1[l], xs, xs_ld);
       reg_product<1, REG_KB_SHORT, 2, NT>(w, gin, kd, red, shared_x);
       reg_epilogue<1, 2, NT>(red, gin, p.B, [&](int m, int n, float v, float) { qkv[(long long)m * 3 * p.dd + n] = f2bf(v); });
       reg_load<1, REG_KB_SHORT, 1>(w, lw.out_w, gd, kd);
-      if (!reg_grid_sync(p.bar, epoch, &ok)) break;
+      if (!reg_grid_sync(p, epoch, &ok)) break;
       reg_attention(p, qkv, l, k);
-      if (!reg_grid_sync(p.bar, epoch, &ok)) break;
+      if (!reg_grid_sync(p, epoch, &ok)) break;
       reg_product<1, REG_KB_SHORT, 1, NT>(w, gd, kd, red, global_x(p.ao, p.dd));
       reg_epilogue<1, 1, NT>(red, gd, p.B, add_to_x);
       reg_load<2, REG_KB_SHORT, 2>(w, lw.lin_in, gf, kd);
-      if (!reg_grid_sync(p.bar, epoch, &ok)) break;
+      if (!reg_grid_sync(p, epoch, &ok)) break;
       reg_stage<NT>(p, p.n2[l], xs, xs_ld);
       reg_product<2, REG_KB_SHORT, 2, NT>(w, gf, kd, red, shared_x);
       reg_epilogue<2, 2, NT>(red, gf, p.B, [&](int m, int n, float g, float u) {      // gating.py:18-20
@@ -285,12 +285,12 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
         p.hbuf[(long long)m * p.F + n] = f2bf(rbf(g / (1.f + expf(-g))) * u);
       });
       reg_load<1, REG_KB_LONG, 1>(w, lw.lin_out, gd, kf);
-      if (!reg_grid_sync(p.bar, epoch, &ok)) break;
+      if (!reg_grid_sync(p, epoch, &ok)) break;
       reg_product<1, REG_KB_LONG, 1, NT>(w, gd, kf, red, global_x(p.hbuf, p.F));
       reg_epilogue<1, 1, NT>(red, gd, p.B, add_to_x);
       if (l + 1 < p.L) reg_load<1, REG_KB_SHORT, 2>(w, p.w[k * p.L + l + 1].in_w, gin, kd);
       else reg_load<1, REG_KB_SHORT, 2>(w, p.heads[k], gh, kd);
-      if (!reg_grid_sync(p.bar, epoch, &ok)) break;
+      if (!reg_grid_sync(p, epoch, &ok)) break;
     }
     if (!ok) break;
     reg_stage<NT>(p, nullptr, xs, xs_ld);    // depformer_norms is Identity (lm.py:197-198): the head reads x itself
@@ -299,14 +299,20 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
       if (n < p.card) p.logits[((long long)k * p.B + m) * p.card + n] = f2bf(v);
     });
     if (k + 1 < p.dep_q) reg_load<1, REG_KB_SHORT, 2>(w, p.w[(k + 1) * p.L].in_w, gin, kd);
-    if (!reg_grid_sync(p.bar, epoch, &ok)) break;
+    if (!reg_grid_sync(p, epoch, &ok)) break;
     for (int m = blockIdx.x; m < p.B; m += gridDim.x) {      // the next sub-step's input rows are the same rows of the same CTA
       lm::sample_row(p.logits + ((long long)k * p.B + m) * p.card, p.noise + (long long)m * p.noise_ld + p.noise_off + (long long)k * p.ka,
                      p.audio_tokens + (long long)k * p.B + m, p.card, p.use_sampling, p.temp, p.top_k);
       __syncthreads();
     }
   }
-  if (threadIdx.x == 0 && !ok && p.err) atomicOr(p.err, REG_ERR_WAIT);
+  if (threadIdx.x == 0 && !ok) {
+    if (p.err) atomicOr(p.err, lm::ERR_WAIT);
+    if (p.gave_up) {
+      *p.gave_up = 1;
+      __threadfence_system();
+    }
+  }
 }
 
 inline size_t dep_reg_smem(int nt, int dd) { return (size_t)8 * nt * (dd * 2 + 64) + (size_t)4 * 8 * 16 * (8 * nt + 1) * 4; }

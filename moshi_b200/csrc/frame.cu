@@ -198,6 +198,7 @@ int b200_frame_step(b200_frame* f, const float* pcm_in_host, const int32_t* upda
   B200_CUDA(cudaMemcpyAsync(f->h_ready, f->ready, B, cudaMemcpyDeviceToHost, st));
   B200_CUDA(cudaEventRecord(f->done, st));
   B200_CUDA(cudaEventSynchronize(f->done));           // the frame's only host wait
+  B200_TRY(b200_lm_check_waits(f->lm));
   memcpy(tokens_out_host, f->h_tokens, B * (f->dep_q + 1) * 8);
   memcpy(pcm_out_host, f->h_pcm_out, B * f->frame * 4);
   if (ready_out_host) memcpy(ready_out_host, f->h_ready, B);

@@ -95,6 +95,8 @@ struct DepFusedConfig {
   const float* noise; long long noise_ld; int noise_off, ka;
   int use_sampling, top_k; float temp;
   unsigned* bar;
+  long long wait_ns;                               // limit of a grid barrier of the few-sessions kernel (0: ten seconds)
+  int* gave_up;                                    // mapped host word that kernel raises when the limit has passed, may be null
   unsigned long long* trace;                       // optional [DEP_TRACE_SLOTS] barrier timestamps of CTA 0 (diagnostics), may be null
 };
 constexpr int DEP_TRACE_SLOTS = 512;

@@ -87,6 +87,7 @@ struct b200_lm {
   int kv_fp8 = 0;                              // b200_lm_set_kv_dtype / B200_KV_DTYPE: opt-in 8-bit KV ring (B200_KV_FP8_E4M3 or B200_KV_INT8; 0 = bf16)
   float *dep_part0 = nullptr, *dep_part1 = nullptr;
   unsigned* dep_bar = nullptr;
+  int* dep_gave_up = nullptr;          // host word that a depformer kernel raises when a wait inside it ran out
   unsigned long long* dep_trace = nullptr;     // B200_DEP_TRACE=1: barrier timestamps of the fused depformer (diagnostics)
   int nsplit = 1, attn_min_per = 0;
   int n_in_static = 0;
@@ -706,6 +707,11 @@ int b200_lm_streaming_begin(b200_lm* h, int batch, void* stream) {
       if (atoi(e)) B200_TRY(A.alloc_t(&h->dep_trace, (size_t)tc::DEP_TRACE_SLOTS));
     }
     fc.trace = h->dep_trace;
+    fc.wait_ns = 0;
+    if (const char* e = getenv("B200_DEP_WAIT_NS")) fc.wait_ns = atoll(e);
+    B200_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h->dep_gave_up), sizeof(int), cudaHostAllocMapped));
+    *h->dep_gave_up = 0;
+    B200_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&fc.gave_up), h->dep_gave_up, 0));
     fc.logits = h->dep_logits; fc.audio_tokens = h->audio_tokens;
     fc.noise = h->noise; fc.noise_ld = noise_per_row(h);
     fc.noise_off = h->top_k_text < c.text_card ? h->top_k_text : c.text_card;
@@ -805,6 +811,8 @@ int b200_lm_streaming_end(b200_lm* h) {
   h->plans.clear();
   tc::dep_fused_destroy(h->depf);
   h->depf = nullptr;
+  if (h->dep_gave_up) cudaFreeHost(h->dep_gave_up);
+  h->dep_gave_up = nullptr;
   h->state.free_all();
   h->cfg_until = nullptr; h->noise_ctr = nullptr; h->err = nullptr; h->cond_sum = nullptr; h->cond_on = 0;
   if (h->pin_in) cudaFreeHost(h->pin_in);
@@ -891,11 +899,27 @@ int b200_lm_error_flags(b200_lm* h, int* flags_out) {
   B200_CUDA(cudaMemcpyAsync(&v, h->err, 4, cudaMemcpyDeviceToHost, h->stream));
   B200_CUDA(cudaStreamSynchronize(h->stream));
   if (v) B200_CUDA(cudaMemsetAsync(h->err, 0, 4, h->stream));
+  if (h->dep_gave_up) *h->dep_gave_up = 0;
   if (flags_out) *flags_out = v;
   return B200_OK;
 }
 
+const char* b200_lm_flag_text(int flags) {
+  if (flags & B200_FLAG_WAIT) return "a wait inside a kernel ran out: a frame's audio tokens are not valid";
+  if (flags & B200_FLAG_KV_CAPACITY) return "a session stepped past its shortened KV ring";
+  if (flags & B200_FLAG_TOKEN_RANGE) return "a token id outside its embedding table reached the model";
+  if (flags & B200_FLAG_CODE_RANGE) return "a code outside its codebook reached the codec";
+  return flags ? "an unknown flag" : "";
+}
+
+int b200_lm_check_waits(b200_lm* h) {
+  if (!h || !h->dep_gave_up || !*static_cast<volatile int*>(h->dep_gave_up)) return B200_OK;
+  *h->dep_gave_up = 0;
+  B200_FAIL(B200_ERR_CUDA, "lm: %s", b200_lm_flag_text(B200_FLAG_WAIT));
+}
+
 static int run_step(b200_lm* h, int n_in, int replace, int internal_noise) {
+  B200_TRY(b200_lm_check_waits(h));
   if (n_in != h->n_in_static || replace != h->replace_static || internal_noise != h->noise_static) {     // the captured graph is specific to all three
     h->n_in_static = n_in;
     h->replace_static = replace;
@@ -989,6 +1013,8 @@ int b200_lm_step_host(b200_lm* h, const int64_t* in_codes_host, int n_in, const 
   if (ready_host) *ready_host = (support_out_of_sync || h->offset_cpu > h->max_delay) ? 1 : 0;
   if (flags) {
     cudaMemsetAsync(h->err, 0, 4, h->stream);
+    if (h->dep_gave_up) *h->dep_gave_up = 0;
+    if (flags & lm::ERR_WAIT) B200_FAIL(B200_ERR_CUDA, "lm_step_host: %s (flags %d)", b200_lm_flag_text(flags), flags);
     if (flags & lm::ERR_KV_CAPACITY)
       B200_FAIL(B200_ERR_STATE, "lm_step_host: a session stepped past its %d-slot KV ring (b200_lm_set_kv_capacity; flags %d)", ring_cap(h), flags);
     B200_FAIL(B200_ERR_INVALID, "lm_step_host: a token id outside its embedding table reached the model (flags %d)", flags);

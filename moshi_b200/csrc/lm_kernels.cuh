@@ -49,7 +49,7 @@ struct TokenRing {
 
 // device error flags: raised instead of reading out of bounds; surfaced by b200_lm_error_flags / b200_mimi_error_flags and by
 // the host-synchronising entry points
-enum { ERR_TOKEN_RANGE = 1, ERR_CODE_RANGE = 2, ERR_KV_CAPACITY = 4 };
+enum { ERR_TOKEN_RANGE = 1, ERR_CODE_RANGE = 2, ERR_KV_CAPACITY = 4, ERR_WAIT = 8 };
 
 // One thread per (b, k): write the user's codes, then build the model input row(s) [MB][Kc].
 static __global__ void lm_prepare_kernel(const TokenRing r, const long long* __restrict__ in_codes, int n_in,

@@ -396,7 +396,7 @@ class LMGen:
 
     def error_flags(self) -> int:
         """Synchronises and returns (and clears) the device error flags (1 = a token id outside its embedding table, 4 = a session
-        stepped past a shortened KV ring, `kv_capacity`)."""
+        stepped past a shortened KV ring, `kv_capacity`, 8 = a wait inside a kernel ran out)."""
         v = C.c_int(0)
         with self._device():
             _lib.check(self._lib.b200_lm_error_flags(self._h, C.byref(v)))
@@ -431,7 +431,8 @@ class LMGen:
             _lib.check(self._lib.b200_lm_step_ex(self._h, _lib.ptr(codes), needed, _lib.ptr(noise), _lib.ptr(replace), _lib.ptr(out),
                                                  int(self.support_out_of_sync), C.byref(ready)))
         if self.check:                                      # lm.py:704-711: no ungenerated / out-of-range token may reach the model
-            assert self.error_flags() == 0, "a token outside its embedding table reached the model"
+            flags = self.error_flags()
+            assert flags == 0, self._lib.b200_lm_flag_text(flags).decode()
         if self.on_text_logits_hook is not None:
             tl = self.read_buffer("text_logits", torch.bfloat16, (B, lm.text_card))
             self.on_text_logits_hook(tl[:, None, None, :])
