@@ -50,6 +50,7 @@ __device__ __forceinline__ bool reg_grid_sync(const DepParams& p, unsigned& epoc
       }
     }
     *ok = met;
+    if (p.trace != nullptr && blockIdx.x == 0 && epoch < (unsigned)DEP_TRACE_SLOTS) p.trace[epoch] = global_timer_ns();
   }
   __syncthreads();
   return *ok != 0;
@@ -248,6 +249,7 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
   for (int i = threadIdx.x * 16; i < 8 * NT * xs_ld; i += THREADS * 16) *reinterpret_cast<uint4*>(xs + i) = make_uint4(0u, 0u, 0u, 0u);
   const int kd = p.dd / 64, kf = (p.F + 63) / 64, gd = p.dd / 16, gin = 3 * p.dd / 16, gf = p.F / 16, gh = (p.card + 15) / 16;
   unsigned epoch = 0;
+  if (p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) p.trace[0] = global_timer_ns();
   RegW w;
   auto shared_x = [&](int m, int byte) { return *reinterpret_cast<const uint4*>(xs + m * xs_ld + byte); };
   auto global_x = [&](const bf16* buf, int K) {

@@ -45,3 +45,18 @@ def test_a_barrier_that_runs_out_is_reported(lm, B, monkeypatch):
             gen.step(codes)
         assert gen.error_flags() == 0
         assert _lib.lib().b200_lm_check_waits(gen._h) == 0
+
+
+@pytest.mark.parametrize("B", [1, 12])
+def test_stamps_of_every_barrier(lm, B, monkeypatch):
+    """B200_DEP_TRACE: a stamp at the start and behind each of the 8 x (2 + 5 x layers) barriers, in order, and none beyond."""
+    from moshi_b200.models import LMGen
+    monkeypatch.setenv("B200_DEP_TRACE", "1")
+    gen = LMGen(lm, use_sampling=False)
+    with gen.streaming(B):
+        gen.step(_codes(lm, B))
+        t = gen.read_buffer("dep_trace", torch.int64, (512,)).cpu()
+        assert gen.error_flags() == 0
+    n = lm.cfg.dep_q * (2 + 5 * lm.cfg.depformer_num_layers)
+    assert (t[:n + 1] > 0).all() and (t[n + 1:] == 0).all()
+    assert (t[1:n + 1] >= t[:n]).all()
