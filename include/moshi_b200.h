@@ -577,6 +577,10 @@ int b200_op_linear_sk(const void* x_dev, const void* w_tiles_dev, void* y_dev, c
  * (b200_op_linear_sk with smem_budget = -1 keeps the swap-AB kernels at every M: the comparison row of tools/kbench.py.) */
 int b200_op_linear_ns(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K,
                       int epi, int gate_rows, int cluster, void* stream);
+/* The kernel with the weights going through registers (csrc/gemm_reg.cu) at every shape that it has: up to 32 rows, gated pairs up to 16.
+ * b200_op_linear_sk takes it where it is ahead: up to 8 rows, and up to 32 where the tiles are no more than the SMs. */
+int b200_op_linear_reg(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K, int epi, int gate_rows,
+                       void* stream);
 /* The decoder LM's linear for more than 256 activation rows (csrc/gemm_wide.cu): y[M,N] = x[M,K] . w^T over packed tiles
  * (b200_op_pack_tiles, epi 0) or, with packed = 0, a row-major w [N,K].  ldy: elements per result row; splits: ranges
  * that k is cut into (0 = the handle's choice).  K % 8 == 0.  Synchronises unless splits = 1 (test helper). */

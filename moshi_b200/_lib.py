@@ -166,6 +166,7 @@ _PROTOTYPES: dict[str, tuple[tp.Any, list]] = {
     "b200_op_linear_wide": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),
     "b200_op_prefill_attention": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, C.c_float, _P]),
     "b200_op_grouped_wide": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, C.c_float, _P]),
+    "b200_op_linear_reg": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P]),
     "b200_op_linear_ns": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),
     "b200_op_set_gemv_max_rows": (_I, [_I]),
     "b200_op_packed_bytes_i8": (C.c_int64, [_I, _I, _I, _I]),

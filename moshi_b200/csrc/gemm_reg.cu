@@ -66,13 +66,12 @@ __device__ __forceinline__ void finish(const RegP& p, int m, int n, float a, flo
   p.y[(long long)m * p.ldy + n] = __float2bfloat16_rn(v);
 }
 
-// gated pairs with 17 and more rows need the registers of a whole SM for one CTA
-constexpr int ctas_per_sm(int epi, int nt) { return epi == EPI_GATE && nt == 4 ? 1 : 2; }
+constexpr int CTAS_PER_SM = 2;             // 128 registers per thread
 
 template <int EPI, int NT, bool I8>
-__global__ void __launch_bounds__(THREADS, ctas_per_sm(EPI, NT)) gemm_reg_kernel(const RegP p) {
+__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gemm_reg_kernel(const RegP p) {
   using Acc = typename std::conditional<I8, int, float>::type;
-  constexpr int A = EPI == EPI_GATE ? 2 : 1, DEPTH = A == 2 ? (NT == 4 ? 4 : 2) : NT == 4 ? 3 : 4;
+  constexpr int A = EPI == EPI_GATE ? 2 : 1, DEPTH = A == 2 ? 2 : NT == 4 ? 3 : 4;
   __shared__ int arrived;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int tile = blockIdx.x / p.S, sp = blockIdx.x - tile * p.S;
@@ -203,29 +202,29 @@ template <int EPI, bool I8>
 cudaError_t launch_nt(const cudaLaunchConfig_t& cfg, const RegP& p) {
   if (p.M <= 8) return cudaLaunchKernelEx(&cfg, gemm_reg_kernel<EPI, 1, I8>, p);
   if (p.M <= 16) return cudaLaunchKernelEx(&cfg, gemm_reg_kernel<EPI, 2, I8>, p);
-  return cudaLaunchKernelEx(&cfg, gemm_reg_kernel<EPI, 4, I8>, p);
+  if constexpr (EPI == EPI_GATE) return cudaErrorInvalidValue;      // not supported (reg_supported)
+  else return cudaLaunchKernelEx(&cfg, gemm_reg_kernel<EPI, 4, I8>, p);
 }
 
 }  // namespace
 
 // Where the kernel is ahead of gemm_sk.cu (7B shapes, bf16, us): everything up to 8 rows (4096 -> 4096 22.9 -> 10.8, -> 12288 30.9 -> 22.1); up to 32
-// rows too (32 rows 41.0 -> 17.0 and 35.7 -> 29.8) but for gated pairs beyond 16 rows, whose fragments leave one CTA per SM (52 -> 64), and
+// rows too (32 rows 41.0 -> 17.0 and 35.7 -> 29.8) but for gated pairs beyond 16 rows, whose fragments left one CTA per SM (52 -> 64; not built), and
 // for 16-bit weights of more tiles than SMs beyond 8 rows, where whole tiles per CTA leave the second CTA of an SM idle (250 tiles, 32 rows
 // 55.6 -> 67.9; 8 rows 53.8 -> 51.9; int8 39.4 -> 38.1).
 bool reg_wins(int M, int N, int epi, int gate_rows, bool i8, int sms) {
   const int tiles = ((epi == EPI_GATE ? gate_rows : N) + ROWS - 1) / ROWS;
-  if (epi == EPI_GATE && M > 16) return false;
   return i8 || M <= 8 || tiles <= sms;
 }
 
-bool reg_supported(int M, const void* x, long long ldx_bytes) {
-  return M >= 1 && M <= REG_MAX_M && ldx_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+bool reg_supported(int M, int epi, const void* x, long long ldx_bytes) {
+  return M >= 1 && M <= (epi == EPI_GATE ? REG_MAX_M / 2 : REG_MAX_M) && ldx_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
 }
 
 int reg_linear(const void* x, long long ldx_bytes, const void* w_tiles, __nv_bfloat16* y, long long ldy, const __nv_bfloat16* res, long long ldr, int M, int N,
                int K, int epi, int gate_rows, const float* sa, const float* sw, float* ws, size_t ws_bytes, int* counters, int n_counters, int sms, int pdl,
                cudaStream_t stream) {
-  if (!reg_supported(M, x, ldx_bytes)) B200_FAIL(B200_ERR_SHAPE, "register GEMM: unsupported shape M=%d", M);
+  if (!reg_supported(M, epi, x, ldx_bytes)) B200_FAIL(B200_ERR_SHAPE, "register GEMM: unsupported shape M=%d", M);
   const bool i8 = sa != nullptr;
   RegP p;
   p.M = M; p.N = N; p.out_rows = epi == EPI_GATE ? gate_rows : N;
@@ -233,7 +232,7 @@ int reg_linear(const void* x, long long ldx_bytes, const void* w_tiles, __nv_bfl
   p.row_bytes = (long long)K * (i8 ? 1 : 2);
   p.num_kb = (int)((p.row_bytes + 127) / 128);
   const size_t slot = (size_t)(epi == EPI_GATE ? 2 : 1) * (M <= 8 ? 8 : M <= 16 ? 16 : 32) * ROWS * 4;
-  const int slots = sms * ctas_per_sm(epi, M <= 8 ? 1 : M <= 16 ? 2 : 4);
+  const int slots = sms * CTAS_PER_SM;
   // one wave where possible; a range of k costs about six blocks of start-up and exchange on top of its own
   int best = 1;
   long long cost = -1;

@@ -1128,7 +1128,7 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   if (tune.norm_alpha) B200_FAIL(B200_ERR_STATE, "sk GEMM: a fused RMSNorm input is only available on the GEMV path (M=%d)", M);
   // 3..32 sessions: weights through registers (gemm_reg.cu); explicit grids, clusters and the copy diagnostics keep the kernels below
   if (M <= REG_MAX_M && tune.grid == 0 && tune.cluster == 0 && !tune.stream_only && !tune.force_split && !tune.no_split && tune.smem_budget == 0 && tune.ns == 0 &&
-      (!i8 || (K % 16 == 0 && tune.sa && tune.sw)) && reg_wins(M, N, epi, gate_rows, i8, g_sms) && reg_supported(M, i8 ? tune.xq : x, i8 ? (long long)K : 2 * ldx))
+      (!i8 || (K % 16 == 0 && tune.sa && tune.sw)) && reg_wins(M, N, epi, gate_rows, i8, g_sms) && reg_supported(M, epi, i8 ? tune.xq : x, i8 ? (long long)K : 2 * ldx))
     return reg_linear(i8 ? tune.xq : x, i8 ? (long long)K : 2 * ldx, w_tiles, y, ldy, res, ldr, M, N, K, epi, gate_rows, i8 ? tune.sa : nullptr, tune.sw, ws,
                       sk_workspace_bytes(M), counters, SK_MAX_TILES, g_sms, tune.pdl, stream);
   // 33..256 sessions: activations as the A operand, two weight tiles (N = 256) per tcgen05.mma (gemm_ns.cu)

@@ -1,4 +1,5 @@
 // Kernel-level C entry points used by the parity tests (same kernels the handles launch).
+#include "gemm_reg.cuh"
 #include "gemm_sk.cuh"
 #include "lm_kernels.cuh"
 #include "mimi_kernels.cuh"
@@ -82,6 +83,18 @@ int b200_op_linear_ns(const void* x_dev, const void* w_tiles_dev, void* y_dev, c
   return tc::ns_linear(cache, static_cast<const __nv_bfloat16*>(x_dev), K, w_tiles_dev, static_cast<__nv_bfloat16*>(y_dev), out_cols,
                        static_cast<const __nv_bfloat16*>(res_dev), out_cols, M, N, K, epi, gate_rows, cluster, 0,
                        static_cast<cudaStream_t>(stream), unit_tiles);
+}
+
+int b200_op_linear_reg(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K, int epi, int gate_rows,
+                       void* stream) {
+  if (!x_dev || !w_tiles_dev || !y_dev) B200_FAIL(B200_ERR_INVALID, "op_linear_reg: null pointer");
+  if (M < 1 || N < 1 || K < 1 || !tc::reg_supported(M, epi, x_dev, (long long)K * 2)) B200_FAIL(B200_ERR_SHAPE, "op_linear_reg: unsupported shape");
+  const int out_cols = epi == 2 ? gate_rows : N;
+  float* ws = nullptr; int* counters = nullptr;
+  B200_TRY(sk_scratch(&ws, &counters));
+  return tc::reg_linear(x_dev, (long long)K * 2, w_tiles_dev, static_cast<__nv_bfloat16*>(y_dev), out_cols, static_cast<const __nv_bfloat16*>(res_dev), out_cols, M, N, K,
+                        epi, gate_rows, nullptr, nullptr, ws, tc::sk_workspace_bytes(M), counters, tc::SK_MAX_TILES, tc::sk_num_sms(), 0,
+                        static_cast<cudaStream_t>(stream));
 }
 
 int b200_op_set_gemv_max_rows(int max_rows) { return tc::sk_set_gemv_max_m(max_rows); }

@@ -21,7 +21,8 @@ def _stream():
 @pytest.mark.parametrize("N,K,epi", [(130, 72, STORE), (128, 8, STORE), (4096, 200, RESADD), (600, 4104, GATE), (4096, 11264, RESADD), (22528, 4096, GATE),
                                      (32000, 512, STORE)])
 def test_register_linear(M, N, K, epi):
-    """Edges of row blocks and tiles, remainders of k, one k-block, k whole and cut; two launches give the same bits."""
+    """Edges of row blocks and tiles, remainders of k, one k-block, k whole and cut; two launches give the same bits, and so does the general
+    entry point wherever its rule takes this kernel.  Gated pairs beyond 16 rows are not this kernel's and are refused."""
     from moshi_b200 import _lib
     lib = _lib.lib()
     g = torch.Generator().manual_seed(M + N + K)
@@ -31,16 +32,22 @@ def test_register_linear(M, N, K, epi):
     res = torch.randn(M, N, generator=g).bfloat16().cuda() if epi == RESADD else None
     wt = torch.empty(lib.b200_op_packed_bytes(N, K, epi, rows), dtype=torch.uint8, device="cuda")
     _lib.check(lib.b200_op_pack_tiles(cptr(w), cptr(wt), N, K, epi, rows, _stream()))
+    ys = [torch.full((M, rows or N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+    if epi == GATE and M > 16:
+        with pytest.raises(AssertionError, match="unsupported"):
+            _lib.check(lib.b200_op_linear_reg(cptr(x), cptr(wt), cptr(ys[0]), cptr(res), M, N, K, epi, rows, _stream()))
+        return
+    for y in ys[:2]:
+        _lib.check(lib.b200_op_linear_reg(cptr(x), cptr(wt), cptr(y), cptr(res), M, N, K, epi, rows, _stream()))
+        torch.cuda.synchronize()
     before = lib.b200_op_set_gemv_max_rows(0)
     try:
-        ys = []
-        for _ in range(2):
-            y = torch.full((M, rows or N), float("nan"), dtype=torch.bfloat16, device="cuda")
-            _lib.check(lib.b200_op_linear_sk(cptr(x), cptr(wt), cptr(y), cptr(res), M, N, K, epi, rows, 0, 0, 0, _stream()))
-            torch.cuda.synchronize()
-            ys.append(y)
+        _lib.check(lib.b200_op_linear_sk(cptr(x), cptr(wt), cptr(ys[2]), cptr(res), M, N, K, epi, rows, 0, 0, 0, _stream()))
+        torch.cuda.synchronize()
     finally:
         lib.b200_op_set_gemv_max_rows(before)
+    if M <= 8 or -(-(rows or N) // 128) <= torch.cuda.get_device_properties(0).multi_processor_count:
+        assert torch.equal(ys[0], ys[2])
     z = x.float() @ w.float().t()
     if epi == RESADD:
         z = res.float() + z.bfloat16().float()
@@ -55,6 +62,7 @@ def test_register_linear(M, N, K, epi):
 @pytest.mark.parametrize("M", [1, 5, 16, 31])
 @pytest.mark.parametrize("N,K,epi", [(130, 144, STORE), (4096, 2816, RESADD), (600, 4096, GATE)])
 def test_register_linear_int8_is_exact(M, N, K, epi):
+    """Exact sums; the gated pair of 31 rows goes to the kernel of gemm_sk.cu, on the other side of the line."""
     from moshi_b200 import _lib
     lib = _lib.lib()
     g = torch.Generator().manual_seed(M + N)
