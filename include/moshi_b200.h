@@ -528,7 +528,8 @@ int b200_dlm_set_stream(b200_dlm* h, void* stream);
  * products on the CUDA cores also where a tensor-core kernel would take them; 2: the tensor-core window / sigmoid attention also for
  * single-token requests; at 1 the sigmoid attention takes it for single tokens once a request holds 512 keys), "scan_segment" (before cache_begin; tokens per segment of the recurrences: portions of at least two
  * segments run as segments side by side; default 256), "delta_chunk" (0: the delta rule walks every portion token by token; default 1:
- * portions of at least 16 tokens run in chunks of 32), "time_kernels" (CUDA events around every
+ * portions of at least 16 tokens run in chunks of 32), "attn_expand" (portions of at least 128 tokens on keys and values expanded from the latents:
+ * 0 none, 1 where that is faster (default), 2 all that fit the buffers), "time_kernels" (CUDA events around every
  * operation, summed per class: a step then waits for its own end). */
 int b200_dlm_set_option(b200_dlm* h, const char* name, int value);
 /* Milliseconds spent so far per class of operation under "time_kernels": [0] linears, [1] attention, [2] the small products

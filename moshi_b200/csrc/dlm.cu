@@ -103,7 +103,13 @@ struct Layer {
 struct TileSig {
   int H, rpt;
   int off_row0 = 0, off_rows = 0, off_slot = 0;     // offsets into the step's metadata block (ints)
-  int count = 0;
+  int count = 0, max_ctx = 0;
+  // gated block: layers of r latent elements whose long portions can attend on expanded keys and values; the step's portions that do, which
+  // then have no tiles, and the rows of the others
+  int r = 0; bool expandable = false;
+  struct Run { int tok0, n; };
+  std::vector<int> expanded;
+  std::vector<Run> runs;
 };
 
 }  // namespace
@@ -115,7 +121,7 @@ struct b200_dlm {
   Arena weights, state;
   bool finalized = false, f32 = false;
   int device = -1;
-  int use_tc = 1, trace_layers = 0, attn_split = 0, attn_tc = 1;
+  int use_tc = 1, trace_layers = 0, attn_split = 0, attn_tc = 1, attn_expand = 1;
   // option "time_kernels": CUDA events around every operation of a step, summed per class (bench.py's per-kernel roofline)
   int time_kernels = 0;
   std::vector<cudaEvent_t> ev_pool; std::vector<int> ev_class; size_t ev_used = 0;
@@ -382,14 +388,14 @@ int run_attention(cudaStream_t st, AttnParams p, int tiles, int rpt, bool tensor
 }
 
 template <typename T>
-int attention(b200_dlm* h, const Layer& L, int max_ctx) {
+int attention(b200_dlm* h, const Layer& L) {
   const TileSig& s = h->sigs[L.sig];
   AttnParams p;
   p.qa = h->qa; p.cache = L.cache; p.sink = L.sink;
   p.tile_row0 = h->meta_dev + s.off_row0; p.tile_rows = h->meta_dev + s.off_rows; p.tile_slot = h->meta_dev + s.off_slot;
   p.tok_pos = h->meta_dev + h->off_pos;
   p.out = h->ol; p.part = h->part; p.cap = h->cap; p.r = L.c.a.kv_rank; p.H = L.c.a.heads; p.err = h->err;
-  p.nsplit = pick_split(h->attn_split, s.count, max_ctx, s.rpt, p.r, h->part_floats);
+  p.nsplit = pick_split(h->attn_split, s.count, s.max_ctx, s.rpt, p.r, h->part_floats);
   return run_attention<T>(h->stream, p, s.count, s.rpt, h->attn_tc != 0);
 }
 
@@ -417,19 +423,53 @@ int finish_logits(b200_dlm* h, const bf16* in_bf, long long ld, int n_want, int 
 }
 
 // Attention of long portions: scoring in the latent space costs r + r products per query, head and key where keys and values of the heads'
-// own size cost 128 + 128, and expanding a latent to all heads is paid once for all queries.  Worth it from 128 queries on (2048 tokens, 16
-// heads, r = 512: 497 us per layer with the folds around the latent kernel, 90 us expanded); shorter portions stay in the latent space.
-constexpr int EXPAND_FROM = 128;
-bool expands_latents(const b200_dlm* h, const Layer& L, int max_ctx) {
-  if (!L.uk || !h->attn_tc || max_ctx > h->flash_rows || !(L.c.a.scale > 0.f) || (L.ldp | L.off_q) % 8) return false;
-  for (const auto& q : h->portions)
-    if (q.n < EXPAND_FROM) return false;
-  return true;
+// own size cost 128 + 128, and expanding a latent to all heads is paid once for all queries.  But an expanded portion is three launches of its
+// own per layer, while the folds and the latent kernel take all of a step's portions at once.  Times per layer, us, in the latent space / expanded:
+//   16 heads, r = 512: 1 x 2048 tokens 742 / 280, 4 x 512 466 / 350, 8 x 256 420 / 447, 8 x 200 353 / 430, 16 x 128 395 / 626, 1 x 128 133 / 117;
+//   behind 2000 tokens: 8 x 128 636 / 570, 4 x 256 647 / 375; 8 heads: 4 x 512 256 / 244, 8 x 256 228 / 337; 32 heads: 8 x 256 1061 / 913.
+// Over 71 such steps (1..16 portions of 128..2048 tokens, 0..8000 tokens before them, 8, 16 and 32 heads) the difference is linear in what a portion
+// brings: LATENT_PAIR per query, key and head, LATENT_FOLD per token and head (both grow with r), EXPAND_FIXED, EXPAND_TILE per key tile that a
+// CTA walks and wave of CTAs, EXPAND_KEY per key and head (with r), and LATENT_FIXED for the latent path's launches, saved where no portion is left to it.
+// So every portion is weighed by itself, and those that would lose by a little are taken along where they are the only ones left.
+constexpr int EXPAND_FROM = 128;             // queries; shorter portions were not measured
+constexpr float LATENT_PAIR = 11e-6f, LATENT_FOLD = 3e-3f, LATENT_FIXED = 30.f, EXPAND_FIXED = 25.f, EXPAND_TILE = 0.55f, EXPAND_KEY = 0.27e-3f;      // us, r = 512
+float expand_gain(int H, int r, int n, int pos0) {
+  const float ctx = (float)(pos0 + n), rows = (float)H * n, scale = r / 512.f;
+  const float latent = scale * (LATENT_PAIR * rows * (pos0 + 0.5f * n) + LATENT_FOLD * rows);
+  const float waves = std::max(1.f, ceil_div(n, 128) * H / 148.f);
+  return latent - (EXPAND_FIXED + EXPAND_TILE * ceil_div(pos0 + n, 128) * waves + scale * EXPAND_KEY * H * ctx);
 }
-int expanded_attention(b200_dlm* h, const Layer& L, const bf16* proj, bf16* ob) {
+// fills s.expanded (portions), s.runs (neighbouring rows of the others)
+void choose_expanded(const b200_dlm* h, TileSig& s) {
+  s.expanded.clear(); s.runs.clear();
+  const int n = (int)h->portions.size();
+  const bool some = s.expandable && h->attn_tc && h->attn_expand && h->max_entry_tokens >= EXPAND_FROM;
+  std::vector<char> take(some ? n : 0, 0);
+  if (some) {
+    float rest = LATENT_FIXED;
+    bool all = true;                         // every portion could be expanded
+    for (int i = 0; i < n; ++i) {
+      const auto& q = h->portions[i];
+      const bool fits = q.n >= EXPAND_FROM && q.pos0 + q.n <= h->flash_rows;
+      const float gain = fits ? expand_gain(s.H, s.r, q.n, q.pos0) : 0.f;
+      take[i] = fits && (h->attn_expand > 1 || gain > 0.f);
+      all = all && fits;
+      if (!take[i]) rest += gain;
+    }
+    if (all && rest > 0.f) std::fill(take.begin(), take.end(), 1);
+  }
+  for (int i = 0; i < n; ++i) {
+    const auto& q = h->portions[i];
+    if (some && take[i]) s.expanded.push_back(i);
+    else if (!s.runs.empty() && s.runs.back().tok0 + s.runs.back().n == q.tok0) s.runs.back().n += q.n;
+    else s.runs.push_back({q.tok0, q.n});
+  }
+}
+int expanded_attention(b200_dlm* h, const Layer& L, const std::vector<int>& which, const bf16* proj, bf16* ob) {
   const int H = L.c.a.heads, r = L.c.a.kv_rank;
   const bf16 *uk = static_cast<const bf16*>(L.uk), *uv = static_cast<const bf16*>(L.uv);
-  for (const auto& q : h->portions) {
+  for (int i : which) {
+    const auto& q = h->portions[i];
     const int ctx = q.pos0 + q.n;
     const bf16* lat = static_cast<const bf16*>(L.cache) + (size_t)q.slot * h->cap * r;
     tc::WideGemm k;
@@ -467,17 +507,17 @@ int step_body(b200_dlm* h, int n_tok, int n_want, int max_ctx, float* logits_out
     TIMED(CLS_ELEMENTWISE, EARLY_LAUNCH(latent_append_kernel<T>, ceil_div(n_tok, 4), 128, 0, st, proj, (long long)L.ldp, L.off_dkv, L.cnorm, static_cast<T*>(L.cache),
                 h->cap, r, meta + h->off_slot, meta + h->off_pos, n_tok, c.norm_eps));
     T* ob = static_cast<T*>(h->obuf);
-    if (expands_latents(h, L, max_ctx)) {
-      if constexpr (sizeof(T) == 2) B200_TRY(expanded_attention(h, L, proj, ob));
-    } else {
-      // query folded through W_uk (and the score scale): qa[t][h][:] = scale * q[t][h][:] . W_uk[h]
-      TIMED(CLS_FOLD, B200_TRY(head_gemm(st, proj + L.off_q, (long long)L.ldp, (long long)dk, static_cast<const T*>(L.ukT), (long long)dk, (long long)r * dk, h->qa,
-                       (long long)H * r, (long long)r, n_tok, r, dk, H, L.c.a.scale, h->attn_tc != 0)));
-      TIMED(CLS_ATTN, B200_TRY(attention<T>(h, L, max_ctx)));
-      // values: o[t][h][:] = W_uv[h] . (sum_j p_j c_j)
-      TIMED(CLS_FOLD, B200_TRY(head_gemm(st, h->ol, (long long)H * r, (long long)r, static_cast<const T*>(L.uv), (long long)r, (long long)dv * r, ob, (long long)H * dv,
-                       (long long)dv, n_tok, dv, r, H, 1.f, h->attn_tc != 0)));
-    }
+    const TileSig& sig = h->sigs[L.sig];
+    if constexpr (sizeof(T) == 2) B200_TRY(expanded_attention(h, L, sig.expanded, proj, ob));
+    // query folded through W_uk (and the score scale): qa[t][h][:] = scale * q[t][h][:] . W_uk[h]
+    for (const auto& run : sig.runs)
+      TIMED(CLS_FOLD, B200_TRY(head_gemm(st, proj + (long long)run.tok0 * L.ldp + L.off_q, (long long)L.ldp, (long long)dk, static_cast<const T*>(L.ukT), (long long)dk,
+                       (long long)r * dk, h->qa + (long long)run.tok0 * H * r, (long long)H * r, (long long)r, run.n, r, dk, H, L.c.a.scale, h->attn_tc != 0)));
+    if (sig.count) TIMED(CLS_ATTN, B200_TRY(attention<T>(h, L)));
+    // values: o[t][h][:] = W_uv[h] . (sum_j p_j c_j)
+    for (const auto& run : sig.runs)
+      TIMED(CLS_FOLD, B200_TRY(head_gemm(st, h->ol + (long long)run.tok0 * H * r, (long long)H * r, (long long)r, static_cast<const T*>(L.uv), (long long)r, (long long)dv * r,
+                       ob + (long long)run.tok0 * H * dv, (long long)H * dv, (long long)dv, run.n, dv, r, H, 1.f, h->attn_tc != 0)));
     T* mixo = static_cast<T*>(h->mixo);
     TIMED(CLS_LINEAR, B200_TRY(linear<T>(h, ob, (long long)H * dv, L.o, mixo, W, n_tok)));
     // feed-forward
@@ -560,9 +600,10 @@ size_t window_attn_smem(const b200_dlm_mixer& m, int QT, int KT, size_t es, int*
   return 4 * (QT * Nq + rows * m.vdim + 2 * rows * (KT + 1) + (size_t)m.heads * m.heads + 3 * rows) + es * ((size_t)KT * *kstride + KT * Nv) + 32;
 }
 
-int add_sig(b200_dlm* h, int H, int rpt) {
-  for (size_t k = 0; k < h->sigs.size(); ++k) if (h->sigs[k].H == H && h->sigs[k].rpt == rpt) return (int)k;
-  TileSig s; s.H = H; s.rpt = rpt; h->sigs.push_back(s);
+int add_sig(b200_dlm* h, int H, int rpt, int r = 0, bool expandable = false) {
+  for (size_t k = 0; k < h->sigs.size(); ++k)
+    if (h->sigs[k].H == H && h->sigs[k].rpt == rpt && h->sigs[k].r == r && h->sigs[k].expandable == expandable) return (int)k;
+  TileSig s; s.H = H; s.rpt = rpt; s.r = r; s.expandable = expandable; h->sigs.push_back(s);
   return (int)h->sigs.size() - 1;
 }
 
@@ -2563,6 +2604,8 @@ int b200_dlm_set_option(b200_dlm* h, const char* name, int value) {
     h->scan_seg = value < 8 ? 8 : value;
   } else if (n == "delta_chunk") {
     h->delta_chunk = value != 0;
+  } else if (n == "attn_expand") {
+    h->attn_expand = value < 0 ? 0 : value;
   } else if (n == "attn_split") {
     h->attn_split = value < 0 ? 0 : value;
   } else {
@@ -2663,11 +2706,8 @@ int b200_dlm_finalize(b200_dlm* h) {
       B200_TRY(seal_weight(h, L.down, wd, (int)W, (int)F, drop, (int)W));
     }
     B200_TRY(get_f32(h, p + "dwa", i + 2, &L.avg));
-    int sig = -1;
-    const int rpt = rows_per_tile((int)r);
-    for (size_t k = 0; k < h->sigs.size(); ++k) if (h->sigs[k].H == H && h->sigs[k].rpt == rpt) sig = (int)k;
-    if (sig < 0) { TileSig s; s.H = (int)H; s.rpt = rpt; h->sigs.push_back(s); sig = (int)h->sigs.size() - 1; }
-    L.sig = sig;
+    const bool expandable = L.uk && L.c.a.scale > 0.f && (L.ldp | L.off_q) % 8 == 0;
+    L.sig = add_sig(h, (int)H, rows_per_tile((int)r), (int)r, expandable);
   }
   B200_TRY(get_f32(h, "final.norm", W, &h->fnw));
   if (parallel && c.norm == B200_NORM_RMS_ZERO_CENTRED) B200_LAUNCH(add_one_kernel, ceil_div((int)W, 256), 256, 0, nullptr, h->fnw, (int)W);      // stored around zero
@@ -3072,12 +3112,19 @@ int b200_dlm_step(b200_dlm* h, int n_entries, const int32_t* slots_host, const i
   int t = 0, max_ctx = 0, n_seg_units = 0, n_chunks = 0;
   h->units.clear();
   h->portions.clear();
-  for (auto& s : h->sigs) s.count = 0;
+  for (int e = 0, t0 = 0; e < n_entries; t0 += counts_host[e++]) h->portions.push_back({t0, counts_host[e], slots_host[e], h->len[slots_host[e]]});
+  h->max_entry_tokens = 0;
+  for (int e = 0; e < n_entries; ++e) h->max_entry_tokens = std::max(h->max_entry_tokens, (int)counts_host[e]);
+  for (auto& s : h->sigs) {
+    s.count = s.max_ctx = 0;
+    if (h->cfg.block == B200_BLOCK_GATED_DEPTH_AVERAGE) choose_expanded(h, s);
+  }
   for (int e = 0; e < n_entries; ++e) {
     const int s = slots_host[e], n = counts_host[e], base = h->len[s];
-    h->portions.push_back({t, n, s, base});
     for (auto& sg : h->sigs) {
+      if (std::binary_search(sg.expanded.begin(), sg.expanded.end(), e)) continue;
       const int rows = n * sg.H;
+      sg.max_ctx = std::max(sg.max_ctx, base + n);
       for (int r0 = 0; r0 < rows; r0 += sg.rpt) {
         m[sg.off_row0 + sg.count] = t * sg.H + r0;
         m[sg.off_rows + sg.count] = std::min(sg.rpt, rows - r0);
@@ -3119,8 +3166,6 @@ int b200_dlm_step(b200_dlm* h, int n_entries, const int32_t* slots_host, const i
   h->n_entries = n_entries;
   h->n_units = (int)h->units.size();
   h->n_chunks = n_chunks;
-  h->max_entry_tokens = 0;
-  for (int e = 0; e < n_entries; ++e) h->max_entry_tokens = std::max(h->max_entry_tokens, (int)counts_host[e]);
   int rc;
   if (h->cfg.block == B200_BLOCK_PRE_NORM_STREAMS) rc = h->f32 ? step_streams<float>(h, t, n_want, max_ctx, logits_dev) : step_streams<bf16>(h, t, n_want, max_ctx, logits_dev);
   else if (h->cfg.block == B200_BLOCK_PARALLEL_RESIDUAL) rc = h->f32 ? step_parallel<float>(h, t, n_want, max_ctx, logits_dev) : step_parallel<bf16>(h, t, n_want, max_ctx, logits_dev);
