@@ -38,7 +38,8 @@ struct Layer {
   int ncat = 0, ldp = 0, off_q = 0, off_dkv = 0, off_up = 0, off_g1 = 0, off_g2 = 0;
   Weight cat, o, down;                 // [q | dkv | up | gate1 | gate2] x width;  width x (heads * vdim);  width x ff
   void *ukT = nullptr, *uv = nullptr;  // [H][r][dim] (transposed per head), [H * vdim][r]
-  void* uk = nullptr;                  // [H * dim][r]: long portions expand the latents to keys (null: not a shape of dlm_flash.cu)
+  bool expandable = false;             // a shape of dlm_flash.cu: long portions can expand the latents to keys and values
+  void* uk = nullptr;                  // [H * dim][r], while a cache with room for that lives
   float *n1w = nullptr, *n1b = nullptr, *cnorm = nullptr, *sink = nullptr, *b1 = nullptr, *b2 = nullptr, *avg = nullptr;
   void* cache = nullptr;               // [slots][cap][r]
   int sig = 0;                         // index of the layer's attention tile list
@@ -156,6 +157,7 @@ struct b200_dlm {
   struct Portion { int tok0, n, slot, pos0; };
   std::vector<Portion> portions;
   bf16 *flash_k = nullptr, *flash_v = nullptr; int flash_rows = 0;
+  Arena flash;                         // what only long portions need; a cache does without where memory is short
   float *segS = nullptr, *segB = nullptr, *segM = nullptr, *tokM = nullptr, *corr = nullptr;
   float *embw = nullptr, *h32 = nullptr, *qkv32 = nullptr, *scan32 = nullptr, *gate32 = nullptr, *attn32 = nullptr, *route32 = nullptr, *moe_w = nullptr, *scan_prep = nullptr, *scan_v = nullptr;
   void *mixo2 = nullptr, *obuf2 = nullptr, *yexp = nullptr;
@@ -598,6 +600,40 @@ size_t window_attn_smem(const b200_dlm_mixer& m, int QT, int KT, size_t es, int*
   const size_t words = ((Nk * es + 3) / 4) | 1;           // an odd number of 32-bit words between staged key rows
   *kstride = (int)(words * 4 / es);
   return 4 * (QT * Nq + rows * m.vdim + 2 * rows * (KT + 1) + (size_t)m.heads * m.heads + 3 * rows) + es * ((size_t)KT * *kstride + KT * Nv) + 32;
+}
+
+// Room for the expanded keys and values of one request, and W_uk as the model has it.  A step that expands a portion has not folded its
+// queries yet, so keys and values take the folded queries' and the weighted sums' buffers (fp32, step tokens x heads x r each: 16384 tokens
+// of context for 2048 step tokens and r = 512).  Where those are smaller they get buffers of their own if there is memory, up to 16384 tokens;
+// longer contexts stay in the latent space, as all portions do where W_uk finds no room or no step can bring a long one.
+void make_room_to_expand(b200_dlm* h, size_t max_hr) {
+  h->flash_rows = 0;
+  size_t hd = 0;
+  for (auto& L : h->layers)
+    if (L.expandable) hd = std::max(hd, (size_t)L.c.a.heads * FLASH_D);
+  if (!hd || h->tmax < EXPAND_FROM) return;
+  bool ok = true;
+  for (auto& L : h->layers) {
+    if (!L.expandable) continue;
+    const int H = L.c.a.heads, r = L.c.a.kv_rank;
+    ok = ok && h->flash.alloc(&L.uk, (size_t)H * FLASH_D * r * sizeof(bf16), false) == B200_OK;
+    if (!ok) break;
+    const long long n = (long long)H * FLASH_D * r;      // back from the folded form: [H][r][dim] -> [H][dim][r]
+    head_transpose_kernel<bf16><<<(unsigned)ceil_div64(n, 256), 256>>>(static_cast<const bf16*>(L.ukT), static_cast<bf16*>(L.uk), H, r, FLASH_D);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+  }
+  const int want = (std::min(h->cap, 16384) + 7) / 8 * 8, shared = (int)std::min<size_t>(want, (size_t)h->tmax * max_hr * 4 / (hd * 2) / 8 * 8);
+  if (ok) {
+    h->flash_k = reinterpret_cast<bf16*>(h->qa); h->flash_v = reinterpret_cast<bf16*>(h->ol); h->flash_rows = shared;
+    bf16* own = nullptr;
+    if (shared < want && h->flash.alloc_t(&own, 2 * hd * want, false) == B200_OK) {
+      h->flash_k = own; h->flash_v = own + hd * want; h->flash_rows = want;
+    }
+  } else {
+    h->flash.free_all();
+    for (auto& L : h->layers) L.uk = nullptr;
+  }
+  cudaGetLastError();                        // an allocation that failed is nothing to report
 }
 
 int add_sig(b200_dlm* h, int H, int rpt, int r = 0, bool expandable = false) {
@@ -2691,8 +2727,7 @@ int b200_dlm_finalize(b200_dlm* h) {
       if (h->f32) B200_LAUNCH(head_transpose_kernel<float>, (unsigned)ceil_div64(n, 256), 256, 0, nullptr, static_cast<const float*>(uk), static_cast<float*>(L.ukT), (int)H, (int)dk, (int)r);
       else B200_LAUNCH(head_transpose_kernel<bf16>, (unsigned)ceil_div64(n, 256), 256, 0, nullptr, static_cast<const bf16*>(uk), static_cast<bf16*>(L.ukT), (int)H, (int)dk, (int)r);
       B200_TRY(check_launch("head_transpose"));
-      if (!h->f32 && dk == FLASH_D && dv == FLASH_D && r % 8 == 0) L.uk = uk;
-      else drop.push_back(uk);
+      drop.push_back(uk);
       h->weight_bytes += n * es;
     }
     B200_TRY(matrix(p + "mix.uv", H * dv, r, &L.uv));
@@ -2706,8 +2741,8 @@ int b200_dlm_finalize(b200_dlm* h) {
       B200_TRY(seal_weight(h, L.down, wd, (int)W, (int)F, drop, (int)W));
     }
     B200_TRY(get_f32(h, p + "dwa", i + 2, &L.avg));
-    const bool expandable = L.uk && L.c.a.scale > 0.f && (L.ldp | L.off_q) % 8 == 0;
-    L.sig = add_sig(h, (int)H, rows_per_tile((int)r), (int)r, expandable);
+    L.expandable = !h->f32 && dk == FLASH_D && dv == FLASH_D && r % 8 == 0 && L.c.a.scale > 0.f && (L.ldp | L.off_q) % 8 == 0;
+    L.sig = add_sig(h, (int)H, rows_per_tile((int)r), (int)r, L.expandable);
   }
   B200_TRY(get_f32(h, "final.norm", W, &h->fnw));
   if (parallel && c.norm == B200_NORM_RMS_ZERO_CENTRED) B200_LAUNCH(add_one_kernel, ceil_div((int)W, 256), 256, 0, nullptr, h->fnw, (int)W);      // stored around zero
@@ -2739,6 +2774,9 @@ int b200_dlm_cache_end(b200_dlm* h) {
   DeviceGuard g(h->device);
   if (h->slots) cudaStreamSynchronize(h->stream);
   h->state.free_all();
+  h->flash.free_all();
+  for (auto& L : h->layers) L.uk = nullptr;
+  h->flash_rows = 0;
   if (h->meta_pin) { cudaFreeHost(h->meta_pin); h->meta_pin = nullptr; }
   for (auto e : h->ev_pool) cudaEventDestroy(e);
   h->ev_pool.clear(); h->ev_class.clear(); h->ev_used = 0;
@@ -2973,15 +3011,6 @@ int b200_dlm_cache_begin(b200_dlm* h, int slots, int capacity, int max_step_toke
     B200_TRY(A.alloc_t(&h->ol, T * max_hr));
     h->part_floats = (size_t)600 * 16 * (max_r + 2);
     B200_TRY(A.alloc(&h->ffo, T * W * es));
-    // expanded keys and values of one request; beyond 16384 tokens of context portions stay in the latent space
-    size_t hd = 0;
-    for (auto& L : h->layers) if (L.uk) hd = std::max(hd, (size_t)L.c.a.heads * FLASH_D);
-    h->flash_rows = 0;
-    if (hd) {
-      h->flash_rows = (std::min(capacity, 16384) + 7) / 8 * 8;
-      B200_TRY(A.alloc_t(&h->flash_k, hd * h->flash_rows, false));
-      B200_TRY(A.alloc_t(&h->flash_v, hd * h->flash_rows, false));
-    }
   } else {
     B200_TRY(A.alloc_t(&h->h32, T * W));
     B200_TRY(A.alloc_t(&h->qkv32, T * max_qkv));
@@ -3071,6 +3100,7 @@ int b200_dlm_cache_begin(b200_dlm* h, int slots, int capacity, int max_step_toke
   h->par.assign(slots, 0);
   h->last_tokens = h->last_want = 0;
   if (!h->f32 && h->use_tc) B200_TRY(tc::prepare_plans(h->plans));
+  if (c.block == B200_BLOCK_GATED_DEPTH_AVERAGE) make_room_to_expand(h, max_hr);
   B200_CUDA(cudaDeviceSynchronize());
   return B200_OK;
 }

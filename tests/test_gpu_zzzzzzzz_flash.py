@@ -131,3 +131,47 @@ def test_long_portions_beside_short_ones(model, mix):
             assert abs(launches - plain - 2 * (3 * long_ones + 2 * (runs - 1))) <= 2      # the merge of key ranges may come or go
         elif expand == RULE:
             assert launches == plain          # two heads: a portion's own launches never pay
+
+
+def test_room_for_long_portions_only_where_they_can_come():
+    """16 heads over 16384 tokens make 134 MB of keys and values: a cache whose steps bring fewer than 128 tokens has none of it, one with room in
+    the buffers of a latent step borrows that, and both answer alike."""
+    import gc
+    from moshi_b200.config import DecoderLMConfig
+    from moshi_b200.models import DecoderLMGen, loaders
+    lay = {"type": "latent_attention", "mixer": {"heads": 16, "dim": 128, "vdim": 128, "kv_rank": 64, "scale": 128 ** -0.5}, "mlp": {"kind": "dense", "ff": 512}}
+    cfg = DecoderLMConfig.from_dict({"architecture": "Likosun", "vocab": 320, "width": 256, "embedding": {"scale": 1.0}, "residual_mult": 0.5,
+                                     "norm": {"eps": 1e-6}, "layers": [lay]})
+    model = loaders.get_decoder_lm(None, cfg, device="cuda:0", synth_seed=5)
+
+    def used():
+        gc.collect()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free, total = torch.cuda.mem_get_info()
+        return (total - free) / 2 ** 20
+
+    toks = torch.randint(0, 320, (300,), generator=torch.Generator().manual_seed(1)).tolist()
+
+    def run(capacity, step, cuts, expand):
+        before = used()
+        with DecoderLMGen(model, slots=1, capacity=capacity, max_step_tokens=step, max_want=300) as gen:
+            took = used() - before
+            gen.set_option("attn_expand", expand)
+            out, at = [], 0
+            for n in cuts:
+                out.append(gen.step([(0, toks[at:at + n])], range(n)))
+                at += n
+            gen.set_option("attn_expand", RULE)
+            assert gen.error_flags() == 0
+            return torch.cat(out), took
+
+    run(320, 320, [300], NONE)                                      # code and first workspaces
+    want, plain = run(16384, 100, [100] * 3, NONE)
+    _, narrow = run(16384, 127, [100] * 3, ALL)
+    assert abs(narrow - plain) < 16
+    for capacity, step in ((320, 320), (16384, 512), (16384, 300)):      # 320 rows fit the step's own buffers, 16384 do not
+        got, took = run(capacity, step, [300], ALL)
+        assert ((got - want).norm() / want.norm()) < 1e-2, (capacity, step)
+        assert (took - plain > 100) == (capacity == 16384), (capacity, took, plain)
+    assert abs(run(16384, 127, [100] * 3, ALL)[1] - plain) < 16      # and given back
