@@ -41,7 +41,7 @@ struct b200_lm {
   // sampling (LMGen defaults, lm.py:556-571)
   int use_sampling = 1, top_k = 250, top_k_text = 25;
   float temp = 0.8f, temp_text = 0.7f;
-  int pdl = 1;                                 // programmatic dependent launch of the GEMMs (B200_PDL=0 disables)
+  int pdl = 1;                                 // programmatic dependent launch of the GEMMs and the small kernels between them (B200_PDL=0 disables)
   int sk_smem = 0;                             // bytes of pipeline stages per GEMM CTA (B200_SK_SMEM_KB; 0 = 200 KB, one CTA per SM)
   float* sk_ws = nullptr;                      // stream-K partial-accumulator slots (L2-resident)
   int* sk_counters = nullptr;                  // per-tile arrival counters (zero between launches)
@@ -154,7 +154,7 @@ int norm_linear(b200_lm* h, const bf16* x, const bf16* alpha, bf16* xn, const bf
                 int epi, int gate_rows, const float* w_scales) {
   if (!h->cfg.quantize && h->fuse_norm && M <= tc::sk_gemv_max_m())
     return linear(h, x, K, w, y, ldy, nullptr, 0, M, N, K, epi, gate_rows, w_scales, alpha);
-  B200_TRY(launch_early(rmsnorm_kernel, dim3(M), dim3(256), 0, h->body, x, alpha, xn, K, 1e-8f));
+  B200_TRY(launch_early_if(h->pdl != 0, rmsnorm_kernel, dim3(M), dim3(256), 0, h->body, x, alpha, xn, K, 1e-8f));
   return linear(h, xn, K, w, y, ldy, nullptr, 0, M, N, K, epi, gate_rows, w_scales);
 }
 
@@ -226,7 +226,7 @@ const bf16* guide(b200_lm* h, const bf16* logits, bf16* guided, int card, bool c
 }
 
 int sample(b200_lm* h, const bf16* logits, int card, const float* noise, long long* out, float temp, int top_k) {
-  B200_TRY(launch_early(sample_kernel, dim3(h->batch), dim3(SAMPLE_THREADS), 0, h->body, logits, (long long)card, noise, (long long)noise_per_row(h), out, card,
+  B200_TRY(launch_early_if(h->pdl != 0, sample_kernel, dim3(h->batch), dim3(SAMPLE_THREADS), 0, h->body, logits, (long long)card, noise, (long long)noise_per_row(h), out, card,
                       h->use_sampling, temp, top_k));
   return check_launch("sample");
 }
@@ -278,13 +278,13 @@ int step_body(b200_lm* h) {
       a.pos = h->pos; a.exec_mask = h->exec_mask_m; a.H = H; a.cap = ring_cap(h); a.nsplit = h->nsplit; a.min_per = h->attn_min_per;
       a.neg_log_period_2_over_d = nl;
       dim3 grid(MB * H, h->nsplit);
-      B200_TRY(launch_early(attn_group_keys() == 2 ? attn_step_kernel<2> : attn_step_kernel<4>, grid, dim3(ATT_THREADS), 0, st, a));
+      B200_TRY(launch_early_if(h->pdl != 0, attn_group_keys() == 2 ? attn_step_kernel<2> : attn_step_kernel<4>, grid, dim3(ATT_THREADS), 0, st, a));
     }
     B200_TRY(linear(h, h->ao, d, L.out_w, h->x, d, h->x, d, MB, d, d, LIN_RESADD, 0, L.out_s));
     B200_TRY(norm_linear(h, h->x, L.n2, h->xn, L.lin_in, h->hbuf, F, MB, F, d, LIN_GATE, F, L.lin_in_s));
     B200_TRY(linear(h, h->hbuf, F, L.lin_out, h->x, d, h->x, d, MB, d, F, LIN_RESADD, 0, L.lin_out_s));
   }
-  B200_TRY(launch_early(rmsnorm_kernel, dim3(MB), dim3(256), 0, st, h->x, h->out_norm, h->tout, d, 1e-8f));
+  B200_TRY(launch_early_if(h->pdl != 0, rmsnorm_kernel, dim3(MB), dim3(256), 0, st, h->x, h->out_norm, h->tout, d, 1e-8f));
   B200_TRY(linear(h, h->tout, d, h->text_linear, h->text_logits, c.text_card, nullptr, 0, MB, c.text_card, d, LIN_STORE, 0, h->text_linear_s));
   // lm.py:728-732: with cfg_is_no_text the text logits are the conditioned rows, otherwise the guided combination
   const bf16* tl = guide(h, h->text_logits, h->text_logits_cfg, c.text_card, !h->cfg_is_no_text);
@@ -311,11 +311,11 @@ int step_body(b200_lm* h) {
   } else {
     for (int k = 0; k < c.dep_q; ++k) {
       const long long* prev = k == 0 ? h->text_token : h->audio_tokens + (long long)(k - 1) * B;
-      B200_TRY(launch_early(dep_input_kernel, dim3(ceil_div(MB * dd, 256)), dim3(256), 0, st, h->din, (long long)c.dep_q * dd, k * dd,
+      B200_TRY(launch_early_if(h->pdl != 0, dep_input_kernel, dim3(ceil_div(MB * dd, 256)), dim3(256), 0, st, h->din, (long long)c.dep_q * dd, k * dd,
                   h->dep_tables[k], prev, h->dx, MB, dd, B, k == 0 ? c.text_card : c.card, h->err));
       for (auto& L : h->dlayers) {
         B200_TRY(norm_linear(h, h->dx, L.n1, h->dxn, L.in_w[k], h->dqkv, 3 * dd, MB, 3 * dd, dd, LIN_STORE, 0, L.in_s[k]));
-        B200_TRY(launch_early(dep_attn_step_kernel, dim3(ceil_div(MB * dH * 32, 128)), dim3(128), 0, st, h->dqkv, L.kc, L.vc, h->dao, MB, dH, c.dep_q, k));
+        B200_TRY(launch_early_if(h->pdl != 0, dep_attn_step_kernel, dim3(ceil_div(MB * dH * 32, 128)), dim3(128), 0, st, h->dqkv, L.kc, L.vc, h->dao, MB, dH, c.dep_q, k));
         B200_TRY(linear(h, h->dao, dd, L.out_w[k], h->dx, dd, h->dx, dd, MB, dd, dd, LIN_RESADD, 0, L.out_s[k]));
         B200_TRY(norm_linear(h, h->dx, L.n2, h->dxn, L.lin_in[k], h->dh, dF, MB, dF, dd, LIN_GATE, dF, L.lin_in_s[k]));
         B200_TRY(linear(h, h->dh, dF, L.lin_out[k], h->dx, dd, h->dx, dd, MB, dd, dF, LIN_RESADD, 0, L.lin_out_s[k]));

@@ -622,7 +622,7 @@ int quantize_frame(b200_mimi* h, const float* lat, long long* codes, long long c
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    cfg.attrs = attr; cfg.numAttrs = mtc::tc_pdl() ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, rvq_level_kernel, a);
     if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "rvq_level launch failed: %s", cudaGetErrorString(e));
     g_launches.fetch_add(1, std::memory_order_relaxed);

@@ -189,7 +189,7 @@ int lin_launch_one(const LinP& p, cudaStream_t st) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  cfg.attrs = attr; cfg.numAttrs = mtc::tc_pdl() ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, mimi_lin_kernel<NO, TOK, KC>, p);
   if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "mimi_lin launch failed: %s", cudaGetErrorString(e));
   g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -325,7 +325,7 @@ int attn_launch_one(const MimiAttn& p, int B, cudaStream_t st) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  cfg.attrs = attr; cfg.numAttrs = mtc::tc_pdl() ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, mimi_attn_kernel<T>, p);
   if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "mimi_attn launch failed: %s", cudaGetErrorString(e));
   g_launches.fetch_add(1, std::memory_order_relaxed);

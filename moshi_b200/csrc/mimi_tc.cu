@@ -287,6 +287,11 @@ bool g_attr = false;
 
 }  // namespace
 
+bool tc_pdl() {
+  static const bool on = [] { const char* e = getenv("B200_MIMI_PDL"); return !e || atoi(e) != 0; }();
+  return on;
+}
+
 int tc_init() {
   if (!g_encode) {
     void* fn = nullptr;
@@ -374,14 +379,13 @@ int tc_plan(TcLayer& L, int n_sessions, int T, int sms, size_t ws_bytes) {
 int tc_launch(const TcLayer& L, cudaStream_t st) {
   // programmatic dependent launch (B200_MIMI_PDL=0: off): the kernel may start while its predecessor drains; it requests its
   // first weight tiles, then waits (griddepcontrol.wait) before it reads an activation or writes anything
-  static const int pdl = [] { const char* e = getenv("B200_MIMI_PDL"); return e ? atoi(e) : 1; }();
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)L.grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = L.smem; cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
+  cfg.attrs = attr; cfg.numAttrs = tc_pdl() ? 1 : 0;
   const cudaError_t le = cudaLaunchKernelEx(&cfg, mimi_tc_kernel, L.map_hi, L.map_lo, L.p);
   if (le != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "mimi_tc launch failed: %s", cudaGetErrorString(le));
   g_launches.fetch_add(1, std::memory_order_relaxed);

@@ -92,6 +92,7 @@ struct TcLayer {
 size_t tc_packed_bytes(int N, int Cin, int n_taps);
 // w: fp32 [N][n_taps * Cin] (k = tap * Cin + ci) -> tiles
 int tc_pack_weights(const float* w_dev, void* out_dev, int N, int Cin, int n_taps, cudaStream_t st);
+bool tc_pdl();                           // the codec's kernels may start while their predecessor drains (B200_MIMI_PDL=0: off)
 int tc_init();
 // 3-D tensor map over a token-major activation buffer base[b][row][Cin] (session stride sb elements, row stride = Cin)
 int tc_make_map(CUtensorMap* m, const float* base, int Cin, long long rows_per_session, long long sb_elems, int n_sessions, int tt,
