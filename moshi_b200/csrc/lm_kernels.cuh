@@ -872,8 +872,9 @@ static __device__ float block_reduce(float v, bool is_max, float* red) {
   return t;
 }
 
-// One row per call; every thread of a SAMPLE_THREADS-wide CTA must call it (block-wide barriers inside).
-static __device__ void sample_row(const bf16* __restrict__ logits, const float* __restrict__ noise, long long* __restrict__ out,
+// One row per call; every thread of a SAMPLE_THREADS-wide CTA must call it (block-wide barriers inside).  No __restrict__ on the logits: the
+// persistent depformers call this between grid barriers, where other CTAs wrote the row after this one may have cached the line it begins in.
+static __device__ void sample_row(const bf16* logits, const float* __restrict__ noise, long long* __restrict__ out,
                                   int card, int use_sampling, float temp, int top_k) {
   __shared__ float red[SAMPLE_THREADS / 32];
   __shared__ unsigned hist[256];
