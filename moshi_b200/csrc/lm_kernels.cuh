@@ -322,15 +322,19 @@ inline int attn_pick_splits(int B, int H, int cap) {
   return ns;
 }
 
-// The same for the 16-bit ring, whose kernel gives a session only the ranges that its own history fills (at least min_per keys each).  Few
-// (session, head) pairs: ranges of 64 keys and more.  592 to 1183 pairs are one uneven wave: ranges of 512 keys even it out (24 full rings
-// 218 -> 196 us, 24 sessions of 0 to 3000 frames 91 -> 86).  From 1184 on whole rings stream best (104 full rings 718 us, in ranges of 512 773).
+// The same for the 16-bit ring, whose kernel gives a session only the ranges that its own history fills (at least min_per keys each).  Four CTAs fit an
+// SM, 592 the GPU.  Fewer (session, head) pairs: ranges of 64 keys and more.  A second wave up to a quarter full costs as much as the first, and
+// ranges even it out; the fuller it is, the longer the ranges may be, and the more there are, the more CTAs are launched for nothing
+// while sessions are young.  us, whole rings / ranges of 1024 / of 512 keys, 32 heads, all sessions of 3000 frames (of 0 to 3000; of 10):
+//   19 sessions 196 / 166 / 165 (85 / 79 / 72; 11 / 11 / 11), 24: 223 / 188 / 200 (95 / 88 / 89; 11 / 11 / 13),
+//   28: 225 / 222 / 232 (101 / 94 / 96; 11 / 11 / 14), 32: 236 / 261 / 262 (119 / 107 / 113; 11 / 13 / 15), 36: 259 / 277 / 296 (131 / 125 / 125; 12 / 13 / 17).
+// From half a second wave on rings stay whole: what mixed ages would gain, full rings would lose.  (104 full rings 718 us, in ranges of 512 773.)
 inline int attn_ragged_splits(int B, int H, int cap, int* min_per) {
   const int pairs = B * H;
   int ns = 1;
   *min_per = cap;
   if (pairs < 148 * 4) { ns = (148 * 4 + pairs - 1) / pairs; *min_per = 64; }
-  else if (pairs < 148 * 8) { ns = (cap + 511) / 512; *min_per = 512; }
+  else if (pairs < 148 * 6) { *min_per = pairs < 148 * 5 ? 512 : 1024; ns = (cap + *min_per - 1) / *min_per; }
   if (ns > 16) ns = 16;
   const int max_by_len = (cap + 63) / 64;
   return ns > max_by_len ? max_by_len : ns;
