@@ -501,21 +501,27 @@ static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const Att
   if (!s_last) return;
   __threadfence();
   const float* pp = a.part + (long long)bh * a.nsplit * (ATT_D + 2);
-  // lane s holds range s's maximum and sum: two round trips to L2 for up to 32 ranges (all that a handle uses)
-  const float m0 = lane < splits ? __ldcg(pp + lane * (ATT_D + 2) + ATT_D) : -INFINITY;
-  const float l0 = lane < splits ? __ldcg(pp + lane * (ATT_D + 2) + ATT_D + 1) : 0.f;
-  float mx = m0;
-  for (int s = lane + 32; s < splits; s += 32) mx = fmaxf(mx, __ldcg(pp + s * (ATT_D + 2) + ATT_D));
-  const float MM = warp_max(mx);
   float LL = 0.f, AA = 0.f;
-  for (int s0 = 0; s0 < splits; s0 += 32) {         // the ranges' sums are added in their order
-    const int mine = s0 + lane, n = min(32, splits - s0);
-    const float ms = s0 == 0 ? m0 : mine < splits ? __ldcg(pp + mine * (ATT_D + 2) + ATT_D) : -INFINITY;
-    const float ls = s0 == 0 ? l0 : mine < splits ? __ldcg(pp + mine * (ATT_D + 2) + ATT_D + 1) : 0.f;
+  if (splits <= 32) {      // all that a handle uses: lane s holds range s's maximum and sum, two round trips to L2 whatever the number of ranges
+    const float ms = lane < splits ? __ldcg(pp + lane * (ATT_D + 2) + ATT_D) : -INFINITY;
+    const float ls = lane < splits ? __ldcg(pp + lane * (ATT_D + 2) + ATT_D + 1) : 0.f;
+    const float MM = warp_max(ms);
     const float cf = ms == -INFINITY ? 0.f : __expf(ms - MM);
-    LL += warp_sum(ls * cf);
+    LL = warp_sum(ls * cf);
 #pragma unroll 8
-    for (int s = 0; s < n; ++s) AA += __ldcg(pp + (s0 + s) * (ATT_D + 2) + tid) * __shfl_sync(0xffffffffu, cf, s);
+    for (int s = 0; s < splits; ++s) AA += __ldcg(pp + s * (ATT_D + 2) + tid) * __shfl_sync(0xffffffffu, cf, s);
+  } else {                 // a warp's width of ranges at a time, in their order
+    float mx = -INFINITY;
+    for (int s = lane; s < splits; s += 32) mx = fmaxf(mx, __ldcg(pp + s * (ATT_D + 2) + ATT_D));
+    const float MM = warp_max(mx);
+    for (int s0 = 0; s0 < splits; s0 += 32) {
+      const int mine = s0 + lane, n = min(32, splits - s0);
+      const float ms = mine < splits ? __ldcg(pp + mine * (ATT_D + 2) + ATT_D) : -INFINITY;
+      const float ls = mine < splits ? __ldcg(pp + mine * (ATT_D + 2) + ATT_D + 1) : 0.f;
+      const float cf = ms == -INFINITY ? 0.f : __expf(ms - MM);
+      LL += warp_sum(ls * cf);
+      for (int s = 0; s < n; ++s) AA += __ldcg(pp + (s0 + s) * (ATT_D + 2) + tid) * __shfl_sync(0xffffffffu, cf, s);
+    }
   }
   a.out[(long long)bh * ATT_D + tid] = f2bf(LL > 0.f ? AA / LL : 0.f);
 }
