@@ -488,7 +488,7 @@ struct DepFused {
   DepParams p;
   CUtensorMap map_xn, map_ao, map_h, map_x;
   int grid = 0; size_t smem = 0;
-  int reg_nt = 0;                 // up to 16 sessions: dep_reg_kernel with this many blocks of 8 (0: dep_fused_kernel)
+  DepRegKernel reg = nullptr;     // up to 16 sessions: dep_reg_kernel with as many blocks of 8 as they fill (null: dep_fused_kernel)
   void* dev_tables = nullptr;     // one allocation holding the pointer tables
 };
 
@@ -576,15 +576,16 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   B200_TRY(make_map(enc, &d->map_x, c.x, c.B, c.dd, p.Mpad));
   d->smem = (size_t)stages * p.stage_bytes + 1024 + 16 * MAX_STAGES + 64;
   if (dep_reg_takes(c, d->grid)) {
-    d->reg_nt = c.B <= 8 ? 1 : 2;
-    d->smem = dep_reg_smem(d->reg_nt, c.dd);
-    B200_CUDA(cudaFuncSetAttribute(d->reg_nt == 1 ? dep_reg_kernel<1> : dep_reg_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem));
+    const int nt = c.B <= 8 ? 1 : 2;
+    d->reg = dep_reg_pick(nt, c.trace || c.wait_ns > 0);
+    d->smem = dep_reg_smem(nt, c.dd);
+    B200_CUDA(cudaFuncSetAttribute(d->reg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem));
   }
   B200_CUDA(cudaFuncSetAttribute(dep_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
   int per_sm = 0, coop = 0, dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
   B200_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-  if (d->reg_nt) B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, d->reg_nt == 1 ? dep_reg_kernel<1> : dep_reg_kernel<2>, THREADS, d->smem));
+  if (d->reg) B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, d->reg, THREADS, d->smem));
   else B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dep_fused_kernel, THREADS, d->smem));
   if (!coop || per_sm < 1) {
     dep_fused_destroy(d);
@@ -617,9 +618,8 @@ int dep_fused_launch(DepFused* d, cudaStream_t stream) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
   bf16* qkv = reinterpret_cast<bf16*>(d->p.part0);      // the partial sums' workspace holds the projections
-  const cudaError_t le = d->reg_nt == 1   ? cudaLaunchKernelEx(&cfg, dep_reg_kernel<1>, d->p, qkv)
-                         : d->reg_nt == 2 ? cudaLaunchKernelEx(&cfg, dep_reg_kernel<2>, d->p, qkv)
-                                          : cudaLaunchKernelEx(&cfg, dep_fused_kernel, d->map_xn, d->map_ao, d->map_h, d->map_x, d->p);
+  const cudaError_t le = d->reg ? cudaLaunchKernelEx(&cfg, d->reg, d->p, qkv)
+                                : cudaLaunchKernelEx(&cfg, dep_fused_kernel, d->map_xn, d->map_ao, d->map_h, d->map_x, d->p);
   if (le != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "fused depformer: cooperative launch failed: %s", cudaGetErrorString(le));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return check_launch("dep_fused");

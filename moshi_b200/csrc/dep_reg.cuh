@@ -32,7 +32,9 @@ __device__ __forceinline__ void reg_mma(float (&d)[4], uint32_t a0, uint32_t a1,
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// all CTAs meet; false: not within the limit
+// all CTAs meet; false: not within the limit.  DIAG: with time stamps and a limit of the caller's, in a kernel of its own (in the one kernel the
+// tests for them cost 0.13 us per barrier, 33 us per frame of 16 sessions).
+template <bool DIAG>
 __device__ __forceinline__ bool reg_grid_sync(const DepParams& p, unsigned& epoch, int* ok) {
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -43,16 +45,16 @@ __device__ __forceinline__ bool reg_grid_sync(const DepParams& p, unsigned& epoc
     uint64_t t0 = 0;
     int met = 1;
     while (ld_acquire(p.bar) < target) {
-      if ((++spins & p.wait_mask) == 0u) {
+      if ((++spins & (DIAG ? p.wait_mask : 4095u)) == 0u) {
         const uint64_t now = global_timer_ns();
         if (t0 == 0) t0 = now;
-        else if (now - t0 > p.wait_ns) { met = 0; break; }
+        else if (now - t0 > (DIAG ? p.wait_ns : WAIT_LIMIT_NS)) { met = 0; break; }
       }
     }
     *ok = met;
-    if (p.trace != nullptr && blockIdx.x == 0 && epoch < (unsigned)DEP_TRACE_SLOTS) p.trace[epoch] = global_timer_ns();
   }
   __syncthreads();
+  if (DIAG && p.trace != nullptr && threadIdx.x == 0 && blockIdx.x == 0 && epoch < (unsigned)DEP_TRACE_SLOTS) p.trace[epoch] = global_timer_ns();
   return *ok != 0;
 }
 
@@ -239,7 +241,7 @@ __device__ __forceinline__ void reg_attention(const DepParams& p, const bf16* qk
   }
 }
 
-template <int NT>
+template <int NT, bool DIAG>
 __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, bf16* qkv) {
   extern __shared__ __align__(16) uint8_t reg_smem[];
   __shared__ int ok;
@@ -249,7 +251,7 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
   for (int i = threadIdx.x * 16; i < 8 * NT * xs_ld; i += THREADS * 16) *reinterpret_cast<uint4*>(xs + i) = make_uint4(0u, 0u, 0u, 0u);
   const int kd = p.dd / 64, kf = (p.F + 63) / 64, gd = p.dd / 16, gin = 3 * p.dd / 16, gf = p.F / 16, gh = (p.card + 15) / 16;
   unsigned epoch = 0;
-  if (p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) p.trace[0] = global_timer_ns();
+  if (DIAG && p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) p.trace[0] = global_timer_ns();
   RegW w;
   auto shared_x = [&](int m, int byte) { return *reinterpret_cast<const uint4*>(xs + m * xs_ld + byte); };
   auto global_x = [&](const bf16* buf, int K) {
@@ -266,20 +268,20 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
   reg_load<1, REG_KB_SHORT, 2>(w, p.w[0].in_w, gin, kd);
   for (int k = 0; k < p.dep_q; ++k) {
     input_rows(p, k);
-    if (!reg_grid_sync(p, epoch, &ok)) break;
+    if (!reg_grid_sync<DIAG>(p, epoch, &ok)) break;
     for (int l = 0; l < p.L; ++l) {
       const DepLayerW lw = p.w[k * p.L + l];
       reg_stage<NT>(p, p.n1[l], xs, xs_ld);
       reg_product<1, REG_KB_SHORT, 2, NT>(w, gin, kd, red, shared_x);
       reg_epilogue<1, 2, NT>(red, gin, p.B, [&](int m, int n, float v, float) { qkv[(long long)m * 3 * p.dd + n] = f2bf(v); });
       reg_load<1, REG_KB_SHORT, 1>(w, lw.out_w, gd, kd);
-      if (!reg_grid_sync(p, epoch, &ok)) break;
+      if (!reg_grid_sync<DIAG>(p, epoch, &ok)) break;
       reg_attention(p, qkv, l, k);
-      if (!reg_grid_sync(p, epoch, &ok)) break;
+      if (!reg_grid_sync<DIAG>(p, epoch, &ok)) break;
       reg_product<1, REG_KB_SHORT, 1, NT>(w, gd, kd, red, global_x(p.ao, p.dd));
       reg_epilogue<1, 1, NT>(red, gd, p.B, add_to_x);
       reg_load<2, REG_KB_SHORT, 2>(w, lw.lin_in, gf, kd);
-      if (!reg_grid_sync(p, epoch, &ok)) break;
+      if (!reg_grid_sync<DIAG>(p, epoch, &ok)) break;
       reg_stage<NT>(p, p.n2[l], xs, xs_ld);
       reg_product<2, REG_KB_SHORT, 2, NT>(w, gf, kd, red, shared_x);
       reg_epilogue<2, 2, NT>(red, gf, p.B, [&](int m, int n, float g, float u) {      // gating.py:18-20
@@ -287,12 +289,12 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
         p.hbuf[(long long)m * p.F + n] = f2bf(rbf(g / (1.f + expf(-g))) * u);
       });
       reg_load<1, REG_KB_LONG, 1>(w, lw.lin_out, gd, kf);
-      if (!reg_grid_sync(p, epoch, &ok)) break;
+      if (!reg_grid_sync<DIAG>(p, epoch, &ok)) break;
       reg_product<1, REG_KB_LONG, 1, NT>(w, gd, kf, red, global_x(p.hbuf, p.F));
       reg_epilogue<1, 1, NT>(red, gd, p.B, add_to_x);
       if (l + 1 < p.L) reg_load<1, REG_KB_SHORT, 2>(w, p.w[k * p.L + l + 1].in_w, gin, kd);
       else reg_load<1, REG_KB_SHORT, 2>(w, p.heads[k], gh, kd);
-      if (!reg_grid_sync(p, epoch, &ok)) break;
+      if (!reg_grid_sync<DIAG>(p, epoch, &ok)) break;
     }
     if (!ok) break;
     reg_stage<NT>(p, nullptr, xs, xs_ld);    // depformer_norms is Identity (lm.py:197-198): the head reads x itself
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
       if (n < p.card) p.logits[((long long)k * p.B + m) * p.card + n] = f2bf(v);
     });
     if (k + 1 < p.dep_q) reg_load<1, REG_KB_SHORT, 2>(w, p.w[(k + 1) * p.L].in_w, gin, kd);
-    if (!reg_grid_sync(p, epoch, &ok)) break;
+    if (!reg_grid_sync<DIAG>(p, epoch, &ok)) break;
     for (int m = blockIdx.x; m < p.B; m += gridDim.x) {      // the next sub-step's input rows are the same rows of the same CTA
       lm::sample_row(p.logits + ((long long)k * p.B + m) * p.card, p.noise + (long long)m * p.noise_ld + p.noise_off + (long long)k * p.ka,
                      p.audio_tokens + (long long)k * p.B + m, p.card, p.use_sampling, p.temp, p.top_k);
@@ -317,6 +319,10 @@ __global__ void __launch_bounds__(THREADS, 1) dep_reg_kernel(const DepParams p, 
   }
 }
 
+typedef void (*DepRegKernel)(const DepParams, bf16*);
+inline DepRegKernel dep_reg_pick(int nt, bool diag) {
+  return nt == 1 ? (diag ? dep_reg_kernel<1, true> : dep_reg_kernel<1, false>) : (diag ? dep_reg_kernel<2, true> : dep_reg_kernel<2, false>);
+}
 inline size_t dep_reg_smem(int nt, int dd) { return (size_t)8 * nt * (dd * 2 + 64) + (size_t)4 * 8 * 16 * (8 * nt + 1) * 4; }
 inline bool dep_reg_takes(const DepFusedConfig& c, int grid) {
   return c.B <= REG_B && c.dd % 64 == 0 && c.dd <= REG_KB_SHORT * 8 * 64 && c.F % 16 == 0 && c.F <= REG_KB_LONG * 8 * 64 && 3 * c.dd / 16 <= REG_GROUPS * grid &&
