@@ -82,7 +82,7 @@ typedef struct {
 } b200_mimi_config;
 
 /* loaders.get_mimi (loaders.py:323-363): build, then feed the state dict tensor by tensor using the
- * reference's key names (SURVEY.md appendix A; legacy names are normalised by the Python shim),
+ * reference's key names (legacy names are normalised by the Python shim),
  * then finalize (derives centroids = embedding_sum / clamp(cluster_usage, 1e-5), core_vq.py:181-183,
  * and repacks weights into the kernels' HBM layouts).  Source tensors may be freed after each call. */
 int b200_mimi_create(const b200_mimi_config* cfg, b200_mimi** out);
@@ -146,7 +146,7 @@ int b200_mimi_set_graph(b200_mimi* h, int enable);
  * "enc.latent", "dec.latent" ([B,C]). */
 int b200_mimi_read_buffer(b200_mimi* h, const char* name, float* dst_dev, int64_t capacity, int64_t* numel);
 /* Bytes of weights + per-step state traffic of one encode+decode frame at the current batch
- * (the algorithmic-bytes figure of DESIGN.md, used for the roofline line in bench.py). */
+ * (the algorithmic-bytes figure used for the roofline line in bench.py). */
 int64_t b200_mimi_algorithmic_bytes(b200_mimi* h);
 
 /* ------------------------------------------------------------------------------------------ */
@@ -270,7 +270,7 @@ const char* b200_lm_flag_text(int flags);
 /* B200_ERR_CUDA, once, if a finished step raised B200_FLAG_WAIT since it was last reported; reads a word of host memory, no synchronisation.
  * Every step asks this first. */
 int b200_lm_check_waits(b200_lm* h);
-/* Algorithmic HBM bytes of one step at the current batch and ring fill (DESIGN.md): weights once
+/* Algorithmic HBM bytes of one step at the current batch and ring fill: weights once
  * + per-row KV read/append + embeddings + logits. */
 int64_t b200_lm_algorithmic_bytes(b200_lm* h, int kv_fill);
 /* Test/bench helper: declare that every row already holds `fill` steps of history (positions and
@@ -282,7 +282,7 @@ int b200_lm_assume_fill(b200_lm* h, int fill);
 int b200_lm_set_graph(b200_lm* h, int enable);
 /* Storage type of the temporal KV rings, chosen before b200_lm_streaming_begin.  B200_KV_BF16 (default) is the
  * reference's ring (RingKVCache, transformer.py:196-288: 1.573 GB per session at context 3000).  B200_KV_FP8_E4M3 is
- * an opt-in extension outside the reference's numerics (SURVEY.md 8f item 3): e4m3 bytes plus one fp32 scale per
+ * an opt-in extension outside the reference's numerics: e4m3 bytes plus one fp32 scale per
  * (session, head, slot), 0.811 GB per session; its logit error is reported by tests/test_gpu_zv_kv_q8.py. */
 #define B200_KV_BF16 0
 #define B200_KV_FP8_E4M3 1
@@ -291,7 +291,7 @@ int b200_lm_set_kv_dtype(b200_lm* h, int kv_dtype);
 /* Slots per temporal KV ring, chosen before b200_lm_streaming_begin (0 or >= context: the reference's ring of `context` slots,
  * RingKVCache transformer.py:196-288).  A shorter ring holds the same keys as the reference's for a session's first `slots`
  * frames (nothing is evicted before position `context`), at slots/context of the 1.573 GB per session: a pool of young sessions
- * (SURVEY.md 8f item 3, "rings sized to live fill").  A row that steps past the capacity raises B200_FLAG_KV_CAPACITY; the
+ * ("rings sized to live fill").  A row that steps past the capacity raises B200_FLAG_KV_CAPACITY; the
  * caller moves such a session to a full-size handle (get / set streaming state) before that. */
 int b200_lm_set_kv_capacity(b200_lm* h, int slots);
 

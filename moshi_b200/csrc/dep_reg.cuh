@@ -5,11 +5,12 @@
 // phases, and a phase is a grid barrier, one L2 round trip for the activations, a few products and one exchange inside the CTA:
 //   * a product's 16-row groups are dealt to the CTAs whole; the eight warps of a CTA share a group's k and add their sums in shared memory,
 //     so no partial sum leaves an SM (dep_fused_kernel exchanges split-K partials through L2 and needs a phase of its own to add them);
-//   * every thread holds its weights of the NEXT product in registers before it enters the barrier;
+//   * every thread asks for its weights of the NEXT product before it enters the barrier.  They are meant for registers, but 255 do not hold all that
+//     is live across the sampler and the long product: with one block of 8 sessions 158 words per thread go through local memory, with two 317;
 //   * RMSNorm is repeated by every CTA on its way to shared memory (B rows of 2 KB), residual, gating and bf16 roundings sit in the epilogues.
 //
-// Frame of 1 session 2.0 (as a chain of launches) -> 1.35 ms, 8 sessions 2.6 (dep_fused_kernel) -> 1.39, 16 sessions 2.7 -> 2.0: 264 barriers of
-// about 5 us, of which the release of the epilogue's stores, the counter and the poll take half.
+// Frame of 1 session 2.0 (as a chain of launches) -> 1.35 ms, 8 sessions 2.6 (dep_fused_kernel) -> 1.39, 16 sessions 2.7 -> 1.8 (1.48 and 1.98 for 1
+// and 16 with sampling): 8 x (2 + 5 x 6) = 256 barriers of about 5 us, of which the release of the epilogue's stores, the counter and the poll take half.
 //
 // A barrier that is not met within ten seconds ends the kernel; the frame's remaining tokens are then the frame's before.  It raises ERR_WAIT, and a
 // word on the host that the handle's next call looks at without a synchronisation.

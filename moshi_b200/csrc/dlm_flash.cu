@@ -7,7 +7,8 @@
 // shared memory.  O is rescaled only when a row's maximum grew by more than 8 in base 2: a weight of up to 256 has
 // the relative error of one below 1, and the final division refers to the same maximum.  The longest tiles start first.
 //
-// Bound by the tensor pipe and, level with it, by 128 exponentials per thread and tile (about 2100 cycles each).
+// A key tile takes about 3800 cycles, of which the tensor pipe and the exponentials' unit are each active a good quarter (2048 tokens, 16 heads): the bound is
+// the chain of the four softmax warps, one per scheduler, whose latencies nothing hides; then the second wave (256 CTAs on 148 SMs).
 // A wait that lasts longer than ten seconds raises the caller's error flag and the kernel winds down.
 #include "dlm_flash.cuh"
 

@@ -34,7 +34,6 @@ using namespace tcp;
 constexpr int BK = 64;                       // 128 bytes of K per row and stage
 constexpr int THREADS = 192;                 // warp 0 producer, warp 1 MMA, warps 2-5 epilogue
 constexpr int MAX_ST = 8;
-constexpr uint32_t A_STAGE = 128 * BK * 2;
 
 struct WideP {
   int M, N, num_kb, stages, mt, nt, packed, act;      // mt x nt tiles (mt: of the table with a grouped product)

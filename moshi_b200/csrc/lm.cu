@@ -673,8 +673,8 @@ int b200_lm_streaming_begin(b200_lm* h, int batch, void* stream) {
     B200_TRY(A.alloc_t(&h->xq, (size_t)MB * kmax, false));
     B200_TRY(A.alloc_t(&h->xq_scale, (size_t)MB, false));
   }
-  // One or two sessions: the depformer's linears take the GEMV path and the PDL-chained launches beat the persistent kernel
-  // (B=1: 5.5 vs 6.4 ms per LM step, B=2: 6.2 vs 7.1; profiles/r01_r_*).  B200_DEP_FUSED=2 forces the kernel at any batch.
+  // One or two sessions of a shape that dep_reg.cuh does not take: the linears take the GEMV path, and the PDL-chained launches beat the
+  // shared-memory kernel (B=1: 5.5 vs 6.4 ms per LM step, B=2: 6.2 vs 7.1; profiles/r01_r_*).  B200_DEP_FUSED=2 forces the kernel at any batch.
   // Under classifier-free guidance the two halves of the batch meet before every sampler (lm.py:828-833): launch chain.
   tc::DepFusedConfig few;
   memset(&few, 0, sizeof(few));

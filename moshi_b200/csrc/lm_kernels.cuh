@@ -1,6 +1,6 @@
 // bf16 kernels of the Moshi LM decode step (one 12.5 Hz frame for B concurrent sessions).
 //
-// Cast points follow the reference exactly (SURVEY.md appendix B): every nn.Linear output is a bf16
+// Cast points follow the reference exactly: every nn.Linear output is a bf16
 // tensor, RMSNorm / RoPE / softmax / SiLU are evaluated in fp32 on bf16 inputs and rounded once,
 // residual adds and the 17-way embedding sum are bf16 adds.
 #pragma once
@@ -527,7 +527,7 @@ static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const Att
 }
 
 // ---------------------------------------------------------------------------------------------
-// Opt-in 8-bit KV rings (SURVEY.md 8f item 3; NOT the reference's numerics): the same fused step as attn_step_kernel
+// Opt-in 8-bit KV rings (NOT the reference's numerics): the same fused step as attn_step_kernel
 // over rings of one byte per element with one fp32 scale per (session, head, slot).  Halves the ring (0.81 GB instead
 // of 1.57 GB per session at context 3000), i.e. doubles the sessions a GPU can hold.  Two encodings of a row x[128]:
 //   KV_E4M3: e4m3(x * 448 / absmax), scale = absmax / 448   (keeps relative precision under outlier channels)

@@ -1042,8 +1042,9 @@ int b200_mimi_streaming_begin(b200_mimi* h, int batch, void* stream) {
   // transformers
   const int H = c.tr_num_heads, D = d / H, ff = c.tr_dim_feedforward;
   const size_t ntok = (size_t)B * T;
-  // encode + decode of a frame on these kernels against mimi_tc_kernel: 1 session 0.77 / 1.49 ms, 8 sessions 1.19 / 1.55, 24 sessions 1.51 / 1.71,
-  // 40 sessions (80 tokens) 1.99 both, 64 sessions 2.39 / 2.19: a product over 80 tokens is worth the tensor cores' two launches
+  // encode + decode of a frame on these kernels against mimi_tc_kernel: 1 session 0.71 / 1.43 ms, 8 sessions 1.15 / 1.51, 24 sessions 1.43 / 1.66,
+  // 32 sessions (64 tokens) 1.62 / 1.74.  Before mimi_tc_kernel had sixteen epilogue warps the two met at 40 sessions (1.99 ms; 1.85 there now):
+  // a product over 80 tokens is worth the tensor cores' two launches
   h->tr_cuda_cores = (int)ntok <= 64 && D == 64 && d == 512 && T <= 4 && lin_takes(3 * d, d) && lin_takes(d, ff) && lin_takes(ff, d);
   B200_TRY(A.alloc_t(&h->tr_xn_hi, ntok * d));
   B200_TRY(A.alloc_t(&h->tr_xn_lo, ntok * d));

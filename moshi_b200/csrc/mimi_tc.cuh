@@ -17,7 +17,7 @@
 //     epilogue), likewise for the weights at load; the product is a_hi*w_hi + a_hi*w_lo + a_lo*w_hi with fp32 accumulation
 //     in TMEM (dropped terms <= 2^-22 relative).  The RVQ indices downstream stay exact up to the margin the parity tests
 //     define (tests/util.py).
-//   * Warp roles (192 threads): warp 0 = TMA producer (A hi + A lo boxes, one contiguous bulk copy of the pre-tiled weight
+//   * Warp roles (576 threads): warp 0 = TMA producer (A hi + A lo boxes, one contiguous bulk copy of the pre-tiled weight
 //     pair per k-block), warp 1 = TMEM owner + single-thread MMA issuer, warps 2-17 = epilogue (TMEM lane = GEMM row = one
 //     token: bias, residual, ELU / GELU / layer-scale, hi/lo split, 64-byte contiguous stores).  Persistent grid, two TMEM
 //     accumulator stages: the epilogue of a tile overlaps the MMAs of the next.  Deep-and-skinny layers are cut along K into

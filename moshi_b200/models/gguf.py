@@ -1,5 +1,5 @@
 """GGUF checkpoints (the quantised form the Rust stack loads: ``rust/moshi-core/src/nn.rs:9-116``, candle's
-``quantized_var_builder::VarBuilder::from_gguf``; SURVEY.md 8f item 4).
+``quantized_var_builder::VarBuilder::from_gguf``).
 
 Reads GGUF v2 / v3 files with ``F32``, ``F16``, ``BF16`` and ``Q8_0`` tensors (ggml ``block_q8_0``: 32 weights as one fp16 scale
 ``d`` followed by 32 int8, value = ``d * q``; rows are whole numbers of blocks).  A ``Q8_0`` tensor is *dequantised at load* to

@@ -1,4 +1,4 @@
-"""Wire protocol of the dialogue servers in front of the batched frame service (SURVEY.md 8f items 1 and 4).
+"""Wire protocol of the dialogue servers in front of the batched frame service.
 
 Message framing: ``rust/protocol.md`` (one byte message type + payload inside each websocket binary message, little endian);
 per-connection behaviour: ``moshi/moshi/server.py:74-152`` (incoming ``\\x01`` + opus bytes -> PCM -> 1920-sample frames ->
@@ -117,7 +117,7 @@ class Connection:
 
 
 class FrontEnd:
-    """Connections <-> session slots <-> one batched frame step (the in-process session manager of SURVEY.md 8f item 4)."""
+    """Connections <-> session slots <-> one batched frame step (the in-process session manager)."""
 
     def __init__(self, service, batch_size: int, frame_size: int = 1920, tokens_per_slot: int = 9,
                  text_tokenizer=None, model_version: int = 0, codec_factory: tp.Callable[[], tuple] | None = None):

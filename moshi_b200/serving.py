@@ -2,7 +2,7 @@
 
 Dialogue sessions are independent (every state tensor is ``[B, ...]`` and every reduction is per
 row), so N GPUs run N replicas of the weights, each owning a contiguous shard of the session slots;
-there is no data-path collective (SURVEY.md 8e; the reference deploys one process per GPU behind a
+there is no data-path collective (the reference deploys one process per GPU behind a
 load balancer, ``swarm-config.yml:48-63``).  ``torch.distributed`` is used only to launch one
 process per GPU and to reduce timings / counts in the benchmark.
 """
@@ -62,7 +62,7 @@ def barrier() -> None:
 
 
 # ---------------------------------------------------------------------------------------------------
-# One frame for every session slot of this GPU (SURVEY.md 8f item 1: the caller's per-frame plumbing)
+# One frame for every session slot of this GPU (the caller's per-frame plumbing)
 # ---------------------------------------------------------------------------------------------------
 NODATA, ACTIVE, RESET = 0, -1, -2      # UpdateFlags of rust/moshi-server/batched_asr.py:23-30
 

@@ -2,8 +2,8 @@
 
 There are no real weights in the build/bench environment (no network), so parity tests, the golden
 fixture generator and both bench arms use these.  Key names and tensor shapes follow what
-``loaders.get_mimi(None)`` / ``LMModel(**cfg)`` produce in the reference (SURVEY.md appendix A;
-``moshi/moshi/models/loaders.py:323-361``, ``lm.py:140-252``), so the same dict loads into the
+``loaders.get_mimi(None)`` / ``LMModel(**cfg)`` produce in the reference
+(``moshi/moshi/models/loaders.py:323-361``, ``lm.py:140-252``), so the same dict loads into the
 reference modules (``load_state_dict``), into the CPU oracle and into the B200 handles.
 
 Values are drawn from a ``torch.Generator`` on the requested device.  Parity work always draws on
@@ -160,7 +160,7 @@ def synth_mimi_state_dict(cfg: MimiConfig | None = None, seed: int = 1234,
 # ----------------------------------------------------------------------------------------------
 
 def lm_tensor_specs(cfg: LMConfig) -> list[tuple[str, tuple[int, ...], float]]:
-    """(key, shape, fan_in) for every tensor of ``LMModel(**cfg)`` (SURVEY.md appendix A)."""
+    """(key, shape, fan_in) for every tensor of ``LMModel(**cfg)``."""
     specs: list[tuple[str, tuple[int, ...], float]] = []
     d, dd = cfg.dim, cfg.depformer_dim
     h, hd = cfg.ffn_hidden, cfg.depformer_ffn_hidden
