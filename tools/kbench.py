@@ -2,9 +2,9 @@
 """Per-kernel micro-benchmarks (CUDA events) of the hot-path kernels through the C ABI.
 
 Every timed launch reads operands that are not L2-resident: weights / KV rings are rotated through
-enough copies to exceed the 126 MB L2.  Prints one JSON object per line; run under gpurun, e.g.
+enough copies to exceed the 126 MB L2.  Prints one JSON object per line, e.g.
 
-    python tools/kbench.py --what gemm,attn,mimi > gpurun_out/kbench.jsonl
+    python tools/kbench.py --what gemm,attn,mimi > kbench.jsonl
 """
 from __future__ import annotations
 

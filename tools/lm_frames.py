@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """A few Moshi 7B `LMGen.step` calls at one batch size (for `ncu` launch lists / captures of the LM's kernels).
 
-    ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file gpurun_out/lm_launches_b1.csv \\
+    ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file lm_launches_b1.csv \\
         python tools/lm_frames.py --B 1 --steps 3 --no-graph
 """
 import argparse

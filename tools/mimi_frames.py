@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """A few Mimi streaming encode + decode frames at one batch size (for `ncu` launch lists / captures of the codec's kernels).
 
-    ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file gpurun_out/mimi_launches.csv \\
+    ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file mimi_launches.csv \\
         python tools/mimi_frames.py --B 104 --frames 3
 """
 import argparse

@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Aggregate an `ncu --metrics gpu__time_duration.sum --csv` launch list into a per-kernel table.
 
-    python tools/ncu_summary.py gpurun_out/launches.csv [--skip N] > profiles/rNN_launches.md
+    python tools/ncu_summary.py launches.csv [--skip N] > profiles/rNN_launches.md
 """
 import collections
 import csv
