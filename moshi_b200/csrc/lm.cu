@@ -709,7 +709,7 @@ int b200_lm_streaming_begin(b200_lm* h, int batch, void* stream) {
     fc.trace = h->dep_trace;
     fc.wait_ns = 0;
     if (const char* e = getenv("B200_DEP_WAIT_NS")) fc.wait_ns = atoll(e);
-    B200_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h->dep_gave_up), sizeof(int), cudaHostAllocMapped));
+    if (!h->dep_gave_up) B200_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h->dep_gave_up), sizeof(int), cudaHostAllocMapped));
     *h->dep_gave_up = 0;
     B200_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&fc.gave_up), h->dep_gave_up, 0));
     fc.logits = h->dep_logits; fc.audio_tokens = h->audio_tokens;
