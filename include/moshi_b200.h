@@ -559,7 +559,7 @@ int64_t b200_dlm_algorithmic_flops(b200_dlm* h, int tokens, int context);
 /* ------------------------------------------------------------------------------------------ */
 
 /* y[M,N] = x[M,K] * w[N,K]^T, bf16 in, fp32 accumulate, bf16 out, on row-major weights: packs them into tiles and runs
- * the LM's linear for this shape (GEMV kernel up to 2 rows, tcgen05 stream-K / whole-tile / cluster split-K kernels above);
+ * the LM's linear for this shape (whole rows per CTA up to 16 rows, tcgen05 stream-K / whole-tile / cluster split-K kernels above);
  * synchronises the stream (test helper).  Reference op: every nn.Linear of the LM (transformer.py:304-305,554-555,588-589). */
 int b200_op_linear_bf16(const void* x_dev, const void* w_dev, void* y_dev, int M, int N, int K, void* stream);
 /* Stream-K tcgen05 GEMM over pre-tiled weights (the LM's linear kernel; csrc/gemm_sk.cu).
@@ -591,8 +591,8 @@ int b200_op_linear_wide(const void* x_dev, const void* w_dev, void* y_dev, int M
  * that interleave gate and value (y has N / 2 columns), 4 erf GELU.  ldy: elements per result row.  Synchronises (test helper). */
 int b200_op_grouped_wide(const void* x_dev, const void* w_dev, void* y_dev, const int32_t* counts_host, int E, int M, int N, int K, int ldy,
                          int act, float limit, void* stream);
-/* Up to how many activation rows the linears take the GEMV path (plain 16-byte loads on the CUDA cores instead of the
- * tensor-core GEMM; csrc/gemm_sk.cu): 0..4, default 2 (or B200_GEMV_MAX_M).  Returns the previous value. */
+/* Up to how many activation rows the linears may take the kernel that gives a CTA whole output rows (csrc/gemm_row.cu) instead of those that cut
+ * K over CTAs: 0..16, default 16 (or B200_ROW_MAX_M).  Returns the previous value. */
 int b200_op_set_gemv_max_rows(int max_rows);
 /* int8 x int8 linear (QLinear, utils/quantize.py:13-40: bitsandbytes row-wise absmax quantisation of weights and
  * activations, int32 accumulation, dequantisation by both row scales / 127^2), on tcgen05 kind::i8.

@@ -12,9 +12,9 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT_DIR = HERE / "_C"
 LIB = OUT_DIR / "libmoshi_b200.so"
-SOURCES = ["common.cu", "mimi.cu", "lm.cu", "ops.cu", "gemm_sk.cu", "gemm_ns.cu", "gemm_reg.cu", "gemm_wide.cu", "dep_fused.cu", "frame.cu", "mimi_tc.cu", "dlm_flash.cu", "dlm.cu"]
+SOURCES = ["common.cu", "mimi.cu", "lm.cu", "ops.cu", "gemm_sk.cu", "gemm_ns.cu", "gemm_reg.cu", "gemm_row.cu", "gemm_wide.cu", "dep_fused.cu", "frame.cu", "mimi_tc.cu", "dlm_flash.cu", "dlm.cu"]
 # the text-only decoder LM alone: its handle, the tcgen05 GEMMs it shares with the Moshi LM, and the common plumbing
-DECODER_SOURCES = ["common.cu", "gemm_sk.cu", "gemm_ns.cu", "gemm_reg.cu", "gemm_wide.cu", "dlm_flash.cu", "dlm.cu"]
+DECODER_SOURCES = ["common.cu", "gemm_sk.cu", "gemm_ns.cu", "gemm_reg.cu", "gemm_row.cu", "gemm_wide.cu", "dlm_flash.cu", "dlm.cu"]
 DECODER_LIB = OUT_DIR / "libmoshi_b200_decoder.so"
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

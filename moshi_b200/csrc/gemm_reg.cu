@@ -1,4 +1,4 @@
-// Linears of 3..32 activation rows with the weights going through registers:  y[M][N] = epi(x[M][K] . w[N][K]^T), same packed tiles, epilogues and
+// Linears of up to 32 activation rows with the weights going through registers:  y[M][N] = epi(x[M][K] . w[N][K]^T), same packed tiles, epilogues and
 // cast points as gemm_sk.cu; bf16, and int8 with int32 sums.
 //
 // With so few rows a linear is a stream of its weights, and what counts is how many bytes of them are under way.  The bulk-copy engine that

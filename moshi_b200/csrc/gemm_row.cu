@@ -1,0 +1,283 @@
+// Linears of 1..16 activation rows:  y[M][N] = epi(x[M][K] . w[N][K]^T), same packed tiles, epilogues and cast points as gemm_sk.cu; bf16, and int8 with int32 sums.
+//
+// A linear of so few rows is a stream of its weights with a start and an end.  A kernel that cuts K over CTAs (gemm_reg.cu) pays for the cut
+// at the end: partial sums written, a fence, an arrival counter, and the last CTA's read of all of them.  Here a CTA owns whole output rows, so
+// nothing leaves an SM but results:
+//   * one CTA of 16 warps per SM; the output rows are dealt in units of 8 (4096 -> 12288: 10.4 a CTA, the fullest has 11), the warps share the k-blocks;
+//   * a warp asks for its weights with cp.async, SLOTS pairs of units x 64 k (2 KB) ahead of the one it multiplies, from before the wait on the preceding
+//     kernel to the last block.  64 KB under way per SM are the full rate of HBM (7 TB/s for a plain stream), 96 KB are slower: the activations' reads queue
+//     behind them.  No registers are held for what is under way;
+//   * a pair of units, or the gate and value rows of one, is the A fragment of mma.sync m16n8k16 (int8 m16n8k32); which k a slot holds does not matter as
+//     long as the activations' fragment agrees, so every thread takes whole 16-byte pieces of the tiles;
+//   * activations of KC k-blocks are in registers; the warps' sums meet in shared memory, as many units at a time as fit;
+//   * every launch asks for more than half of an SM's shared memory.  With two CTAs to an SM an early launch (programmatic dependent launch) puts both of the
+//     next linear's on whichever SM is done first, and the kernel takes as long as that SM: a step of one session 4457 -> 4537 us, and 4107 with one.
+//
+// Bound by HBM, start and end.  7B shapes, cold weights, launched alone, us, before (K cut over CTAs) / now / weights at 6.55 TB/s:
+//   1 row: 4096 -> 12288 24.4 / 20.5 / 15.4, 4096 -> 4096 12.4 / 10.3 / 5.1, gated -> 11264 36.6 / 31.2 / 28.2, 11264 -> 4096 20.5 / 18.5 / 14.1, -> 32000 49.6 / 43.3 / 40.0;
+//   8 rows: 24.1 / 21.2, 12.9 / 10.5, 33.0 / 33.7, 23.1 / 19.6, 52.6 / 45.7; 16 rows: 26.2 / 22.6, 14.5 / 12.4, -, 26.1 / 22.6, 55.4 / 51.3;
+//   1024 -> 3072 8.3 / 6.2, 2816 -> 1024 9.5 / 6.2; int8 4096 -> 12288 19.4 / 16.5, 11264 -> 4096 18.5 / 18.5.
+// Steps of the 7B: 1 session 4470 -> 4014 us, 3: 4610 -> 4223, 8: 4765 -> 4397, 16 with full rings 6980 -> 6560.
+#include "gemm_row.cuh"
+
+#include <algorithm>
+#include <type_traits>
+
+#include "tc_prims.cuh"
+
+namespace b200 {
+namespace tc {
+
+namespace {
+
+using namespace tcp;
+
+constexpr int EPI_STORE = 0, EPI_RESADD = 1, EPI_GATE = 2;
+constexpr int THREADS = 512, WARPS = 16, UNIT = 8;
+constexpr int TILE = 16384, UNIT_BYTES = 1024;   // a tile: 128 rows x 128 bytes of k
+constexpr int SLOTS = 2;                         // pairs of units under way per warp: 64 KB per SM
+constexpr int RING_BYTES = SLOTS * WARPS * 2 * UNIT_BYTES;
+constexpr int RED_BYTES = 128 * 1024;            // the warps' sums of one pass
+constexpr int ONE_PER_SM = 116 * 1024;           // shared memory of which no two fit an SM
+
+struct RowP {
+  int M, out_rows, units, num_kb, subs_pass;     // subs_pass: 8-row pieces (gate and value rows apart) of a pass, even
+  int row_bytes;                                 // bytes of x per row that exist (K elements)
+  const uint8_t* wt;
+  const uint8_t* x; long long ldx;               // bytes
+  __nv_bfloat16* y; long long ldy;
+  const __nv_bfloat16* res; long long ldr;
+  const float *sa, *sw;                          // int8: scales of activation and weight rows
+};
+
+__device__ __forceinline__ float rbf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ uint4 lds16(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_step(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// A piece c of a packed row r lies at position c ^ (r & 7).  Fragment rows are taken as 0, 4, 1, 5, ..: the eight lanes of a 16-byte read phase hold two of
+// them, whose pieces then lie in the two halves of the banks.
+__device__ __forceinline__ int row_of(int g) { return (g >> 1) | ((g & 1) << 2); }
+
+template <int EPI, int NT, bool I8>
+__global__ void __launch_bounds__(THREADS, 1) gemm_row_kernel(const RowP p) {
+  using Acc = typename std::conditional<I8, int, float>::type;
+  constexpr int G = EPI == EPI_GATE ? 1 : 0;     // gated: the tiles of gate and value rows lie behind each other
+  constexpr int KC = NT == 1 ? 4 : 2;            // k-blocks of a warp whose activations are in registers together
+  extern __shared__ __align__(16) uint8_t smem[];
+  Acc* red = reinterpret_cast<Acc*>(smem + RING_BYTES);      // [warp][sub][row of x][8]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, M = p.M;
+  const int u0 = (int)((unsigned)p.units * blockIdx.x / gridDim.x), subs = ((int)((unsigned)p.units * (blockIdx.x + 1) / gridDim.x) - u0) << G;
+  const uint32_t ring = smem_u32(smem) + warp * 2 * UNIT_BYTES, tile_bytes = (uint32_t)p.num_kb << (14 + G), step = (uint32_t)(WARPS * TILE) << G;
+  constexpr uint32_t SLOT = WARPS * 2 * UNIT_BYTES;
+
+  // the stream of this warp: per pass, KC of its k-blocks at a time, and for these every pair of subs, k-block by k-block
+  const int my_kb = (p.num_kb - warp + WARPS - 1) / WARPS;
+  const uint8_t* const w0 = p.wt + (size_t)(u0 >> 4) * tile_bytes + ((uint32_t)(warp * TILE) << G) + lane * 16;
+  const uint8_t* base = my_kb > 0 && subs > 0 ? w0 : nullptr;      // the next k-block asked for (null: none left)
+  int a_pass = 0, a_end = min(p.subs_pass, subs), a_sub = 0, a_j = 0, a_nj = min(KC, my_kb), a_left = my_kb;
+  auto ask = [&](uint32_t at) {
+    if (base) {
+      const uint32_t to = ring + at + lane * 16;
+      const int ua = (u0 & 15) + (a_sub >> G), ub = ua + 1;
+      const uint8_t* s = base + ((ua >> 4) * tile_bytes + (ua & 15) * UNIT_BYTES);
+      copy16(to, s);
+      copy16(to + 512, s + 512);
+      if (a_sub + 1 < a_end) {
+        s = G ? s + TILE : base + ((ub >> 4) * tile_bytes + (ub & 15) * UNIT_BYTES);
+        copy16(to + 1024, s);
+        copy16(to + 1536, s + 512);
+      }
+      base += step;
+      if (++a_j == a_nj) {
+        a_j = 0;
+        a_sub += 2;
+        if (a_sub < a_end) base -= a_nj * step;
+        else {
+          a_left -= a_nj;
+          if (a_left == 0) {                     // the next pass
+            a_pass = a_end;
+            a_end = min(a_end + p.subs_pass, subs);
+            a_left = my_kb;
+            base = a_pass < subs ? w0 : nullptr;
+          }
+          a_nj = min(KC, a_left);
+          a_sub = a_pass;
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll 1
+  for (int s = 0; s < SLOTS; ++s) ask((uint32_t)s * SLOT);
+  uint32_t slot = 0;
+  pdl_trigger();
+  pdl_wait();
+
+  for (int pass = 0; pass < subs; pass += p.subs_pass) {
+    const int n = min(p.subs_pass, subs - pass);
+    Acc* mine = red + (warp * n * M + 2 * t) * 8 + row_of(g);
+#pragma unroll 1
+    for (int kb0 = warp; kb0 == warp || kb0 < p.num_kb; kb0 += WARPS * KC) {      // once at least: a warp without a k-block stores zeros
+      uint4 xb[KC][NT][2];
+#pragma unroll
+      for (int i = 0; i < KC; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int k = (kb0 + i * WARPS) * 128 + h * 64 + t * 16;
+            xb[i][j][h] = 8 * j + g < M && k < p.row_bytes ? __ldcg(reinterpret_cast<const uint4*>(p.x + (8 * j + g) * p.ldx + k)) : make_uint4(0u, 0u, 0u, 0u);
+          }
+#pragma unroll 1
+      for (int sub = 0; sub < n; sub += 2) {
+        Acc acc[NT][4];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0;
+#pragma unroll
+        for (int i = 0; i < KC; ++i) {
+          if (kb0 + i * WARPS >= p.num_kb) break;
+          const uint32_t row = ring + slot + row_of(g) * 128, c = (uint32_t)(t ^ row_of(g)) << 4;
+          asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS - 1) : "memory");
+          __syncwarp();
+          const uint4 a[2] = {lds16(row + c), lds16(row + (c ^ 64))}, b[2] = {lds16(row + 1024 + c), lds16(row + 1024 + (c ^ 64))};
+          __syncwarp();
+          ask(slot);
+          slot = slot + SLOT == SLOTS * SLOT ? 0u : slot + SLOT;
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              mma_step(acc[j], a[h].x, b[h].x, a[h].y, b[h].y, xb[i][j][h].x, xb[i][j][h].y);
+              mma_step(acc[j], a[h].z, b[h].z, a[h].w, b[h].w, xb[i][j][h].z, xb[i][j][h].w);
+            }
+        }
+        // rows g of either sub; the second of a last odd pair is whatever its slot held before, and is not stored
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (8 * j + 2 * t + (e & 1) < M && sub + (e >> 1) < n) {
+              Acc* o = mine + ((sub + (e >> 1)) * M + 8 * j + (e & 1)) * 8;
+              *o = kb0 == warp ? acc[j][e] : *o + acc[j][e];
+            }
+      }
+    }
+    __syncthreads();
+    // results of the pass: the warps' sums in warp order
+    const int rows = (n >> G) * UNIT, first = (u0 + (pass >> G)) * UNIT;
+    for (int i = tid; i < rows * M; i += THREADS) {
+      const int m = i / rows, r = i - m * rows, o = first + r;
+      if (o >= p.out_rows) continue;
+      Acc v[2] = {0, 0};
+#pragma unroll
+      for (int a = 0; a <= G; ++a)
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) v[a] += red[((w * n + ((r >> 3) << G) + a) * M + m) * 8 + (r & 7)];
+      float f[2] = {(float)v[0], (float)v[1]};
+      if (I8) {                                  // the sums are whole numbers in 32 bits
+        const float s = p.sa[m];
+        f[0] *= s * p.sw[o] * (1.f / 16129.f);
+        if (G) f[1] *= s * p.sw[o + p.out_rows] * (1.f / 16129.f);
+      }
+      float out;
+      if (EPI == EPI_STORE) out = f[0];
+      else if (EPI == EPI_RESADD) out = __bfloat162float(p.res[(long long)m * p.ldr + o]) + rbf16(f[0]);
+      else { const float gt = rbf16(f[0]), u = rbf16(f[1]); out = rbf16(gt / (1.f + expf(-gt))) * u; }
+      p.y[(long long)m * p.ldy + o] = __float2bfloat16_rn(out);
+    }
+    if (pass + p.subs_pass < subs) __syncthreads();
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// 8-row pieces of the fullest CTA, and how many of them a pass takes: as few equal passes as the warps' sums fit, an even number of pieces each
+int subs_at_most(int out_rows, int epi, int sms) {
+  const int units = (out_rows + UNIT - 1) / UNIT, grid = std::min(sms, units);
+  return ((units + grid - 1) / grid) << (epi == EPI_GATE ? 1 : 0);
+}
+int pass_of(int M, int most) {
+  const int fit = RED_BYTES / (WARPS * M * UNIT * 4) / 2 * 2, passes = (most + fit - 1) / fit;
+  return ((most + passes - 1) / passes + 1) / 2 * 2;
+}
+
+template <int EPI, bool I8>
+cudaError_t launch_nt(const cudaLaunchConfig_t& cfg, const RowP& p) {
+  if (p.M <= 8) return cudaLaunchKernelEx(&cfg, gemm_row_kernel<EPI, 1, I8>, p);
+  return cudaLaunchKernelEx(&cfg, gemm_row_kernel<EPI, 2, I8>, p);
+}
+template <int EPI, bool I8>
+cudaError_t allow_smem() {
+  const int most = RING_BYTES + RED_BYTES;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_row_kernel<EPI, 1, I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_row_kernel<EPI, 2, I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
+}  // namespace
+
+// Everything but 16-bit gated pairs
+//   * of so many rows that their sums need a second pass, which reads the activations again (4096 -> 11264, us, register kernel / this one: 12 rows, one
+//     pass 36.3 / 34.9; 16 rows, two passes 36.3 / 37.1);
+//   * of 3 to 8 rows launched by themselves (6 rows 32.4 / 32.8, 8 rows 33.0 / 33.7).  Launched early, behind the linear in front, this one is ahead there too (a
+//     step of 3 sessions 4305 / 4223 us, of 8 4461 / 4397).
+bool row_wins(int M, int N, int epi, int gate_rows, bool i8, int sms, int pdl) {
+  if (M > ROW_MAX_M) return false;
+  if (epi != EPI_GATE || i8) return true;
+  const int most = subs_at_most(gate_rows, epi, sms);
+  return pass_of(M, most) >= most && (pdl || M <= 2 || M > 8);
+}
+
+bool row_supported(int M, int K, bool i8, const void* x, long long ldx_bytes) {
+  return M >= 1 && M <= ROW_MAX_M && K % (i8 ? 16 : 8) == 0 && ldx_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+}
+
+int row_linear(const void* x, long long ldx_bytes, const void* w_tiles, __nv_bfloat16* y, long long ldy, const __nv_bfloat16* res, long long ldr, int M, int N,
+               int K, int epi, int gate_rows, const float* sa, const float* sw, int sms, int pdl, cudaStream_t stream) {
+  const bool i8 = sa != nullptr;
+  if (!row_supported(M, K, i8, x, ldx_bytes)) B200_FAIL(B200_ERR_SHAPE, "row GEMM: unsupported shape M=%d K=%d", M, K);
+  static const cudaError_t once = [] {
+    cudaError_t e = allow_smem<EPI_STORE, false>();
+    if (e == cudaSuccess) e = allow_smem<EPI_RESADD, false>();
+    if (e == cudaSuccess) e = allow_smem<EPI_GATE, false>();
+    if (e == cudaSuccess) e = allow_smem<EPI_STORE, true>();
+    if (e == cudaSuccess) e = allow_smem<EPI_RESADD, true>();
+    return e == cudaSuccess ? allow_smem<EPI_GATE, true>() : e;
+  }();
+  B200_CUDA(once);
+  RowP p;
+  p.M = M; p.out_rows = epi == EPI_GATE ? gate_rows : N;
+  p.units = (p.out_rows + UNIT - 1) / UNIT;
+  p.row_bytes = K * (i8 ? 1 : 2);
+  p.num_kb = (p.row_bytes + 127) / 128;
+  p.wt = static_cast<const uint8_t*>(w_tiles); p.x = static_cast<const uint8_t*>(x); p.ldx = ldx_bytes;
+  p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr; p.sa = sa; p.sw = sw;
+  const int grid = std::min(sms, p.units), most = subs_at_most(p.out_rows, epi, sms);
+  p.subs_pass = pass_of(M, most);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(THREADS); cfg.stream = stream;
+  cfg.dynamicSmemBytes = std::max<size_t>(ONE_PER_SM, RING_BYTES + (size_t)WARPS * std::min(p.subs_pass, most) * M * UNIT * 4);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
+  cudaError_t e;
+  if (i8) e = epi == EPI_STORE ? launch_nt<EPI_STORE, true>(cfg, p) : epi == EPI_RESADD ? launch_nt<EPI_RESADD, true>(cfg, p) : launch_nt<EPI_GATE, true>(cfg, p);
+  else e = epi == EPI_STORE ? launch_nt<EPI_STORE, false>(cfg, p) : epi == EPI_RESADD ? launch_nt<EPI_RESADD, false>(cfg, p) : launch_nt<EPI_GATE, false>(cfg, p);
+  if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "gemm_row launch failed: %s", cudaGetErrorString(e));
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return check_launch("gemm_row");
+}
+
+}  // namespace tc
+}  // namespace b200

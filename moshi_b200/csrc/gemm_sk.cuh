@@ -46,12 +46,9 @@ struct SkTuning {
   const void* xq = nullptr; const float* sa = nullptr; const float* sw = nullptr;
   int pdl = 0;           // launch with programmatic stream serialization (the kernel waits on its own)
   int ns = 0;            // 33..256 sessions: 0 = the non-swapped kernel (gemm_ns.cu) unless B200_GEMM_NS=0, -1 = never, 1 = always (tests)
-  // GEMV path only (M <= sk_gemv_max_m()): x is the residual stream and the linear's input is rmsnorm(x, norm_alpha)
-  const __nv_bfloat16* norm_alpha = nullptr;
 };
 int sk_num_sms();
-int sk_gemv_max_m();
-int sk_set_gemv_max_m(int max_m);      // rows up to which the GEMV path is taken (0..4); returns the previous value
+int sk_set_row_max_m(int max_m);       // rows up to which gemm_row.cu is considered (0..16); returns the previous value
 bool sk_supported(int M, int N, int K, int epi);
 size_t sk_packed_bytes(int N, int K, int epi, int gate_rows);
 int sk_pack_weights(const __nv_bfloat16* w, void* out, int N, int K, int epi, int gate_rows, cudaStream_t stream);

@@ -82,7 +82,6 @@ struct b200_lm {
   int* attn_counters = nullptr;                // split arrival counters [B*H]
   tc::DepFused* depf = nullptr;                // the depformer of a frame as one persistent kernel (B200_DEP_FUSED=0: off)
   int dep_fused = 1;
-  int fuse_norm = 1;                           // B200_FUSE_NORM=0: keep rmsnorm_kernel in front of the GEMV path too (diagnostics)
   int kv_cap = 0;                              // b200_lm_set_kv_capacity: slots per ring (0 = cfg.context, the reference's ring)
   int kv_fp8 = 0;                              // b200_lm_set_kv_dtype / B200_KV_DTYPE: opt-in 8-bit KV ring (B200_KV_FP8_E4M3 or B200_KV_INT8; 0 = bf16)
   float *dep_part0 = nullptr, *dep_part1 = nullptr;
@@ -134,12 +133,10 @@ int noise_per_row(const b200_lm* h) {
 
 // y[M][N] = epi(x[M][K] . w[N][K]^T); `w` is the packed-tile form of gemm_sk.cu.
 int linear(b200_lm* h, const bf16* x, long long ldx, const bf16* w, bf16* y, long long ldy, const bf16* res,
-           long long ldr, int M, int N, int K, int epi, int gate_rows, const float* w_scales = nullptr,
-           const bf16* norm_alpha = nullptr) {
+           long long ldr, int M, int N, int K, int epi, int gate_rows, const float* w_scales = nullptr) {
   tc::SkTuning t;
   t.pdl = h->pdl;
   t.smem_budget = h->sk_smem;
-  t.norm_alpha = norm_alpha;
   if (h->cfg.quantize) {       // QLinear.forward (utils/quantize.py:22-40): row-wise int8 activations, int8 x int8 -> int32
     if (!w_scales) B200_FAIL(B200_ERR_STATE, "quantised LM: linear without weight scales");
     B200_TRY(tc::sk_quantize_rows(x, ldx, h->xq, h->xq_scale, M, K, h->body, h->pdl));
@@ -148,12 +145,10 @@ int linear(b200_lm* h, const bf16* x, long long ldx, const bf16* w, bf16* y, lon
   return tc::sk_linear(h->plans, x, ldx, w, y, ldy, res, ldr, M, N, K, epi, gate_rows, h->sk_ws, h->sk_counters, t, h->body);
 }
 
-// y = epi(rmsnorm(x, alpha) . w^T).  One or two sessions: the norm is folded into the GEMV's activation staging (one kernel
-// and one dependency less per linear); otherwise rmsnorm_kernel writes xn and the GEMM reads it.
+// y = epi(rmsnorm(x, alpha) . w^T).  (The norm folded into the linear, every CTA summing the squares itself, is slower: 4107 -> 4172 us per step at 2
+// sessions, 4445 -> 4716 at 8.)
 int norm_linear(b200_lm* h, const bf16* x, const bf16* alpha, bf16* xn, const bf16* w, bf16* y, long long ldy, int M, int N, int K,
                 int epi, int gate_rows, const float* w_scales) {
-  if (!h->cfg.quantize && h->fuse_norm && M <= tc::sk_gemv_max_m())
-    return linear(h, x, K, w, y, ldy, nullptr, 0, M, N, K, epi, gate_rows, w_scales, alpha);
   B200_TRY(launch_early_if(h->pdl != 0, rmsnorm_kernel, dim3(M), dim3(256), 0, h->body, x, alpha, xn, K, 1e-8f));
   return linear(h, xn, K, w, y, ldy, nullptr, 0, M, N, K, epi, gate_rows, w_scales);
 }
@@ -373,7 +368,6 @@ int b200_lm_create(const b200_lm_config* cfg, b200_lm** out) {
   if (const char* e = getenv("B200_PDL")) h->pdl = atoi(e) != 0;
   if (const char* e = getenv("B200_SK_SMEM_KB")) h->sk_smem = atoi(e) * 1024;
   if (const char* e = getenv("B200_DEP_FUSED")) h->dep_fused = atoi(e);
-  if (const char* e = getenv("B200_FUSE_NORM")) h->fuse_norm = atoi(e) != 0;
   if (const char* e = getenv("B200_KV_DTYPE")) {
     const std::string v = e;
     h->kv_fp8 = (v == "fp8" || v == "fp8_e4m3") ? B200_KV_FP8_E4M3 : v == "int8" ? B200_KV_INT8 : 0;
@@ -673,13 +667,13 @@ int b200_lm_streaming_begin(b200_lm* h, int batch, void* stream) {
     B200_TRY(A.alloc_t(&h->xq, (size_t)MB * kmax, false));
     B200_TRY(A.alloc_t(&h->xq_scale, (size_t)MB, false));
   }
-  // One or two sessions of a shape that dep_reg.cuh does not take: the linears take the GEMV path, and the PDL-chained launches beat the
+  // One or two sessions of a shape that dep_reg.cuh does not take: PDL-chained launches beat the
   // shared-memory kernel (B=1: 5.5 vs 6.4 ms per LM step, B=2: 6.2 vs 7.1; profiles/r01_r_*).  B200_DEP_FUSED=2 forces the kernel at any batch.
   // Under classifier-free guidance the two halves of the batch meet before every sampler (lm.py:828-833): launch chain.
   tc::DepFusedConfig few;
   memset(&few, 0, sizeof(few));
   few.B = B; few.dd = dd; few.F = c.depformer_ffn_hidden; few.card = c.card;
-  const bool dep_small = B <= tc::sk_gemv_max_m() && h->dep_fused != 2 && !tc::dep_fused_in_registers(few);
+  const bool dep_small = B <= 2 && h->dep_fused != 2 && !tc::dep_fused_in_registers(few);
   h->depf = nullptr;
   if (c.dep_q > 0 && !cfg && !c.quantize && h->dep_fused && !dep_small && B <= 256 && dd <= 1024 && dd % 64 == 0) {
     tc::DepFusedConfig fc;

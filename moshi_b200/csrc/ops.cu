@@ -97,7 +97,7 @@ int b200_op_linear_reg(const void* x_dev, const void* w_tiles_dev, void* y_dev, 
                         static_cast<cudaStream_t>(stream));
 }
 
-int b200_op_set_gemv_max_rows(int max_rows) { return tc::sk_set_gemv_max_m(max_rows); }
+int b200_op_set_gemv_max_rows(int max_rows) { return tc::sk_set_row_max_m(max_rows); }
 
 int64_t b200_op_packed_bytes_i8(int N, int K, int epi, int gate_rows) { return (int64_t)tc::sk_packed_bytes_i8(N, K, epi, gate_rows); }
 
