@@ -47,6 +47,7 @@ struct NsParams {
   const uint8_t* wt;
   __nv_bfloat16* y; long long ldy;
   const __nv_bfloat16* res; long long ldr;
+  int late;                                      // nothing is read before the wait on the preceding kernel
 };
 
 __device__ __forceinline__ uint32_t ns_map_to_rank(uint32_t local_smem_addr, uint32_t rank) {
@@ -135,6 +136,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tptr_generic;
+  if (p.late) pdl_wait();
   pdl_trigger();
 
   if (warp == 0) {
@@ -413,6 +415,7 @@ int ns_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
     if (r != CUDA_SUCCESS) B200_FAIL(B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) M=%d K=%d ld=%lld", (int)r, M, K, ldx);
     it = cache.maps.emplace(key, mp).first;
   }
+  p.late = pdl != PDL_WEIGHTS_FIRST;
   const size_t smem = (size_t)stages * stage_bytes + 1024 + 16 * MAX_STAGES + 64;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));

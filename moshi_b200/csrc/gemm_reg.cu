@@ -34,6 +34,7 @@ struct RegP {
   __nv_bfloat16* y; long long ldy;
   const __nv_bfloat16* res; long long ldr;
   const float *sa, *sw;                   // int8: scales of activation and weight rows
+  int late;                               // nothing is read before the wait on the preceding kernel
   float* ws; int* counters;               // partial sums [tile][split][A][8 NT][128], arrivals per tile
 };
 
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gemm_reg_kernel(const Re
   // piece c of row r lies at position c ^ (r & 7) of the row; rows g and g + 8 of the warp's 16 share r & 7 = g
   const uint4* wrow = p.wt + ((size_t)tile * p.num_kb + kb0) * (A * TILE16) + (warp * 16 + g) * 8;
   const int c0 = t ^ g, c1 = (t + 4) ^ g;
+  if (p.late) pdl_wait();
   uint4 w[DEPTH][A][4];
   auto load_w = [&](int i, uint4 (&d)[A][4]) {
     const uint4* s = wrow + (size_t)i * (A * TILE16);
@@ -244,6 +246,7 @@ int reg_linear(const void* x, long long ldx_bytes, const void* w_tiles, __nv_bfl
   }
   p.kbps = (p.num_kb + best - 1) / best;
   p.S = (p.num_kb + p.kbps - 1) / p.kbps;
+  p.late = pdl != PDL_WEIGHTS_FIRST;
   p.wt = static_cast<const uint4*>(w_tiles); p.x = static_cast<const uint8_t*>(x); p.ldx = ldx_bytes;
   p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr; p.sa = sa; p.sw = sw; p.ws = ws; p.counters = counters;
   cudaLaunchConfig_t cfg;

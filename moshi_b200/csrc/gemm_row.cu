@@ -43,6 +43,7 @@ constexpr int ONE_PER_SM = 116 * 1024;           // shared memory of which no tw
 struct RowP {
   int M, out_rows, units, num_kb, subs_pass;     // subs_pass: 8-row pieces (gate and value rows apart) of a pass, even
   int row_bytes;                                 // bytes of x per row that exist (K elements)
+  int late;                                      // nothing is read before the wait on the preceding kernel
   const uint8_t* wt;
   const uint8_t* x; long long ldx;               // bytes
   __nv_bfloat16* y; long long ldy;
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_row_kernel(const RowP p) {
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  if (p.late) pdl_wait();
 #pragma unroll 1
   for (int s = 0; s < SLOTS; ++s) ask((uint32_t)s * SLOT);
   uint32_t slot = 0;
@@ -234,7 +236,7 @@ bool row_wins(int M, int N, int epi, int gate_rows, bool i8, int sms, int pdl) {
   if (M > ROW_MAX_M) return false;
   if (epi != EPI_GATE || i8) return true;
   const int most = subs_at_most(gate_rows, epi, sms);
-  return pass_of(M, most) >= most && (pdl || M <= 2 || M > 8);
+  return pass_of(M, most) >= most && (pdl == PDL_WEIGHTS_FIRST || M <= 2 || M > 8);
 }
 
 bool row_supported(int M, int K, bool i8, const void* x, long long ldx_bytes) {
@@ -258,6 +260,7 @@ int row_linear(const void* x, long long ldx_bytes, const void* w_tiles, __nv_bfl
   p.M = M; p.out_rows = epi == EPI_GATE ? gate_rows : N;
   p.units = (p.out_rows + UNIT - 1) / UNIT;
   p.row_bytes = K * (i8 ? 1 : 2);
+  p.late = pdl != PDL_WEIGHTS_FIRST;
   p.num_kb = (p.row_bytes + 127) / 128;
   p.wt = static_cast<const uint8_t*>(w_tiles); p.x = static_cast<const uint8_t*>(x); p.ldx = ldx_bytes;
   p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr; p.sa = sa; p.sw = sw;

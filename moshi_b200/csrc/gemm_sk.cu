@@ -43,6 +43,7 @@ struct SkParams {
   // int8 x int8 -> int32 (QLinear, utils/quantize.py:13-40): activations / weights are row-wise absmax int8, the
   // accumulator is dequantised as acc * sa[m] * sw[n] / 127^2; whole tiles only (exact integer sums)
   int i8; const float* sa; const float* sw;
+  int late;                     // nothing is read before the wait on the preceding kernel
 };
 
 using namespace tcp;
@@ -144,6 +145,7 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmap_x, const SkParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tptr_generic;
+  if (p.late) pdl_wait();
   pdl_trigger();
 
   if (warp == 0) {
@@ -369,6 +371,7 @@ struct CkParams {
   const __nv_bfloat16* res; long long ldr;
   uint32_t tmem_cols, stage_bytes;
   int i8; const float* sa; const float* sw;      // int8 operands: partials are exact int32, scaled once after the reduction
+  int late;                                      // nothing is read before the wait on the preceding kernel
 };
 
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t local_smem_addr, uint32_t rank) {
@@ -417,6 +420,7 @@ gemm_ck_kernel(const __grid_constant__ CUtensorMap tmap_x, const CkParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tptr_generic;
+  if (p.late) pdl_wait();
   pdl_trigger();
 
   if (warp == 0) {
@@ -893,7 +897,7 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
         p.num_kb = num_kb; p.kb_per = (num_kb + cs - 1) / cs;
         p.wt = static_cast<const uint8_t*>(w_tiles);
         p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr;
-        p.i8 = i8 ? 1 : 0; p.sa = tune.sa; p.sw = tune.sw;
+        p.i8 = i8 ? 1 : 0; p.sa = tune.sa; p.sw = tune.sw; p.late = tune.pdl != PDL_WEIGHTS_FIRST;
         p.stage_bytes = (uint32_t)(TILE_BYTES + p.Mpad * BLOCK_K * 2);      // 128 bytes of K per row, bf16 or int8
         const size_t recv_bytes = (size_t)cs * BLOCK_ROWS * (p.Wc + 4) * 4;
         int stages = (int)((200 * 1024 - recv_bytes) / p.stage_bytes);
@@ -933,7 +937,7 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   p.wt = static_cast<const uint8_t*>(w_tiles);
   p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr;
   p.ws = ws; p.counters = counters;
-  p.i8 = i8 ? 1 : 0; p.sa = tune.sa; p.sw = tune.sw;
+  p.i8 = i8 ? 1 : 0; p.sa = tune.sa; p.sw = tune.sw; p.late = tune.pdl != PDL_WEIGHTS_FIRST;
   p.num_kb = i8 ? (K + 127) / 128 : (K + BLOCK_K - 1) / BLOCK_K;      // a k-block is 128 bytes of K per row
   p.n_tiles = (p.out_rows + BLOCK_ROWS - 1) / BLOCK_ROWS;
   if (p.n_tiles > 1024) B200_FAIL(B200_ERR_SHAPE, "sk GEMM: more than 1024 row tiles");

@@ -34,6 +34,11 @@ struct GemmPlanCache {
 int prepare_plans(GemmPlanCache& cache);
 
 // ---- stream-K kernel over pre-tiled weights (gemm_sk.cu) --------------------------------------
+// How a linear's launch stands to the kernel in front of it.  PDL_WEIGHTS_FIRST: it may begin while that one drains and asks for its weights at once: for a
+// handle, whose weights were complete long before.  PDL_WAIT_FIRST: the same launch, but nothing is read before the wait: for the entry points
+// on bare pointers, whose weights the kernel in front may be writing.
+enum { PDL_OFF = 0, PDL_WEIGHTS_FIRST = 1, PDL_WAIT_FIRST = 2 };
+
 struct SkTuning {
   int grid = 0;          // CTAs (0 = one per SM)
   int smem_budget = 0;   // bytes of pipeline stages per CTA (0 = 200 KB)
@@ -44,7 +49,7 @@ struct SkTuning {
   int cluster = 0;       // force a cluster size (tests)
   // int8 path (QLinear): row-wise absmax int8 activations [M][K] + their scales, and the weight-row scales [N]
   const void* xq = nullptr; const float* sa = nullptr; const float* sw = nullptr;
-  int pdl = 0;           // launch with programmatic stream serialization (the kernel waits on its own)
+  int pdl = 0;           // early launch (programmatic stream serialization): PDL_* above
   int ns = 0;            // 33..256 sessions: 0 = the non-swapped kernel (gemm_ns.cu) unless B200_GEMM_NS=0, -1 = never, 1 = always (tests)
 };
 int sk_num_sms();

@@ -355,10 +355,12 @@ struct AttnStep {
   float* part; int* counters;                  // [B*H][nsplit][ATT_D + 2], [B*H] (zero between launches)
   const long long* pos; const uint8_t* exec_mask;
   int H, cap, nsplit, min_per; float neg_log_period_2_over_d;      // nsplit: ranges at most; min_per: keys of a range at least
+  int late = 0;                                // nothing is read before the wait on the preceding kernel, which may be writing the ring
 };
 
 template <int ATT_U>       // keys per half-warp per register buffer
 static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const AttnStep a) {
+  if (a.late) pdl_wait();
   pdl_trigger();
   const int bh = blockIdx.x, split = blockIdx.y;
   const int b = bh / a.H, h = bh - b * a.H;
