@@ -155,13 +155,14 @@ __device__ void row_phase(const P& p, int dd, int S, const float* part, int N, b
 }
 
 // x = depformer_in[k](transformer_out) + emb_k(prev)   (lm.py:475-486; token -1 -> zero row, lm_utils.py:103-121)
+template <int WIDTH>
 __device__ void input_rows(const DepParams& p, int k) {
   const long long* prev = k == 0 ? p.text_token : p.audio_tokens + (long long)(k - 1) * p.B;
   const bf16* table = p.tables[k];
   for (int m = blockIdx.x; m < p.B; m += gridDim.x) {
     const long long id = prev[m];
     const bool ok = lm::embed_id_ok(id, k == 0 ? p.text_card : p.card, p.err);
-    for (int j = threadIdx.x; j < p.dd; j += THREADS) {
+    for (int j = threadIdx.x; j < p.dd; j += WIDTH) {
       const float e = ok ? bf2f(table[id * p.dd + j]) : 0.f;
       p.x[(long long)m * p.dd + j] = f2bf(bf2f(p.din[(long long)m * p.din_ld + (long long)k * p.dd + j]) + e);
     }
@@ -406,7 +407,7 @@ dep_fused_kernel(const __grid_constant__ CUtensorMap map_xn, const __grid_consta
   };
   Gemm cur = gemm_at(0, 0, 0);
   for (int k = 0; k < p.dep_q; ++k) {
-    input_rows(p, k);
+    input_rows<THREADS>(p, k);
     row_phase<4>(p, p.dd, 0, nullptr, 0, false, p.n1[0], red);
     grid_sync(p.bar, epoch, p.trace);
     for (int l = 0; l < p.L; ++l) {
@@ -578,14 +579,14 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   if (dep_reg_takes(c, d->grid)) {
     const int nt = c.B <= 8 ? 1 : 2;
     d->reg = dep_reg_pick(nt, c.trace || c.wait_ns > 0);
-    d->smem = dep_reg_smem(nt, c.dd);
+    d->smem = dep_reg_smem(c, d->grid);
     B200_CUDA(cudaFuncSetAttribute(d->reg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem));
   }
   B200_CUDA(cudaFuncSetAttribute(dep_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
   int per_sm = 0, coop = 0, dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
   B200_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-  if (d->reg) B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, d->reg, THREADS, d->smem));
+  if (d->reg) B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, d->reg, REG_THREADS, d->smem));
   else B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dep_fused_kernel, THREADS, d->smem));
   if (!coop || per_sm < 1) {
     dep_fused_destroy(d);
@@ -612,7 +613,7 @@ int dep_fused_launch(DepFused* d, cudaStream_t stream) {
   B200_CUDA(cudaMemsetAsync(d->p.bar, 0, sizeof(unsigned), stream));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)d->grid); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = d->smem; cfg.stream = stream;
+  cfg.gridDim = dim3((unsigned)d->grid); cfg.blockDim = dim3((unsigned)(d->reg ? REG_THREADS : THREADS)); cfg.dynamicSmemBytes = d->smem; cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;

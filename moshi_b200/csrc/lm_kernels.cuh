@@ -884,27 +884,28 @@ static __device__ float block_reduce(float v, bool is_max, float* red) {
   return t;
 }
 
-// One row per call; every thread of a SAMPLE_THREADS-wide CTA must call it (block-wide barriers inside).  No __restrict__ on the logits: the
+// One row per call; every thread of a WIDTH-wide CTA must call it (256 at least) (block-wide barriers inside).  No __restrict__ on the logits: the
 // persistent depformers call this between grid barriers, where other CTAs wrote the row after this one may have cached the line it begins in.
+template <int WIDTH = SAMPLE_THREADS>
 static __device__ void sample_row(const bf16* logits, const float* __restrict__ noise, long long* __restrict__ out,
                                   int card, int use_sampling, float temp, int top_k) {
-  __shared__ float red[SAMPLE_THREADS / 32];
+  __shared__ float red[WIDTH / 32];
   __shared__ unsigned hist[256];
   __shared__ unsigned s_prefix, s_remaining, s_count;
   __shared__ unsigned sel[SAMPLE_MAX_K];
-  __shared__ float s_best[SAMPLE_THREADS / 32];
-  __shared__ int s_brank[SAMPLE_THREADS / 32];
+  __shared__ float s_best[WIDTH / 32];
+  __shared__ int s_brank[WIDTH / 32];
   const int tid = threadIdx.x;
 
   if (!(use_sampling && temp > 0.f)) {        // greedy: argmax, first maximum (sampling.py:102-103)
     unsigned best = 0;
-    for (int i = tid; i < card; i += SAMPLE_THREADS) best = max(best, sample_key(logits, i));
+    for (int i = tid; i < card; i += WIDTH) best = max(best, sample_key(logits, i));
     for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
     if ((tid & 31) == 0) hist[tid >> 5] = best;
     __syncthreads();
     if (tid == 0) {
       unsigned bb = 0;
-      for (int w = 0; w < SAMPLE_THREADS / 32; ++w) bb = max(bb, hist[w]);
+      for (int w = 0; w < WIDTH / 32; ++w) bb = max(bb, hist[w]);
       *out = 0xFFFFu - (bb & 0xFFFFu);
     }
     return;
@@ -912,21 +913,21 @@ static __device__ void sample_row(const bf16* logits, const float* __restrict__ 
   const int k = min(min(top_k, card), SAMPLE_MAX_K);
   // softmax statistics in fp32 on logits / temp
   float mx = -INFINITY;
-  for (int i = tid; i < card; i += SAMPLE_THREADS) mx = fmaxf(mx, bf2f(logits[i]) / temp);
+  for (int i = tid; i < card; i += WIDTH) mx = fmaxf(mx, bf2f(logits[i]) / temp);
   mx = block_reduce(mx, true, red);
   float sum = 0.f;
-  for (int i = tid; i < card; i += SAMPLE_THREADS) sum += expf(bf2f(logits[i]) / temp - mx);
+  for (int i = tid; i < card; i += WIDTH) sum += expf(bf2f(logits[i]) / temp - mx);
   sum = block_reduce(sum, false, red);
 
   // radix select of the k-th largest 32-bit key (keys are unique)
   if (tid == 0) { s_prefix = 0; s_remaining = (unsigned)k; }
   __syncthreads();
   for (int pass = 3; pass >= 0; --pass) {
-    hist[tid] = 0;
+    if (tid < 256) hist[tid] = 0;
     __syncthreads();
     const unsigned prefix = s_prefix;
     const unsigned mask = pass == 3 ? 0u : (0xFFFFFFFFu << ((pass + 1) * 8));
-    for (int i = tid; i < card; i += SAMPLE_THREADS) {
+    for (int i = tid; i < card; i += WIDTH) {
       const unsigned key = sample_key(logits, i);
       if ((key & mask) == prefix) atomicAdd(&hist[(key >> (pass * 8)) & 0xFFu], 1u);
     }
@@ -963,9 +964,9 @@ static __device__ void sample_row(const bf16* logits, const float* __restrict__ 
   // pad the sort buffer
   int p2 = 1;
   while (p2 < k) p2 <<= 1;
-  for (int i = tid; i < p2; i += SAMPLE_THREADS) sel[i] = 0u;
+  for (int i = tid; i < p2; i += WIDTH) sel[i] = 0u;
   __syncthreads();
-  for (int i = tid; i < card; i += SAMPLE_THREADS) {
+  for (int i = tid; i < card; i += WIDTH) {
     const unsigned key = sample_key(logits, i);
     if (key >= thr) {
       const unsigned slot = atomicAdd(&s_count, 1u);
@@ -976,7 +977,7 @@ static __device__ void sample_row(const bf16* logits, const float* __restrict__ 
   // bitonic sort, descending
   for (int size = 2; size <= p2; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = tid; i < p2 / 2; i += SAMPLE_THREADS) {
+      for (int i = tid; i < p2 / 2; i += WIDTH) {
         const int lo = 2 * i - (i & (stride - 1));
         const int hi = lo + stride;
         const bool desc = ((lo & size) == 0);
@@ -989,7 +990,7 @@ static __device__ void sample_row(const bf16* logits, const float* __restrict__ 
   // argmax over ranks of p / q (first maximum wins, like torch.argmax)
   float best = -INFINITY;
   int brank = 0x7fffffff;
-  for (int j = tid; j < k; j += SAMPLE_THREADS) {
+  for (int j = tid; j < k; j += WIDTH) {
     const int idx = 0xFFFF - (int)(sel[j] & 0xFFFFu);
     const float p = expf(bf2f(logits[idx]) / temp - mx) / sum;
     const float s = p / noise[j];
@@ -1003,7 +1004,7 @@ static __device__ void sample_row(const bf16* logits, const float* __restrict__ 
   if ((tid & 31) == 0) { s_best[tid >> 5] = best; s_brank[tid >> 5] = brank; }
   __syncthreads();
   if (tid == 0) {
-    for (int w = 1; w < SAMPLE_THREADS / 32; ++w)
+    for (int w = 1; w < WIDTH / 32; ++w)
       if (s_best[w] > best || (s_best[w] == best && s_brank[w] < brank)) { best = s_best[w]; brank = s_brank[w]; }
     if (brank == 0x7fffffff) brank = 0;
     *out = 0xFFFF - (int)(sel[brank] & 0xFFFFu);
