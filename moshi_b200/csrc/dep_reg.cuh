@@ -11,6 +11,9 @@
 //   * a warp has one k-block of the width, so its share of the RMSNorm is what it multiplies: the sums of squares meet in shared memory; residual, gating
 //     and bf16 roundings sit in the epilogues; old keys and values of the attention are asked for before the barrier.
 //
+// A frame with sampling: 1 session 1.48 ms with the weights in registers -> 1.09, 16 sessions 1.98 -> 1.33: 8 x (2 + 5 x 6) = 256 barriers of 3 to 5 us at one
+// session (in_proj with its norm 4.9 us, attention 2.9, out_proj 2.9, gated input with its norm 5.1, linear_out 4.0), sampling 15.6 us a sub-step.
+//
 // A barrier that is not met within ten seconds ends the kernel; the frame's remaining tokens are then the frame's before.  It raises ERR_WAIT, and a
 // word on the host that the handle's next call looks at without a synchronisation.
 #pragma once

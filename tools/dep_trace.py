@@ -18,7 +18,7 @@ import torch  # noqa: E402
 
 
 def phase_names(dep_q: int, L: int, in_registers: bool) -> list[str]:
-    """Phase that ENDS at barrier e (1-based), in the kernel's order (dep_reg.cuh: few sessions, weights in registers; dep_fused.cu)."""
+    """Phase that ENDS at barrier e (1-based), in the kernel's order (dep_reg.cuh: few sessions; dep_fused.cu)."""
     names = []
     for k in range(dep_q):
         if in_registers:
