@@ -227,16 +227,13 @@ cudaError_t allow_smem() {
 
 }  // namespace
 
-// Everything but 16-bit gated pairs
-//   * of so many rows that their sums need a second pass, which reads the activations again (4096 -> 11264, us, register kernel / this one: 12 rows, one
-//     pass 36.3 / 34.9; 16 rows, two passes 36.3 / 37.1);
-//   * of 3 to 8 rows launched by themselves (6 rows 32.4 / 32.8, 8 rows 33.0 / 33.7).  Launched early, behind the linear in front, this one is ahead there too (a
-//     step of 3 sessions 4305 / 4223 us, of 8 4461 / 4397).
-bool row_wins(int M, int N, int epi, int gate_rows, bool i8, int sms, int pdl) {
+// Everything but 16-bit gated pairs of so many rows that their sums need a second pass, which reads the activations again (4096 -> 11264, us, register
+// kernel / this one: 12 rows, one pass 36.3 / 34.9; 16 rows, two passes 36.3 / 37.1).
+bool row_wins(int M, int epi, int gate_rows, bool i8, int sms) {
   if (M > ROW_MAX_M) return false;
   if (epi != EPI_GATE || i8) return true;
   const int most = subs_at_most(gate_rows, epi, sms);
-  return pass_of(M, most) >= most && (pdl == PDL_WEIGHTS_FIRST || M <= 2 || M > 8);
+  return pass_of(M, most) >= most;
 }
 
 bool row_supported(int M, int K, bool i8, const void* x, long long ldx_bytes) {

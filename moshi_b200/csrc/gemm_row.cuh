@@ -7,7 +7,7 @@ namespace b200 {
 namespace tc {
 
 constexpr int ROW_MAX_M = 16;
-bool row_wins(int M, int N, int epi, int gate_rows, bool i8, int sms, int pdl);
+bool row_wins(int M, int epi, int gate_rows, bool i8, int sms);
 bool row_supported(int M, int K, bool i8, const void* x, long long ldx_bytes);
 // x: bf16 rows, or int8 with the scales of its rows (sa) and of the weight rows (sw); w_tiles as packed for gemm_sk.cu
 int row_linear(const void* x, long long ldx_bytes, const void* w_tiles, __nv_bfloat16* y, long long ldy, const __nv_bfloat16* res, long long ldr, int M, int N,

@@ -870,7 +870,7 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   const void* rows = i8 ? tune.xq : x;
   const long long row_ld = i8 ? (long long)K : 2 * ldx;
   const bool scaled = !i8 || (K % 16 == 0 && tune.sa && tune.sw);
-  if (chosen && scaled && M <= g_row_max_m && row_wins(M, N, epi, gate_rows, i8, g_sms, tune.pdl) && row_supported(M, K, i8, rows, row_ld))
+  if (chosen && scaled && M <= g_row_max_m && row_wins(M, epi, gate_rows, i8, g_sms) && row_supported(M, K, i8, rows, row_ld))
     return row_linear(rows, row_ld, w_tiles, y, ldy, res, ldr, M, N, K, epi, gate_rows, i8 ? tune.sa : nullptr, tune.sw, g_sms, tune.pdl, stream);
   // up to 32 sessions: weights through registers (gemm_reg.cu)
   if (chosen && scaled && M <= REG_MAX_M && reg_wins(M, N, epi, gate_rows, i8, g_sms) && reg_supported(M, epi, rows, row_ld))

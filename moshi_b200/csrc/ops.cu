@@ -25,7 +25,7 @@ static int sk_scratch(float** ws, int** counters, int which = 0) {
 }
 
 // The entry points of a step's kernels are launched early and wait before they read anything (B200_PDL=0: ordinary launches): behind one
-// another the next one's CTAs are set up while the last one drains (us, ordinary / early: gated linear of 6 rows 33.4 / 31.2, 4096 -> 12288 of 104 rows
+// another the next one's CTAs are set up while the last one drains (us, ordinary / early: gated linear of 6 rows in the register kernel 33.4 / 31.2, 4096 -> 12288 of 104 rows
 // 30.8 / 29.1, attention of 48 sessions 159.2 / 157.5).
 static int op_pdl() {
   static const int on = [] { const char* e = getenv("B200_PDL"); return !e || atoi(e) != 0; }();
