@@ -159,6 +159,25 @@ struct DeviceGuard {
   ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
 
+// Raises the limit of dynamic shared memory of kernels.  The limit belongs to a kernel on one device, and a process may drive several: it is set once on each device
+// that is current at a call, and again where it could not be set.  `done`: a static of the caller's, for this group of kernels.
+template <typename... Kernels>
+int allow_smem(std::atomic<uint64_t>& done, int bytes, Kernels*... kernels) {
+  int dev = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_acquire) & bit) return B200_OK;
+  for (const void* k : {reinterpret_cast<const void*>(kernels)...}) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) continue;
+    cudaGetLastError();                          // reported here, and not by the next launch as well
+    set_error("%d bytes of shared memory refused on device %d: %s", bytes, dev, cudaGetErrorString(e));
+    return B200_ERR_CUDA;
+  }
+  done.fetch_or(bit, std::memory_order_release);
+  return B200_OK;
+}
+
 // shared body of b200_{lm,mimi}_state_{count,entry,read,write}
 int state_entry_info(const Arena& a, int index, const char** name, int* dtype, int* ndim, int64_t* shape8, int64_t* nbytes);
 int state_entry_copy(const Arena& a, const char* name, void* dst_dev, const void* src_dev, int64_t nbytes, cudaStream_t st);

@@ -218,12 +218,6 @@ cudaError_t launch_nt(const cudaLaunchConfig_t& cfg, const RowP& p) {
   if (p.M <= 8) return cudaLaunchKernelEx(&cfg, gemm_row_kernel<EPI, 1, I8>, p);
   return cudaLaunchKernelEx(&cfg, gemm_row_kernel<EPI, 2, I8>, p);
 }
-template <int EPI, bool I8>
-cudaError_t allow_smem() {
-  const int most = RING_BYTES + RED_BYTES;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_row_kernel<EPI, 1, I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_row_kernel<EPI, 2, I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-}
 
 }  // namespace
 
@@ -244,15 +238,11 @@ int row_linear(const void* x, long long ldx_bytes, const void* w_tiles, __nv_bfl
                int K, int epi, int gate_rows, const float* sa, const float* sw, int sms, int pdl, cudaStream_t stream) {
   const bool i8 = sa != nullptr;
   if (!row_supported(M, K, i8, x, ldx_bytes)) B200_FAIL(B200_ERR_SHAPE, "row GEMM: unsupported shape M=%d K=%d", M, K);
-  static const cudaError_t once = [] {
-    cudaError_t e = allow_smem<EPI_STORE, false>();
-    if (e == cudaSuccess) e = allow_smem<EPI_RESADD, false>();
-    if (e == cudaSuccess) e = allow_smem<EPI_GATE, false>();
-    if (e == cudaSuccess) e = allow_smem<EPI_STORE, true>();
-    if (e == cudaSuccess) e = allow_smem<EPI_RESADD, true>();
-    return e == cudaSuccess ? allow_smem<EPI_GATE, true>() : e;
-  }();
-  B200_CUDA(once);
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, RING_BYTES + RED_BYTES, gemm_row_kernel<EPI_STORE, 1, false>, gemm_row_kernel<EPI_STORE, 2, false>, gemm_row_kernel<EPI_RESADD, 1, false>,
+                      gemm_row_kernel<EPI_RESADD, 2, false>, gemm_row_kernel<EPI_GATE, 1, false>, gemm_row_kernel<EPI_GATE, 2, false>, gemm_row_kernel<EPI_STORE, 1, true>,
+                      gemm_row_kernel<EPI_STORE, 2, true>, gemm_row_kernel<EPI_RESADD, 1, true>, gemm_row_kernel<EPI_RESADD, 2, true>, gemm_row_kernel<EPI_GATE, 1, true>,
+                      gemm_row_kernel<EPI_GATE, 2, true>));
   RowP p;
   p.M = M; p.out_rows = epi == EPI_GATE ? gate_rows : N;
   p.units = (p.out_rows + UNIT - 1) / UNIT;
