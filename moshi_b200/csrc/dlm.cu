@@ -321,11 +321,8 @@ int projection_with_unit(b200_dlm* h, const Layer& L, const T* hb, T* proj, T* a
 template <typename T, int NCH, int RPW>
 int launch_attn(cudaStream_t st, const AttnParams& p, int tiles, int nsplit) {
   const size_t smem = (size_t)32 * p.r * sizeof(T);
-  static bool attr_set = false;
-  if (!attr_set && smem > 48 * 1024) {
-    B200_CUDA(cudaFuncSetAttribute(latent_attn_kernel<T, NCH, RPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0};
+  if (smem > 48 * 1024) B200_TRY(allow_smem(limits, 200 * 1024, latent_attn_kernel<T, NCH, RPW>));
   B200_LAUNCH((latent_attn_kernel<T, NCH, RPW>), dim3(tiles, nsplit), 128, smem, st, p);
   return check_launch("latent_attn");
 }
@@ -348,11 +345,8 @@ int pick_split(int forced, int tiles, int max_ctx, int rpt, int r, size_t part_f
 template <int NKS>
 int launch_attn_mma(cudaStream_t st, const AttnParams& p, int tiles) {
   const size_t smem = (size_t)2 * 32 * (p.r + 8) * 2 + (size_t)4 * 16 * 32 * 4 + (size_t)16 * 40 * 2 + (size_t)3 * 16 * 4 + 16;      // keys, partial scores, weights, row state, mbarriers
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute(latent_attn_mma_kernel<NKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, 100 * 1024, latent_attn_mma_kernel<NKS>));
   EARLY_LAUNCH(latent_attn_mma_kernel<NKS>, dim3(tiles, p.nsplit), 128, smem, st, p);
   return check_launch("latent_attn_mma");
 }
@@ -799,12 +793,8 @@ int finalize_sandwich_layer(b200_dlm* h, int i, std::vector<void*>& drop) {
 
 template <typename T>
 int small_proj(b200_dlm* h, const T* x, long long ldx, const void* w, const float* b, float* out, int M, int N, int K) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute((small_proj_f32_kernel<T, 1>), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    B200_CUDA(cudaFuncSetAttribute((small_proj_f32_kernel<T, 8>), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, 200 * 1024, (small_proj_f32_kernel<T, 1>), (small_proj_f32_kernel<T, 8>)));
   const int vec = K % 8 == 0 && (ldx * sizeof(T)) % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
   const size_t row = (size_t)K * sizeof(T);
   if (M >= 512 && 8 * row <= 100 * 1024) B200_LAUNCH((small_proj_f32_kernel<T, 8>), dim3(ceil_div(M, 8), ceil_div(N, 32)), 256, 8 * row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
@@ -817,11 +807,8 @@ int launch_scan_r(cudaStream_t st, const ScanParams& p, int n_entries) {
   constexpr int NC = 128 / LPC * CB;
   const dim3 grid(n_entries * p.heads, ceil_div(p.vdim, NC));
   const size_t smem = (size_t)2 * p.stage * (p.prow + NC) * 4;
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute((matrix_memory_scan_kernel<MODE, R, LPC, CB, VL>), cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, 100 * 1024, (matrix_memory_scan_kernel<MODE, R, LPC, CB, VL>)));
   B200_LAUNCH((matrix_memory_scan_kernel<MODE, R, LPC, CB, VL>), grid, 128, smem, st, p);
   return check_launch("matrix_memory_scan");
 }
@@ -939,14 +926,9 @@ int window_attention(b200_dlm* h, const Layer& L, int n_tok, int max_ctx, long l
   const bool one = !mma && h->max_entry_tokens == 1 && L.sig_one >= 0;
   const TileSig& s = h->sigs[mma ? L.sig_mma : one ? L.sig_one : L.sig];
   const int QT = mma ? 16 : one ? 1 : L.QT, KT = mma ? 32 : one ? L.KT_one : L.KT;
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute(window_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    B200_CUDA(cudaFuncSetAttribute(window_attn_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    B200_CUDA(cudaFuncSetAttribute(window_attn_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    B200_CUDA(cudaFuncSetAttribute(window_attn_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0}, limits_mma{0};
+  B200_TRY(allow_smem(limits, 200 * 1024, window_attn_kernel<T>));
+  B200_TRY(allow_smem(limits_mma, 220 * 1024, window_attn_mma_kernel<1>, window_attn_mma_kernel<2>, window_attn_mma_kernel<4>));
   WindowAttnParams p;
   p.q = h->qkv32; p.ldq = ldq > 0 ? ldq : L.Nq + L.Nk + L.Nv; p.kcache = L.kcache; p.vcache = L.vcache; p.mix = L.mixhh; p.sink = L.sink;
   p.tile_row0 = h->meta_dev + s.off_row0; p.tile_rows = h->meta_dev + s.off_rows; p.tile_slot = h->meta_dev + s.off_slot;
@@ -1696,14 +1678,9 @@ int sigmoid_attention(b200_dlm* h, const Layer& L, int n_tok, int max_ctx) {
   const bool one = !mma && h->max_entry_tokens == 1 && L.sig_one >= 0;
   const TileSig& s = h->sigs[mma ? L.sig_mma : one ? L.sig_one : L.sig];
   const int QT = mma ? 16 : one ? 1 : L.QT, KT = mma ? 32 : one ? L.KT_one : L.KT;
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute(sigmoid_attn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    B200_CUDA(cudaFuncSetAttribute((sigmoid_attn_mma_kernel<1, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    B200_CUDA(cudaFuncSetAttribute((sigmoid_attn_mma_kernel<2, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    B200_CUDA(cudaFuncSetAttribute((sigmoid_attn_mma_kernel<4, 8>), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0}, limits_mma{0};
+  B200_TRY(allow_smem(limits, 200 * 1024, sigmoid_attn_kernel<T>));
+  B200_TRY(allow_smem(limits_mma, 220 * 1024, (sigmoid_attn_mma_kernel<1, 16>), (sigmoid_attn_mma_kernel<2, 16>), (sigmoid_attn_mma_kernel<4, 8>)));
   SigmoidAttnParams p;
   p.q = h->qkv32; p.ldq = L.Nq; p.kcache = L.kcache; p.vcache = L.vcache; p.mix = L.mixhh; p.bias = L.pbias;
   p.gate_in = h->small32 + L.s_gate; p.ldg = L.nsmall;
@@ -1755,11 +1732,8 @@ UnitParams unit_params(b200_dlm* h, const Layer& L) {
 
 template <int NM, int VT, bool SK>
 int launch_map_mma(cudaStream_t st, const MapAttnParams& p, size_t smem) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute((map_attn_mma_kernel<NM, VT, SK>), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, 220 * 1024, (map_attn_mma_kernel<NM, VT, SK>)));
   EARLY_LAUNCH_IF(SK, (map_attn_mma_kernel<NM, VT, SK>), dim3(p.n_tiles * p.G, p.nsplit), 128, smem, st, p);
   return check_launch("map_attn_mma");
 }
@@ -1824,11 +1798,8 @@ int map_attention(b200_dlm* h, const Layer& L, int n_tok, int max_ctx) {
   if (mma) {
     if constexpr (sizeof(T) == 2) B200_TRY(one ? (launch_map_mma_vt<NM, true>(st, p, L.mma_vt, L.smem_mma_one)) : (launch_map_mma_vt<NM, false>(st, p, L.mma_vt, L.mma_smem)));
   } else {
-    static bool attr_set = false;
-    if (!attr_set) {
-      B200_CUDA(cudaFuncSetAttribute((map_attn_kernel<T, NM>), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr_set = true;
-    }
+    static std::atomic<uint64_t> limits{0};
+    B200_TRY(allow_smem(limits, 200 * 1024, (map_attn_kernel<T, NM>)));
     B200_LAUNCH((map_attn_kernel<T, NM>), dim3(ctas, nsplit), 256, L.attn_smem, st, p);
     B200_TRY(check_launch("map_attn"));
   }
@@ -1953,11 +1924,8 @@ int routed_experts_glu(b200_dlm* h, const Layer& L, const T* hb, int n_tok) {
   if (silu || gelu) {
     const int n = E + L.c.identity, groups = std::max(L.c.groups, 1);
     const size_t smem = (size_t)4 * (2 * n + groups) * sizeof(float);
-    static bool attr_set = false;
-    if (!attr_set) {
-      B200_CUDA(cudaFuncSetAttribute(moe_route_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr_set = true;
-    }
+    static std::atomic<uint64_t> limits{0};
+    B200_TRY(allow_smem(limits, 200 * 1024, moe_route_grouped_kernel));
     EARLY_LAUNCH_IF(n_tok < EARLY_TOKENS, moe_route_grouped_kernel, ceil_div(n_tok, 4), 128, smem, st, h->small32 + L.s_router, (long long)L.nsmall, L.correction, n, top, groups, L.c.groups_keep,
                 gelu ? 1 : 0, gelu ? 2 : 1, gelu ? 1 : 0, L.c.router_scale, h->moe_idx, h->moe_w, n_tok);
   } else {
@@ -1995,11 +1963,8 @@ template <int R4, bool CHD = false>
 int launch_delta_chunk(cudaStream_t st, const DeltaChunkParams& p, int n_entries) {
   constexpr int C = DELTA_CH, DP = 32 * R4;
   const size_t smem = (size_t)((R4 <= 4 ? 2 : 1) * ((CHD ? 3 : 2) * C * DP + C * 32 + 2 * C + 2 * C * C) + 16 * C * 32 + 3 * C * 32 + 2 * C) * sizeof(float);
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute((delta_chunk_kernel<R4, CHD>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, (int)smem, (delta_chunk_kernel<R4, CHD>)));
   B200_LAUNCH((delta_chunk_kernel<R4, CHD>), dim3(n_entries * p.heads, ceil_div(p.vdim, 32)), 256, smem, st, p);
   return check_launch("delta_chunk");
 }
@@ -2014,11 +1979,8 @@ int delta_chunks(b200_dlm* h, const ScanParams& sp) {
   p.ent_pos0 = h->meta_dev + h->off_whole_pos0;
   p.St = sp.St; p.out = sp.out; p.heads = sp.heads; p.dim = sp.dim; p.vdim = sp.vdim;
   const size_t gsm = (size_t)(2 * DELTA_CH * (sp.dim + 1) + 2 * DELTA_CH + DELTA_CH * DELTA_CH) * sizeof(float);
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute(delta_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((2 * DELTA_CH * 257 + 2 * DELTA_CH + DELTA_CH * DELTA_CH) * sizeof(float))));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, (int)((2 * DELTA_CH * 257 + 2 * DELTA_CH + DELTA_CH * DELTA_CH) * sizeof(float)), delta_gram_kernel));
   B200_LAUNCH(delta_gram_kernel, dim3(h->n_chunks, sp.heads), 256, gsm, h->stream, p);
   B200_TRY(check_launch("delta_gram"));
   const int d = sp.dim;
@@ -2037,11 +1999,8 @@ int chdelta_chunks(b200_dlm* h, const ScanParams& sp) {
   p.ent_pos0 = h->meta_dev + h->off_whole_pos0;
   p.St = sp.St; p.out = sp.out; p.heads = sp.heads; p.dim = sp.dim; p.vdim = sp.vdim;
   const size_t gsm = (size_t)(3 * DELTA_CH * (sp.dim + 1) + DELTA_CH + DELTA_CH * DELTA_CH) * sizeof(float);
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute(chdelta_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((3 * DELTA_CH * 257 + DELTA_CH + DELTA_CH * DELTA_CH) * sizeof(float))));
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, (int)((3 * DELTA_CH * 257 + DELTA_CH + DELTA_CH * DELTA_CH) * sizeof(float)), chdelta_gram_kernel));
   B200_LAUNCH(chdelta_gram_kernel, dim3(h->n_chunks, sp.heads), 256, gsm, h->stream, p);
   B200_TRY(check_launch("chdelta_gram"));
   const int d = sp.dim;

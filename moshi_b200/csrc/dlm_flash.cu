@@ -301,13 +301,8 @@ int flash_attention(const FlashAttn& a, cudaStream_t st) {
   B200_TRY(make_map(&mq, a.q, a.T, (long long)a.H * FLASH_D, a.ldq));
   B200_TRY(make_map(&mk, a.k, ctx, (long long)a.H * FLASH_D, a.ldk));
   B200_TRY(make_map(&mv, a.vt, (long long)a.H * FLASH_D, ctx, a.ldv));
-  int dev = 0;
-  B200_CUDA(cudaGetDevice(&dev));
-  static std::atomic<uint64_t> attr_set{0};             // per device
-  if (!(attr_set.load() >> (dev & 63) & 1)) {
-    B200_CUDA(cudaFuncSetAttribute(flash_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
-    attr_set.fetch_or(1ull << (dev & 63));
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, (int)SMEM, flash_attention_kernel));
   FlashP p;
   p.sink = a.sink; p.out = a.out; p.ldo = a.ldo; p.T = a.T; p.pos0 = a.pos0; p.H = a.H; p.q_tiles = ceil_div(a.T, ROWS); p.scale2 = a.scale * LOG2E; p.err = a.err;
   cudaLaunchConfig_t cfg;

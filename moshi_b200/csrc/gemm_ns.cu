@@ -301,7 +301,6 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn g_ns_encode = nullptr;
-bool g_ns_attr = false;
 int g_ns_sms = 0;
 
 int ns_init() {
@@ -312,15 +311,12 @@ int ns_init() {
     if (!fn || qres != cudaDriverEntryPointSuccess) B200_FAIL(B200_ERR_CUDA, "cuTensorMapEncodeTiled not available");
     g_ns_encode = reinterpret_cast<EncodeTiledFn>(fn);
   }
-  if (!g_ns_attr) {
-    const int max_smem = 220 * 1024;
-    B200_CUDA(cudaFuncSetAttribute(gemm_ns_kernel<EPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    B200_CUDA(cudaFuncSetAttribute(gemm_ns_kernel<EPI_RESADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    B200_CUDA(cudaFuncSetAttribute(gemm_ns_kernel<EPI_GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, 220 * 1024, gemm_ns_kernel<EPI_STORE>, gemm_ns_kernel<EPI_RESADD>, gemm_ns_kernel<EPI_GATE>));
+  if (!g_ns_sms) {
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
     B200_CUDA(cudaDeviceGetAttribute(&g_ns_sms, cudaDevAttrMultiProcessorCount, dev));
-    g_ns_attr = true;
   }
   return B200_OK;
 }

@@ -715,7 +715,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn g_encode = nullptr;
-bool g_attr_set = false;
+bool g_settings_read = false;
 int g_sms = 0;
 int g_row_max_m = ROW_MAX_M;     // B200_ROW_MAX_M (0..16): rows up to which gemm_row_kernel is considered
 int g_use_ns = 1;                // B200_GEMM_NS=0: keep the swap-AB kernels above 32 sessions (A/B measurements)
@@ -728,19 +728,16 @@ int init_once() {
     if (!fn || qres != cudaDriverEntryPointSuccess) B200_FAIL(B200_ERR_CUDA, "cuTensorMapEncodeTiled not available");
     g_encode = reinterpret_cast<EncodeTiledFn>(fn);
   }
-  if (!g_attr_set) {
-    const int max_smem = 220 * 1024;     // the kernel also has a few bytes of static shared memory
-    B200_CUDA(cudaFuncSetAttribute(gemm_sk_kernel<EPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    B200_CUDA(cudaFuncSetAttribute(gemm_sk_kernel<EPI_RESADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    B200_CUDA(cudaFuncSetAttribute(gemm_sk_kernel<EPI_GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    B200_CUDA(cudaFuncSetAttribute(gemm_ck_kernel<EPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    B200_CUDA(cudaFuncSetAttribute(gemm_ck_kernel<EPI_RESADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+  static std::atomic<uint64_t> limits{0};
+  // the kernels also have a few bytes of static shared memory
+  B200_TRY(allow_smem(limits, 220 * 1024, gemm_sk_kernel<EPI_STORE>, gemm_sk_kernel<EPI_RESADD>, gemm_sk_kernel<EPI_GATE>, gemm_ck_kernel<EPI_STORE>, gemm_ck_kernel<EPI_RESADD>));
+  if (!g_settings_read) {
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
     B200_CUDA(cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev));
     if (const char* e = getenv("B200_ROW_MAX_M")) g_row_max_m = atoi(e);
     if (const char* e = getenv("B200_GEMM_NS")) g_use_ns = atoi(e);
-    g_attr_set = true;
+    g_settings_read = true;
   }
   return B200_OK;
 }

@@ -428,13 +428,8 @@ int launch(const WideGemm& g, WideP p, int clusters, cudaStream_t st) {
   p.stage_bytes = (p.a_bytes + 1023) / 1024 * 1024 + WROWS * BK * 2;
   p.stages = std::min(MAX_ST, 200 * 1024 / (int)p.stage_bytes);
   const size_t smem = (size_t)p.stages * p.stage_bytes + 1024 + 16 * MAX_ST + 64;
-  int dev = 0;
-  B200_CUDA(cudaGetDevice(&dev));
-  static std::atomic<uint64_t> attr_set{0};             // per device
-  if (!(attr_set.load() >> (dev & 63) & 1)) {
-    B200_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<CG, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    attr_set.fetch_or(1ull << (dev & 63));
-  }
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, 220 * 1024, gemm_wide_kernel<CG, BN>));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(std::min(clusters, p.mt * p.nt * p.splits) * CG)); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;

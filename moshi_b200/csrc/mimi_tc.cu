@@ -283,7 +283,6 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn g_encode = nullptr;
-bool g_attr = false;
 
 }  // namespace
 
@@ -300,11 +299,8 @@ int tc_init() {
     if (!fn || qres != cudaDriverEntryPointSuccess) B200_FAIL(B200_ERR_CUDA, "cuTensorMapEncodeTiled not available");
     g_encode = reinterpret_cast<EncodeTiledFn>(fn);
   }
-  if (!g_attr) {
-    B200_CUDA(cudaFuncSetAttribute(mimi_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    g_attr = true;
-  }
-  return B200_OK;
+  static std::atomic<uint64_t> limits{0};
+  return allow_smem(limits, 220 * 1024, mimi_tc_kernel);
 }
 
 static int pick_nt(int N) { return N >= TC_MAX_NT ? TC_MAX_NT : N; }

@@ -1,7 +1,10 @@
 """Host state that belongs to one device (kernels' limits of shared memory, workspaces), with a second device in the same process."""
 import ctypes as C
+import re
 
 import pytest
+
+from moshi_b200.build import CSRC
 
 from . import fake_cuda
 
@@ -37,3 +40,29 @@ def test_a_refused_limit_is_asked_for_again(fake):
     fake.fake_refuse_attributes(1)
     assert _linear(fake, 1) != 0
     fake_cuda.check(fake, _linear(fake, 1))
+
+
+def _stores(fake, op):
+    p = C.create_string_buffer(1 << 22)
+    return op(C.c_void_p((C.addressof(p) + 255) // 256 * 256))
+
+
+@pytest.mark.parametrize("name,call", [
+    ("gemm_sk_kernel", lambda f: _linear(f, 24, 22528, 4096, GATE)), ("gemm_ns_kernel", lambda f: _linear(f, 104)),
+    ("gemm_ck_kernel", lambda f: _linear(f, 104, i8=True)), ("gemm_wide_kernel", lambda f: _stores(f, lambda p: f.b200_op_linear_wide(p, p, p, 512, 512, 512, 512, 1, 1, None))),
+    ("mimi_tc_kernel", lambda f: _stores(f, lambda p: f.b200_op_tc_linear_f32(p, p, p, 64, 256, 64, None))),
+    ("flash_attention_kernel", lambda f: _stores(f, lambda p: f.b200_op_prefill_attention(p, p, p, None, p, 128, 1, 0, 128, 1.0, None)))])
+def test_other_kernels_on_a_second_device(fake, name, call):
+    for dev in (0, 1):
+        fake.cudaSetDevice(dev)
+        fake_cuda.check(fake, call(fake))
+        got = fake_cuda.launches(fake)
+        assert any(name in n for _, n in got) and all(at == dev for at, _ in got)
+
+
+def test_limits_are_raised_per_device_everywhere():
+    """The one place that raises a kernel's limit is the one that keeps book per device (dep_fused.cu: with every handle)."""
+    at = [(f.name, f.read_text().count("cudaFuncSetAttribute")) for f in sorted(CSRC.glob("*.cu*"))]
+    assert {n for n, c in at if c} <= {"common.cuh", "dep_fused.cu"}
+    for f in CSRC.glob("*.cu*"):
+        assert not re.search(r"static (bool|const cudaError_t) \w*(attr|once)", f.read_text()), f.name
