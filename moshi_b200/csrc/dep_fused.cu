@@ -38,6 +38,7 @@ constexpr int BLOCK_ROWS = 128, BLOCK_K = 64, UMMA_K = 16;
 constexpr int THREADS = 256;                 // warp 0 producer, 1 MMA, 2-5 epilogue, 6-7 extra hands in the SIMT phases
 constexpr int TILE_BYTES = BLOCK_ROWS * BLOCK_K * 2;
 constexpr int MAX_STAGES = 8;
+constexpr int SMEM_LIMIT = 220 * 1024;       // dynamic shared memory of a CTA at most; the kernels have up to 7 KB of static beside it
 constexpr int DD = 64;                       // depformer head dim
 static_assert(THREADS == lm::SAMPLE_THREADS, "sample_row needs a SAMPLE_THREADS-wide CTA");
 
@@ -515,6 +516,9 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   B200_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
   if (!fn || qres != cudaDriverEntryPointSuccess) B200_FAIL(B200_ERR_CUDA, "cuTensorMapEncodeTiled not available");
   EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(fn);
+  // one limit for every handle: a kernel has one, and a handle that set its own need would take a larger one's away
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, SMEM_LIMIT, dep_fused_kernel, dep_reg_kernel<1, false>, dep_reg_kernel<1, true>, dep_reg_kernel<2, false>, dep_reg_kernel<2, true>));
   DepFused* d = new DepFused();
   DepParams& p = d->p;
   memset(&p, 0, sizeof(p));
@@ -580,9 +584,7 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
     const int nt = c.B <= 8 ? 1 : 2;
     d->reg = dep_reg_pick(nt, c.trace || c.wait_ns > 0);
     d->smem = dep_reg_smem(c, d->grid);
-    B200_CUDA(cudaFuncSetAttribute(d->reg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem));
   }
-  B200_CUDA(cudaFuncSetAttribute(dep_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
   int per_sm = 0, coop = 0, dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
   B200_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));

@@ -6,7 +6,12 @@ import os
 import subprocess
 from pathlib import Path
 
+import torch
+
 from moshi_b200 import _lib, build
+from moshi_b200.models.lm import _config_struct
+from moshi_b200.models.state_dict import normalize_lm_state_dict
+from moshi_b200.synth import synth_lm_state_dict
 
 
 def load(folder: Path) -> C.CDLL:
@@ -41,3 +46,30 @@ def launches(lib: C.CDLL) -> list[tuple[int, str]]:
 
 def check(lib: C.CDLL, rc: int) -> None:
     assert rc == 0, lib.b200_last_error().decode()
+
+
+class LM:
+    """A Moshi LM of the library on the fake runtime; its weights are what they are."""
+
+    def __init__(self, lib: C.CDLL, cfg, weights=None):
+        self.lib, self.cfg, self.h = lib, cfg, C.c_void_p()
+        check(lib, lib.b200_lm_create(C.byref(_config_struct(cfg)), C.byref(self.h)))
+        for name, t in normalize_lm_state_dict(weights or synth_lm_state_dict(cfg, seed=1)).items():
+            t = t.to(torch.bfloat16).contiguous()
+            check(lib, lib.b200_lm_load_tensor(self.h, name.encode(), C.c_void_p(t.data_ptr()), _lib.dtype_code(torch.bfloat16), t.dim(), (C.c_int64 * t.dim())(*t.shape)))
+        check(lib, lib.b200_lm_finalize(self.h))
+
+    def begin(self, sessions: int) -> None:
+        self.sessions = sessions
+        check(self.lib, self.lib.b200_lm_set_graph(self.h, 0))
+        check(self.lib, self.lib.b200_lm_streaming_begin(self.h, sessions, None))
+
+    def step(self) -> list[tuple[int, str]]:
+        n, out, ready = self.cfg.n_q - self.cfg.dep_q, torch.zeros(self.sessions, self.cfg.dep_q + 1, dtype=torch.int64), C.c_int()
+        codes, noise = torch.zeros(self.sessions, n, dtype=torch.int64), torch.ones(self.sessions * self.lib.b200_lm_noise_per_row(self.h))
+        launches(self.lib)
+        check(self.lib, self.lib.b200_lm_step(self.h, C.c_void_p(codes.data_ptr()), n, C.c_void_p(noise.data_ptr()), C.c_void_p(out.data_ptr()), 1, C.byref(ready)))
+        return launches(self.lib)
+
+    def close(self) -> None:
+        self.lib.b200_lm_destroy(self.h)
