@@ -382,5 +382,5 @@ inline size_t dep_reg_smem(const DepFusedConfig& c, int grid) {
 }
 inline bool dep_reg_takes(const DepFusedConfig& c, int grid) {
   return c.B <= REG_B && c.dd % 64 == 0 && c.dd <= REG_WARPS * 64 && c.F % 8 == 0 && c.F <= REG_KC * REG_WARPS * 64 && grid >= 1 && dep_reg_subs(c, grid) <= REG_SUBS &&
-         c.B * (c.dd / DD) <= REG_WARPS * grid && c.dep_q * (4 * c.L + 1) <= 1024;
+         c.B * (c.dd / DD) <= REG_WARPS * grid && dep_reg_smem(c, grid) <= SMEM_LIMIT;
 }

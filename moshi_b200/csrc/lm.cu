@@ -672,7 +672,7 @@ int b200_lm_streaming_begin(b200_lm* h, int batch, void* stream) {
   // Under classifier-free guidance the two halves of the batch meet before every sampler (lm.py:828-833): launch chain.
   tc::DepFusedConfig few;
   memset(&few, 0, sizeof(few));
-  few.B = B; few.dd = dd; few.F = c.depformer_ffn_hidden; few.card = c.card;
+  few.B = B; few.dd = dd; few.F = c.depformer_ffn_hidden; few.card = c.card; few.dep_q = c.dep_q; few.L = c.depformer_num_layers;
   const bool dep_small = B <= 2 && h->dep_fused != 2 && !tc::dep_fused_in_registers(few);
   h->depf = nullptr;
   if (c.dep_q > 0 && !cfg && !c.quantize && h->dep_fused && !dep_small && B <= 256 && dd <= 1024 && dd % 64 == 0) {

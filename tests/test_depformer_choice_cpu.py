@@ -24,3 +24,26 @@ def test_a_second_stream_leaves_the_first_its_shared_memory(fake):
     assert len(_dep(small.step())) == 1
     assert len(_dep(big.step())) == 1
     big.close(), small.close()
+
+
+@pytest.mark.parametrize("sessions", [1, 2, 3, 16])
+@pytest.mark.parametrize("layers,dep_q", [(2, 8), (16, 16), (40, 16)])
+def test_few_sessions_of_deep_depformers(fake, sessions, layers, dep_q):
+    """As many weights as its shared memory holds the addresses of: the kernel of few sessions."""
+    lm = fake_cuda.LM(fake, tiny_lm_config(depformer_num_layers=layers, dep_q=dep_q, n_q=2 * dep_q))
+    lm.begin(sessions)
+    (name,) = _dep(lm.step())
+    assert "dep_reg_kernel" in name
+    lm.close()
+
+
+@pytest.mark.parametrize("sessions", [1, 2, 3])
+@pytest.mark.parametrize("over", [dict(card=9480), dict(depformer_dim=64, depformer_num_heads=1, depformer_dim_feedforward=96, dep_q=16, n_q=32, depformer_num_layers=190)])
+def test_few_sessions_of_shapes_that_only_the_shared_memory_kernel_takes(fake, sessions, over):
+    """More rows of logits than eight 8-row pieces a CTA, more weights than addresses fit: one and two sessions take a chain of launches, more the
+    shared-memory kernel."""
+    lm = fake_cuda.LM(fake, tiny_lm_config(**over))
+    lm.begin(sessions)
+    names = _dep(lm.step())
+    assert (not names) if sessions <= 2 else "dep_fused_kernel" in names[0]
+    lm.close()
