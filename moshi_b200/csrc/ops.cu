@@ -1,4 +1,6 @@
 // Kernel-level C entry points used by the parity tests (same kernels the handles launch).
+#include <mutex>
+
 #include "gemm_reg.cuh"
 #include "gemm_sk.cuh"
 #include "lm_kernels.cuh"
@@ -10,18 +12,38 @@ using namespace b200;
 
 extern "C" {
 
-// split-K workspace + arrival counters of the kernel-level entry points (a handle owns its own); separate sets for the bf16 and
-// the int8 kernels, like the handles keep them
-static int sk_scratch(float** ws, int** counters, int which = 0) {
-  static float* g_ws[2] = {nullptr, nullptr};
-  static int* g_counters[2] = {nullptr, nullptr};
-  if (!g_ws[which]) {
-    B200_CUDA(cudaMalloc(&g_ws[which], tc::sk_workspace_bytes(256)));
-    B200_CUDA(cudaMalloc(&g_counters[which], tc::SK_MAX_TILES * sizeof(int)));
-    B200_CUDA(cudaMemset(g_counters[which], 0, tc::SK_MAX_TILES * sizeof(int)));
+// Partial sums and arrival counters (zero between launches) of the kernel-level entry points; a handle owns its own.  They lie on the device that is
+// current at the call, one set per kind of kernel, and grow with the largest call.
+enum { SCRATCH_BF16 = 0, SCRATCH_I8, SCRATCH_ATTN, SCRATCH_ATTN_Q8, SCRATCH_KINDS };
+struct Scratch { float* part; int* counters; size_t part_n, counters_n; };
+static int scratch(int kind, size_t part_n, size_t counters_n, float** part, int** counters) {
+  constexpr int DEVICES = 64;
+  static std::mutex mu;
+  static Scratch all[DEVICES][SCRATCH_KINDS];
+  int dev = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  if (dev >= DEVICES) B200_FAIL(B200_ERR_INVALID, "kernel-level entry points: device %d of %d", dev, DEVICES);
+  std::lock_guard<std::mutex> guard(mu);
+  Scratch& s = all[dev][kind];
+  if (part_n > s.part_n) {
+    cudaFree(s.part);
+    s.part = nullptr; s.part_n = 0;
+    B200_CUDA(cudaMalloc(&s.part, part_n * sizeof(float)));
+    s.part_n = part_n;
   }
-  *ws = g_ws[which]; *counters = g_counters[which];
+  if (counters_n > s.counters_n) {
+    cudaFree(s.counters);
+    s.counters = nullptr; s.counters_n = 0;
+    B200_CUDA(cudaMalloc(&s.counters, counters_n * sizeof(int)));
+    B200_CUDA(cudaMemset(s.counters, 0, counters_n * sizeof(int)));
+    B200_CUDA(cudaStreamSynchronize(nullptr));   // the caller's stream may not wait for this one
+    s.counters_n = counters_n;
+  }
+  *part = s.part; *counters = s.counters;
   return B200_OK;
+}
+static int sk_scratch(float** ws, int** counters, int kind = SCRATCH_BF16) {
+  return scratch(kind, tc::sk_workspace_bytes(256) / sizeof(float), tc::SK_MAX_TILES, ws, counters);
 }
 
 // The entry points of a step's kernels are launched early and wait before they read anything (B200_PDL=0: ordinary launches): behind one
@@ -128,7 +150,7 @@ int b200_op_linear_i8(const void* xq_dev, const float* sa_dev, const void* w_til
   if (!tc::sk_supported(M, N, K, epi)) B200_FAIL(B200_ERR_SHAPE, "op_linear_i8: unsupported shape");
   static tc::GemmPlanCache cache;
   float* ws = nullptr; int* counters = nullptr;
-  B200_TRY(sk_scratch(&ws, &counters, 1));   // int32 partials of cut tiles
+  B200_TRY(sk_scratch(&ws, &counters, SCRATCH_I8));   // int32 partials of cut tiles
   tc::SkTuning t;
   t.xq = xq_dev; t.sa = sa_dev; t.sw = sw_dev; t.pdl = op_pdl();
   const int out_cols = epi == 2 ? gate_rows : N;
@@ -181,21 +203,8 @@ int b200_op_attn_step(const void* qkv_dev, void* k_dev, void* v_dev, void* out_d
   if (B < 1 || H < 1 || cap < 1) B200_FAIL(B200_ERR_SHAPE, "op_attn_step: bad shape");
   int min_per = 1;
   if (nsplit <= 0) nsplit = attn_ragged_splits(B, H, cap, &min_per);
-  static float* part = nullptr;
-  static int* counters = nullptr;
-  static size_t part_n = 0, cnt_n = 0;
-  const size_t need = (size_t)B * H * nsplit * (ATT_D + 2);
-  if (need > part_n) {
-    if (part) cudaFree(part);
-    B200_CUDA(cudaMalloc(&part, need * sizeof(float)));
-    part_n = need;
-  }
-  if ((size_t)B * H > cnt_n) {
-    if (counters) cudaFree(counters);
-    B200_CUDA(cudaMalloc(&counters, (size_t)B * H * sizeof(int)));
-    B200_CUDA(cudaMemset(counters, 0, (size_t)B * H * sizeof(int)));
-    cnt_n = (size_t)B * H;
-  }
+  float* part = nullptr; int* counters = nullptr;
+  B200_TRY(scratch(SCRATCH_ATTN, (size_t)B * H * nsplit * (ATT_D + 2), (size_t)B * H, &part, &counters));
   AttnStep a;
   a.qkv = static_cast<const bf16*>(qkv_dev); a.kc = static_cast<bf16*>(k_dev); a.vc = static_cast<bf16*>(v_dev);
   a.out = static_cast<bf16*>(out_dev); a.part = part; a.counters = counters;
@@ -215,21 +224,8 @@ int b200_op_attn_step_q8(const void* qkv_dev, void* k8_dev, void* v8_dev, float*
   if (B < 1 || H < 1 || cap < 1) B200_FAIL(B200_ERR_SHAPE, "op_attn_step_q8: bad shape");
   if (kv_dtype != B200_KV_FP8_E4M3 && kv_dtype != B200_KV_INT8) B200_FAIL(B200_ERR_INVALID, "op_attn_step_q8: kv_dtype %d", kv_dtype);
   if (nsplit <= 0) nsplit = attn_pick_splits(B, H, cap);
-  static float* part = nullptr;
-  static int* counters = nullptr;
-  static size_t part_n = 0, cnt_n = 0;
-  const size_t need = (size_t)B * H * nsplit * (ATT_D + 2);
-  if (need > part_n) {
-    if (part) cudaFree(part);
-    B200_CUDA(cudaMalloc(&part, need * sizeof(float)));
-    part_n = need;
-  }
-  if ((size_t)B * H > cnt_n) {
-    if (counters) cudaFree(counters);
-    B200_CUDA(cudaMalloc(&counters, (size_t)B * H * sizeof(int)));
-    B200_CUDA(cudaMemset(counters, 0, (size_t)B * H * sizeof(int)));
-    cnt_n = (size_t)B * H;
-  }
+  float* part = nullptr; int* counters = nullptr;
+  B200_TRY(scratch(SCRATCH_ATTN_Q8, (size_t)B * H * nsplit * (ATT_D + 2), (size_t)B * H, &part, &counters));
   AttnStepQ8 a;
   a.qkv = static_cast<const bf16*>(qkv_dev); a.kc = static_cast<uint8_t*>(k8_dev); a.vc = static_cast<uint8_t*>(v8_dev);
   a.ks = ks_dev; a.vs = vs_dev; a.out = static_cast<bf16*>(out_dev); a.part = part; a.counters = counters;

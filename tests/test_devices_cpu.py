@@ -66,3 +66,30 @@ def test_limits_are_raised_per_device_everywhere():
     assert {n for n, c in at if c} <= {"common.cuh", "dep_fused.cu"}
     for f in CSRC.glob("*.cu*"):
         assert not re.search(r"static (bool|const cudaError_t) \w*(attr|once)", f.read_text()), f.name
+
+
+def _attention(fake, sessions, q8):
+    def op(p):
+        if q8:
+            return fake.b200_op_attn_step_q8(p, p, p, p, p, p, p, None, sessions, 32, 3000, 0, 1e4, 1, None)
+        return fake.b200_op_attn_step(p, p, p, p, p, None, sessions, 32, 3000, 0, 1e4, None)
+    return _stores(fake, op)
+
+
+@pytest.mark.parametrize("call,larger", [(lambda f: _linear(f, 20), None), (lambda f: _linear(f, 20, i8=True), None),
+                                         (lambda f: _attention(f, 1, False), lambda f: _attention(f, 48, False)), (lambda f: _attention(f, 1, True), lambda f: _attention(f, 48, True))])
+def test_workspaces_lie_on_the_device_of_the_call(fake, call, larger):
+    """Partial results of work that is cut: another device's kernels could not write them.  They are kept, and grow with the largest call."""
+    for dev in (0, 1):
+        fake.cudaSetDevice(dev)
+        before = fake.fake_held(dev)
+        fake_cuda.check(fake, call(fake))
+        once = fake.fake_held(dev)
+        assert once > before
+        fake_cuda.check(fake, call(fake))
+        assert fake.fake_held(dev) == once
+        if larger:
+            fake_cuda.check(fake, larger(fake))
+            assert (most := fake.fake_held(dev)) > once
+            fake_cuda.check(fake, call(fake))
+            assert fake.fake_held(dev) == most
