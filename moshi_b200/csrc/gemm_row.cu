@@ -17,6 +17,8 @@
 //   1 row: 4096 -> 12288 24.4 / 20.5 / 15.4, 4096 -> 4096 12.4 / 10.3 / 5.1, gated -> 11264 36.6 / 31.2 / 28.2, 11264 -> 4096 20.5 / 18.5 / 14.1, -> 32000 49.6 / 43.3 / 40.0;
 //   8 rows: 24.1 / 21.2, 12.9 / 10.5, 33.0 / 33.7, 23.1 / 19.6, 52.6 / 45.7; 16 rows: 26.2 / 22.6, 14.5 / 12.4, -, 26.1 / 22.6, 55.4 / 51.3;
 //   1024 -> 3072 8.3 / 6.2, 2816 -> 1024 9.5 / 6.2; int8 4096 -> 12288 19.4 / 16.5, 11264 -> 4096 18.5 / 18.5.
+// Error of the sums alone (terms whose exact sum is 0, over the rms of a random sum of them), 4096 -> 12288: 1 row 6.9e-8 (fp32 FMAs 7.4e-8; chains of 16 instructions
+// 1.27e-7), 12 rows 8.4e-8 (gemm_reg.cu 6.7e-7); 11264 -> 4096: 1 row 7.7e-8 (8.5e-8; 1.31e-7).
 // Steps of the 7B: 1 session 4470 -> 4014 us, 3: 4610 -> 4223, 8: 4765 -> 4397, 16 with full rings 6980 -> 6560.
 #include "gemm_row.cuh"
 
@@ -75,6 +77,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_row_kernel(const RowP p) {
   using Acc = typename std::conditional<I8, int, float>::type;
   constexpr int G = EPI == EPI_GATE ? 1 : 0;     // gated: the tiles of gate and value rows lie behind each other
   constexpr int KC = NT == 1 ? 4 : 2;            // k-blocks of a warp whose activations are in registers together
+  // The tensor core cuts its fp32 sums off where an FMA rounds, and the error grows with the chain: up to 8 rows two instructions (32 k) at a time, added in fp32,
+  // are as exact as fp32 FMAs throughout, at no cost in time (above 8 rows they cost 2 % of 11264 -> 4096; there the kernels that cut K chain far more).
+  constexpr bool SHORT_CHAINS = NT == 1 && !I8;
   extern __shared__ __align__(16) uint8_t smem[];
   Acc* red = reinterpret_cast<Acc*>(smem + RING_BYTES);      // [warp][sub][row of x][8]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, M = p.M;
@@ -156,13 +161,24 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_row_kernel(const RowP p) {
           __syncwarp();
           ask(slot);
           slot = slot + SLOT == SLOTS * SLOT ? 0u : slot + SLOT;
+          if constexpr (SHORT_CHAINS) {
+            Acc part[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-              mma_step(acc[j], a[h].x, b[h].x, a[h].y, b[h].y, xb[i][j][h].x, xb[i][j][h].y);
-              mma_step(acc[j], a[h].z, b[h].z, a[h].w, b[h].w, xb[i][j][h].z, xb[i][j][h].w);
+            for (int h = 0; h < 2; ++h) {
+              mma_step(part[h], a[h].x, b[h].x, a[h].y, b[h].y, xb[i][0][h].x, xb[i][0][h].y);
+              mma_step(part[h], a[h].z, b[h].z, a[h].w, b[h].w, xb[i][0][h].z, xb[i][0][h].w);
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[0][e] += part[0][e] + part[1][e];
+          } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int j = 0; j < NT; ++j) {
+                mma_step(acc[j], a[h].x, b[h].x, a[h].y, b[h].y, xb[i][j][h].x, xb[i][j][h].y);
+                mma_step(acc[j], a[h].z, b[h].z, a[h].w, b[h].w, xb[i][j][h].z, xb[i][j][h].w);
+              }
+          }
         }
         // rows g of either sub; the second of a last odd pair is whatever its slot held before, and is not stored
 #pragma unroll
@@ -176,17 +192,24 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_row_kernel(const RowP p) {
       }
     }
     __syncthreads();
-    // results of the pass: the warps' sums in warp order
+    // results of the pass: the warps' sums in pairs, always the same
     const int rows = (n >> G) * UNIT, first = (u0 + (pass >> G)) * UNIT;
     for (int i = tid; i < rows * M; i += THREADS) {
       const int m = i / rows, r = i - m * rows, o = first + r;
       if (o >= p.out_rows) continue;
-      Acc v[2] = {0, 0};
+      Acc v[2];
 #pragma unroll
-      for (int a = 0; a <= G; ++a)
+      for (int a = 0; a <= G; ++a) {
+        Acc s[WARPS];
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) v[a] += red[((w * n + ((r >> 3) << G) + a) * M + m) * 8 + (r & 7)];
-      float f[2] = {(float)v[0], (float)v[1]};
+        for (int w = 0; w < WARPS; ++w) s[w] = red[((w * n + ((r >> 3) << G) + a) * M + m) * 8 + (r & 7)];
+#pragma unroll
+        for (int d = WARPS / 2; d > 0; d >>= 1)
+#pragma unroll
+          for (int w = 0; w < d; ++w) s[w] += s[w + d];
+        v[a] = s[0];
+      }
+      float f[2] = {(float)v[0], (float)v[G]};
       if (I8) {                                  // the sums are whole numbers in 32 bits
         const float s = p.sa[m];
         f[0] *= s * p.sw[o] * (1.f / 16129.f);
