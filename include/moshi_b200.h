@@ -592,7 +592,8 @@ int b200_op_linear_wide(const void* x_dev, const void* w_dev, void* y_dev, int M
 int b200_op_grouped_wide(const void* x_dev, const void* w_dev, void* y_dev, const int32_t* counts_host, int E, int M, int N, int K, int ldy,
                          int act, float limit, void* stream);
 /* Up to how many activation rows the linears may take the kernel that gives a CTA whole output rows (csrc/gemm_row.cu) instead of those that cut
- * K over CTAs: 0..16, default 16 (or B200_ROW_MAX_M).  Returns the previous value. */
+ * K over CTAs: 0..16, default 16 (or B200_ROW_MAX_M, or B200_GEMV_MAX_M: the kernel was a GEMV for up to 4 rows once, and the setting keeps its
+ * names).  Returns the previous value. */
 int b200_op_set_gemv_max_rows(int max_rows);
 /* int8 x int8 linear (QLinear, utils/quantize.py:13-40: bitsandbytes row-wise absmax quantisation of weights and
  * activations, int32 accumulation, dequantisation by both row scales / 127^2), on tcgen05 kind::i8.

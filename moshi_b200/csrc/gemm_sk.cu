@@ -735,7 +735,9 @@ int init_once() {
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
     B200_CUDA(cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev));
-    if (const char* e = getenv("B200_ROW_MAX_M")) g_row_max_m = atoi(e);
+    const char* rows = getenv("B200_ROW_MAX_M");
+    if (!rows) rows = getenv("B200_GEMV_MAX_M");      // the name that it had when fewer rows were possible
+    if (rows) g_row_max_m = atoi(rows);
     if (const char* e = getenv("B200_GEMM_NS")) g_use_ns = atoi(e);
     g_settings_read = true;
   }
