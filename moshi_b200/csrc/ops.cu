@@ -200,6 +200,7 @@ int b200_op_attn_step(const void* qkv_dev, void* k_dev, void* v_dev, void* out_d
                       const uint8_t* exec_mask_dev, int B, int H, int cap, int nsplit, float max_period, void* stream) {
   using namespace b200::lm;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (!qkv_dev || !k_dev || !v_dev || !out_dev || !pos_dev || !exec_mask_dev) B200_FAIL(B200_ERR_INVALID, "op_attn_step: null pointer");
   if (B < 1 || H < 1 || cap < 1) B200_FAIL(B200_ERR_SHAPE, "op_attn_step: bad shape");
   int min_per = 1;
   if (nsplit <= 0) nsplit = attn_ragged_splits(B, H, cap, &min_per);
@@ -221,6 +222,7 @@ int b200_op_attn_step_q8(const void* qkv_dev, void* k8_dev, void* v8_dev, float*
                          int kv_dtype, void* stream) {
   using namespace b200::lm;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (!qkv_dev || !k8_dev || !v8_dev || !ks_dev || !vs_dev || !out_dev || !pos_dev || !exec_mask_dev) B200_FAIL(B200_ERR_INVALID, "op_attn_step_q8: null pointer");
   if (B < 1 || H < 1 || cap < 1) B200_FAIL(B200_ERR_SHAPE, "op_attn_step_q8: bad shape");
   if (kv_dtype != B200_KV_FP8_E4M3 && kv_dtype != B200_KV_INT8) B200_FAIL(B200_ERR_INVALID, "op_attn_step_q8: kv_dtype %d", kv_dtype);
   if (nsplit <= 0) nsplit = attn_pick_splits(B, H, cap);

@@ -71,8 +71,8 @@ def test_limits_are_raised_per_device_everywhere():
 def _attention(fake, sessions, q8):
     def op(p):
         if q8:
-            return fake.b200_op_attn_step_q8(p, p, p, p, p, p, p, None, sessions, 32, 3000, 0, 1e4, 1, None)
-        return fake.b200_op_attn_step(p, p, p, p, p, None, sessions, 32, 3000, 0, 1e4, None)
+            return fake.b200_op_attn_step_q8(p, p, p, p, p, p, p, p, sessions, 32, 3000, 0, 1e4, 1, None)
+        return fake.b200_op_attn_step(p, p, p, p, p, p, sessions, 32, 3000, 0, 1e4, None)
     return _stores(fake, op)
 
 

@@ -4,15 +4,23 @@ import ctypes as C
 import pytest
 
 from . import fake_cuda
+from .test_gpu_zzzzzzzz_op_launches import LINEARS, RESADD, WRITERS, linear
 
 
-def _kernel(fake, M):
+def _kernel(fake, shape):
     p = C.create_string_buffer(64)
     at = C.c_void_p((C.addressof(p) + 15) // 16 * 16)
     fake_cuda.launches(fake)
-    fake_cuda.check(fake, fake.b200_op_linear_sk(at, at, at, None, M, 4096, 4096, 0, 0, 0, 0, 0, None))
+    fake_cuda.check(fake, linear(fake, shape, at, at, at, at if shape[3] == RESADD else None, at, at))
     ((_, name),) = fake_cuda.launches(fake)
     return name
+
+
+def test_linears_of_the_early_launch_tests_take_the_kernels_they_name(tmp_path):
+    fake = fake_cuda.load(tmp_path)
+    for kernel, shapes in [*LINEARS.items(), *((k, [s]) for k, s in WRITERS.items())]:
+        for shape in shapes:
+            assert kernel in _kernel(fake, shape), (kernel, shape)
 
 
 @pytest.mark.parametrize("name", ["B200_ROW_MAX_M", "B200_GEMV_MAX_M"])
@@ -20,7 +28,18 @@ def test_rows_up_to_which_whole_rows_per_cta_are_considered(tmp_path, monkeypatc
     """The older name of the setting counts too."""
     monkeypatch.setenv(name, "2")
     fake = fake_cuda.load(tmp_path)
-    assert "gemm_row_kernel" in _kernel(fake, 2)
-    assert "gemm_reg_kernel" in _kernel(fake, 3)
+    assert "gemm_row_kernel" in _kernel(fake, (2, 4096, 4096, 0, False))
+    assert "gemm_reg_kernel" in _kernel(fake, (3, 4096, 4096, 0, False))
     assert fake.b200_op_set_gemv_max_rows(16) == 2
-    assert "gemm_row_kernel" in _kernel(fake, 3)
+    assert "gemm_row_kernel" in _kernel(fake, (3, 4096, 4096, 0, False))
+
+
+@pytest.mark.parametrize("q8", [False, True])
+def test_attention_steps_refuse_null_pointers(tmp_path, q8):
+    """On a GPU the kernel would read address 0."""
+    fake = fake_cuda.load(tmp_path)
+    p = C.create_string_buffer(64)
+    for gone in range(8 if q8 else 6):
+        at = [None if i == gone else C.addressof(p) for i in range(8 if q8 else 6)]
+        rc = fake.b200_op_attn_step_q8(*at, 1, 2, 8, 0, 1e4, 1, None) if q8 else fake.b200_op_attn_step(*at, 1, 2, 8, 0, 1e4, None)
+        assert rc != 0 and not fake_cuda.launches(fake)
