@@ -1,10 +1,10 @@
-"""GPU: BASELINE.json's own LM configuration (configs/moshi_7b_202409.json: dim 4096, 32 layers, context 3000, 32000 / 2048
-vocabularies) stepped beside the CPU oracle on the same synthetic weights ("what's weak" #1).
+"""GPU: the 7B configuration (configs/moshi_7b_202409.json: dim 4096, 32 layers, context 3000, 32000 / 2048 vocabularies) stepped beside the CPU oracle on the
+same synthetic weights.
 
-The oracle steps the 7B model on the host cores in 1-8 s per step, so each batch size runs a handful of
-teacher-synchronised steps.  Batch sizes pick the three linear schedules: 1 (GEMV kernel + chained depformer), 3 (stream-K
-tcgen05 + fused depformer), 40 (whole-tile + cluster split-K tcgen05 + fused depformer).  Greedy ids are compared
-margin-aware: a mismatch is excused only where the oracle's own top-2 logit gap is below twice the logit tolerance."""
+The oracle steps the 7B model on the host cores in 1-8 s per step, so each batch size runs a handful of teacher-synchronised steps.  Batch sizes pick the
+schedules: 1 and 3 (whole output rows per CTA; depformer of few sessions), 20 (weights through registers, gated pairs and wide heads in the swap-AB kernel; fused
+depformer from 17 sessions on), 40 (non-swapped tcgen05 kernel; int8: whole tiles and clusters; fused depformer).  int8 takes the launch chain for the
+depformer.  Greedy ids are compared margin-aware: a mismatch is excused only where the oracle's own top-2 logit gap is below twice the logit tolerance."""
 import pytest
 import torch
 
@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 # bf16 logits after 32 layers (+ 6 depformer layers) of bf16 casts: the GPU (fp32 accumulation in TMEM, split-K partial sums) and
 # torch's CPU kernels (their own blocking) round differently at every cast, and every rounding random-walks through the residual
-# stream.  Measured on a B200 (profiles/r02_*_tests.log): text logits worst 0.11 (0.17 behind a ring of random keys), depformer
+# stream.  Measured on a B200: text logits worst 0.11 (0.17 behind a ring of random keys), depformer
 # logits worst 0.23 (0.34); for scale, the SAME session stepped by the GPU alone and inside a batch of five (another summation
 # order, nothing else) differs by 0.17 (tests/test_gpu_lm.py::test_full_size_7b_properties).  The id gate below is the strict one:
 # a greedy id may only differ from the oracle's where the oracle's own top-2 gap is below twice these tolerances.
@@ -80,7 +80,7 @@ def _compare(cfg, sd, lm, B, steps, seed, tol_text, tol_dep, quantize=False, pre
     return worst_t, worst_d, mism, unexc, total
 
 
-@pytest.mark.parametrize("B,steps", [(1, 4), (3, 4), (40, 3)])
+@pytest.mark.parametrize("B,steps", [(1, 4), (3, 4), (20, 3), (40, 3)])
 def test_7b_bf16_steps_match_the_oracle(seven_b, B, steps):
     sd, lm = seven_b
     wt, wd, mism, unexc, total = _compare(MOSHI_7B, sd, lm, B, steps, seed=100 + B, tol_text=TEXT_ATOL_7B, tol_dep=DEP_ATOL_7B)
@@ -126,9 +126,9 @@ def test_7b_ring_wraps_at_3000_like_the_oracle(seven_b):
     assert wt < TEXT_ATOL_7B and wd < DEP_ATOL_7B and unexc == 0
 
 
-@pytest.mark.parametrize("B,steps", [(1, 3), (3, 3), (40, 3)])
+@pytest.mark.parametrize("B,steps", [(1, 3), (3, 3), (20, 2), (40, 3)])
 def test_7b_shapes_int8_steps_match_the_quantised_oracle(B, steps):
-    """BASELINE config 5 (``LMModel(quantize=True)``: every linear an int8 QLinear) at the 7B model's real matrix shapes.  The
+    """``LMModel(quantize=True)`` (every linear an int8 QLinear) at the 7B model's real matrix shapes.  The
     CPU restatement of QLinear (oracle/quant.py: exact integer products in float64) cannot step 32 layers of them in the time
     a GPU box is worth, so this member of the family keeps every dimension of the 7B configuration (4096 / 11264 / 32000 /
     depformer 1024 / 2816 / 2048, context 3000) and cuts the depth to 4 temporal + 2 depformer layers."""

@@ -17,12 +17,13 @@ def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-@pytest.mark.parametrize("M", [1, 2, 8, 9, 16])
+@pytest.mark.parametrize("M", [1, 2, 8, 9, 12, 16])
 @pytest.mark.parametrize("N,K,epi", [(12, 72, STORE), (130, 8, STORE), (1192, 1024, RESADD), (600, 4104, GATE), (4096, 11264, RESADD), (22528, 4096, GATE),
                                      (32000, 512, STORE)])
 def test_row_linear(M, N, K, epi):
     """Fewer units than CTAs, one and several per CTA (odd counts, across tiles), rows beyond the last, one k-block and more than registers hold, sums in
-    one pass and in two (32000 outputs of 16 rows); two launches give the same bits; every other kernel agrees to a bf16 ulp."""
+    one pass and in two (32000 outputs of 16 rows); two launches give the same bits, and another kernel other bits here and there only.  (16 gated rows of 22528 x 4096
+    would take two passes and go to the register kernel.)"""
     from moshi_b200 import _lib
     lib = _lib.lib()
     g = torch.Generator().manual_seed(M + N + K)
@@ -52,6 +53,8 @@ def test_row_linear(M, N, K, epi):
     assert torch.equal(ys[0], ys[1])
     torch.testing.assert_close(ys[0].float(), z, rtol=2.0 ** -7, atol=3e-2)
     torch.testing.assert_close(ys[0].float(), ys[2].float(), rtol=2.0 ** -7, atol=3e-2)
+    # sums in another order move a result across a rounding now and then: some 1e-6 of its size against roundings 2^-8 apart, twice or thrice on the way
+    assert (ys[0] != ys[2]).float().mean() < 0.02
 
 
 @pytest.mark.parametrize("M", [1, 8, 13, 16])
