@@ -24,6 +24,7 @@
 // tile, k-split) and every unit writes its fp32 partial [M x 128] to an L2-resident workspace; the consumer phase
 // sums the splits in split order (deterministic, independent of the batch) and applies the reference's cast points.
 #include "gemm_sk.cuh"
+#include "row_stream.cuh"
 #include "tc_prims.cuh"
 #include "lm_kernels.cuh"
 
@@ -494,7 +495,7 @@ struct DepFused {
   void* dev_tables = nullptr;     // one allocation holding the pointer tables
 };
 
-bool dep_fused_in_registers(const DepFusedConfig& c) { return dep_reg_takes(c, sk_num_sms()); }
+bool dep_fused_few_sessions(const DepFusedConfig& c) { return dep_reg_takes(c, sk_num_sms()); }
 
 size_t dep_fused_partial_floats(const DepFusedConfig& c) {
   const int grid = sk_num_sms();

@@ -7,7 +7,8 @@
 //     memory, so no partial sum leaves an SM (dep_fused_kernel exchanges split-K partials through L2 and needs a phase of its own to add them);
 //   * every warp asks for its weights with cp.async up to four pairs of units x 64 k ahead, through all products, layers and sub-steps and across the
 //     barriers.  (Held in registers they did not fit: 632 to 1268 bytes per thread went through local memory, and a spilled load has to
-//     arrive before the thread can go on to the barrier.)
+//     arrive before the thread can go on to the barrier.  Of
+//     what is left 12 bytes per thread are spilled for up to 8 sessions, 120 for up to 16.)
 //   * a warp has one k-block of the width, so its share of the RMSNorm is what it multiplies: the sums of squares meet in shared memory; residual, gating
 //     and bf16 roundings sit in the epilogues; old keys and values of the attention are asked for before the barrier.
 //
@@ -26,17 +27,6 @@ constexpr int REG_SUBS = 8;                  // 8-row pieces (gate and value row
 constexpr int REG_UNIT = 8, REG_UNIT_BYTES = 1024;
 constexpr uint32_t REG_SLOT_BYTES = REG_WARPS * 2 * REG_UNIT_BYTES;
 enum { REG_IN = 0, REG_OUT = 1, REG_GATE = 2, REG_LINEAR_OUT = 3, REG_HEAD = 4, REG_KINDS = 5 };
-
-__device__ __forceinline__ void reg_copy16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ uint4 reg_lds16(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void reg_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 // all CTAs meet; false: not within the limit.  DIAG: with time stamps and a limit of the caller's, in a kernel of its own (in the one kernel the
 // tests for them cost 0.13 us per barrier, 33 us per frame of 16 sessions).
@@ -74,10 +64,6 @@ __device__ __forceinline__ RegPart reg_part(int num_kb, int gated, int rows) {
   return p;
 }
 
-// A piece c of a packed row r lies at position c ^ r.  Fragment rows are taken as 0, 4, 1, 5, ..: the eight lanes of a 16-byte read phase hold two of
-// them, whose pieces then lie in the two halves of the banks.
-__device__ __forceinline__ int reg_row_of(int g) { return (g >> 1) | ((g & 1) << 2); }
-
 // The stream of one warp through the frame: weights w[0 .. n) in the order of use, `per` to a sub-step (four a layer, then the head); a slot holds a pair of
 // 8-row pieces of one k-block.
 struct RegStream {
@@ -109,12 +95,12 @@ struct RegStream {
       const uint32_t step = (uint32_t)(REG_WARPS * TILE_BYTES) << gated, to = ring + to_slot + (threadIdx.x & 31) * 16;
       const int u0 = first + (sub >> gated), u1 = u0 + 1;
       const uint8_t* s = base + ((u0 >> 4) * tile_bytes + (u0 & 15) * REG_UNIT_BYTES);
-      reg_copy16(to, s);
-      reg_copy16(to + 512, s + 512);
+      rows::copy16(to, s);
+      rows::copy16(to + 512, s + 512);
       if (sub + 1 < subs) {
         s = gated ? s + TILE_BYTES : base + ((u1 >> 4) * tile_bytes + (u1 & 15) * REG_UNIT_BYTES);
-        reg_copy16(to + 1024, s);
-        reg_copy16(to + 1536, s + 512);
+        rows::copy16(to + 1024, s);
+        rows::copy16(to + 1536, s + 512);
       }
       base += step;
       if (++j == nj) {
@@ -126,14 +112,14 @@ struct RegStream {
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  // the next pair of 8 rows x 64 k: pieces t and t + 4 of row reg_row_of(g) of either
+  // the next pair of 8 rows x 64 k: pieces t and t + 4 of row rows::row_of(g) of either
   __device__ __forceinline__ void take(uint4 (&a)[2], uint4 (&b)[2]) {
-    const int lane = threadIdx.x & 31, r = reg_row_of(lane >> 2);
+    const int lane = threadIdx.x & 31, r = rows::row_of(lane >> 2);
     const uint32_t row = ring + slot + r * 128, c = (uint32_t)((lane & 3) ^ r) << 4;
     asm volatile("cp.async.wait_group %0;" ::"n"(REG_SLOTS - 1) : "memory");
     __syncwarp();
-    a[0] = reg_lds16(row + c); a[1] = reg_lds16(row + (c ^ 64));
-    b[0] = reg_lds16(row + 1024 + c); b[1] = reg_lds16(row + 1024 + (c ^ 64));
+    a[0] = rows::lds16(row + c); a[1] = rows::lds16(row + (c ^ 64));
+    b[0] = rows::lds16(row + 1024 + c); b[1] = rows::lds16(row + 1024 + (c ^ 64));
     __syncwarp();
     ask(slot);
     slot = slot + REG_SLOT_BYTES == REG_SLOTS * REG_SLOT_BYTES ? 0u : slot + REG_SLOT_BYTES;
@@ -193,7 +179,7 @@ __device__ __forceinline__ void reg_product(RegStream& st, const RegPart& p, con
       }
     }
   }
-  float* mine = red + ((warp * subs) * B + 2 * t) * 8 + reg_row_of(g);
+  float* mine = red + ((warp * subs) * B + 2 * t) * 8 + rows::row_of(g);
 #pragma unroll 1
   for (int sub = 0; sub < subs; sub += 2) {
     float acc[NT][4];
@@ -208,8 +194,8 @@ __device__ __forceinline__ void reg_product(RegStream& st, const RegPart& p, con
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-          reg_mma(acc[n], a[h].x, b[h].x, a[h].y, b[h].y, xb[i][n][h].x, xb[i][n][h].y);
-          reg_mma(acc[n], a[h].z, b[h].z, a[h].w, b[h].w, xb[i][n][h].z, xb[i][n][h].w);
+          rows::mma_step(acc[n], a[h].x, b[h].x, a[h].y, b[h].y, xb[i][n][h].x, xb[i][n][h].y);
+          rows::mma_step(acc[n], a[h].z, b[h].z, a[h].w, b[h].w, xb[i][n][h].z, xb[i][n][h].w);
         }
     }
 #pragma unroll

@@ -3,7 +3,7 @@
 // gemm_sk.cu feeds the 128-row weight tile as the UMMA *A* operand and the sessions as N ("swap-AB"): right while the batch is
 // tiny, but a tcgen05.mma with M = 128 occupies the tensor pipe for ~120-140 cycles whatever N <= 128 is (measured: the stream-K
 // kernel runs the same copy pipeline 1.8x slower with its MMAs switched on than with them off, and cuBLAS beats it on every LM
-// shape from 48 sessions up, profiles/r02_a_kbench_gemm_vs_cublas_mimi.jsonl).  Here the operands keep their textbook roles:
+// shape from 48 sessions up).  Here the operands keep their textbook roles:
 //
 //   * A = the activations, one [128 sessions x 64 k] SWIZZLE_128B box per k-block (2-D TMA, rows beyond M zero-filled; two such
 //     blocks and two accumulators above 128 sessions);
@@ -330,8 +330,7 @@ bool ns_supported(int M, int N, int K, int epi) {
 
 int ns_prepare() { return ns_init(); }
 
-// The LM's choice of unit and K-split for a shape, from measurements on B200 at 48 / 104 sessions
-// (profiles/r02_c_kbench_ns_sweep.jsonl, profiles/r02_d_kbench_ns_sweep_m104.jsonl):
+// The LM's choice of unit and K-split for a shape, from measurements on B200 at 48 / 104 sessions:
 //   * >= 40 pairs of tiles (in_proj 48, the gated MLP's input 88, the text head 125): N = 256 units, two K-splits while both CTAs
 //     of every unit are resident at once (in_proj: 96 CTAs), else one;
 //   * fewer (out_proj / linear_out: 32 tiles, depformer_in: 64): single-tile units (N = 128) so that more SMs pull on the

@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "gemm_reg.cuh"
+#include "row_stream.cuh"
 #include "tc_prims.cuh"
 
 namespace b200 {
@@ -22,6 +23,7 @@ namespace tc {
 namespace {
 
 using namespace tcp;
+using namespace rows;
 
 constexpr int EPI_STORE = 0, EPI_RESADD = 1, EPI_GATE = 2;
 constexpr int THREADS = 256, ROWS = 128, TILE16 = 1024;      // 16-byte pieces of a tile (128 rows x 128 bytes)
@@ -45,14 +47,6 @@ __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
   uint4 v;
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
-}
-__device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_step(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 template <int EPI, bool I8>
@@ -212,10 +206,10 @@ cudaError_t launch_nt(const cudaLaunchConfig_t& cfg, const RegP& p) {
 
 }  // namespace
 
-// Where the kernel is ahead of gemm_sk.cu (7B shapes, bf16, us): everything up to 8 rows (4096 -> 4096 22.9 -> 10.8, -> 12288 30.9 -> 22.1); up to 32
-// rows too (32 rows 41.0 -> 17.0 and 35.7 -> 29.8) but for gated pairs beyond 16 rows, whose fragments left one CTA per SM (52 -> 64; not built), and
-// for 16-bit weights of more tiles than SMs beyond 8 rows, where whole tiles per CTA leave the second CTA of an SM idle (250 tiles, 32 rows
-// 55.6 -> 67.9; 8 rows 53.8 -> 51.9; int8 39.4 -> 38.1).
+// Where the kernel is ahead of gemm_sk.cu, asked where gemm_row.cu does not take the shape: 17 to 32 rows, and 16-bit gated pairs of up to 16 rows that it leaves (fewer
+// rows come here through b200_op_linear_reg and B200_ROW_MAX_M only).  7B shapes, bf16, us: up to 32 rows of as many tiles as SMs (4096 -> 4096 41.0 -> 17.0, -> 12288
+// 35.7 -> 29.8), and any width up to 8 rows, but not gated pairs beyond 16 rows, whose fragments left one CTA per SM (52 -> 64; not built), nor 16-bit weights of
+// more tiles than SMs beyond 8 rows, where whole tiles per CTA leave the second CTA of an SM idle (250 tiles, 32 rows 55.6 -> 67.9; int8 39.4 -> 38.1).
 bool reg_wins(int M, int N, int epi, int gate_rows, bool i8, int sms) {
   const int tiles = ((epi == EPI_GATE ? gate_rows : N) + ROWS - 1) / ROWS;
   return i8 || M <= 8 || tiles <= sms;

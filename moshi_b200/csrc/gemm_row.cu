@@ -10,21 +10,25 @@
 //   * a pair of units, or the gate and value rows of one, is the A fragment of mma.sync m16n8k16 (int8 m16n8k32); which k a slot holds does not matter as
 //     long as the activations' fragment agrees, so every thread takes whole 16-byte pieces of the tiles;
 //   * activations of KC k-blocks are in registers; the warps' sums meet in shared memory, as many units at a time as fit;
-//   * every launch asks for more than half of an SM's shared memory.  With two CTAs to an SM an early launch (programmatic dependent launch) puts both of the
-//     next linear's on whichever SM is done first, and the kernel takes as long as that SM: a step of one session 4457 -> 4537 us, and 4107 with one.
+//   * one CTA fits an SM (512 threads of 98 to 109 registers): with two, early launches would put both of the next linear's on whichever SM is done first.
 //
-// Bound by HBM, start and end.  7B shapes, cold weights, launched alone, us, before (K cut over CTAs) / now / weights at 6.55 TB/s:
-//   1 row: 4096 -> 12288 24.4 / 20.5 / 15.4, 4096 -> 4096 12.4 / 10.3 / 5.1, gated -> 11264 36.6 / 31.2 / 28.2, 11264 -> 4096 20.5 / 18.5 / 14.1, -> 32000 49.6 / 43.3 / 40.0;
-//   8 rows: 24.1 / 21.2, 12.9 / 10.5, 33.0 / 33.7, 23.1 / 19.6, 52.6 / 45.7; 16 rows: 26.2 / 22.6, 14.5 / 12.4, -, 26.1 / 22.6, 55.4 / 51.3;
-//   1024 -> 3072 8.3 / 6.2, 2816 -> 1024 9.5 / 6.2; int8 4096 -> 12288 19.4 / 16.5, 11264 -> 4096 18.5 / 18.5.
+// Bound by HBM, start and end.  7B shapes, cold weights, behind one another through the entry points (early launches that wait), us, gemm_reg.cu (K cut over CTAs) /
+// this kernel / weights at 6.55 TB/s:
+//   1 row: 4096 -> 12288 22.4 / 18.0 / 15.4, 4096 -> 4096 11.0 / 7.6 / 5.1, gated -> 11264 31.8 / 29.5 / 28.2, 11264 -> 4096 21.2 / 16.5 / 14.1, -> 32000 51.2 / 40.9 / 40.0;
+//   8 rows: 22.9 / 19.1, 11.2 / 8.1, 32.2 / 31.4, 21.5 / 17.1, 51.4 / 43.6; 16 rows: 24.8 / 20.6, 13.1 / 9.8, -, 24.2 / 20.1, 53.2 / 48.0;
+//   1024 -> 3072 5.6 / 3.9, 2816 -> 1024 6.3 / 4.2; int8 4096 -> 12288 13.5 / 10.2, 11264 -> 4096 13.0 / 9.9.
+// Launched alone (clean caches, with about 5 us of launch and events): 1 row 26.6 / 22.5, 16.4 / 12.3, 36.8 / 34.0, 26.5 / 20.5, 55.3 / 45.1; gated 8 rows 36.9 / 36.4.
+// Counters (1 row of 4096 -> 12288): DRAM 60 % over the whole launch, L2 hits 0.6 %, warps wait for their weights (6.3 of 11.4 cycles an instruction).
 // Error of the sums alone (terms whose exact sum is 0, over the rms of a random sum of them), 4096 -> 12288: 1 row 6.9e-8 (fp32 FMAs 7.4e-8; chains of 16 instructions
 // 1.27e-7), 12 rows 8.4e-8 (gemm_reg.cu 6.7e-7); 11264 -> 4096: 1 row 7.7e-8 (8.5e-8; 1.31e-7).
-// Steps of the 7B: 1 session 4470 -> 4014 us, 3: 4610 -> 4223, 8: 4765 -> 4397, 16 with full rings 6980 -> 6560.
+// Steps of the 7B, before this kernel and the weight streams of dep_reg.cuh / with this kernel alone / now: 1 session 4482 / 4014 / 3657 us, 3: 4605 / 4223 / 3857, 8: 4761 / 4397 /
+// 4053, 16 with full rings 6960 / 6560 / 6017.
 #include "gemm_row.cuh"
 
 #include <algorithm>
 #include <type_traits>
 
+#include "row_stream.cuh"
 #include "tc_prims.cuh"
 
 namespace b200 {
@@ -33,6 +37,7 @@ namespace tc {
 namespace {
 
 using namespace tcp;
+using namespace rows;
 
 constexpr int EPI_STORE = 0, EPI_RESADD = 1, EPI_GATE = 2;
 constexpr int THREADS = 512, WARPS = 16, UNIT = 8;
@@ -40,7 +45,6 @@ constexpr int TILE = 16384, UNIT_BYTES = 1024;   // a tile: 128 rows x 128 bytes
 constexpr int SLOTS = 2;                         // pairs of units under way per warp: 64 KB per SM
 constexpr int RING_BYTES = SLOTS * WARPS * 2 * UNIT_BYTES;
 constexpr int RED_BYTES = 128 * 1024;            // the warps' sums of one pass
-constexpr int ONE_PER_SM = 116 * 1024;           // shared memory of which no two fit an SM
 
 struct RowP {
   int M, out_rows, units, num_kb, subs_pass;     // subs_pass: 8-row pieces (gate and value rows apart) of a pass, even
@@ -54,23 +58,6 @@ struct RowP {
 };
 
 __device__ __forceinline__ float rbf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-__device__ __forceinline__ void copy16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ uint4 lds16(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_step(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// A piece c of a packed row r lies at position c ^ (r & 7).  Fragment rows are taken as 0, 4, 1, 5, ..: the eight lanes of a 16-byte read phase hold two of
-// them, whose pieces then lie in the two halves of the banks.
-__device__ __forceinline__ int row_of(int g) { return (g >> 1) | ((g & 1) << 2); }
 
 template <int EPI, int NT, bool I8>
 __global__ void __launch_bounds__(THREADS, 1) gemm_row_kernel(const RowP p) {
@@ -244,8 +231,9 @@ cudaError_t launch_nt(const cudaLaunchConfig_t& cfg, const RowP& p) {
 
 }  // namespace
 
-// Everything but 16-bit gated pairs of so many rows that their sums need a second pass, which reads the activations again (4096 -> 11264, us, register
-// kernel / this one: 12 rows, one pass 36.3 / 34.9; 16 rows, two passes 36.3 / 37.1).
+// Everything but 16-bit gated pairs of so many rows that their sums need a second pass, which reads the activations again.  Behind one another, us, register kernel /
+// this one: 4096 -> 11264, one pass, 3 rows 32.0 / 29.9, 6 rows 32.1 / 30.7, 8 rows 32.2 / 31.4, 12 rows 35.2 / 32.4; two passes, 16 rows 35.4 / 34.9 (alone the same); but
+// 4096 -> 28672, two passes, 6 rows 72.6 / 74.4, four, 16 rows 78.8 / 84.4 (there gemm_sk.cu's kernel).
 bool row_wins(int M, int epi, int gate_rows, bool i8, int sms) {
   if (M > ROW_MAX_M) return false;
   if (epi != EPI_GATE || i8) return true;
@@ -279,7 +267,7 @@ int row_linear(const void* x, long long ldx_bytes, const void* w_tiles, __nv_bfl
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(THREADS); cfg.stream = stream;
-  cfg.dynamicSmemBytes = std::max<size_t>(ONE_PER_SM, RING_BYTES + (size_t)WARPS * std::min(p.subs_pass, most) * M * UNIT * 4);
+  cfg.dynamicSmemBytes = RING_BYTES + (size_t)WARPS * std::min(p.subs_pass, most) * M * UNIT * 4;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;

@@ -948,7 +948,7 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   // Cutting a tile into S pieces moves S fp32 partials of [128 x Mpad] through L2 (written + read back): allow it
   // only while that stays under half of the tile's weight bytes, i.e. S <= 8 * num_kb / Mpad.
   int s_max = tune.no_split ? 1 : (8 * p.num_kb) / p.Mpad;      // int8 partials are int32 and add exactly
-  // measured on B200 (profiles/r01_c_kbench.jsonl): with more than 32 sessions the publish / count / re-read protocol
+  // measured on B200: with more than 32 sessions the publish / count / re-read protocol
   // costs more than the idle SMs it recovers, so tiles stay whole there
   if (p.Mpad > 32 && tune.force_split == 0) s_max = 1;
   if (s_max < 1) s_max = 1;

@@ -103,7 +103,7 @@ struct DepFusedConfig {
 };
 constexpr int DEP_TRACE_SLOTS = 512;
 struct DepFused;
-bool dep_fused_in_registers(const DepFusedConfig& c);      // few sessions: the kernel of dep_reg.cuh
+bool dep_fused_few_sessions(const DepFusedConfig& c);      // few sessions: the kernel of dep_reg.cuh
 size_t dep_fused_partial_floats(const DepFusedConfig& c);
 int dep_fused_create(const DepFusedConfig& c, DepFused** out);
 void dep_fused_set_sampling(DepFused* d, int use_sampling, float temp, int top_k);

@@ -145,8 +145,8 @@ int linear(b200_lm* h, const bf16* x, long long ldx, const bf16* w, bf16* y, lon
   return tc::sk_linear(h->plans, x, ldx, w, y, ldy, res, ldr, M, N, K, epi, gate_rows, h->sk_ws, h->sk_counters, t, h->body);
 }
 
-// y = epi(rmsnorm(x, alpha) . w^T).  (The norm folded into the linear, every CTA summing the squares itself, is slower: 4107 -> 4172 us per step at 2
-// sessions, 4445 -> 4716 at 8.)
+// y = epi(rmsnorm(x, alpha) . w^T).  (The norm folded into the linear, every CTA summing the squares itself, is slower: 2 sessions 4107 -> 4172 us per step, 8 sessions
+// 4445 -> 4716, both before the depformer's weight streams.)
 int norm_linear(b200_lm* h, const bf16* x, const bf16* alpha, bf16* xn, const bf16* w, bf16* y, long long ldy, int M, int N, int K,
                 int epi, int gate_rows, const float* w_scales) {
   B200_TRY(launch_early_if(h->pdl != 0, rmsnorm_kernel, dim3(M), dim3(256), 0, h->body, x, alpha, xn, K, 1e-8f));
@@ -668,12 +668,12 @@ int b200_lm_streaming_begin(b200_lm* h, int batch, void* stream) {
     B200_TRY(A.alloc_t(&h->xq_scale, (size_t)MB, false));
   }
   // One or two sessions of a shape that dep_reg.cuh does not take: PDL-chained launches beat the
-  // shared-memory kernel (B=1: 5.5 vs 6.4 ms per LM step, B=2: 6.2 vs 7.1; profiles/r01_r_*).  B200_DEP_FUSED=2 forces the kernel at any batch.
+  // shared-memory kernel (B=1: 5.5 vs 6.4 ms per LM step, B=2: 6.2 vs 7.1).  B200_DEP_FUSED=2 forces the kernel at any batch.
   // Under classifier-free guidance the two halves of the batch meet before every sampler (lm.py:828-833): launch chain.
   tc::DepFusedConfig few;
   memset(&few, 0, sizeof(few));
   few.B = B; few.dd = dd; few.F = c.depformer_ffn_hidden; few.card = c.card; few.dep_q = c.dep_q; few.L = c.depformer_num_layers;
-  const bool dep_small = B <= 2 && h->dep_fused != 2 && !tc::dep_fused_in_registers(few);
+  const bool dep_small = B <= 2 && h->dep_fused != 2 && !tc::dep_fused_few_sessions(few);
   h->depf = nullptr;
   if (c.dep_q > 0 && !cfg && !c.quantize && h->dep_fused && !dep_small && B <= 256 && dd <= 1024 && dd % 64 == 0) {
     tc::DepFusedConfig fc;

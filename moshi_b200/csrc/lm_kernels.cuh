@@ -884,7 +884,7 @@ static __device__ float block_reduce(float v, bool is_max, float* red) {
   return t;
 }
 
-// One row per call; every thread of a WIDTH-wide CTA must call it (256 at least) (block-wide barriers inside).  No __restrict__ on the logits: the
+// One row per call; every thread of a CTA of WIDTH (at least 256) must call it, for there are block-wide barriers inside.  No __restrict__ on the logits: the
 // persistent depformers call this between grid barriers, where other CTAs wrote the row after this one may have cached the line it begins in.
 template <int WIDTH = SAMPLE_THREADS>
 static __device__ void sample_row(const bf16* logits, const float* __restrict__ noise, long long* __restrict__ out,

@@ -46,9 +46,9 @@ static int sk_scratch(float** ws, int** counters, int kind = SCRATCH_BF16) {
   return scratch(kind, tc::sk_workspace_bytes(256) / sizeof(float), tc::SK_MAX_TILES, ws, counters);
 }
 
-// The entry points of a step's kernels are launched early and wait before they read anything (B200_PDL=0: ordinary launches): behind one
-// another the next one's CTAs are set up while the last one drains (us, ordinary / early: gated linear of 6 rows in the register kernel 33.4 / 31.2, 4096 -> 12288 of 104 rows
-// 30.8 / 29.1, attention of 48 sessions 159.2 / 157.5).
+// The entry points of a step's kernels are launched early and wait before they read anything (B200_PDL=0: ordinary launches): behind one another the next one's
+// CTAs are set up while the last one drains (us, ordinary / early: gated linear of 6 rows 32.8 / 30.5, 4096 -> 12288 of 104 rows 30.7 / 28.6, int8 11264 -> 4096 of 24 rows
+// 20.5 / 18.5, attention of 48 sessions 159.2 / 157.5).  A call on an idle stream gains nothing: 34.8, 32.8, 24.5 either way, launch and events included.
 static int op_pdl() {
   static const int on = [] { const char* e = getenv("B200_PDL"); return !e || atoi(e) != 0; }();
   return on ? tc::PDL_WAIT_FIRST : tc::PDL_OFF;

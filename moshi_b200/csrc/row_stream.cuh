@@ -1,0 +1,29 @@
+// What the kernels have in common that stream packed weights past activations in registers (gemm_row.cu, dep_reg.cuh, gemm_reg.cu): 16-byte copies into a warp's own
+// ring, and products of 16 weight rows and 8 activation rows.
+#pragma once
+
+#include "common.cuh"
+
+namespace b200 {
+namespace rows {
+
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ uint4 lds16(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_step(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// A piece c of a packed row r lies at position c ^ (r & 7).  Fragment rows are taken as 0, 4, 1, 5, ..: the eight lanes of a 16-byte read phase hold two of
+// them, whose pieces then lie in the two halves of the banks.
+__device__ __forceinline__ int row_of(int g) { return (g >> 1) | ((g & 1) << 2); }
+
+}  // namespace rows
+}  // namespace b200

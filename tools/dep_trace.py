@@ -17,11 +17,11 @@ os.environ["B200_DEP_TRACE"] = "1"
 import torch  # noqa: E402
 
 
-def phase_names(dep_q: int, L: int, in_registers: bool) -> list[str]:
+def phase_names(dep_q: int, L: int, few_sessions: bool) -> list[str]:
     """Phase that ENDS at barrier e (1-based), in the kernel's order (dep_reg.cuh: few sessions; dep_fused.cu)."""
     names = []
     for k in range(dep_q):
-        if in_registers:
+        if few_sessions:
             names.append("input" if k == 0 else "sample+input")
             names += ["norm+in_proj", "attn", "out_proj", "norm+lin_in+gate", "lin_out"] * L + ["head"]
             continue
