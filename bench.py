@@ -9,7 +9,7 @@ so scaling is weak and ``value`` sums the sessions of all ranks.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference] [--sessions B_per_gpu]
 
-Prints ONE JSON line (rank 0).  See DESIGN.md "Measurement" for the definition of every field.
+Prints ONE JSON line (rank 0).
 """
 from __future__ import annotations
 
@@ -31,7 +31,7 @@ import torch  # noqa: E402
 
 METRIC = "concurrent real-time sessions @ <=80 ms/step (Mimi encode + Moshi 7B LMGen.step + Mimi decode)"
 FRAME_MS = 80.0
-KV_BYTES_PER_SESSION_STEP = 524288      # 32 layers x 2 x 4096 x bf16 per cached position (SURVEY.md 8d)
+KV_BYTES_PER_SESSION_STEP = 524288      # 32 layers x 2 x 4096 x bf16 per cached position
 
 
 def sessions_sustained(total_sessions: float, ms_per_step: float) -> float:
@@ -285,7 +285,7 @@ def _gemm_roofline(B: int, device) -> dict:
 
 
 def _lm_single_session(lm, device, peak: float) -> dict:
-    """BASELINE config 3: Moshi 7B bf16 ``LMGen.step`` for ONE session (what scripts/moshi_benchmark.py:76-95 times): p50 / p90 of
+    """Moshi 7B bf16 ``LMGen.step`` for ONE session (what scripts/moshi_benchmark.py:76-95 times): p50 / p90 of
     200 steps after 20 warm-up steps, CUDA events per step, at ring fill 200 and with the ring full; xRT = 80 ms / p50."""
     from moshi_b200.models import LMGen
     out = {}
@@ -1343,7 +1343,7 @@ def main() -> None:
     ap.add_argument("--kv-dtype", choices=["bf16", "fp8_e4m3", "int8"], default="bf16",
                     help="storage of the temporal KV rings; fp8_e4m3 / int8 are opt-in extensions outside the reference's numerics "
                          "(half the ring, twice the sessions per GPU; logit error in tests/test_gpu_zv_kv_q8.py)")
-    ap.add_argument("--quantize", action="store_true", help="BASELINE config 5: int8 (W8A8 QLinear) Moshi 7B instead of bf16")
+    ap.add_argument("--quantize", action="store_true", help="int8 (W8A8 QLinear) Moshi 7B instead of bf16")
     ap.add_argument("--decoder-lm", action="store_true",
                     help="instead of the default workload: prefill / decode throughput of the text-only decoder LM (Likosun design, random "
                          "weights) beside the Moshi temporal transformer at equal width and depth; prints its own JSON line")

@@ -42,7 +42,7 @@ def mimi_fixtures(manifest: dict) -> None:
     ref = loaders.get_mimi(None, device="cpu", num_codebooks=cfg.num_codebooks)
     ref.load_state_dict(sd, strict=True)
 
-    # --- config 1: 1 s 440 Hz sine, B=1 (BASELINE.json configs[0]) -------------------------
+    # --- config 1: 1 s 440 Hz sine, B=1 -------------------------
     sine = scenarios.sine_1s()
     codes_batch = ref.encode(scenarios.sine_1s_full())   # non-streaming, 24000 samples: pads to 13 frames
     pcm_batch = ref.decode(codes_batch)

@@ -4,7 +4,7 @@ reference (CPU); records whether the oracle agrees bit for bit.  Build container
 
     python -m oracle.gen_golden_cfg
 
-Oracle groundwork for SURVEY.md 8(f) item 2; the CUDA path does not build CFG yet.
+Test infrastructure.
 """
 from __future__ import annotations
 

@@ -4,7 +4,7 @@
 
     python -m oracle.gen_golden_stt          # build container only: needs /root/reference
 
-Test infrastructure for the next row of SURVEY.md 8(f) item 2; the CUDA path does not implement this configuration yet.
+Test infrastructure.
 """
 from __future__ import annotations
 

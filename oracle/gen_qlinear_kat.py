@@ -2,7 +2,7 @@
 
 The reference's arithmetic for this path lives in bitsandbytes (``moshi/moshi/utils/quantize.py:13-40`` calls
 ``bnbF.int8_vectorwise_quant`` and ``bnb.matmul``), which is neither installed nor vendored, and no reference test or fixture
-touches it: the parity of BASELINE config 5 therefore stays *unpinned against the reference*.  What this KAT
+touches it: the parity of int8 models therefore stays *unpinned against the reference*.  What this KAT
 pins is the restatement itself, against an independent implementation of the published algorithm:
 
   * quantiser: numpy float32, ``q = rint(v * (127 / absmax_row))`` (``np.rint`` rounds half to even), weights through float16

@@ -98,7 +98,7 @@ def sample_token(logits: torch.Tensor, use_sampling: bool, temp: float, top_k: i
     among *equal* probabilities is unspecified (and differs between torch's CPU and CUDA kernels);
     the noise is indexed by rank, so tied bf16 logits make the sample depend on that order.
     "torch" keeps torch.topk (bit-exact with a CPU reference run); "index" ranks ties by ascending
-    token id, which is the order the CUDA sampler defines (tolerances)."""
+    token id, which is the order the CUDA sampler defines."""
     if not (use_sampling and temp > 0.0):
         return torch.argmax(logits, dim=-1)
     probs = torch.softmax(logits / temp, dim=-1)

@@ -11,7 +11,7 @@ Restates the reference's ``MimiModel`` data path with explicit per-layer state:
                                                ``quantization/vq.py:126-151, 269-287``
 * orchestration                              – ``models/compression.py:338-429``
 
-State-dict keys are the reference's (SURVEY.md appendix A).
+State-dict keys are the reference's.
 """
 from __future__ import annotations
 

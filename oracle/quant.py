@@ -7,7 +7,7 @@ row-wise absmax int8 quantisation of the activations too, an int8 x int8 -> int3
 ``SCA[m] * SCB[n] / 127^2``.
 
 **Parity unpinned**: bitsandbytes (``>=0.45,<0.50``, ``moshi/pyproject.toml:9``) is not installed and not vendored, and no
-reference test or fixture touches this path (SURVEY.md 8c), so this file restates the *published* algorithm; the rounding
+reference test or fixture touches this path, so this file restates the *published* algorithm; the rounding
 mode of the quantiser (ties to even, like ``torch.round``) and the fp32 order of the dequantisation are this repo's
 definition, and the CUDA path is checked against it bit for bit (exact integer accumulation).  Deviation from the
 reference kept on purpose: activations and outputs stay bfloat16 (the reference round-trips through float16).

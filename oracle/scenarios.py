@@ -19,7 +19,7 @@ LM_STEPS = 30
 
 
 def sine_1s() -> torch.Tensor:
-    """BASELINE.json configs[0] / SURVEY.md 8(d) config 1: 0.5*sin(2*pi*440*t), 1 s at 24 kHz."""
+    """0.5*sin(2*pi*440*t), 1 s at 24 kHz."""
     t = torch.arange(24000, dtype=torch.float32) / 24000
     x = 0.5 * torch.sin(2 * math.pi * 440 * t)
     return x[None, None, :23040].contiguous()
@@ -77,7 +77,7 @@ def lm_noise(cfg, batch: int, top_k_text: int = 25, top_k: int = 250):
     return nt, na
 
 
-# ---- STT-style member of the family (SURVEY.md 8f item 2): no depformer, extra heads on the temporal output -----------------
+# ---- STT-style member of the family: no depformer, extra heads on the temporal output -----------------
 STT_SEED = 777
 STT_B = 2
 STT_STEPS = 14

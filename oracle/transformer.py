@@ -33,7 +33,7 @@ class TransformerSpec:
     positional_scale: float = 1.0
     quantize: bool = False                # every nn.Linear replaced by QLinear (transformer.py:885-888, utils/quantize.py)
     kv_quant: str = ""                    # NOT a reference option: restates the opt-in 8-bit KV rings of the CUDA path
-                                          # ("fp8_e4m3" | "int8"; DESIGN.md)
+                                          # ("fp8_e4m3" | "int8")
 
 
 @dataclass

@@ -154,7 +154,7 @@ def test_step_outside_streaming_raises(lm):
 
 @torch.no_grad()
 def test_shortened_kv_ring_is_the_reference_ring_until_it_is_full(lm, tiny):
-    """`kv_capacity` (b200_lm_set_kv_capacity; SURVEY 8f item 3, rings sized to live fill): a ring of 8 slots gives the same
+    """`kv_capacity` (b200_lm_set_kv_capacity, rings sized to live fill): a ring of 8 slots gives the same
     logits and tokens as the model's own 12-slot ring for a session's first 8 frames (nothing is evicted before position
     `context`), and the frame that would overwrite a live key raises error flag 4 instead of silently forgetting."""
     from moshi_b200.models import LMGen
@@ -192,8 +192,8 @@ def test_shortened_kv_ring_is_the_reference_ring_until_it_is_full(lm, tiny):
 def test_rows_independent_graph_invariant_and_host_path():
     """Mid-size member of the 7B family at a serving batch, full 3000-slot ring machinery:
     (1) graph replay == eager launches bit for bit, (2) a session's tokens do not depend on its slot or its neighbours
-    (the batch with its rows reversed gives the reversed tokens; a *different batch size* may run other kernels — the GEMV
-    path below five sessions, other split points — so "alone" is only equal up to summation order and is checked on the
+    (the batch with its rows reversed gives the reversed tokens; a *different batch size* may run other kernels and
+    other split points, so "alone" is only equal up to summation order and is checked on the
     7B model's logits below), (3) the host-buffer entry point returns the same tokens, (4) masked rows do not advance."""
     from moshi_b200.models import LMGen, LMModel
     cfg = LMConfig(dim=1024, num_heads=8, num_layers=4, context=3000, text_card=32000, card=2048,
@@ -286,9 +286,9 @@ def test_depformer_replace_tokens(lm, tiny):
 
 
 def test_full_size_7b_properties():
-    """BASELINE's own configuration (configs/moshi_7b_202409.json, random block-tiled weights) is too large for the CPU
+    """The 7B configuration (configs/moshi_7b_202409.json, random block-tiled weights) is too large for the CPU
     oracle, so the full-size step is checked through size-independent properties: graph replay == eager launches; a
-    session's tokens do not depend on its slot or on its neighbours (no cross-row op anywhere, SURVEY 8e: the batch with
+    session's tokens do not depend on its slot or on its neighbours (no cross-row op anywhere: the batch with
     its rows permuted gives the permuted tokens, bit for bit); alone in a batch of one the same session gives the same
     logits up to the fp32 summation order of the split-KV / split-K schedules, which are chosen per batch size; paused
     rows do not move; outputs in range; the ring wraps at slot 3000."""
@@ -326,8 +326,8 @@ def test_full_size_7b_properties():
     paused = run(rows, True, paused=1)
     d = (la[0][3] - ls[0][0]).abs().max().item()
     print(f"7B: text logits of session 3 in a batch of {B} vs alone: max |d| = {d:.3e}")
-    # alone, the linears take the GEMV path (fp32 FMA chains) instead of the tensor-core GEMM: another summation order in every
-    # one of the 32 layers' four linears; bf16 rounding noise (2^-9 per cast) random-walks to ~0.2 on logits of |x| ~ 4
+    # alone, the attention cuts its keys into other ranges than in a batch of five (the linears add in the same order): another rounding in every one of the 32
+    # layers; bf16 rounding noise (2^-9 per cast) random-walks to ~0.2 on logits of |x| ~ 4
     assert d < 0.35
     for i in range(1, steps):
         assert torch.equal(eager[i], graph[i]), i
@@ -405,9 +405,8 @@ def test_fused_depformer_equals_launch_chain(B, monkeypatch):
 
 
 @pytest.mark.parametrize("B", [1, 2])
-def test_one_and_two_sessions_take_the_gemv_path(lm, tiny, B):
-    """Below three sessions every linear runs as gemv_kernel (plain loads, RMSNorm folded into the activation staging) and
-    the depformer as a launch chain: same oracle, same tolerance, teacher-synchronised greedy steps across the ring wrap."""
+def test_one_and_two_sessions_match_the_oracle(lm, tiny, B):
+    """One and two sessions (whole output rows per CTA; the depformer of few sessions): same oracle, same tolerance, teacher-synchronised greedy steps across the ring wrap."""
     from moshi_b200.models import LMGen
     cfg, sd = tiny
     steps = 16
@@ -436,7 +435,7 @@ def test_one_and_two_sessions_take_the_gemv_path(lm, tiny, B):
             for b in range(B):
                 orc.cache[b, 0, pos[b]] = tt[b]
                 orc.cache[b, 1:cfg.dep_q + 1, pos[b]] = at[:, b]
-    print(f"B={B} (GEMV path): worst logit diff {worst:.3e}, greedy tokens equal {agree}/{total}")
+    print(f"B={B} (few rows): worst logit diff {worst:.3e}, greedy tokens equal {agree}/{total}")
     assert worst < LOGIT_ATOL
     assert agree / total > 0.95
 

@@ -77,7 +77,7 @@ def test_layer_by_layer_first_frames(gpu, sd):
 
 @torch.no_grad()
 def test_rvq_kernel_is_exact_on_the_oracle_latent(gpu, sd):
-    """Isolates the nearest-codebook search from encoder numerics (SURVEY.md 7 'minimum slice')."""
+    """Isolates the nearest-codebook search from encoder numerics."""
     orc = MimiOracle(sd, MimiConfig())
     B, frames = 4, 6
     orc.streaming(B)
@@ -98,7 +98,7 @@ def test_rvq_kernel_is_exact_on_the_oracle_latent(gpu, sd):
 
 @torch.no_grad()
 def test_golden_sine_roundtrip(gpu, sd, golden_dir):
-    """BASELINE.json configs[0]: 1 s 440 Hz sine, B=1; codes exact (margin-aware), PCM within tolerance."""
+    """1 s 440 Hz sine, B=1; codes exact (margin-aware), PCM within tolerance."""
     gold = load_file(golden_dir / "mimi_sine.safetensors")
     cfg = MimiConfig()
     orc = MimiOracle(sd, cfg)
@@ -157,7 +157,7 @@ def test_golden_masked_rows_and_reset(gpu, sd, golden_dir):
 
 @torch.no_grad()
 def test_long_stream_ten_thousand_frames(gpu, sd):
-    """40 sessions x 260 frames = 10 400 session-frames of streaming encode + decode beside the oracle (VERDICT r1 item 2: the
+    """40 sessions x 260 frames = 10 400 session-frames of streaming encode + decode beside the oracle (the
     3xTF32 tensor-core path must keep the RVQ indices exact over long streams): every code compared margin-aware (zero
     unexcused flips), PCM within tolerance on every frame, and the 250-slot rings of both bottleneck transformers wrap on
     the way (frames 250..259 overwrite the oldest keys)."""

@@ -1,4 +1,4 @@
-"""GPU: other members of the model family behind the same kernels (SURVEY.md 8f item 2)."""
+"""GPU: other members of the model family behind the same kernels."""
 import pytest
 import torch
 from safetensors.torch import load_file
@@ -232,13 +232,13 @@ def test_2b_shape_family_member_against_the_oracle():
     agree, total, worst, _ = _run_greedy(cfg, sd, None, steps, B, codes)
     print(f"2B-shaped tiny model: tokens equal to oracle {agree}/{total}, worst logit diff {worst:.3e}")
     assert worst < LOGIT_ATOL and agree / total > 0.95
-    # batch >= 3 runs the fused depformer kernel; B = 1 takes the GEMV launch chain
+    # one session: the same kernels with a part-empty block of eight
     agree, total, worst, _ = _run_greedy(cfg, sd, None, steps, 1, codes[:, :1])
     assert worst < LOGIT_ATOL and agree / total > 0.95
 
 
 def test_out_of_range_tokens_raise_a_flag_instead_of_reading_out_of_bounds():
-    """token ids outside the embedding tables (the reference would hit a device assert in F.embedding) embed as
+    """Token ids outside the embedding tables (the reference would hit a device assert in F.embedding) embed as
     the zero row and raise the device error flag; ``check=True`` surfaces it like lm.py:704-711."""
     from moshi_b200.config import tiny_lm_config
     from moshi_b200.models import LMGen, LMModel

@@ -1,7 +1,7 @@
 """GPU: the opt-in 8-bit temporal KV rings (one byte per element + one fp32 scale per key row): e4m3 and int8.
 
 This is NOT the reference's numerics (its ring is bf16, transformer.py:196-288); it exists to halve the 1.57 GB a
-session's rings take (SURVEY.md 8f item 3).  Two levels:
+session's rings take.  Two levels:
   * the fused attention step kernel against an fp32 emulation that stores ``e4m3(x * 448/absmax) * absmax/448`` (or
     ``round(x * 127/absmax) * absmax/127``) for the appended key / value row and attends over the dequantised ring: the
     kernel must agree with that to bf16 rounding, and the bytes + scales it wrote must be the emulation's;

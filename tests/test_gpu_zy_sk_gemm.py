@@ -135,9 +135,9 @@ def test_cluster_split_k(M, N, K, epi):
 @pytest.mark.parametrize("M", [1, 2, 3, 4])
 @pytest.mark.parametrize("N,K,epi", [(4096, 4096, STORE), (12288, 4096, STORE), (4096, 11264, RESADD), (1024, 2816, RESADD),
                                      (22528, 4096, GATE), (5632, 1024, GATE), (200, 192, STORE)])
-def test_gemv_path_equals_tensor_core_path(M, N, K, epi):
-    """One to four sessions: the same pre-tiled weights streamed with plain loads on the CUDA cores (gemv_kernel) against fp32
-    math and against the tensor-core GEMM (both accumulate in fp32; only the summation order differs)."""
+def test_whole_rows_equal_the_register_kernel(M, N, K, epi):
+    """One to four sessions: the kernel of whole output rows per CTA against fp32 math and against the one that cuts K over CTAs (gemm_reg.cu), on the same
+    packed weights (both accumulate in fp32; only the summation order differs)."""
     from moshi_b200 import _lib
     lib = _lib.lib()
     g = torch.Generator().manual_seed(M * 5 + N)
@@ -157,17 +157,17 @@ def test_gemv_path_equals_tensor_core_path(M, N, K, epi):
         want = (F.silu(h[:, :gate_rows].float()).bfloat16() * h[:, gate_rows:]).float()
     before = lib.b200_op_set_gemv_max_rows(4)
     try:
-        y_gemv = _run(lib, x, wt, res, M, N, K, epi, gate_rows)
+        y_rows = _run(lib, x, wt, res, M, N, K, epi, gate_rows)
         again = _run(lib, x, wt, res, M, N, K, epi, gate_rows)
         lib.b200_op_set_gemv_max_rows(0)
-        y_mma = _run(lib, x, wt, res, M, N, K, epi, gate_rows)
+        y_reg = _run(lib, x, wt, res, M, N, K, epi, gate_rows)
     finally:
         lib.b200_op_set_gemv_max_rows(before)
-    print(stats(f"gemv {M}x{N}x{K} epi={epi}", y_gemv, want), "| vs tensor-core path:", stats("", y_gemv, y_mma.float()))
-    assert not torch.isnan(y_gemv.float()).any()
-    torch.testing.assert_close(y_gemv.float(), want, rtol=2e-2, atol=3e-2)
-    assert torch.equal(y_gemv, again)                                   # split partials are summed in split order
-    assert ((y_gemv.float() - y_mma.float()).abs() > 0).float().mean() < 0.05      # a bf16 ulp apart now and then
+    print(stats(f"rows {M}x{N}x{K} epi={epi}", y_rows, want), "| vs register kernel:", stats("", y_rows, y_reg.float()))
+    assert not torch.isnan(y_rows.float()).any()
+    torch.testing.assert_close(y_rows.float(), want, rtol=2e-2, atol=3e-2)
+    assert torch.equal(y_rows, again)                                   # the warps' sums are added in a fixed order
+    assert ((y_rows.float() - y_reg.float()).abs() > 0).float().mean() < 0.05      # a bf16 ulp apart now and then
 
 
 def _run_ns(lib, x, wt, res, M, N, K, epi, gate_rows, cluster=0):

@@ -17,13 +17,13 @@ ROOT = Path(__file__).resolve().parent.parent
 
 
 def test_7b_config_matches_reference_json():
-    # values of configs/moshi_7b_202409.json (SURVEY.md 8a)
+    # values of configs/moshi_7b_202409.json
     c = MOSHI_7B
     assert (c.dim, c.num_layers, c.num_heads, c.context) == (4096, 32, 32, 3000)
     assert c.ffn_hidden == 11264 and c.depformer_ffn_hidden == 2816
     assert c.max_delay == 1 and c.num_codebooks == 17
     total = sum(int(torch.tensor(shape).prod()) for _, shape, _ in lm_tensor_specs(c))
-    assert abs(total / 1e9 - 7.688) < 0.01            # SURVEY.md: 7.688 B parameters
+    assert abs(total / 1e9 - 7.688) < 0.01            # 7.688 B parameters
 
 
 def test_lm_config_rejects_options_outside_hot_path():
@@ -36,7 +36,7 @@ def test_lm_config_rejects_options_outside_hot_path():
         LMConfig.from_dict({**d, "conditioners": {"speaker": {"type": "tensor", "tensor": {"dim": 512}}}})
     with pytest.raises(ValueError):
         LMConfig.from_dict({**d, "fuser": {"cross": ["description"]}})
-    with pytest.raises(ValueError):                    # ADVICE r1: options that used to load silently
+    with pytest.raises(ValueError):                    # options that used to load silently
         LMConfig.from_dict({**d, "causal": False})
     with pytest.raises(ValueError):
         LMConfig.from_dict({**d, "depformer_context": 4})
@@ -58,7 +58,7 @@ def test_mimi_config_roundtrip_and_layout():
     assert cfg.frame_size == 1920 and cfg.hop_length == 960 and cfg.resample_stride == 2
     assert MimiConfig.from_reference_dict(cfg.to_reference_dict()) == cfg
     enc, dec = seanet_layout(cfg)
-    assert [l[1] for l in enc if l[0] == "conv"] == [0, 3, 6, 9, 12, 14]     # SURVEY.md appendix A
+    assert [l[1] for l in enc if l[0] == "conv"] == [0, 3, 6, 9, 12, 14]
     assert [l[1] for l in dec if l[0] == "convtr"] == [2, 5, 8, 11]
     for section, key, value in (("seanet", "pad_mode", "reflect"), ("seanet", "activation", "ReLU"), ("seanet", "causal", False),
                                 ("seanet", "disable_norm_outer_blocks", 1), ("transformer", "causal", False),

@@ -98,7 +98,7 @@ def test_step_outside_streaming_raises():
 def test_lm_stt_extra_heads(golden_dir):
     """STT-style member of the family (no depformer, ``extra_heads``; ``LMGen.step_with_extra_heads``, lm.py:793-807 — what
     ``rust/moshi-server/batched_asr.py:197`` calls): the oracle reproduces the fixture recorded from the unmodified reference
-    bit for bit, including the recycled slot.  Groundwork for SURVEY.md 8(f) item 2; the CUDA path does not build it yet."""
+    bit for bit, including the recycled slot."""
     import json
 
     info = json.loads((golden_dir / "lm_stt_tiny.json").read_text())
@@ -146,7 +146,7 @@ def test_lm_delay2_pattern(golden_dir):
 def test_lm_cfg_without_conditioner(golden_dir, mode):
     """Classifier-free guidance without a conditioner (``cfg_coef != 1`` with ``cfg_is_no_text`` / ``cfg_is_masked_until``,
     lm.py:596-604, 646-662, 714-732, 820-833): 2B model rows, guided text and depformer logits; the oracle reproduces the
-    fixture recorded from the unmodified reference, including a slot reset.  Groundwork for SURVEY.md 8(f) item 2."""
+    fixture recorded from the unmodified reference, including a slot reset."""
     info = json.loads((golden_dir / "lm_tiny_cfg.json").read_text())
     assert info["modes"][mode]["oracle_bit_exact_tokens"] is True
     gold = load_file(golden_dir / "lm_tiny_cfg.safetensors")[mode]

@@ -57,7 +57,7 @@ def test_quantized_lm_oracle_steps_close_to_bf16():
 
 
 def test_qlinear_known_answers(golden_dir):
-    """The KAT SURVEY.md 8(c) asks for: ``oracle/quant.py`` against an independent implementation of the published QLinear
+    """``oracle/quant.py`` against an independent implementation of the published QLinear
     algorithm (numpy float32 quantiser with half-to-even rounding, exact Python-integer products, float64 dequantisation;
     ``oracle/gen_qlinear_kat.py``).  It pins the restatement, not bitsandbytes itself (absent: parity stays unpinned)."""
     import json

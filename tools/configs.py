@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""BASELINE.json configs 2-5 through the reference-shaped API, one JSON object per line.
+"""The workloads 2-5 below through the reference-shaped API, one JSON object per line.
 
     python tools/configs.py --config 2              # Mimi streaming encode+decode, B = 1 .. 256
     python tools/configs.py --config 3              # Moshi 7B LMGen.step, B = 1: p50/p90 latency, xRT (fill 200 and full ring)
@@ -133,7 +133,7 @@ def config4(sessions: int):
 
 def config4_shards():
     """The 512-session configuration as written (512 / N sessions per GPU): which history the bf16 rings can hold when that many
-    sessions share one GPU ("the fill level at which 512 fit"), with the rings sized to it (`kv_capacity`,
+    sessions share one GPU (the fill level at which 512 fit), with the rings sized to it (`kv_capacity`,
     reference numerics until a session is that old) — N = 2 (256 sessions per GPU) and N = 4 (128)."""
     from moshi_b200.models import LMGen, loaders
     lm, cfg = _lm()
