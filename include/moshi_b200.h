@@ -559,14 +559,16 @@ int64_t b200_dlm_algorithmic_flops(b200_dlm* h, int tokens, int context);
 /* ------------------------------------------------------------------------------------------ */
 
 /* y[M,N] = x[M,K] * w[N,K]^T, bf16 in, fp32 accumulate, bf16 out, on row-major weights: packs them into tiles and runs
- * the LM's linear for this shape (whole rows per CTA up to 16 rows, tcgen05 stream-K / whole-tile / cluster split-K kernels above);
+ * the LM's linear for this shape (whole rows per CTA up to 16 rows, weights through registers or tcgen05 kernels above);
  * synchronises the stream (test helper).  Reference op: every nn.Linear of the LM (transformer.py:304-305,554-555,588-589). */
 int b200_op_linear_bf16(const void* x_dev, const void* w_dev, void* y_dev, int M, int N, int K, void* stream);
 /* Stream-K tcgen05 GEMM over pre-tiled weights (the LM's linear kernel; csrc/gemm_sk.cu).
  *   b200_op_packed_bytes / b200_op_pack_tiles: repack w bf16 [N,K] (epi 2: [2*gate_rows,K], rows gate|value,
  *   gating.py:18-20) into 16 KB SWIZZLE_128B tiles.
  *   b200_op_linear_sk: y = epi(x . W^T); epi 0 store [M,N], 1 residual add (y = res + .), 2 silu(gate)*value
- *   -> [M,gate_rows].  grid / smem_budget / stream_only are tuning & diagnostics knobs (0 = defaults). */
+ *   -> [M,gate_rows].  grid / smem_budget / stream_only are tuning & diagnostics knobs (0 = defaults).
+ * This one, b200_op_linear_i8, b200_op_quantize_rows and b200_op_attn_step are launched early (programmatic dependent launch; B200_PDL=0: not): they may begin
+ * beside the kernel in front on the stream, and read nothing before it is done. */
 int64_t b200_op_packed_bytes(int N, int K, int epi, int gate_rows);
 int b200_op_pack_tiles(const void* w_dev, void* out_dev, int N, int K, int epi, int gate_rows, void* stream);
 int b200_op_linear_sk(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N,
@@ -579,7 +581,8 @@ int b200_op_linear_sk(const void* x_dev, const void* w_tiles_dev, void* y_dev, c
 int b200_op_linear_ns(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K,
                       int epi, int gate_rows, int cluster, void* stream);
 /* The kernel with the weights going through registers (csrc/gemm_reg.cu) at every shape that it has: up to 32 rows, gated pairs up to 16.
- * b200_op_linear_sk takes it where it is ahead: up to 8 rows, and up to 32 where the tiles are no more than the SMs. */
+ * b200_op_linear_sk takes it where it is ahead: 17 to 32 rows where the tiles are no more than the SMs, and the gated pairs of fewer rows that
+ * gemm_row.cu leaves. */
 int b200_op_linear_reg(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K, int epi, int gate_rows,
                        void* stream);
 /* The decoder LM's linear for more than 256 activation rows (csrc/gemm_wide.cu): y[M,N] = x[M,K] . w^T over packed tiles
