@@ -104,3 +104,34 @@ def test_ends_of_the_shapes_agree_with_the_chain(pair, B):
             assert torch.equal(tg[q], first)
             same &= tg[q] == tw[q]
     assert compared >= B
+
+
+@torch.no_grad()
+def test_two_streams_of_different_sizes_side_by_side():
+    """Sixteen sessions of one model and nine of another, step by step in turn: each as it is alone."""
+    from moshi_b200.models import LMGen
+    cfg = LMConfig(**dict(BASE, depformer_dim=512, depformer_num_heads=8, depformer_dim_feedforward=2112, depformer_num_layers=2, card=2048))
+    models = [_model(cfg, synth_lm_state_dict(cfg, seed=s, device="cuda")) for s in (1, 2)]
+    sizes, steps = (16, 9), 3
+    codes = [torch.randint(0, cfg.card, (steps, B, 8, 1), generator=torch.Generator().manual_seed(B)).cuda() for B in sizes]
+
+    def tokens(gen, B):
+        return gen.read_buffer("audio_tokens", torch.int64, (cfg.dep_q, B))
+
+    def gens():
+        made = [LMGen(m, use_sampling=False) for m in models]
+        for g in made:
+            g.use_graph = False
+        return made
+
+    alone = []
+    for gen, B, c in zip(gens(), sizes, codes):
+        with gen.streaming(B):
+            alone.append([(gen.step(x), tokens(gen, B))[1] for x in c])
+    a, b = gens()
+    with a.streaming(sizes[0]), b.streaming(sizes[1]):
+        for i in range(steps):
+            for gen, B, c, want in zip((a, b), sizes, codes, alone):
+                gen.step(c[i])
+                assert torch.equal(tokens(gen, B), want[i])
+        assert a.error_flags() == 0 and b.error_flags() == 0
