@@ -626,6 +626,10 @@ int b200_op_tc_linear_f32(const float* x_dev, const float* w_dev, float* y_dev, 
 /* Row-major fp32 weights out of what a Mimi handle keeps of them (packed hi / lo tiles and one bit per weight; csrc/mimi_lin.cuh), as
  * b200_mimi_streaming_begin makes them for small batches: rows[N,K] = w[N,K] bit for bit.  K % 512 == 0, N % 16 == 0.  Synchronises (test helper). */
 int b200_op_tc_rows(const float* w_dev, float* rows_dev, int N, int K, void* stream);
+/* one linear of Mimi's bottleneck transformers as up to 64 tokens take it (fp32; N % 16 == 0, K % 512 == 0): y[M][N] = epi(norm(x[M][K]) . w[N][K]^T).  gamma_dev and
+ * beta_dev (layer norm, eps 1e-5; K == 512) may be null.  epi 0: as it is, 1: GELU, 2: res[M][N] + scale[N] times it */
+int b200_op_mimi_linear(const float* x_dev, const float* gamma_dev, const float* beta_dev, const float* w_dev, const float* res_dev, const float* scale_dev, float* y_dev,
+                        int M, int N, int K, int epi, void* stream);
 int b200_op_tc_conv1d(const float* x_dev, const float* w_dev, const float* bias_dev, float* prev_dev, const uint8_t* exec_mask_dev,
                       float* y_dev, int B, int Cin, int Cout, int T, int K, int stride, int dilation, int elu_in, int transposed,
                       void* stream);

@@ -12,6 +12,7 @@
 #include "mimi_tc.cuh"
 #include "mimi_lin.cuh"
 #include "mimi_rvq.cuh"
+#include "mimi_tile.cuh"
 #include "mimi_tm_kernels.cuh"
 
 using namespace b200;
@@ -122,7 +123,7 @@ struct b200_mimi {
   float* tap_scratch = nullptr; size_t tap_scratch_n = 0;
   std::map<std::string, Tap> taps;
   int64_t weight_bytes = 0;
-  bool tr_cuda_cores = false;                  // the bottleneck transformers run on mimi_lin_kernel / mimi_attn_kernel at this batch
+  bool tr_cuda_cores = false;                  // the bottleneck transformers run on the CUDA cores at this batch (mimi_lin.cuh, mimi_tile.cuh)
 };
 
 namespace {
@@ -1042,9 +1043,9 @@ int b200_mimi_streaming_begin(b200_mimi* h, int batch, void* stream) {
   // transformers
   const int H = c.tr_num_heads, D = d / H, ff = c.tr_dim_feedforward;
   const size_t ntok = (size_t)B * T;
-  // encode + decode of a frame on these kernels against mimi_tc_kernel: 1 session 0.71 / 1.43 ms, 8 sessions 1.15 / 1.51, 24 sessions 1.43 / 1.66,
-  // 32 sessions (64 tokens) 1.62 / 1.74.  Before mimi_tc_kernel had sixteen epilogue warps the two met at 40 sessions (1.99 ms; 1.85 there now):
-  // a product over 80 tokens is worth the tensor cores' two launches
+  // encode + decode of a frame on these kernels against mimi_tc_kernel: 1 session 0.70 / 1.43 ms, 8 sessions 0.87 / 1.51, 24 sessions 1.16 / 1.66,
+  // 32 sessions (64 tokens) 1.26 / 1.74.  Beyond, the row-major weights are not held: with the tiles read from the packed hi / lo pairs 40 sessions
+  // are at 1.78 / 1.86, 104 at 3.03 / 2.51
   h->tr_cuda_cores = (int)ntok <= 64 && D == 64 && d == 512 && T <= 4 && lin_takes(3 * d, d) && lin_takes(d, ff) && lin_takes(ff, d);
   B200_TRY(A.alloc_t(&h->tr_xn_hi, ntok * d));
   B200_TRY(A.alloc_t(&h->tr_xn_lo, ntok * d));

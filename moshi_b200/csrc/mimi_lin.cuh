@@ -6,7 +6,8 @@
 //   mimi_lin_kernel: a warp owns NO outputs for TOK tokens.  Its weights (fp32, row-major) are requested before the wait on the
 //     preceding kernel (programmatic dependent launch), up to 2048 elements per output at a time; every CTA brings the tokens' rows into
 //     shared memory, normed in front of in_proj and linear1; lanes own k, their sums meet in a transposing butterfly that leaves each
-//     lane one output; epilogues as in mimi_tc.cu (GELU, residual + layer scale, hi / lo parts for a convolution behind).
+//     lane one output; epilogues as in mimi_tc.cu (GELU, residual + layer scale, hi / lo parts for a convolution behind).  Up to two tokens everywhere;
+//     with more of them most linears take mimi_tile.cuh.
 //   mimi_attn_kernel: a half-warp per key, keys and values of four keys in flight, running maximum; the eight half-warps meet in
 //     shared memory.
 #pragma once
@@ -30,6 +31,20 @@ struct LinP {
   float *a_hi, *a_lo; long long a_sb, a_row; int a_elu;      // hi / lo parts of the result at session * a_sb + step * a_row + n (null: none)
   float eps;
 };
+
+__device__ __forceinline__ void lin_result(const LinP& p, int tok, int n, float v) {
+  if (p.epi == LIN_GELU) v = gelu_erf(v);
+  else if (p.epi == LIN_RESIDUAL) v = p.res[(long long)tok * p.N + n] + p.scale[n] * v;
+  if (p.y) p.y[(long long)tok * p.N + n] = v;
+  if (p.a_hi) {
+    float hi, lo;
+    mtc::split_tf32(p.a_elu ? elu1(v) : v, hi, lo);
+    const int b = tok / p.T;
+    const long long at = (long long)b * p.a_sb + (long long)(tok - b * p.T) * p.a_row + n;
+    p.a_hi[at] = hi;
+    p.a_lo[at] = lo;
+  }
+}
 
 // lanes hold V partial sums each; afterwards a lane holds the totals of R = max(1, V / 32) of them: values index * R .. index * R + R - 1, with
 // index made of the leading lane bits
@@ -130,20 +145,8 @@ __global__ void __launch_bounds__(128) mimi_lin_kernel(const LinP p) {
   if (COPIES > 1 && (lane & (COPIES - 1))) return;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int i = index * R + r, t = i / NO, n = n0 + i - t * NO, tok = tok0 + t;
-    if (t >= nt) continue;
-    float v = acc[r];
-    if (p.epi == LIN_GELU) v = gelu_erf(v);
-    else if (p.epi == LIN_RESIDUAL) v = p.res[(long long)tok * p.N + n] + p.scale[n] * v;
-    if (p.y) p.y[(long long)tok * p.N + n] = v;
-    if (p.a_hi) {
-      float hi, lo;
-      mtc::split_tf32(p.a_elu ? elu1(v) : v, hi, lo);
-      const int b = tok / p.T;
-      const long long at = (long long)b * p.a_sb + (long long)(tok - b * p.T) * p.a_row + n;
-      p.a_hi[at] = hi;
-      p.a_lo[at] = lo;
-    }
+    const int i = index * R + r, t = i / NO, n = n0 + i - t * NO;
+    if (t < nt) lin_result(p, tok0 + t, n, acc[r]);
   }
 }
 
@@ -181,28 +184,13 @@ inline int lin_rows(const uint8_t* tiles, const uint32_t* bits, float* rows, int
 }
 
 template <int NO, int TOK, int KC>
-int lin_launch_one(const LinP& p, cudaStream_t st) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)(p.N / (4 * NO)), (unsigned)ceil_div(p.n_tok, TOK)); cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = (size_t)TOK * KC * 128 * 4; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = mtc::tc_pdl() ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, mimi_lin_kernel<NO, TOK, KC>, p);
-  if (e != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "mimi_lin launch failed: %s", cudaGetErrorString(e));
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return B200_OK;
-}
-
-// few tokens: one output per warp and as much of its row in flight as registers hold; many: four outputs share a read of the tokens
-inline int lin_launch(const LinP& p, cudaStream_t st) {
-  const bool deep = p.K % 2048 == 0 && !p.gamma;
-  if (p.n_tok <= 2) return deep ? lin_launch_one<1, 2, 16>(p, st) : lin_launch_one<1, 2, 4>(p, st);
-  if (p.n_tok <= 4) return deep ? lin_launch_one<1, 4, 16>(p, st) : lin_launch_one<1, 4, 4>(p, st);
-  if (p.n_tok <= 8) return lin_launch_one<2, 8, 4>(p, st);
-  return lin_launch_one<4, 16, 4>(p, st);
+int lin_launch_one(const LinP& p, cudaStream_t st, bool early) {
+  constexpr int SMEM = TOK * KC * 128 * 4;
+  if constexpr (SMEM > 48 * 1024) {
+    static std::atomic<uint64_t> limits{0};
+    B200_TRY(allow_smem(limits, SMEM, mimi_lin_kernel<NO, TOK, KC>));
+  }
+  return launch_early_if(early, mimi_lin_kernel<NO, TOK, KC>, dim3((unsigned)(p.N / (4 * NO)), (unsigned)ceil_div(p.n_tok, TOK)), dim3(128), SMEM, st, p);
 }
 
 // One attention step of T <= 4 tokens per session: RoPE (rope.py:45-82), ring append for executing sessions, attention over the ring under

@@ -5,7 +5,7 @@
 #include "gemm_sk.cuh"
 #include "lm_kernels.cuh"
 #include "mimi_kernels.cuh"
-#include "mimi_lin.cuh"
+#include "mimi_tile.cuh"
 #include "mimi_tc.cuh"
 
 using namespace b200;
@@ -336,6 +336,20 @@ int b200_op_tc_rows(const float* w_dev, float* rows_dev, int N, int K, void* str
   B200_TRY(mimi::lin_rows(wt, lost, rows_dev, N, K, N >= TC_MAX_NT ? TC_MAX_NT : N, st));
   B200_CUDA(cudaStreamSynchronize(st));
   return B200_OK;
+}
+int b200_op_mimi_linear(const float* x_dev, const float* gamma_dev, const float* beta_dev, const float* w_dev, const float* res_dev, const float* scale_dev, float* y_dev,
+                        int M, int N, int K, int epi, void* stream) {
+  using namespace b200::mimi;
+  if (!x_dev || !w_dev || !y_dev || (epi == LIN_RESIDUAL && (!res_dev || !scale_dev)) || !gamma_dev != !beta_dev) B200_FAIL(B200_ERR_INVALID, "op_mimi_linear: null pointer");
+  if (M < 1 || N < 1 || K < 1 || !lin_takes(N, K) || (gamma_dev && K != 512) || epi < LIN_STORE || epi > LIN_RESIDUAL) B200_FAIL(B200_ERR_SHAPE, "op_mimi_linear: bad shape");
+  if ((reinterpret_cast<uintptr_t>(x_dev) | reinterpret_cast<uintptr_t>(w_dev) | reinterpret_cast<uintptr_t>(gamma_dev) | reinterpret_cast<uintptr_t>(beta_dev)) & 15)
+    B200_FAIL(B200_ERR_INVALID, "op_mimi_linear: pointers must be 16-byte aligned");
+  LinP p;
+  memset(&p, 0, sizeof(p));
+  p.x = x_dev; p.gamma = gamma_dev; p.beta = beta_dev; p.w = w_dev; p.n_tok = M; p.N = N; p.K = K; p.T = 1; p.epi = epi; p.y = y_dev; p.res = res_dev; p.scale = scale_dev;
+  p.eps = 1e-5f;
+  B200_TRY(lin_launch(p, static_cast<cudaStream_t>(stream), false));
+  return check_launch("op_mimi_linear");
 }
 int b200_op_tc_linear_f32(const float* x_dev, const float* w_dev, float* y_dev, int M, int N, int K, void* stream) {
   using namespace b200::mtc;
