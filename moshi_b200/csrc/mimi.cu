@@ -106,7 +106,7 @@ struct b200_mimi {
   float* rvq_best[2] = {nullptr, nullptr};
   int* rvq_idx[2] = {nullptr, nullptr};
   int rvq_cap = 0;
-  float* splitk_ws = nullptr; size_t splitk_bytes = 0;   // split-K partial sums of the deep / skinny layers
+  float* splitk_ws = nullptr; size_t splitk_bytes = 0;   // partial sums of the down-sampling conv
   int* err = nullptr;                                     // device error flags (B200_FLAG_CODE_RANGE)
   // one-frame encode / decode as CUDA graphs over static buffers (frame in enc[0].ext -> enc_codes, dec_codes -> out_frame)
   cudaStream_t body = nullptr;                 // stream the kernels are being enqueued on (caller's, or gstream in capture)
@@ -440,7 +440,7 @@ int run_transformer(b200_mimi* h, Transformer& tr, const float* x_in, float* x, 
       q.gamma = L.n1w; q.beta = L.n1b;
       B200_TRY(lin_launch(q, h->body));
       MimiAttn a;
-      a.qkv = h->tr_qkv; a.kc = L.kc; a.vc = L.vc; a.out = h->tr_ao_hi; a.offset = tr.offset; a.exec_mask = h->exec_mask; a.H = H; a.cap = c.tr_context;
+      a.qkv = h->tr_qkv; a.kc = L.kc; a.vc = L.vc; a.out = h->tr_ao_hi; a.out_lo = nullptr; a.offset = tr.offset; a.exec_mask = h->exec_mask; a.H = H; a.cap = c.tr_context;
       a.context = c.tr_context; a.neg_log_period_2_over_d = nl;
       B200_TRY(attn_launch(a, B, T, h->body));
       q = lin(h->tr_ao_hi, L.w_out, d, d, LIN_RESIDUAL, x);
@@ -461,12 +461,19 @@ int run_transformer(b200_mimi* h, Transformer& tr, const float* x_in, float* x, 
   for (size_t li = 0; li < tr.layers.size(); ++li) {
     TrLayer& L = tr.layers[li];
     const float* cur = li == 0 ? x_in : x;
-    B200_LAUNCH(layernorm_split_kernel, ceil_div(ntok * 32, 256), 256, 0, h->body, cur, L.n1w, L.n1b, h->tr_xn_hi, h->tr_xn_lo, ntok, d, 1e-5f);
+    B200_TRY(launch_early_if(mtc::tc_pdl(), layernorm_split_kernel, dim3(ceil_div(ntok, 2)), dim3(64), 0, h->body, cur, L.n1w, L.n1b, h->tr_xn_hi, h->tr_xn_lo, ntok, d, 1e-5f));
     B200_TRY(launch_tc(h, L.in_proj));
-    B200_LAUNCH((ring_attn_step_kernel<64>), B * H, 128, attn_smem, h->body, h->tr_qkv, L.kc, L.vc, h->tr_ao_hi, h->tr_ao_lo, tr.offset,
-                h->exec_mask, T, H, c.tr_context, c.tr_context, nl);
+    if (T <= 4) {
+      MimiAttn a;
+      a.qkv = h->tr_qkv; a.kc = L.kc; a.vc = L.vc; a.out = h->tr_ao_hi; a.out_lo = h->tr_ao_lo; a.offset = tr.offset; a.exec_mask = h->exec_mask; a.H = H; a.cap = c.tr_context;
+      a.context = c.tr_context; a.neg_log_period_2_over_d = nl;
+      B200_TRY(attn_launch(a, B, T, h->body));
+    } else {
+      B200_LAUNCH((ring_attn_step_kernel<64>), B * H, 128, attn_smem, h->body, h->tr_qkv, L.kc, L.vc, h->tr_ao_hi, h->tr_ao_lo, tr.offset,
+                  h->exec_mask, T, H, c.tr_context, c.tr_context, nl);
+    }
     B200_TRY(launch_tc(h, L.out_proj));       // x = cur + layer_scale_1 * out_proj(attention)
-    B200_LAUNCH(layernorm_split_kernel, ceil_div(ntok * 32, 256), 256, 0, h->body, x, L.n2w, L.n2b, h->tr_xn_hi, h->tr_xn_lo, ntok, d, 1e-5f);
+    B200_TRY(launch_early_if(mtc::tc_pdl(), layernorm_split_kernel, dim3(ceil_div(ntok, 2)), dim3(64), 0, h->body, x, L.n2w, L.n2b, h->tr_xn_hi, h->tr_xn_lo, ntok, d, 1e-5f));
     B200_TRY(launch_tc(h, L.l1));             // h = gelu(linear1(xn)) as a hi / lo pair
     B200_TRY(launch_tc(h, L.l2));             // x = x + layer_scale_2 * linear2(h)
   }
@@ -795,10 +802,9 @@ int plan_layer(b200_mimi* h, mtc::TcLayer& L, const float* in_hi, const float* i
   int tt = 0, bb = 0;
   if (tile_shape(T, L.stride, &tt, &bb) != B200_OK) B200_FAIL(B200_ERR_INVALID, "mimi: %d steps per frame do not tile", T);
   L.p.tt = tt; L.p.bb = bb; L.p.row0 = row0;
-  L.p.ws = h->splitk_ws;
   B200_TRY(mtc::tc_make_map(&L.map_hi, in_hi, L.Cin, rows_per_session, (long long)rows_per_session * L.Cin, B, tt, bb, L.stride));
   B200_TRY(mtc::tc_make_map(&L.map_lo, in_lo, L.Cin, rows_per_session, (long long)rows_per_session * L.Cin, B, tt, bb, L.stride));
-  return mtc::tc_plan(L, B, T, h->sms, h->splitk_bytes);
+  return mtc::tc_plan(L, B, T, h->sms);
 }
 
 }  // namespace
@@ -1043,9 +1049,7 @@ int b200_mimi_streaming_begin(b200_mimi* h, int batch, void* stream) {
   // transformers
   const int H = c.tr_num_heads, D = d / H, ff = c.tr_dim_feedforward;
   const size_t ntok = (size_t)B * T;
-  // encode + decode of a frame on these kernels against mimi_tc_kernel: 1 session 0.70 / 1.43 ms, 8 sessions 0.87 / 1.51, 24 sessions 1.16 / 1.66,
-  // 32 sessions (64 tokens) 1.26 / 1.74.  Beyond, the row-major weights are not held: with the tiles read from the packed hi / lo pairs 40 sessions
-  // are at 1.78 / 1.86, 104 at 3.03 / 2.51
+  // encode + decode of a frame: 32 sessions (64 tokens) on these kernels 1122 us, 33 on mimi_tc_kernel 1218.  Beyond 64 tokens the row-major weights are not held
   h->tr_cuda_cores = (int)ntok <= 64 && D == 64 && d == 512 && T <= 4 && lin_takes(3 * d, d) && lin_takes(d, ff) && lin_takes(ff, d);
   B200_TRY(A.alloc_t(&h->tr_xn_hi, ntok * d));
   B200_TRY(A.alloc_t(&h->tr_xn_lo, ntok * d));

@@ -1,8 +1,8 @@
 // The linears and the attention of Mimi's bottleneck transformers in fp32 on the CUDA cores (transformer.py:752-777, 557-597).
 //
-// A frame brings two tokens per session and layer: what a layer costs is the chain of its launches, not its products.  mimi_tc_kernel
-// plus the split-K reduction behind it take 9-11 us per linear whether there are 2 tokens or 80, a layer is four of them, two layer
-// norms and an attention of 9 us.  Here a layer is five launches:
+// A frame brings two tokens per session and layer: what a layer costs is the chain of its launches, not its products.  A launch
+// of mimi_tc_kernel takes about 6 us whether there are 2 tokens or 80, a layer is four of them, two layer norms and an attention.  Here a
+// layer is five launches of 2 to 3:
 //   mimi_lin_kernel: a warp owns NO outputs for TOK tokens.  Its weights (fp32, row-major) are requested before the wait on the
 //     preceding kernel (programmatic dependent launch), up to 2048 elements per output at a time; every CTA brings the tokens' rows into
 //     shared memory, normed in front of in_proj and linear1; lanes own k, their sums meet in a transposing butterfly that leaves each
@@ -196,7 +196,7 @@ int lin_launch_one(const LinP& p, cudaStream_t st, bool early) {
 // One attention step of T <= 4 tokens per session: RoPE (rope.py:45-82), ring append for executing sessions, attention over the ring under
 // the causal / context mask (transformer.py:247-286, 557-597) -> [n_tok][C].  Head size 64, one CTA per (session, head).
 struct MimiAttn {
-  const float* qkv; float *kc, *vc, *out;
+  const float* qkv; float *kc, *vc, *out, *out_lo;      // out_lo: the result as a hi / lo pair (null: out alone, in full)
   const long long* offset; const uint8_t* exec_mask;
   int H, cap, context; float neg_log_period_2_over_d;
 };
@@ -301,7 +301,10 @@ __global__ void __launch_bounds__(128) mimi_attn_kernel(const MimiAttn p) {
         a = fmaf(f, so[w][t][d], a);
       }
     }
-    p.out[((long long)b * T + t) * C + h * D + d] = den > 0.f ? a / den : 0.f;
+    const long long o = ((long long)b * T + t) * C + h * D + d;
+    const float v = den > 0.f ? a / den : 0.f;
+    if (p.out_lo) mtc::split_tf32(v, p.out[o], p.out_lo[o]);
+    else p.out[o] = v;
   }
 }
 

@@ -18,10 +18,21 @@
 //     in TMEM (dropped terms <= 2^-22 relative).  The RVQ indices downstream stay exact up to the margin the parity tests
 //     define (tests/util.py).
 //   * Warp roles (576 threads): warp 0 = TMA producer (A hi + A lo boxes, one contiguous bulk copy of the pre-tiled weight
-//     pair per k-block), warp 1 = TMEM owner + single-thread MMA issuer, warps 2-17 = epilogue (TMEM lane = GEMM row = one
-//     token: bias, residual, ELU / GELU / layer-scale, hi/lo split, 64-byte contiguous stores).  Persistent grid, two TMEM
-//     accumulator stages: the epilogue of a tile overlaps the MMAs of the next.  Deep-and-skinny layers are cut along K into
-//     fp32 partials reduced in split order by mimi_tc_reduce_kernel (deterministic).
+//     pair per k-block), warp 1 = TMEM owner + MMA issuer, warps 2-17 = epilogue: the sums go through shared memory, so that a
+//     warp stores and reads whole lines (bias, residual, ELU / GELU / layer-scale, hi/lo split).  Persistent grid, two TMEM
+//     accumulator stages: the epilogue of a tile overlaps the MMAs of the next.
+//   * Few tiles: a cluster of 2 to 8 CTAs shares a tile's k, every CTA adds the sums of all of them over distributed shared
+//     memory for its share of the rows, in order, and finishes those (one tile per CTA).
+//   * Few rows against 128 features: the features are the tensor core's rows and the activation rows its 16..112 columns.
+//   * A chain of more than TC_CHAIN k-blocks is summed up in fp32 registers piece by piece: the tensor core cuts off where an
+//     addition rounds (2 x 8192 -> 1024: error 7.2e-6 in chains of 32 k-blocks, 9e-7 in chains of 4).
+//
+// What bounds a launch of a few tiles is a chain of latencies, 4 to 6 us behind the wait: load 1.1, products 0.35 a k-block, TMEM
+// to shared memory 0.5, the cluster's barrier 0.3, exchange and epilogue 1.2.  Found on the way, encode + decode of a frame of 1 / 40
+// sessions, us: partial sums through L2 and a second launch 695 / 1857; clusters and whole lines 645 / 1811; residual, bias and all
+// index divisions (a tenth of a microsecond each) in front of the waits, layer norm and attention of many tokens launched early,
+// 604 / 1498; the issuing warp walking along as a whole with its operands in uniform registers, 548 / 1378 (one thread issued
+// an instruction every 90 to 100 clocks at any size).
 #pragma once
 
 #include <cuda.h>
@@ -33,26 +44,29 @@ namespace mtc {
 
 constexpr int TC_ROWS = 128;            // GEMM rows (tokens) per tile = UMMA M
 constexpr int TC_KB = 32;               // fp32 elements per k-block row: 128 bytes = one SWIZZLE_128B row
-constexpr int TC_MAX_NT = 128;          // output features per tile = UMMA N (<= 128: 64 KB per stage, 3 stages)
+constexpr int TC_MAX_NT = 128;          // output features per tile (64 KB per stage and 3 stages where all 128 rows exist)
 constexpr int TC_EPI_WARPS = 16;         // four per TMEM quadrant: the epilogue is a chain of latencies per run of 16 features
-                                        // (one per quadrant: a frame of 40 sessions took 1982 us, of one session 739; four: 1850 and 690)
+                                        // (one per quadrant, before the sums went through shared memory: a frame of 40 sessions took 1982 us, of one session 739; four: 1850 and 690)
 constexpr int TC_THREADS = 64 + 32 * TC_EPI_WARPS;
-constexpr int TC_MAX_STAGES = 6;
+constexpr int TC_MAX_STAGES = 8;
+constexpr int TC_MAX_SPLIT = 8;         // CTAs of a cluster that share a tile's k
+constexpr int TC_CHAIN = 4;              // k-blocks that the tensor core sums up by itself: it cuts off where an fp32 addition rounds
+constexpr int TC_SMEM = 225 * 1024;     // ring and sums
 
 enum { TC_EPI_CONV = 0, TC_EPI_GELU = 1, TC_EPI_RES_SCALE = 2 };
 enum { TC_ACT_NONE = 0, TC_ACT_SPLIT = 1, TC_ACT_FULL = 2 };      // how the consumer wants its input: hi/lo pair or plain fp32
 
 struct TcParams {
   // ---- geometry of the A operand (tensor maps are kernel arguments)
-  int tt, bb;                 // tile = bb sessions x tt steps, tt * bb == 128
+  int tt, bb, tt_log2;        // tile = bb sessions x tt steps, tt * bb == 128
   int T;                      // output steps per session (tt divides T, or T < tt == 128 for the flat linear case)
   int n_sessions;             // B (rows beyond it are zero-filled by TMA and masked in the epilogue)
-  int n_taps, dil, stride, row0, Cin;
+  int n_taps, dil, stride, row0, Cin, cb_per_tap, tiles_per_group;
   // ---- B operand: pre-tiled weights [n_tile][kb][hi | lo][NT rows][32] (SWIZZLE_128B), kb = tap * (Cin / 32) + ci_block
   const uint8_t* wt; int NT, n_tiles_n, num_kb, N;
   // ---- schedule
   int m_tiles, ksplit, kb_per_split;
-  float* ws;                  // split-K partials [split][rows_total][N] (rows_total = m_tiles * 128)
+  int swap;                   // 0, or: weights are the tensor core's rows, and this many (a multiple of 16) activation rows its columns
   // ---- epilogue
   int epi;
   const float* bias; int bias_mod;                 // bias[n % bias_mod] (conv: bias_mod = N; convtr: Cout)
@@ -61,7 +75,7 @@ struct TcParams {
   const float* scale;                              // lin RES_SCALE: per-feature layer scale
   int act_mode, act_elu;
   float *a_hi, *a_lo; long long a_sb, a_row;       // activated copy for the consumer: a[b * a_sb + t * a_row + n]
-  uint32_t stage_bytes, tmem_cols; int stages;
+  uint32_t stage_bytes, box_bytes, a_bytes, bars_at, tmem_cols; int stages;      // box: the rows of a tile that can exist; bars_at: mbarriers, behind the ring and the sums
 };
 
 // y = hi + lo with hi = tf32(y) and lo = tf32(y - hi), both round-to-nearest (cvt.rna): |y - hi - lo| <= 2^-23 |y|
@@ -97,7 +111,7 @@ int tc_init();
 // 3-D tensor map over a token-major activation buffer base[b][row][Cin] (session stride sb elements, row stride = Cin)
 int tc_make_map(CUtensorMap* m, const float* base, int Cin, long long rows_per_session, long long sb_elems, int n_sessions, int tt,
                 int bb, int stride);
-int tc_plan(TcLayer& L, int n_sessions, int T, int sms, size_t ws_bytes);
+int tc_plan(TcLayer& L, int n_sessions, int T, int sms);
 int tc_launch(const TcLayer& L, cudaStream_t st);
 
 }  // namespace mtc

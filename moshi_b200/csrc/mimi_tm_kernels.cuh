@@ -5,6 +5,7 @@
 
 #include "common.cuh"
 #include "mimi_tc.cuh"
+#include "tc_prims.cuh"
 
 namespace b200 {
 namespace mimi {
@@ -124,25 +125,51 @@ static __global__ void tm_zero_kernel(float* hi, float* lo, int P, int rowlen, l
   if (lo != nullptr) lo[o] = 0.f;
 }
 
-// LayerNorm (eps 1e-5, affine; transformer.py:126) -> the following linear's input as a hi / lo pair
-static __global__ void layernorm_split_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ bta,
-                                       float* __restrict__ y_hi, float* __restrict__ y_lo, int n_tok, int C, float eps) {
-  pdl_trigger_next();
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= n_tok) return;
-  const float* xr = x + (long long)warp * C;
+// LayerNorm (eps 1e-5, affine; transformer.py:126) -> the following linear's input as a hi / lo pair.  One warp per token, the row in registers (C <= 512, a
+// multiple of 128) or read three times.
+static __global__ void __launch_bounds__(64) layernorm_split_kernel(const float* x, const float* __restrict__ g, const float* __restrict__ bta, float* y_hi, float* y_lo, int n_tok, int C,
+                                                                    float eps) {
+  const int tok = blockIdx.x * 2 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
+  if (tok >= n_tok) return;
+  const float* xr = x + (long long)tok * C;
+  const long long o = (long long)tok * C;
+  if (C <= 512 && C % 128 == 0) {
+    float4 v[4];
+    float s = 0.f, q = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] = c * 128 < C ? *reinterpret_cast<const float4*>(xr + c * 128 + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s += (v[c].x + v[c].y) + (v[c].z + v[c].w);
+    const float mean = warp_sum(s) / C;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c * 128 >= C) break;
+      v[c].x -= mean; v[c].y -= mean; v[c].z -= mean; v[c].w -= mean;
+      q += (v[c].x * v[c].x + v[c].y * v[c].y) + (v[c].z * v[c].z + v[c].w * v[c].w);
+    }
+    const float r = rsqrtf(warp_sum(q) / C + eps);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c * 128 >= C) break;
+      const int i = c * 128 + lane * 4;
+      const float4 gv = __ldg(reinterpret_cast<const float4*>(g + i)), bv = __ldg(reinterpret_cast<const float4*>(bta + i));
+      float4 hi, lo;
+      mtc::split_tf32(v[c].x * r * gv.x + bv.x, hi.x, lo.x); mtc::split_tf32(v[c].y * r * gv.y + bv.y, hi.y, lo.y);
+      mtc::split_tf32(v[c].z * r * gv.z + bv.z, hi.z, lo.z); mtc::split_tf32(v[c].w * r * gv.w + bv.w, hi.w, lo.w);
+      *reinterpret_cast<float4*>(y_hi + o + i) = hi;
+      *reinterpret_cast<float4*>(y_lo + o + i) = lo;
+    }
+    return;
+  }
   float s = 0.f;
   for (int c = lane; c < C; c += 32) s += xr[c];
   const float mean = warp_sum(s) / C;
   float v = 0.f;
   for (int c = lane; c < C; c += 32) { float d = xr[c] - mean; v += d * d; }
   const float rstd = rsqrtf(warp_sum(v) / C + eps);
-  for (int c = lane; c < C; c += 32) {
-    float hi, lo;
-    mtc::split_tf32((xr[c] - mean) * rstd * g[c] + bta[c], hi, lo);
-    y_hi[(long long)warp * C + c] = hi;
-    y_lo[(long long)warp * C + c] = lo;
-  }
+  for (int c = lane; c < C; c += 32) mtc::split_tf32((xr[c] - mean) * rstd * g[c] + bta[c], y_hi[o + c], y_lo[o + c]);
 }
 
 // One attention step of a bottleneck transformer layer in ONE launch (transformer.py:557-597 for T tokens per frame):

@@ -357,12 +357,10 @@ int b200_op_tc_linear_f32(const float* x_dev, const float* w_dev, float* y_dev, 
   if (!x_dev || !w_dev || !y_dev || M < 1 || K % 32 || N % 16) B200_FAIL(B200_ERR_SHAPE, "op_tc_linear_f32: bad shape");
   B200_TRY(tc_init());
   DevBufs d;
-  float *hi, *lo, *ws; uint8_t* wt;
+  float *hi, *lo; uint8_t* wt;
   B200_TRY(d.get(&hi, (size_t)M * K * 4));
   B200_TRY(d.get(&lo, (size_t)M * K * 4));
   B200_TRY(d.get(&wt, tc_packed_bytes(N, K, 1)));
-  const size_t ws_bytes = (size_t)64 << 20;
-  B200_TRY(d.get(&ws, ws_bytes));
   const long long n = (long long)M * K;
   // x is already [M][K] token-major: a flat hi/lo split is tm_pack_in with B = M "sessions" of Cin = K, T = 1, P = 0
   B200_LAUNCH(tm_pack_in_kernel, (unsigned)ceil_div64(n, 256), 256, 0, st, x_dev, (const float*)nullptr, hi, lo, M, K, 1, 0, 0);
@@ -372,12 +370,12 @@ int b200_op_tc_linear_f32(const float* x_dev, const float* w_dev, float* y_dev, 
   L.NT = N >= TC_MAX_NT ? TC_MAX_NT : N; L.n_tiles_n = (N + L.NT - 1) / L.NT; L.num_kb = K / TC_KB;
   memset(&L.p, 0, sizeof(L.p));
   L.p.tt = 128; L.p.bb = 1; L.p.row0 = 0;
-  L.p.epi = TC_EPI_CONV; L.p.y = y_dev; L.p.y_sb = 0; L.p.y_row = N; L.p.ws = ws;
+  L.p.epi = TC_EPI_CONV; L.p.y = y_dev; L.p.y_sb = 0; L.p.y_row = N;
   B200_TRY(tc_make_map(&L.map_hi, hi, K, M, (long long)M * K, 1, 128, 1, 1));
   B200_TRY(tc_make_map(&L.map_lo, lo, K, M, (long long)M * K, 1, 128, 1, 1));
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  B200_TRY(tc_plan(L, 1, M, sms, ws_bytes));
+  B200_TRY(tc_plan(L, 1, M, sms));
   B200_TRY(tc_launch(L, st));
   B200_CUDA(cudaStreamSynchronize(st));
   return B200_OK;
@@ -397,15 +395,13 @@ int b200_op_tc_conv1d(const float* x_dev, const float* w_dev, const float* bias_
   if (Cin % 32 || N % 16 || (N > 128 && N % 128) || P < 0 || (!transposed && T % stride) || (transposed && K != 2 * S))
     B200_FAIL(B200_ERR_SHAPE, "op_tc_conv1d: unsupported shape");
   DevBufs d;
-  float *hi, *lo, *ws, *wk, *ytm; uint8_t* wt;
+  float *hi, *lo, *wk, *ytm; uint8_t* wt;
   const size_t E = (size_t)P + T;
   B200_TRY(d.get(&hi, (size_t)B * E * Cin * 4));
   B200_TRY(d.get(&lo, (size_t)B * E * Cin * 4));
   B200_TRY(d.get(&wk, (size_t)N * n_taps * Cin * 4));
   B200_TRY(d.get(&wt, tc_packed_bytes(N, Cin, n_taps)));
   B200_TRY(d.get(&ytm, (size_t)B * Tout * N * 4));
-  const size_t ws_bytes = (size_t)64 << 20;
-  B200_TRY(d.get(&ws, ws_bytes));
   const long long n_in = (long long)B * E * Cin, n_w = (long long)N * n_taps * Cin;
   B200_LAUNCH(tm_pack_in_kernel, (unsigned)ceil_div64(n_in, 256), 256, 0, st, x_dev, (const float*)prev_dev, hi, lo, B, Cin, T, P, elu_in);
   if (transposed) B200_LAUNCH(tm_weight_convtr_kernel, (unsigned)ceil_div64(n_w, 256), 256, 0, st, w_dev, wk, Cin, Cout, S);
@@ -419,12 +415,12 @@ int b200_op_tc_conv1d(const float* x_dev, const float* w_dev, const float* bias_
   if (tc_tile_shape(Tout, &L.p.tt, &L.p.bb) != B200_OK) B200_FAIL(B200_ERR_SHAPE, "op_tc_conv1d: T");
   while (L.p.tt * L.stride > 256) { L.p.tt /= 2; L.p.bb *= 2; }
   L.p.row0 = 0;
-  L.p.epi = TC_EPI_CONV; L.p.y = ytm; L.p.y_sb = (long long)Tout * N; L.p.y_row = N; L.p.ws = ws;
+  L.p.epi = TC_EPI_CONV; L.p.y = ytm; L.p.y_sb = (long long)Tout * N; L.p.y_row = N;
   B200_TRY(tc_make_map(&L.map_hi, hi, Cin, (long long)E, (long long)E * Cin, B, L.p.tt, L.p.bb, L.stride));
   B200_TRY(tc_make_map(&L.map_lo, lo, Cin, (long long)E, (long long)E * Cin, B, L.p.tt, L.p.bb, L.stride));
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  B200_TRY(tc_plan(L, B, Tout, sms, ws_bytes));
+  B200_TRY(tc_plan(L, B, Tout, sms));
   B200_TRY(tc_launch(L, st));
   // token-major [B][Tout][N] -> the reference layout: conv [B][Cout][Tout]; convtr [B][Cout][Tout * S] (row t holds S steps of Cout)
   const int Tr = transposed ? Tout * S : Tout;
