@@ -99,13 +99,14 @@ struct b200_mimi {
   uint8_t* exec_mask = nullptr;
   uint8_t* first_flags = nullptr; int n_first = 0;
   ConvCommit* enc_commits = nullptr; int n_enc_commits = 0, max_enc_rows = 0;
-  ConvTrCommit* dec_tr_commits = nullptr; int n_dec_tr_commits = 0; long long max_tr_rows = 0;
+  TmZero* zeroed = nullptr; int n_zero = 0; long long max_zero = 0;      // what a reset clears
   TmCommit *enc_tm = nullptr, *dec_tm = nullptr; int n_enc_tm = 0, n_dec_tm = 0; long long max_enc_tm = 0, max_dec_tm = 0;
   long long* scratch_codes = nullptr;          // [B][K][1] for the host variants
   float* rvq_res[2] = {nullptr, nullptr};      // RVQ workspace: residuals, per-chunk partial argmin
   float* rvq_best[2] = {nullptr, nullptr};
   int* rvq_idx[2] = {nullptr, nullptr};
   int rvq_cap = 0;
+  float* down_x = nullptr;                     // [B][k][C]: what the down-sampling conv reads, as rows of a linear (null: not a shape of lin_launch)
   float* splitk_ws = nullptr; size_t splitk_bytes = 0;   // partial sums of the down-sampling conv
   int* err = nullptr;                                     // device error flags (B200_FLAG_CODE_RANGE)
   // one-frame encode / decode as CUDA graphs over static buffers (frame in enc[0].ext -> enc_codes, dec_codes -> out_frame)
@@ -454,7 +455,6 @@ int run_transformer(b200_mimi* h, Transformer& tr, const float* x_in, float* x, 
       q.res = x; q.scale = L.ls2; q.a_hi = e.a_hi; q.a_lo = e.a_lo; q.a_sb = e.a_sb; q.a_row = e.a_row; q.a_elu = e.act_elu;
       B200_TRY(lin_launch(q, h->body));
     }
-    B200_LAUNCH(advance_offsets_kernel, ceil_div(B, 128), 128, 0, h->body, tr.offset, h->exec_mask, B, T);
     return check_launch("mimi transformer");
   }
   const size_t attn_smem = (size_t)(T * D + T * c.tr_context) * sizeof(float);
@@ -477,7 +477,6 @@ int run_transformer(b200_mimi* h, Transformer& tr, const float* x_in, float* x, 
     B200_TRY(launch_tc(h, L.l1));             // h = gelu(linear1(xn)) as a hi / lo pair
     B200_TRY(launch_tc(h, L.l2));             // x = x + layer_scale_2 * linear2(h)
   }
-  B200_LAUNCH(advance_offsets_kernel, ceil_div(B, 128), 128, 0, h->body, tr.offset, h->exec_mask, B, T);
   return check_launch("mimi transformer");
 }
 
@@ -496,14 +495,16 @@ int run_seanet(b200_mimi* h, std::vector<SeaLayer>& layers) {
       const long long n = (long long)B * l.t_out;
       if (l.cout % 4 || 128 % (l.cout / 4) || l.k > 8) B200_FAIL(B200_ERR_INVALID, "mimi: first conv with %d channels / %d taps", l.cout, l.k);
       const int per_pass = 128 / (l.cout / 4);
-      q.tok_per_block = per_pass * 16;           // 16 passes per CTA: the 4 x K weights of a thread are loaded once
+      // the 4 x K weights of a thread are loaded once for all passes of its CTA; few sessions spread over the chip (16 passes always: 14.1 us at one session, 22.1 at 40; so 4.2 and 20.2)
+      const long long passes = n / ((long long)per_pass * 8 * h->sms);
+      q.tok_per_block = per_pass * (int)std::min<long long>(std::max<long long>(passes, 1), 16);
       B200_LAUNCH(conv_first_tm_kernel, (unsigned)ceil_div64(n, q.tok_per_block), 128, 0, h->body, q);
     } else if (l.simt_last) {
       ConvLast q;
       q.ext = l.ext_hi; q.e_sb = (long long)(l.P + l.t_in) * l.cin; q.Cin = l.cin; q.w = l.w_simt; q.bias = l.bias;
       q.y = l.y; q.y_sb = l.t_out; q.B = B; q.K = l.k; q.dil = l.dil; q.T = l.t_out;
       const long long n = (long long)B * l.t_out;
-      B200_LAUNCH(conv_last_tm_kernel, (unsigned)ceil_div64(n, 128), 128, (size_t)l.k * l.cin * 4, h->body, q);
+      B200_TRY(launch_early_if(mtc::tc_pdl(), conv_last_tm_kernel, dim3((unsigned)ceil_div64(n, 16)), dim3(128), (size_t)l.k * l.cin * 4, h->body, q));
     } else {
       B200_TRY(launch_tc(h, l.tc));
     }
@@ -513,26 +514,21 @@ int run_seanet(b200_mimi* h, std::vector<SeaLayer>& layers) {
 
 int commit_states(b200_mimi* h, bool encoder) {
   const int B = h->batch;
-  if (encoder) {
-    if (h->n_enc_commits) {      // the down-sampling conv (first-generation state layout + replicate flags)
-      dim3 grid(ceil_div(h->max_enc_rows, 128), h->n_enc_commits);
-      B200_LAUNCH(conv_commit_kernel, grid, 128, 0, h->body, h->enc_commits, h->n_enc_commits, h->exec_mask, B);
-      B200_LAUNCH(conv_clear_first_kernel, ceil_div(h->n_enc_commits * B, 128), 128, 0, h->body, h->enc_commits,
-                  h->n_enc_commits, h->exec_mask, B);
-    }
-    if (h->n_enc_tm) {
-      dim3 grid((unsigned)ceil_div64(h->max_enc_tm, 128), h->n_enc_tm);
-      B200_LAUNCH(tm_commit_kernel, grid, 128, 0, h->body, h->enc_tm, h->exec_mask, B);
-    }
-  } else {
-    if (h->n_dec_tm) {
-      dim3 grid((unsigned)ceil_div64(h->max_dec_tm, 128), h->n_dec_tm);
-      B200_LAUNCH(tm_commit_kernel, grid, 128, 0, h->body, h->dec_tm, h->exec_mask, B);
-    }
-    dim3 g2((unsigned)ceil_div64(h->max_tr_rows, 256), h->n_dec_tr_commits);      // the depth-wise up-sampling's overlap-add carry
-    B200_LAUNCH(convtr_commit_kernel, g2, 256, 0, h->body, h->dec_tr_commits, h->exec_mask, B);
+  if (encoder && !h->down_x) {   // the down-sampling conv (first-generation state layout + replicate flags), where down_gather_kernel has not done it
+    dim3 grid(ceil_div(h->max_enc_rows, 128), h->n_enc_commits);
+    B200_LAUNCH(conv_commit_kernel, grid, 128, 0, h->body, h->enc_commits, h->n_enc_commits, h->exec_mask, B);
+    B200_LAUNCH(conv_clear_first_kernel, ceil_div(h->n_enc_commits * B, 128), 128, 0, h->body, h->enc_commits,
+                h->n_enc_commits, h->exec_mask, B);
   }
-  return check_launch("commit_states");
+  TmCarry c;
+  memset(&c, 0, sizeof(c));
+  c.offset = encoder ? h->enc_tr.offset : h->dec_tr.offset;
+  c.T = h->rs;
+  if (!encoder) { c.partial = h->up_partial; c.scratch = h->up_scratch; c.per_row = h->cfg.dimension * h->rs; }      // the depth-wise up-sampling's overlap-add carry
+  const int n = encoder ? h->n_enc_tm : h->n_dec_tm;
+  const long long most = std::max(encoder ? h->max_enc_tm : h->max_dec_tm, (long long)B * c.per_row);
+  const dim3 grid((unsigned)std::min<long long>(ceil_div64(most, 128), 256), (unsigned)n + 1);
+  return launch_early_if(mtc::tc_pdl(), tm_commit_kernel, grid, dim3(128), 0, h->body, (const TmCommit*)(encoder ? h->enc_tm : h->dec_tm), n, c, (const uint8_t*)h->exec_mask, B);
 }
 
 // frame in enc[0].ext -> latent [B][C]   (static buffers only: this is what gets captured into a graph)
@@ -541,7 +537,16 @@ int encode_body(b200_mimi* h) {
   const int T = h->frame_size / h->hop;   // encoder tokens per frame (2)
   B200_TRY(run_seanet(h, h->enc));        // the last conv's raw output is tok_in_enc, token-major [B][T][C]
   B200_TRY(run_transformer(h, h->enc_tr, h->tok_in_enc, h->tok_enc, T));
-  {                                       // learnt down-sampling conv reads token-major, writes latent [B][C][1]
+  if (h->down_x) {                        // learnt down-sampling conv reads token-major, writes latent [B][C][1]
+    const DownLayer& l = h->down;
+    DownGather g;
+    g.tok = h->tok_enc; g.st = l.state; g.first = l.first; g.exec_mask = h->exec_mask; g.x = h->down_x; g.C = l.cin; g.P = l.P; g.T = l.t_in; g.k = l.k;
+    B200_TRY(launch_early_if(mtc::tc_pdl(), down_gather_kernel, dim3((unsigned)h->batch), dim3(256), 0, h->body, g));
+    LinP p;
+    memset(&p, 0, sizeof(p));
+    p.x = h->down_x; p.w = l.w; p.n_tok = h->batch; p.N = l.cout; p.K = l.k * l.cin; p.T = 1; p.epi = LIN_STORE; p.y = h->latent;
+    B200_TRY(lin_launch(p, h->body));
+  } else {
     const DownLayer& l = h->down;
     ConvP p;
     p.x = h->tok_enc; p.xb = (long long)T * d; p.xc = 1; p.xt = d; p.Tin = l.t_in;
@@ -725,8 +730,8 @@ int decode_latent_body(b200_mimi* h) {
   const int T = S;   // tokens per frame after up-sampling
   {
     const long long total = (long long)B * 2 * S * d;   // (T_in + 1) * S * C with T_in = 1
-    B200_LAUNCH(upsample_dw_kernel, (unsigned)ceil_div64(total, 256), 256, 0, h->body, h->latent_q, (long long)d, 1LL, 1LL, 1,
-                h->up_w, h->up_partial, h->up_scratch, h->tok_in_dec, B, d, S);
+    B200_TRY(launch_early_if(mtc::tc_pdl(), upsample_dw_kernel, dim3((unsigned)ceil_div64(total, 256)), dim3(256), 0, h->body, h->latent_q, (long long)d, 1LL, 1LL, 1,
+                h->up_w, h->up_partial, h->up_scratch, h->tok_in_dec, B, d, S));
   }
   B200_TRY(run_transformer(h, h->dec_tr, h->tok_in_dec, h->tok_dec, T));   // its last linear also fills dec[0]'s ext
   B200_TRY(run_seanet(h, h->dec));
@@ -917,8 +922,14 @@ int b200_mimi_streaming_begin(b200_mimi* h, int batch, void* stream) {
   B200_TRY(A.alloc_t(&h->exec_mask, B, false));
   B200_CUDA(cudaMemset(h->exec_mask, 1, B));
   B200_TRY(A.alloc_t(&h->err, 1));
-  h->splitk_bytes = (size_t)64 << 20;
-  B200_TRY(A.alloc(reinterpret_cast<void**>(&h->splitk_ws), h->splitk_bytes, false));
+  h->down_x = nullptr;
+  h->splitk_ws = nullptr; h->splitk_bytes = 0;
+  if (h->rs == h->down.stride && lin_takes(h->down.cout, h->down.k * h->down.cin)) {      // one output step per frame
+    B200_TRY(A.alloc_t(&h->down_x, (size_t)B * h->down.k * h->down.cin, false));
+  } else {
+    h->splitk_bytes = (size_t)64 << 20;
+    B200_TRY(A.alloc(reinterpret_cast<void**>(&h->splitk_ws), h->splitk_bytes, false));
+  }
 
   // flags for replicate-padded convs (only the down-sampling conv in Mimi)
   h->n_first = 1;
@@ -1024,27 +1035,31 @@ int b200_mimi_streaming_begin(b200_mimi* h, int batch, void* stream) {
     h->max_enc_rows = B * l.cin;
   }
   // up-sampling depth-wise convtr
-  std::vector<ConvTrCommit> dec_t;
   B200_TRY(A.alloc_t(&h->up_partial, (size_t)B * d * h->rs));
   B200_TRY(A.alloc_t(&h->up_scratch, (size_t)B * d * h->rs));
-  {
-    ConvTrCommit tc;
-    tc.partial = h->up_partial; tc.scratch = h->up_scratch; tc.per_row = d * h->rs;
-    dec_t.push_back(tc);
-    h->max_tr_rows = (long long)B * tc.per_row;
-  }
   h->n_enc_commits = (int)enc_c.size();
-  h->n_dec_tr_commits = (int)dec_t.size();
   h->n_enc_tm = (int)enc_tm.size();
   h->n_dec_tm = (int)dec_tm.size();
   B200_TRY(A.alloc_t(&h->enc_commits, enc_c.size(), false));
-  B200_TRY(A.alloc_t(&h->dec_tr_commits, dec_t.size(), false));
   B200_TRY(A.alloc_t(&h->enc_tm, enc_tm.size() ? enc_tm.size() : 1, false));
   B200_TRY(A.alloc_t(&h->dec_tm, dec_tm.size() ? dec_tm.size() : 1, false));
   B200_CUDA(cudaMemcpy(h->enc_commits, enc_c.data(), enc_c.size() * sizeof(ConvCommit), cudaMemcpyHostToDevice));
-  B200_CUDA(cudaMemcpy(h->dec_tr_commits, dec_t.data(), dec_t.size() * sizeof(ConvTrCommit), cudaMemcpyHostToDevice));
   if (!enc_tm.empty()) B200_CUDA(cudaMemcpy(h->enc_tm, enc_tm.data(), enc_tm.size() * sizeof(TmCommit), cudaMemcpyHostToDevice));
   if (!dec_tm.empty()) B200_CUDA(cudaMemcpy(h->dec_tm, dec_tm.data(), dec_tm.size() * sizeof(TmCommit), cudaMemcpyHostToDevice));
+
+  {
+    std::vector<TmZero> z;
+    for (auto* layers : {&h->enc, &h->dec})
+      for (auto& l : *layers)
+        for (float* p : {l.ext_hi, l.ext_lo})
+          if (l.P > 0 && p) z.push_back({p, (long long)l.P * l.cin, (long long)(l.P + l.t_in) * l.cin});
+    if (h->down.P > 0) z.push_back({h->down.state, (long long)h->down.cin * h->down.P, (long long)h->down.cin * h->down.P});
+    z.push_back({h->up_partial, (long long)d * h->rs, (long long)d * h->rs});
+    h->n_zero = (int)z.size(); h->max_zero = 0;
+    for (auto& e : z) h->max_zero = std::max(h->max_zero, e.per_row);
+    B200_TRY(A.alloc_t(&h->zeroed, z.size(), false));
+    B200_CUDA(cudaMemcpy(h->zeroed, z.data(), z.size() * sizeof(TmZero), cudaMemcpyHostToDevice));
+  }
 
   // transformers
   const int H = c.tr_num_heads, D = d / H, ff = c.tr_dim_feedforward;
@@ -1189,20 +1204,10 @@ int b200_mimi_reset(b200_mimi* h, const uint8_t* reset_mask_dev) {
   B200_TRY(ensure_streaming(h, "mimi_reset"));
   DeviceGuard g(h->device);
   const int B = h->batch;
-  auto zero = [&](float* buf, long long per_row) {
-    if (!buf || per_row <= 0) return;
-    B200_LAUNCH(zero_rows_kernel, (unsigned)ceil_div64((long long)B * per_row, 256), 256, 0, h->stream, buf, per_row,
-                reset_mask_dev, B);
-  };
-  for (auto* layers : {&h->enc, &h->dec})
-    for (auto& l : *layers)
-      if (l.P > 0)
-        B200_LAUNCH(tm_zero_kernel, (unsigned)ceil_div64((long long)B * l.P * l.cin, 256), 256, 0, h->stream, l.ext_hi, l.ext_lo, l.P,
-                    l.cin, (long long)(l.P + l.t_in) * l.cin, reset_mask_dev, B);
-  zero(h->down.state, (long long)h->down.cin * h->down.P);
-  zero(h->up_partial, (long long)h->cfg.dimension * h->rs);
-  B200_LAUNCH(reset_flags_kernel, ceil_div(B, 128), 128, 0, h->stream, h->first_flags, h->n_first, h->enc_tr.offset,
-              h->dec_tr.offset, h->exec_mask, reset_mask_dev, B);
+  TmFlags f;
+  f.first = h->first_flags; f.exec_mask = h->exec_mask; f.n_first = h->n_first; f.off_a = h->enc_tr.offset; f.off_b = h->dec_tr.offset;
+  const dim3 grid((unsigned)std::min<long long>(ceil_div64((long long)B * h->max_zero, 256), 128), (unsigned)h->n_zero + 1);
+  B200_LAUNCH(tm_reset_kernel, grid, 256, 0, h->stream, h->zeroed, h->n_zero, f, reset_mask_dev, B);
   return check_launch("mimi_reset");
 }
 

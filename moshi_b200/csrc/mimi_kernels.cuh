@@ -13,6 +13,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tc_prims.cuh"
 
 namespace b200 {
 namespace mimi {
@@ -220,10 +221,6 @@ struct ConvCommit {   // previous <- last P samples of cat(previous, act(x))   (
   float* st; int P, Cin, elu_in;
   uint8_t* first;     // replicate flags (cleared where exec_mask) or nullptr
 };
-struct ConvTrCommit { // partial <- scratch   (conv.py:357-360)
-  float* partial; const float* scratch; int per_row;   // Cout * S
-};
-
 static __global__ void conv_commit_kernel(const ConvCommit* descs, int n_desc, const uint8_t* exec_mask, int B) {
   const ConvCommit d = descs[blockIdx.y];
   const int row = blockIdx.x * blockDim.x + threadIdx.x;   // (b, ci)
@@ -255,38 +252,16 @@ static __global__ void conv_clear_first_kernel(const ConvCommit* descs, int n_de
   if (d.first != nullptr && exec_mask[b]) d.first[b] = 0;
 }
 
-static __global__ void convtr_commit_kernel(const ConvTrCommit* descs, const uint8_t* exec_mask, int B) {
-  const ConvTrCommit d = descs[blockIdx.y];
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)B * d.per_row) return;
-  if (exec_mask[i / d.per_row]) d.partial[i] = d.scratch[i];
-}
-
-// reset: zero the state of the rows in reset_mask (conv.py:166-169, 281-286)
-static __global__ void zero_rows_kernel(float* buf, long long per_row, const uint8_t* mask, int B) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)B * per_row) return;
-  if (mask == nullptr || mask[i / per_row]) buf[i] = 0.f;
-}
-static __global__ void reset_flags_kernel(uint8_t* first /*[n_first][B]*/, int n_first, long long* off_a, long long* off_b,
-                                   uint8_t* exec_mask, const uint8_t* mask, int B) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  if (mask != nullptr && !mask[b]) return;
-  exec_mask[b] = 1;                                       // State.reset (streaming.py:41-42)
-  for (int i = 0; i < n_first; ++i) first[(long long)i * B + b] = 1;
-  if (off_a) off_a[b] = 0;                                // _MHAState.reset / RingKVCache.reset
-  if (off_b) off_b[b] = 0;
-}
-
 // ---------------------------------------------------------------------------------------------
 // depth-wise ConvTranspose1d up-sampling (resample.py:68-119 with channel_wise=True, k=2S, no bias)
 // latent [B][C] (one frame) -> tokens [B][S][C] (token-major for the decoder transformer)
 // ---------------------------------------------------------------------------------------------
-static __global__ void upsample_dw_kernel(const float* __restrict__ lat, long long lb, long long lc, long long lt, int T,
-                                   const float* __restrict__ w /*[C][2S]*/, const float* __restrict__ partial,
-                                   float* __restrict__ scratch, float* __restrict__ y /*[B][T*S][C]*/,
+static __global__ void upsample_dw_kernel(const float* lat, long long lb, long long lc, long long lt, int T,
+                                   const float* __restrict__ w /*[C][2S]*/, const float* partial,
+                                   float* scratch, float* y /*[B][T*S][C]*/,
                                    int B, int C, int S) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long total = (long long)B * (T + 1) * S * C;
   if (i >= total) return;
@@ -302,12 +277,6 @@ static __global__ void upsample_dw_kernel(const float* __restrict__ lat, long lo
   if (t == 0) v += partial[sidx];
   else v += w[c * 2 * S + r + S] * xr[(long long)(t - 1) * lt];
   y[((long long)b * T * S + (long long)t * S + r) * C + c] = v;
-}
-
-// per-session token counters of a bottleneck transformer (== RingKVCache.end_offset == _MHAState.offset), advanced where exec_mask
-static __global__ void advance_offsets_kernel(long long* off, const uint8_t* exec_mask, int B, int T) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < B && exec_mask[b]) off[b] += T;
 }
 
 // ---------------------------------------------------------------------------------------------

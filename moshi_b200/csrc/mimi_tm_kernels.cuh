@@ -65,7 +65,8 @@ static __global__ void __launch_bounds__(128) conv_first_tm_kernel(const ConvFir
   }
 }
 
-// Last decoder conv (Cout = 1; seanet.py:380-388): one thread per (b, t) reduces over (tap, ci) from a plain fp32 ext
+// Last decoder conv (Cout = 1; seanet.py:380-388): eight lanes per (b, t) reduce over (tap, ci) from a plain fp32 ext, 16 bytes each of a row of 128 at a time
+// (one thread per (b, t), as many rows apart as there are lanes: 22.0 us at 40 sessions, 7.8 at one; so 10.8 and 5.4)
 struct ConvLast {
   const float* ext; long long e_sb; int Cin;  // [B][P + T][Cin], activation already applied
   const float* w;                             // [K][Cin]
@@ -74,23 +75,28 @@ struct ConvLast {
   int B, K, dil, T;
 };
 static __global__ void __launch_bounds__(128) conv_last_tm_kernel(const ConvLast p) {
-  extern __shared__ float sw[];               // [K * Cin]
+  extern __shared__ __align__(16) float sw[];      // [K * Cin]
   for (int i = threadIdx.x; i < p.K * p.Cin; i += blockDim.x) sw[i] = p.w[i];
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
   __syncthreads();
-  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= (long long)p.B * p.T) return;
-  const int b = (int)(n / p.T), t = (int)(n - (long long)b * p.T);
-  float acc = p.bias ? p.bias[0] : 0.f;
-  for (int kw = 0; kw < p.K; ++kw) {
-    const float4* e = reinterpret_cast<const float4*>(p.ext + (long long)b * p.e_sb + (long long)(t + kw * p.dil) * p.Cin);
-    const float* wk = sw + kw * p.Cin;
-    for (int c4 = 0; c4 < p.Cin / 4; ++c4) {
-      const float4 v = e[c4];
-      acc = fmaf(wk[4 * c4], v.x, acc); acc = fmaf(wk[4 * c4 + 1], v.y, acc);
-      acc = fmaf(wk[4 * c4 + 2], v.z, acc); acc = fmaf(wk[4 * c4 + 3], v.w, acc);
+  const int l = threadIdx.x & 7;
+  const long long n = (long long)blockIdx.x * 16 + (threadIdx.x >> 3);
+  const bool some = n < (long long)p.B * p.T;
+  const int b = some ? (int)(n / p.T) : 0, t = some ? (int)(n - (long long)b * p.T) : 0;
+  const float4* e = reinterpret_cast<const float4*>(p.ext + (long long)b * p.e_sb + (long long)t * p.Cin);
+  const float4* w = reinterpret_cast<const float4*>(sw);
+  const int n4 = p.Cin / 4;
+  float acc = 0.f;
+  for (int kw = 0; kw < p.K; ++kw)
+#pragma unroll 2
+    for (int c = l; c < n4; c += 8) {
+      const float4 v = e[(long long)kw * p.dil * n4 + c], f = w[kw * n4 + c];
+      acc = fmaf(f.x, v.x, acc); acc = fmaf(f.y, v.y, acc); acc = fmaf(f.z, v.z, acc); acc = fmaf(f.w, v.w, acc);
     }
-  }
-  p.y[(long long)b * p.y_sb + t] = acc;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (some && l == 0) p.y[(long long)b * p.y_sb + t] = acc + (p.bias ? p.bias[0] : 0.f);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -99,30 +105,93 @@ static __global__ void __launch_bounds__(128) conv_last_tm_kernel(const ConvLast
 // (conv.py:349-361) is the same thing with P = 1 (the last input step).  Buffers are described once per direction.
 // ---------------------------------------------------------------------------------------------
 struct TmCommit { float* hi; float* lo; int P, T, rowlen; long long sb; };       // rowlen = Cin floats per row
-static __global__ void tm_commit_kernel(const TmCommit* descs, const uint8_t* exec_mask, int B) {
-  pdl_trigger_next();
-  const TmCommit d = descs[blockIdx.y];
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;      // (b, ci)
-  if (i >= (long long)B * d.rowlen) return;
-  const int b = (int)(i / d.rowlen), ci = (int)(i - (long long)b * d.rowlen);
-  if (!exec_mask[b]) return;
-  float* h = d.hi + (long long)b * d.sb + ci;
-  for (int j = 0; j < d.P; ++j) h[(long long)j * d.rowlen] = h[(long long)(d.T + j) * d.rowlen];      // ascending: reads stay ahead of writes
-  if (d.lo != nullptr) {
-    float* l = d.lo + (long long)b * d.sb + ci;
-    for (int j = 0; j < d.P; ++j) l[(long long)j * d.rowlen] = l[(long long)(d.T + j) * d.rowlen];
+// What else a direction carries: its transformer's token counters (== RingKVCache.end_offset == _MHAState.offset), the depth-wise up-sampling's overlap-add
+// (conv.py:357-360; partial <- scratch)
+struct TmCarry { long long* offset; int T; float* partial; const float* scratch; int per_row; };
+
+template <typename V>
+__device__ __forceinline__ void shift_rows(V* h, V* l, int P, int T, int row) {
+  for (int j0 = 0; j0 < P; j0 += 8) {            // eight rows at a time, read before any of them is written: reads stay ahead of writes
+    V a[8], c[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j0 + j < P) {
+        a[j] = h[(long long)(T + j0 + j) * row];
+        if (l) c[j] = l[(long long)(T + j0 + j) * row];
+      }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j0 + j < P) {
+        h[(long long)(j0 + j) * row] = a[j];
+        if (l) l[(long long)(j0 + j) * row] = c[j];
+      }
   }
 }
-// reset (conv.py:166-169, 281-286): zero the carried rows of the sessions in mask (null = all)
-static __global__ void tm_zero_kernel(float* hi, float* lo, int P, int rowlen, long long sb, const uint8_t* mask, int B) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long per = (long long)P * rowlen;
-  if (i >= (long long)B * per) return;
-  const int b = (int)(i / per);
-  if (mask != nullptr && !mask[b]) return;
-  const long long o = (long long)b * sb + (i - (long long)b * per);
-  hi[o] = 0.f;
-  if (lo != nullptr) lo[o] = 0.f;
+// grid (.., n_desc + 1).  Row by row, every load behind the store before it, and with launches of their own for the counters and the up-sampling: 14.6 us at one
+// session, 16.6 at 40; so 4.5 and 8.4
+static __global__ void __launch_bounds__(128) tm_commit_kernel(const TmCommit* descs, int n_desc, const TmCarry c, const uint8_t* exec_mask, int B) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  if ((int)blockIdx.y == n_desc) {
+    for (long long i = first; i < B; i += step)
+      if (exec_mask[i]) c.offset[i] += c.T;
+    for (long long i = first; i < (long long)B * c.per_row; i += step)
+      if (exec_mask[i / c.per_row]) c.partial[i] = c.scratch[i];
+    return;
+  }
+  const TmCommit d = descs[blockIdx.y];
+  const int per = d.rowlen % 4 == 0 ? 4 : 1, row = d.rowlen / per;      // the buffers start on 16 bytes
+  for (long long i = first; i < (long long)B * row; i += step) {        // (b, ci / per)
+    const int b = (int)(i / row);
+    if (!exec_mask[b]) continue;
+    const long long o = (long long)b * d.sb + (i - (long long)b * row) * per;
+    if (per == 4) shift_rows(reinterpret_cast<float4*>(d.hi + o), d.lo ? reinterpret_cast<float4*>(d.lo + o) : nullptr, d.P, d.T, row);
+    else shift_rows(d.hi + o, d.lo ? d.lo + o : nullptr, d.P, d.T, row);
+  }
+}
+
+// reset (conv.py:166-169, 281-286; streaming.py:41-42): everything carried by the sessions in mask (null = all), in one launch (22 launches of 2.3 us before).  grid (.., n + 1)
+struct TmZero { float* p; long long per_row, stride; };      // per session: floats, and from one session to the next
+struct TmFlags { uint8_t *first, *exec_mask; int n_first; long long *off_a, *off_b; };
+static __global__ void __launch_bounds__(256) tm_reset_kernel(const TmZero* descs, int n, const TmFlags f, const uint8_t* mask, int B) {
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  if ((int)blockIdx.y == n) {
+    for (long long b = first; b < B; b += step) {
+      if (mask != nullptr && !mask[b]) continue;
+      f.exec_mask[b] = 1;
+      for (int i = 0; i < f.n_first; ++i) f.first[(long long)i * B + b] = 1;
+      f.off_a[b] = 0;
+      f.off_b[b] = 0;
+    }
+    return;
+  }
+  const TmZero d = descs[blockIdx.y];
+  for (long long i = first; i < (long long)B * d.per_row; i += step) {
+    const long long b = i / d.per_row;
+    if (mask == nullptr || mask[b]) d.p[b * d.stride + (i - b * d.per_row)] = 0.f;
+  }
+}
+
+// The learnt down-sampling conv (resample.py:14-65) as a linear: x[b] = its k steps of cat(previous, tokens) side by side (replicated on a session's first frame,
+// conv.py:255-262), and on the way previous <- the last P of them where exec_mask.  One CTA per session; one output step per frame.  Gather and linear 4.9 + 4.2 us at
+// one session; k cut over 256 CTAs, a launch that adds, one that commits and one that clears the flags: 28.9.
+struct DownGather { const float* tok; float* st; uint8_t* first; const uint8_t* exec_mask; float* x; int C, P, T, k; };      // tok [B][T][C], st [B][C][P], x [B][k][C]
+static __global__ void __launch_bounds__(256) down_gather_kernel(const DownGather p) {
+  tcp::pdl_trigger();
+  tcp::pdl_wait();
+  const int b = blockIdx.x;
+  const bool rep = p.first[b] != 0, exec = p.exec_mask[b] != 0;
+  const float* tok = p.tok + (long long)b * p.T * p.C;
+  for (int c = threadIdx.x; c < p.C; c += blockDim.x) {
+    float* st = p.st + ((long long)b * p.C + c) * p.P;
+    auto at = [&](int e) { return e >= p.P ? tok[(long long)(e - p.P) * p.C + c] : rep ? tok[c] : st[e]; };
+    for (int e = 0; e < p.k; ++e) p.x[((long long)b * p.k + e) * p.C + c] = at(e);
+    if (exec)
+      for (int j = 0; j < p.P; ++j) st[j] = at(p.T + j);      // ascending: reads run ahead of writes
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && exec) p.first[b] = 0;
 }
 
 // LayerNorm (eps 1e-5, affine; transformer.py:126) -> the following linear's input as a hi / lo pair.  One warp per token, the row in registers (C <= 512, a
