@@ -47,7 +47,7 @@ struct WideP {
   int vec;                                            // results in 16-byte stores
   int act_from, act_to; __nv_bfloat16* y2; long long ldy2;
   uint32_t stage_bytes;
-  uint32_t a_bytes;                                   // bytes of a box of x rows (128 rows; fewer where no tile has more)
+  uint32_t a_bytes, bars_at;                          // bytes of a box of x rows (128 rows; fewer where no tile has more); mbarriers of gemm_expert_kernel
   int* err;
 };
 
@@ -160,12 +160,13 @@ __device__ __forceinline__ void store_run(__nv_bfloat16* row, int col, int cols,
   }
 }
 
-// 32 neighbouring sums of one row through the epilogue
+// NV (16 or 32) neighbouring sums of one row through the epilogue
+template <int NV>
 __device__ __forceinline__ void finish_run(const WideP& p, __nv_bfloat16* y, long long yr, int n, float* v) {
   if (p.act == WIDE_CLAMPED_GLU || p.act == WIDE_SILU_GLU) {      // weight rows interleave gate and value
-    float o[16];
+    float o[NV / 2];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < NV / 2; ++j) {
       const float g = v[2 * j], w = v[2 * j + 1];
       if (p.act == WIDE_SILU_GLU) {
         o[j] = g / (1.f + expf(-g)) * w;
@@ -174,19 +175,19 @@ __device__ __forceinline__ void finish_run(const WideP& p, __nv_bfloat16* y, lon
         o[j] = gc / (1.f + expf(-1.702f * gc)) * (wc + 1.f);
       }
     }
-    store_run<16>(y, n >> 1, p.N >> 1, o, p.vec);
+    store_run<NV / 2>(y, n >> 1, p.N >> 1, o, p.vec);
     return;
   }
   const bool aside = n >= p.act_from && n < p.act_to;
   if (p.act == WIDE_RELU2 || aside) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) { v[j] = fmaxf(v[j], 0.f); v[j] *= v[j]; }
+    for (int j = 0; j < NV; ++j) { v[j] = fmaxf(v[j], 0.f); v[j] *= v[j]; }
   } else if (p.act == WIDE_GELU) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = 0.5f * v[j] * (1.f + erff(v[j] * 0.7071067811865476f));
+    for (int j = 0; j < NV; ++j) v[j] = 0.5f * v[j] * (1.f + erff(v[j] * 0.7071067811865476f));
   }
-  if (aside) store_run<32>(p.y2 + yr * p.ldy2, n - p.act_from, p.act_to - p.act_from, v, p.vec);
-  else store_run<32>(y, n, p.N, v, p.vec);
+  if (aside) store_run<NV>(p.y2 + yr * p.ldy2, n - p.act_from, p.act_to - p.act_from, v, p.vec);
+  else store_run<NV>(y, n, p.N, v, p.vec);
 }
 
 // whether all 128 epilogue threads say so (a barrier of theirs)
@@ -368,7 +369,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
               }
             }
           }
-          if (row_ok && n < p.N) finish_run(p, y, yr, n, v);
+          if (row_ok && n < p.N) finish_run<32>(p, y, yr, n, v);
         }
       }
       if (whole) {
@@ -383,6 +384,172 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   if (warp == 1) dealloc_tmem<CG>(tmem, 2 * BN);
   if (threadIdx.x == 0 && quit && p.err) atomicOr(p.err, WIDE_ERR_WAIT);
   pair_sync<CG>();
+}
+
+// Grouped product of few rows per expert (one tile each): a stream of the experts' weights.  Their rows, laid end to end, are dealt to the CTAs in units of 16, so that
+// every SM streams the same number of them to within one unit; a CTA takes its share in tiles of up to 128 rows of one expert.  With whole tiles of 256 columns dealt over
+// 148 SMs the last of few waves was mostly empty: 10 experts of 8192 x 2048 are 320 tiles in three waves, and of 2048 x 4096 80 tiles for 148 SMs.
+// us, tiles of 256 columns / here / the weights at 6.55 TB/s: 8192 x 2048, 2 experts 33.1 / 16.5 / 10.2, 10 81.4 / 62.2 / 51.2, 16 with 4 rows each 126.3 / 100.6 / 81.9, with
+// 16 rows 157.1 / 118.1; 2048 x 4096, 2 experts 25.9 / 11.1 / 5.1, 10 34.3 / 31.0 / 25.6, 16 with 16 rows 48.6 / 49.8 / 41.0.
+// What bounded it on the way is how fast a thread asks and issues: a copy per unit and products from one thread 90 us for 10 experts of 8192 x 2048, both loops
+// walked by whole warps 60.8 (2048 x 4096: 60 and 37.3), one copy and two k-blocks per stage 62.2 and 31.0.
+__device__ __forceinline__ bool elected() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
+  return r != 0;
+}
+__device__ __forceinline__ void commit_elected(uint32_t bar) {
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
+}
+// low word of make_desc (tc_prims.cuh); the high word is the same for every operand
+constexpr uint32_t DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_low(uint32_t smem) { return ((smem & 0x3FFFFu) >> 4) | (1u << 16); }
+// the four products of a k-block, by one thread of the warp: rows at desc a, columns w_at 16-byte pieces behind them
+__device__ __forceinline__ void umma_bf16_block(uint32_t d, uint32_t a, uint32_t w_at, uint32_t idesc, uint32_t accumulate) {
+  const uint32_t w = a + w_at;
+  asm volatile(
+      "{\n\t.reg .pred p, t, q;\n\t.reg .b64 a0, a1, a2, a3, w0, w1, w2, w3;\n\t"
+      "mov.b64 a0, {%1, %11};\n\tmov.b64 a1, {%2, %11};\n\tmov.b64 a2, {%3, %11};\n\tmov.b64 a3, {%4, %11};\n\t"
+      "mov.b64 w0, {%5, %11};\n\tmov.b64 w1, {%6, %11};\n\tmov.b64 w2, {%7, %11};\n\tmov.b64 w3, {%8, %11};\n\t"
+      "setp.ne.b32 p, %10, 0;\n\tsetp.ne.b32 t, %11, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a0, w0, %9, p;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, w1, %9, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, w2, %9, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, w3, %9, t;\n\t}"
+      ::"r"(d), "r"(a), "r"(a + 2), "r"(a + 4), "r"(a + 6), "r"(w), "r"(w + 2), "r"(w + 4), "r"(w + 6), "r"(idesc), "r"(accumulate), "r"(DESC_HIGH) : "memory");
+}
+constexpr int EXPERT_SMEM = 216 * 1024;
+constexpr int UNIT = 16, TILE_UNITS = 8, EXPERT_ST = 6, STAGE_KB = 2;      // STAGE_KB: k-blocks per stage
+struct alignas(64) ExpertMaps { CUtensorMap x, w[TILE_UNITS]; };             // w[n - 1]: boxes of n units, so that a tile's rows come in one copy per k-block
+struct ExpertTile { int m, row, units; };      // tile of the table, first weight row of the expert, units of 16
+__device__ __forceinline__ ExpertTile expert_tile(int u, int end, int per_expert) {
+  ExpertTile t;
+  t.m = u / per_expert;
+  const int left = min(end, (t.m + 1) * per_expert) - u, tiles = (left + TILE_UNITS - 1) / TILE_UNITS;
+  t.row = (u - t.m * per_expert) * UNIT;
+  t.units = (left + tiles - 1) / tiles;        // tiles of equal length
+  return t;
+}
+
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_expert_kernel(const __grid_constant__ ExpertMaps maps, const WideP p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ volatile int quit;
+  constexpr int COLS = TILE_UNITS * UNIT;
+  const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
+  const uint32_t stage_bytes = p.stage_bytes, x_bytes = (p.a_bytes + 1023u) / 1024u * 1024u, w_at = STAGE_KB * x_bytes;      // x rows of the k-blocks first, then weight rows
+  const uint32_t bars = base + p.bars_at;
+  const uint32_t full0 = bars, empty0 = bars + 8 * EXPERT_ST, tfull0 = bars + 16 * EXPERT_ST, tempty0 = tfull0 + 16, tptr = tempty0 + 16;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    quit = 0;
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(tfull0 + 8 * a, 1);
+      mbar_init(tempty0 + 8 * a, 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x) : "memory");
+  }
+  if (warp == 1) tmem_alloc(tptr, 2 * COLS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<const uint32_t*>(smem_raw + (tptr - raw));
+  pdl_trigger();
+  pdl_wait();                                           // rows, table and results are the preceding kernels' business
+  const int per_expert = (p.N + UNIT - 1) / UNIT;
+  const unsigned units = (unsigned)(p.n_tiles[0] * per_expert);
+  const int u0 = (int)((unsigned long long)units * blockIdx.x / gridDim.x), u1 = (int)((unsigned long long)units * (blockIdx.x + 1) / gridDim.x);
+
+  // both loops are walked by their whole warps, so that what the copies and products take is in uniform registers, and one thread issues
+  if (warp == 0) {
+    int s = 0; uint32_t ph = 0;
+    bool ok = true;
+    for (int u = u0; ok && u < u1;) {
+      const ExpertTile t = expert_tile(u, u1, per_expert);
+      const int row0 = p.tile_r0[t.m], w0 = p.tile_e[t.m] * p.e_rows + t.row;
+      const uint32_t bytes = STAGE_KB * (p.a_bytes + (uint32_t)t.units * UNIT * BK * 2);
+      const CUtensorMap* map_w = &maps.w[t.units - 1];
+      for (int kb = 0; kb < p.num_kb; kb += STAGE_KB) {      // blocks beyond the last are zeroes
+        const uint32_t bar = full0 + 8 * s, sa = base + (uint32_t)s * stage_bytes;
+        if (!wait_or_quit(empty0 + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
+        if (elected()) {
+          mbar_expect_tx(bar, bytes);
+#pragma unroll
+          for (int j = 0; j < STAGE_KB; ++j) {
+            tma_load_2d(sa + w_at + j * COLS * BK * 2, map_w, bar, (kb + j) * BK, w0);
+            tma_load_2d(sa + j * x_bytes, &maps.x, bar, (kb + j) * BK, row0);
+          }
+        }
+        __syncwarp();
+        if (++s == p.stages) { s = 0; ph ^= 1u; }
+      }
+      u += t.units;
+    }
+    if (!ok) {                                          // let copies in flight land before the block ends
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 2000000ull) {}
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    int s = 0, it = 0; uint32_t ph = 0;
+    bool ok = true;
+    for (int u = u0; ok && u < u1; ++it) {
+      const ExpertTile t = expert_tile(u, u1, per_expert);
+      const uint32_t a = it & 1, d = tmem + a * COLS, idesc = make_idesc(128, t.units * UNIT);
+      if (!wait_or_quit(tempty0 + 8 * a, ((it >> 1) & 1) ^ 1u, &quit)) break;
+      tc_fence_after();
+      for (int kb = 0; kb < p.num_kb; kb += STAGE_KB) {
+        if (!wait_or_quit(full0 + 8 * s, ph, &quit)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sa = desc_low(base + (uint32_t)s * stage_bytes);
+#pragma unroll
+        for (int j = 0; j < STAGE_KB; ++j) umma_bf16_block(d, sa + j * (x_bytes >> 4), (w_at + j * (COLS * BK * 2 - x_bytes)) >> 4, idesc, kb + j > 0 ? 1u : 0u);
+        commit_elected(empty0 + 8 * s);
+        if (++s == p.stages) { s = 0; ph ^= 1u; }
+      }
+      if (ok) commit_elected(tfull0 + 8 * a);
+      u += t.units;
+    }
+    __syncwarp();
+  } else {
+    const int q4 = warp & 3, r = q4 * 32 + lane;        // row of the tile
+    int it = 0;
+    for (int u = u0; u < u1; ++it) {
+      const ExpertTile t = expert_tile(u, u1, per_expert);
+      const int rows = p.tile_n[t.m], row0 = p.tile_r0[t.m];
+      const bool row_ok = r < rows;
+      const long long yr = row_ok && p.y_rows ? p.y_rows[row0 + r] : row0 + r;
+      __nv_bfloat16* y = p.y + yr * p.ldy;
+      const uint32_t a = it & 1;
+      if (!epilogue_all(wait_or_quit(tfull0 + 8 * a, (it >> 1) & 1, &quit))) break;
+      tc_fence_after();
+      if (q4 * 32 < rows) {
+#pragma unroll 1
+        for (int c = 0; c < t.units * UNIT; c += UNIT) {
+          uint32_t v[16];
+          __syncwarp();
+          tmem_ld16(tmem + ((uint32_t)(q4 * 32) << 16) + a * COLS + (uint32_t)c, v);
+          tmem_ld_wait();
+          float f[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(v[j]);
+          if (row_ok && t.row + c < p.N) finish_run<16>(p, y, yr, t.row + c, f);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty0 + 8 * a);
+      u += t.units;
+    }
+  }
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, 2 * COLS);
+  if (threadIdx.x == 0 && quit && p.err) atomicOr(p.err, WIDE_ERR_WAIT);
 }
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -445,6 +612,23 @@ int launch(const WideGemm& g, WideP p, int clusters, cudaStream_t st) {
   return check_launch("gemm_wide");
 }
 
+int launch_experts(const WideGemm& g, WideP p, int sms, cudaStream_t st) {
+  ExpertMaps maps;
+  const int box_rows = ceil_div(g.max_rows, 8) * 8;
+  p.a_bytes = (uint32_t)box_rows * BK * 2;
+  B200_TRY(make_map(&maps.x, g.x, g.x_rows, g.K, g.ldx, box_rows, true));
+  for (int n = 1; n <= TILE_UNITS; ++n) B200_TRY(make_map(&maps.w[n - 1], g.w, (long long)g.w_rows, g.K, g.K, n * UNIT, true));
+  p.stage_bytes = STAGE_KB * ((p.a_bytes + 1023) / 1024 * 1024 + TILE_UNITS * UNIT * BK * 2);
+  p.stages = std::min(EXPERT_ST, EXPERT_SMEM / (int)p.stage_bytes);
+  // the products read 128 rows of x from a stage, which run into what lies behind a smaller box: a tile's accumulator rows beyond it are not stored
+  p.bars_at = (uint32_t)p.stages * p.stage_bytes;
+  const size_t smem = p.bars_at + 1024 + 16 * EXPERT_ST + 64;
+  static std::atomic<uint64_t> limits{0};
+  B200_TRY(allow_smem(limits, EXPERT_SMEM + 1024 + 16 * EXPERT_ST + 64, gemm_expert_kernel));
+  B200_TRY(launch_early(gemm_expert_kernel, dim3((unsigned)sms), dim3(THREADS), smem, st, maps, p));
+  return check_launch("gemm_expert");
+}
+
 }  // namespace
 
 bool wide_supported(const WideGemm& g) {
@@ -470,6 +654,7 @@ int wide_gemm(const WideGemm& g, cudaStream_t st) {
   if (g.tile_e) {
     p.tile_e = g.tile_e; p.tile_r0 = g.tile_r0; p.tile_n = g.tile_n; p.n_tiles = g.n_tiles; p.y_rows = g.y_rows; p.e_rows = g.e_rows;
     p.mt = g.max_tiles; p.nt = ceil_div(g.N, 256); p.splits = 1; p.kb_per = p.num_kb;
+    if (g.max_rows > 0 && g.max_rows <= WIDE_EXPERT_ROWS) return launch_experts(g, p, sms, st);      // one tile per expert
     return launch<1, 256>(g, p, sms, st);
   }
   p.mt = ceil_div(g.M, 256);
