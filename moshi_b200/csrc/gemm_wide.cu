@@ -86,24 +86,42 @@ __device__ __forceinline__ void load_box(uint32_t dst, const CUtensorMap* map, u
   else
     tma_load_2d(dst, map, bar, c0, c1);
 }
-template <int CG>
-__device__ __forceinline__ void mma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  if constexpr (CG == 2)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-  else
-    umma_bf16(d, da, db, idesc, accumulate);
+__device__ __forceinline__ bool elected() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
+  return r != 0;
 }
+// low word of make_desc (tc_prims.cuh); the high word is the same for every operand
+constexpr uint32_t DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_low(uint32_t smem) { return ((smem & 0x3FFFFu) >> 4) | (1u << 16); }
+// the four products of a k-block, by one thread of the warp: rows at desc a, columns w_at 16-byte pieces behind them
+#define UMMA_BLOCK(GROUP)                                                                                                                              \
+  asm volatile(                                                                                                                                        \
+      "{\n\t.reg .pred p, t, q;\n\t.reg .b64 a0, a1, a2, a3, w0, w1, w2, w3;\n\t"                                                                     \
+      "mov.b64 a0, {%1, %11};\n\tmov.b64 a1, {%2, %11};\n\tmov.b64 a2, {%3, %11};\n\tmov.b64 a3, {%4, %11};\n\t"                                     \
+      "mov.b64 w0, {%5, %11};\n\tmov.b64 w1, {%6, %11};\n\tmov.b64 w2, {%7, %11};\n\tmov.b64 w3, {%8, %11};\n\t"                                     \
+      "setp.ne.b32 p, %10, 0;\n\tsetp.ne.b32 t, %11, 0;\n\telect.sync _|q, 0xffffffff;\n\t"                                                         \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a0, w0, %9, p;\n\t"                                                                         \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a1, w1, %9, t;\n\t"                                                                         \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a2, w2, %9, t;\n\t"                                                                         \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a3, w3, %9, t;\n\t}"                                                                        \
+      ::"r"(d), "r"(a), "r"(a + 2), "r"(a + 4), "r"(a + 6), "r"(w), "r"(w + 2), "r"(w + 4), "r"(w + 6), "r"(idesc), "r"(accumulate), "r"(DESC_HIGH) : "memory")
+template <int CG>
+__device__ __forceinline__ void umma_block(uint32_t d, uint32_t a, uint32_t w_at, uint32_t idesc, uint32_t accumulate) {
+  const uint32_t w = a + w_at;
+  if constexpr (CG == 2) UMMA_BLOCK("2");
+  else UMMA_BLOCK("1");
+}
+#undef UMMA_BLOCK
 template <int CG>
 __device__ __forceinline__ void commit(uint32_t bar) {                 // signals the barrier in both CTAs of a pair
   if constexpr (CG == 2) {
     const uint16_t both = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(both) : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"(both) : "memory");
   } else {
-    umma_commit(bar);
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
   }
 }
 template <int CG>
@@ -216,7 +234,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   const uint32_t stage_bytes = p.stage_bytes, a_stage = stage_bytes - B_STAGE;      // x rows first (at least the box), then weight rows
   const uint32_t bars = base + (uint32_t)p.stages * stage_bytes;
   const uint32_t full0 = bars, empty0 = bars + 8 * MAX_ST, tfull0 = bars + 16 * MAX_ST, tempty0 = tfull0 + 16, tptr = tempty0 + 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int rank = CG == 2 ? (int)(blockIdx.x & 1) : 0;
   const int first = blockIdx.x / CG, step = gridDim.x / CG;
   const bool grouped = p.tile_e != nullptr;
@@ -246,20 +264,22 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   const int mt = grouped ? p.n_tiles[0] : p.mt;
   const int tiles = mt * p.nt, units = tiles * p.splits;      // unit: a tile's sums over one range of k
 
+  // Both loops are walked by their whole warps, so that what the copies and products take is in uniform registers, and one thread issues.  (One thread alone: a prompt
+  // of 2048 tokens 1181 us, so 1131; 895 tokens scored 1271 and 1243.)
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      bool ok = true;
-      for (int u = first; ok && u < units; u += step) {
-        const int t = u % tiles, m = t % mt, n = t / mt;
-        const int kb0 = u / tiles * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
-        const int row0 = (grouped ? p.tile_r0[m] : m * 128 * CG) + rank * 128;
-        const int w0 = n * BN + rank * WROWS;           // first weight row (of the expert) of this CTA
-        const int wbase = grouped ? p.tile_e[m] * p.e_rows : 0;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!wait_or_quit(empty0 + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
+    int s = 0; uint32_t ph = 0;
+    bool ok = true;
+    for (int u = first; ok && u < units; u += step) {
+      const int t = u % tiles, m = t % mt, n = t / mt;
+      const int kb0 = u / tiles * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
+      const int row0 = (grouped ? p.tile_r0[m] : m * 128 * CG) + rank * 128;
+      const int w0 = n * BN + rank * WROWS;             // first weight row (of the expert) of this CTA
+      const int wbase = grouped ? p.tile_e[m] * p.e_rows : 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!wait_or_quit(empty0 + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
+        const uint32_t sa = base + (uint32_t)s * stage_bytes, bar = leader_addr<CG>(full0 + 8 * s);
+        if (elected()) {
           if (rank == 0) mbar_expect_tx(full0 + 8 * s, CG * (p.a_bytes + B_STAGE));
-          const uint32_t sa = base + (uint32_t)s * stage_bytes, bar = leader_addr<CG>(full0 + 8 * s);
           load_box<CG>(sa, &map_x, bar, kb * BK, row0);
 #pragma unroll
           for (int j = 0; j < WROWS / BOX; ++j) {
@@ -268,17 +288,18 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (p.packed) load_box<CG>(sa + a_stage + j * BOX * BK * 2, &map_w, bar, 0, ((w >> 7) * p.num_kb + kb) * 128 + (w & 127));
             else load_box<CG>(sa + a_stage + j * BOX * BK * 2, &map_w, bar, kb * BK, wbase + w);
           }
-          if (++s == p.stages) { s = 0; ph ^= 1u; }
         }
+        __syncwarp();
+        if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
-      if (!ok) {                                        // let copies in flight land before the block ends
-        const uint64_t t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 2000000ull) {}
-      }
+    }
+    if (!ok) {                                          // let copies in flight land before the block ends
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 2000000ull) {}
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc = make_idesc(128 * CG, BN);
       int s = 0; uint32_t ph = 0;
       bool ok = true;
@@ -290,10 +311,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!wait_or_quit(full0 + 8 * s, ph, &quit)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sa = base + (uint32_t)s * stage_bytes;
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            mma<CG>(d, make_desc(sa + k * 32), make_desc(sa + a_stage + k * 32), idesc, (kb > kb0 || k) ? 1u : 0u);
+          umma_block<CG>(d, desc_low(base + (uint32_t)s * stage_bytes), a_stage >> 4, idesc, kb > kb0 ? 1u : 0u);
           commit<CG>(empty0 + 8 * s);
           if (++s == p.stages) { s = 0; ph ^= 1u; }
         }
@@ -393,31 +411,6 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // 16 rows 157.1 / 118.1; 2048 x 4096, 2 experts 25.9 / 11.1 / 5.1, 10 34.3 / 31.0 / 25.6, 16 with 16 rows 48.6 / 49.8 / 41.0.
 // What bounded it on the way is how fast a thread asks and issues: a copy per unit and products from one thread 90 us for 10 experts of 8192 x 2048, both loops
 // walked by whole warps 60.8 (2048 x 4096: 60 and 37.3), one copy and two k-blocks per stage 62.2 and 31.0.
-__device__ __forceinline__ bool elected() {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
-  return r != 0;
-}
-__device__ __forceinline__ void commit_elected(uint32_t bar) {
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
-}
-// low word of make_desc (tc_prims.cuh); the high word is the same for every operand
-constexpr uint32_t DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t desc_low(uint32_t smem) { return ((smem & 0x3FFFFu) >> 4) | (1u << 16); }
-// the four products of a k-block, by one thread of the warp: rows at desc a, columns w_at 16-byte pieces behind them
-__device__ __forceinline__ void umma_bf16_block(uint32_t d, uint32_t a, uint32_t w_at, uint32_t idesc, uint32_t accumulate) {
-  const uint32_t w = a + w_at;
-  asm volatile(
-      "{\n\t.reg .pred p, t, q;\n\t.reg .b64 a0, a1, a2, a3, w0, w1, w2, w3;\n\t"
-      "mov.b64 a0, {%1, %11};\n\tmov.b64 a1, {%2, %11};\n\tmov.b64 a2, {%3, %11};\n\tmov.b64 a3, {%4, %11};\n\t"
-      "mov.b64 w0, {%5, %11};\n\tmov.b64 w1, {%6, %11};\n\tmov.b64 w2, {%7, %11};\n\tmov.b64 w3, {%8, %11};\n\t"
-      "setp.ne.b32 p, %10, 0;\n\tsetp.ne.b32 t, %11, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a0, w0, %9, p;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, w1, %9, t;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, w2, %9, t;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, w3, %9, t;\n\t}"
-      ::"r"(d), "r"(a), "r"(a + 2), "r"(a + 4), "r"(a + 6), "r"(w), "r"(w + 2), "r"(w + 4), "r"(w + 6), "r"(idesc), "r"(accumulate), "r"(DESC_HIGH) : "memory");
-}
 constexpr int EXPERT_SMEM = 216 * 1024;
 constexpr int UNIT = 16, TILE_UNITS = 8, EXPERT_ST = 6, STAGE_KB = 2;      // STAGE_KB: k-blocks per stage
 struct alignas(64) ExpertMaps { CUtensorMap x, w[TILE_UNITS]; };             // w[n - 1]: boxes of n units, so that a tile's rows come in one copy per k-block
@@ -508,11 +501,11 @@ gemm_expert_kernel(const __grid_constant__ ExpertMaps maps, const WideP p) {
         tc_fence_after();
         const uint32_t sa = desc_low(base + (uint32_t)s * stage_bytes);
 #pragma unroll
-        for (int j = 0; j < STAGE_KB; ++j) umma_bf16_block(d, sa + j * (x_bytes >> 4), (w_at + j * (COLS * BK * 2 - x_bytes)) >> 4, idesc, kb + j > 0 ? 1u : 0u);
-        commit_elected(empty0 + 8 * s);
+        for (int j = 0; j < STAGE_KB; ++j) umma_block<1>(d, sa + j * (x_bytes >> 4), (w_at + j * (COLS * BK * 2 - x_bytes)) >> 4, idesc, kb + j > 0 ? 1u : 0u);
+        commit<1>(empty0 + 8 * s);
         if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
-      if (ok) commit_elected(tfull0 + 8 * a);
+      if (ok) commit<1>(tfull0 + 8 * a);
       u += t.units;
     }
     __syncwarp();
