@@ -54,6 +54,8 @@ __device__ __forceinline__ bool wait_or_quit(uint32_t bar, uint32_t parity, vola
     }
   }
 }
+// the same for a whole warp: all of it goes on, or all of it gives up
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* quit) { return __all_sync(0xffffffffu, wait_or_quit(bar, parity, quit)); }
 #define FLASH_R32(r, o) "=r"((r)[o]), "=r"((r)[o + 1]), "=r"((r)[o + 2]), "=r"((r)[o + 3]), "=r"((r)[o + 4]), "=r"((r)[o + 5]), "=r"((r)[o + 6]), "=r"((r)[o + 7])
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
   asm volatile(
@@ -83,7 +85,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const uint32_t sq = base, sk = base + TILE, sv = sk + STAGES * TILE, sp = sv + STAGES * TILE, bars = sp + TILE;
   const uint32_t q_full = bars, k_full = bars + 8, k_empty = k_full + 8 * STAGES, v_full = k_empty + 8 * STAGES, v_empty = v_full + 8 * STAGES, s_full = v_empty + 8 * STAGES, s_free = s_full + 16,
                  p_full = s_free + 16, o_done = p_full + 8, tptr = o_done + 8;      // o_done: the sum over a tile is in O, its weights are free
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int qt = p.q_tiles - 1 - (int)blockIdx.x / p.H, h = (int)blockIdx.x % p.H;
   const int q0 = qt * ROWS, last_row = min(q0 + ROWS, p.T) - 1;
   const int n = (p.pos0 + last_row) / KEYS + 1;      // key tiles
@@ -106,63 +108,62 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   pdl_trigger();
   pdl_wait();
 
+  // both loops are walked by their whole warps, and one thread issues (tc_prims.cuh)
   if (warp == 0) {
-    if (lane == 0) {
-      auto load = [&](uint32_t dst, const CUtensorMap* m, uint32_t bar, int c, int r) {      // two halves along the inner dimension
+    auto load = [&](uint32_t dst, const CUtensorMap* m, uint32_t bar, int c, int r) {      // two halves along the inner dimension
+      if (elected()) {
+        mbar_expect_tx(bar, TILE);
         tma_load_2d(dst, m, bar, c, r);
         tma_load_2d(dst + HALF, m, bar, c + 64, r);
-      };
-      mbar_expect_tx(q_full, TILE);
-      load(sq, &map_q, q_full, h * FLASH_D, q0);
-      bool ok = true;
-      for (int i = 0; ok && i < n; ++i) {
-        const int s = i % STAGES;
-        const uint32_t use = (uint32_t)(i / STAGES);
-        // a stage's keys are free once its scores are there, its values once their sum is
-        if (!wait_or_quit(k_empty + 8 * s, (use & 1) ^ 1u, &quit)) { ok = false; break; }
-        mbar_expect_tx(k_full + 8 * s, TILE);
-        load(sk + s * TILE, &map_k, k_full + 8 * s, h * FLASH_D, i * KEYS);
-        if (!wait_or_quit(v_empty + 8 * s, (use & 1) ^ 1u, &quit)) { ok = false; break; }
-        mbar_expect_tx(v_full + 8 * s, TILE);
-        load(sv + s * TILE, &map_v, v_full + 8 * s, i * KEYS, h * FLASH_D);
       }
-      if (!ok) {                             // let copies in flight land before the block ends
-        const uint64_t t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 2000000ull) {}
-      }
+      __syncwarp();
+    };
+    load(sq, &map_q, q_full, h * FLASH_D, q0);
+    bool ok = true;
+    int s = 0; uint32_t ph = 0;
+    for (int i = 0; ok && i < n; ++i) {
+      // a stage's keys are free once its scores are there, its values once their sum is
+      if (!warp_wait(k_empty + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
+      load(sk + s * TILE, &map_k, k_full + 8 * s, h * FLASH_D, i * KEYS);
+      if (!warp_wait(v_empty + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
+      load(sv + s * TILE, &map_v, v_full + 8 * s, i * KEYS, h * FLASH_D);
+      if (++s == STAGES) { s = 0; ph ^= 1u; }
+    }
+    if (!ok) {                               // let copies in flight land before the block ends
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 2000000ull) {}
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(ROWS, 128);
-      auto product = [&](uint32_t d, uint32_t a, uint32_t b, bool add) {      // 128 x 128 x 128
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t off = (uint32_t)(k >> 2) * HALF + (uint32_t)(k & 3) * 32;
-          umma_bf16(d, make_desc(a + off), make_desc(b + off), idesc, add || k > 0 ? 1u : 0u);
-        }
-      };
-      auto scores = [&](int i) {
-        const int s = i % STAGES, b = i & 1;
-        if (!wait_or_quit(k_full + 8 * s, (uint32_t)(i / STAGES) & 1u, &quit)) return false;
-        if (!wait_or_quit(s_free + 8 * b, ((uint32_t)(i >> 1) & 1u) ^ 1u, &quit)) return false;
-        tc_fence_after();
-        product(tmem + b * 128, sq, sk + s * TILE, false);
-        umma_commit(k_empty + 8 * s);
-        umma_commit(s_full + 8 * b);
-        return true;
-      };
-      bool ok = wait_or_quit(q_full, 0, &quit) && scores(0);
-      for (int i = 0; ok && i < n; ++i) {
-        if (i + 1 < n) ok = scores(i + 1);
-        const int s = i % STAGES;
-        ok = ok && wait_or_quit(v_full + 8 * s, (uint32_t)(i / STAGES) & 1u, &quit) && wait_or_quit(p_full, (uint32_t)i & 1u, &quit);
-        if (!ok) break;
-        tc_fence_after();
-        product(tmem_o, sp, sv + s * TILE, i > 0);
-        umma_commit(v_empty + 8 * s);
-        umma_commit(o_done);
-      }
+    const uint32_t idesc = make_idesc(ROWS, 128);
+    auto product = [&](uint32_t d, uint32_t a, uint32_t b, bool add) {      // 128 x 128 x 128, in two halves of k
+      const uint32_t da = desc_low(a), to = desc_low(b) - da;
+      umma_block<1>(d, da, to, idesc, add ? 1u : 0u);
+      umma_block<1>(d, da + (HALF >> 4), to, idesc, 1u);
+    };
+    int ks = 0; uint32_t kph = 0;            // stage and phase of the next keys
+    auto scores = [&](int i) {
+      const int b = i & 1;
+      if (!warp_wait(k_full + 8 * ks, kph, &quit)) return false;
+      if (!warp_wait(s_free + 8 * b, ((uint32_t)(i >> 1) & 1u) ^ 1u, &quit)) return false;
+      tc_fence_after();
+      product(tmem + b * 128, sq, sk + ks * TILE, false);
+      commit_elected(k_empty + 8 * ks);
+      commit_elected(s_full + 8 * b);
+      if (++ks == STAGES) { ks = 0; kph ^= 1u; }
+      return true;
+    };
+    bool ok = warp_wait(q_full, 0, &quit) && scores(0);
+    int s = 0; uint32_t ph = 0;
+    for (int i = 0; ok && i < n; ++i) {
+      if (i + 1 < n) ok = scores(i + 1);
+      ok = ok && warp_wait(v_full + 8 * s, ph, &quit) && warp_wait(p_full, (uint32_t)i & 1u, &quit);
+      if (!ok) break;
+      tc_fence_after();
+      product(tmem_o, sp, sv + s * TILE, i > 0);
+      commit_elected(v_empty + 8 * s);
+      commit_elected(o_done);
+      if (++s == STAGES) { s = 0; ph ^= 1u; }
     }
     __syncwarp();
   } else {

@@ -1,22 +1,20 @@
 // tcgen05 GEMM for the LM linears at 33..256 sessions:  y[M][N] = epi(x[M][K] . w[N][K]^T), bf16 in, fp32 in TMEM, bf16 out.
 //
-// gemm_sk.cu feeds the 128-row weight tile as the UMMA *A* operand and the sessions as N ("swap-AB"): right while the batch is
-// tiny, but a tcgen05.mma with M = 128 occupies the tensor pipe for ~120-140 cycles whatever N <= 128 is (measured: the stream-K
-// kernel runs the same copy pipeline 1.8x slower with its MMAs switched on than with them off, and cuBLAS beats it on every LM
-// shape from 48 sessions up).  Here the operands keep their textbook roles:
+// gemm_sk.cu feeds the 128-row weight tile as the UMMA *A* operand and the sessions as N ("swap-AB").  Here the operands keep their textbook roles:
 //
 //   * A = the activations, one [128 sessions x 64 k] SWIZZLE_128B box per k-block (2-D TMA, rows beyond M zero-filled; two such
 //     blocks and two accumulators above 128 sessions);
 //   * B = TWO pre-tiled 128-row weight tiles side by side (N = 256 per instruction: twice the weight bytes per tensor-pipe
 //     cycle); for the gated MLP the pair is (gate rows, value rows) of the same outputs, already stored back to back, so the
 //     accumulator holds gate in columns 0..127 and value in 128..255 of the SAME thread and silu(g) * u needs no exchange;
-//   * D = [128 sessions (TMEM lanes) x 256 weight rows (columns)] fp32: an epilogue thread owns one session and writes 16
-//     consecutive outputs (32 bytes) per TMEM load.
-//   * shapes with fewer units than SMs are cut along K over a cluster of 2..4 CTAs (in_proj: 48 pairs x 2; out_proj / linear_out:
-//     32 single tiles x 4, N = 128 per instruction there so that 128 SMs pull on the weights); the partial accumulators are
-//     reduce-scattered over distributed shared memory by output columns (the stage ring is dead by then and serves as the
-//     receive buffer), summed in rank order (deterministic) and stored by the owning rank: no workspace, no atomics.
-//     ns_default_plan() holds the measured choice per shape.
+//   * D = [128 sessions (TMEM lanes) x 128 or 256 weight rows (columns)] fp32.  Results go through shared memory (the stage ring, empty by then), so that a warp stores and
+//     reads whole lines: 3 us less per launch than 32 bytes per session and instruction;
+//   * shapes with few units are cut along K over a cluster of 2..4 CTAs; every CTA adds the sums of all of them over distributed shared memory for its share of the
+//     sessions, in rank order (deterministic): no workspace, no atomics.  ns_default_plan() holds the measured choice per shape;
+//   * copies and products are issued from uniform registers (tc_prims.cuh).
+// us, one launch behind the other through the entry point with cold weights, before these three / now: 104 sessions 4096 -> 12288 28.8 / 22.1, 4096 -> 4096 16.8 / 13.8, 11264 ->
+// 4096 27.6 / 24.2, 4096 -> 32000 51.5 / 45.3, gated -> 11264 38.7 / 38.7; 33: 25.4 / 20.8, 13.5 / 9.8, 24.2 / 19.9, 48.7 / 42.8, 37.6 / 37.6; 256: 46 / 33.4, 30 / 26.6, 44 / 38, 70.5 / 60.8, 55.2 /
+// 54.7.  A step of the 7B with 40 sessions 6.83 -> 6.41 ms, with 72 7.56 -> 7.11.
 //
 // Same packed weights, same epilogues and cast points as gemm_sk.cu (residual add bf16(res + bf16(acc)), gated SiLU
 // bf16(bf16(silu(g)) * u), gating.py:18-20); same PDL protocol (weights requested before griddepcontrol.wait).
@@ -43,20 +41,29 @@ constexpr int MAX_STAGES = 8;
 constexpr int MAX_CS = 8;
 
 struct NsParams {
-  int M, N, K, out_rows, gate_rows, CS, num_kb, kb_per, stages, n_tiles, ldw, unit_tiles, mblocks;
+  int M, N, K, out_rows, gate_rows, CS, num_kb, kb_per, stages, n_tiles, unit_tiles, mblocks;
   const uint8_t* wt;
   __nv_bfloat16* y; long long ldy;
   const __nv_bfloat16* res; long long ldr;
   int late;                                      // nothing is read before the wait on the preceding kernel
 };
 
-__device__ __forceinline__ uint32_t ns_map_to_rank(uint32_t local_smem_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
-  return r;
+__device__ __forceinline__ float4 ns_lds_of(uint32_t at, int rank) {      // the same shared address in CTA `rank` of the cluster
+  float4 v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at), "r"(rank) : "memory");
+  return v;
 }
-__device__ __forceinline__ void ns_st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+__device__ __forceinline__ uint4 ns_lds(uint32_t at) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ void ns_sts(uint32_t at, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void ns_cluster_meet() {      // orders nothing
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void ns_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -64,36 +71,67 @@ __device__ __forceinline__ void ns_cluster_sync() {
 }
 __device__ __forceinline__ float ns_bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-// first accumulator column of rank q's share of `width` columns (multiples of 16; the last rank takes the remainder)
-__device__ __forceinline__ int col_begin(int width, int cs, int q) { return q >= cs ? width : ((width * q / cs) >> 4) << 4; }
-
-// 16 consecutive outputs of one session row -> y (two 16-byte stores)
-__device__ __forceinline__ void store16(__nv_bfloat16* dst, const float* v, int valid) {
-  if (valid >= 16) {
-    __nv_bfloat162 o[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-    uint4* d4 = reinterpret_cast<uint4*>(dst);
-    d4[0] = *reinterpret_cast<const uint4*>(&o[0]);
-    d4[1] = *reinterpret_cast<const uint4*>(&o[4]);
-  } else {
-    for (int j = 0; j < valid; ++j) dst[j] = __float2bfloat16_rn(v[j]);
-  }
+__device__ __forceinline__ uint32_t ns_pack(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
 }
-__device__ __forceinline__ void load16(const __nv_bfloat16* src, float* v, int valid) {
-  if (valid >= 16) {
-    const uint4* s4 = reinterpret_cast<const uint4*>(src);
-    const uint4 a = s4[0], b = s4[1];
-    const __nv_bfloat162* ha = reinterpret_cast<const __nv_bfloat162*>(&a);
-    const __nv_bfloat162* hb = reinterpret_cast<const __nv_bfloat162*>(&b);
+// Results and partial sums lie in shared memory as rows of 16-byte pieces, piece c of row r at position c ^ (r & 7): lanes write a row each, and read neighbouring pieces.
+__device__ __forceinline__ uint32_t ns_piece(uint32_t base, int row, int c, int per_row_log2) { return base + (uint32_t)(((row << per_row_log2) + (c ^ (row & 7))) << 4); }
+
+// eight neighbouring residuals of session m from output column o on (valid: how many exist)
+__device__ __forceinline__ uint4 ns_residual(const NsParams& p, int m, int o, int valid) {
+  const __nv_bfloat16* src = p.res + (long long)m * p.ldr + o;
+  if (valid >= 8) return *reinterpret_cast<const uint4*>(src);
+  uint32_t v[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = __bfloat1622float2(ha[j]), g = __bfloat1622float2(hb[j]);
-      v[2 * j] = f.x; v[2 * j + 1] = f.y; v[8 + 2 * j] = g.x; v[8 + 2 * j + 1] = g.y;
+  for (int j = 0; j < 8; ++j)
+    if (j < valid) v[j >> 1] |= (uint32_t)__bfloat16_as_ushort(src[j]) << (16 * (j & 1));
+  return make_uint4(v[0], v[1], v[2], v[3]);
+}
+// Session rows row, row + step, .. below end of a block (m0: its first session), a thread's eight columns from output column o on (piece c of a row).  The block's sums lie at
+// `sums`: in fp32 in every CTA of a cluster, added in rank order, or (CS == 1) rounded to bf16, what the epilogues do anyway.
+template <int EPI>
+__device__ __forceinline__ void ns_finish(const NsParams& p, uint32_t sums, int m0, int row, int end, int step, int c, int width_log2, int o, uint4 res) {
+  const int valid = p.out_rows - o;
+  if (valid <= 0) return;
+#pragma unroll 1
+  for (; row < end; row += step) {
+    const uint4 old = res;
+    if (EPI == EPI_RESADD && row + step < end) res = ns_residual(p, m0 + row + step, o, valid);
+    uint4 v;
+    if (EPI == EPI_GATE || p.CS == 1) {
+      v = ns_lds(ns_piece(sums, row, c, width_log2 - 3));
+    } else {
+      const uint32_t a0 = ns_piece(sums, row, 2 * c, width_log2 - 2), a1 = ns_piece(sums, row, 2 * c + 1, width_log2 - 2);
+      float4 x[MAX_CS], y[MAX_CS];
+#pragma unroll
+      for (int r = 0; r < MAX_CS; ++r)
+        if (r < p.CS) { x[r] = ns_lds_of(a0, r); y[r] = ns_lds_of(a1, r); }
+      float4 f = make_float4(0.f, 0.f, 0.f, 0.f), g = f;
+#pragma unroll
+      for (int r = 0; r < MAX_CS; ++r)
+        if (r < p.CS) { f.x += x[r].x; f.y += x[r].y; f.z += x[r].z; f.w += x[r].w; g.x += y[r].x; g.y += y[r].y; g.z += y[r].z; g.w += y[r].w; }
+      v = make_uint4(ns_pack(f.x, f.y), ns_pack(f.z, f.w), ns_pack(g.x, g.y), ns_pack(g.z, g.w));
     }
-  } else {
+    if (EPI == EPI_RESADD) {
+      const __nv_bfloat162 *a = reinterpret_cast<const __nv_bfloat162*>(&v), *b = reinterpret_cast<const __nv_bfloat162*>(&old);
+      uint4 w;
+      uint32_t* u = reinterpret_cast<uint32_t*>(&w);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = j < valid ? __bfloat162float(src[j]) : 0.f;
+      for (int j = 0; j < 4; ++j) {
+        const float2 s = __bfloat1622float2(a[j]), r = __bfloat1622float2(b[j]);
+        u[j] = ns_pack(r.x + s.x, r.y + s.y);
+      }
+      v = w;
+    }
+    __nv_bfloat16* dst = p.y + (long long)(m0 + row) * p.ldy + o;
+    if (valid >= 8) *reinterpret_cast<uint4*>(dst) = v;
+    else {
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < valid) dst[j] = __ushort_as_bfloat16((unsigned short)(u[j >> 1] >> (16 * (j & 1))));
+    }
   }
 }
 
@@ -110,9 +148,8 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
   const uint32_t full0 = bars, empty0 = bars + 8 * MAX_STAGES, tfull = bars + 16 * MAX_STAGES;
   const uint32_t tptr = tfull + 8;
   uint32_t* tptr_generic = reinterpret_cast<uint32_t*>(smem_raw + (tptr - raw));
-  const float* recv_generic = reinterpret_cast<const float*>(smem_raw + (base - raw));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int unit = blockIdx.x / p.CS, me = blockIdx.x - unit * p.CS;
   const int kb0 = me * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
   const int n_items = kb1 > kb0 ? kb1 - kb0 : 0;
@@ -139,162 +176,140 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
   if (p.late) pdl_wait();
   pdl_trigger();
 
+  // both loops are walked by their whole warps, and one thread issues (tc_prims.cuh)
   if (warp == 0) {
-    if (lane == 0) {
-      auto load_b = [&](int i, int s) {
-        const int kb = kb0 + i;
-        const uint32_t sb = base + (uint32_t)s * stage_bytes;
-        if (EPI == EPI_GATE) {
-          bulk_load(sb, p.wt + ((size_t)unit * p.num_kb + kb) * (2 * TILE_BYTES), 2 * TILE_BYTES, full0 + 8 * s);
-        } else {
-          bulk_load(sb, p.wt + ((size_t)tile0 * p.num_kb + kb) * TILE_BYTES, TILE_BYTES, full0 + 8 * s);
-          if (two) bulk_load(sb + TILE_BYTES, p.wt + ((size_t)(tile0 + 1) * p.num_kb + kb) * TILE_BYTES, TILE_BYTES, full0 + 8 * s);
-        }
-      };
-      // weights first (they do not depend on the preceding kernel), activations after the dependency wait
-      const int pre = n_items < p.stages ? n_items : p.stages;
-      for (int i = 0; i < pre; ++i) {
+    auto load_b = [&](int i, int s) {
+      const int kb = kb0 + i;
+      const uint32_t sb = base + (uint32_t)s * stage_bytes;
+      if (EPI == EPI_GATE) {
+        bulk_load(sb, p.wt + ((size_t)unit * p.num_kb + kb) * (2 * TILE_BYTES), 2 * TILE_BYTES, full0 + 8 * s);
+      } else {
+        bulk_load(sb, p.wt + ((size_t)tile0 * p.num_kb + kb) * TILE_BYTES, TILE_BYTES, full0 + 8 * s);
+        if (two) bulk_load(sb + TILE_BYTES, p.wt + ((size_t)(tile0 + 1) * p.num_kb + kb) * TILE_BYTES, TILE_BYTES, full0 + 8 * s);
+      }
+    };
+    // weights first (they do not depend on the preceding kernel), activations after the dependency wait
+    const int pre = n_items < p.stages ? n_items : p.stages;
+    for (int i = 0; i < pre; ++i) {
+      if (elected()) {
         mbar_expect_tx(full0 + 8 * i, b_bytes + a_bytes);
         load_b(i, i);
       }
-      pdl_wait();
-      int s = 0; uint32_t ph = 0;
-      for (int i = 0; i < n_items; ++i) {
+      __syncwarp();
+    }
+    pdl_wait();
+    int s = 0; uint32_t ph = 0;
+    for (int i = 0; i < n_items; ++i) {
+      if (i >= pre) mbar_wait(empty0 + 8 * s, ph ^ 1u);
+      if (elected()) {
         if (i >= pre) {
-          mbar_wait(empty0 + 8 * s, ph ^ 1u);
           mbar_expect_tx(full0 + 8 * s, b_bytes + a_bytes);
           load_b(i, s);
         }
         tma_load_2d(base + (uint32_t)s * stage_bytes + a_off, &tmap_x, full0 + 8 * s, (kb0 + i) * BLOCK_K, 0);
-        if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
+      __syncwarp();
+      if (++s == p.stages) { s = 0; ph ^= 1u; }
     }
-    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(128, width);
-      int s = 0; uint32_t ph = 0;
-      for (int i = 0; i < n_items; ++i) {
-        mbar_wait(full0 + 8 * s, ph);
-        tc_fence_after();
-        const uint32_t sb = base + (uint32_t)s * stage_bytes;
-        const uint32_t sa = sb + a_off;
-        for (int mb = 0; mb < p.mblocks; ++mb) {
-#pragma unroll
-          for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
-            umma_bf16(tmem_base + (uint32_t)(mb * 256), make_desc(sa + mb * A_BYTES + k * UMMA_K * 2), make_desc(sb + k * UMMA_K * 2), idesc,
-                      (i == 0 && k == 0) ? 0u : 1u);
-        }
-        umma_commit(empty0 + 8 * s);
-        if (++s == p.stages) { s = 0; ph ^= 1u; }
-      }
-      umma_commit(tfull);
+    const uint32_t idesc = make_idesc(128, width);
+    int s = 0; uint32_t ph = 0;
+    for (int i = 0; i < n_items; ++i) {
+      mbar_wait(full0 + 8 * s, ph);
+      tc_fence_after();
+      const uint32_t sb = desc_low(base + (uint32_t)s * stage_bytes), sa = sb + (a_off >> 4);
+      for (int mb = 0; mb < p.mblocks; ++mb)
+        umma_block<1>(tmem_base + (uint32_t)(mb * 256), sa + (uint32_t)mb * (A_BYTES >> 4), sb - (sa + (uint32_t)mb * (A_BYTES >> 4)), idesc, i == 0 ? 0u : 1u);
+      commit_elected(empty0 + 8 * s);
+      if (++s == p.stages) { s = 0; ph ^= 1u; }
     }
+    commit_elected(tfull);
     __syncwarp();
   }
 
-  const int q4 = warp & 3, run0 = ((warp - 2) >> 2) * 16;             // TMEM quadrant; first run of columns of an epilogue warp
-  const int my_c0 = col_begin(width, p.CS, me), my_c1 = col_begin(width, p.CS, me + 1);
-  if (warp >= 2) {
-    mbar_wait(tfull, 0);
-    tc_fence_after();
-  }
-  bool waited = false;
-  for (int mb = 0; mb < p.mblocks; ++mb) {      // blocks of 128 sessions: one accumulator each, the receive buffer is reused
-    const int m = mb * 128 + q4 * 32 + lane;    // session row of an epilogue thread (TMEM lane q4*32 + lane of accumulator mb)
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(mb * 256);
-    const bool m_ok = m < p.M;
-    if (p.CS > 1) {
-      ns_cluster_sync();                        // every rank's MMAs have retired / has read the previous block: the rings are free to receive
-      if (warp >= 2) {
-        for (int q = 0; q < p.CS; ++q) {
-          if (q == me) continue;
-          const int c0q = col_begin(width, p.CS, q), c1q = col_begin(width, p.CS, q + 1);
-          const int slot = me < q ? me : me - 1;
-          const uint32_t dst = ns_map_to_rank(base + (uint32_t)((slot * 128 + q4 * 32 + lane) * p.ldw) * 4u, (uint32_t)q);
-          for (int c = c0q + run0; c < c1q; c += EPI_STEP) {
-            uint32_t r[16];
-            if (n_items > 0) {
-              tmem_ld16(lane_addr + (uint32_t)c, r);
-              tmem_ld_wait();
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) r[j] = 0u;
-            }
-            if (m_ok) {
-#pragma unroll
-              for (int j = 0; j < 16; j += 4) ns_st_cluster_v4(dst + (uint32_t)(c - c0q + j) * 4u, r[j], r[j + 1], r[j + 2], r[j + 3]);
-            }
-          }
-        }
-        tc_fence_before();
-      }
-      ns_cluster_sync();                        // every partial has landed in its owner's receive buffer
-    }
+  // ===== epilogue: TMEM lane = session row.  Results go through the ring, which is empty by then, so that what is stored and read is whole lines =====
+  const int q4 = warp & 3, sub = (warp - 2) >> 2, qt = sub * 32 + lane, tid = threadIdx.x - 64;      // TMEM quadrant, this warp's place among its four
+  const int out_log2 = EPI == EPI_GATE || !two ? 7 : 8, out_width = 1 << out_log2, pieces = out_width >> 3;      // output columns of the unit, in pieces of eight
+  const int nb = tile0 * BLOCK_ROWS;
+  // CS == 1: a quadrant's 128 threads finish its 32 rows; else every CTA of the cluster its share of the block's rows, 512 threads
+  const int t = p.CS == 1 ? qt : tid, step = (p.CS == 1 ? 128 : 512) >> (out_log2 - 3), c = t & (pieces - 1), o = nb + c * 8;
+  for (int mb = 0; mb < p.mblocks; ++mb) {      // blocks of 128 sessions: one accumulator each
+    const int rows = min(128, p.M - mb * 128);
+    const int row0 = (p.CS == 1 ? q4 * 32 : rows * me / p.CS) + (t >> (out_log2 - 3)), end = p.CS == 1 ? min(rows, q4 * 32 + 32) : rows * (me + 1) / p.CS;
     if (warp >= 2) {
-      if (!waited) { pdl_wait(); waited = true; }   // y / res may still be in use by the predecessor
-      if (EPI == EPI_GATE) {
-        // columns j (gate) and 128 + j (value) of the same output; CS == 1 (the pair never needs a split: 88 units at 7B)
-        const int nb = unit * BLOCK_ROWS;
-        for (int c = run0; c < 128; c += EPI_STEP) {
-          uint32_t g[16], u[16];
-          tmem_ld16(lane_addr + (uint32_t)c, g);
-          tmem_ld16(lane_addr + (uint32_t)(128 + c), u);
-          tmem_ld_wait();
-          const int valid = p.out_rows - (nb + c);
-          if (m_ok && valid > 0) {
-            float v[16];
+      uint4 res = make_uint4(0u, 0u, 0u, 0u);
+      if (mb == 0) pdl_wait();                  // y / res may still be in use by the predecessor
+      if (EPI == EPI_RESADD && row0 < end && o < p.out_rows) res = ns_residual(p, mb * 128 + row0, o, p.out_rows - o);
+      if (mb == 0) {
+        mbar_wait(tfull, 0);
+        tc_fence_after();
+      }
+      const int row = q4 * 32 + lane;
+      const bool m_ok = row < rows;
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(mb * 256);
+#pragma unroll EPI == EPI_GATE ? 2 : 1
+      for (int c0 = sub * 16; c0 < (EPI == EPI_GATE ? 128 : out_width); c0 += EPI_STEP) {
+        float v[16];
+        if (n_items > 0) {
+          uint32_t g[16];
+          __syncwarp();
+          tmem_ld16(lane_addr + (uint32_t)c0, g);
+          if (EPI == EPI_GATE) {
+            // columns j (gate) and 128 + j (value) of the same output; CS == 1 (the pair never needs a split: 88 units at 7B)
+            uint32_t u[16];
+            tmem_ld16(lane_addr + (uint32_t)(128 + c0), u);
+            tmem_ld_wait();
+            if (m_ok) {                         // not for rows of zeroes: a division of zero takes the long way (33 to 104 rows: 41 us instead of 35)
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float gt = ns_bf16_round(__uint_as_float(g[j])), ut = ns_bf16_round(__uint_as_float(u[j]));
-              v[j] = ns_bf16_round(gt / (1.f + expf(-gt))) * ut;
+              for (int j = 0; j < 16; ++j) {
+                const float gt = ns_bf16_round(__uint_as_float(g[j])), ut = ns_bf16_round(__uint_as_float(u[j]));
+                v[j] = ns_bf16_round(gt / (1.f + expf(-gt))) * ut;
+              }
             }
-            store16(p.y + (long long)m * p.ldy + nb + c, v, valid);
+          } else {
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(g[j]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = 0.f;
+        }
+        if (m_ok) {
+          if (EPI == EPI_GATE || p.CS == 1) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              ns_sts(ns_piece(base, row, (c0 >> 3) + j, out_log2 - 3), make_uint4(ns_pack(v[8 * j], v[8 * j + 1]), ns_pack(v[8 * j + 2], v[8 * j + 3]), ns_pack(v[8 * j + 4], v[8 * j + 5]),
+                                                                                   ns_pack(v[8 * j + 6], v[8 * j + 7])));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              ns_sts(ns_piece(base, row, (c0 >> 2) + j, out_log2 - 2),
+                     make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3])));
           }
         }
+      }
+      if (EPI == EPI_GATE || p.CS == 1) {
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + q4) : "memory");
+        ns_finish<EPI>(p, base, mb * 128, row0, end, step, c, out_log2, o, res);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + q4) : "memory");
       } else {
-        const int nb = tile0 * BLOCK_ROWS;
-        for (int c = my_c0 + run0; c < my_c1; c += EPI_STEP) {
-          float acc[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-          const int valid = p.out_rows - (nb + c);
-          float rv[16];
-          if (EPI == EPI_RESADD && m_ok && valid > 0) load16(p.res + (long long)m * p.ldr + nb + c, rv, valid);
-          for (int r = 0; r < p.CS; ++r) {      // rank order: the sum does not depend on which rank does it
-            if (r == me) {
-              if (n_items > 0) {
-                uint32_t t[16];
-                tmem_ld16(lane_addr + (uint32_t)c, t);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; ++j) acc[j] += __uint_as_float(t[j]);
-              }
-            } else if (m_ok) {
-              const int slot = r < me ? r : r - 1;
-              const float4* src = reinterpret_cast<const float4*>(recv_generic + (size_t)(slot * 128 + q4 * 32 + lane) * p.ldw + (c - my_c0));
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float4 t = src[j];
-                acc[4 * j] += t.x; acc[4 * j + 1] += t.y; acc[4 * j + 2] += t.z; acc[4 * j + 3] += t.w;
-              }
-            }
-          }
-          if (m_ok && valid > 0) {
-            if (EPI == EPI_RESADD) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) acc[j] = rv[j] + ns_bf16_round(acc[j]);
-            }
-            store16(p.y + (long long)m * p.ldy + nb + c, acc, valid);
-          }
-        }
+        __syncwarp();
+        ns_cluster_sync();
+        ns_finish<EPI>(p, base, mb * 128, row0, end, step, c, out_log2, o, res);
       }
       tc_fence_before();
+    } else if (p.CS > 1) {
+      __syncwarp();
+      ns_cluster_sync();
+    }
+    if (p.CS > 1) {
+      __syncwarp();
+      ns_cluster_meet();                        // the block's sums have been read everywhere
     }
   }
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 256u * p.mblocks);
-  if (p.CS > 1) ns_cluster_sync();              // no CTA exits while a peer could still address its shared memory
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -330,20 +345,15 @@ bool ns_supported(int M, int N, int K, int epi) {
 
 int ns_prepare() { return ns_init(); }
 
-// The LM's choice of unit and K-split for a shape, from measurements on B200 at 48 / 104 sessions:
-//   * >= 40 pairs of tiles (in_proj 48, the gated MLP's input 88, the text head 125): N = 256 units, two K-splits while both CTAs
-//     of every unit are resident at once (in_proj: 96 CTAs), else one;
-//   * fewer (out_proj / linear_out: 32 tiles, depformer_in: 64): single-tile units (N = 128) so that more SMs pull on the
-//     weights, K cut over the largest power of two <= 4 that keeps the grid resident (32 x 4, 64 x 2 = 128 CTAs).
-// Wider clusters lose more to the receive traffic (~10 B/clk per SM over DSMEM) and to cluster placement than they gain.
+// The LM's choice of unit and K-split for a shape (us, one behind the other with cold weights through the entry point):
+//   * tiles for more than half the SMs, and no more than there are: one tile per CTA, K whole.  (4096 -> 12288, 96 tiles: pairs of tiles with K cut in two 28.5 us at 104
+//     sessions, 43.7 at 160, 49.2 at 256; so 25.4, 39.4 and 42.9.  The pairs read 48 KB per k-block and SM for 64 and exchange 128 columns.)
+//   * more (the gated MLP's input 88 pairs, the text head 250 tiles): pairs of tiles, N = 256, K whole (text head: 51.7, single tiles in two waves 55);
+//   * fewer (out_proj / linear_out: 32 tiles, depformer_in: 64): single tiles so that more SMs pull on the weights, K cut over the largest power of two <= 4
+//     that keeps the grid resident (32 x 4, 64 x 2 = 128 CTAs).
 static void ns_default_plan(int n_tiles, int num_kb, int epi, int* unit_tiles, int* cs) {
   if (epi == EPI_GATE) { *unit_tiles = 2; *cs = 1; return; }
-  const int pairs = (n_tiles + 1) / 2;
-  if (pairs >= 40) {
-    *unit_tiles = 2;
-    *cs = (2 * pairs <= g_ns_sms && num_kb >= 8) ? 2 : 1;
-    return;
-  }
+  if (n_tiles > g_ns_sms) { *unit_tiles = 2; *cs = 1; return; }
   *unit_tiles = 1;
   int c = 1;
   while (c < 4 && n_tiles * c * 2 <= g_ns_sms && num_kb / (c * 2) >= 4) c *= 2;
@@ -376,22 +386,12 @@ int ns_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   if (cs > p.num_kb) cs = p.num_kb;
   p.CS = cs;
   p.kb_per = (p.num_kb + cs - 1) / cs;
-  // receive buffer rows: the widest column share + 4, an odd number of 16-byte units (conflict-free float4 rows)
-  int wmax = 0;
-  for (int q = 0; q < cs; ++q) {
-    const int a = q >= cs ? 256 : ((256 * q / cs) >> 4) << 4, b = q + 1 >= cs ? 256 : ((256 * (q + 1) / cs) >> 4) << 4;
-    if (b - a > wmax) wmax = b - a;
-  }
-  p.ldw = wmax + 4;
-  if (((p.ldw / 4) & 1) == 0) p.ldw += 4;
   int stages = (200 * 1024) / (int)stage_bytes;
   if (stages > MAX_STAGES) stages = MAX_STAGES;
   if (stages > p.kb_per && p.kb_per >= 2) stages = p.kb_per;
   if (stages < 2) stages = 2;
-  const size_t recv_bytes = cs > 1 ? (size_t)(cs - 1) * 128 * p.ldw * 4 : 0;
-  while ((size_t)stages * stage_bytes < recv_bytes) ++stages;          // the ring doubles as the receive buffer
-  if (stages > MAX_STAGES || (size_t)stages * stage_bytes > 204 * 1024)
-    B200_FAIL(B200_ERR_SHAPE, "ns GEMM: the receive buffer of a %d-way split does not fit", cs);
+  const size_t sums = (size_t)128 * (p.unit_tiles == 2 && epi != EPI_GATE ? 256 : 128) * (cs > 1 ? 4 : 2);      // a block's results or partial sums, in the ring
+  while ((size_t)stages * stage_bytes < sums) ++stages;
   p.stages = stages;
   p.wt = static_cast<const uint8_t*>(w_tiles);
   p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr;

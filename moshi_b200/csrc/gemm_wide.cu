@@ -71,6 +71,9 @@ __device__ __forceinline__ bool wait_or_quit(uint32_t bar, uint32_t parity, vola
   }
 }
 
+// the same for a whole warp: all of it goes on, or all of it gives up
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* quit) { return __all_sync(0xffffffffu, wait_or_quit(bar, parity, quit)); }
+
 template <int CG>
 __device__ __forceinline__ uint32_t leader_addr(uint32_t local) {      // the same address in the first CTA of the pair
   if (CG == 1) return local;
@@ -86,33 +89,6 @@ __device__ __forceinline__ void load_box(uint32_t dst, const CUtensorMap* map, u
   else
     tma_load_2d(dst, map, bar, c0, c1);
 }
-__device__ __forceinline__ bool elected() {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
-  return r != 0;
-}
-// low word of make_desc (tc_prims.cuh); the high word is the same for every operand
-constexpr uint32_t DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t desc_low(uint32_t smem) { return ((smem & 0x3FFFFu) >> 4) | (1u << 16); }
-// the four products of a k-block, by one thread of the warp: rows at desc a, columns w_at 16-byte pieces behind them
-#define UMMA_BLOCK(GROUP)                                                                                                                              \
-  asm volatile(                                                                                                                                        \
-      "{\n\t.reg .pred p, t, q;\n\t.reg .b64 a0, a1, a2, a3, w0, w1, w2, w3;\n\t"                                                                     \
-      "mov.b64 a0, {%1, %11};\n\tmov.b64 a1, {%2, %11};\n\tmov.b64 a2, {%3, %11};\n\tmov.b64 a3, {%4, %11};\n\t"                                     \
-      "mov.b64 w0, {%5, %11};\n\tmov.b64 w1, {%6, %11};\n\tmov.b64 w2, {%7, %11};\n\tmov.b64 w3, {%8, %11};\n\t"                                     \
-      "setp.ne.b32 p, %10, 0;\n\tsetp.ne.b32 t, %11, 0;\n\telect.sync _|q, 0xffffffff;\n\t"                                                         \
-      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a0, w0, %9, p;\n\t"                                                                         \
-      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a1, w1, %9, t;\n\t"                                                                         \
-      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a2, w2, %9, t;\n\t"                                                                         \
-      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a3, w3, %9, t;\n\t}"                                                                        \
-      ::"r"(d), "r"(a), "r"(a + 2), "r"(a + 4), "r"(a + 6), "r"(w), "r"(w + 2), "r"(w + 4), "r"(w + 6), "r"(idesc), "r"(accumulate), "r"(DESC_HIGH) : "memory")
-template <int CG>
-__device__ __forceinline__ void umma_block(uint32_t d, uint32_t a, uint32_t w_at, uint32_t idesc, uint32_t accumulate) {
-  const uint32_t w = a + w_at;
-  if constexpr (CG == 2) UMMA_BLOCK("2");
-  else UMMA_BLOCK("1");
-}
-#undef UMMA_BLOCK
 template <int CG>
 __device__ __forceinline__ void commit(uint32_t bar) {                 // signals the barrier in both CTAs of a pair
   if constexpr (CG == 2) {
@@ -121,7 +97,7 @@ __device__ __forceinline__ void commit(uint32_t bar) {                 // signal
         "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"(both) : "memory");
   } else {
-    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
+    commit_elected(bar);
   }
 }
 template <int CG>
@@ -276,7 +252,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       const int w0 = n * BN + rank * WROWS;             // first weight row (of the expert) of this CTA
       const int wbase = grouped ? p.tile_e[m] * p.e_rows : 0;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!wait_or_quit(empty0 + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
+        if (!warp_wait(empty0 + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
         const uint32_t sa = base + (uint32_t)s * stage_bytes, bar = leader_addr<CG>(full0 + 8 * s);
         if (elected()) {
           if (rank == 0) mbar_expect_tx(full0 + 8 * s, CG * (p.a_bytes + B_STAGE));
@@ -306,10 +282,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       for (int u = first, it = 0; ok && u < units; u += step, ++it) {
         const uint32_t a = it & 1, d = tmem + a * BN;
         const int kb0 = u / tiles * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
-        if (!wait_or_quit(tempty0 + 8 * a, ((it >> 1) & 1) ^ 1u, &quit)) break;
+        if (!warp_wait(tempty0 + 8 * a, ((it >> 1) & 1) ^ 1u, &quit)) break;
         tc_fence_after();
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!wait_or_quit(full0 + 8 * s, ph, &quit)) { ok = false; break; }
+          if (!warp_wait(full0 + 8 * s, ph, &quit)) { ok = false; break; }
           tc_fence_after();
           umma_block<CG>(d, desc_low(base + (uint32_t)s * stage_bytes), a_stage >> 4, idesc, kb > kb0 ? 1u : 0u);
           commit<CG>(empty0 + 8 * s);
@@ -469,7 +445,7 @@ gemm_expert_kernel(const __grid_constant__ ExpertMaps maps, const WideP p) {
       const CUtensorMap* map_w = &maps.w[t.units - 1];
       for (int kb = 0; kb < p.num_kb; kb += STAGE_KB) {      // blocks beyond the last are zeroes
         const uint32_t bar = full0 + 8 * s, sa = base + (uint32_t)s * stage_bytes;
-        if (!wait_or_quit(empty0 + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
+        if (!warp_wait(empty0 + 8 * s, ph ^ 1u, &quit)) { ok = false; break; }
         if (elected()) {
           mbar_expect_tx(bar, bytes);
 #pragma unroll
@@ -494,10 +470,10 @@ gemm_expert_kernel(const __grid_constant__ ExpertMaps maps, const WideP p) {
     for (int u = u0; ok && u < u1; ++it) {
       const ExpertTile t = expert_tile(u, u1, per_expert);
       const uint32_t a = it & 1, d = tmem + a * COLS, idesc = make_idesc(128, t.units * UNIT);
-      if (!wait_or_quit(tempty0 + 8 * a, ((it >> 1) & 1) ^ 1u, &quit)) break;
+      if (!warp_wait(tempty0 + 8 * a, ((it >> 1) & 1) ^ 1u, &quit)) break;
       tc_fence_after();
       for (int kb = 0; kb < p.num_kb; kb += STAGE_KB) {
-        if (!wait_or_quit(full0 + 8 * s, ph, &quit)) { ok = false; break; }
+        if (!warp_wait(full0 + 8 * s, ph, &quit)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sa = desc_low(base + (uint32_t)s * stage_bytes);
 #pragma unroll

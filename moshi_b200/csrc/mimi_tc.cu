@@ -74,9 +74,6 @@ __device__ __forceinline__ void store_four(const TcParams& p, int b, int t, int 
   }
 }
 
-// The low word of make_desc (tc_prims.cuh); the high word is the same for every operand.
-constexpr uint32_t DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t desc_at(uint32_t smem) { return ((smem & 0x3FFFFu) >> 4) | (1u << 16); }
 // A step of 8 k with 3xTF32 parts, small terms first: lo * hi, hi * lo, hi * hi.  The whole warp calls, so that the operands are in uniform registers, and one
 // thread issues.  A k-block of four steps takes 0.35 us so with few columns; 0.58 where one thread alone walks the loop, 0.64 where it also makes whole
 // descriptors.
@@ -89,10 +86,6 @@ __device__ __forceinline__ void umma_tf32_split(uint32_t d, uint32_t m_hi, uint3
       "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], mh, nl, %5, t;\n\t"
       "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], mh, nh, %5, t;\n\t}"
       ::"r"(d), "r"(m_hi), "r"(m_lo), "r"(n_hi), "r"(n_lo), "r"(idesc), "r"(accumulate), "r"(DESC_HIGH) : "memory");
-}
-
-__device__ __forceinline__ void commit_elected(uint32_t bar) {
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ float4 lds_four(uint32_t at) {
@@ -240,7 +233,7 @@ mimi_tc_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant
         for (int kb = k0; kb < min(tl.kb1, k0 + TC_CHAIN); ++kb) {
           mbar_wait(full0 + 8 * s, ph);
           tc_fence_after();
-          const uint32_t sa = desc_at(base + (uint32_t)s * p.stage_bytes), sm = sa + m_at, sn = sa + n_at;
+          const uint32_t sa = desc_low(base + (uint32_t)s * p.stage_bytes), sm = sa + m_at, sn = sa + n_at;
 #pragma unroll
           for (int k = 0; k < TC_KB / 8; ++k)                // 8 tf32 = 32 bytes of K per step
             umma_tf32_split(d0, sm + 2 * k, sm + m_lo + 2 * k, sn + 2 * k, sn + n_lo + 2 * k, idesc, (kb == k0 && k == 0) ? 0u : 1u);
