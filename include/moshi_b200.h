@@ -573,7 +573,7 @@ int64_t b200_op_packed_bytes(int N, int K, int epi, int gate_rows);
 int b200_op_pack_tiles(const void* w_dev, void* out_dev, int N, int K, int epi, int gate_rows, void* stream);
 int b200_op_linear_sk(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N,
                       int K, int epi, int gate_rows, int grid, int smem_budget, int stream_only, void* stream);
-/* The LM's linear kernel for 33..256 sessions (csrc/gemm_ns.cu): activations as the UMMA A operand, two pre-tiled weight tiles
+/* The LM's linear kernel for 17..256 sessions (csrc/gemm_ns.cu): activations as the UMMA A operand, two pre-tiled weight tiles
  * as B (N = 256 per tcgen05.mma), K cut over a cluster of `cluster` CTAs and reduced over distributed shared memory
  * (0 = the LM's own choice; 100 + n = single-tile units, N = 128 per instruction, n K-splits); same packed weights and
  * epilogues as b200_op_linear_sk, any M <= 256.
@@ -581,8 +581,8 @@ int b200_op_linear_sk(const void* x_dev, const void* w_tiles_dev, void* y_dev, c
 int b200_op_linear_ns(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K,
                       int epi, int gate_rows, int cluster, void* stream);
 /* The kernel with the weights going through registers (csrc/gemm_reg.cu) at every shape that it has: up to 32 rows, gated pairs up to 16.
- * b200_op_linear_sk takes it where it is ahead: 17 to 32 rows where the tiles are no more than the SMs, and the gated pairs of fewer rows that
- * gemm_row.cu leaves. */
+ * b200_op_linear_sk takes it for the gated pairs of up to 16 rows that gemm_row.cu leaves, and for 17 to 32 rows that csrc/gemm_ns.cu cannot take
+ * (results off a 16-byte border) or while b200_op_set_gemv_max_rows has cut gemm_row.cu's range short. */
 int b200_op_linear_reg(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K, int epi, int gate_rows,
                        void* stream);
 /* The decoder LM's linear for more than 256 activation rows (csrc/gemm_wide.cu): y[M,N] = x[M,K] . w^T over packed tiles

@@ -1,20 +1,28 @@
-// tcgen05 GEMM for the LM linears at 33..256 sessions:  y[M][N] = epi(x[M][K] . w[N][K]^T), bf16 in, fp32 in TMEM, bf16 out.
+// tcgen05 GEMM for the LM linears at 17..256 sessions:  y[M][N] = epi(x[M][K] . w[N][K]^T), bf16 in, fp32 in TMEM, bf16 out; int8 in, exact int32 sums, scaled, bf16 out.
 //
 // gemm_sk.cu feeds the 128-row weight tile as the UMMA *A* operand and the sessions as N ("swap-AB").  Here the operands keep their textbook roles:
 //
-//   * A = the activations, one [128 sessions x 64 k] SWIZZLE_128B box per k-block (2-D TMA, rows beyond M zero-filled; two such
-//     blocks and two accumulators above 128 sessions);
+//   * A = the activations, one SWIZZLE_128B box of 128 bytes of k per k-block (2-D TMA; two blocks of rows above 128 sessions).  The box has as many rows as there are
+//     sessions, to whole eights: a row-wise copy costs about 2.7 ns per row and SM, zeroes too.  The instruction reads 128 rows all the same: what lies behind the box (the
+//     next stage's weights, free space behind the last) goes into rows of the accumulator that nobody reads.  The stages that this leaves room for are in flight instead;
 //   * B = TWO pre-tiled 128-row weight tiles side by side (N = 256 per instruction: twice the weight bytes per tensor-pipe
 //     cycle); for the gated MLP the pair is (gate rows, value rows) of the same outputs, already stored back to back, so the
 //     accumulator holds gate in columns 0..127 and value in 128..255 of the SAME thread and silu(g) * u needs no exchange;
-//   * D = [128 sessions (TMEM lanes) x 128 or 256 weight rows (columns)] fp32.  Results go through shared memory (the stage ring, empty by then), so that a warp stores and
-//     reads whole lines: 3 us less per launch than 32 bytes per session and instruction;
+//   * D = [128 sessions (TMEM lanes) x 128 or 256 weight rows (columns)] fp32.  k-blocks go to the accumulators that fit into TMEM in turn (4 of single tiles, 2 of pairs; half
+//     above 128 sessions), which are added in fp32: the tensor cores cut off what a long chain's additions leave over.  Error of the sums alone (terms whose exact sum is 0, over
+//     the rms of a random sum of them), 24 rows, one accumulator / these / what took 17..32 rows before: 4096 -> 12288 2.0e-6 / 4.8e-7 / 6.6e-7, 4096 -> 4096 4.8e-7 / 1.3e-7
+//     / 2.4e-7, 11264 -> 4096 1.5e-6 / 3.4e-7 / 6.2e-7, 4096 -> 32000 2.0e-6 / 1.0e-6 / 1.7e-6.  The epilogue keeps its registers without a stack for it: a stack
+//     frame of a few words costs a launch 2 to 3 us.  int8 sums are exact: one accumulator;
+//   * results go through shared memory (the stage ring, empty by then), so that a warp stores and reads whole lines: 3 us less per launch than 32 bytes per session and
+//     instruction;
 //   * shapes with few units are cut along K over a cluster of 2..4 CTAs; every CTA adds the sums of all of them over distributed shared memory for its share of the
 //     sessions, in rank order (deterministic): no workspace, no atomics.  ns_default_plan() holds the measured choice per shape;
 //   * copies and products are issued from uniform registers (tc_prims.cuh).
-// us, one launch behind the other through the entry point with cold weights, before these three / now: 104 sessions 4096 -> 12288 28.8 / 22.1, 4096 -> 4096 16.8 / 13.8, 11264 ->
-// 4096 27.6 / 24.2, 4096 -> 32000 51.5 / 45.3, gated -> 11264 38.7 / 38.7; 33: 25.4 / 20.8, 13.5 / 9.8, 24.2 / 19.9, 48.7 / 42.8, 37.6 / 37.6; 256: 46 / 33.4, 30 / 26.6, 44 / 38, 70.5 / 60.8, 55.2 /
-// 54.7.  A step of the 7B with 40 sessions 6.83 -> 6.41 ms, with 72 7.56 -> 7.11.
+// us, one launch behind the other through the entry point with cold weights, before these / now.  104 sessions: 4096 -> 12288 27.9 / 20.5, 4096 -> 4096 16.1 / 13.1, 11264 -> 4096
+// 26.4 / 22.0, 4096 -> 32000 50.9 / 45.3, gated -> 11264 38.2 / 37.8.  48: 25.3 / 20.0, 13.5 / 10.7, 23.6 / 19.3, 48.5 / 44.0, 37.3 / 37.3.  256: 44.3 / 31.8, 27.5 / 21.8, 42.3 /
+// 34.3, 70.7 / 63.2, 54.8 / 54.5.  24 sessions (gemm_reg.cu, gemm_sk.cu / now): 28.0 / 19.9, 15.0 / 10.0, 28.0 / 18.4, 53.6 / 43.1, 48.8 / 36.6.  int8 (gemm_reg.cu, gemm_sk.cu /
+// now): 24 17.6 / 11.8, 11.3 / 7.4, 18.3 / 11.0, 34.3 / 24.5, 34.3 / 22.1; 104 26.5 / 12.1, 17.6 / 10.3, 23.2 / 14.4, 41.2 / 25.9, 40.6 / 22.7; 256 40.4 / 17.1, 57.3 / 18.1, 88.6 /
+// 23.9, 72.6 / 37.3, 69.9 / 33.7.  A step of the 7B with 24 sessions 7.29 -> 5.88 ms, with 40 6.81 -> 6.32, with 72 7.56 -> 7.22.
 //
 // Same packed weights, same epilogues and cast points as gemm_sk.cu (residual add bf16(res + bf16(acc)), gated SiLU
 // bf16(bf16(silu(g)) * u), gating.py:18-20); same PDL protocol (weights requested before griddepcontrol.wait).
@@ -36,15 +44,17 @@ constexpr int BLOCK_ROWS = 128, BLOCK_K = 64, UMMA_K = 16;
 constexpr int NUM_THREADS = 576;
 constexpr int EPI_STEP = 64;                 // columns between the runs of one epilogue warp
 constexpr int TILE_BYTES = BLOCK_ROWS * BLOCK_K * 2;
-constexpr int A_BYTES = 128 * BLOCK_K * 2;   // one activation box: 128 session rows x 64 k
-constexpr int MAX_STAGES = 8;
+constexpr int A_BYTES = 128 * BLOCK_K * 2;   // a block of 128 session rows x 128 bytes of k
+constexpr int MAX_STAGES = 12;
 constexpr int MAX_CS = 8;
+constexpr int TMEM_COLS = 512;               // all of it: one CTA per SM
 
 struct NsParams {
-  int M, N, K, out_rows, gate_rows, CS, num_kb, kb_per, stages, n_tiles, unit_tiles, mblocks;
+  int M, N, K, out_rows, gate_rows, CS, num_kb, kb_per, stages, n_tiles, unit_tiles, mblocks, n_acc, box_rows;
   const uint8_t* wt;
   __nv_bfloat16* y; long long ldy;
   const __nv_bfloat16* res; long long ldr;
+  const float *sa, *sw;                          // int8: scales of activation and weight rows
   int late;                                      // nothing is read before the wait on the preceding kernel
 };
 
@@ -58,6 +68,10 @@ __device__ __forceinline__ uint4 ns_lds(uint32_t at) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
   return v;
+}
+__device__ __forceinline__ float4 ns_lds_f4(uint32_t at) {
+  const uint4 v = ns_lds(at);
+  return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
 }
 __device__ __forceinline__ void ns_sts(uint32_t at, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
@@ -78,6 +92,42 @@ __device__ __forceinline__ uint32_t ns_pack(float a, float b) {
 // Results and partial sums lie in shared memory as rows of 16-byte pieces, piece c of row r at position c ^ (r & 7): lanes write a row each, and read neighbouring pieces.
 __device__ __forceinline__ uint32_t ns_piece(uint32_t base, int row, int c, int per_row_log2) { return base + (uint32_t)(((row << per_row_log2) + (c ^ (row & 7))) << 4); }
 
+// sixteen columns' sums over the accumulators, which lie `cols` columns apart (whole warps); int8: one accumulator of whole numbers
+template <int MOST>
+__device__ __forceinline__ void ns_sums(uint32_t at, uint32_t cols, int n_acc, float (&v)[16]) {
+  uint32_t g[16], h[16];
+  tmem_ld16(at, g);
+  if (MOST > 1 && n_acc > 1) tmem_ld16(at + cols, h);
+  tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = MOST > 1 && n_acc > 1 ? __uint_as_float(g[j]) + __uint_as_float(h[j]) : __uint_as_float(g[j]);
+  if (MOST > 2 && n_acc > 2) {
+    tmem_ld16(at + 2 * cols, g);
+    if (n_acc > 3) tmem_ld16(at + 3 * cols, h);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] += n_acc > 3 ? __uint_as_float(g[j]) + __uint_as_float(h[j]) : __uint_as_float(g[j]);
+  }
+}
+// int8: the value of a sum, scaled as everywhere else (gemm_sk.cu)
+__device__ __forceinline__ float ns_scaled(float bits, float sa, float sw) { return (float)__float_as_int(bits) * (sa * sw * (1.f / 16129.f)); }
+__device__ __forceinline__ float ns_lds1(uint32_t at) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ void ns_sts1(uint32_t at, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory"); }
+// one more rank's partial sums
+template <bool I8>
+__device__ __forceinline__ void ns_add(float4& f, const float4& x) {
+  if (I8) {
+    f.x = __int_as_float(__float_as_int(f.x) + __float_as_int(x.x)); f.y = __int_as_float(__float_as_int(f.y) + __float_as_int(x.y));
+    f.z = __int_as_float(__float_as_int(f.z) + __float_as_int(x.z)); f.w = __int_as_float(__float_as_int(f.w) + __float_as_int(x.w));
+  } else {
+    f.x += x.x; f.y += x.y; f.z += x.z; f.w += x.w;
+  }
+}
+
 // eight neighbouring residuals of session m from output column o on (valid: how many exist)
 __device__ __forceinline__ uint4 ns_residual(const NsParams& p, int m, int o, int valid) {
   const __nv_bfloat16* src = p.res + (long long)m * p.ldr + o;
@@ -90,8 +140,8 @@ __device__ __forceinline__ uint4 ns_residual(const NsParams& p, int m, int o, in
 }
 // Session rows row, row + step, .. below end of a block (m0: its first session), a thread's eight columns from output column o on (piece c of a row).  The block's sums lie at
 // `sums`: in fp32 in every CTA of a cluster, added in rank order, or (CS == 1) rounded to bf16, what the epilogues do anyway.
-template <int EPI>
-__device__ __forceinline__ void ns_finish(const NsParams& p, uint32_t sums, int m0, int row, int end, int step, int c, int width_log2, int o, uint4 res) {
+template <int EPI, bool I8>
+__device__ __forceinline__ void ns_finish(const NsParams& p, uint32_t sums, uint32_t sa, uint32_t sw, int m0, int row, int end, int step, int c, int width_log2, int o, uint4 res) {
   const int valid = p.out_rows - o;
   if (valid <= 0) return;
 #pragma unroll 1
@@ -103,14 +153,23 @@ __device__ __forceinline__ void ns_finish(const NsParams& p, uint32_t sums, int 
       v = ns_lds(ns_piece(sums, row, c, width_log2 - 3));
     } else {
       const uint32_t a0 = ns_piece(sums, row, 2 * c, width_log2 - 2), a1 = ns_piece(sums, row, 2 * c + 1, width_log2 - 2);
-      float4 x[MAX_CS], y[MAX_CS];
-#pragma unroll
-      for (int r = 0; r < MAX_CS; ++r)
-        if (r < p.CS) { x[r] = ns_lds_of(a0, r); y[r] = ns_lds_of(a1, r); }
       float4 f = make_float4(0.f, 0.f, 0.f, 0.f), g = f;
+#pragma unroll 1
+      for (int r0 = 0; r0 < p.CS; r0 += 4) {     // four ranks' sums under way: eight were more than the registers hold
+        float4 x[4], y[4];
 #pragma unroll
-      for (int r = 0; r < MAX_CS; ++r)
-        if (r < p.CS) { f.x += x[r].x; f.y += x[r].y; f.z += x[r].z; f.w += x[r].w; g.x += y[r].x; g.y += y[r].y; g.z += y[r].z; g.w += y[r].w; }
+        for (int r = 0; r < 4; ++r)
+          if (r0 + r < p.CS) { x[r] = ns_lds_of(a0, r0 + r); y[r] = ns_lds_of(a1, r0 + r); }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (r0 + r < p.CS) { ns_add<I8>(f, x[r]); ns_add<I8>(g, y[r]); }
+      }
+      if (I8) {
+        const float m = ns_lds1(sa + 4u * (uint32_t)(m0 + row));
+        const float4 u = ns_lds_f4(sw + 32u * (uint32_t)c), w = ns_lds_f4(sw + 32u * (uint32_t)c + 16u);
+        f = make_float4(ns_scaled(f.x, m, u.x), ns_scaled(f.y, m, u.y), ns_scaled(f.z, m, u.z), ns_scaled(f.w, m, u.w));
+        g = make_float4(ns_scaled(g.x, m, w.x), ns_scaled(g.y, m, w.y), ns_scaled(g.z, m, w.z), ns_scaled(g.w, m, w.w));
+      }
       v = make_uint4(ns_pack(f.x, f.y), ns_pack(f.z, f.w), ns_pack(g.x, g.y), ns_pack(g.z, g.w));
     }
     if (EPI == EPI_RESADD) {
@@ -135,19 +194,20 @@ __device__ __forceinline__ void ns_finish(const NsParams& p, uint32_t sums, int 
   }
 }
 
-template <int EPI>
+template <int EPI, bool I8>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   const uint32_t a_off = (uint32_t)p.unit_tiles * TILE_BYTES;             // stage = B (one or two weight tiles) | A (activation box)
-  const uint32_t a_bytes = (uint32_t)p.mblocks * A_BYTES;                // one or two blocks of 128 sessions (M <= 256)
+  const uint32_t a_bytes = (uint32_t)p.box_rows * 128u;                   // the rows that exist, to whole eights: what follows them is multiplied too, into rows that nobody reads
   const uint32_t stage_bytes = a_off + a_bytes;
-  const uint32_t bars = base + (uint32_t)p.stages * stage_bytes;
+  const uint32_t bars = base + (uint32_t)p.stages * stage_bytes + ((uint32_t)p.mblocks * A_BYTES - a_bytes);      // the last stage's products read as far
   const uint32_t full0 = bars, empty0 = bars + 8 * MAX_STAGES, tfull = bars + 16 * MAX_STAGES;
   const uint32_t tptr = tfull + 8;
   uint32_t* tptr_generic = reinterpret_cast<uint32_t*>(smem_raw + (tptr - raw));
+  const uint32_t sa = bars + 16 * MAX_STAGES + 64, sw = sa + 4 * 256;      // int8: scales of the sessions and of the unit's weight rows
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int unit = blockIdx.x / p.CS, me = blockIdx.x - unit * p.CS;
@@ -157,6 +217,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
   const bool two = EPI == EPI_GATE || (p.unit_tiles == 2 && 2 * unit + 1 < p.n_tiles);
   const int tile0 = EPI == EPI_GATE ? unit : unit * p.unit_tiles;
   const int width = two ? 256 : 128;                                      // accumulator columns in use
+  const uint32_t acc_cols = 128u * p.unit_tiles;                          // and those that an accumulator is given: mblocks x n_acc x acc_cols = TMEM_COLS
   const uint32_t b_bytes = two ? 2u * TILE_BYTES : (uint32_t)TILE_BYTES;
 
   if (warp == 0 && lane == 0) {
@@ -168,7 +229,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
     mbar_init(tfull, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(tptr, 256u * p.mblocks);
+  if (warp == 1) tmem_alloc(tptr, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -206,21 +267,25 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
           mbar_expect_tx(full0 + 8 * s, b_bytes + a_bytes);
           load_b(i, s);
         }
-        tma_load_2d(base + (uint32_t)s * stage_bytes + a_off, &tmap_x, full0 + 8 * s, (kb0 + i) * BLOCK_K, 0);
+        tma_load_2d(base + (uint32_t)s * stage_bytes + a_off, &tmap_x, full0 + 8 * s, (kb0 + i) * (I8 ? 2 * BLOCK_K : BLOCK_K), 0);
       }
       __syncwarp();
       if (++s == p.stages) { s = 0; ph ^= 1u; }
     }
   } else if (warp == 1) {
-    const uint32_t idesc = make_idesc(128, width);
-    int s = 0; uint32_t ph = 0;
+    const uint32_t idesc = I8 ? make_idesc_i8(128, width) : make_idesc(128, width);
+    int s = 0, acc = 0; uint32_t ph = 0;
     for (int i = 0; i < n_items; ++i) {
       mbar_wait(full0 + 8 * s, ph);
       tc_fence_after();
-      const uint32_t sb = desc_low(base + (uint32_t)s * stage_bytes), sa = sb + (a_off >> 4);
-      for (int mb = 0; mb < p.mblocks; ++mb)
-        umma_block<1>(tmem_base + (uint32_t)(mb * 256), sa + (uint32_t)mb * (A_BYTES >> 4), sb - (sa + (uint32_t)mb * (A_BYTES >> 4)), idesc, i == 0 ? 0u : 1u);
+      const uint32_t sb = desc_low(base + (uint32_t)s * stage_bytes);
+      for (int mb = 0; mb < p.mblocks; ++mb) {
+        const uint32_t d = tmem_base + (uint32_t)(mb * p.n_acc + acc) * acc_cols, sa = sb + ((a_off + (uint32_t)mb * A_BYTES) >> 4), first = i < p.n_acc ? 0u : 1u;
+        if constexpr (I8) umma_block_i8(d, sa, sb - sa, idesc, first);
+        else umma_block<1>(d, sa, sb - sa, idesc, first);
+      }
       commit_elected(empty0 + 8 * s);
+      if (++acc == p.n_acc) acc = 0;
       if (++s == p.stages) { s = 0; ph ^= 1u; }
     }
     commit_elected(tfull);
@@ -233,7 +298,17 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
   const int nb = tile0 * BLOCK_ROWS;
   // CS == 1: a quadrant's 128 threads finish its 32 rows; else every CTA of the cluster its share of the block's rows, 512 threads
   const int t = p.CS == 1 ? qt : tid, step = (p.CS == 1 ? 128 : 512) >> (out_log2 - 3), c = t & (pieces - 1), o = nb + c * 8;
-  for (int mb = 0; mb < p.mblocks; ++mb) {      // blocks of 128 sessions: one accumulator each
+  const int n_acc = min(p.n_acc, n_items);
+  if (I8 && warp >= 2) {                        // scales: the weights' like the weights, the sessions' after the wait
+    if (tid < width) {
+      const int n = EPI == EPI_GATE ? (tid < 128 ? nb + tid : p.gate_rows + nb + tid - 128) : nb + tid;
+      ns_sts1(sw + 4u * (uint32_t)tid, (EPI == EPI_GATE ? nb + (tid & 127) : n) < p.out_rows ? p.sw[n] : 0.f);
+    }
+    pdl_wait();
+    if (tid < p.M) ns_sts1(sa + 4u * (uint32_t)tid, p.sa[tid]);
+    asm volatile("bar.sync 5, 512;" ::: "memory");
+  }
+  for (int mb = 0; mb < p.mblocks; ++mb) {      // blocks of 128 sessions
     const int rows = min(128, p.M - mb * 128);
     const int row0 = (p.CS == 1 ? q4 * 32 : rows * me / p.CS) + (t >> (out_log2 - 3)), end = p.CS == 1 ? min(rows, q4 * 32 + 32) : rows * (me + 1) / p.CS;
     if (warp >= 2) {
@@ -246,30 +321,32 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
       }
       const int row = q4 * 32 + lane;
       const bool m_ok = row < rows;
-      const uint32_t lane_addr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(mb * 256);
+      const float m_scale = I8 && m_ok ? ns_lds1(sa + 4u * (uint32_t)(mb * 128 + row)) : 0.f;
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(mb * p.n_acc) * acc_cols;
 #pragma unroll EPI == EPI_GATE ? 2 : 1
       for (int c0 = sub * 16; c0 < (EPI == EPI_GATE ? 128 : out_width); c0 += EPI_STEP) {
         float v[16];
         if (n_items > 0) {
-          uint32_t g[16];
           __syncwarp();
-          tmem_ld16(lane_addr + (uint32_t)c0, g);
+          ns_sums<I8 ? 1 : EPI == EPI_GATE ? 2 : 4>(lane_addr + (uint32_t)c0, acc_cols, n_acc, v);
           if (EPI == EPI_GATE) {
             // columns j (gate) and 128 + j (value) of the same output; CS == 1 (the pair never needs a split: 88 units at 7B)
-            uint32_t u[16];
-            tmem_ld16(lane_addr + (uint32_t)(128 + c0), u);
-            tmem_ld_wait();
+            float u[16];
+            ns_sums<I8 ? 1 : 2>(lane_addr + (uint32_t)(128 + c0), acc_cols, n_acc, u);
             if (m_ok) {                         // not for rows of zeroes: a division of zero takes the long way (33 to 104 rows: 41 us instead of 35)
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
-                const float gt = ns_bf16_round(__uint_as_float(g[j])), ut = ns_bf16_round(__uint_as_float(u[j]));
+                if (I8) {
+                  v[j] = ns_scaled(v[j], m_scale, ns_lds1(sw + 4u * (uint32_t)(c0 + j)));
+                  u[j] = ns_scaled(u[j], m_scale, ns_lds1(sw + 4u * (uint32_t)(128 + c0 + j)));
+                }
+                const float gt = ns_bf16_round(v[j]), ut = ns_bf16_round(u[j]);
                 v[j] = ns_bf16_round(gt / (1.f + expf(-gt))) * ut;
               }
             }
-          } else {
-            tmem_ld_wait();
+          } else if (I8 && p.CS == 1) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(g[j]);
+            for (int j = 0; j < 16; ++j) v[j] = ns_scaled(v[j], m_scale, ns_lds1(sw + 4u * (uint32_t)(c0 + j)));
           }
         } else {
 #pragma unroll
@@ -291,12 +368,12 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
       }
       if (EPI == EPI_GATE || p.CS == 1) {
         asm volatile("bar.sync %0, 128;" ::"r"(1 + q4) : "memory");
-        ns_finish<EPI>(p, base, mb * 128, row0, end, step, c, out_log2, o, res);
+        ns_finish<EPI, I8>(p, base, sa, sw, mb * 128, row0, end, step, c, out_log2, o, res);
         asm volatile("bar.sync %0, 128;" ::"r"(1 + q4) : "memory");
       } else {
         __syncwarp();
         ns_cluster_sync();
-        ns_finish<EPI>(p, base, mb * 128, row0, end, step, c, out_log2, o, res);
+        ns_finish<EPI, I8>(p, base, sa, sw, mb * 128, row0, end, step, c, out_log2, o, res);
       }
       tc_fence_before();
     } else if (p.CS > 1) {
@@ -309,7 +386,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
     }
   }
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, 256u * p.mblocks);
+  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -327,7 +404,8 @@ int ns_init() {
     g_ns_encode = reinterpret_cast<EncodeTiledFn>(fn);
   }
   static std::atomic<uint64_t> limits{0};
-  B200_TRY(allow_smem(limits, 220 * 1024, gemm_ns_kernel<EPI_STORE>, gemm_ns_kernel<EPI_RESADD>, gemm_ns_kernel<EPI_GATE>));
+  B200_TRY(allow_smem(limits, 220 * 1024, gemm_ns_kernel<EPI_STORE, false>, gemm_ns_kernel<EPI_RESADD, false>, gemm_ns_kernel<EPI_GATE, false>, gemm_ns_kernel<EPI_STORE, true>,
+                      gemm_ns_kernel<EPI_RESADD, true>, gemm_ns_kernel<EPI_GATE, true>));
   if (!g_ns_sms) {
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
@@ -347,7 +425,7 @@ int ns_prepare() { return ns_init(); }
 
 // The LM's choice of unit and K-split for a shape (us, one behind the other with cold weights through the entry point):
 //   * tiles for more than half the SMs, and no more than there are: one tile per CTA, K whole.  (4096 -> 12288, 96 tiles: pairs of tiles with K cut in two 28.5 us at 104
-//     sessions, 43.7 at 160, 49.2 at 256; so 25.4, 39.4 and 42.9.  The pairs read 48 KB per k-block and SM for 64 and exchange 128 columns.)
+//     sessions, 43.7 at 160, 49.2 at 256; so, with whole boxes and one accumulator, 25.4, 39.4 and 42.9.  The pairs read 48 KB per k-block and SM for 64 and exchange 128 columns.)
 //   * more (the gated MLP's input 88 pairs, the text head 250 tiles): pairs of tiles, N = 256, K whole (text head: 51.7, single tiles in two waves 55);
 //   * fewer (out_proj / linear_out: 32 tiles, depformer_in: 64): single tiles so that more SMs pull on the weights, K cut over the largest power of two <= 4
 //     that keeps the grid resident (32 x 4, 64 x 2 = 128 CTAs).
@@ -360,10 +438,12 @@ static void ns_default_plan(int n_tiles, int num_kb, int epi, int* unit_tiles, i
   *cs = c;
 }
 
-int ns_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const void* w_tiles, __nv_bfloat16* y, long long ldy,
+int ns_linear(GemmPlanCache& cache, const void* x, long long ldx, const void* w_tiles, __nv_bfloat16* y, long long ldy,
               const __nv_bfloat16* res, long long ldr, int M, int N, int K, int epi, int gate_rows, int cluster, int pdl,
-              cudaStream_t stream, int unit_tiles) {
-  if (!ns_supported(M, N, K, epi) || ldx % 8) B200_FAIL(B200_ERR_SHAPE, "ns GEMM: unsupported shape M=%d N=%d K=%d", M, N, K);
+              cudaStream_t stream, int unit_tiles, const float* sa, const float* sw) {
+  const bool i8 = sa != nullptr;
+  const int elem = i8 ? 1 : 2;
+  if (!ns_supported(M, N, K, epi) || ldx * elem % 16 || (i8 && K % 16)) B200_FAIL(B200_ERR_SHAPE, "ns GEMM: unsupported shape M=%d N=%d K=%d", M, N, K);
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_tiles) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(res)) & 15)
     B200_FAIL(B200_ERR_SHAPE, "ns GEMM: operands must be 16-byte aligned");
   if ((ldy % 8) || (res && ldr % 8)) B200_FAIL(B200_ERR_SHAPE, "ns GEMM: row strides must be multiples of 8");
@@ -372,13 +452,15 @@ int ns_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   p.M = M; p.N = N; p.K = K; p.gate_rows = gate_rows;
   p.out_rows = epi == EPI_GATE ? gate_rows : N;
   p.n_tiles = (p.out_rows + BLOCK_ROWS - 1) / BLOCK_ROWS;
-  p.num_kb = (K + BLOCK_K - 1) / BLOCK_K;
+  p.num_kb = (K * elem + 127) / 128;
   int def_ut = 2, def_cs = 1;
   ns_default_plan(p.n_tiles, p.num_kb, epi, &def_ut, &def_cs);
   if (unit_tiles == 0) unit_tiles = cluster > 0 ? 2 : def_ut;
   p.unit_tiles = (unit_tiles == 1 && epi != EPI_GATE) ? 1 : 2;
   p.mblocks = M > 128 ? 2 : 1;
-  const uint32_t stage_bytes = (uint32_t)p.unit_tiles * TILE_BYTES + (uint32_t)p.mblocks * A_BYTES;
+  p.n_acc = i8 ? 1 : TMEM_COLS / (p.mblocks * p.unit_tiles * 128);
+  p.box_rows = (M + 7) & ~7;
+  const uint32_t stage_bytes = (uint32_t)p.unit_tiles * TILE_BYTES + (uint32_t)p.box_rows * 128u, beyond = (uint32_t)p.mblocks * A_BYTES - (uint32_t)p.box_rows * 128u;
   const int n_units = (epi == EPI_GATE || p.unit_tiles == 1) ? p.n_tiles : (p.n_tiles + 1) / 2;
   int cs = cluster > 0 ? cluster : def_cs;
   if (epi == EPI_GATE) cs = 1;
@@ -386,7 +468,7 @@ int ns_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   if (cs > p.num_kb) cs = p.num_kb;
   p.CS = cs;
   p.kb_per = (p.num_kb + cs - 1) / cs;
-  int stages = (200 * 1024) / (int)stage_bytes;
+  int stages = (int)((208 * 1024 - beyond) / stage_bytes);
   if (stages > MAX_STAGES) stages = MAX_STAGES;
   if (stages > p.kb_per && p.kb_per >= 2) stages = p.kb_per;
   if (stages < 2) stages = 2;
@@ -396,22 +478,23 @@ int ns_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   p.wt = static_cast<const uint8_t*>(w_tiles);
   p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr;
   // activations x [M][K]: boxes of [128 rows x 64 k]; rows >= M are zero-filled by the TMA unit
-  PlanKey key{x, ldx, M, K, 128 * p.mblocks};
+  PlanKey key{x, ldx, M, K, p.box_rows + (i8 ? 1024 : 0)};
   auto it = cache.maps.find(key);
   if (it == cache.maps.end()) {
     CUtensorMap mp;
     cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    cuuint64_t strides[1] = {(cuuint64_t)ldx * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BLOCK_K, (cuuint32_t)(128 * p.mblocks)};
+    cuuint64_t strides[1] = {(cuuint64_t)ldx * elem};
+    cuuint32_t box[2] = {(cuuint32_t)(128 / elem), (cuuint32_t)p.box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = g_ns_encode(&mp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(x), dims, strides, box, estr,
+    CUresult r = g_ns_encode(&mp, i8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) B200_FAIL(B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) M=%d K=%d ld=%lld", (int)r, M, K, ldx);
     it = cache.maps.emplace(key, mp).first;
   }
   p.late = pdl != PDL_WEIGHTS_FIRST;
-  const size_t smem = (size_t)stages * stage_bytes + 1024 + 16 * MAX_STAGES + 64;
+  p.sa = sa; p.sw = sw;
+  const size_t smem = (size_t)stages * stage_bytes + beyond + 1024 + 16 * MAX_STAGES + 64 + (i8 ? 2048 : 0);
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(n_units * cs)); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
@@ -428,10 +511,10 @@ int ns_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
     ++na;
   }
   cfg.attrs = attr; cfg.numAttrs = na;
-  cudaError_t le;
-  if (epi == EPI_STORE) le = cudaLaunchKernelEx(&cfg, gemm_ns_kernel<EPI_STORE>, it->second, p);
-  else if (epi == EPI_RESADD) le = cudaLaunchKernelEx(&cfg, gemm_ns_kernel<EPI_RESADD>, it->second, p);
-  else le = cudaLaunchKernelEx(&cfg, gemm_ns_kernel<EPI_GATE>, it->second, p);
+  void (*kernel)(const CUtensorMap, const NsParams) =
+      i8 ? (epi == EPI_STORE ? gemm_ns_kernel<EPI_STORE, true> : epi == EPI_RESADD ? gemm_ns_kernel<EPI_RESADD, true> : gemm_ns_kernel<EPI_GATE, true>)
+         : (epi == EPI_STORE ? gemm_ns_kernel<EPI_STORE, false> : epi == EPI_RESADD ? gemm_ns_kernel<EPI_RESADD, false> : gemm_ns_kernel<EPI_GATE, false>);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, it->second, p);
   if (le != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "gemm_ns launch failed: %s", cudaGetErrorString(le));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return check_launch("gemm_ns");

@@ -9,8 +9,8 @@
 // tiles of a gated pair), eight warps a tile; DEPTH k-blocks of weights are in flight per thread and the first ones are requested before
 // the wait on the preceding kernel.  Where tiles are few, k is cut; the CTA that arrives last adds the ranges in order.
 //
-// Against the tcgen05 stream-K kernel of gemm_sk.cu: gated 4096 -> 11264, 6 rows 44.8 -> 33.3 us (185 MB of weights, 28 us at the measured copy rate);
-// int8 11264 -> 4096 with its quantisation, 24 rows 47.0 -> 24.0; a width-2048 decoder layer's linears at 8 rows 26 -> 18.6 us each.
+// Against the tcgen05 stream-K kernel of gemm_sk.cu: gated 4096 -> 11264, 6 rows 44.8 -> 33.3 us (185 MB of weights, 28 us at the measured copy rate); a width-2048 decoder
+// layer's linears at 8 rows 26 -> 18.6 us each.  From 17 rows on gemm_ns.cu is ahead (24 rows: 4096 -> 12288 28.0 us here, 19.9 there) and this one has what that cannot take.
 #include <algorithm>
 
 #include "gemm_reg.cuh"

@@ -1,5 +1,5 @@
 // Stream-K tcgen05 GEMM for the LM linears (see gemm_sk.cuh):  y[M][N] = epi(x[M][K] . w[N][K]^T), bf16 in,
-// fp32 accumulate in TMEM, bf16 out.  M = concurrent sessions (<= 256), so the kernel is a weight
+// fp32 accumulate in TMEM, bf16 out; for what the kernels that sk_linear() asks first leave.  M = concurrent sessions (<= 256), so the kernel is a weight
 // streamer: every weight byte crosses HBM -> SMEM exactly once and the whole chip pulls on it.
 //
 //   * Weights are repacked once at load into UMMA-ready tiles: [n_tile][k_block][A][128 rows x 64 k] bf16,
@@ -121,7 +121,7 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmap_x, const SkParams p) {
   const uint32_t tptr = tempty0 + 16;
   uint32_t* tptr_generic = reinterpret_cast<uint32_t*>(smem_raw + (tptr - raw));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   constexpr int A_TILES = EPI == EPI_GATE ? 2 : 1;
   constexpr uint32_t a_bytes = A_TILES * TILE_BYTES;
   const int c = blockIdx.x;
@@ -148,80 +148,74 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmap_x, const SkParams p) {
   if (p.late) pdl_wait();
   pdl_trigger();
 
+  // both loops are walked by their whole warps, and one thread issues (tc_prims.cuh)
   if (warp == 0) {
-    if (lane == 0) {
-      // ===== producer: one contiguous bulk copy of the weight tile(s) + one TMA box of activations per k-block =====
-      // Weights do not depend on the preceding kernel: the first `stages` weight tiles are requested before the
-      // dependency wait, so under programmatic dependent launch the HBM stream starts while the producer of x
-      // is still running.  The activation boxes (and everything the epilogue touches) come after pdl_wait.
-      int s = 0; uint32_t ph = 0;
-      int pre = 0;                                   // stages whose weight copy is already in flight
-      {
-        int ps = 0;
-        for (int si = 0; si < n_seg && pre < p.stages; ++si) {
-          const Seg sg = seg_get(p, c, n_sk, si);
-          const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
-          for (int kb = sg.kb0; kb < sg.kb1 && pre < p.stages; ++kb, src += a_bytes, ++pre, ++ps) {
-            mbar_expect_tx(full0 + 8 * ps, p.stage_bytes);
-            bulk_load(base + (uint32_t)ps * p.stage_bytes, src, a_bytes, full0 + 8 * ps);
-          }
+    // ===== producer: one contiguous bulk copy of the weight tile(s) + one TMA box of activations per k-block =====
+    // Weights do not depend on the preceding kernel: the first `stages` weight tiles are requested before the
+    // dependency wait, so under programmatic dependent launch the HBM stream starts while the producer of x
+    // is still running.  The activation boxes (and everything the epilogue touches) come after pdl_wait.
+    int s = 0; uint32_t ph = 0;
+    int pre = 0;                                     // stages whose weight copy is already in flight
+    for (int si = 0; si < n_seg && pre < p.stages; ++si) {
+      const Seg sg = seg_get(p, c, n_sk, si);
+      const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
+      for (int kb = sg.kb0; kb < sg.kb1 && pre < p.stages; ++kb, src += a_bytes, ++pre) {
+        if (elected()) {
+          mbar_expect_tx(full0 + 8 * pre, p.stage_bytes);
+          bulk_load(base + (uint32_t)pre * p.stage_bytes, src, a_bytes, full0 + 8 * pre);
         }
+        __syncwarp();
       }
-      pdl_wait();
-      int item = 0;
-      for (int si = 0; si < n_seg; ++si) {
-        const Seg sg = seg_get(p, c, n_sk, si);
-        const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb, src += a_bytes, ++item) {
-          const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
+    }
+    pdl_wait();
+    int item = 0;
+    for (int si = 0; si < n_seg; ++si) {
+      const Seg sg = seg_get(p, c, n_sk, si);
+      const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
+      for (int kb = sg.kb0; kb < sg.kb1; ++kb, src += a_bytes, ++item) {
+        const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
+        if (item >= pre) mbar_wait(empty0 + 8 * s, ph ^ 1u);
+        if (elected()) {
           if (item >= pre) {
-            mbar_wait(empty0 + 8 * s, ph ^ 1u);
             mbar_expect_tx(full0 + 8 * s, p.stage_bytes);
             bulk_load(sa, src, a_bytes, full0 + 8 * s);
           }
           tma_load_2d(sa + a_bytes, &tmap_x, full0 + 8 * s, kb * (p.i8 ? 2 * BLOCK_K : BLOCK_K), 0);   // 128 bytes of K either way
-          if (++s == p.stages) { s = 0; ph ^= 1u; }
         }
+        __syncwarp();
+        if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ===== MMA issuer =====
-      const uint32_t idesc = p.i8 ? make_idesc_i8(BLOCK_ROWS, p.Mpad) : make_idesc(BLOCK_ROWS, p.Mpad);
-      int s = 0; uint32_t ph = 0;
-      int acc = 0; uint32_t acc_bits = 0u;       // bit a = phase parity of accumulator stage a
-      for (int si = 0; si < n_seg; ++si) {
-        const Seg sg = seg_get(p, c, n_sk, si);
-        mbar_wait(tempty0 + 8 * acc, ((acc_bits >> acc) & 1u) ^ 1u);        // epilogue has drained this accumulator
+    // ===== MMA issuer =====
+    const uint32_t idesc = p.i8 ? make_idesc_i8(BLOCK_ROWS, p.Mpad) : make_idesc(BLOCK_ROWS, p.Mpad);
+    int s = 0; uint32_t ph = 0;
+    int acc = 0; uint32_t acc_bits = 0u;         // bit a = phase parity of accumulator stage a
+    for (int si = 0; si < n_seg; ++si) {
+      const Seg sg = seg_get(p, c, n_sk, si);
+      mbar_wait(tempty0 + 8 * acc, ((acc_bits >> acc) & 1u) ^ 1u);          // epilogue has drained this accumulator
+      tc_fence_after();
+      const uint32_t d0 = tmem_base + (uint32_t)(acc * p.acc_cols);
+      for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+        mbar_wait(full0 + 8 * s, ph);
         tc_fence_after();
-        const uint32_t d0 = tmem_base + (uint32_t)(acc * p.acc_cols);
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          mbar_wait(full0 + 8 * s, ph);
-          tc_fence_after();
-          if (!p.stream_only) {
-            const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
-            const uint32_t sb = sa + a_bytes;
-#pragma unroll
-            for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-              const uint64_t db = make_desc(sb + k * UMMA_K * 2);
-              const uint32_t accum = (kb == sg.kb0 && k == 0) ? 0u : 1u;
-              // one MMA consumes 32 bytes of K per row either way: 16 bf16 or 32 int8
-              if (p.i8) {
-                umma_i8(d0, make_desc(sa + k * UMMA_K * 2), db, idesc, accum);
-                if (EPI == EPI_GATE) umma_i8(d0 + (uint32_t)p.Mpad, make_desc(sa + TILE_BYTES + k * UMMA_K * 2), db, idesc, accum);
-              } else {
-                umma_bf16(d0, make_desc(sa + k * UMMA_K * 2), db, idesc, accum);
-                if (EPI == EPI_GATE) umma_bf16(d0 + (uint32_t)p.Mpad, make_desc(sa + TILE_BYTES + k * UMMA_K * 2), db, idesc, accum);
-              }
-            }
+        if (!p.stream_only) {
+          const uint32_t sa = desc_low(base + (uint32_t)s * p.stage_bytes), accum = kb == sg.kb0 ? 0u : 1u;
+          // one MMA consumes 32 bytes of K per row either way: 16 bf16 or 32 int8
+          if (p.i8) {
+            umma_block_i8(d0, sa, a_bytes >> 4, idesc, accum);
+            if (EPI == EPI_GATE) umma_block_i8(d0 + (uint32_t)p.Mpad, sa + (TILE_BYTES >> 4), (a_bytes - TILE_BYTES) >> 4, idesc, accum);
+          } else {
+            umma_block<1>(d0, sa, a_bytes >> 4, idesc, accum);
+            if (EPI == EPI_GATE) umma_block<1>(d0 + (uint32_t)p.Mpad, sa + (TILE_BYTES >> 4), (a_bytes - TILE_BYTES) >> 4, idesc, accum);
           }
-          umma_commit(empty0 + 8 * s);           // frees the smem stage once these MMAs have read it
-          if (++s == p.stages) { s = 0; ph ^= 1u; }
         }
-        umma_commit(tfull0 + 8 * acc);           // segment accumulated
-        acc_bits ^= 1u << acc;
-        if (p.n_acc == 2) acc ^= 1;
+        commit_elected(empty0 + 8 * s);          // frees the smem stage once these MMAs have read it
+        if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
+      commit_elected(tfull0 + 8 * acc);          // segment accumulated
+      acc_bits ^= 1u << acc;
+      if (p.n_acc == 2) acc ^= 1;
     }
     __syncwarp();
   } else {
@@ -402,7 +396,7 @@ gemm_ck_kernel(const __grid_constant__ CUtensorMap tmap_x, const CkParams p) {
   const uint32_t recv = (tptr + 8 + 15u) & ~15u;
   float* recv_generic = reinterpret_cast<float*>(smem_raw + (recv - raw));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int tile = blockIdx.x / p.CS, me = blockIdx.x - tile * p.CS;
   const int kb0 = me * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
 
@@ -423,49 +417,47 @@ gemm_ck_kernel(const __grid_constant__ CUtensorMap tmap_x, const CkParams p) {
   if (p.late) pdl_wait();
   pdl_trigger();
 
+  // both loops are walked by their whole warps, and one thread issues (tc_prims.cuh)
   if (warp == 0) {
-    if (lane == 0) {
-      // weights first (they do not depend on the preceding kernel), activations after the dependency wait
-      const uint8_t* src = p.wt + ((size_t)tile * p.num_kb + kb0) * TILE_BYTES;
-      const int n_items = kb1 - kb0;
-      const int pre = n_items < p.stages ? n_items : p.stages;
-      for (int i = 0; i < pre; ++i) {
+    // weights first (they do not depend on the preceding kernel), activations after the dependency wait
+    const uint8_t* src = p.wt + ((size_t)tile * p.num_kb + kb0) * TILE_BYTES;
+    const int n_items = kb1 - kb0;
+    const int pre = n_items < p.stages ? n_items : p.stages;
+    for (int i = 0; i < pre; ++i) {
+      if (elected()) {
         mbar_expect_tx(full0 + 8 * i, p.stage_bytes);
         bulk_load(base + (uint32_t)i * p.stage_bytes, src + (size_t)i * TILE_BYTES, TILE_BYTES, full0 + 8 * i);
       }
-      pdl_wait();
-      int s = 0; uint32_t ph = 0;
-      for (int i = 0; i < n_items; ++i) {
-        const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
+      __syncwarp();
+    }
+    pdl_wait();
+    int s = 0; uint32_t ph = 0;
+    for (int i = 0; i < n_items; ++i) {
+      const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
+      if (i >= pre) mbar_wait(empty0 + 8 * s, ph ^ 1u);
+      if (elected()) {
         if (i >= pre) {
-          mbar_wait(empty0 + 8 * s, ph ^ 1u);
           mbar_expect_tx(full0 + 8 * s, p.stage_bytes);
           bulk_load(sa, src + (size_t)i * TILE_BYTES, TILE_BYTES, full0 + 8 * s);
         }
         tma_load_2d(sa + TILE_BYTES, &tmap_x, full0 + 8 * s, (kb0 + i) * (p.i8 ? 2 * BLOCK_K : BLOCK_K), 0);
-        if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
+      __syncwarp();
+      if (++s == p.stages) { s = 0; ph ^= 1u; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = p.i8 ? make_idesc_i8(BLOCK_ROWS, p.Mpad) : make_idesc(BLOCK_ROWS, p.Mpad);
-      int s = 0; uint32_t ph = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        mbar_wait(full0 + 8 * s, ph);
-        tc_fence_after();
-        const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
-        const uint32_t sb = sa + TILE_BYTES;
-#pragma unroll
-        for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-          const uint32_t accum = (kb == kb0 && k == 0) ? 0u : 1u;
-          if (p.i8) umma_i8(tmem_base, make_desc(sa + k * UMMA_K * 2), make_desc(sb + k * UMMA_K * 2), idesc, accum);
-          else umma_bf16(tmem_base, make_desc(sa + k * UMMA_K * 2), make_desc(sb + k * UMMA_K * 2), idesc, accum);
-        }
-        umma_commit(empty0 + 8 * s);
-        if (++s == p.stages) { s = 0; ph ^= 1u; }
-      }
-      umma_commit(tfull);
+    const uint32_t idesc = p.i8 ? make_idesc_i8(BLOCK_ROWS, p.Mpad) : make_idesc(BLOCK_ROWS, p.Mpad);
+    int s = 0; uint32_t ph = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      mbar_wait(full0 + 8 * s, ph);
+      tc_fence_after();
+      const uint32_t sa = desc_low(base + (uint32_t)s * p.stage_bytes), accum = kb == kb0 ? 0u : 1u;
+      if (p.i8) umma_block_i8(tmem_base, sa, TILE_BYTES >> 4, idesc, accum);
+      else umma_block<1>(tmem_base, sa, TILE_BYTES >> 4, idesc, accum);
+      commit_elected(empty0 + 8 * s);
+      if (++s == p.stages) { s = 0; ph ^= 1u; }
     }
+    commit_elected(tfull);
     __syncwarp();
   }
   float own[64];                               // this rank's column block of its own accumulator (Wc <= 64)
@@ -871,14 +863,18 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   const bool scaled = !i8 || (K % 16 == 0 && tune.sa && tune.sw);
   if (chosen && scaled && M <= g_row_max_m && row_wins(M, epi, gate_rows, i8, g_sms) && row_supported(M, K, i8, rows, row_ld))
     return row_linear(rows, row_ld, w_tiles, y, ldy, res, ldr, M, N, K, epi, gate_rows, i8 ? tune.sa : nullptr, tune.sw, g_sms, tune.pdl, stream);
-  // up to 32 sessions: weights through registers (gemm_reg.cu)
-  if (chosen && scaled && M <= REG_MAX_M && reg_wins(M, N, epi, gate_rows, i8, g_sms) && reg_supported(M, epi, rows, row_ld))
+  // 17..256 sessions: activations as the A operand (gemm_ns.cu, figures there: ahead at every shape from 17 rows on).  It stores 16-byte pieces; rows that do not lie so keep
+  // the kernels below, and (bf16) its refusal above 32
+  const bool lines = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(rows)) & 15) == 0;
+  const bool ns_fits = scaled && tune.ns >= 0 && M <= 256 && tune.grid == 0 && tune.cluster == 0 && !tune.stream_only && !tune.force_split && ns_supported(M, N, K, epi) &&
+                       ldy % 8 == 0 && (!res || ldr % 8 == 0) && ((!i8 && M > REG_MAX_M) || (lines && (chosen || tune.ns > 0)));
+  // up to 32 that the row kernel and that one leave: weights through registers (gemm_reg.cu).  With the row kernel's range cut short this one has all of its own.
+  if (chosen && scaled && M <= REG_MAX_M && !(ns_fits && g_use_ns && M > ROW_MAX_M && g_row_max_m == ROW_MAX_M) && reg_wins(M, N, epi, gate_rows, i8, g_sms) &&
+      reg_supported(M, epi, rows, row_ld))
     return reg_linear(rows, row_ld, w_tiles, y, ldy, res, ldr, M, N, K, epi, gate_rows, i8 ? tune.sa : nullptr, tune.sw, ws, sk_workspace_bytes(M), counters,
                       SK_MAX_TILES, g_sms, tune.pdl, stream);
-  // 33..256 sessions: activations as the A operand, two weight tiles (N = 256) per tcgen05.mma (gemm_ns.cu)
-  if (!i8 && tune.ns >= 0 && (tune.ns > 0 || (g_use_ns && M > 32)) && M <= 256 && tune.grid == 0 && tune.cluster == 0 && !tune.stream_only &&
-      !tune.force_split && ns_supported(M, N, K, epi) && ldy % 8 == 0 && (!res || ldr % 8 == 0))
-    return ns_linear(cache, x, ldx, w_tiles, y, ldy, res, ldr, M, N, K, epi, gate_rows, 0, tune.pdl, stream);
+  if (ns_fits && (tune.ns > 0 || (g_use_ns && M > ROW_MAX_M)))
+    return ns_linear(cache, rows, i8 ? K : ldx, w_tiles, y, ldy, res, ldr, M, N, K, epi, gate_rows, 0, tune.pdl, stream, 0, i8 ? tune.sa : nullptr, i8 ? tune.sw : nullptr);
   // more than 32 sessions and few row tiles: a cluster of CTAs per tile, split along K, reduced over DSMEM
   if (i8 && (K % 16 || !tune.sa || !tune.sw)) B200_FAIL(B200_ERR_SHAPE, "int8 GEMM: K must be a multiple of 16 and both scale vectors given");
   if (epi != EPI_GATE && tune.no_cluster == 0 && tune.grid == 0 && M > 32) {

@@ -50,7 +50,7 @@ struct SkTuning {
   // int8 path (QLinear): row-wise absmax int8 activations [M][K] + their scales, and the weight-row scales [N]
   const void* xq = nullptr; const float* sa = nullptr; const float* sw = nullptr;
   int pdl = 0;           // early launch (programmatic stream serialization): PDL_* above
-  int ns = 0;            // 33..256 sessions: 0 = the non-swapped kernel (gemm_ns.cu) unless B200_GEMM_NS=0, -1 = never, 1 = always (tests)
+  int ns = 0;            // 17..256 sessions: 0 = the non-swapped kernel (gemm_ns.cu) unless B200_GEMM_NS=0, -1 = never, 1 = always (tests)
 };
 int sk_num_sms();
 int sk_set_row_max_m(int max_m);       // rows up to which gemm_row.cu is considered (0..16); returns the previous value
@@ -71,14 +71,15 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
               long long ldy, const __nv_bfloat16* res, long long ldr, int M, int N, int K, int epi, int gate_rows,
               float* ws, int* counters, const SkTuning& tune, cudaStream_t stream);
 
-// ---- non-swapped kernel for 33..256 sessions (gemm_ns.cu): A = activations, B = two weight tiles (N = 256) ------------
+// ---- non-swapped kernel for 17..256 sessions (gemm_ns.cu): A = activations, B = two weight tiles (N = 256) ------------
 bool ns_supported(int M, int N, int K, int epi);
 int ns_prepare();
 // cluster: K-splits (0 = the measured choice for the shape); same packed weights and epilogues as sk_linear
 // unit_tiles: weight tiles per CTA as the B operand (2 = N 256; 1 = N 128: twice the units for few-tile shapes; 0 = the LM's choice)
-int ns_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const void* w_tiles, __nv_bfloat16* y, long long ldy,
+// sa, sw: scales of int8 rows (x is int8 then); both or neither
+int ns_linear(GemmPlanCache& cache, const void* x, long long ldx, const void* w_tiles, __nv_bfloat16* y, long long ldy,
               const __nv_bfloat16* res, long long ldr, int M, int N, int K, int epi, int gate_rows, int cluster, int pdl,
-              cudaStream_t stream, int unit_tiles = 0);
+              cudaStream_t stream, int unit_tiles = 0, const float* sa = nullptr, const float* sw = nullptr);
 
 // ---- the depformer of one frame as one persistent kernel (dep_fused.cu) ---------------------------
 struct DepFusedConfig {

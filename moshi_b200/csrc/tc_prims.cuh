@@ -145,23 +145,27 @@ __device__ __forceinline__ void commit_elected(uint32_t bar) {
 // low word of make_desc; the high word is the same for every operand
 constexpr uint32_t DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_low(uint32_t smem) { return ((smem & 0x3FFFFu) >> 4) | (1u << 16); }
-// the four products of a k-block, by one thread of the warp: rows at desc a, columns w_at 16-byte pieces behind them
-#define UMMA_BLOCK(GROUP)                                                                                                                              \
+// The four products of a k-block (128 bytes of k), by one thread of the warp: rows at desc a, columns w_at 16-byte pieces behind them.
+#define UMMA_BLOCK(GROUP, KIND)                                                                                                                        \
   asm volatile(                                                                                                                                        \
       "{\n\t.reg .pred p, t, q;\n\t.reg .b64 a0, a1, a2, a3, w0, w1, w2, w3;\n\t"                                                                     \
       "mov.b64 a0, {%1, %11};\n\tmov.b64 a1, {%2, %11};\n\tmov.b64 a2, {%3, %11};\n\tmov.b64 a3, {%4, %11};\n\t"                                     \
       "mov.b64 w0, {%5, %11};\n\tmov.b64 w1, {%6, %11};\n\tmov.b64 w2, {%7, %11};\n\tmov.b64 w3, {%8, %11};\n\t"                                     \
       "setp.ne.b32 p, %10, 0;\n\tsetp.ne.b32 t, %11, 0;\n\telect.sync _|q, 0xffffffff;\n\t"                                                         \
-      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a0, w0, %9, p;\n\t"                                                                         \
-      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a1, w1, %9, t;\n\t"                                                                         \
-      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a2, w2, %9, t;\n\t"                                                                         \
-      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a3, w3, %9, t;\n\t}"                                                                        \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a0, w0, %9, p;\n\t"                                                                    \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a1, w1, %9, t;\n\t"                                                                    \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a2, w2, %9, t;\n\t"                                                                    \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a3, w3, %9, t;\n\t}"                                                                   \
       ::"r"(d), "r"(a), "r"(a + 2), "r"(a + 4), "r"(a + 6), "r"(w), "r"(w + 2), "r"(w + 4), "r"(w + 6), "r"(idesc), "r"(accumulate), "r"(DESC_HIGH) : "memory")
 template <int CG>
 __device__ __forceinline__ void umma_block(uint32_t d, uint32_t a, uint32_t w_at, uint32_t idesc, uint32_t accumulate) {
   const uint32_t w = a + w_at;
-  if constexpr (CG == 2) UMMA_BLOCK("2");
-  else UMMA_BLOCK("1");
+  if constexpr (CG == 2) UMMA_BLOCK("2", "f16");
+  else UMMA_BLOCK("1", "f16");
+}
+__device__ __forceinline__ void umma_block_i8(uint32_t d, uint32_t a, uint32_t w_at, uint32_t idesc, uint32_t accumulate) {
+  const uint32_t w = a + w_at;
+  UMMA_BLOCK("1", "i8");
 }
 #undef UMMA_BLOCK
 
