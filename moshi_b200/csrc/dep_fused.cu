@@ -157,14 +157,13 @@ __device__ void row_phase(const P& p, int dd, int S, const float* part, int N, b
 }
 
 // x = depformer_in[k](transformer_out) + emb_k(prev)   (lm.py:475-486; token -1 -> zero row, lm_utils.py:103-121)
-template <int WIDTH>
 __device__ void input_rows(const DepParams& p, int k) {
   const long long* prev = k == 0 ? p.text_token : p.audio_tokens + (long long)(k - 1) * p.B;
   const bf16* table = p.tables[k];
   for (int m = blockIdx.x; m < p.B; m += gridDim.x) {
     const long long id = prev[m];
     const bool ok = lm::embed_id_ok(id, k == 0 ? p.text_card : p.card, p.err);
-    for (int j = threadIdx.x; j < p.dd; j += WIDTH) {
+    for (int j = threadIdx.x; j < p.dd; j += THREADS) {
       const float e = ok ? bf2f(table[id * p.dd + j]) : 0.f;
       p.x[(long long)m * p.dd + j] = f2bf(bf2f(p.din[(long long)m * p.din_ld + (long long)k * p.dd + j]) + e);
     }
@@ -409,7 +408,7 @@ dep_fused_kernel(const __grid_constant__ CUtensorMap map_xn, const __grid_consta
   };
   Gemm cur = gemm_at(0, 0, 0);
   for (int k = 0; k < p.dep_q; ++k) {
-    input_rows<THREADS>(p, k);
+    input_rows(p, k);
     row_phase<4>(p, p.dd, 0, nullptr, 0, false, p.n1[0], red);
     grid_sync(p.bar, epoch, p.trace);
     for (int l = 0; l < p.L; ++l) {
@@ -493,6 +492,7 @@ struct DepFused {
   int grid = 0; size_t smem = 0;
   DepRegKernel reg = nullptr;     // up to 16 sessions: dep_reg_kernel with as many blocks of 8 as they fill (null: dep_fused_kernel)
   void* dev_tables = nullptr;     // one allocation holding the pointer tables
+  RegWords io{}; size_t io_bytes = 0;      // dep_reg_kernel: what its CTAs pass to one another
 };
 
 bool dep_fused_few_sessions(const DepFusedConfig& c) { return dep_reg_takes(c, sk_num_sms()); }
@@ -519,7 +519,9 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(fn);
   // one limit for every handle: a kernel has one, and a handle that set its own need would take a larger one's away
   static std::atomic<uint64_t> limits{0};
-  B200_TRY(allow_smem(limits, SMEM_LIMIT, dep_fused_kernel, dep_reg_kernel<1, false>, dep_reg_kernel<1, true>, dep_reg_kernel<2, false>, dep_reg_kernel<2, true>));
+  B200_TRY(allow_smem(limits, SMEM_LIMIT, dep_fused_kernel, dep_reg_pick(1, 8, false), dep_reg_pick(1, 8, true), dep_reg_pick(1, lm::DEP_MAX_Q, false),
+                      dep_reg_pick(1, lm::DEP_MAX_Q, true), dep_reg_pick(REG_B, 8, false), dep_reg_pick(REG_B, 8, true), dep_reg_pick(REG_B, lm::DEP_MAX_Q, false),
+                      dep_reg_pick(REG_B, lm::DEP_MAX_Q, true)));
   DepFused* d = new DepFused();
   DepParams& p = d->p;
   memset(&p, 0, sizeof(p));
@@ -582,9 +584,14 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   B200_TRY(make_map(enc, &d->map_x, c.x, c.B, c.dd, p.Mpad));
   d->smem = (size_t)stages * p.stage_bytes + 1024 + 16 * MAX_STAGES + 64;
   if (dep_reg_takes(c, d->grid)) {
-    const int nt = c.B <= 8 ? 1 : 2;
-    d->reg = dep_reg_pick(nt, c.trace || c.wait_ns > 0);
+    d->reg = dep_reg_pick(c.B, c.dep_q, c.trace || c.wait_ns > 0);
     d->smem = dep_reg_smem(c, d->grid);
+    d->io_bytes = dep_reg_words(c) * REG_WORD;
+    if (cudaMalloc(&d->io.x, d->io_bytes) != cudaSuccess) { dep_fused_destroy(d); B200_FAIL(B200_ERR_CUDA, "fused depformer: cudaMalloc failed"); }
+    d->io.qkv = d->io.x + (size_t)c.B * (c.dd / 2);
+    d->io.ao = d->io.qkv + (size_t)c.B * (3 * c.dd / 2);
+    d->io.h = d->io.ao + (size_t)c.B * (c.dd / 2);
+    d->io.logits = d->io.h + (size_t)c.B * (c.F / 2);
   }
   int per_sm = 0, coop = 0, dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
@@ -607,13 +614,15 @@ void dep_fused_set_sampling(DepFused* d, int use_sampling, float temp, int top_k
 void dep_fused_destroy(DepFused* d) {
   if (!d) return;
   if (d->dev_tables) cudaFree(d->dev_tables);
+  if (d->io.x) cudaFree(d->io.x);
   delete d;
 }
 
 // Cooperative launch: the driver guarantees that all CTAs of the grid are co-resident (or fails the launch), so the grid
 // barrier cannot deadlock against another handle's persistent kernel, an MPS neighbour or a second replica on the same GPU.
 int dep_fused_launch(DepFused* d, cudaStream_t stream) {
-  B200_CUDA(cudaMemsetAsync(d->p.bar, 0, sizeof(unsigned), stream));
+  if (d->reg && d->p.B <= 8) B200_CUDA(cudaMemsetAsync(d->io.x, 0, d->io_bytes, stream));
+  else B200_CUDA(cudaMemsetAsync(d->p.bar, 0, sizeof(unsigned), stream));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)d->grid); cfg.blockDim = dim3((unsigned)(d->reg ? REG_THREADS : THREADS)); cfg.dynamicSmemBytes = d->smem; cfg.stream = stream;
@@ -621,8 +630,7 @@ int dep_fused_launch(DepFused* d, cudaStream_t stream) {
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  bf16* qkv = reinterpret_cast<bf16*>(d->p.part0);      // the partial sums' workspace holds the projections
-  const cudaError_t le = d->reg ? cudaLaunchKernelEx(&cfg, d->reg, d->p, qkv)
+  const cudaError_t le = d->reg ? cudaLaunchKernelEx(&cfg, d->reg, d->p, d->io)
                                 : cudaLaunchKernelEx(&cfg, dep_fused_kernel, d->map_xn, d->map_ao, d->map_h, d->map_x, d->p);
   if (le != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "fused depformer: cooperative launch failed: %s", cudaGetErrorString(le));
   g_launches.fetch_add(1, std::memory_order_relaxed);

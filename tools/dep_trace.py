@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Per-phase timing of the depformer's persistent kernels (diagnostics): with B200_DEP_TRACE=1 CTA 0 records %globaltimer after every
-grid barrier; this prints the time between consecutive barriers grouped by the phase that ran in between.
+grid barrier (up to 8 sessions: when its first thread has what a step wrote); this prints the time between consecutive barriers grouped by the phase that ran in between.
 
     B200_DEP_TRACE=1 python tools/dep_trace.py --B 104 > dep_trace_b104.json
 """
