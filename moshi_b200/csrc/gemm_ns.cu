@@ -5,11 +5,11 @@
 //   * A = the activations, one SWIZZLE_128B box of 128 bytes of k per k-block (2-D TMA; two blocks of rows above 128 sessions).  The box has as many rows as there are
 //     sessions, to whole eights: a row-wise copy costs about 2.7 ns per row and SM, zeroes too.  The instruction reads 128 rows all the same: what lies behind the box (the
 //     next stage's weights, free space behind the last) goes into rows of the accumulator that nobody reads.  The stages that this leaves room for are in flight instead;
-//   * B = TWO pre-tiled 128-row weight tiles side by side (N = 256 per instruction: twice the weight bytes per tensor-pipe
-//     cycle); for the gated MLP the pair is (gate rows, value rows) of the same outputs, already stored back to back, so the
-//     accumulator holds gate in columns 0..127 and value in 128..255 of the SAME thread and silu(g) * u needs no exchange;
-//   * D = [128 sessions (TMEM lanes) x 128 or 256 weight rows (columns)] fp32.  k-blocks go to the accumulators that fit into TMEM in turn (4 of single tiles, 2 of pairs; half
-//     above 128 sessions), which are added in fp32: the tensor cores cut off what a long chain's additions leave over.  Error of the sums alone (terms whose exact sum is 0, over
+//   * B = the weight rows of a unit, 16 to 256 of them in one instruction; gated: as many of the gate and behind them those of the value, so that the accumulator holds gate
+//     and value of an output in the SAME thread and silu(g) * u needs no exchange.  Eight rows of a packed tile are 1024 bytes on end, so a unit need not be whole tiles:
+//     where K is whole every SM gets the same share of the rows (ns_default_plan);
+//   * D = [128 sessions (TMEM lanes) x 128 or 256 weight rows (columns)] fp32.  k-blocks go to the accumulators that fit into TMEM in turn (4 up to 128 columns, 2 beyond or gated;
+//     half above 128 sessions), which are added in fp32: the tensor cores cut off what a long chain's additions leave over.  Error of the sums alone (terms whose exact sum is 0, over
 //     the rms of a random sum of them), 24 rows, one accumulator / these / what took 17..32 rows before: 4096 -> 12288 2.0e-6 / 4.8e-7 / 6.6e-7, 4096 -> 4096 4.8e-7 / 1.3e-7
 //     / 2.4e-7, 11264 -> 4096 1.5e-6 / 3.4e-7 / 6.2e-7, 4096 -> 32000 2.0e-6 / 1.0e-6 / 1.7e-6.  The epilogue keeps its registers without a stack for it: a stack
 //     frame of a few words costs a launch 2 to 3 us.  int8 sums are exact: one accumulator;
@@ -18,14 +18,17 @@
 //   * shapes with few units are cut along K over a cluster of 2..4 CTAs; every CTA adds the sums of all of them over distributed shared memory for its share of the
 //     sessions, in rank order (deterministic): no workspace, no atomics.  ns_default_plan() holds the measured choice per shape;
 //   * copies and products are issued from uniform registers (tc_prims.cuh).
-// us, one launch behind the other through the entry point with cold weights, before these / now.  104 sessions: 4096 -> 12288 27.9 / 20.5, 4096 -> 4096 16.1 / 13.1, 11264 -> 4096
-// 26.4 / 22.0, 4096 -> 32000 50.9 / 45.3, gated -> 11264 38.2 / 37.8.  48: 25.3 / 20.0, 13.5 / 10.7, 23.6 / 19.3, 48.5 / 44.0, 37.3 / 37.3.  256: 44.3 / 31.8, 27.5 / 21.8, 42.3 /
-// 34.3, 70.7 / 63.2, 54.8 / 54.5.  24 sessions (gemm_reg.cu, gemm_sk.cu / now): 28.0 / 19.9, 15.0 / 10.0, 28.0 / 18.4, 53.6 / 43.1, 48.8 / 36.6.  int8 (gemm_reg.cu, gemm_sk.cu /
-// now): 24 17.6 / 11.8, 11.3 / 7.4, 18.3 / 11.0, 34.3 / 24.5, 34.3 / 22.1; 104 26.5 / 12.1, 17.6 / 10.3, 23.2 / 14.4, 41.2 / 25.9, 40.6 / 22.7; 256 40.4 / 17.1, 57.3 / 18.1, 88.6 /
-// 23.9, 72.6 / 37.3, 69.9 / 33.7.  A step of the 7B with 24 sessions 7.29 -> 5.88 ms, with 40 6.81 -> 6.32, with 72 7.56 -> 7.22.
+// us, one launch behind the other through the entry point with cold weights, before these / now.  104 sessions: 4096 -> 12288 27.9 / 20.6, 4096 -> 4096 16.1 / 13.3, 11264 -> 4096
+// 26.4 / 22.1, 4096 -> 32000 50.9 / 44.0, gated -> 11264 37.9 / 33.5 (37.6 in whole tiles), gated 1024 -> 2816 12.8 / 9.0 (12.2).  48: 25.3 / 20.0, 13.5 / 10.7, 23.6 / 19.3, 48.5 /
+// 42.7, 37.1 / 33.2, 12.2 / 8.2.  256: 44.3 / 32.2, 27.5 / 21.8, 42.3 / 34.6, 70.8 / 61.2, 54.6 / 45.2, 20.5 / 12.0.  24 sessions (gemm_reg.cu, gemm_sk.cu / now): 28.0 / 19.9, 15.0 /
+// 10.0, 28.0 / 18.4, 53.5 / 42.7, 50.3 / 33.3, 19.1 / 8.0.  int8 (gemm_reg.cu, gemm_sk.cu / now): 24 17.6 / 11.8, 11.3 / 7.4, 18.3 / 11.0, 34.2 / 24.1, 34.5 / 20.9, 11.6 / 6.5; 104
+// 26.5 / 12.2, 17.6 / 10.3, 23.2 / 14.4, 41.0 / 25.6, 40.5 / 22.1, 25.3 / 7.2; 256 40.4 / 17.2, 57.3 / 18.0, 88.6 / 23.2, 68.5 / 37.1, 69.8 / 32.4, 51.5 / 10.1.  A step of the 7B with 24
+// sessions 7.29 -> 5.82 ms, with 40 6.81 -> 6.31, with 72 7.56 -> 7.11.
 //
 // Same packed weights, same epilogues and cast points as gemm_sk.cu (residual add bf16(res + bf16(acc)), gated SiLU
 // bf16(bf16(silu(g)) * u), gating.py:18-20); same PDL protocol (weights requested before griddepcontrol.wait).
+#include <algorithm>
+
 #include "gemm_sk.cuh"
 #include "tc_prims.cuh"
 
@@ -50,7 +53,7 @@ constexpr int MAX_CS = 8;
 constexpr int TMEM_COLS = 512;               // all of it: one CTA per SM
 
 struct NsParams {
-  int M, N, K, out_rows, gate_rows, CS, num_kb, kb_per, stages, n_tiles, unit_tiles, mblocks, n_acc, box_rows;
+  int M, N, K, out_rows, gate_rows, CS, num_kb, kb_per, stages, n_tiles, unit_rows, acc_cols, mblocks, n_acc, box_rows;
   const uint8_t* wt;
   __nv_bfloat16* y; long long ldy;
   const __nv_bfloat16* res; long long ldr;
@@ -141,8 +144,8 @@ __device__ __forceinline__ uint4 ns_residual(const NsParams& p, int m, int o, in
 // Session rows row, row + step, .. below end of a block (m0: its first session), a thread's eight columns from output column o on (piece c of a row).  The block's sums lie at
 // `sums`: in fp32 in every CTA of a cluster, added in rank order, or (CS == 1) rounded to bf16, what the epilogues do anyway.
 template <int EPI, bool I8>
-__device__ __forceinline__ void ns_finish(const NsParams& p, uint32_t sums, uint32_t sa, uint32_t sw, int m0, int row, int end, int step, int c, int width_log2, int o, uint4 res) {
-  const int valid = p.out_rows - o;
+__device__ __forceinline__ void ns_finish(const NsParams& p, uint32_t sums, uint32_t sa, uint32_t sw, int m0, int row, int end, int step, int c, int width_log2, int nb, int o_end, uint4 res) {
+  const int o = nb + c * 8, valid = o_end - o;
   if (valid <= 0) return;
 #pragma unroll 1
   for (; row < end; row += step) {
@@ -200,7 +203,8 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  const uint32_t a_off = (uint32_t)p.unit_tiles * TILE_BYTES;             // stage = B (one or two weight tiles) | A (activation box)
+  const int R = p.unit_rows;                                              // output rows of a unit (gated: of the gate, and as many of the value)
+  const uint32_t a_off = (uint32_t)(EPI == EPI_GATE ? 2 * R : R) * 128u;  // stage = B (the unit's weight rows) | A (activation box)
   const uint32_t a_bytes = (uint32_t)p.box_rows * 128u;                   // the rows that exist, to whole eights: what follows them is multiplied too, into rows that nobody reads
   const uint32_t stage_bytes = a_off + a_bytes;
   const uint32_t bars = base + (uint32_t)p.stages * stage_bytes + ((uint32_t)p.mblocks * A_BYTES - a_bytes);      // the last stage's products read as far
@@ -213,12 +217,8 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
   const int unit = blockIdx.x / p.CS, me = blockIdx.x - unit * p.CS;
   const int kb0 = me * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
   const int n_items = kb1 > kb0 ? kb1 - kb0 : 0;
-  // weight tiles of this unit: the (gate, value) pair, or row tiles 2u and 2u+1 (the last unit of an odd count has one)
-  const bool two = EPI == EPI_GATE || (p.unit_tiles == 2 && 2 * unit + 1 < p.n_tiles);
-  const int tile0 = EPI == EPI_GATE ? unit : unit * p.unit_tiles;
-  const int width = two ? 256 : 128;                                      // accumulator columns in use
-  const uint32_t acc_cols = 128u * p.unit_tiles;                          // and those that an accumulator is given: mblocks x n_acc x acc_cols = TMEM_COLS
-  const uint32_t b_bytes = two ? 2u * TILE_BYTES : (uint32_t)TILE_BYTES;
+  const int nb = unit * R, width = EPI == EPI_GATE ? 2 * R : R;           // first output row; accumulator columns in use
+  const uint32_t acc_cols = (uint32_t)p.acc_cols;                         // and those that an accumulator is given: mblocks x n_acc x acc_cols = TMEM_COLS
 
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
@@ -239,14 +239,18 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
 
   // both loops are walked by their whole warps, and one thread issues (tc_prims.cuh)
   if (warp == 0) {
+    const int there = min(R, p.n_tiles * BLOCK_ROWS - nb);                  // the last unit may reach beyond the last tile: its columns there are multiplied and not stored
+    const uint32_t b_bytes = (uint32_t)(EPI == EPI_GATE ? 2 * there : there) * 128u;
     auto load_b = [&](int i, int s) {
-      const int kb = kb0 + i;
+      // eight rows of a tile are 1024 bytes on end: one copy per tile that the unit has rows of (gated: one of each of a pair's tiles)
       const uint32_t sb = base + (uint32_t)s * stage_bytes;
-      if (EPI == EPI_GATE) {
-        bulk_load(sb, p.wt + ((size_t)unit * p.num_kb + kb) * (2 * TILE_BYTES), 2 * TILE_BYTES, full0 + 8 * s);
-      } else {
-        bulk_load(sb, p.wt + ((size_t)tile0 * p.num_kb + kb) * TILE_BYTES, TILE_BYTES, full0 + 8 * s);
-        if (two) bulk_load(sb + TILE_BYTES, p.wt + ((size_t)(tile0 + 1) * p.num_kb + kb) * TILE_BYTES, TILE_BYTES, full0 + 8 * s);
+#pragma unroll 1
+      for (int r = 0; r < there; ) {
+        const int tile = (nb + r) >> 7, in = (nb + r) & 127, n = min(128 - in, there - r);
+        const uint8_t* src = p.wt + ((size_t)tile * p.num_kb + (kb0 + i)) * (EPI == EPI_GATE ? 2 * TILE_BYTES : TILE_BYTES) + in * 128;
+        bulk_load(sb + (uint32_t)r * 128u, src, (uint32_t)n * 128u, full0 + 8 * s);
+        if (EPI == EPI_GATE) bulk_load(sb + (uint32_t)(R + r) * 128u, src + TILE_BYTES, (uint32_t)n * 128u, full0 + 8 * s);
+        r += n;
       }
     };
     // weights first (they do not depend on the preceding kernel), activations after the dependency wait
@@ -294,15 +298,15 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
 
   // ===== epilogue: TMEM lane = session row.  Results go through the ring, which is empty by then, so that what is stored and read is whole lines =====
   const int q4 = warp & 3, sub = (warp - 2) >> 2, qt = sub * 32 + lane, tid = threadIdx.x - 64;      // TMEM quadrant, this warp's place among its four
-  const int out_log2 = EPI == EPI_GATE || !two ? 7 : 8, out_width = 1 << out_log2, pieces = out_width >> 3;      // output columns of the unit, in pieces of eight
-  const int nb = tile0 * BLOCK_ROWS;
+  const int out_log2 = R <= 128 ? 7 : 8, pieces = 1 << (out_log2 - 3);      // a row of results in shared memory has 128 or 256 columns, R of which are in use
   // CS == 1: a quadrant's 128 threads finish its 32 rows; else every CTA of the cluster its share of the block's rows, 512 threads
-  const int t = p.CS == 1 ? qt : tid, step = (p.CS == 1 ? 128 : 512) >> (out_log2 - 3), c = t & (pieces - 1), o = nb + c * 8;
+  const int t = p.CS == 1 ? qt : tid, step = (p.CS == 1 ? 128 : 512) >> (out_log2 - 3), c = t & (pieces - 1), o_end = min(p.out_rows, nb + R);
   const int n_acc = min(p.n_acc, n_items);
   if (I8 && warp >= 2) {                        // scales: the weights' like the weights, the sessions' after the wait
     if (tid < width) {
-      const int n = EPI == EPI_GATE ? (tid < 128 ? nb + tid : p.gate_rows + nb + tid - 128) : nb + tid;
-      ns_sts1(sw + 4u * (uint32_t)tid, (EPI == EPI_GATE ? nb + (tid & 127) : n) < p.out_rows ? p.sw[n] : 0.f);
+      const bool value = EPI == EPI_GATE && tid >= R;
+      const int n = nb + (value ? tid - R : tid);
+      ns_sts1(sw + 4u * (uint32_t)tid, n < p.out_rows ? p.sw[value ? p.gate_rows + n : n] : 0.f);
     }
     pdl_wait();
     if (tid < p.M) ns_sts1(sa + 4u * (uint32_t)tid, p.sa[tid]);
@@ -314,7 +318,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
     if (warp >= 2) {
       uint4 res = make_uint4(0u, 0u, 0u, 0u);
       if (mb == 0) pdl_wait();                  // y / res may still be in use by the predecessor
-      if (EPI == EPI_RESADD && row0 < end && o < p.out_rows) res = ns_residual(p, mb * 128 + row0, o, p.out_rows - o);
+      if (EPI == EPI_RESADD && row0 < end && nb + c * 8 < o_end) res = ns_residual(p, mb * 128 + row0, nb + c * 8, o_end - nb - c * 8);
       if (mb == 0) {
         mbar_wait(tfull, 0);
         tc_fence_after();
@@ -324,21 +328,21 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
       const float m_scale = I8 && m_ok ? ns_lds1(sa + 4u * (uint32_t)(mb * 128 + row)) : 0.f;
       const uint32_t lane_addr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(mb * p.n_acc) * acc_cols;
 #pragma unroll EPI == EPI_GATE ? 2 : 1
-      for (int c0 = sub * 16; c0 < (EPI == EPI_GATE ? 128 : out_width); c0 += EPI_STEP) {
+      for (int c0 = sub * 16; c0 < R; c0 += EPI_STEP) {
         float v[16];
         if (n_items > 0) {
           __syncwarp();
           ns_sums<I8 ? 1 : EPI == EPI_GATE ? 2 : 4>(lane_addr + (uint32_t)c0, acc_cols, n_acc, v);
           if (EPI == EPI_GATE) {
-            // columns j (gate) and 128 + j (value) of the same output; CS == 1 (the pair never needs a split: 88 units at 7B)
+            // columns j (gate) and R + j (value) of the same output; K whole
             float u[16];
-            ns_sums<I8 ? 1 : 2>(lane_addr + (uint32_t)(128 + c0), acc_cols, n_acc, u);
+            ns_sums<I8 ? 1 : 2>(lane_addr + (uint32_t)(R + c0), acc_cols, n_acc, u);
             if (m_ok) {                         // not for rows of zeroes: a division of zero takes the long way (33 to 104 rows: 41 us instead of 35)
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
                 if (I8) {
                   v[j] = ns_scaled(v[j], m_scale, ns_lds1(sw + 4u * (uint32_t)(c0 + j)));
-                  u[j] = ns_scaled(u[j], m_scale, ns_lds1(sw + 4u * (uint32_t)(128 + c0 + j)));
+                  u[j] = ns_scaled(u[j], m_scale, ns_lds1(sw + 4u * (uint32_t)(R + c0 + j)));
                 }
                 const float gt = ns_bf16_round(v[j]), ut = ns_bf16_round(u[j]);
                 v[j] = ns_bf16_round(gt / (1.f + expf(-gt))) * ut;
@@ -368,12 +372,12 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
       }
       if (EPI == EPI_GATE || p.CS == 1) {
         asm volatile("bar.sync %0, 128;" ::"r"(1 + q4) : "memory");
-        ns_finish<EPI, I8>(p, base, sa, sw, mb * 128, row0, end, step, c, out_log2, o, res);
+        ns_finish<EPI, I8>(p, base, sa, sw, mb * 128, row0, end, step, c, out_log2, nb, o_end, res);
         asm volatile("bar.sync %0, 128;" ::"r"(1 + q4) : "memory");
       } else {
         __syncwarp();
         ns_cluster_sync();
-        ns_finish<EPI, I8>(p, base, sa, sw, mb * 128, row0, end, step, c, out_log2, o, res);
+        ns_finish<EPI, I8>(p, base, sa, sw, mb * 128, row0, end, step, c, out_log2, nb, o_end, res);
       }
       tc_fence_before();
     } else if (p.CS > 1) {
@@ -423,19 +427,21 @@ bool ns_supported(int M, int N, int K, int epi) {
 
 int ns_prepare() { return ns_init(); }
 
-// The LM's choice of unit and K-split for a shape (us, one behind the other with cold weights through the entry point):
-//   * tiles for more than half the SMs, and no more than there are: one tile per CTA, K whole.  (4096 -> 12288, 96 tiles: pairs of tiles with K cut in two 28.5 us at 104
-//     sessions, 43.7 at 160, 49.2 at 256; so, with whole boxes and one accumulator, 25.4, 39.4 and 42.9.  The pairs read 48 KB per k-block and SM for 64 and exchange 128 columns.)
-//   * more (the gated MLP's input 88 pairs, the text head 250 tiles): pairs of tiles, N = 256, K whole (text head: 51.7, single tiles in two waves 55);
-//   * fewer (out_proj / linear_out: 32 tiles, depformer_in: 64): single tiles so that more SMs pull on the weights, K cut over the largest power of two <= 4
+// The LM's choice of unit and K-split for a shape:
+//   * gated, or more tiles than SMs: K whole, and as many output rows per CTA as put the same share (in sixteens; at most 128 pairs or 256) on every SM.  In whole tiles
+//     the 88 pairs of the 7B leave 60 SMs without work;
+//   * plain, tiles for more than half the SMs: tiles, K whole (equal shares of the 96 of 4096 -> 12288 gave 20.5 us for 19.7 at 64 sessions, 27.0 for 28.4 at 160);
+//   * fewer (out_proj / linear_out: 32 tiles, depformer_in: 64): tiles, so that activations are not copied too often, K cut over the largest power of two <= 4
 //     that keeps the grid resident (32 x 4, 64 x 2 = 128 CTAs).
-static void ns_default_plan(int n_tiles, int num_kb, int epi, int* unit_tiles, int* cs) {
-  if (epi == EPI_GATE) { *unit_tiles = 2; *cs = 1; return; }
-  if (n_tiles > g_ns_sms) { *unit_tiles = 2; *cs = 1; return; }
-  *unit_tiles = 1;
-  int c = 1;
-  while (c < 4 && n_tiles * c * 2 <= g_ns_sms && num_kb / (c * 2) >= 4) c *= 2;
-  *cs = c;
+static void ns_default_plan(int out_rows, int n_tiles, int num_kb, int epi, int* unit_rows, int* cs) {
+  *cs = 1;
+  if (epi == EPI_GATE || n_tiles > g_ns_sms) {
+    const int most = epi == EPI_GATE ? 128 : 256, waves = (out_rows + g_ns_sms * most - 1) / (g_ns_sms * most), ctas = waves * g_ns_sms;
+    *unit_rows = ((out_rows + ctas - 1) / ctas + 15) & ~15;
+    return;
+  }
+  *unit_rows = BLOCK_ROWS;
+  while (*cs < 4 && n_tiles * *cs * 2 <= g_ns_sms && num_kb / (*cs * 2) >= 4) *cs *= 2;
 }
 
 int ns_linear(GemmPlanCache& cache, const void* x, long long ldx, const void* w_tiles, __nv_bfloat16* y, long long ldy,
@@ -453,15 +459,16 @@ int ns_linear(GemmPlanCache& cache, const void* x, long long ldx, const void* w_
   p.out_rows = epi == EPI_GATE ? gate_rows : N;
   p.n_tiles = (p.out_rows + BLOCK_ROWS - 1) / BLOCK_ROWS;
   p.num_kb = (K * elem + 127) / 128;
-  int def_ut = 2, def_cs = 1;
-  ns_default_plan(p.n_tiles, p.num_kb, epi, &def_ut, &def_cs);
-  if (unit_tiles == 0) unit_tiles = cluster > 0 ? 2 : def_ut;
-  p.unit_tiles = (unit_tiles == 1 && epi != EPI_GATE) ? 1 : 2;
+  int def_rows = 0, def_cs = 1;
+  ns_default_plan(p.out_rows, p.n_tiles, p.num_kb, epi, &def_rows, &def_cs);
+  p.unit_rows = unit_tiles == 0 && cluster <= 0 ? def_rows : (unit_tiles == 1 || epi == EPI_GATE) ? BLOCK_ROWS : 2 * BLOCK_ROWS;
+  const int b_rows = epi == EPI_GATE ? 2 * p.unit_rows : p.unit_rows;
+  p.acc_cols = b_rows <= 128 ? 128 : 256;
   p.mblocks = M > 128 ? 2 : 1;
-  p.n_acc = i8 ? 1 : TMEM_COLS / (p.mblocks * p.unit_tiles * 128);
+  p.n_acc = i8 ? 1 : std::min(epi == EPI_GATE ? 2 : 4, TMEM_COLS / (p.mblocks * p.acc_cols));
   p.box_rows = (M + 7) & ~7;
-  const uint32_t stage_bytes = (uint32_t)p.unit_tiles * TILE_BYTES + (uint32_t)p.box_rows * 128u, beyond = (uint32_t)p.mblocks * A_BYTES - (uint32_t)p.box_rows * 128u;
-  const int n_units = (epi == EPI_GATE || p.unit_tiles == 1) ? p.n_tiles : (p.n_tiles + 1) / 2;
+  const uint32_t stage_bytes = (uint32_t)b_rows * 128u + (uint32_t)p.box_rows * 128u, beyond = (uint32_t)p.mblocks * A_BYTES - (uint32_t)p.box_rows * 128u;
+  const int n_units = (p.out_rows + p.unit_rows - 1) / p.unit_rows;
   int cs = cluster > 0 ? cluster : def_cs;
   if (epi == EPI_GATE) cs = 1;
   if (cs > MAX_CS) cs = MAX_CS;
@@ -472,7 +479,7 @@ int ns_linear(GemmPlanCache& cache, const void* x, long long ldx, const void* w_
   if (stages > MAX_STAGES) stages = MAX_STAGES;
   if (stages > p.kb_per && p.kb_per >= 2) stages = p.kb_per;
   if (stages < 2) stages = 2;
-  const size_t sums = (size_t)128 * (p.unit_tiles == 2 && epi != EPI_GATE ? 256 : 128) * (cs > 1 ? 4 : 2);      // a block's results or partial sums, in the ring
+  const size_t sums = (size_t)128 * (p.unit_rows <= 128 ? 128 : 256) * (cs > 1 ? 4 : 2);      // a block's results or partial sums, in the ring
   while ((size_t)stages * stage_bytes < sums) ++stages;
   p.stages = stages;
   p.wt = static_cast<const uint8_t*>(w_tiles);

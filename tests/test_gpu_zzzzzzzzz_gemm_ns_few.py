@@ -1,5 +1,6 @@
 """GPU: linears of 17 rows on through gemm_ns_kernel by the general entry points: boxes of as many activation rows as there are (to whole eights), what the tensor cores read
-beyond them, accumulators taken in turn, int8."""
+beyond them, accumulators taken in turn, int8; output rows shared
+out in sixteens: units inside a tile, across two or three, a last one that is not full, one more wave."""
 import ctypes as C
 
 import pytest
@@ -10,7 +11,8 @@ from .util import cptr
 
 pytestmark = pytest.mark.gpu
 STORE, RESIDUAL, GATED = 0, 1, 2
-SHAPES = [(130, 144, STORE), (264, 4112, RESIDUAL), (75 * 128, 80, RESIDUAL), (149 * 128 - 8, 256, STORE), (2 * 392, 336, GATED), (4096, 1024, RESIDUAL)]
+SHAPES = [(130, 144, STORE), (264, 4112, RESIDUAL), (75 * 128, 80, RESIDUAL), (149 * 128 - 8, 256, STORE), (2 * 392, 336, GATED), (4096, 1024, RESIDUAL),
+          (2 * 2824, 592, GATED), (2 * (148 * 32 + 8), 128, GATED), (2 * 18952, 80, GATED), (37896, 144, STORE)]
 
 
 def _stream():
