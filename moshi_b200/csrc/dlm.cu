@@ -794,10 +794,10 @@ int finalize_sandwich_layer(b200_dlm* h, int i, std::vector<void*>& drop) {
 template <typename T>
 int small_proj(b200_dlm* h, const T* x, long long ldx, const void* w, const float* b, float* out, int M, int N, int K) {
   static std::atomic<uint64_t> limits{0};
-  B200_TRY(allow_smem(limits, 200 * 1024, (small_proj_f32_kernel<T, 1>), (small_proj_f32_kernel<T, 8>)));
+  B200_TRY(allow_smem(limits, 200 * 1024, (small_proj_f32_kernel<T, 1>), (small_proj_f32_kernel<T, 4>)));
   const int vec = K % 8 == 0 && (ldx * sizeof(T)) % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
   const size_t row = (size_t)K * sizeof(T);
-  if (M >= 512 && 8 * row <= 100 * 1024) B200_LAUNCH((small_proj_f32_kernel<T, 8>), dim3(ceil_div(M, 8), ceil_div(N, 32)), 256, 8 * row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
+  if (M >= 512 && 4 * row <= 100 * 1024) B200_LAUNCH((small_proj_f32_kernel<T, 4>), dim3(ceil_div(M, 4), ceil_div(N, 8)), 256, 4 * row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
   else EARLY_LAUNCH_IF(M < EARLY_TOKENS, (small_proj_f32_kernel<T, 1>), dim3(M, M >= 512 ? 1 : ceil_div(N, 8)), 256, row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
   return check_launch("small_proj_f32");
 }

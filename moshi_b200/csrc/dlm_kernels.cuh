@@ -229,6 +229,29 @@ __global__ void __launch_bounds__(128) latent_append_kernel(const T* proj, long 
   if (t >= n_tok) return;
   const T* raw = proj + (long long)t * ldp + off;
   float s = 0.f;
+  if (r % 256 == 0 && r <= 1024 && ((ldp | off) & 7) == 0) {      // runs of eight, a row in registers (element by element and read twice: 9.3 us for 2048 tokens, so 4.7)
+    T* to = cache + ((long long)tok_slot[t] * cap + tok_pos[t]) * r;
+    float v[4][8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k * 256 < r) load8(raw + k * 256 + l * 8, v[k]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (k * 256 < r) s = fmaf(v[k][e], v[k][e], s);
+    const float rs = 1.f / sqrtf(warp_sum(s) / (float)r + eps);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k * 256 < r) {
+        float wv[8];
+        load8(w + k * 256 + l * 8, wv);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[k][e] = v[k][e] * rs * wv[e];
+        store8(to + k * 256 + l * 8, v[k]);
+      }
+    return;
+  }
   for (int i = l; i < r; i += 32) { const float v = to_f(raw[i]); s += v * v; }
   const float rs = 1.f / sqrtf(warp_sum(s) / (float)r + eps);
   T* dst = cache + ((long long)tok_slot[t] * cap + tok_pos[t]) * r;

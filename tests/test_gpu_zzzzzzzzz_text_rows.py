@@ -1,0 +1,34 @@
+"""GPU: the decoder LMs' small kernels by rows: latents appended in runs of eight (ranks of 256 to 1024), projections to fp32 with four tokens to a CTA from 512 tokens on."""
+import pytest
+import torch
+
+from .test_gpu_zz_decoder_lm import assert_close, build, gen_for, layer, make_cfg, tokens
+from . import test_gpu_zzzzzz_megolorn as megolorn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rank", [256, 264, 512, 1024])
+def test_latents(rank, dtype):
+    """One run a lane, two, four; a rank between that keeps single elements: the whole model at the suite's tolerance, every token's latent read by the ones behind."""
+    cfg = make_cfg([layer(2, 16, 8, rank, 0.2, 64), layer(2, 16, 8, rank, 0.2, None)], vocab=80, width=64)
+    model, orc = build(cfg, dtype)
+    toks = tokens(14, cfg.vocab, rank)
+    with gen_for(model) as gen:
+        got = gen.step([(0, toks[:9])], list(range(9))).cpu()
+        got = torch.cat([got, gen.step([(0, toks[9:])], list(range(5))).cpu()])
+    assert_close(got, orc.forward(toks), dtype)
+
+
+@pytest.mark.parametrize("n", [511, 512, 513, 515])
+@pytest.mark.parametrize("experts,width", [(5, 52), (16, 96), (11, 264)])
+def test_small_projections(experts, width, n):
+    """Router logits of as many tokens as fill the last CTA and of one to three more; outputs of two groups of eight that are full and not, rows on 16 bytes and off them: in
+    fp32 every logit of the model at the suite's tolerance."""
+    cfg = megolorn.make_cfg([megolorn.attention(2, 1, 16, 16, 0.2, chunk=64, mlp=megolorn.moe(experts, 2, 24))], vocab=97, width=width)
+    model, orc = megolorn.build(cfg, torch.float32)
+    toks = tokens(n, cfg.vocab, n)
+    with gen_for(model, capacity=1024, max_step_tokens=1024) as gen:
+        got = gen.step([(0, toks)], list(range(n))).cpu()
+    megolorn.assert_close(got, orc.forward(toks), torch.float32)
