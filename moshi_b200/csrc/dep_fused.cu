@@ -492,7 +492,7 @@ struct DepFused {
   int grid = 0; size_t smem = 0;
   DepRegKernel reg = nullptr;     // up to 16 sessions: dep_reg_kernel with as many blocks of 8 as they fill (null: dep_fused_kernel)
   void* dev_tables = nullptr;     // one allocation holding the pointer tables
-  RegWords io{}; size_t io_bytes = 0;      // dep_reg_kernel: what its CTAs pass to one another
+  RegWords io{}; size_t io_bytes = 0;      // dep_reg_kernel: what its CTAs pass to one another, and how much of it is zeroed for a launch
 };
 
 bool dep_fused_few_sessions(const DepFusedConfig& c) { return dep_reg_takes(c, sk_num_sms()); }
@@ -586,10 +586,13 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   if (dep_reg_takes(c, d->grid)) {
     d->reg = dep_reg_pick(c.B, c.dep_q, c.trace || c.wait_ns > 0);
     d->smem = dep_reg_smem(c, d->grid);
-    d->io_bytes = dep_reg_words(c) * REG_WORD;
-    if (cudaMalloc(&d->io.x, d->io_bytes) != cudaSuccess) { dep_fused_destroy(d); B200_FAIL(B200_ERR_CUDA, "fused depformer: cudaMalloc failed"); }
-    d->io.qkv = d->io.x + (size_t)c.B * (c.dd / 2);
-    d->io.ao = d->io.qkv + (size_t)c.B * (3 * c.dd / 2);
+    uint64_t* io = nullptr;
+    if (cudaMalloc(&io, dep_reg_words(c) * REG_WORD) != cudaSuccess) { dep_fused_destroy(d); B200_FAIL(B200_ERR_CUDA, "fused depformer: cudaMalloc failed"); }
+    d->io_bytes = (c.B <= 8 ? dep_reg_words(c) : dep_reg_front(c)) * REG_WORD;
+    d->io.qkv = io;
+    d->io.meet = io + dep_reg_front(c) - 16;
+    d->io.x = io + dep_reg_front(c);
+    d->io.ao = d->io.x + (size_t)c.B * (c.dd / 2);
     d->io.h = d->io.ao + (size_t)c.B * (c.dd / 2);
     d->io.logits = d->io.h + (size_t)c.B * (c.F / 2);
   }
@@ -614,14 +617,14 @@ void dep_fused_set_sampling(DepFused* d, int use_sampling, float temp, int top_k
 void dep_fused_destroy(DepFused* d) {
   if (!d) return;
   if (d->dev_tables) cudaFree(d->dev_tables);
-  if (d->io.x) cudaFree(d->io.x);
+  if (d->io.qkv) cudaFree(d->io.qkv);
   delete d;
 }
 
 // Cooperative launch: the driver guarantees that all CTAs of the grid are co-resident (or fails the launch), so the grid
 // barrier cannot deadlock against another handle's persistent kernel, an MPS neighbour or a second replica on the same GPU.
 int dep_fused_launch(DepFused* d, cudaStream_t stream) {
-  if (d->reg && d->p.B <= 8) B200_CUDA(cudaMemsetAsync(d->io.x, 0, d->io_bytes, stream));
+  if (d->reg) B200_CUDA(cudaMemsetAsync(d->io.qkv, 0, d->io_bytes, stream));
   else B200_CUDA(cudaMemsetAsync(d->p.bar, 0, sizeof(unsigned), stream));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));

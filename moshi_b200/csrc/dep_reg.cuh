@@ -8,7 +8,7 @@
 //   * up to 8 sessions there is no barrier: what a step writes carries the step's number word by word (reg_put), and who needs it asks for just that until it is there.  A
 //     buffer is written again only by a CTA that has seen results for which its last readers had to be done (x: of the products that read it; qkv: of the attention; ao and h:
 //     of the products behind them), so nothing is overwritten that somebody still reads.  Above 8 sessions twice the bytes from L2 into every SM cost more than the barrier
-//     (16 sessions: 4.6 ms a step of the 7B instead of 4.4), which stays there;
+//     (16 sessions: 4.6 ms a step of the 7B instead of 4.4), which stays there in front of the products; the attention, a warp of which reads one head, takes words;
 //   * every warp asks for its weights up to four pairs of units x 64 k ahead, through all products, layers and sub-steps and across the exchanges, by bulk copies from a list
 //     that is made once: the addresses worked out on the way and four 16-byte copies per lane took 0.4 us of a pair's 0.7;
 //   * a warp has one k-block of the width, so its share of the RMSNorm is what it multiplies: the sums of squares meet in shared memory; residual, gating
@@ -16,8 +16,9 @@
 //   * the activations of a k-block are in registers while the next ones are under way, and the attention keeps as many keys as there are sub-steps (8, or up to 16): with all
 //     k-blocks and 16 keys the kernel spilled.
 //
-// A step of the 7B with sampling (all but the depformer unchanged), ms, barriers and 16-byte copies / so: 1 session 3.59 / 3.33, 2 3.64 / 3.44, 8 3.83 / 3.62, 9 4.08 / 4.07, 16 4.43 /
-// 4.38.  Of a layer's 15 us at one session the waits for other CTAs' words are about 5, norms 1.6, products 6, the rest sums and epilogues.
+// A step of the 7B with sampling (all but the depformer unchanged), ms, barriers and 16-byte copies / so: 1 session 3.59 / 3.32, 2 3.64 / 3.44, 8 3.83 / 3.61, 9 4.08 / 3.99, 16 4.43 /
+// 4.29.  Words that straddle lines (a buffer that begins off a border of 128 bytes) cost 0.3 ms of it.  Of a layer's 15 us at one session the waits for other CTAs' words are about 5,
+// norms 1.6, products 6, the rest sums and epilogues.
 //
 // Whoever waits for ten seconds in vain stops waiting; the CTA agrees on it at the end of a product, ends, and so do the others.  The frame's remaining tokens are then the
 // frame's before.  It raises ERR_WAIT, and a word on the host that the handle's next call looks at without a synchronisation.
@@ -35,8 +36,8 @@ enum { REG_IN = 0, REG_OUT = 1, REG_GATE = 2, REG_LINEAR_OUT = 3, REG_HEAD = 4, 
 // What passes from CTA to CTA goes as words of 8 bytes, two bf16 and the number of the step that wrote them, written and read whole: a reader asks for its words until their
 // numbers are the step's, and what it has then is the data.
 constexpr int REG_WORD = 8;
-struct RegWords {                                // [session][pair of elements] of what a frame's steps pass on, zero at launch; above 8 sessions pairs without a number
-  uint64_t *x, *qkv, *ao, *h, *logits;
+struct RegWords {                                // [session][pair of elements] of what a frame's steps pass on, zero at launch; above 8 sessions pairs without a number but for qkv
+  uint64_t *qkv, *meet, *x, *ao, *h, *logits;    // one allocation; meet: the barrier's count, in a line of its own
 };
 template <int NT>
 __device__ __forceinline__ void reg_put(uint64_t* base, long long i, unsigned pair, unsigned step) {
@@ -77,14 +78,16 @@ struct RegWait {
 
 // above 8 sessions: all CTAs meet; false: not within the limit
 template <bool DIAG>
-__device__ __forceinline__ bool reg_grid_sync(const DepParams& p, unsigned step, int* ok) {
+__device__ __forceinline__ bool reg_grid_sync(const DepParams& p, const RegWords& io, unsigned& meets, int* ok) {
+  meets += 1;
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned target = step * gridDim.x;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.bar) : "memory");
+    const unsigned target = meets * gridDim.x;
+    unsigned* const count = reinterpret_cast<unsigned*>(io.meet);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
     RegWait<DIAG> wait;
     int met = 1;
-    while (ld_acquire(p.bar) < target)
+    while (ld_acquire(count) < target)
       if (!wait.again(p)) { met = 0; break; }
     *ok = met;
   }
@@ -221,7 +224,7 @@ __device__ __forceinline__ void reg_stamp(const DepParams& p, unsigned step) {  
 // added up by then.  The second sub of a last odd pair is whatever its slot held before; its sums are not stored.  false: something was waited for in vain.
 template <int NT, bool DIAG>
 __device__ __forceinline__ bool reg_product(RegStream& st, const RegPart& p, const DepParams& dep, RegWait<DIAG>& wait, const uint64_t* x, unsigned step, int K, int B, bool normed,
-                                            const uint4 (&alpha)[2], float (*s_sq)[REG_WARPS], float* red, int* met) {
+                                            const uint4 (&alpha)[2], float (*s_sq)[REG_WARPS], float* red, const RegWords& io, unsigned& meets, int* met) {
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int subs = reg_subs(p), nk = (p.num_kb - warp + REG_WARPS - 1) / REG_WARPS;
   uint4 xb[NT][2];                               // of one k-block; the next one is asked for meanwhile
@@ -273,7 +276,7 @@ __device__ __forceinline__ bool reg_product(RegStream& st, const RegPart& p, con
       }
     __syncwarp();
   };
-  if (NT > 1 && !reg_grid_sync<DIAG>(dep, step, met)) return false;
+  if (NT > 1 && !reg_grid_sync<DIAG>(dep, io, meets, met)) return false;
   request(0);
   settle(0);
   if (DIAG) reg_stamp(dep, step);
@@ -411,6 +414,7 @@ __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams
   st.open();
 #pragma unroll 1
   for (uint32_t s = 0; s < REG_SLOTS; ++s) st.ask(s);
+  unsigned meets = 0;                            // barriers so far
   unsigned step = 0;                             // the last step, written or (from its first reader on) waited for
   RegWait<DIAG> wait;
   bool ok = true;
@@ -440,7 +444,7 @@ __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams
       const int m0 = pairs > 0 ? tid / pairs : 0, n0 = tid - m0 * pairs, dm = pairs > 0 ? REG_THREADS / pairs : 0, dn = REG_THREADS - dm * pairs;
       // depformer_norms is Identity (lm.py:197-198): the head reads x itself
       ok = reg_product<NT, DIAG>(st, a, p, wait, kind == REG_OUT ? io.ao : kind == REG_LINEAR_OUT ? io.h : io.x, step, kind == REG_LINEAR_OUT ? p.F : dd, B,
-                                 kind == REG_IN || kind == REG_GATE, alpha, s_sq, red, &met);
+                                 kind == REG_IN || kind == REG_GATE, alpha, s_sq, red, io, meets, &met);
       if (!ok) break;
       if (i == 0 && adds_x) {                    // the sub-step's input
         old = reg_take<NT, DIAG>(p, wait, io.x, my_x, step);
@@ -467,7 +471,7 @@ __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams
           }
           const float2 v = reg_total<NT>(red, a.units, r >> 3, m, r & 7);
           const unsigned w = reg_pair(v.x, v.y);
-          if (kind == REG_IN) reg_put<NT>(io.qkv, (long long)m * (3 * dd / 2) + n, w, step);
+          if (kind == REG_IN) reg_put<1>(io.qkv, (long long)m * (3 * dd / 2) + n, w, step);
           else if (2 * n < p.card) {
             reg_put<NT>(io.logits, (long long)m * ((p.card + 7) / 8 * 4) + n, w, step);
             bf16* to = p.logits + ((long long)k * B + m) * p.card + 2 * n;
@@ -489,23 +493,16 @@ __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams
           for (int j = 0; j < MQ; ++j)
             if (j < k) { ko[j] = kc[j * (DD / 2)]; vo[j] = vc[j * (DD / 2)]; }
         }
-        if (NT > 1 && !(ok = reg_grid_sync<DIAG>(p, step, &met))) break;
         if (some) {
           const long long src = (long long)b * (3 * C / 2) + h * (DD / 2) + lane;
-          unsigned qw, kw, vw;
-          if constexpr (NT == 1) {
-            uint64_t w[3];
-            wait.begin();
-            do {
+          uint64_t w[3];
+          wait.begin();
+          do {
 #pragma unroll
-              for (int j = 0; j < 3; ++j) w[j] = reg_get(io.qkv + src + j * (C / 2));
-            } while (!(reg_new(w[0], step) && reg_new(w[1], step) && reg_new(w[2], step)) && wait.again(p));
-            __syncwarp();
-            qw = (unsigned)w[0]; kw = (unsigned)w[1]; vw = (unsigned)w[2];
-          } else {
-            const unsigned* from = reinterpret_cast<const unsigned*>(io.qkv) + src;
-            qw = __ldcg(from); kw = __ldcg(from + C / 2); vw = __ldcg(from + C);
-          }
+            for (int j = 0; j < 3; ++j) w[j] = reg_get(io.qkv + src + j * (C / 2));
+          } while (!(reg_new(w[0], step) && reg_new(w[1], step) && reg_new(w[2], step)) && wait.again(p));
+          __syncwarp();
+          const unsigned qw = (unsigned)w[0], kw = (unsigned)w[1], vw = (unsigned)w[2];
           kc[k * (DD / 2)] = kw;
           vc[k * (DD / 2)] = vw;
           const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qw));
@@ -550,7 +547,7 @@ __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams
       else if (kind == REG_LINEAR_OUT && l + 1 < p.L) norm_of(p.n1[l + 1]);
     }
     if (!ok) break;
-    if (NT > 1 && !(ok = reg_grid_sync<DIAG>(p, step, &met))) break;
+    if (NT > 1 && !(ok = reg_grid_sync<DIAG>(p, io, meets, &met))) break;
     if (NT == 1) __syncthreads();                // red has been read: the row of logits goes there
     for (int m = blockIdx.x; m < B; m += gridDim.x) {      // the next sub-step's input rows are the same rows of the same CTA
       unsigned* row = reinterpret_cast<unsigned*>(red);
@@ -589,7 +586,9 @@ inline size_t dep_reg_smem(const DepFusedConfig& c, int grid) {
   const size_t sums = (size_t)REG_WARPS * ((dep_reg_subs(c, grid) + 1) & ~1) * REG_UNIT * (c.B <= 8 ? 10 : 18) * 4, logits = ((size_t)c.card + 1) / 2 * 4;
   return (size_t)REG_SLOTS * REG_SLOT_BYTES + REG_WARPS * REG_ASKS * sizeof(RegAsk) + ((size_t)c.dep_q * (4 * c.L + 1) * 8 + 15) / 16 * 16 + std::max(sums, logits);
 }
-inline size_t dep_reg_words(const DepFusedConfig& c) { return (size_t)c.B * (c.dd / 2 + 3 * c.dd / 2 + c.dd / 2 + c.F / 2 + (c.card + 7) / 8 * 4); }
+// words of the qkv and the barrier's, which are zeroed above 8 sessions too, and of everything
+inline size_t dep_reg_front(const DepFusedConfig& c) { return (size_t)c.B * (3 * c.dd / 2) + 16; }      // words stay on lines
+inline size_t dep_reg_words(const DepFusedConfig& c) { return dep_reg_front(c) + (size_t)c.B * (c.dd / 2 + c.dd / 2 + c.F / 2 + (c.card + 7) / 8 * 4); }
 inline bool dep_reg_takes(const DepFusedConfig& c, int grid) {
   return c.B <= REG_B && c.dd % 64 == 0 && c.dd <= REG_WARPS * 64 && c.F % 8 == 0 && c.F <= REG_KC * REG_WARPS * 64 && grid >= 1 && dep_reg_subs(c, grid) <= REG_SUBS &&
          c.B * (c.dd / DD) <= REG_WARPS * grid && dep_reg_smem(c, grid) <= SMEM_LIMIT;
