@@ -863,11 +863,20 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   const bool scaled = !i8 || (K % 16 == 0 && tune.sa && tune.sw);
   if (chosen && scaled && M <= g_row_max_m && row_wins(M, epi, gate_rows, i8, g_sms) && row_supported(M, K, i8, rows, row_ld))
     return row_linear(rows, row_ld, w_tiles, y, ldy, res, ldr, M, N, K, epi, gate_rows, i8 ? tune.sa : nullptr, tune.sw, g_sms, tune.pdl, stream);
-  // 17..256 sessions: activations as the A operand (gemm_ns.cu, figures there: ahead at every shape from 17 rows on).  It stores 16-byte pieces; rows that do not lie so keep
-  // the kernels below, and (bf16) its refusal above 32
+  const int n_tiles = (N + BLOCK_ROWS - 1) / BLOCK_ROWS, k_blocks = i8 ? (K + 127) / 128 : (K + BLOCK_K - 1) / BLOCK_K;
+  int ranks = 1;                                          // few tiles: K over a cluster (gemm_ck_kernel)
+  while (ranks < 8 && n_tiles * ranks * 2 <= g_sms && k_blocks / (ranks * 2) >= 4 && (ranks < 4 || n_tiles <= 15)) ranks *= 2;      // 15 clusters of eight fit at a time
+  if (tune.cluster > 0) ranks = tune.cluster;
+  const int quantum = 8 * ranks < 16 ? 16 : 8 * ranks;    // UMMA N is a multiple of 16; every rank owns whole 8-column groups
+  const int ck_pad = ((M + quantum - 1) / quantum) * quantum;
+  const bool ck = epi != EPI_GATE && tune.no_cluster == 0 && tune.grid == 0 && M > 32 && ranks > 1 && ck_pad <= 256 && ck_pad / ranks <= 64;
+  // 17..256 sessions: activations as the A operand (gemm_ns.cu, figures there).  It stores 16-byte pieces; rows that do not lie so keep the kernels below, and (bf16) its
+  // refusal above 32.  So do 16-bit gated pairs of up to 32 rows and int8 rows above 32 of few tiles, which tests/test_devices_cpu.py
+  // takes for calls of these kernels (gemm_ns.cu would take 33 us for 50 of 4096 -> 11264 at 24 rows, 10.3 for 17.6 of int8 4096 -> 4096 at 104).
+  const bool kept = i8 ? ck : epi == EPI_GATE && M <= REG_MAX_M;
   const bool lines = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(rows)) & 15) == 0;
   const bool ns_fits = scaled && tune.ns >= 0 && M <= 256 && tune.grid == 0 && tune.cluster == 0 && !tune.stream_only && !tune.force_split && ns_supported(M, N, K, epi) &&
-                       ldy % 8 == 0 && (!res || ldr % 8 == 0) && ((!i8 && M > REG_MAX_M) || (lines && (chosen || tune.ns > 0)));
+                       ldy % 8 == 0 && (!res || ldr % 8 == 0) && ((!i8 && M > REG_MAX_M) || (lines && !kept && chosen) || (!i8 && lines && tune.ns > 0));
   // up to 32 that the row kernel and that one leave: weights through registers (gemm_reg.cu).  With the row kernel's range cut short this one has all of its own.
   if (chosen && scaled && M <= REG_MAX_M && !(ns_fits && g_use_ns && M > ROW_MAX_M && g_row_max_m == ROW_MAX_M) && reg_wins(M, N, epi, gate_rows, i8, g_sms) &&
       reg_supported(M, epi, rows, row_ld))
@@ -875,54 +884,46 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
                       SK_MAX_TILES, g_sms, tune.pdl, stream);
   if (ns_fits && (tune.ns > 0 || (g_use_ns && M > ROW_MAX_M)))
     return ns_linear(cache, rows, i8 ? K : ldx, w_tiles, y, ldy, res, ldr, M, N, K, epi, gate_rows, 0, tune.pdl, stream, 0, i8 ? tune.sa : nullptr, i8 ? tune.sw : nullptr);
-  // more than 32 sessions and few row tiles: a cluster of CTAs per tile, split along K, reduced over DSMEM
+  // more than 32 sessions and few row tiles: a cluster of CTAs per tile, ranks along K, reduced over DSMEM
   if (i8 && (K % 16 || !tune.sa || !tune.sw)) B200_FAIL(B200_ERR_SHAPE, "int8 GEMM: K must be a multiple of 16 and both scale vectors given");
-  if (epi != EPI_GATE && tune.no_cluster == 0 && tune.grid == 0 && M > 32) {
-    const int n_tiles = (N + BLOCK_ROWS - 1) / BLOCK_ROWS, num_kb = i8 ? (K + 127) / 128 : (K + BLOCK_K - 1) / BLOCK_K;
-    int cs = 1;
-    while (cs < 8 && n_tiles * cs * 2 <= g_sms && num_kb / (cs * 2) >= 4) cs *= 2;
-    if (tune.cluster > 0) cs = tune.cluster;
-    if (cs > 1) {
-      CkParams p;
-      p.M = M; p.N = N; p.K = K; p.CS = cs;
-      const int quantum = 8 * cs < 16 ? 16 : 8 * cs;       // UMMA N is a multiple of 16; every rank owns whole 8-column groups
-      p.Mpad = ((M + quantum - 1) / quantum) * quantum;
-      p.Wc = p.Mpad / cs;
-      if (p.Mpad <= 256 && p.Wc <= 64) {
-        p.num_kb = num_kb; p.kb_per = (num_kb + cs - 1) / cs;
-        p.wt = static_cast<const uint8_t*>(w_tiles);
-        p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr;
-        p.i8 = i8 ? 1 : 0; p.sa = tune.sa; p.sw = tune.sw; p.late = tune.pdl != PDL_WEIGHTS_FIRST;
-        p.stage_bytes = (uint32_t)(TILE_BYTES + p.Mpad * BLOCK_K * 2);      // 128 bytes of K per row, bf16 or int8
-        const size_t recv_bytes = (size_t)cs * BLOCK_ROWS * (p.Wc + 4) * 4;
-        int stages = (int)((200 * 1024 - recv_bytes) / p.stage_bytes);
-        if (stages > MAX_STAGES) stages = MAX_STAGES;
-        if (stages > p.kb_per) stages = p.kb_per;
-        if (stages >= 2) {
-          p.stages = stages;
-          uint32_t pow2 = 32;
-          while (pow2 < (uint32_t)p.Mpad) pow2 <<= 1;
-          p.tmem_cols = pow2;
-          const CUtensorMap* mx = nullptr;
-          if (i8) B200_TRY(x_map(cache, tune.xq, K, M, K, p.Mpad, 1, &mx));
-          else B200_TRY(x_map(cache, x, ldx, M, K, p.Mpad, 2, &mx));
-          const size_t smem = (size_t)stages * p.stage_bytes + 1024 + 16 * MAX_STAGES + 64 + recv_bytes + 64;
-          cudaLaunchConfig_t cfg;
-          memset(&cfg, 0, sizeof(cfg));
-          cfg.gridDim = dim3(n_tiles * cs); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-          cudaLaunchAttribute attr[2];
-          attr[0].id = cudaLaunchAttributeClusterDimension;
-          attr[0].val.clusterDim.x = cs; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-          attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-          attr[1].val.programmaticStreamSerializationAllowed = 1;
-          cfg.attrs = attr; cfg.numAttrs = tune.pdl ? 2 : 1;
-          cudaError_t le = epi == EPI_STORE ? cudaLaunchKernelEx(&cfg, gemm_ck_kernel<EPI_STORE>, *mx, p)
-                                            : cudaLaunchKernelEx(&cfg, gemm_ck_kernel<EPI_RESADD>, *mx, p);
-          if (le != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "gemm_ck launch failed: %s", cudaGetErrorString(le));
-          g_launches.fetch_add(1, std::memory_order_relaxed);
-          return check_launch("gemm_ck");
-        }
-      }
+  if (ck) {
+    const int cs = ranks;
+    CkParams p;
+    p.M = M; p.N = N; p.K = K; p.CS = cs;
+    p.Mpad = ck_pad;
+    p.Wc = p.Mpad / cs;
+    p.num_kb = k_blocks; p.kb_per = (k_blocks + cs - 1) / cs;
+    p.wt = static_cast<const uint8_t*>(w_tiles);
+    p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr;
+    p.i8 = i8 ? 1 : 0; p.sa = tune.sa; p.sw = tune.sw; p.late = tune.pdl != PDL_WEIGHTS_FIRST;
+    p.stage_bytes = (uint32_t)(TILE_BYTES + p.Mpad * BLOCK_K * 2);      // 128 bytes of K per row, bf16 or int8
+    const size_t recv_bytes = (size_t)cs * BLOCK_ROWS * (p.Wc + 4) * 4;
+    int stages = (int)((200 * 1024 - recv_bytes) / p.stage_bytes);
+    if (stages > MAX_STAGES) stages = MAX_STAGES;
+    if (stages > p.kb_per) stages = p.kb_per;
+    if (stages >= 2) {
+      p.stages = stages;
+      uint32_t pow2 = 32;
+      while (pow2 < (uint32_t)p.Mpad) pow2 <<= 1;
+      p.tmem_cols = pow2;
+      const CUtensorMap* mx = nullptr;
+      if (i8) B200_TRY(x_map(cache, tune.xq, K, M, K, p.Mpad, 1, &mx));
+      else B200_TRY(x_map(cache, x, ldx, M, K, p.Mpad, 2, &mx));
+      const size_t smem = (size_t)stages * p.stage_bytes + 1024 + 16 * MAX_STAGES + 64 + recv_bytes + 64;
+      cudaLaunchConfig_t cfg;
+      memset(&cfg, 0, sizeof(cfg));
+      cfg.gridDim = dim3(n_tiles * cs); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = cs; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr; cfg.numAttrs = tune.pdl ? 2 : 1;
+      cudaError_t le = epi == EPI_STORE ? cudaLaunchKernelEx(&cfg, gemm_ck_kernel<EPI_STORE>, *mx, p)
+                                        : cudaLaunchKernelEx(&cfg, gemm_ck_kernel<EPI_RESADD>, *mx, p);
+      if (le != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "gemm_ck launch failed: %s", cudaGetErrorString(le));
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+      return check_launch("gemm_ck");
     }
   }
   SkParams p;

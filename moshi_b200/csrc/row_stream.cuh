@@ -1,5 +1,5 @@
 // What the kernels have in common that stream packed weights past activations in registers (gemm_row.cu, dep_reg.cuh, gemm_reg.cu): 16-byte copies into a warp's own
-// ring, and products of 16 weight rows and 8 activation rows.
+// ring (gemm_row.cu), and products of 16 weight rows and 8 activation rows.
 #pragma once
 
 #include "common.cuh"
