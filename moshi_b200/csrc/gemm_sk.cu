@@ -871,9 +871,9 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   const int ck_pad = ((M + quantum - 1) / quantum) * quantum;
   const bool ck = epi != EPI_GATE && tune.no_cluster == 0 && tune.grid == 0 && M > 32 && ranks > 1 && ck_pad <= 256 && ck_pad / ranks <= 64;
   // 17..256 sessions: activations as the A operand (gemm_ns.cu, figures there).  It stores 16-byte pieces; rows that do not lie so keep the kernels below, and (bf16) its
-  // refusal above 32.  So do 16-bit gated pairs of up to 32 rows and int8 rows above 32 of few tiles, which tests/test_devices_cpu.py
-  // takes for calls of these kernels (gemm_ns.cu would take 33 us for 50 of 4096 -> 11264 at 24 rows, 10.3 for 17.6 of int8 4096 -> 4096 at 104).
-  const bool kept = i8 ? ck : epi == EPI_GATE && M <= REG_MAX_M;
+  // refusal above 32.  Up to 32 rows it takes k of 4096 on, where it gains most (24 rows: 4096 -> 12288 28.0 us / 19.9, int8 11264 -> 4096 18.3 / 11.0; of 2048 it would gain 2 to 4);
+  // 16-bit gated pairs of as many rows, shorter k and int8 rows above 32 of few tiles are left with the kernels that tests/test_devices_cpu.py and tests/test_op_routes_cpu.py name.
+  const bool kept = (M <= REG_MAX_M && (K < 4096 || (!i8 && epi == EPI_GATE))) || (i8 && ck);
   const bool lines = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(rows)) & 15) == 0;
   const bool ns_fits = scaled && tune.ns >= 0 && M <= 256 && tune.grid == 0 && tune.cluster == 0 && !tune.stream_only && !tune.force_split && ns_supported(M, N, K, epi) &&
                        ldy % 8 == 0 && (!res || ldr % 8 == 0) && ((!i8 && M > REG_MAX_M) || (lines && !kept && chosen) || (!i8 && lines && tune.ns > 0));
