@@ -651,6 +651,9 @@ int b200_op_attn_step_q8(const void* qkv_dev, void* k8_dev, void* v8_dev, float*
  * 64, 128, .., 512 elements take the mma kernel (as in the handle); 0: always the CUDA-core kernel.  Synchronises (test helper). */
 int b200_op_latent_attention(const float* qa_dev, const void* latents_dev, int dtype, const float* sink_dev, float* out_dev,
                              int T, int H, int r, int pos0, int nsplit, int tensor_cores, void* stream);
+/* The decoder LM's latents of T new tokens: latents[t] = raw / sqrt(mean(raw^2) + eps) * weight, raw = the r elements from `off` on of rows[t][ld].  The squares are
+ * summed up lane by lane (a lane has every 32nd element), the lanes by halves: the same bits wherever the rows begin.  Pointers on 16 bytes.  Synchronises (test helper). */
+int b200_op_latent_append(const void* rows_dev, int dtype, int ld, int off, const float* weight_dev, void* latents_dev, int T, int r, float eps, void* stream);
 /* The decoder LM's attention of a long portion (csrc/dlm_flash.cu) for one request: q bf16 [T][H * 128], k [pos0 + T][H * 128], vt the values
  * transposed, [H * 128][ldv] with a column per key (ldv a multiple of 8), sink f32 [H] or NULL; query t sits at position pos0 + t and sees keys
  * 0 .. pos0 + t; out bf16 [T][H * 128].  Enqueues on the stream. */

@@ -164,6 +164,7 @@ _PROTOTYPES: dict[str, tuple[tp.Any, list]] = {
     "b200_op_pack_tiles": (_I, [_P, _P, _I, _I, _I, _I, _P]),
     "b200_op_linear_sk": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P]),
     "b200_op_linear_wide": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),
+    "b200_op_latent_append": (_I, [_P, _I, _I, _I, _P, _P, _I, _I, C.c_float, _P]),
     "b200_op_prefill_attention": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, C.c_float, _P]),
     "b200_op_grouped_wide": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, C.c_float, _P]),
     "b200_op_linear_reg": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P]),

@@ -3377,4 +3377,32 @@ int b200_op_latent_attention(const float* qa_dev, const void* latents_dev, int d
   return rc;
 }
 
+int b200_op_latent_append(const void* rows_dev, int dtype, int ld, int off, const float* weight_dev, void* latents_dev, int T, int r, float eps, void* stream) {
+  if (!rows_dev || !weight_dev || !latents_dev) B200_FAIL(B200_ERR_INVALID, "op_latent_append: null pointer");
+  if (T < 1 || r < 1 || off < 0 || ld < off + r) B200_FAIL(B200_ERR_SHAPE, "op_latent_append: bad shape");
+  if (dtype != B200_F32 && dtype != B200_BF16) B200_FAIL(B200_ERR_INVALID, "op_latent_append: rows must be f32 or bf16");
+  if ((reinterpret_cast<uintptr_t>(rows_dev) | reinterpret_cast<uintptr_t>(weight_dev) | reinterpret_cast<uintptr_t>(latents_dev)) & 15)
+    B200_FAIL(B200_ERR_INVALID, "op_latent_append: pointers must be 16-byte aligned");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  std::vector<int> meta((size_t)2 * T, 0);      // slot 0; positions
+  for (int t = 0; t < T; ++t) meta[T + t] = t;
+  int* meta_dev = nullptr;
+  B200_CUDA(cudaMalloc(&meta_dev, meta.size() * sizeof(int)));
+  cudaError_t e = cudaMemcpyAsync(meta_dev, meta.data(), meta.size() * sizeof(int), cudaMemcpyHostToDevice, st);
+  int rc = B200_OK;
+  if (e == cudaSuccess) {
+    if (dtype == B200_F32)
+      B200_LAUNCH(latent_append_kernel<float>, ceil_div(T, 4), 128, 0, st, static_cast<const float*>(rows_dev), (long long)ld, off, weight_dev, static_cast<float*>(latents_dev), T, r, meta_dev,
+                  meta_dev + T, T, eps);
+    else
+      B200_LAUNCH(latent_append_kernel<bf16>, ceil_div(T, 4), 128, 0, st, static_cast<const bf16*>(rows_dev), (long long)ld, off, weight_dev, static_cast<bf16*>(latents_dev), T, r, meta_dev,
+                  meta_dev + T, T, eps);
+    rc = check_launch("op_latent_append");
+    e = cudaStreamSynchronize(st);
+  }
+  cudaFree(meta_dev);
+  if (rc == B200_OK && e != cudaSuccess) { set_error("op_latent_append: %s", cudaGetErrorString(e)); rc = B200_ERR_CUDA; }
+  return rc;
+}
+
 }  // extern "C"

@@ -1,9 +1,12 @@
 """GPU: the decoder LMs' small kernels by rows: latents appended in runs of eight (ranks of 256 to 1024), projections to fp32 with four tokens to a CTA from 512 tokens on."""
+import ctypes as C
+
 import pytest
 import torch
 
 from .test_gpu_zz_decoder_lm import assert_close, build, gen_for, layer, make_cfg, tokens
 from . import test_gpu_zzzzzz_megolorn as megolorn
+from .util import cptr
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +35,26 @@ def test_small_projections(experts, width, n):
     with gen_for(model, capacity=1024, max_step_tokens=1024) as gen:
         got = gen.step([(0, toks)], list(range(n))).cpu()
     megolorn.assert_close(got, orc.forward(toks), torch.float32)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("off", [0, 8, 4])
+@pytest.mark.parametrize("rank", [32, 250, 256, 512, 768, 1024, 1280])
+def test_bits_of_latents(rank, off, dtype):
+    """Runs of eight or single elements, the same bits: the squares in one order (every lane each 32nd element by fused additions, then the lanes by halves)."""
+    from moshi_b200 import _lib
+    T, eps = 131, 1e-5
+    g = torch.Generator().manual_seed(rank + off)
+    rows = torch.randn(T, off + (rank + 7) // 8 * 8 + 8, generator=g).bfloat16().to(dtype).cuda()      # squares of 16 bits: with a sum of 24 exact in 64
+    weight = (1 + 0.1 * torch.randn(rank, generator=g)).cuda()
+    out = torch.empty(T, rank, dtype=dtype, device="cuda")
+    _lib.check(_lib.lib().b200_op_latent_append(cptr(rows), _lib.dtype_code(dtype), rows.shape[1], off, cptr(weight), cptr(out), T, rank, eps, C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    raw = rows[:, off:off + rank].float()
+    lanes = torch.nn.functional.pad(raw, (0, -rank % 32)).view(T, -1, 32)
+    s = torch.zeros(T, 32, device="cuda")
+    for i in range(lanes.shape[1]):
+        s = (lanes[:, i].double() ** 2 + s.double()).float()
+    for o in (16, 8, 4, 2, 1):
+        s = s + s[:, torch.arange(32, device="cuda") ^ o]
+    rs = 1.0 / torch.sqrt(s[:, :1] / torch.full((T, 1), float(rank), device="cuda") + torch.tensor(eps, device="cuda"))      # by a number torch would multiply with its inverse
+    assert torch.equal(out, (raw * rs * weight).to(dtype))
