@@ -386,7 +386,8 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
     }
     if (p.CS > 1) {
       __syncwarp();
-      ns_cluster_meet();                        // the block's sums have been read everywhere
+      if (mb + 1 < p.mblocks) ns_cluster_sync();      // the block's sums have been read everywhere, before the next block's take their place
+      else ns_cluster_meet();                   // nobody leaves while its sums are read
     }
   }
   __syncthreads();

@@ -44,3 +44,26 @@ def test_linear_ns(M, N, K, epi, cluster):
         want, err = z, err + 2.0 ** -8 * z.abs()
     assert bool(((y[:M].double() - want).abs() <= err + 1e-30).all())
     assert (y[M] == 7.0).all()
+
+
+@pytest.mark.parametrize("M", [128, 129, 200, 256])
+@pytest.mark.parametrize("N,K,epi,cluster", [(4096, 4096, RESIDUAL, 0), (4096, 1024, STORE, 0), (2056, 520, RESIDUAL, 0), (640, 1024, STORE, 8), (648, 576, RESIDUAL, 102), (640, 1024, STORE, 108)])
+def test_blocks_of_sessions_one_after_the_other(M, N, K, epi, cluster):
+    """Two blocks of 128 sessions pass their sums through the same shared memory of a cluster: the second may overwrite what its neighbours have read.  Small whole numbers, whose
+    sums are exact in whatever order they are added: the bits of the plain computation, launch after launch."""
+    from moshi_b200 import _lib
+    lib = _lib.lib()
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randint(-8, 9, (M, K), generator=g).bfloat16().cuda()
+    w = torch.randint(-8, 9, (N, K), generator=g).bfloat16().cuda()
+    res = torch.randn(M, N, generator=g).bfloat16().cuda() if epi == RESIDUAL else None
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    wt = torch.empty(lib.b200_op_packed_bytes(N, K, epi, 0), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.b200_op_pack_tiles(cptr(w), cptr(wt), N, K, epi, 0, stream))
+    y = torch.full((12, M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    for i in range(12):
+        _lib.check(lib.b200_op_linear_ns(cptr(x), cptr(wt), cptr(y[i]), cptr(res), M, N, K, epi, 0, cluster, stream))
+    want = (x.double() @ w.double().t()).bfloat16()          # below 2^24: what fp32 holds exactly, rounded once
+    if res is not None:
+        want = (res.float() + want.float()).bfloat16()
+    assert all(torch.equal(y[i], want) for i in range(12))
