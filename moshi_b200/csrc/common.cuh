@@ -159,23 +159,33 @@ struct DeviceGuard {
   ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
 
-// Raises the limit of dynamic shared memory of kernels.  The limit belongs to a kernel on one device, and a process may drive several: it is set once on each device
-// that is current at a call, and again where it could not be set.  `done`: a static of the caller's, for this group of kernels.
+// Sets an attribute of kernels.  It belongs to a kernel on one device, and a process may drive several: it is set once on each device that is current at a call, and again
+// where it could not be set.  `done`: a static of the caller's, for this group of kernels.
 template <typename... Kernels>
-int allow_smem(std::atomic<uint64_t>& done, int bytes, Kernels*... kernels) {
+int kernel_attribute(std::atomic<uint64_t>& done, cudaFuncAttribute attribute, int value, const char* what, Kernels*... kernels) {
   int dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
   const uint64_t bit = dev < 64 ? 1ull << dev : 0;
   if (done.load(std::memory_order_acquire) & bit) return B200_OK;
   for (const void* k : {reinterpret_cast<const void*>(kernels)...}) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const cudaError_t e = cudaFuncSetAttribute(k, attribute, value);
     if (e == cudaSuccess) continue;
     cudaGetLastError();                          // reported here, and not by the next launch as well
-    set_error("%d bytes of shared memory refused on device %d: %s", bytes, dev, cudaGetErrorString(e));
+    set_error("%d %s refused on device %d: %s", value, what, dev, cudaGetErrorString(e));
     return B200_ERR_CUDA;
   }
   done.fetch_or(bit, std::memory_order_release);
   return B200_OK;
+}
+// the limit of dynamic shared memory
+template <typename... Kernels>
+int allow_smem(std::atomic<uint64_t>& done, int bytes, Kernels*... kernels) {
+  return kernel_attribute(done, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes, "bytes of shared memory", kernels...);
+}
+// How much of an SM's L1 is shared memory while the kernel runs there, in percent.  Left to the driver it is what the SM had before if that is enough.
+template <typename... Kernels>
+int prefer_smem(std::atomic<uint64_t>& done, int percent, Kernels*... kernels) {
+  return kernel_attribute(done, cudaFuncAttributePreferredSharedMemoryCarveout, percent, "percent of shared memory", kernels...);
 }
 
 // shared body of b200_{lm,mimi}_state_{count,entry,read,write}

@@ -273,7 +273,7 @@ int step_body(b200_lm* h) {
       a.pos = h->pos; a.exec_mask = h->exec_mask_m; a.H = H; a.cap = ring_cap(h); a.nsplit = h->nsplit; a.min_per = h->attn_min_per;
       a.neg_log_period_2_over_d = nl;
       dim3 grid(MB * H, h->nsplit);
-      B200_TRY(launch_early_if(h->pdl != 0, attn_group_keys() == 2 ? attn_step_kernel<2> : attn_step_kernel<4>, grid, dim3(ATT_THREADS), 0, st, a));
+      B200_TRY(attn_step_launch(a, grid, h->pdl != 0, st));
     }
     B200_TRY(linear(h, h->ao, d, L.out_w, h->x, d, h->x, d, MB, d, d, LIN_RESADD, 0, L.out_s));
     B200_TRY(norm_linear(h, h->x, L.n2, h->xn, L.lin_in, h->hbuf, F, MB, F, d, LIN_GATE, F, L.lin_in_s));

@@ -528,6 +528,18 @@ static __global__ void __launch_bounds__(ATT_THREADS) attn_step_kernel(const Att
   a.out[(long long)bh * ATT_D + tid] = f2bf(LL > 0.f ? AA / LL : 0.f);
 }
 
+// What an SM has on the way from the ring lies in its L1: four CTAs' two groups of keys and values, 128 KB.  An SM that a linear has just left has 228 of its 256 KB as shared
+// memory, and where a kernel names no preference the SM stays like that if it is enough for it.  So the attention asks for a quarter, which holds the CTAs' 21 KB.  Layers of 104
+// sessions with rings of 3000, from the end of in_proj to the end of the attention: 786 us as the SMs were, 719 with a quarter; 720 as they were with an in_proj of fewer registers, beside
+// which CTAs of the attention were at home earlier.  A step of the 7B, ms, as they were / a quarter: 1 and 16 sessions the same, 24 sessions 9.33 / 8.78, 48
+// 11.70 / 10.73, 64 13.44 / 12.33, 104 (full rings) 31.95 / 29.83.
+constexpr int ATT_SMEM_PERCENT = 25;
+static int attn_step_launch(const AttnStep& a, dim3 grid, bool early, cudaStream_t st) {
+  static std::atomic<uint64_t> set{0};
+  B200_TRY(prefer_smem(set, ATT_SMEM_PERCENT, attn_step_kernel<2>, attn_step_kernel<4>));
+  return launch_early_if(early, attn_group_keys() == 2 ? attn_step_kernel<2> : attn_step_kernel<4>, grid, dim3(ATT_THREADS), 0, st, a);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Opt-in 8-bit KV rings (NOT the reference's numerics): the same fused step as attn_step_kernel
 // over rings of one byte per element with one fp32 scale per (session, head, slot).  Halves the ring (0.81 GB instead

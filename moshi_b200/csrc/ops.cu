@@ -213,7 +213,7 @@ int b200_op_attn_step(const void* qkv_dev, void* k_dev, void* v_dev, void* out_d
   a.neg_log_period_2_over_d = -logf(max_period) * 2.f / (float)ATT_D;
   dim3 grid(B * H, nsplit);
   a.late = 1;
-  B200_TRY(launch_early_if(op_pdl() != 0, attn_group_keys() == 2 ? attn_step_kernel<2> : attn_step_kernel<4>, grid, dim3(ATT_THREADS), 0, st, a));
+  B200_TRY(attn_step_launch(a, grid, op_pdl() != 0, st));
   return check_launch("op_attn_step");
 }
 

@@ -19,9 +19,10 @@ thread_local int device = 0;
 thread_local cudaError_t last = cudaSuccess;
 std::map<const void*, std::string>& names() { static std::map<const void*, std::string> m; return m; }
 std::map<std::pair<const void*, int>, size_t> limits;
+std::map<std::pair<const void*, int>, int> shares;      // of an SM's L1 that a kernel asks for as shared memory, in percent
 std::map<void*, std::pair<int, size_t>> blocks;
 size_t held[DEVICES];
-int attributes_to_refuse = 0;
+int attributes_to_refuse = 0, last_share = cudaSharedmemCarveoutDefault;
 std::string launches;
 struct Call { dim3 grid, block; size_t smem; cudaStream_t stream; };
 thread_local std::vector<Call> calls;
@@ -34,6 +35,8 @@ cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t smem) {
   std::lock_guard<std::recursive_mutex> g(mu);
   const auto it = limits.find({f, device});
   if (smem > (it == limits.end() ? DEFAULT_SMEM : it->second) || grid.x == 0 || block.x * block.y * block.z > 1024) return done(cudaErrorInvalidValue);
+  const auto share = shares.find({f, device});
+  last_share = share == shares.end() ? cudaSharedmemCarveoutDefault : share->second;
   launches += std::to_string(device) + " " + names()[f] + " " + std::to_string(grid.x * grid.y * grid.z) + "\n";
   return cudaSuccess;
 }
@@ -66,6 +69,7 @@ extern "C" {
 // ---- what a test asks and sets ----
 const char* fake_launches() { return launches.c_str(); }      // "device kernel blocks" per line, since the last fake_clear
 void fake_clear() { launches.clear(); }
+int fake_share() { return last_share; }                        // the last launch's
 size_t fake_held(int dev) { return held[dev]; }
 void fake_refuse_attributes(int n) { attributes_to_refuse = n; }
 
@@ -87,6 +91,7 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   std::lock_guard<std::recursive_mutex> g(mu);
   if (attributes_to_refuse > 0) { --attributes_to_refuse; return done(cudaErrorInvalidValue); }
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) limits[{f, device}] = v;
+  if (a == cudaFuncAttributePreferredSharedMemoryCarveout) shares[{f, device}] = v;
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t smem, unsigned) { *n = smem <= MOST_SMEM ? 1 : 0; return cudaSuccess; }

@@ -93,3 +93,13 @@ def test_workspaces_lie_on_the_device_of_the_call(fake, call, larger):
             assert (most := fake.fake_held(dev)) > once
             fake_cuda.check(fake, call(fake))
             assert fake.fake_held(dev) == most
+
+
+@pytest.mark.parametrize("sessions", [1, 104])
+def test_the_attention_says_how_much_l1_it_wants(fake, sessions):
+    """On every device: the ring's keys and values on their way need most of an SM's L1, whose division a kernel without a preference takes over from the linear in front of it."""
+    for dev in (0, 1):
+        fake.cudaSetDevice(dev)
+        fake_cuda.check(fake, _attention(fake, sessions, False))
+        assert "attn_step_kernel" in fake_cuda.launches(fake)[-1][1]
+        assert 10 <= fake.fake_share() <= 50            # four CTAs' shared memory, and room for what they have under way
