@@ -519,9 +519,10 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(fn);
   // one limit for every handle: a kernel has one, and a handle that set its own need would take a larger one's away
   static std::atomic<uint64_t> limits{0};
-  B200_TRY(allow_smem(limits, SMEM_LIMIT, dep_fused_kernel, dep_reg_pick(1, 8, false), dep_reg_pick(1, 8, true), dep_reg_pick(1, lm::DEP_MAX_Q, false),
-                      dep_reg_pick(1, lm::DEP_MAX_Q, true), dep_reg_pick(REG_B, 8, false), dep_reg_pick(REG_B, 8, true), dep_reg_pick(REG_B, lm::DEP_MAX_Q, false),
-                      dep_reg_pick(REG_B, lm::DEP_MAX_Q, true)));
+  constexpr int Q = lm::DEP_MAX_Q;
+  B200_TRY(allow_smem(limits, SMEM_LIMIT, dep_fused_kernel, dep_reg_pick(1, 8, false, false), dep_reg_pick(1, 8, true, false), dep_reg_pick(1, Q, false, false), dep_reg_pick(1, Q, true, false),
+                      dep_reg_pick(REG_B, 8, false, false), dep_reg_pick(REG_B, 8, true, false), dep_reg_pick(REG_B, Q, false, false), dep_reg_pick(REG_B, Q, true, false),
+                      dep_reg_pick(1, Q, false, true), dep_reg_pick(1, Q, true, true), dep_reg_pick(REG_B, Q, false, true), dep_reg_pick(REG_B, Q, true, true)));
   DepFused* d = new DepFused();
   DepParams& p = d->p;
   memset(&p, 0, sizeof(p));
@@ -542,9 +543,12 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   p.g_lin_in = plan(c.F, c.dd, 2, c.B, d->grid);
   p.g_lin_out = plan(c.dd, c.F, 1, c.B, d->grid);
   p.g_head = plan(c.card, c.dd, 1, c.B, d->grid);
+  const bool few = dep_reg_takes(c, d->grid);
+  bool far = false;               // dep_reg_kernel reads its weights' addresses from memory
+  if (few) d->smem = dep_reg_smem(c, d->grid, &far);
   // pointer tables -> one device allocation
   const size_t n_w = (size_t)c.dep_q * c.L;
-  const size_t bytes = n_w * sizeof(DepLayerW) + (size_t)c.dep_q * 8 * 2 + (size_t)c.L * 8 * 4;
+  const size_t bytes = n_w * sizeof(DepLayerW) + (size_t)c.dep_q * 8 * 2 + (size_t)c.L * 8 * 4 + (far ? dep_reg_addresses(c) : 0);
   std::vector<uint8_t> host(bytes);
   uint8_t* hp = host.data();
   size_t off = 0;
@@ -558,6 +562,11 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   const size_t o_n2 = put(c.n2, (size_t)c.L * 8);
   const size_t o_kc = put(c.kc, (size_t)c.L * 8);
   const size_t o_vc = put(c.vc, (size_t)c.L * 8);
+  const size_t o_frame = off;     // four a layer and the head, sub-step after sub-step
+  for (int k = 0; far && k < c.dep_q; ++k) {
+    put(&w[(size_t)k * c.L], c.L * sizeof(DepLayerW));
+    put(&c.heads[k], 8);
+  }
   if (cudaMalloc(&d->dev_tables, bytes) != cudaSuccess) { delete d; B200_FAIL(B200_ERR_CUDA, "fused depformer: cudaMalloc failed"); }
   B200_CUDA(cudaMemcpy(d->dev_tables, hp, bytes, cudaMemcpyHostToDevice));
   uint8_t* dv = static_cast<uint8_t*>(d->dev_tables);
@@ -582,10 +591,10 @@ int dep_fused_create(const DepFusedConfig& c, DepFused** out) {
   B200_TRY(make_map(enc, &d->map_ao, c.ao, c.B, c.dd, p.Mpad));
   B200_TRY(make_map(enc, &d->map_h, c.hbuf, c.B, c.F, p.Mpad));
   B200_TRY(make_map(enc, &d->map_x, c.x, c.B, c.dd, p.Mpad));
-  d->smem = (size_t)stages * p.stage_bytes + 1024 + 16 * MAX_STAGES + 64;
-  if (dep_reg_takes(c, d->grid)) {
-    d->reg = dep_reg_pick(c.B, c.dep_q, c.trace || c.wait_ns > 0);
-    d->smem = dep_reg_smem(c, d->grid);
+  if (!few) d->smem = (size_t)stages * p.stage_bytes + 1024 + 16 * MAX_STAGES + 64;
+  if (few) {
+    d->reg = dep_reg_pick(c.B, c.dep_q, c.trace || c.wait_ns > 0, far);
+    d->io.w = far ? reinterpret_cast<const uint8_t* const*>(dv + o_frame) : nullptr;
     uint64_t* io = nullptr;
     if (cudaMalloc(&io, dep_reg_words(c) * REG_WORD) != cudaSuccess) { dep_fused_destroy(d); B200_FAIL(B200_ERR_CUDA, "fused depformer: cudaMalloc failed"); }
     d->io_bytes = (c.B <= 8 ? dep_reg_words(c) : dep_reg_front(c)) * REG_WORD;

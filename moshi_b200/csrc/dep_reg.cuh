@@ -38,6 +38,7 @@ enum { REG_IN = 0, REG_OUT = 1, REG_GATE = 2, REG_LINEAR_OUT = 3, REG_HEAD = 4, 
 constexpr int REG_WORD = 8;
 struct RegWords {                                // [session][pair of elements] of what a frame's steps pass on, zero at launch; above 8 sessions pairs without a number but for qkv
   uint64_t *qkv, *meet, *x, *ao, *h, *logits;    // one allocation; meet: the barrier's count, in a line of its own
+  const uint8_t* const* w;                       // addresses of the frame's weights, four a layer and the head, sub-step after sub-step (null: they lie in shared memory)
 };
 template <int NT>
 __device__ __forceinline__ void reg_put(uint64_t* base, long long i, unsigned pair, unsigned step) {
@@ -375,7 +376,7 @@ __device__ __forceinline__ void reg_input(const DepParams& p, uint64_t* x, int k
   }
 }
 
-template <int NT, int MQ, bool DIAG>      // MQ: sub-steps at most
+template <int NT, int MQ, bool DIAG, bool FAR>      // MQ: sub-steps at most; FAR: the addresses of the weights are read from memory
 __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams p, const RegWords io) {
   extern __shared__ __align__(128) uint8_t reg_smem[];
   __shared__ int met;
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams
   __shared__ __align__(16) float s_sq[8 * NT][REG_WARPS];
   __shared__ __align__(8) uint64_t ring_bars[REG_WARPS][REG_SLOTS];
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, t = lane & 3, B = p.B, dd = p.dd;
-  const int per = 4 * p.L + 1, n_w = p.dep_q * per;
+  const int per = 4 * p.L + 1, n_w = FAR ? 0 : p.dep_q * per;
   const uint8_t** weights = reinterpret_cast<const uint8_t**>(reg_smem + REG_SLOTS * REG_SLOT_BYTES + REG_WARPS * REG_ASKS * sizeof(RegAsk));
   float* red = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(weights) + ((size_t)n_w * 8 + 15) / 16 * 16);
   for (int i = tid; i < n_w; i += REG_THREADS) {
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams
   int layer_asks = 0, n_asks = 0;
   if (lane == 0) n_asks = RegStream::list(parts, warp, asks, &layer_asks);
   RegStream st;
-  st.w = weights; st.asks = asks; st.L = p.L; st.per = per;
+  st.w = FAR ? io.w : weights; st.asks = asks; st.L = p.L; st.per = per;
   st.layer_n = __shfl_sync(0xffffffffu, layer_asks, 0); st.n = __shfl_sync(0xffffffffu, n_asks, 0); st.steps = st.n > 0 ? p.dep_q : 0;
   st.ring = smem_u32(reg_smem) + warp * 2 * REG_UNIT_BYTES; st.bars = smem_u32(ring_bars[warp]);
   st.open();
@@ -572,24 +573,37 @@ __global__ void __launch_bounds__(REG_THREADS, 1) dep_reg_kernel(const DepParams
 }
 
 typedef void (*DepRegKernel)(const DepParams, const RegWords);
-template <int NT, int MQ> inline DepRegKernel dep_reg_pick(bool diag) { return diag ? dep_reg_kernel<NT, MQ, true> : dep_reg_kernel<NT, MQ, false>; }
-inline DepRegKernel dep_reg_pick(int sessions, int steps, bool diag) {
-  if (sessions <= 8) return steps <= 8 ? dep_reg_pick<1, 8>(diag) : dep_reg_pick<1, lm::DEP_MAX_Q>(diag);
-  return steps <= 8 ? dep_reg_pick<2, 8>(diag) : dep_reg_pick<2, lm::DEP_MAX_Q>(diag);
+template <int NT, int MQ, bool FAR> inline DepRegKernel dep_reg_pick(bool diag) { return diag ? dep_reg_kernel<NT, MQ, true, FAR> : dep_reg_kernel<NT, MQ, false, FAR>; }
+inline DepRegKernel dep_reg_pick(int sessions, int steps, bool diag, bool far) {
+  if (far) return sessions <= 8 ? dep_reg_pick<1, lm::DEP_MAX_Q, true>(diag) : dep_reg_pick<2, lm::DEP_MAX_Q, true>(diag);
+  if (sessions <= 8) return steps <= 8 ? dep_reg_pick<1, 8, false>(diag) : dep_reg_pick<1, lm::DEP_MAX_Q, false>(diag);
+  return steps <= 8 ? dep_reg_pick<2, 8, false>(diag) : dep_reg_pick<2, lm::DEP_MAX_Q, false>(diag);
 }
 // 8-row pieces of the fullest CTA in the largest product
 inline int dep_reg_subs(const DepFusedConfig& c, int grid) {
   auto per_cta = [&](int rows) { return ((rows + REG_UNIT - 1) / REG_UNIT + grid - 1) / grid; };
   return std::max(std::max(per_cta(3 * c.dd), 2 * per_cta(c.F)), per_cta(c.card));
 }
-inline size_t dep_reg_smem(const DepFusedConfig& c, int grid) {
+inline size_t dep_reg_addresses(const DepFusedConfig& c) { return ((size_t)c.dep_q * (4 * c.L + 1) * 8 + 15) / 16 * 16; }      // of the frame's weights, bytes
+// Shared memory: the ring, the lists of what is asked for, the sums (or a row of logits in their place) and, where there is room, the addresses.  far: there is none, and a kernel of its
+// own reads them from memory (both in one kernel: 20 us more for a step of the 7B with one session).  16 sub-steps of 140 layers of width 64, ms: 1 session 24.1, as a chain of launches
+// 29.1; 8 sessions 23.7, dep_fused_kernel 53.2; 16 36.9, 54.7.
+inline size_t dep_reg_smem(const DepFusedConfig& c, int grid, bool* far) {
   const size_t sums = (size_t)REG_WARPS * ((dep_reg_subs(c, grid) + 1) & ~1) * REG_UNIT * (c.B <= 8 ? 10 : 18) * 4, logits = ((size_t)c.card + 1) / 2 * 4;
-  return (size_t)REG_SLOTS * REG_SLOT_BYTES + REG_WARPS * REG_ASKS * sizeof(RegAsk) + ((size_t)c.dep_q * (4 * c.L + 1) * 8 + 15) / 16 * 16 + std::max(sums, logits);
+  const size_t rest = (size_t)REG_SLOTS * REG_SLOT_BYTES + REG_WARPS * REG_ASKS * sizeof(RegAsk) + std::max(sums, logits);
+  *far = rest + dep_reg_addresses(c) > SMEM_LIMIT;
+  return rest + (*far ? 0 : dep_reg_addresses(c));
+}
+// Depformers so deep that their weights' addresses, the ring and the bare sums are more than shared memory holds are left to the other kernels (the 7B's widths with 16 sub-steps: from 178
+// layers on at one session, from 88 at 16).
+inline bool dep_reg_deep(const DepFusedConfig& c, int grid) {
+  return (size_t)REG_SLOTS * REG_SLOT_BYTES + dep_reg_addresses(c) + (size_t)REG_WARPS * dep_reg_subs(c, grid) * c.B * REG_UNIT * 4 > SMEM_LIMIT;
 }
 // words of the qkv and the barrier's, which are zeroed above 8 sessions too, and of everything
 inline size_t dep_reg_front(const DepFusedConfig& c) { return (size_t)c.B * (3 * c.dd / 2) + 16; }      // words stay on lines
 inline size_t dep_reg_words(const DepFusedConfig& c) { return dep_reg_front(c) + (size_t)c.B * (c.dd / 2 + c.dd / 2 + c.F / 2 + (c.card + 7) / 8 * 4); }
 inline bool dep_reg_takes(const DepFusedConfig& c, int grid) {
+  bool far;
   return c.B <= REG_B && c.dd % 64 == 0 && c.dd <= REG_WARPS * 64 && c.F % 8 == 0 && c.F <= REG_KC * REG_WARPS * 64 && grid >= 1 && dep_reg_subs(c, grid) <= REG_SUBS &&
-         c.B * (c.dd / DD) <= REG_WARPS * grid && dep_reg_smem(c, grid) <= SMEM_LIMIT;
+         c.B * (c.dd / DD) <= REG_WARPS * grid && !dep_reg_deep(c, grid) && dep_reg_smem(c, grid, &far) <= SMEM_LIMIT;
 }

@@ -37,6 +37,16 @@ def test_few_sessions_of_deep_depformers(fake, sessions, layers, dep_q):
     lm.close()
 
 
+@pytest.mark.parametrize("sessions", [1, 2, 3, 9, 16])
+def test_few_sessions_of_depformers_whose_addresses_lie_in_memory(fake, sessions):
+    """More addresses than fit beside the kernel's other shared memory, but no more than it took before that had grown."""
+    lm = fake_cuda.LM(fake, tiny_lm_config(depformer_dim=64, depformer_num_heads=1, depformer_dim_feedforward=96, dep_q=16, n_q=32, depformer_num_layers=150))
+    lm.begin(sessions)
+    (name,) = _dep(lm.step())
+    assert "dep_reg_kernel" in name
+    lm.close()
+
+
 @pytest.mark.parametrize("sessions", [1, 2, 3])
 @pytest.mark.parametrize("over", [dict(card=9480), dict(depformer_dim=64, depformer_num_heads=1, depformer_dim_feedforward=96, dep_q=16, n_q=32, depformer_num_layers=190)])
 def test_few_sessions_of_shapes_that_only_the_shared_memory_kernel_takes(fake, sessions, over):

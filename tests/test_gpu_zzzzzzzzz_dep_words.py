@@ -49,3 +49,32 @@ def test_sub_steps_and_replays(dep_q, monkeypatch):
                 err = (lg[k] - lw[k]).norm(dim=-1) / lw[k].norm(dim=-1)
                 assert (err[same] < 3e-2).all(), (B, k, err)
                 same &= tg[k] == tw[k]
+
+
+DEEP = dict(card=200, depformer_dim=64, depformer_num_heads=1, depformer_dim_feedforward=96, depformer_num_layers=140)
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("over,sessions", [(dict(card=9401, depformer_num_layers=8), 16), (DEEP, 1), (DEEP, 16)])
+def test_addresses_in_memory(over, sessions, monkeypatch):
+    """More weights than their addresses fit into shared memory: many rows of logits, many layers.  Replays of the graph give the launches' bits; every head's logits are the launch
+    chain's while the tokens before were the same.  Two residual additions a layer, each rounded to bf16 (2^-9) on both sides: independent errors grow with the root of their number,
+    and as much again for the roundings of the products."""
+    from moshi_b200.models import LMModel
+    cfg = dataclasses.replace(BASE, n_q=32, dep_q=16, depformer_context=16, delays=(0,) * 33, **over)
+    tol = 2 * (2 * cfg.depformer_num_layers) ** 0.5 * 2.0 ** -8
+    sd = synth_lm_state_dict(cfg, seed=5, device="cuda")
+    lms = {}
+    for name, value in (("kernel", "1"), ("chain", "0")):
+        monkeypatch.setenv("B200_DEP_FUSED", value)
+        lms[name] = LMModel(cfg, sd, device="cuda")
+    got, again, want = _frames(lms["kernel"], sessions, True, 3), _frames(lms["kernel"], sessions, False, 3), _frames(lms["chain"], sessions, False, 3)
+    same, compared = torch.ones(sessions, dtype=torch.bool, device="cuda"), 0
+    for (lg, tg), (la, ta), (lw, tw) in zip(got, again, want):
+        assert torch.equal(lg, la) and torch.equal(tg, ta)
+        for k in range(cfg.dep_q):
+            err = (lg[k] - lw[k]).norm(dim=-1) / lw[k].norm(dim=-1)
+            assert (err[same] < tol).all(), (k, err)
+            compared += int(same.sum())
+            same &= tg[k] == tw[k]
+    assert compared >= sessions
