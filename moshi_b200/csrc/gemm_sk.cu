@@ -10,8 +10,8 @@
 //     (out_proj has 32 n-tiles, the text head 250).  A tile whose k-range is cut across CTAs is
 //     finished by whichever CTA arrives last: partial accumulators go to an L2-resident workspace and
 //     are summed in CTA order, so the result is bit-reproducible and independent of arrival order.
-//   * Warp roles (192 threads): warp 0 = bulk-copy/TMA producer, warp 1 = TMEM owner + single-thread
-//     tcgen05.mma issuer, warps 2..5 = epilogue (TMEM lane quadrant = warp % 4).  Two TMEM accumulator
+//   * Warp roles (192 threads): warp 0 = bulk-copy/TMA producer, warp 1 = TMEM owner + tcgen05.mma issuer
+//     (one thread of either, or the whole warps: sk_linear), warps 2..5 = epilogue (TMEM lane quadrant = warp % 4).  Two TMEM accumulator
 //     stages let the epilogue of one segment overlap the MMAs of the next.
 #include "gemm_reg.cuh"
 #include "gemm_row.cuh"
@@ -24,7 +24,7 @@ namespace tc {
 namespace {
 
 constexpr int EPI_STORE = 0, EPI_RESADD = 1, EPI_GATE = 2;   // == lm::LIN_*
-constexpr int BLOCK_ROWS = 128, BLOCK_K = 64, UMMA_K = 16;
+constexpr int BLOCK_ROWS = 128, BLOCK_K = 64;
 constexpr int NUM_THREADS = 192;
 constexpr int TILE_BYTES = BLOCK_ROWS * BLOCK_K * 2;   // 16 KB
 constexpr int MAX_STAGES = 12;
@@ -109,7 +109,7 @@ __device__ __forceinline__ float epilogue_value(const SkParams& p, float a, floa
   return bf16_round(g / (1.f + expf(-g))) * u;     // bf16(silu(gate)) * value   (gating.py:18-20)
 }
 
-template <int EPI>
+template <int EPI, bool WARPS>      // WARPS: whole warps walk the loops of copies and products (sk_linear)
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_sk_kernel(const __grid_constant__ CUtensorMap tmap_x, const SkParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -121,7 +121,7 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmap_x, const SkParams p) {
   const uint32_t tptr = tempty0 + 16;
   uint32_t* tptr_generic = reinterpret_cast<uint32_t*>(smem_raw + (tptr - raw));
 
-  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = WARPS ? __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0) : threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int A_TILES = EPI == EPI_GATE ? 2 : 1;
   constexpr uint32_t a_bytes = A_TILES * TILE_BYTES;
   const int c = blockIdx.x;
@@ -148,42 +148,71 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmap_x, const SkParams p) {
   if (p.late) pdl_wait();
   pdl_trigger();
 
-  // both loops are walked by their whole warps, and one thread issues (tc_prims.cuh)
+  // both loops are walked by their whole warps, and one thread issues (tc_prims.cuh), or by one thread
   if (warp == 0) {
     // ===== producer: one contiguous bulk copy of the weight tile(s) + one TMA box of activations per k-block =====
     // Weights do not depend on the preceding kernel: the first `stages` weight tiles are requested before the
     // dependency wait, so under programmatic dependent launch the HBM stream starts while the producer of x
     // is still running.  The activation boxes (and everything the epilogue touches) come after pdl_wait.
-    int s = 0; uint32_t ph = 0;
-    int pre = 0;                                     // stages whose weight copy is already in flight
-    for (int si = 0; si < n_seg && pre < p.stages; ++si) {
-      const Seg sg = seg_get(p, c, n_sk, si);
-      const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
-      for (int kb = sg.kb0; kb < sg.kb1 && pre < p.stages; ++kb, src += a_bytes, ++pre) {
-        if (elected()) {
+    if constexpr (WARPS) {
+      int s = 0; uint32_t ph = 0;
+      int pre = 0;                                     // stages whose weight copy is already in flight
+      for (int si = 0; si < n_seg && pre < p.stages; ++si) {
+        const Seg sg = seg_get(p, c, n_sk, si);
+        const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
+        for (int kb = sg.kb0; kb < sg.kb1 && pre < p.stages; ++kb, src += a_bytes, ++pre) {
+          if (elected()) {
+            mbar_expect_tx(full0 + 8 * pre, p.stage_bytes);
+            bulk_load(base + (uint32_t)pre * p.stage_bytes, src, a_bytes, full0 + 8 * pre);
+          }
+          __syncwarp();
+        }
+      }
+      pdl_wait();
+      int item = 0;
+      for (int si = 0; si < n_seg; ++si) {
+        const Seg sg = seg_get(p, c, n_sk, si);
+        const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
+        for (int kb = sg.kb0; kb < sg.kb1; ++kb, src += a_bytes, ++item) {
+          const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
+          if (item >= pre) mbar_wait(empty0 + 8 * s, ph ^ 1u);
+          if (elected()) {
+            if (item >= pre) {
+              mbar_expect_tx(full0 + 8 * s, p.stage_bytes);
+              bulk_load(sa, src, a_bytes, full0 + 8 * s);
+            }
+            tma_load_2d(sa + a_bytes, &tmap_x, full0 + 8 * s, kb * (p.i8 ? 2 * BLOCK_K : BLOCK_K), 0);   // 128 bytes of K either way
+          }
+          __syncwarp();
+          if (++s == p.stages) { s = 0; ph ^= 1u; }
+        }
+      }
+    } else if (lane == 0) {
+      int s = 0; uint32_t ph = 0;
+      int pre = 0;                                   // stages whose weight copy is already in flight
+      for (int si = 0; si < n_seg && pre < p.stages; ++si) {
+        const Seg sg = seg_get(p, c, n_sk, si);
+        const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
+        for (int kb = sg.kb0; kb < sg.kb1 && pre < p.stages; ++kb, src += a_bytes, ++pre) {
           mbar_expect_tx(full0 + 8 * pre, p.stage_bytes);
           bulk_load(base + (uint32_t)pre * p.stage_bytes, src, a_bytes, full0 + 8 * pre);
         }
-        __syncwarp();
       }
-    }
-    pdl_wait();
-    int item = 0;
-    for (int si = 0; si < n_seg; ++si) {
-      const Seg sg = seg_get(p, c, n_sk, si);
-      const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
-      for (int kb = sg.kb0; kb < sg.kb1; ++kb, src += a_bytes, ++item) {
-        const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
-        if (item >= pre) mbar_wait(empty0 + 8 * s, ph ^ 1u);
-        if (elected()) {
+      pdl_wait();
+      int item = 0;
+      for (int si = 0; si < n_seg; ++si) {
+        const Seg sg = seg_get(p, c, n_sk, si);
+        const uint8_t* src = p.wt + ((size_t)sg.tile * p.num_kb + sg.kb0) * a_bytes;
+        for (int kb = sg.kb0; kb < sg.kb1; ++kb, src += a_bytes, ++item) {
+          const uint32_t sa = base + (uint32_t)s * p.stage_bytes;
           if (item >= pre) {
+            mbar_wait(empty0 + 8 * s, ph ^ 1u);
             mbar_expect_tx(full0 + 8 * s, p.stage_bytes);
             bulk_load(sa, src, a_bytes, full0 + 8 * s);
           }
           tma_load_2d(sa + a_bytes, &tmap_x, full0 + 8 * s, kb * (p.i8 ? 2 * BLOCK_K : BLOCK_K), 0);   // 128 bytes of K either way
+          if (++s == p.stages) { s = 0; ph ^= 1u; }
         }
-        __syncwarp();
-        if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 1) {
@@ -191,31 +220,64 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmap_x, const SkParams p) {
     const uint32_t idesc = p.i8 ? make_idesc_i8(BLOCK_ROWS, p.Mpad) : make_idesc(BLOCK_ROWS, p.Mpad);
     int s = 0; uint32_t ph = 0;
     int acc = 0; uint32_t acc_bits = 0u;         // bit a = phase parity of accumulator stage a
-    for (int si = 0; si < n_seg; ++si) {
-      const Seg sg = seg_get(p, c, n_sk, si);
-      mbar_wait(tempty0 + 8 * acc, ((acc_bits >> acc) & 1u) ^ 1u);          // epilogue has drained this accumulator
-      tc_fence_after();
-      const uint32_t d0 = tmem_base + (uint32_t)(acc * p.acc_cols);
-      for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-        mbar_wait(full0 + 8 * s, ph);
+    if constexpr (WARPS) {
+      for (int si = 0; si < n_seg; ++si) {
+        const Seg sg = seg_get(p, c, n_sk, si);
+        mbar_wait(tempty0 + 8 * acc, ((acc_bits >> acc) & 1u) ^ 1u);          // epilogue has drained this accumulator
         tc_fence_after();
-        if (!p.stream_only) {
-          const uint32_t sa = desc_low(base + (uint32_t)s * p.stage_bytes), accum = kb == sg.kb0 ? 0u : 1u;
-          // one MMA consumes 32 bytes of K per row either way: 16 bf16 or 32 int8
-          if (p.i8) {
-            umma_block_i8(d0, sa, a_bytes >> 4, idesc, accum);
-            if (EPI == EPI_GATE) umma_block_i8(d0 + (uint32_t)p.Mpad, sa + (TILE_BYTES >> 4), (a_bytes - TILE_BYTES) >> 4, idesc, accum);
-          } else {
-            umma_block<1>(d0, sa, a_bytes >> 4, idesc, accum);
-            if (EPI == EPI_GATE) umma_block<1>(d0 + (uint32_t)p.Mpad, sa + (TILE_BYTES >> 4), (a_bytes - TILE_BYTES) >> 4, idesc, accum);
+        const uint32_t d0 = tmem_base + (uint32_t)(acc * p.acc_cols);
+        for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+          mbar_wait(full0 + 8 * s, ph);
+          tc_fence_after();
+          if (!p.stream_only) {
+            const uint32_t sa = desc_low(base + (uint32_t)s * p.stage_bytes), accum = kb == sg.kb0 ? 0u : 1u;
+            // one MMA consumes 32 bytes of K per row either way: 16 bf16 or 32 int8
+            if (p.i8) {
+              umma_block_i8(d0, sa, a_bytes >> 4, idesc, accum);
+              if (EPI == EPI_GATE) umma_block_i8(d0 + (uint32_t)p.Mpad, sa + (TILE_BYTES >> 4), (a_bytes - TILE_BYTES) >> 4, idesc, accum);
+            } else {
+              umma_block<1>(d0, sa, a_bytes >> 4, idesc, accum);
+              if (EPI == EPI_GATE) umma_block<1>(d0 + (uint32_t)p.Mpad, sa + (TILE_BYTES >> 4), (a_bytes - TILE_BYTES) >> 4, idesc, accum);
+            }
           }
+          commit_elected(empty0 + 8 * s);        // frees the smem stage once these MMAs have read it
+          if (++s == p.stages) { s = 0; ph ^= 1u; }
         }
-        commit_elected(empty0 + 8 * s);          // frees the smem stage once these MMAs have read it
-        if (++s == p.stages) { s = 0; ph ^= 1u; }
+        commit_elected(tfull0 + 8 * acc);        // segment accumulated
+        acc_bits ^= 1u << acc;
+        if (p.n_acc == 2) acc ^= 1;
       }
-      commit_elected(tfull0 + 8 * acc);          // segment accumulated
-      acc_bits ^= 1u << acc;
-      if (p.n_acc == 2) acc ^= 1;
+    } else if (lane == 0) {
+      for (int si = 0; si < n_seg; ++si) {
+        const Seg sg = seg_get(p, c, n_sk, si);
+        mbar_wait(tempty0 + 8 * acc, ((acc_bits >> acc) & 1u) ^ 1u);
+        tc_fence_after();
+        const uint32_t d0 = tmem_base + (uint32_t)(acc * p.acc_cols);
+        for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+          mbar_wait(full0 + 8 * s, ph);
+          tc_fence_after();
+          if (!p.stream_only) {
+            const uint32_t sa = base + (uint32_t)s * p.stage_bytes, sb = sa + a_bytes;
+#pragma unroll
+            for (int k = 0; k < BLOCK_K * 2; k += 32) {
+              const uint64_t db = make_desc(sb + k);
+              const uint32_t accum = (kb == sg.kb0 && k == 0) ? 0u : 1u;
+              if (p.i8) {
+                umma_i8(d0, make_desc(sa + k), db, idesc, accum);
+                if (EPI == EPI_GATE) umma_i8(d0 + (uint32_t)p.Mpad, make_desc(sa + TILE_BYTES + k), db, idesc, accum);
+              } else {
+                umma_bf16(d0, make_desc(sa + k), db, idesc, accum);
+                if (EPI == EPI_GATE) umma_bf16(d0 + (uint32_t)p.Mpad, make_desc(sa + TILE_BYTES + k), db, idesc, accum);
+              }
+            }
+          }
+          umma_commit(empty0 + 8 * s);
+          if (++s == p.stages) { s = 0; ph ^= 1u; }
+        }
+        umma_commit(tfull0 + 8 * acc);
+        acc_bits ^= 1u << acc;
+        if (p.n_acc == 2) acc ^= 1;
+      }
     }
     __syncwarp();
   } else {
@@ -722,7 +784,8 @@ int init_once() {
   }
   static std::atomic<uint64_t> limits{0};
   // the kernels also have a few bytes of static shared memory
-  B200_TRY(allow_smem(limits, 220 * 1024, gemm_sk_kernel<EPI_STORE>, gemm_sk_kernel<EPI_RESADD>, gemm_sk_kernel<EPI_GATE>, gemm_ck_kernel<EPI_STORE>, gemm_ck_kernel<EPI_RESADD>));
+  B200_TRY(allow_smem(limits, 220 * 1024, gemm_sk_kernel<EPI_STORE, false>, gemm_sk_kernel<EPI_RESADD, false>, gemm_sk_kernel<EPI_GATE, false>, gemm_sk_kernel<EPI_GATE, true>,
+                      gemm_ck_kernel<EPI_STORE>, gemm_ck_kernel<EPI_RESADD>));
   if (!g_settings_read) {
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
@@ -970,6 +1033,11 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   while (pow2 < cols) pow2 <<= 1;
   p.tmem_cols = pow2;
   p.stream_only = tune.stream_only;
+  // Loops walked by whole warps or by one thread (gated pairs; plain products: one thread).  Whole warps are ahead where the CTAs' tiles are whole, where few tiles leave each little to
+  // stream, and where long tiles come in more than one round; the tiles in between, and plain products, they made slower.  24 rows, one thread / warps, us.  Gated, k 2048: 22 tiles 23.1 /
+  // 21.5, 44 29.0 / 28.1, 80 32.9 / 35.8, 148 31.4 / 30.1, 152 45.9 / 37.8, 170 56.1 / 57.9; k 1024: 200 tiles 39.3 / 46.0, 260 44.0 / 49.6; k 4096: 88 51.9 / 53.1, 112 59.4 / 60.0, 148 53.7 /
+  // 51.9, 200 79.8 / 80.1; k 8192: 88 79.0 / 78.4, 130 84.6 / 86.5, 148 99.6 / 95.7, 200 142.8 / 133.6.  Plain 1024 -> 32000 25.2 / 27.9, 2048 -> 32000 32.9 / 37.7.
+  const bool warps = split ? 2 * p.n_tiles <= g_sms || (p.whole_rounds > 0 && p.num_kb >= 80) : p.num_kb < 128 || p.n_tiles >= g_sms;
   const CUtensorMap* mx = nullptr;
   if (i8) B200_TRY(x_map(cache, tune.xq, K, M, K, p.Mpad, 1, &mx));
   else B200_TRY(x_map(cache, x, ldx, M, K, p.Mpad, 2, &mx));
@@ -981,10 +1049,9 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = tune.pdl ? 1 : 0;
-  cudaError_t le;
-  if (epi == EPI_STORE) le = cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_STORE>, *mx, p);
-  else if (epi == EPI_RESADD) le = cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_RESADD>, *mx, p);
-  else le = cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_GATE>, *mx, p);
+  const cudaError_t le = epi == EPI_STORE ? cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_STORE, false>, *mx, p)
+                         : epi == EPI_RESADD ? cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_RESADD, false>, *mx, p)
+                         : warps ? cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_GATE, true>, *mx, p) : cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_GATE, false>, *mx, p);
   if (le != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "gemm_sk launch failed: %s", cudaGetErrorString(le));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return check_launch("gemm_sk");

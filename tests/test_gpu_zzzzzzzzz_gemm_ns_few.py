@@ -12,7 +12,8 @@ from .util import cptr
 pytestmark = pytest.mark.gpu
 STORE, RESIDUAL, GATED = 0, 1, 2
 SHAPES = [(130, 144, STORE), (264, 4112, RESIDUAL), (75 * 128, 80, RESIDUAL), (149 * 128 - 8, 256, STORE), (2 * 392, 336, GATED), (4096, 1024, RESIDUAL),
-          (2 * 2824, 592, GATED), (2 * (148 * 32 + 8), 128, GATED), (2 * 18952, 80, GATED), (37896, 144, STORE)]
+          (2 * 2824, 592, GATED), (2 * (148 * 32 + 8), 128, GATED), (2 * 18952, 80, GATED), (37896, 144, STORE),
+          (2 * 11264, 512, GATED), (2 * 25600, 1024, GATED)]
 
 
 def _stream():

@@ -4,7 +4,7 @@ import ctypes as C
 import pytest
 
 from . import fake_cuda
-from .test_gpu_zzzzzzzz_op_launches import LINEARS, RESADD, WRITERS, linear
+from .test_gpu_zzzzzzzz_op_launches import GATE, LINEARS, RESADD, STORE, WRITERS, linear
 
 
 def _kernel(fake, shape):
@@ -21,6 +21,14 @@ def test_linears_of_the_early_launch_tests_take_the_kernels_they_name(tmp_path):
     for kernel, shapes in [*LINEARS.items(), *((k, [s]) for k, s in WRITERS.items())]:
         for shape in shapes:
             assert kernel in _kernel(fake, shape), (kernel, shape)
+
+
+@pytest.mark.parametrize("shape,kernel", [((24, 32000, 2048, STORE, False), "gemm_sk_kernelILi0ELb0E"), *(((24, 256 * tiles, k, GATE, False), "gemm_sk_kernelILi2ELb" + str(int(warps)) + "E")
+                                          for tiles, k, warps in [(22, 2048, True), (74, 1024, True), (75, 1024, False), (88, 4096, False), (130, 4096, True), (130, 8192, False), (148, 8192, True),
+                                                                  (152, 1024, True), (200, 1024, False), (200, 4096, False), (200, 5120, True)])])
+def test_who_walks_the_loops_of_the_swapped_kernel(tmp_path, shape, kernel):
+    """Whole warps for gated pairs in whole tiles, in few tiles and in long ones of several rounds; one thread elsewhere."""
+    assert kernel in _kernel(fake_cuda.load(tmp_path), shape)
 
 
 @pytest.mark.parametrize("name", ["B200_ROW_MAX_M", "B200_GEMV_MAX_M"])
