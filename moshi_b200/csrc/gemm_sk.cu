@@ -934,9 +934,13 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   const int ck_pad = ((M + quantum - 1) / quantum) * quantum;
   const bool ck = epi != EPI_GATE && tune.no_cluster == 0 && tune.grid == 0 && M > 32 && ranks > 1 && ck_pad <= 256 && ck_pad / ranks <= 64;
   // 17..256 sessions: activations as the A operand (gemm_ns.cu, figures there).  It stores 16-byte pieces; rows that do not lie so keep the kernels below, and (bf16) its
-  // refusal above 32.  Up to 32 rows it takes k of 4096 on, where it gains most (24 rows: 4096 -> 12288 28.0 us / 19.9, int8 11264 -> 4096 18.3 / 11.0; of 2048 it would gain 2 to 4);
-  // 16-bit gated pairs of as many rows, shorter k and int8 rows above 32 of few tiles are left with the kernels that tests/test_devices_cpu.py and tests/test_op_routes_cpu.py name.
-  const bool kept = (M <= REG_MAX_M && (K < 4096 || (!i8 && epi == EPI_GATE))) || (i8 && ck);
+  // refusal above 32.  Up to 32 rows it takes k of 4096 on, where it gains most (24 rows: 4096 -> 12288 28.0 us / 19.9, int8 11264 -> 4096 18.3 / 11.0; of 2048 it would gain 2 to 4),
+  // but not few tiles of long k, which gemm_reg.cu cuts into more than four ranges (24 rows, there / here: 11264 -> 256 12.5 / 13.2, -> 640 15.2 / 13.4; 14336 -> 512 14.3 / 15.7, -> 768 16.6 /
+  // 15.8; 22016 -> 1024 21.2 / 21.9, -> 256 16.9 / 21.7; 32 rows 18.8 / 21.8, -> 640 22.4 / 22.0).  16-bit gated pairs of as many rows and int8 rows above 32 of few tiles stay with gemm_sk.cu's
+  // kernels, where this one would be ahead too (gated 4096 -> 11264, 24 rows 51.9 / 33.3; int8 4096 -> 4096, 104 rows 17.6 / 10.3): tests/test_devices_cpu.py and
+  // tests/test_op_routes_cpu.py hold them there.
+  const bool long_k = !i8 && ((M <= 24 && k_blocks >= 176 && n_tiles <= 4) || (k_blocks >= 300 && n_tiles <= (M <= 24 ? 8 : 4)));
+  const bool kept = (M <= REG_MAX_M && (K < 4096 || long_k || (!i8 && epi == EPI_GATE))) || (i8 && ck);
   const bool lines = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(rows)) & 15) == 0;
   const bool ns_fits = scaled && tune.ns >= 0 && M <= 256 && tune.grid == 0 && tune.cluster == 0 && !tune.stream_only && !tune.force_split && ns_supported(M, N, K, epi) &&
                        ldy % 8 == 0 && (!res || ldr % 8 == 0) && ((!i8 && M > REG_MAX_M) || (lines && !kept && chosen) || (!i8 && lines && tune.ns > 0));

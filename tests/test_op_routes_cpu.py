@@ -31,6 +31,13 @@ def test_who_walks_the_loops_of_the_swapped_kernel(tmp_path, shape, kernel):
     assert kernel in _kernel(fake_cuda.load(tmp_path), shape)
 
 
+@pytest.mark.parametrize("M,N,K,kernel", [(24, 512, 11264, "reg"), (24, 520, 11264, "ns"), (25, 256, 11264, "ns"), (24, 256, 11256, "reg"), (24, 256, 8192, "ns"), (24, 1024, 22016, "reg"), (24, 1032, 22016, "ns"),
+                                          (32, 512, 22016, "reg"), (32, 640, 22016, "ns"), (17, 128, 19200, "reg"), (32, 128, 19136, "ns")])
+def test_few_rows_and_tiles_of_long_k(tmp_path, M, N, K, kernel):
+    """Few tiles of long k are cut into more ranges by the kernel with weights in registers than a cluster has."""
+    assert f"gemm_{kernel}_kernel" in _kernel(fake_cuda.load(tmp_path), (M, N, K, STORE, False))
+
+
 @pytest.mark.parametrize("name", ["B200_ROW_MAX_M", "B200_GEMV_MAX_M"])
 def test_rows_up_to_which_whole_rows_per_cta_are_considered(tmp_path, monkeypatch, name):
     """The older name of the setting counts too."""
