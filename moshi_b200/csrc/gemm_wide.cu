@@ -21,6 +21,7 @@
 #include "gemm_wide.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 #include "tc_prims.cuh"
 
@@ -598,6 +599,18 @@ int launch_experts(const WideGemm& g, WideP p, int sms, cudaStream_t st) {
   return check_launch("gemm_expert");
 }
 
+// Few rows per expert: units of rows dealt over the SMs (gemm_expert_kernel) or tiles of 256 columns, a wave of them after the other?  The tiles lose what the last wave leaves idle
+// and have the longer way through a gated unit's epilogue; the units bring every CTA's rows of x once per 128 weight rows instead of 256.  How many experts have rows is the router's
+// business; as many as an even one would choose are reckoned with.  us, tiles / units, rows of x per box after the @:
+//   one wave, 2048 x 4096: 2 experts 26 / 14, 10 34 / 31, 14 of 16 (0.76 of a wave) 52.8 / 55.5 @32, 16 (0.86) 59.9 / 61.5 @8, 62.1 / 70.5 @128; 4096 x 8192, 7 (0.76) 89.8 / 99.2 @8, 6 83.7 / 79.0;
+//   more, 4096 x 4096: 15 experts (1.6 waves) 94.7 / 96.4, 60 (6.4) 304 / 308, 128 (13.8) 648 / 674;
+//   gated, 8192 x 2048: 16 experts 126 / 101 @4, 173 / 130 @128, 48 (10.8) 276 / 297 @16, 64 (13.8) 473 / 416 @128, 108 (22) 576 / 599 @32; 4096 x 1024: 58 experts 152 / 113.
+bool experts_win(const WideGemm& g, int sms) {
+  const double E = (double)g.w_rows / g.e_rows, used = E * (1. - pow(1. - 1. / E, (double)g.M)), waves = used * ceil_div(g.N, 256) / sms;
+  if (g.act == WIDE_CLAMPED_GLU || g.act == WIDE_SILU_GLU) return waves < 9. || (waves < 16. && g.max_rows >= 64);
+  return ceil(waves) * sms * 256. > used * g.N * (waves <= 1. ? 1.45 : 1.25);
+}
+
 }  // namespace
 
 bool wide_supported(const WideGemm& g) {
@@ -623,7 +636,7 @@ int wide_gemm(const WideGemm& g, cudaStream_t st) {
   if (g.tile_e) {
     p.tile_e = g.tile_e; p.tile_r0 = g.tile_r0; p.tile_n = g.tile_n; p.n_tiles = g.n_tiles; p.y_rows = g.y_rows; p.e_rows = g.e_rows;
     p.mt = g.max_tiles; p.nt = ceil_div(g.N, 256); p.splits = 1; p.kb_per = p.num_kb;
-    if (g.max_rows > 0 && g.max_rows <= WIDE_EXPERT_ROWS) return launch_experts(g, p, sms, st);      // one tile per expert
+    if (g.max_rows > 0 && g.max_rows <= WIDE_EXPERT_ROWS && experts_win(g, sms)) return launch_experts(g, p, sms, st);      // one tile per expert
     return launch<1, 256>(g, p, sms, st);
   }
   p.mt = ceil_div(g.M, 256);

@@ -58,3 +58,15 @@ def test_attention_steps_refuse_null_pointers(tmp_path, q8):
         at = [None if i == gone else C.addressof(p) for i in range(8 if q8 else 6)]
         rc = fake.b200_op_attn_step_q8(*at, 1, 2, 8, 0, 1e4, 1, None) if q8 else fake.b200_op_attn_step(*at, 1, 2, 8, 0, 1e4, None)
         assert rc != 0 and not fake_cuda.launches(fake)
+
+
+@pytest.mark.parametrize("counts,N,K,act,units", [([1] * 2 + [0] * 14, 2048, 4096, 0, True), ([8] * 16, 2048, 4096, 0, False), ([128] + [8] * 15, 2048, 4096, 0, False), ([1] * 10 + [0] * 6, 2048, 4096, 0, True),
+                                                  ([4] * 16, 8192, 2048, 2, True), ([16] * 16, 4096, 4096, 0, False), ([2] * 64, 8192, 2048, 3, False), ([64] * 64, 8192, 2048, 3, True),
+                                                  ([129] + [1] * 15, 8192, 2048, 2, False)])
+def test_products_of_few_rows_per_expert(tmp_path, counts, N, K, act, units):
+    """Units of weight rows dealt over the SMs where tiles would leave a last wave idle or have a gated unit behind them, tiles elsewhere and above 128 rows."""
+    fake, p = fake_cuda.load(tmp_path), C.create_string_buffer(256)
+    at, E = C.c_void_p((C.addressof(p) + 15) // 16 * 16), len(counts)
+    fake_cuda.check(fake, fake.b200_op_grouped_wide(at, at, at, (C.c_int32 * E)(*counts), E, sum(counts), N, K, N, act, 1.0, None))
+    ((_, name),) = fake_cuda.launches(fake)
+    assert ("gemm_expert_kernel" if units else "gemm_wide_kernel") in name
