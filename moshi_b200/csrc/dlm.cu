@@ -794,10 +794,15 @@ int finalize_sandwich_layer(b200_dlm* h, int i, std::vector<void*>& drop) {
 template <typename T>
 int small_proj(b200_dlm* h, const T* x, long long ldx, const void* w, const float* b, float* out, int M, int N, int K) {
   static std::atomic<uint64_t> limits{0};
-  B200_TRY(allow_smem(limits, 200 * 1024, (small_proj_f32_kernel<T, 1>), (small_proj_f32_kernel<T, 4>)));
+  B200_TRY(allow_smem(limits, 200 * 1024, (small_proj_f32_kernel<T, 1>), (small_proj_f32_kernel<T, 4>), (small_proj_f32_kernel<T, 8>)));
   const int vec = K % 8 == 0 && (ldx * sizeof(T)) % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
   const size_t row = (size_t)K * sizeof(T);
-  if (M >= 512 && 4 * row <= 100 * 1024) B200_LAUNCH((small_proj_f32_kernel<T, 4>), dim3(ceil_div(M, 4), ceil_div(N, 8)), 256, 4 * row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
+  // From 512 tokens on four of them and eight outputs to a CTA, so that few outputs spread over the chip, or eight and 32, which read less, where that many CTAs are there anyway and
+  // a CTA's rows leave room for others on its SM.  bf16 rows, four / eight tokens, us: 2048 wide, 895 tokens, 16 outputs 10.4 / 18.4, 64 24.2 / 27.6, 128 42.3 / 39.3, 256 78.8 / 68.2; 2048
+  // tokens, 64 48.2 / 50.2, 128 89.4 / 77.4, 256 171 / 142; 1024 wide 55.0 / 43.8 at 128, 104 / 80.0 at 256; 4096 wide 162 / 162 and 310 / 310.
+  const bool many = K <= 3072 && (long long)ceil_div(M, 8) * ceil_div(N, 32) >= (row <= 6144 ? 500 : 640) && 8 * row <= 100 * 1024;
+  if (M >= 512 && many) B200_LAUNCH((small_proj_f32_kernel<T, 8>), dim3(ceil_div(M, 8), ceil_div(N, 32)), 256, 8 * row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
+  else if (M >= 512 && 4 * row <= 100 * 1024) B200_LAUNCH((small_proj_f32_kernel<T, 4>), dim3(ceil_div(M, 4), ceil_div(N, 8)), 256, 4 * row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
   else EARLY_LAUNCH_IF(M < EARLY_TOKENS, (small_proj_f32_kernel<T, 1>), dim3(M, M >= 512 ? 1 : ceil_div(N, 8)), 256, row, h->stream, x, ldx, static_cast<const T*>(w), b, out, M, N, K, vec);
   return check_launch("small_proj_f32");
 }

@@ -533,8 +533,7 @@ __global__ void rows_from_f32_kernel(const float* __restrict__ in, T* __restrict
 // ---------------------------------------------------------------------------------------------------------------------------
 // Small projections whose result must be fp32 (gates of a recurrence, router logits): out[t][n] = x[t] . w[n] + b[n].  A CTA takes
 // TOK tokens (their rows in shared memory) and, over grid.y, every gridDim.y-th group of eight outputs, one warp per output: many
-// tokens share a read of the weights (four: eight left 112 CTAs for 895 tokens, each with up to four outputs per warp one after the other, 23.4 us for 16 and 32 outputs of 4096;
-// so 10.0 and 14.8), few tokens spread over the GPU.  The sum over k has the same order in every layout: a lane
+// tokens share a read of the weights (small_proj has the choice), few tokens spread over the GPU.  The sum over k has the same order in every layout: a lane
 // adds runs of eight elements (single elements where rows do not start on 16 bytes), then the lanes meet.
 // ---------------------------------------------------------------------------------------------------------------------------
 template <typename T, int TOK>

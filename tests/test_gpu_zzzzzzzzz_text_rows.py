@@ -25,10 +25,10 @@ def test_latents(rank, dtype):
 
 
 @pytest.mark.parametrize("n", [511, 512, 513, 515])
-@pytest.mark.parametrize("experts,width", [(5, 52), (16, 96), (11, 264)])
+@pytest.mark.parametrize("experts,width", [(5, 52), (16, 96), (11, 264), (250, 52), (259, 264)])
 def test_small_projections(experts, width, n):
-    """Router logits of as many tokens as fill the last CTA and of one to three more; outputs of two groups of eight that are full and not, rows on 16 bytes and off them: in
-    fp32 every logit of the model at the suite's tolerance."""
+    """Router logits of as many tokens as fill the last CTA and of one to three more; outputs of two groups of eight that are full and not, of eight and nine groups of 32 where eight tokens
+    share a CTA, rows on 16 bytes and off them: in fp32 every logit of the model at the suite's tolerance."""
     cfg = megolorn.make_cfg([megolorn.attention(2, 1, 16, 16, 0.2, chunk=64, mlp=megolorn.moe(experts, 2, 24))], vocab=97, width=width)
     model, orc = megolorn.build(cfg, torch.float32)
     toks = tokens(n, cfg.vocab, n)
@@ -58,3 +58,16 @@ def test_bits_of_latents(rank, off, dtype):
         s = s + s[:, torch.arange(32, device="cuda") ^ o]
     rs = 1.0 / torch.sqrt(s[:, :1] / torch.full((T, 1), float(rank), device="cuda") + torch.tensor(eps, device="cuda"))      # by a number torch would multiply with its inverse
     assert torch.equal(out, (raw * rs * weight).to(dtype))
+
+
+@pytest.mark.parametrize("experts,width,n,tok", [(16, 96, 512, 4), (270, 96, 504, 1), (270, 96, 512, 8), (100, 96, 992, 4), (100, 96, 1000, 8), (100, 3072, 1000, 8), (100, 3080, 1000, 4)])
+def test_tokens_that_share_a_projection(experts, width, n, tok):
+    """Eight tokens and 32 outputs to a CTA where there are many such CTAs, four and eight outputs elsewhere, one below 512 tokens."""
+    from torch.profiler import ProfilerActivity, profile
+    cfg = megolorn.make_cfg([megolorn.attention(2, 1, 16, 16, 0.2, chunk=64, mlp=megolorn.moe(experts, 2, 24))], vocab=97, width=width)
+    model, _ = megolorn.build(cfg, torch.bfloat16)
+    with gen_for(model, capacity=1024, max_step_tokens=1024) as gen, profile(activities=[ProfilerActivity.CUDA]) as prof:
+        gen.step([(0, tokens(n, cfg.vocab, n))], [0])
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "small_proj_f32_kernel" in e.name]
+    assert names and all(f", {tok}>" in name for name in names), names
