@@ -40,7 +40,7 @@ namespace {
 using namespace tcp;
 
 constexpr int EPI_STORE = 0, EPI_RESADD = 1, EPI_GATE = 2;
-constexpr int BLOCK_ROWS = 128, BLOCK_K = 64, UMMA_K = 16;
+constexpr int BLOCK_ROWS = 128, BLOCK_K = 64;
 // warp 0 producer, warp 1 MMA, warps 2-17 epilogue: four per TMEM quadrant, every fourth run of 16 columns each.  The epilogue is a chain
 // of latencies per run (TMEM load, silu, store) that nothing hides.  One warp per quadrant: the gated product 22528 x 4096 took 57.5 us at
 // 104 sessions and 92.4 at 200, of which 29 did not depend on K (half the K: 43.3); four: 41.8 and 60.2.  Plain products gain 0-1 us.
@@ -50,7 +50,9 @@ constexpr int TILE_BYTES = BLOCK_ROWS * BLOCK_K * 2;
 constexpr int A_BYTES = 128 * BLOCK_K * 2;   // a block of 128 session rows x 128 bytes of k
 constexpr int MAX_STAGES = 12;
 constexpr int MAX_CS = 8;
-constexpr int TMEM_COLS = 512;               // all of it: one CTA per SM
+// All of it: one CTA per SM.  A CTA that asks for columns beside this one waits until it ends, in nobody's way, for this kernel needs nothing of the other.  None gets that far: registers
+// (576 threads of up to 96) or shared memory (200 KB) keep the CTAs of the other tensor-core kernels off the SM.
+constexpr int TMEM_COLS = 512;
 
 struct NsParams {
   int M, N, K, out_rows, gate_rows, CS, num_kb, kb_per, stages, n_tiles, unit_rows, acc_cols, mblocks, n_acc, box_rows;

@@ -784,8 +784,8 @@ int init_once() {
   }
   static std::atomic<uint64_t> limits{0};
   // the kernels also have a few bytes of static shared memory
-  B200_TRY(allow_smem(limits, 220 * 1024, gemm_sk_kernel<EPI_STORE, false>, gemm_sk_kernel<EPI_RESADD, false>, gemm_sk_kernel<EPI_GATE, false>, gemm_sk_kernel<EPI_GATE, true>,
-                      gemm_ck_kernel<EPI_STORE>, gemm_ck_kernel<EPI_RESADD>));
+  B200_TRY(allow_smem(limits, 220 * 1024, gemm_sk_kernel<EPI_STORE, false>, gemm_sk_kernel<EPI_STORE, true>, gemm_sk_kernel<EPI_RESADD, false>, gemm_sk_kernel<EPI_RESADD, true>,
+                      gemm_sk_kernel<EPI_GATE, false>, gemm_sk_kernel<EPI_GATE, true>, gemm_ck_kernel<EPI_STORE>, gemm_ck_kernel<EPI_RESADD>));
   if (!g_settings_read) {
     int dev = 0;
     B200_CUDA(cudaGetDevice(&dev));
@@ -1037,11 +1037,13 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   while (pow2 < cols) pow2 <<= 1;
   p.tmem_cols = pow2;
   p.stream_only = tune.stream_only;
-  // Loops walked by whole warps or by one thread (gated pairs; plain products: one thread).  Whole warps are ahead where the CTAs' tiles are whole, where few tiles leave each little to
-  // stream, and where long tiles come in more than one round; the tiles in between, and plain products, they made slower.  24 rows, one thread / warps, us.  Gated, k 2048: 22 tiles 23.1 /
-  // 21.5, 44 29.0 / 28.1, 80 32.9 / 35.8, 148 31.4 / 30.1, 152 45.9 / 37.8, 170 56.1 / 57.9; k 1024: 200 tiles 39.3 / 46.0, 260 44.0 / 49.6; k 4096: 88 51.9 / 53.1, 112 59.4 / 60.0, 148 53.7 /
-  // 51.9, 200 79.8 / 80.1; k 8192: 88 79.0 / 78.4, 130 84.6 / 86.5, 148 99.6 / 95.7, 200 142.8 / 133.6.  Plain 1024 -> 32000 25.2 / 27.9, 2048 -> 32000 32.9 / 37.7.
-  const bool warps = split ? 2 * p.n_tiles <= g_sms || (p.whole_rounds > 0 && p.num_kb >= 80) : p.num_kb < 128 || p.n_tiles >= g_sms;
+  // Loops walked by whole warps or by one thread?  Whole warps are ahead where the CTAs' tiles are whole, and of gated pairs also where few tiles leave each CTA little to stream and where
+  // long tiles come in more than one round; the split tiles in between they make slower.  24 rows, one thread / warps, us.  Gated, k 2048: 22 tiles 23.1 / 21.5, 44 29.0 / 28.1, 80 32.9 /
+  // 35.8, 148 31.4 / 30.1, 152 45.9 / 37.8, 170 56.1 / 57.9; k 1024: 200 tiles 39.3 / 46.0, 260 44.0 / 49.6; k 4096: 88 51.9 / 53.1, 112 59.4 / 60.0, 148 53.7 / 51.9, 200 79.8 / 80.1; k 8192:
+  // 88 79.0 / 78.4, 130 84.6 / 86.5, 148 99.6 / 95.7, 200 142.8 / 133.6.  Plain, k 2048: 149 tiles whole 32.4 / 19.3, 192 split 29.8 / 32.7, 250 32.9 / 37.5, 297 whole 46.0 / 28.8; k 3072: 400
+  // split 62.7 / 59.2; int8, 200 rows, 11264 -> 2048 in whole tiles 56.6 / 45.6.
+  const bool gate = epi == EPI_GATE;
+  const bool warps = split ? gate && (2 * p.n_tiles <= g_sms || (p.whole_rounds > 0 && p.num_kb >= 80)) : !gate || p.num_kb < 128 || p.n_tiles >= g_sms;
   const CUtensorMap* mx = nullptr;
   if (i8) B200_TRY(x_map(cache, tune.xq, K, M, K, p.Mpad, 1, &mx));
   else B200_TRY(x_map(cache, x, ldx, M, K, p.Mpad, 2, &mx));
@@ -1053,9 +1055,10 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = tune.pdl ? 1 : 0;
-  const cudaError_t le = epi == EPI_STORE ? cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_STORE, false>, *mx, p)
-                         : epi == EPI_RESADD ? cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_RESADD, false>, *mx, p)
-                         : warps ? cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_GATE, true>, *mx, p) : cudaLaunchKernelEx(&cfg, gemm_sk_kernel<EPI_GATE, false>, *mx, p);
+  void (*kernel)(const CUtensorMap, const SkParams) =
+      epi == EPI_STORE ? (warps ? gemm_sk_kernel<EPI_STORE, true> : gemm_sk_kernel<EPI_STORE, false>) : epi == EPI_RESADD ? (warps ? gemm_sk_kernel<EPI_RESADD, true> : gemm_sk_kernel<EPI_RESADD, false>)
+                       : (warps ? gemm_sk_kernel<EPI_GATE, true> : gemm_sk_kernel<EPI_GATE, false>);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, *mx, p);
   if (le != cudaSuccess) B200_FAIL(B200_ERR_CUDA, "gemm_sk launch failed: %s", cudaGetErrorString(le));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return check_launch("gemm_sk");

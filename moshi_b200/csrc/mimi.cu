@@ -439,21 +439,21 @@ int run_transformer(b200_mimi* h, Transformer& tr, const float* x_in, float* x, 
       };
       LinP q = lin(cur, L.w_in, 3 * d, d, LIN_STORE, h->tr_qkv);
       q.gamma = L.n1w; q.beta = L.n1b;
-      B200_TRY(lin_launch(q, h->body));
+      B200_TRY(lin_launch(q, h->sms, h->body));
       MimiAttn a;
       a.qkv = h->tr_qkv; a.kc = L.kc; a.vc = L.vc; a.out = h->tr_ao_hi; a.out_lo = nullptr; a.offset = tr.offset; a.exec_mask = h->exec_mask; a.H = H; a.cap = c.tr_context;
       a.context = c.tr_context; a.neg_log_period_2_over_d = nl;
       B200_TRY(attn_launch(a, B, T, h->body));
       q = lin(h->tr_ao_hi, L.w_out, d, d, LIN_RESIDUAL, x);
       q.res = cur; q.scale = L.ls1;
-      B200_TRY(lin_launch(q, h->body));
+      B200_TRY(lin_launch(q, h->sms, h->body));
       q = lin(x, L.w_1, c.tr_dim_feedforward, d, LIN_GELU, h->tr_h_hi);
       q.gamma = L.n2w; q.beta = L.n2b;
-      B200_TRY(lin_launch(q, h->body));
+      B200_TRY(lin_launch(q, h->sms, h->body));
       q = lin(h->tr_h_hi, L.w_2, d, c.tr_dim_feedforward, LIN_RESIDUAL, x);
       const mtc::TcParams& e = L.l2.p;           // the decoder's last layer also feeds dec[0]
       q.res = x; q.scale = L.ls2; q.a_hi = e.a_hi; q.a_lo = e.a_lo; q.a_sb = e.a_sb; q.a_row = e.a_row; q.a_elu = e.act_elu;
-      B200_TRY(lin_launch(q, h->body));
+      B200_TRY(lin_launch(q, h->sms, h->body));
     }
     return check_launch("mimi transformer");
   }
@@ -545,7 +545,7 @@ int encode_body(b200_mimi* h) {
     LinP p;
     memset(&p, 0, sizeof(p));
     p.x = h->down_x; p.w = l.w; p.n_tok = h->batch; p.N = l.cout; p.K = l.k * l.cin; p.T = 1; p.epi = LIN_STORE; p.y = h->latent;
-    B200_TRY(lin_launch(p, h->body));
+    B200_TRY(lin_launch(p, h->sms, h->body));
   } else {
     const DownLayer& l = h->down;
     ConvP p;
@@ -606,7 +606,7 @@ int quantize_frame(b200_mimi* h, const float* lat, long long* codes, long long c
   LinP p;
   memset(&p, 0, sizeof(p));
   p.x = lat; p.w = h->w_rvq_in; p.n_tok = Q; p.N = 2 * RVL_D; p.K = c.dimension; p.T = 1; p.epi = LIN_STORE; p.y = h->rvq_proj;
-  B200_TRY(lin_launch(p, h->body));
+  B200_TRY(lin_launch(p, h->sms, h->body));
   int levels[2];
   levels[0] = std::min(c.q_n_semantic, h->num_codebooks);
   levels[1] = h->num_codebooks - levels[0];
@@ -668,7 +668,7 @@ int dequantize_frame(b200_mimi* h, const long long* codes, long long cs_b, long 
   LinP p;
   memset(&p, 0, sizeof(p));
   p.x = h->rvq_sum; p.w = h->w_rvq_out; p.n_tok = h->batch; p.N = c.dimension; p.K = 2 * RVL_D; p.T = 1; p.epi = LIN_STORE; p.y = out;
-  B200_TRY(lin_launch(p, h->body));
+  B200_TRY(lin_launch(p, h->sms, h->body));
   return check_launch("rvq_decode");
 }
 

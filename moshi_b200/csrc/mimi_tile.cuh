@@ -143,7 +143,7 @@ int tile_launch_one(const LinP& p, cudaStream_t st, bool early) {
 //   16 9.8 / 4.9 / 6.5, 32 13.0 / 5.7 / 7.4, 48 13.2 / - / 9.1, 64 13.4 / 10.8 / 9.4
 // Here the smallest token tile is the best one with which the CTAs fit the chip together, two to an SM (one with two stages).
 // early: the launch may begin under the preceding kernel, which does not write the weights
-inline int lin_launch(const LinP& p, cudaStream_t st, bool early = mtc::tc_pdl()) {
+inline int lin_launch(const LinP& p, int sms, cudaStream_t st, bool early = mtc::tc_pdl()) {
   if (p.K % 2048 == 0 && !p.gamma) {
     if (p.n_tok <= 2) return lin_launch_one<1, 2, 16>(p, st, early);
     if (p.n_tok <= 4) return lin_launch_one<1, 4, 16>(p, st, early);
@@ -151,10 +151,10 @@ inline int lin_launch(const LinP& p, cudaStream_t st, bool early = mtc::tc_pdl()
     if (p.n_tok <= 32) return lin_launch_one<2, 8, 8>(p, st, early);
   } else if (p.n_tok <= 2) {
     return lin_launch_one<1, 2, 4>(p, st, early);
-  } else if (p.n_tok <= 8 && p.N <= 4 * 148) {   // one output per warp, one CTA per SM
+  } else if (p.n_tok <= 8 && p.N <= 4 * sms) {   // one output per warp, one CTA per SM
     return p.n_tok <= 4 ? lin_launch_one<1, 4, 4>(p, st, early) : lin_launch_one<2, 8, 4>(p, st, early);
   }
-  const int wide = p.N / 32, room = p.K > TILE_K ? 148 : 2 * 148;
+  const int wide = p.N / 32, room = p.K > TILE_K ? sms : 2 * sms;
   if (p.N % 32) return tile_launch_one<2, 4>(p, st, early);
   if (p.n_tok <= 4) return tile_launch_one<2, 1>(p, st, early);
   if (wide * ceil_div(p.n_tok, 4) <= room) return tile_launch_one<4, 1>(p, st, early);

@@ -348,7 +348,10 @@ int b200_op_mimi_linear(const float* x_dev, const float* gamma_dev, const float*
   memset(&p, 0, sizeof(p));
   p.x = x_dev; p.gamma = gamma_dev; p.beta = beta_dev; p.w = w_dev; p.n_tok = M; p.N = N; p.K = K; p.T = 1; p.epi = epi; p.y = y_dev; p.res = res_dev; p.scale = scale_dev;
   p.eps = 1e-5f;
-  B200_TRY(lin_launch(p, static_cast<cudaStream_t>(stream), false));
+  int dev = 0, sms = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  B200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  B200_TRY(lin_launch(p, sms, static_cast<cudaStream_t>(stream), false));
   return check_launch("op_mimi_linear");
 }
 int b200_op_tc_linear_f32(const float* x_dev, const float* w_dev, float* y_dev, int M, int N, int K, void* stream) {

@@ -1,6 +1,6 @@
-"""GPU: linears of 17 rows on through gemm_ns_kernel by the general entry points: boxes of as many activation rows as there are (to whole eights), what the tensor cores read
-beyond them, accumulators taken in turn, int8; output rows shared
-out in sixteens: units inside a tile, across two or three, a last one that is not full, one more wave."""
+"""GPU: gemm_ns_kernel from 17 rows on: boxes of as many activation rows as there are (to whole eights), what the tensor cores read beyond them, accumulators taken in turn, int8;
+output rows shared out in sixteens: units inside a tile, across two or three, a last one that is not full, one more wave.  By its own entry point at every shape, and by the general
+ones, which send some of the shapes of up to 32 rows to gemm_reg.cu and gemm_sk.cu (`general` has the kernel of each; test_op_routes_cpu.py holds it to that)."""
 import ctypes as C
 
 import pytest
@@ -13,7 +13,21 @@ pytestmark = pytest.mark.gpu
 STORE, RESIDUAL, GATED = 0, 1, 2
 SHAPES = [(130, 144, STORE), (264, 4112, RESIDUAL), (75 * 128, 80, RESIDUAL), (149 * 128 - 8, 256, STORE), (2 * 392, 336, GATED), (4096, 1024, RESIDUAL),
           (2 * 2824, 592, GATED), (2 * (148 * 32 + 8), 128, GATED), (2 * 18952, 80, GATED), (37896, 144, STORE),
-          (2 * 11264, 512, GATED), (2 * 25600, 1024, GATED)]
+          (2 * 11264, 512, GATED), (2 * 25600, 1024, GATED), (2 * 392, 4112, GATED), (2 * 2824, 4112, GATED), (2 * 18952, 4112, GATED), (149 * 128 - 8, 4112, STORE), (4096, 4112, RESIDUAL)]
+ROWS = [17, 24, 25, 32, 33, 127, 129, 136, 256]
+
+
+def general(M, N, K, epi, i8):
+    """The kernels, one of which the general entry points take for these shapes."""
+    if i8 and M > 32:
+        tiles, blocks, ranks = -(-N // 128), -(-K // 128), 1            # few tiles: k over a cluster, each of whose CTAs finishes up to 64 rows
+        while ranks < 8 and tiles * ranks * 2 <= 148 and blocks >= 8 * ranks and (ranks < 4 or tiles <= 15):
+            ranks *= 2
+        pad = -(-M // (8 * ranks)) * 8 * ranks
+        return ("gemm_ck", "gemm_sk") if epi != GATED and ranks > 1 and pad <= 256 and pad <= 64 * ranks else ("gemm_sk",) if N % 8 else ("gemm_ns",)
+    if M > 32 or (K >= 4096 and (i8 or epi != GATED)):
+        return ("gemm_ns",)
+    return ("gemm_sk",) if epi == GATED or (not i8 and N > 148 * 128) else ("gemm_reg",)
 
 
 def _stream():
@@ -29,7 +43,7 @@ def _case(M, N, K, epi, whole):
     return x, w, torch.randn(M, N, generator=g).bfloat16().cuda() if epi == RESIDUAL else None, N // 2 if epi == GATED else 0
 
 
-@pytest.mark.parametrize("M", [17, 24, 25, 32, 33, 127, 129, 136, 256])
+@pytest.mark.parametrize("M", ROWS)
 @pytest.mark.parametrize("N,K,epi", SHAPES)
 def test_int8(M, N, K, epi):
     """Whole numbers, scaled by the same three products and rounded once: the bits of the plain computation; gated: the unit's two roundings apart (a bf16 step each of unit and
@@ -58,11 +72,14 @@ def test_int8(M, N, K, epi):
     assert (y[M] == 7.0).all()
 
 
-@pytest.mark.parametrize("M", [17, 24, 25, 32])
+@pytest.mark.parametrize("M", ROWS)
 @pytest.mark.parametrize("N,K,epi", SHAPES)
-@pytest.mark.parametrize("shift", [0, 1])
-def test_bf16(M, N, K, epi, shift):
-    """Every sum within the bound of K products in fp32, the epilogue's bf16 roundings behind it; results on a 16-byte border and (other kernels) not."""
+@pytest.mark.parametrize("entry,shift", [("ns", 0), ("general", 0), ("general", 1)])
+def test_bf16(M, N, K, epi, entry, shift):
+    """Every sum within the bound of K products in fp32, the epilogue's bf16 roundings behind it; up to 32 rows by the general entry point too, with results on a 16-byte border and
+    (other kernels) not."""
+    if (entry == "general" and M > 32) or (entry == "ns" and N % 8):
+        pytest.skip("the kernel's own entry point, whose rows lie on 16 bytes")
     from moshi_b200 import _lib
     lib = _lib.lib()
     x, w, res, gate = _case(M, N, K, epi, False)
@@ -71,7 +88,10 @@ def test_bf16(M, N, K, epi, shift):
     cols = gate or N
     flat = torch.full((M * cols + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
     y = flat[shift:shift + M * cols].view(M, cols)
-    _lib.check(lib.b200_op_linear_sk(cptr(x), cptr(wt), cptr(y), cptr(res), M, N, K, epi, gate, 0, 0, 0, _stream()))
+    if entry == "ns":
+        _lib.check(lib.b200_op_linear_ns(cptr(x), cptr(wt), cptr(y), cptr(res), M, N, K, epi, gate, 0, _stream()))
+    else:
+        _lib.check(lib.b200_op_linear_sk(cptr(x), cptr(wt), cptr(y), cptr(res), M, N, K, epi, gate, 0, 0, 0, _stream()))
     z, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     err = (K + 8) * 2.0 ** -23 * size
     if epi == GATED:

@@ -4,6 +4,7 @@ import ctypes as C
 import pytest
 
 from . import fake_cuda
+from . import test_gpu_zzzzzzzzz_gemm_ns_few as ns_few
 from .test_gpu_zzzzzzzz_op_launches import GATE, LINEARS, RESADD, STORE, WRITERS, linear
 
 
@@ -23,11 +24,12 @@ def test_linears_of_the_early_launch_tests_take_the_kernels_they_name(tmp_path):
             assert kernel in _kernel(fake, shape), (kernel, shape)
 
 
-@pytest.mark.parametrize("shape,kernel", [((24, 32000, 2048, STORE, False), "gemm_sk_kernelILi0ELb0E"), *(((24, 256 * tiles, k, GATE, False), "gemm_sk_kernelILi2ELb" + str(int(warps)) + "E")
+@pytest.mark.parametrize("shape,kernel", [((24, 32000, 2048, STORE, False), "gemm_sk_kernelILi0ELb0E"), ((24, 19072, 2048, STORE, False), "gemm_sk_kernelILi0ELb1E"),
+                                          ((200, 2048, 4096, RESADD, True), "gemm_sk_kernelILi1ELb1E"), *(((24, 256 * tiles, k, GATE, False), "gemm_sk_kernelILi2ELb" + str(int(warps)) + "E")
                                           for tiles, k, warps in [(22, 2048, True), (74, 1024, True), (75, 1024, False), (88, 4096, False), (130, 4096, True), (130, 8192, False), (148, 8192, True),
                                                                   (152, 1024, True), (200, 1024, False), (200, 4096, False), (200, 5120, True)])])
 def test_who_walks_the_loops_of_the_swapped_kernel(tmp_path, shape, kernel):
-    """Whole warps for gated pairs in whole tiles, in few tiles and in long ones of several rounds; one thread elsewhere."""
+    """Whole warps where tiles are whole, for gated pairs also in few tiles and in long ones of several rounds; one thread elsewhere."""
     assert kernel in _kernel(fake_cuda.load(tmp_path), shape)
 
 
@@ -70,3 +72,13 @@ def test_products_of_few_rows_per_expert(tmp_path, counts, N, K, act, units):
     fake_cuda.check(fake, fake.b200_op_grouped_wide(at, at, at, (C.c_int32 * E)(*counts), E, sum(counts), N, K, N, act, 1.0, None))
     ((_, name),) = fake_cuda.launches(fake)
     assert ("gemm_expert_kernel" if units else "gemm_wide_kernel") in name
+
+
+@pytest.mark.parametrize("i8", [False, True])
+def test_linears_of_the_sixteens_take_the_kernels_they_name(tmp_path, i8):
+    """What the tests of gemm_ns_kernel send through the general entry points."""
+    fake = fake_cuda.load(tmp_path)
+    got = {(M, *shape): _kernel(fake, (M, *shape, i8)) for shape in ns_few.SHAPES for M in ns_few.ROWS if i8 or M <= 32}
+    wrong = {shape: name for shape, name in got.items() if not any(k + "_kernel" in name for k in ns_few.general(*shape, i8))}
+    assert not wrong
+    assert any("gemm_ns" in n for s, n in got.items() if s[0] <= 32 and s[3] == (GATE if i8 else STORE))
