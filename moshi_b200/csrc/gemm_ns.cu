@@ -60,6 +60,7 @@ struct NsParams {
   __nv_bfloat16* y; long long ldy;
   const __nv_bfloat16* res; long long ldr;
   const float *sa, *sw;                          // int8: scales of activation and weight rows
+  uint32_t block_step;                           // bytes between two blocks' sums in a cluster's shared memory (0: in the same place)
   int late;                                      // nothing is read before the wait on the preceding kernel
 };
 
@@ -315,6 +316,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
     asm volatile("bar.sync 5, 512;" ::: "memory");
   }
   for (int mb = 0; mb < p.mblocks; ++mb) {      // blocks of 128 sessions
+    const uint32_t sums = base + (uint32_t)mb * p.block_step;
     const int rows = min(128, p.M - mb * 128);
     const int row0 = (p.CS == 1 ? q4 * 32 : rows * me / p.CS) + (t >> (out_log2 - 3)), end = p.CS == 1 ? min(rows, q4 * 32 + 32) : rows * (me + 1) / p.CS;
     if (warp >= 2) {
@@ -367,7 +369,7 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
           } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              ns_sts(ns_piece(base, row, (c0 >> 2) + j, out_log2 - 2),
+              ns_sts(ns_piece(sums, row, (c0 >> 2) + j, out_log2 - 2),
                      make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3])));
           }
         }
@@ -379,18 +381,21 @@ gemm_ns_kernel(const __grid_constant__ CUtensorMap tmap_x, const NsParams p) {
       } else {
         __syncwarp();
         ns_cluster_sync();
-        ns_finish<EPI, I8>(p, base, sa, sw, mb * 128, row0, end, step, c, out_log2, nb, o_end, res);
+        ns_finish<EPI, I8>(p, sums, sa, sw, mb * 128, row0, end, step, c, out_log2, nb, o_end, res);
       }
       tc_fence_before();
     } else if (p.CS > 1) {
       __syncwarp();
       ns_cluster_sync();
     }
-    if (p.CS > 1) {
+    if (p.CS > 1 && mb + 1 < p.mblocks && p.block_step == 0) {
       __syncwarp();
-      if (mb + 1 < p.mblocks) ns_cluster_sync();      // the block's sums have been read everywhere, before the next block's take their place
-      else ns_cluster_meet();                   // nobody leaves while its sums are read
+      ns_cluster_sync();                        // the block's sums have been read everywhere, before the next block's take their place
     }
+  }
+  if (p.CS > 1) {
+    __syncwarp();
+    ns_cluster_meet();                          // nobody leaves while its sums are read
   }
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
@@ -484,6 +489,14 @@ int ns_linear(GemmPlanCache& cache, const void* x, long long ldx, const void* w_
   if (stages < 2) stages = 2;
   const size_t sums = (size_t)128 * (p.unit_rows <= 128 ? 128 : 256) * (cs > 1 ? 4 : 2);      // a block's results or partial sums, in the ring
   while ((size_t)stages * stage_bytes < sums) ++stages;
+  // a cluster's sums of two blocks lie side by side where there is room: in one place the second's have to wait until the first's have been read everywhere, and a barrier that orders this
+  // waits for the first block's results to be stored as well (4096 -> 4096, 160 sessions 18.4 us, side by side 17.5)
+  p.block_step = 0;
+  if (cs > 1 && p.mblocks > 1) {
+    int wide = stages;
+    while ((size_t)wide * stage_bytes < 2 * sums) ++wide;
+    if ((size_t)wide * stage_bytes + beyond <= 208 * 1024) { stages = wide; p.block_step = (uint32_t)sums; }
+  }
   p.stages = stages;
   p.wt = static_cast<const uint8_t*>(w_tiles);
   p.y = y; p.ldy = ldy; p.res = res; p.ldr = ldr;
