@@ -573,7 +573,8 @@ int64_t b200_op_packed_bytes(int N, int K, int epi, int gate_rows);
 int b200_op_pack_tiles(const void* w_dev, void* out_dev, int N, int K, int epi, int gate_rows, void* stream);
 int b200_op_linear_sk(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N,
                       int K, int epi, int gate_rows, int grid, int smem_budget, int stream_only, void* stream);
-/* The LM's linear kernel for 17..256 sessions (csrc/gemm_ns.cu): activations as the UMMA A operand, weight rows
+/* The LM's linear kernel for 33..256 sessions, and for 17..32 at k of 4096 and more but for bf16 gated pairs and few tiles of long k; int8 above 32 where the tiles are not few
+ * (csrc/gemm_ns.cu): activations as the UMMA A operand, weight rows
  * as B (up to 256 per tcgen05.mma), K cut over a cluster of `cluster` CTAs and reduced over distributed shared memory
  * (0 = the LM's own choice of both; else units of two tiles; 100 + n = of one, n K-splits); same packed weights and
  * epilogues as b200_op_linear_sk, any M <= 256.
@@ -581,8 +582,8 @@ int b200_op_linear_sk(const void* x_dev, const void* w_tiles_dev, void* y_dev, c
 int b200_op_linear_ns(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K,
                       int epi, int gate_rows, int cluster, void* stream);
 /* The kernel with the weights going through registers (csrc/gemm_reg.cu) at every shape that it has: up to 32 rows, gated pairs up to 16.
- * b200_op_linear_sk takes it for the gated pairs of up to 16 rows that gemm_row.cu leaves, and for 17 to 32 rows that csrc/gemm_ns.cu cannot take
- * (results off a 16-byte border) or while b200_op_set_gemv_max_rows has cut gemm_row.cu's range short. */
+ * b200_op_linear_sk takes it for the gated pairs of up to 16 rows that gemm_row.cu leaves, and for 17 to 32 rows that are not gated pairs nor (bf16) more tiles than SMs where
+ * csrc/gemm_ns.cu does not: k below 4096, few tiles of long k, results off a 16-byte border, or while b200_op_set_gemv_max_rows has cut gemm_row.cu's range short. */
 int b200_op_linear_reg(const void* x_dev, const void* w_tiles_dev, void* y_dev, const void* res_dev, int M, int N, int K, int epi, int gate_rows,
                        void* stream);
 /* The decoder LM's linear for more than 256 activation rows (csrc/gemm_wide.cu): y[M,N] = x[M,K] . w^T over packed tiles

@@ -1,4 +1,4 @@
-// tcgen05 GEMM for the LM linears at 17..256 sessions:  y[M][N] = epi(x[M][K] . w[N][K]^T), bf16 in, fp32 in TMEM, bf16 out; int8 in, exact int32 sums, scaled, bf16 out.
+// tcgen05 GEMM for the LM linears at 17..256 sessions (which of them: sk_linear):  y[M][N] = epi(x[M][K] . w[N][K]^T), bf16 in, fp32 in TMEM, bf16 out; int8 in, exact int32 sums, scaled, bf16 out.
 //
 // gemm_sk.cu feeds the 128-row weight tile as the UMMA *A* operand and the sessions as N ("swap-AB").  Here the operands keep their textbook roles:
 //
@@ -18,10 +18,10 @@
 //   * shapes with few units are cut along K over a cluster of 2..4 CTAs; every CTA adds the sums of all of them over distributed shared memory for its share of the
 //     sessions, in rank order (deterministic): no workspace, no atomics.  ns_default_plan() holds the measured choice per shape;
 //   * copies and products are issued from uniform registers (tc_prims.cuh).
-// us, one launch behind the other through the entry point with cold weights, before these / now.  104 sessions: 4096 -> 12288 27.9 / 20.6, 4096 -> 4096 16.1 / 13.3, 11264 -> 4096
+// us, launches behind one another in a graph, cold weights (launched one by one 2 us more), before these / now.  104 sessions: 4096 -> 12288 27.9 / 20.6, 4096 -> 4096 16.1 / 13.3, 11264 -> 4096
 // 26.4 / 22.1, 4096 -> 32000 50.9 / 44.0, gated -> 11264 37.9 / 33.5 (37.6 in whole tiles), gated 1024 -> 2816 12.8 / 9.0 (12.2).  48: 25.3 / 20.0, 13.5 / 10.7, 23.6 / 19.3, 48.5 /
 // 42.7, 37.1 / 33.2, 12.2 / 8.2.  256: 44.3 / 32.2, 27.5 / 21.8, 42.3 / 34.6, 70.8 / 61.2, 54.6 / 45.2, 20.5 / 12.0.  24 sessions (gemm_reg.cu, gemm_sk.cu / now): 28.0 / 19.9, 15.0 /
-// 10.0, 28.0 / 18.4, 53.5 / 42.7; gated pairs of up to 32 rows stay with those two (50.3, this kernel 33.3).  int8 (gemm_reg.cu, gemm_sk.cu / now): 24 17.6 / 11.8, 11.3 / 7.4, 18.3 / 11.0, 34.2 / 24.1, 34.5 / 20.9, 11.6 / 6.5; more than 32 of few tiles stay with gemm_sk.cu; 104
+// 10.0, 28.0 / 18.4, 53.5 / 42.7; gated pairs of up to 32 rows stay with those two (50.3, this kernel 33.3).  int8 (gemm_reg.cu, gemm_sk.cu / this kernel, which has not all of them): 24 17.6 / 11.8, 11.3 / 7.4, 18.3 / 11.0, 34.2 / 24.1, 34.5 / 20.9, 11.6 / 6.5 (k below 4096 stays); more than 32 of few tiles stay with gemm_sk.cu; 104
 // 26.5 / 12.2, 17.6 / 10.3, 23.2 / 14.4, 41.0 / 25.6, 40.5 / 22.1, 25.3 / 7.2; 256 40.4 / 17.2, 57.3 / 18.0, 88.6 / 23.2, 68.5 / 37.1, 69.8 / 32.4, 51.5 / 10.1.  A step of the 7B with 40
 // sessions 6.81 -> 6.31 ms, with 72 7.56 -> 7.11.
 //

@@ -10,7 +10,8 @@
 // the wait on the preceding kernel.  Where tiles are few, k is cut; the CTA that arrives last adds the ranges in order.
 //
 // Against the tcgen05 stream-K kernel of gemm_sk.cu: gated 4096 -> 11264, 6 rows 44.8 -> 33.3 us (185 MB of weights, 28 us at the measured copy rate); a width-2048 decoder
-// layer's linears at 8 rows 26 -> 18.6 us each.  From 17 rows on gemm_ns.cu is ahead (24 rows: 4096 -> 12288 28.0 us here, 19.9 there) and this one has what that cannot take.
+// layer's linears at 8 rows 26 -> 18.6 us each.  From 17 rows on gemm_ns.cu has k of 4096 and more (24 rows: 4096 -> 12288 28.0 us here,
+// 19.9 there) but for few tiles of long k, whose ranges are more here, and results off a 16-byte border; shorter k stays here.
 #include <algorithm>
 
 #include "gemm_reg.cuh"

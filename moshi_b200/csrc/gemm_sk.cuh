@@ -71,7 +71,7 @@ int sk_linear(GemmPlanCache& cache, const __nv_bfloat16* x, long long ldx, const
               long long ldy, const __nv_bfloat16* res, long long ldr, int M, int N, int K, int epi, int gate_rows,
               float* ws, int* counters, const SkTuning& tune, cudaStream_t stream);
 
-// ---- non-swapped kernel for 17..256 sessions (gemm_ns.cu): A = activations, B = two weight tiles (N = 256) ------------
+// ---- non-swapped kernel for 17..256 sessions (gemm_ns.cu): A = activations, B = 16 to 256 weight rows ------------
 bool ns_supported(int M, int N, int K, int epi);
 int ns_prepare();
 // cluster: K-splits (0 = the measured choice for the shape); same packed weights and epilogues as sk_linear
