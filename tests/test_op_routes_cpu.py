@@ -4,6 +4,7 @@ import ctypes as C
 import pytest
 
 from . import fake_cuda
+from . import test_gpu_zzzzzzzzz_gemm_expert as gemm_expert
 from . import test_gpu_zzzzzzzzz_gemm_ns_few as ns_few
 from .test_gpu_zzzzzzzz_op_launches import GATE, LINEARS, RESADD, STORE, WRITERS, linear
 
@@ -64,7 +65,8 @@ def test_attention_steps_refuse_null_pointers(tmp_path, q8):
 
 @pytest.mark.parametrize("counts,N,K,act,units", [([1] * 2 + [0] * 14, 2048, 4096, 0, True), ([8] * 16, 2048, 4096, 0, False), ([128] + [8] * 15, 2048, 4096, 0, False), ([1] * 10 + [0] * 6, 2048, 4096, 0, True),
                                                   ([4] * 16, 8192, 2048, 2, True), ([16] * 16, 4096, 4096, 0, False), ([2] * 64, 8192, 2048, 3, False), ([64] * 64, 8192, 2048, 3, True),
-                                                  ([129] + [1] * 15, 8192, 2048, 2, False)])
+                                                  ([129] + [1] * 15, 8192, 2048, 2, False),
+                                                  *((*case, act, not (act == 0 and case[1] == 148 * 64)) for case in gemm_expert.CASES for act in (0, 2))])
 def test_products_of_few_rows_per_expert(tmp_path, counts, N, K, act, units):
     """Units of weight rows dealt over the SMs where tiles would leave a last wave idle or have a gated unit behind them, tiles elsewhere and above 128 rows."""
     fake, p = fake_cuda.load(tmp_path), C.create_string_buffer(256)
