@@ -8,17 +8,16 @@ import torch.nn.functional as F
 from .util import cptr
 
 pytestmark = pytest.mark.gpu
-
-
-@pytest.mark.parametrize("act", [0, 2])
 CASES = [([1], 16, 64), ([1], 8, 64), ([2, 0, 1], 24, 72), ([3], 148 * 16, 64), ([3], 148 * 16 + 2, 128), ([128, 1, 127], 148 * 64, 72), ([128, 1, 127], 148 * 32, 72), ([1, 0, 128], 4096, 2048),
          ([1] * 16, 8192, 136), ([5, 2, 0, 9] * 10, 1038, 200)]
 
 
+@pytest.mark.parametrize("act", [0, 2])
 @pytest.mark.parametrize("counts,N,K", CASES)
 def test_grouped_product_of_few_rows(counts, N, K, act):
-    """(The plain product of 256 rows and 148 x 64 columns takes gemm_wide_kernel: its tiles fill three quarters of a wave.)  One unit for the whole chip, one per CTA and one more, rows that do not fill a unit, shares that span several experts, tiles of 1 to 8 units; each sum of K bf16
-    products in fp32, rounded to bf16 (2^-8 of the result; the gated unit's slope stays below 16)."""
+    """(The plain product of 256 rows and 148 x 64 columns takes gemm_wide_kernel: its tiles fill three quarters of a wave.)  One unit for the whole chip, one
+    per CTA and one more, rows that do not fill a unit, shares that span several experts, tiles of 1 to 8 units; each sum of K bf16 products in fp32, rounded to bf16 (2^-8 of the result; the
+    gated unit's slope stays below 16)."""
     from moshi_b200 import _lib
     M, E = sum(counts), len(counts)
     g = torch.Generator().manual_seed(M + N + act)
